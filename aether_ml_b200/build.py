@@ -6,12 +6,13 @@ import os
 import shutil
 import subprocess
 import sys
+from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB_PATH = os.path.join(HERE, "libaether_b200.so")
 DIGEST_PATH = LIB_PATH + ".digest"
-SOURCES = ["api.cu", "conv_tc.cu", "conv_halo.cu", "conv_halo_dw.cu", "conv_dw_rows.cu", "conv_generic.cu", "conv_smallc.cu", "conv_first_tc.cu", "layers.cu",
+SOURCES = ["api.cu", "conv_tc.cu", "conv_halo.cu", "conv_halo_dw.cu", "conv_dw_rows.cu", "conv_generic.cu", "conv_simt.cu", "conv_smallc.cu", "conv_first_tc.cu", "layers.cu",
            "block_fused.cu"]
 # tcgen05 / TMA PTX only assembles for the arch-specific target, hence compute_100a + sm_100a.
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -51,11 +52,11 @@ def build_library(force=False, verbose=False):
     """Compile the library if it is missing or older than its sources.  Returns the .so path."""
     if not force and not _stale():
         return LIB_PATH
-    objs = []
     nvcc = _nvcc()
     build_dir = os.path.join(HERE, "build")
     os.makedirs(build_dir, exist_ok=True)
-    for src in SOURCES:
+
+    def compile_one(src):
         obj = os.path.join(build_dir, src.replace(".cu", ".o"))
         cmd = [nvcc, "-c", os.path.join(CSRC, src), "-o", obj] + NVCC_FLAGS + (["-Xptxas", "-v"] if verbose else [])
         r = subprocess.run(cmd, capture_output=True, text=True)
@@ -63,7 +64,10 @@ def build_library(force=False, verbose=False):
             raise RuntimeError("nvcc failed for %s:\n%s\n%s" % (src, r.stdout, r.stderr))
         if verbose:
             print(r.stderr)
-        objs.append(obj)
+        return obj
+
+    with ThreadPoolExecutor(max_workers=os.cpu_count() or 1) as pool:
+        objs = list(pool.map(compile_one, SOURCES))
     cmd = [nvcc, "-shared", "-o", LIB_PATH] + objs + ["-gencode", "arch=compute_100a,code=sm_100a"]
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:

@@ -62,7 +62,14 @@ static inline size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; 
 static inline int ceil_div(int a, int b) { return (a + b - 1) / b; }
 static inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
-// ---- conv_generic.cu : fp32 CUDA-core convolution for any filter/stride/padding
+// ---- conv_simt.cu : fp32 CUDA-core convolution for any filter/stride/padding/channel count, tiled implicit GEMMs
+int simt_conv_fwd(const AetherConvDesc& d, const float* x, const float* w, const float* b, float* y, cudaStream_t st);
+int simt_conv_bwd_data(const AetherConvDesc& d, const float* dy, const float* w, float* dx, cudaStream_t st);
+int simt_conv_bwd_filter(const AetherConvDesc& d, const float* x, const float* dy, float* dw, float* db, void* ws,
+                         size_t ws_bytes, cudaStream_t st);
+size_t simt_conv_workspace_bytes(const AetherConvDesc& d);
+
+// ---- conv_generic.cu : classifier heads and dX of first layers on the CUDA cores; everything else goes to conv_simt.cu
 int generic_conv_fwd(const AetherConvDesc& d, const float* x, const float* w, const float* b, float* y, cudaStream_t st);
 int generic_conv_bwd_data(const AetherConvDesc& d, const float* dy, const float* w, float* dx, cudaStream_t st);
 int generic_conv_bwd_filter(const AetherConvDesc& d, const float* x, const float* dy, float* dw, float* db, void* ws,
