@@ -82,6 +82,7 @@ SIGNATURES = {
     "aether_dropout_fwd": (_I, [_P, _P, _P, _I64, _F, _U64, _U64, _P]),
     "aether_mul": (_I, [_P, _P, _P, _I64, _P]),
     "aether_adam_step": (_I, [_P, _P, _P, _P, _I64, _F, _F, _F, _F, _F, _F, _F, _P]),
+    "aether_adam_steps": (_I, [_P, _I, _F, _F, _F, _F, _F, _F, _F, _P]),
     "aether_adam_step_dev": (_I, [_P, _P, _P, _P, _I64, _F, _F, _F, _F, _F, _F, _P, _P]),
     "aether_dropout_fwd_dev": (_I, [_P, _P, _P, _I64, _F, _U64, _U64, _P, _P]),
     "aether_channel_mask_dev": (_I, [_P, _I, _F, _U64, _P, _P]),
@@ -114,6 +115,24 @@ def lib():
             fn.argtypes = args
         _lib = h
     return _lib
+
+
+_host = None
+
+
+def host():
+    """The native host path (csrc/host.cpp), bound to the loaded library; raises if it has not been built."""
+    global _host
+    if _host is None:
+        lib()
+        try:
+            from . import _host as mod
+        except ImportError as e:
+            raise AetherError("the native host module is missing or does not load (%s) -- build it with "
+                              "`python -m aether_ml_b200.build` (there is no fallback path)" % e) from None
+        mod.bind(LIB_PATH, AetherError)
+        _host = mod
+    return _host
 
 
 def check(rc, what=""):

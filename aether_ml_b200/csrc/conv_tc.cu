@@ -1010,7 +1010,7 @@ bool cta_pairs_available() {
     return v == 1;
 }
 
-static TcPlan make_plan(const AetherConvDesc& d) {
+static TcPlan compute_plan(const AetherConvDesc& d) {
     TcPlan pl{};
     pl.tf32 = (d.math_mode == AETHER_MATH_TF32);
     conv_out_hw(d, pl.Ho, pl.Wo);
@@ -1081,6 +1081,29 @@ static TcPlan make_plan(const AetherConvDesc& d) {
     return pl;
 }
 
+// The tile search above costs some ten microseconds of host time, as much as the launches of a small layer, and a
+// network asks for the same few shapes again on every pass (workspace size, operand layout, statistics blocks, forward,
+// backward): each host thread keeps the plans it used last, direct-mapped.  A plan depends on the shape and the device only.
+static const TcPlan& make_plan(const AetherConvDesc& d) {
+    struct Slot {
+        AetherConvDesc key;
+        int dev = -1;
+        TcPlan plan;
+    };
+    static thread_local Slot slots[64];
+    const int dev = current_device();
+    uint32_t h = 2166136261u;
+    const int32_t* f = reinterpret_cast<const int32_t*>(&d);
+    for (size_t i = 0; i < sizeof(d) / sizeof(int32_t); ++i) h = (h ^ (uint32_t)f[i]) * 16777619u;
+    Slot& s = slots[(h ^ (h >> 16)) & 63u];
+    if (s.dev != dev || memcmp(&s.key, &d, sizeof(d)) != 0) {
+        s.plan = compute_plan(d);
+        s.key = d;
+        s.dev = dev;
+    }
+    return s.plan;
+}
+
 bool tc_conv_eligible(const AetherConvDesc& d) {
     if (d.math_mode != AETHER_MATH_BF16 && d.math_mode != AETHER_MATH_TF32) return false;
     if (d.sH != 1 || d.sW != 1) return false;
@@ -1097,7 +1120,7 @@ size_t tc_conv_workspace_bytes(const AetherConvDesc& d) { return make_plan(d).to
 
 bool tc_conv_operand_layout(const AetherConvDesc& d, AetherOperandLayout* out) {
     if (!tc_conv_eligible(d) || d.math_mode != AETHER_MATH_BF16) return false;
-    const TcPlan pl = make_plan(d);
+    const TcPlan& pl = make_plan(d);
     out->x_copy_offset = pl.off_xsh;
     out->x_copy_ld = pl.Cin_p;
     out->dy_copy_offset = pl.off_dysh;
@@ -1255,7 +1278,7 @@ static int launch_cast(const float* src, __nv_bfloat16* dst, long long rows, int
 
 long long tc_conv_stats_blocks(const AetherConvDesc& d) {
     if (!tc_conv_eligible(d)) return 0;
-    const TcPlan pl = make_plan(d);
+    const TcPlan& pl = make_plan(d);
     const long long hb = halo_igemm_stats_blocks(pl.tf32, pl.tf32 ? d.Cin : pl.Cin_p, d.S, pl.taps, d.Cout, pl.Ho, pl.Wo,
                                                  pl.Cout_p, d.fH, d.fW);
     if (hb > 0) return hb;
@@ -1274,7 +1297,7 @@ long long tc_conv_stats_blocks(const AetherConvDesc& d) {
 
 int tc_conv_fwd(const AetherConvDesc& d, const float* x, const float* w, const float* b, float* y, float* stats, void* ws,
                 size_t ws_bytes, int flags, cudaStream_t st) {
-    const TcPlan pl = make_plan(d);
+    const TcPlan& pl = make_plan(d);
     if (ws_bytes < pl.total || !ws) return set_error(AE_BAD_ARG, "conv workspace too small: %zu < %zu", ws_bytes, pl.total);
     uint8_t* wsb = static_cast<uint8_t*>(ws);
     int rc;
@@ -1330,7 +1353,7 @@ static int launch_dw(const DwParams& p, int splits, int grid_y, cudaStream_t st)
 
 int tc_conv_bwd(const AetherConvDesc& d, const float* x, const float* dy, const float* w, float* dx, float* dw,
                 float* db, void* ws, size_t ws_bytes, int x_shadow_valid, int dy_colsum_rows, cudaStream_t st) {
-    const TcPlan pl = make_plan(d);
+    const TcPlan& pl = make_plan(d);
     if (ws_bytes < pl.total || !ws) return set_error(AE_BAD_ARG, "conv workspace too small: %zu < %zu", ws_bytes, pl.total);
     uint8_t* wsb = static_cast<uint8_t*>(ws);
     int rc;

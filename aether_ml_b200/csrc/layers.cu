@@ -979,22 +979,56 @@ __global__ void __launch_bounds__(256) mul_kernel(const float* __restrict__ a, c
 }
 
 // ====================================================================================== Adam
-// One launch updates a whole flat parameter buffer (Optimizer_Adam.update_parameters, :710-734):
+// One launch updates a whole flat parameter buffer or a list of tensors (Optimizer_Adam.update_parameters, :710-734):
 //   g' = g * gscale;  m = b1*m + (1-b1)*g';  v = b2*v + (1-b2)*g'^2
 //   p -= lr * (m / bc1) / (sqrt(v / bc2) + eps)        with bc = 1 - beta^(iterations+1)
-__global__ void __launch_bounds__(256) adam_kernel(float* __restrict__ p, const float* __restrict__ g,
-                                                   float* __restrict__ m, float* __restrict__ v, long long n, float lr,
-                                                   float b1, float b2, float eps, float inv_bc1, float inv_bc2,
-                                                   float gscale) {
-    const long long stride = (long long)gridDim.x * blockDim.x;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += stride) {
-        const float gi = g[i] * gscale;
-        const float mi = b1 * m[i] + (1.f - b1) * gi;
-        const float vi = b2 * v[i] + (1.f - b2) * gi * gi;
-        m[i] = mi;
-        v[i] = vi;
-        p[i] -= lr * (mi * inv_bc1) / (sqrtf(vi * inv_bc2) + eps);
+struct AdamScalars {
+    float lr, b1, b2, eps, inv_bc1, inv_bc2, gscale;
+};
+__device__ __forceinline__ void adam_update(const AdamScalars& a, float& p, float g, float& m, float& v) {
+    const float gi = g * a.gscale;
+    m = a.b1 * m + (1.f - a.b1) * gi;
+    v = a.b2 * v + (1.f - a.b2) * gi * gi;
+    p -= a.lr * (m * a.inv_bc1) / (sqrtf(v * a.inv_bc2) + a.eps);
+}
+// Elements first, first + step, ... of one tensor; four at a time where its arrays are 16-byte aligned (28 bytes move per
+// parameter: the update of a dense head is a pass over HBM).
+__device__ __forceinline__ void adam_range(const AdamScalars& a, float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m,
+                                           float* __restrict__ v, long long n, long long first, long long step) {
+    const bool vec = ((reinterpret_cast<uintptr_t>(p) | reinterpret_cast<uintptr_t>(g) | reinterpret_cast<uintptr_t>(m) |
+                       reinterpret_cast<uintptr_t>(v)) & 15u) == 0;
+    const long long n4 = vec ? n >> 2 : 0;
+    for (long long i = first; i < n4; i += step) {
+        float4 pv = reinterpret_cast<float4*>(p)[i], mv = reinterpret_cast<float4*>(m)[i], vv = reinterpret_cast<float4*>(v)[i];
+        const float4 gv = reinterpret_cast<const float4*>(g)[i];
+        adam_update(a, pv.x, gv.x, mv.x, vv.x);
+        adam_update(a, pv.y, gv.y, mv.y, vv.y);
+        adam_update(a, pv.z, gv.z, mv.z, vv.z);
+        adam_update(a, pv.w, gv.w, mv.w, vv.w);
+        reinterpret_cast<float4*>(m)[i] = mv;
+        reinterpret_cast<float4*>(v)[i] = vv;
+        reinterpret_cast<float4*>(p)[i] = pv;
     }
+    for (long long i = n4 * 4 + first; i < n; i += step) adam_update(a, p[i], g[i], m[i], v[i]);
+}
+__global__ void __launch_bounds__(256) adam_kernel(float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m,
+                                                   float* __restrict__ v, long long n, const AdamScalars a) {
+    adam_range(a, p, g, m, v, n, blockIdx.x * (long long)blockDim.x + threadIdx.x, (long long)gridDim.x * blockDim.x);
+}
+
+// A list of tensors: tensor t owns the blocks [first_block[t], first_block[t + 1]).
+static constexpr int ADAM_LIST = 32;
+struct AdamList {
+    AetherAdamTensor t[ADAM_LIST];
+    int first_block[ADAM_LIST + 1];
+    int count;
+};
+__global__ void __launch_bounds__(256) adam_list_kernel(const __grid_constant__ AdamList l, const AdamScalars a) {
+    int t = 0;
+    while (t + 1 < l.count && (int)blockIdx.x >= l.first_block[t + 1]) ++t;
+    const int blocks = l.first_block[t + 1] - l.first_block[t];
+    adam_range(a, l.t[t].p, l.t[t].g, l.t[t].m, l.t[t].v, l.t[t].n, (blockIdx.x - l.first_block[t]) * (long long)blockDim.x + threadIdx.x,
+               (long long)blocks * blockDim.x);
 }
 
 // The same update with the step count read from device memory, so that a captured CUDA graph replays it with the
@@ -1004,19 +1038,18 @@ __global__ void __launch_bounds__(256) adam_dev_kernel(float* __restrict__ p, co
                                                        float* __restrict__ m, float* __restrict__ v, long long n, float lr0,
                                                        float decay, float b1, float b2, float eps, float gscale,
                                                        const long long* __restrict__ iterations) {
-    const double it = (double)*iterations;
-    const float lr = decay != 0.f ? (float)((double)lr0 * (1.0 / (1.0 + (double)decay * it))) : lr0;
-    const float inv_bc1 = (float)(1.0 / (1.0 - pow((double)b1, it + 1.0)));
-    const float inv_bc2 = (float)(1.0 / (1.0 - pow((double)b2, it + 1.0)));
-    const long long stride = (long long)gridDim.x * blockDim.x;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += stride) {
-        const float gi = g[i] * gscale;
-        const float mi = b1 * m[i] + (1.f - b1) * gi;
-        const float vi = b2 * v[i] + (1.f - b2) * gi * gi;
-        m[i] = mi;
-        v[i] = vi;
-        p[i] -= lr * (mi * inv_bc1) / (sqrtf(vi * inv_bc2) + eps);
+    // two powers in double precision, once per block (every thread computing them cost the small networks 5 us)
+    __shared__ AdamScalars a;
+    if (threadIdx.x == 0) {
+        const double it = (double)*iterations;
+        a.lr = decay != 0.f ? (float)((double)lr0 * (1.0 / (1.0 + (double)decay * it))) : lr0;
+        a.inv_bc1 = (float)(1.0 / (1.0 - pow((double)b1, it + 1.0)));
+        a.b1 = b1; a.b2 = b2; a.eps = eps; a.gscale = gscale;
+    } else if (threadIdx.x == 32) {
+        a.inv_bc2 = (float)(1.0 / (1.0 - pow((double)b2, (double)*iterations + 1.0)));
     }
+    __syncthreads();
+    adam_range(a, p, g, m, v, n, blockIdx.x * (long long)blockDim.x + threadIdx.x, (long long)gridDim.x * blockDim.x);
 }
 
 // g += l1 * sign(w) + 2 * l2 * w   (Layer_Dense.backward regulariser terms, :337-351; sign(0) = +1)
@@ -1271,7 +1304,7 @@ extern "C" int aether_adam_step_dev(float* p, const float* g, float* m, float* v
     if (!p || !g || !m || !v || !iterations_dev || n <= 0) return set_error(AE_BAD_ARG, "aether_adam_step_dev: bad argument");
     if (!(beta1 >= 0.f && beta1 < 1.f) || !(beta2 >= 0.f && beta2 < 1.f))
         return set_error(AE_BAD_ARG, "aether_adam_step_dev: betas must be in [0, 1)");
-    adam_dev_kernel<<<blocks_for(n, 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+    adam_dev_kernel<<<blocks_for(n / 4 + 1, 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
         p, g, m, v, n, lr0, decay, beta1, beta2, eps, grad_scale, reinterpret_cast<const long long*>(iterations_dev));
     count_launch();
     return check_launch("aether_adam_step_dev");
@@ -1289,10 +1322,33 @@ extern "C" int aether_adam_step(float* p, const float* g, float* m, float* v, in
                                 void* stream) {
     if (!p || !g || !m || !v || n <= 0) return set_error(AE_BAD_ARG, "aether_adam_step: bad argument");
     if (!(bias_corr1 > 0.f) || !(bias_corr2 > 0.f)) return set_error(AE_BAD_ARG, "aether_adam_step: bias corrections must be > 0");
-    adam_kernel<<<blocks_for(n, 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(p, g, m, v, n, lr, beta1, beta2, eps, 1.f / bias_corr1,
-                                                                                   1.f / bias_corr2, grad_scale);
+    const AdamScalars a = {lr, beta1, beta2, eps, 1.f / bias_corr1, 1.f / bias_corr2, grad_scale};
+    adam_kernel<<<blocks_for(n / 4 + 1, 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(p, g, m, v, n, a);
     count_launch();
     return check_launch("aether_adam_step");
+}
+
+extern "C" int aether_adam_steps(const AetherAdamTensor* tensors, int count, float lr, float beta1, float beta2, float eps,
+                                 float bias_corr1, float bias_corr2, float grad_scale, void* stream) {
+    if (!tensors || count <= 0) return set_error(AE_BAD_ARG, "aether_adam_steps: bad argument");
+    if (!(bias_corr1 > 0.f) || !(bias_corr2 > 0.f)) return set_error(AE_BAD_ARG, "aether_adam_steps: bias corrections must be > 0");
+    for (int i = 0; i < count; ++i)
+        if (!tensors[i].p || !tensors[i].g || !tensors[i].m || !tensors[i].v || tensors[i].n <= 0)
+            return set_error(AE_BAD_ARG, "aether_adam_steps: bad tensor %d", i);
+    const AdamScalars a = {lr, beta1, beta2, eps, 1.f / bias_corr1, 1.f / bias_corr2, grad_scale};
+    for (int begin = 0; begin < count; begin += ADAM_LIST) {
+        AdamList l;
+        l.count = count - begin < ADAM_LIST ? count - begin : ADAM_LIST;
+        l.first_block[0] = 0;
+        for (int i = 0; i < l.count; ++i) {
+            l.t[i] = tensors[begin + i];
+            l.first_block[i + 1] = l.first_block[i] + blocks_for(l.t[i].n / 4 + 1, 256);
+        }
+        adam_list_kernel<<<l.first_block[l.count], 256, 0, static_cast<cudaStream_t>(stream)>>>(l, a);
+        count_launch();
+        if (int rc = check_launch("aether_adam_steps")) return rc;
+    }
+    return AE_OK;
 }
 
 extern "C" int aether_regularizer_grad(const float* w, float* g, int64_t n, float l1, float l2, void* stream) {

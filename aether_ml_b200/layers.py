@@ -16,7 +16,7 @@ import numpy as np
 import torch
 
 from . import _lib
-from ._lib import AetherConvDesc, check, lib
+from ._lib import AetherConvDesc, host, lib
 
 DEFAULT_MATH_MODE = os.environ.get("AETHER_MATH_MODE", "bf16")
 
@@ -29,6 +29,10 @@ def _device():
 
 def to_device(a, dtype=torch.float32):
     """Return `a` as a contiguous CUDA tensor of `dtype` (no copy when it already is one)."""
+    if dtype is torch.float32:
+        t = host().ready(a)
+        if t is not None:
+            return t
     if isinstance(a, torch.Tensor):
         t = a
     elif hasattr(a, "__cuda_array_interface__"):
@@ -40,18 +44,6 @@ def to_device(a, dtype=torch.float32):
     if t.dtype != dtype:
         t = t.to(dtype)
     return t if t.is_contiguous() else t.contiguous()
-
-
-def _ptr(t):
-    return C.c_void_p(t.data_ptr()) if t is not None else C.c_void_p(0)
-
-
-def _stream():
-    return C.c_void_p(torch.cuda.current_stream().cuda_stream)
-
-
-def _empty(shape, dtype=torch.float32):
-    return torch.empty(shape, dtype=dtype, device=_device())
 
 
 class _Saved:
@@ -89,11 +81,13 @@ class _Workspace:
 
     def __init__(self):
         self.buf = None
+        self.size = 0
 
     def get(self, nbytes):
-        nbytes = max(int(nbytes), 256)
-        if self.buf is None or self.buf.numel() < nbytes:
+        if self.size < nbytes or self.buf is None:
+            nbytes = max(int(nbytes), 256)
             self.buf = torch.empty(nbytes, dtype=torch.uint8, device=_device())
+            self.size = nbytes
         return self.buf
 
 
@@ -108,31 +102,34 @@ class _OperandCopies:
         self.x = None
         self.w = None
 
-    @staticmethod
-    def _tag(t):
-        return (t.data_ptr(), t._version, tuple(t.shape))
-
     def record(self, ws, x, w):
         self.ws_ptr = ws.data_ptr()
-        self.x = self._tag(x)
-        self.w = self._tag(w)
+        tag = host().tag
+        self.x = tag(x)
+        self.w = tag(w)
 
     def flags(self, ws, x, w):
         """Bit 0: the copy of x is valid; bit 1: the copies of the weights are (aether_conv2d_bwd's x_shadow_valid)."""
         if self.ws_ptr is None or ws.data_ptr() != self.ws_ptr:
             return 0
-        return (1 if self._tag(x) == self.x else 0) | (2 if self._tag(w) == self.w else 0)
+        tag = host().tag
+        return (1 if tag(x) == self.x else 0) | (2 if tag(w) == self.w else 0)
+
+
+_unwritten_exist = False        # whether any array has ever been marked (the check below is on every layer's path)
 
 
 def _mark_unwritten(t):
     """Marks a device array whose fp32 contents were deliberately not written (lean mode: only its bf16 operand copy
     exists, inside the consuming layer's workspace).  A layer that would have to READ such an array raises."""
+    global _unwritten_exist
+    _unwritten_exist = True
     t._aether_unwritten = True
     return t
 
 
 def _require_written(t, who):
-    if getattr(t, "_aether_unwritten", False):
+    if _unwritten_exist and getattr(t, "_aether_unwritten", False):
         raise _lib.AetherError("%s: the input array was not materialised (Model.finalize(lean=True)) and its operand copy is "
                                "no longer current; run the producing layer again" % who)
 
@@ -140,7 +137,7 @@ def _require_written(t, who):
 def _array_tag(t):
     """Identity of a device array's contents as far as the host can tell: address, element count, version counter
     (a reshaped view of the same memory has the same tag)."""
-    return (t.data_ptr(), t.numel(), t._version)
+    return host().tag(t)[:3]
 
 
 class _HandedIn:
@@ -165,6 +162,23 @@ def _operand_layout(d):
     """AetherOperandLayout of a convolution descriptor, or None when the shape reads no bf16 operand copies."""
     lay = _lib.AetherOperandLayout()
     return lay if lib().aether_conv2d_operand_layout(C.byref(d), C.byref(lay)) else None
+
+
+class _ConvPlan:
+    """Sizes and queries of one convolution shape: the descriptor's bytes, the output shape (None when the filter does
+    not fit the padded input), the workspace, the operand layout and the blocks of epilogue statistics."""
+
+    def __init__(self, desc, Ho, Wo):
+        d = C.byref(desc)
+        self.raw = bytes(desc)
+        self.x_shape = (desc.S, desc.H, desc.W, desc.Cin)
+        self.y_shape = (desc.S, Ho, Wo, desc.Cout) if Ho >= 1 and Wo >= 1 else None
+        self.b_shape = (desc.Cout,)
+        self.layout, self.ws_bytes, self.stats_blocks = None, 0, 0
+        if self.y_shape is not None:
+            self.ws_bytes = int(lib().aether_conv2d_workspace_bytes(d))
+            self.stats_blocks = int(lib().aether_conv2d_bnstats_blocks(d))
+            self.layout = _operand_layout(desc)
 
 
 # ------------------------------------------------------------------------------------- Conv_Layer
@@ -203,7 +217,8 @@ class Conv_Layer(_Saved):
         self._stats_ws = _Workspace()
         self.emit_bn_stats = False      # set when a Batch_Norm consumes this layer's output (Model.finalize does it)
         self.bn_partials = None         # (buffer, blocks, data_ptr of the output they describe) after a training forward
-        self._desc = None
+        self._desc = None               # the plan of the last forward pass
+        self._plans = {}
         self._copies = _OperandCopies()
         self._handed = _HandedIn()
         self.first_in_model = False     # Model.finalize: this layer's dinputs are never needed
@@ -213,6 +228,7 @@ class Conv_Layer(_Saved):
         self._stats_ws = _Workspace()
         self.bn_partials = None
         self._desc = None
+        self._plans = {}
         self._copies = _OperandCopies()
         self._handed = _HandedIn()
         self.emit_bn_stats = False
@@ -228,14 +244,23 @@ class Conv_Layer(_Saved):
     def weights(self, value):
         self.filter_weights = value
 
-    def _make_desc(self, S, H, W, Cin):
+    def _plan(self, shape):
+        """What follows from an input shape and this layer's settings, worked out once per combination."""
+        key = (shape, *self.filter_size, *self.strides, self.padding, self.math_mode, self.num_filters, host().device())
+        p = self._plans.get(key)
+        if p is None:
+            if len(self._plans) >= 64:          # a caller with ever new batch sizes: start over
+                self._plans.clear()
+            p = self._plans[key] = self._make_plan(*shape)
+        return p
+
+    def _make_plan(self, S, H, W, Cin):
         fH, fW = self.filter_size
         sH, sW = self.strides
         P = (fH - 1) // 2 if self.padding == "same" else 0      # :78-81, same amount on both axes
         Ho = int((H + 2 * P - fH) / sH + 1)
         Wo = int((W + 2 * P - fW) / sW + 1)
-        d = AetherConvDesc(S, H, W, Cin, self.num_filters, fH, fW, sH, sW, P, P, _lib.MATH_MODES[self.math_mode])
-        return d, Ho, Wo
+        return _ConvPlan(AetherConvDesc(S, H, W, Cin, self.num_filters, fH, fW, sH, sW, P, P, _lib.MATH_MODES[self.math_mode]), Ho, Wo)
 
     # -- operand-copy hand-off: the kernel that produces this layer's x (going forward) or dy (going back) may write
     # the bf16 copy the tensor-core kernels read straight into this layer's workspace
@@ -243,11 +268,11 @@ class Conv_Layer(_Saved):
         """(address, row length) where the bf16 copy of an input of `shape` goes, or None."""
         if len(shape) != 4 or shape[3] != self.filter_weights.shape[2]:
             return None
-        d, Ho, Wo = self._make_desc(*shape)
-        lay = _operand_layout(d) if (Ho >= 1 and Wo >= 1) else None
+        p = self._plan(tuple(shape))
+        lay = p.layout
         if lay is None or lay.x_copy_ld == 0:          # (first layers gather x themselves: no copy of x is read)
             return None
-        ws = self._ws.get(lib().aether_conv2d_workspace_bytes(C.byref(d)))
+        ws = self._ws.get(p.ws_bytes)
         return ws.data_ptr() + lay.x_copy_offset, lay.x_copy_ld
 
     def x_copy_written(self, x):
@@ -257,14 +282,14 @@ class Conv_Layer(_Saved):
         """(address, row length, column-sum address, rows available) for the bf16 copy of the coming dvalues, or None."""
         if self._desc is None:
             return None
-        lay = _operand_layout(self._desc)
+        lay = self._desc.layout
         if lay is None:
             return None
         # A first layer's filter-gradient kernel takes the copy, but its dX runs on the CUDA cores from the fp32 array:
         # the hand-off is only for a layer whose dinputs nobody asks for (the first layer of a Model).
         if lay.x_copy_ld == 0 and not self.first_in_model:
             return None
-        ws = self._ws.get(lib().aether_conv2d_workspace_bytes(C.byref(self._desc)))
+        ws = self._ws.get(self._desc.ws_bytes)
         return ws.data_ptr() + lay.dy_copy_offset, lay.dy_copy_ld, ws.data_ptr() + lay.dy_colsum_offset, lay.dy_colsum_rows_max
 
     def dy_copy_written(self, dy, rows):
@@ -274,72 +299,71 @@ class Conv_Layer(_Saved):
         x = to_device(inputs)
         if x.ndim != 4:
             raise ValueError(f"Expected a 4D tensor, got {x.ndim} instead.")
-        S, H, W, Cin = x.shape
-        if Cin != self.filter_weights.shape[2]:
-            raise ValueError(f"input has {Cin} channels, filters expect {self.filter_weights.shape[2]}")
-        d, Ho, Wo = self._make_desc(S, H, W, Cin)
-        if Ho < 1 or Wo < 1:
+        shape = x.shape
+        if shape[3] != self.filter_weights.shape[2]:
+            raise ValueError(f"input has {shape[3]} channels, filters expect {self.filter_weights.shape[2]}")
+        p = self._plan(shape)
+        if p.y_shape is None:
             raise ValueError("filter larger than the padded input")
-        L = lib()
-        ws = self._ws.get(L.aether_conv2d_workspace_bytes(C.byref(d)))
-        y = _empty((S, Ho, Wo, self.num_filters))
-        flags = _lib.CONV_X_COPY_READY if self._handed.x_ready(ws, x) else 0
-        self._handed.x = None
+        H = host()
+        ws = self._ws.get(p.ws_bytes)
+        y = H.empty(p.y_shape)
+        flags = 0
+        if self._handed.x is not None:
+            flags = _lib.CONV_X_COPY_READY if self._handed.x_ready(ws, x) else 0
+            self._handed.x = None
         if not flags:
             _require_written(x, "Conv_Layer.forward")
         # With emit_bn_stats the kernel's epilogue also writes the per-channel partial statistics that the
         # Batch_Norm behind this layer would otherwise compute in a pass of its own over y (:467-470).
-        nblk = int(L.aether_conv2d_bnstats_blocks(C.byref(d))) if (training and self.emit_bn_stats) else 0
+        nblk = p.stats_blocks if (training and self.emit_bn_stats) else 0
         self.bn_partials = None
+        w = self.filter_weights
         if nblk > 0:
             stats = self._stats_ws.get(nblk * 3 * self.num_filters * 4)
-            check(L.aether_conv2d_fwd_ex(C.byref(d), _ptr(x), _ptr(self.filter_weights), _ptr(self.biases), _ptr(y),
-                                         _ptr(stats), stats.numel(), _ptr(ws), ws.numel(), flags, _stream()),
-                  "aether_conv2d_fwd_ex")
+            H.aether_conv2d_fwd_ex(p.raw, x, w, self.biases, y, stats, self._stats_ws.size, ws, self._ws.size, flags)
             self.bn_partials = (stats, nblk, y.data_ptr())
         else:
-            check(L.aether_conv2d_fwd_ex(C.byref(d), _ptr(x), _ptr(self.filter_weights), _ptr(self.biases), _ptr(y),
-                                         None, 0, _ptr(ws), ws.numel(), flags, _stream()), "aether_conv2d_fwd_ex")
+            H.aether_conv2d_fwd_ex(p.raw, x, w, self.biases, y, None, 0, ws, self._ws.size, flags)
         self.inputs = x
         self.output = y
-        self._desc = d
-        self._copies.record(ws, x, self.filter_weights)
-        return self.output
+        self._desc = p
+        self._copies.record(ws, x, w)
+        return y
 
     def backward(self, dvalues, need_dinputs=True):
-        if self._desc is None:
+        p = self._desc
+        if p is None:
             raise RuntimeError("Conv_Layer.backward called before forward")
         dy = to_device(dvalues)
-        d = self._desc
         x = self.inputs
-        Ho = (d.H + 2 * d.padH - d.fH) // d.sH + 1
-        Wo = (d.W + 2 * d.padW - d.fW) // d.sW + 1
-        if tuple(dy.shape) != (d.S, Ho, Wo, d.Cout):
-            raise ValueError(f"dvalues has shape {tuple(dy.shape)}, expected {(d.S, Ho, Wo, d.Cout)}")
-        L = lib()
-        ws = self._ws.get(L.aether_conv2d_workspace_bytes(C.byref(d)))
+        if dy.shape != p.y_shape:
+            raise ValueError(f"dvalues has shape {tuple(dy.shape)}, expected {p.y_shape}")
+        H = host()
+        ws = self._ws.get(p.ws_bytes)
+        w = self.filter_weights
         if getattr(self, "_grad_views", None) is not None:
             self.dweights, self.dbiases = self._grad_views
         else:
-            self.dweights = _empty(tuple(self.filter_weights.shape))
-            self.dbiases = _empty((d.Cout,))
-        dx = _empty((d.S, d.H, d.W, d.Cin)) if need_dinputs else None
-        shadow_ok = self._copies.flags(ws, x, self.filter_weights)
-        rows = self._handed.dy_rows(ws, dy)
-        self._handed.dy = None
+            self.dweights = H.empty(w.shape)
+            self.dbiases = H.empty(p.b_shape)
+        dx = H.empty(p.x_shape) if need_dinputs else None
+        shadow_ok = self._copies.flags(ws, x, w)
+        rows = 0
+        if self._handed.dy is not None:
+            rows = self._handed.dy_rows(ws, dy)
+            self._handed.dy = None
         if rows and self.first_in_model and need_dinputs:
             rows = 0                        # a first layer asked for dinputs after all: that path reads the fp32 array
         if rows:
             shadow_ok |= _lib.CONV_DY_COPY_READY
         else:
             _require_written(dy, "Conv_Layer.backward")
-        if not (shadow_ok & _lib.CONV_X_COPY_READY) and self.dweights is not None:
+        if not (shadow_ok & _lib.CONV_X_COPY_READY):
             _require_written(x, "Conv_Layer.backward")
-        check(L.aether_conv2d_bwd_ex(C.byref(d), _ptr(x), _ptr(dy), _ptr(self.filter_weights), _ptr(dx),
-                                     _ptr(self.dweights), _ptr(self.dbiases), _ptr(ws), ws.numel(), shadow_ok, rows,
-                                     _stream()), "aether_conv2d_bwd_ex")
+        H.aether_conv2d_bwd_ex(p.raw, x, dy, w, dx, self.dweights, self.dbiases, ws, self._ws.size, shadow_ok, rows)
         self.dinputs = dx
-        return self.dinputs
+        return dx
 
     def get_parameters(self):
         return self.filter_weights, self.biases
@@ -395,10 +419,10 @@ class Pooling(_Saved):
         Ho = (H - fH) // sH + 1
         Wo = (W - fW) // sW + 1
         kind = self._kind()
-        y = _empty((S, Ho, Wo, Cc))
-        self._argmax = _empty((S, Ho, Wo, Cc), torch.uint8) if kind == _lib.POOL_MAX else None
-        check(lib().aether_pool_fwd(_ptr(x), _ptr(y), _ptr(self._argmax), S, H, W, Cc, fH, fW, sH, sW, kind,
-                                    _stream()), "aether_pool_fwd")
+        h = host()
+        y = h.empty((S, Ho, Wo, Cc))
+        self._argmax = h.empty_u8((S, Ho, Wo, Cc)) if kind == _lib.POOL_MAX else None
+        h.aether_pool_fwd(x, y, self._argmax, S, H, W, Cc, fH, fW, sH, sW, kind)
         self.inputs = x
         self.output = y
         return self.output
@@ -417,9 +441,8 @@ class Pooling(_Saved):
         S, H, W, Cc = self.inputs.shape
         fH, fW = self.filter_size
         sH, sW = self.strides
-        dx = _empty((S, H, W, Cc))
-        check(lib().aether_pool_bwd(_ptr(dy), _ptr(self._argmax), _ptr(dx), S, H, W, Cc, fH, fW, sH, sW,
-                                    self._kind(), _stream()), "aether_pool_bwd")
+        dx = host().empty_like(self.inputs)
+        host().aether_pool_bwd(dy, self._argmax, dx, S, H, W, Cc, fH, fW, sH, sW, self._kind())
         self.dinputs = dx
         return self.dinputs
 
@@ -437,9 +460,9 @@ class ReLU(_Saved):
         if self.fused_into_prev:
             self.inputs = self.output = x
             return self.output
-        y = torch.empty_like(x)
-        check(lib().aether_leaky_relu_fwd(_ptr(x), _ptr(y), x.numel(), float(self._alpha), _stream()),
-              "aether_leaky_relu_fwd")
+        h = host()
+        y = h.empty_like(x)
+        h.aether_leaky_relu_fwd(x, y, x.numel(), self._alpha)
         self.inputs = x
         self.output = y
         return self.output
@@ -449,9 +472,9 @@ class ReLU(_Saved):
         if self.fused_into_prev:
             self.dinputs = dy
             return self.dinputs
-        dx = torch.empty_like(dy)
-        check(lib().aether_leaky_relu_bwd(_ptr(self.inputs), _ptr(dy), _ptr(dx), dy.numel(), float(self._alpha),
-                                          _stream()), "aether_leaky_relu_bwd")
+        h = host()
+        dx = h.empty_like(dy)
+        h.aether_leaky_relu_bwd(self.inputs, dy, dx, dy.numel(), self._alpha)
         self.dinputs = dx
         return self.dinputs
 
@@ -493,9 +516,8 @@ class Layer_Dropout_Spatial(_Saved):
     def draw_mask(self, Cc):
         """Draws this step's channel mask (Bernoulli(keep)/keep per channel) into ``channel_mask``."""
         if self.fixed_mask is None and self.step_dev is not None:
-            self.channel_mask = _empty((1, 1, 1, Cc))
-            check(lib().aether_channel_mask_dev(_ptr(self.channel_mask), Cc, float(self.keep_prob), self.seed,
-                                                _ptr(self.step_dev), _stream()), "aether_channel_mask_dev")
+            self.channel_mask = host().empty((1, 1, 1, Cc))
+            host().aether_channel_mask_dev(self.channel_mask, Cc, self.keep_prob, self.seed, self.step_dev)
         else:
             if self.fixed_mask is not None:
                 mask = np.asarray(self.fixed_mask, dtype=np.float32).reshape(1, 1, 1, Cc)
@@ -515,9 +537,9 @@ class Layer_Dropout_Spatial(_Saved):
             return self.output
         Cc = x.shape[-1]
         self.draw_mask(Cc)
-        y = torch.empty_like(x)
-        check(lib().aether_channel_scale(_ptr(x), _ptr(self.channel_mask), _ptr(y), x.numel(), Cc, _stream()),
-              "aether_channel_scale")
+        h = host()
+        y = h.empty_like(x)
+        h.aether_channel_scale(x, self.channel_mask, y, x.numel(), Cc)
         self.output = y
         return self.output
 
@@ -526,9 +548,9 @@ class Layer_Dropout_Spatial(_Saved):
         if self.fused_into_prev:
             self.dinputs = dy
             return self.dinputs
-        dx = torch.empty_like(dy)
-        check(lib().aether_channel_scale(_ptr(dy), _ptr(self.channel_mask), _ptr(dx), dy.numel(), dy.shape[-1],
-                                         _stream()), "aether_channel_scale")
+        h = host()
+        dx = h.empty_like(dy)
+        h.aether_channel_scale(dy, self.channel_mask, dx, dy.numel(), dy.shape[-1])
         self.dinputs = dx
         return self.dinputs
 
@@ -558,24 +580,23 @@ class Layer_Dropout(_Saved):
         if not training:
             self.output = x.clone()
             return self.output
-        y = torch.empty_like(x)
-        self.binary_mask = torch.empty_like(x)
+        h = host()
+        y = h.empty_like(x)
+        self.binary_mask = h.empty_like(x)
         if self.step_dev is not None:   # the call counter lives on the device (CUDA-graph train step)
-            check(lib().aether_dropout_fwd_dev(_ptr(x), _ptr(y), _ptr(self.binary_mask), x.numel(), float(self.rate),
-                                               self.seed, self.rank_offset << 32, _ptr(self.step_dev), _stream()),
-                  "aether_dropout_fwd_dev")
+            h.aether_dropout_fwd_dev(x, y, self.binary_mask, x.numel(), self.rate, self.seed, self.rank_offset << 32, self.step_dev)
         else:
             offset = (self._calls << 40) + (self.rank_offset << 32)
             self._calls += 1
-            check(lib().aether_dropout_fwd(_ptr(x), _ptr(y), _ptr(self.binary_mask), x.numel(), float(self.rate),
-                                           self.seed, offset, _stream()), "aether_dropout_fwd")
+            h.aether_dropout_fwd(x, y, self.binary_mask, x.numel(), self.rate, self.seed, offset)
         self.output = y
         return self.output
 
     def backward(self, dvalues):
         dy = to_device(dvalues)
-        dx = torch.empty_like(dy)
-        check(lib().aether_mul(_ptr(dy), _ptr(self.binary_mask), _ptr(dx), dy.numel(), _stream()), "aether_mul")
+        h = host()
+        dx = h.empty_like(dy)
+        h.aether_mul(dy, self.binary_mask, dx, dy.numel())
         self.dinputs = dx
         return self.dinputs
 
@@ -600,7 +621,7 @@ class Batch_Norm(_Saved):
         self.bias_regularizer_l1 = 0
         self.bias_regularizer_l2 = 0
         self._ws = _Workspace()
-        self._keep = None
+        self._ws_for = self._views = None
         self.stats_from = None          # a Conv_Layer whose forward leaves `bn_partials` for this layer's input
         self.fused_alpha = None         # slope of the (Leaky_)ReLU applied inside this layer's kernels (None: not fused)
         self.fused_dropout = None       # a Layer_Dropout_Spatial behind that activation whose mask is applied here too
@@ -614,7 +635,7 @@ class Batch_Norm(_Saved):
 
     def _restore_transient(self):
         self._ws = _Workspace()
-        self._keep = None
+        self._ws_for = self._views = None
         self.stats_from = None
         self.fused_alpha = None
         self.fused_dropout = None
@@ -663,12 +684,12 @@ class Batch_Norm(_Saved):
             self._create(Cc)
         rows = x.numel() // Cc
         keep = (1,) * (x.ndim - 1) + (Cc,)
-        L = lib()
-        ws = self._ws.get(L.aether_bn_workspace_bytes(rows, Cc))
+        h = host()
+        ws = self._workspace(rows, Cc)
         part = None
         if training:
-            self._bm = _empty((Cc,))
-            self._bv = _empty((Cc,))
+            self._bm = h.empty(keep)
+            self._bv = h.empty(keep)
             part = getattr(self.stats_from, "bn_partials", None) if self.stats_from is not None else None
             if part is not None and part[2] != x.data_ptr():
                 part = None
@@ -681,22 +702,19 @@ class Batch_Norm(_Saved):
             S, H, W = x.shape[0], x.shape[1], x.shape[2]
             if H % fH == 0 and W % fW == 0:
                 mask = self.fused_dropout.draw_mask(Cc) if (training and self.fused_dropout is not None) else None
-                pooled = _empty((S, H // fH, W // fW, Cc))
-                self._pool_arg = _empty((S, H // fH, W // fW, Cc), torch.uint8)
+                pshape = (S, H // fH, W // fW, Cc)
+                pooled = h.empty(pshape)
+                self._pool_arg = h.empty_u8(pshape)
                 # the layer behind the pooling reads a bf16 copy of the pooled tensor: written by this same pass
-                target = self.copy_consumer.x_copy_target(tuple(pooled.shape)) if self.copy_consumer is not None else None
+                target = self.copy_consumer.x_copy_target(pshape) if self.copy_consumer is not None else None
                 # x at every window's selected cell, for the backward statistics pass (training only)
-                self._xsel = _empty(tuple(pooled.shape)) if training else None
-                check(L.aether_bn_act_pool_fwd_copy(_ptr(x), _ptr(part[0]) if part else None, part[1] if part else 0,
-                                                    _ptr(self.gamma), _ptr(self.beta), _ptr(self._rm), _ptr(self._rv),
-                                                    _ptr(self._bm) if training else None, _ptr(self._bv) if training else None,
-                                                    None if (self.lean and target) else _ptr(pooled), _ptr(self._pool_arg),
-                                                    S, H, W, Cc, fH, fW,
-                                                    float(self.epsilon), float(self.momentum), float(self.fused_alpha),
-                                                    _ptr(mask), 1 if training else 0,
-                                                    C.c_void_p(target[0]) if target else None, target[1] if target else 0,
-                                                    _ptr(self._xsel), _ptr(ws), ws.numel(), _stream()),
-                      "aether_bn_act_pool_fwd_copy")
+                self._xsel = h.empty(pshape) if training else None
+                h.aether_bn_act_pool_fwd_copy(x, part[0] if part else None, part[1] if part else 0, self.gamma, self.beta,
+                                              self._rm, self._rv, self._bm if training else None, self._bv if training else None,
+                                              None if (self.lean and target) else pooled, self._pool_arg, S, H, W, Cc, fH, fW,
+                                              self.epsilon, self.momentum, self.fused_alpha, mask, 1 if training else 0,
+                                              target[0] if target else None, target[1] if target else 0, self._xsel, ws,
+                                              self._ws.size)
                 if target:
                     if self.lean:
                         _mark_unwritten(pooled)
@@ -704,63 +722,63 @@ class Batch_Norm(_Saved):
                 self._fused_mask = mask
                 self.pooled_now = True
                 if training:
-                    self.batch_mean = self._bm.view(keep)
-                    self.batch_var = self._bv.view(keep)
-                    self.running_mean = self._rm.view(keep)
-                    self.running_var = self._rv.view(keep)
+                    self._expose_statistics(keep)
                 self.inputs = x
                 self.output = pooled
                 return self.output
-        y = torch.empty_like(x)
+        y = h.empty_like(x)
         if training:
             if self.fused_alpha is not None:
                 # y = act(bn(x)) [* spatial-dropout mask] in the same passes; the layers behind only hand y through
                 mask = self.fused_dropout.draw_mask(Cc) if self.fused_dropout is not None else None
-                check(L.aether_bn_act_fwd_train(_ptr(x), _ptr(part[0]) if part else None, part[1] if part else 0,
-                                                _ptr(self.gamma), _ptr(self.beta), _ptr(self._rm), _ptr(self._rv),
-                                                _ptr(self._bm), _ptr(self._bv), _ptr(y), rows, Cc, float(self.epsilon),
-                                                float(self.momentum), float(self.fused_alpha), _ptr(mask), _ptr(ws),
-                                                ws.numel(), _stream()), "aether_bn_act_fwd_train")
+                h.aether_bn_act_fwd_train(x, part[0] if part else None, part[1] if part else 0, self.gamma, self.beta, self._rm,
+                                          self._rv, self._bm, self._bv, y, rows, Cc, self.epsilon, self.momentum,
+                                          self.fused_alpha, mask, ws, self._ws.size)
                 self._fused_mask = mask
             elif part is not None:
                 # the convolution that produced x already reduced it per channel: merge its partials, read x once
-                check(L.aether_bn_fwd_train_partials(_ptr(x), _ptr(part[0]), part[1], _ptr(self.gamma), _ptr(self.beta),
-                                                     _ptr(self._rm), _ptr(self._rv), _ptr(self._bm), _ptr(self._bv),
-                                                     _ptr(y), rows, Cc, float(self.epsilon), float(self.momentum),
-                                                     _ptr(ws), ws.numel(), _stream()), "aether_bn_fwd_train_partials")
+                h.aether_bn_fwd_train_partials(x, part[0], part[1], self.gamma, self.beta, self._rm, self._rv, self._bm, self._bv,
+                                               y, rows, Cc, self.epsilon, self.momentum, ws, self._ws.size)
             else:
-                check(L.aether_bn_fwd_train(_ptr(x), _ptr(self.gamma), _ptr(self.beta), _ptr(self._rm), _ptr(self._rv),
-                                            _ptr(self._bm), _ptr(self._bv), _ptr(y), rows, Cc, float(self.epsilon),
-                                            float(self.momentum), _ptr(ws), ws.numel(), _stream()), "aether_bn_fwd_train")
-            self.batch_mean = self._bm.view(keep)
-            self.batch_var = self._bv.view(keep)
-            self.running_mean = self._rm.view(keep)       # the reference's stats pick up keep-dims here (:475-476)
-            self.running_var = self._rv.view(keep)
+                h.aether_bn_fwd_train(x, self.gamma, self.beta, self._rm, self._rv, self._bm, self._bv, y, rows, Cc,
+                                      self.epsilon, self.momentum, ws, self._ws.size)
+            self._expose_statistics(keep)
         elif self.fused_alpha is not None:
-            check(L.aether_bn_act_fwd_eval(_ptr(x), _ptr(self.gamma), _ptr(self.beta), _ptr(self._rm), _ptr(self._rv),
-                                           _ptr(y), rows, Cc, float(self.epsilon), float(self.fused_alpha), _ptr(ws),
-                                           ws.numel(), _stream()), "aether_bn_act_fwd_eval")
+            h.aether_bn_act_fwd_eval(x, self.gamma, self.beta, self._rm, self._rv, y, rows, Cc, self.epsilon, self.fused_alpha, ws,
+                                     self._ws.size)
         else:
-            check(L.aether_bn_fwd_eval(_ptr(x), _ptr(self.gamma), _ptr(self.beta), _ptr(self._rm), _ptr(self._rv),
-                                       _ptr(y), rows, Cc, float(self.epsilon), _ptr(ws), ws.numel(), _stream()),
-                  "aether_bn_fwd_eval")
+            h.aether_bn_fwd_eval(x, self.gamma, self.beta, self._rm, self._rv, y, rows, Cc, self.epsilon, ws, self._ws.size)
         self.inputs = x
         self.output = y
         return self.output
+
+    def _workspace(self, rows, Cc):
+        if self._ws_for != (rows, Cc):
+            self._ws_bytes = int(lib().aether_bn_workspace_bytes(rows, Cc))
+            self._ws_for = (rows, Cc)
+        return self._ws.get(self._ws_bytes)
+
+    def _expose_statistics(self, keep):
+        self.batch_mean = self._bm
+        self.batch_var = self._bv
+        if self._views is None or self._views[0] is not self._rm or self._views[1] is not self._rv or self._views[2] != keep:
+            self._views = (self._rm, self._rv, keep, self._rm.view(keep), self._rv.view(keep))
+        self.running_mean = self._views[3]       # the reference's stats pick up keep-dims here (:475-476)
+        self.running_var = self._views[4]
 
     def backward(self, dvalues):
         dy = to_device(dvalues)
         x = self.inputs
         Cc = x.shape[-1]
         rows = x.numel() // Cc
-        L = lib()
-        ws = self._ws.get(L.aether_bn_workspace_bytes(rows, Cc))
-        dx = torch.empty_like(x)
+        h = host()
+        ws = self._workspace(rows, Cc)
+        dx = h.empty_like(x)
         if getattr(self, "_grad_views", None) is not None:
             self.dweights, self.dbiases = self._grad_views
         else:
-            self.dweights = _empty((Cc,))
-            self.dbiases = _empty((Cc,))
+            self.dweights = h.empty((Cc,))
+            self.dbiases = h.empty((Cc,))
         if self.pooled_now:                  # dvalues is the gradient w.r.t. the POOLED output of the fused block tail
             S, H, W = x.shape[0], x.shape[1], x.shape[2]
             fH, fW = self.fused_pool.filter_size
@@ -769,29 +787,22 @@ class Batch_Norm(_Saved):
             conv = self.copy_dy_consumer
             target = conv.dy_copy_target() if (conv is not None and conv.output is x and 256 % max(Cc // 4, 1) == 0
                                                and Cc // 4 <= 256) else None
-            rows = C.c_int(0)
-            check(L.aether_bn_act_pool_bwd_copy(_ptr(x), _ptr(dy), _ptr(self._pool_arg), _ptr(self.gamma), _ptr(self.beta),
-                                                _ptr(self._bm), _ptr(self._bv), None if (self.lean and target) else _ptr(dx),
-                                                _ptr(self.dweights),
-                                                _ptr(self.dbiases), S, H, W, Cc, fH, fW, float(self.epsilon),
-                                                float(self.fused_alpha), _ptr(getattr(self, "_fused_mask", None)),
-                                                C.c_void_p(target[0]) if target else None, target[1] if target else 0,
-                                                C.c_void_p(target[2]) if target else None, target[3] if target else 0,
-                                                C.byref(rows), _ptr(getattr(self, "_xsel", None)), _ptr(ws), ws.numel(),
-                                                _stream()), "aether_bn_act_pool_bwd_copy")
+            sums = h.aether_bn_act_pool_bwd_copy(x, dy, self._pool_arg, self.gamma, self.beta, self._bm, self._bv,
+                                                 None if (self.lean and target) else dx, self.dweights, self.dbiases, S, H, W, Cc,
+                                                 fH, fW, self.epsilon, self.fused_alpha, getattr(self, "_fused_mask", None),
+                                                 target[0] if target else None, target[1] if target else 0,
+                                                 target[2] if target else None, target[3] if target else 0,
+                                                 getattr(self, "_xsel", None), ws)
             if target:
                 if self.lean:
                     _mark_unwritten(dx)
-                conv.dy_copy_written(dx, rows.value)
+                conv.dy_copy_written(dx, sums)
         elif self.fused_alpha is not None:   # dvalues is the gradient w.r.t. the ACTIVATED output
-            check(L.aether_bn_act_bwd(_ptr(x), _ptr(self.beta), _ptr(dy), _ptr(self.gamma), _ptr(self._bm),
-                                      _ptr(self._bv), _ptr(dx), _ptr(self.dweights), _ptr(self.dbiases), rows, Cc,
-                                      float(self.epsilon), float(self.fused_alpha), _ptr(getattr(self, "_fused_mask", None)),
-                                      _ptr(ws), ws.numel(), _stream()), "aether_bn_act_bwd")
+            h.aether_bn_act_bwd(x, self.beta, dy, self.gamma, self._bm, self._bv, dx, self.dweights, self.dbiases, rows, Cc,
+                                self.epsilon, self.fused_alpha, getattr(self, "_fused_mask", None), ws, self._ws.size)
         else:
-            check(L.aether_bn_bwd(_ptr(x), _ptr(dy), _ptr(self.gamma), _ptr(self._bm), _ptr(self._bv), _ptr(dx),
-                                  _ptr(self.dweights), _ptr(self.dbiases), rows, Cc, float(self.epsilon), _ptr(ws),
-                                  ws.numel(), _stream()), "aether_bn_bwd")
+            h.aether_bn_bwd(x, dy, self.gamma, self._bm, self._bv, dx, self.dweights, self.dbiases, rows, Cc, self.epsilon, ws,
+                            self._ws.size)
         self.dinputs = dx
         return self.dinputs
 
@@ -842,11 +853,13 @@ class Layer_Dense(_Saved):
         self.bias_regularizer_l2 = bias_regularizer_l2
         self.math_mode = math_mode or DEFAULT_MATH_MODE
         self._ws = _Workspace()
+        self._plans = {}
         self._copies = _OperandCopies()
         self._handed = _HandedIn()
 
     def _restore_transient(self):
         self._ws = _Workspace()
+        self._plans = {}
         self._copies = _OperandCopies()
         self._handed = _HandedIn()
 
@@ -859,66 +872,72 @@ class Layer_Dense(_Saved):
             total *= int(v)
         if len(shape) < 2 or total != int(shape[0]) * n_in:
             return None
-        d = self._desc(int(shape[0]))
-        lay = _operand_layout(d)
+        p = self._plan(int(shape[0]))
+        lay = p.layout
         # A row of the copy is one SAMPLE here, but the producer writes one PIXEL (shape[-1] channels) per row: the two
         # are the same bytes only when the sample's row is not padded (n_inputs a multiple of 64).
         if lay is None or lay.x_copy_ld != n_in:
             return None
-        ws = self._ws.get(lib().aether_conv2d_workspace_bytes(C.byref(d)))
+        ws = self._ws.get(p.ws_bytes)
         return ws.data_ptr() + lay.x_copy_offset, int(shape[-1])
 
     def x_copy_written(self, x):
         self._handed.x = (self._ws.buf.data_ptr(), _array_tag(x))
 
-    def _desc(self, S):
+    def _plan(self, S):
         n_in, n_out = self.weights.shape
-        return AetherConvDesc(S, 1, 1, n_in, n_out, 1, 1, 1, 1, 0, 0, _lib.MATH_MODES[self.math_mode])
+        key = (S, n_in, n_out, self.math_mode, host().device())
+        p = self._plans.get(key)
+        if p is None:
+            if len(self._plans) >= 64:
+                self._plans.clear()
+            p = self._plans[key] = _ConvPlan(AetherConvDesc(S, 1, 1, n_in, n_out, 1, 1, 1, 1, 0, 0, _lib.MATH_MODES[self.math_mode]), 1, 1)
+        return p
 
     def forward(self, inputs, training):
         x = to_device(inputs)
-        if x.ndim != 2 or x.shape[1] != self.weights.shape[0]:
-            raise ValueError(f"Layer_Dense expects (samples, {self.weights.shape[0]}), got {tuple(x.shape)}")
-        d = self._desc(x.shape[0])
-        L = lib()
-        ws = self._ws.get(L.aether_conv2d_workspace_bytes(C.byref(d)))
-        y = _empty((x.shape[0], self.weights.shape[1]))
-        flags = _lib.CONV_X_COPY_READY if self._handed.x_ready(ws, x) else 0
-        self._handed.x = None
+        w = self.weights
+        if x.ndim != 2 or x.shape[1] != w.shape[0]:
+            raise ValueError(f"Layer_Dense expects (samples, {w.shape[0]}), got {tuple(x.shape)}")
+        S = x.shape[0]
+        p = self._plan(S)
+        H = host()
+        ws = self._ws.get(p.ws_bytes)
+        y = H.empty((S, w.shape[1]))
+        flags = 0
+        if self._handed.x is not None:
+            flags = _lib.CONV_X_COPY_READY if self._handed.x_ready(ws, x) else 0
+            self._handed.x = None
         if not flags:
             _require_written(x, "Layer_Dense.forward")
-        check(L.aether_conv2d_fwd_ex(C.byref(d), _ptr(x), _ptr(self.weights), _ptr(self.biases), _ptr(y), None, 0, _ptr(ws),
-                                     ws.numel(), flags, _stream()), "aether_conv2d_fwd_ex")
+        H.aether_conv2d_fwd_ex(p.raw, x, w, self.biases, y, None, 0, ws, self._ws.size, flags)
         self.inputs = x
         self.output = y
-        self._copies.record(ws, x, self.weights)
-        return self.output
+        self._copies.record(ws, x, w)
+        return y
 
     def backward(self, dvalues):
         dy = to_device(dvalues)
         x = self.inputs
-        d = self._desc(x.shape[0])
-        L = lib()
-        ws = self._ws.get(L.aether_conv2d_workspace_bytes(C.byref(d)))
+        w = self.weights
+        p = self._plan(x.shape[0])
+        H = host()
+        ws = self._ws.get(p.ws_bytes)
         if getattr(self, "_grad_views", None) is not None:
             self.dweights, self.dbiases = self._grad_views
         else:
-            self.dweights = torch.empty_like(self.weights)
-            self.dbiases = torch.empty_like(self.biases)
-        dx = torch.empty_like(x)
-        copy_flags = self._copies.flags(ws, x, self.weights)
+            self.dweights = H.empty_like(w)
+            self.dbiases = H.empty_like(self.biases)
+        dx = H.empty_like(x)
+        copy_flags = self._copies.flags(ws, x, w)
         if not (copy_flags & _lib.CONV_X_COPY_READY):
             _require_written(x, "Layer_Dense.backward")
-        check(L.aether_conv2d_bwd(C.byref(d), _ptr(x), _ptr(dy), _ptr(self.weights), _ptr(dx), _ptr(self.dweights),
-                                  _ptr(self.dbiases), _ptr(ws), ws.numel(), copy_flags, _stream()), "aether_conv2d_bwd")
+        H.aether_conv2d_bwd_ex(p.raw, x, dy, w, dx, self.dweights, self.dbiases, ws, self._ws.size, copy_flags, 0)
         if self.weight_regularizer_l1 > 0 or self.weight_regularizer_l2 > 0:
-            check(L.aether_regularizer_grad(_ptr(self.weights), _ptr(self.dweights), self.weights.numel(),
-                                            float(self.weight_regularizer_l1), float(self.weight_regularizer_l2),
-                                            _stream()), "aether_regularizer_grad")
+            H.aether_regularizer_grad(w, self.dweights, w.numel(), self.weight_regularizer_l1, self.weight_regularizer_l2)
         if self.bias_regularizer_l1 > 0 or self.bias_regularizer_l2 > 0:
-            check(L.aether_regularizer_grad(_ptr(self.biases), _ptr(self.dbiases), self.biases.numel(),
-                                            float(self.bias_regularizer_l1), float(self.bias_regularizer_l2),
-                                            _stream()), "aether_regularizer_grad")
+            H.aether_regularizer_grad(self.biases, self.dbiases, self.biases.numel(), self.bias_regularizer_l1,
+                                      self.bias_regularizer_l2)
         self.dinputs = dx
         return self.dinputs
 
@@ -942,20 +961,17 @@ def _labels_i32(y_true):
 
 def _softmax_cce(z, labels, want_prob, want_loss, want_dz, want_correct, smooth_fwd, smooth_bwd, input_is_prob=False):
     rows, classes = z.shape
-    prob = _empty((rows, classes)) if want_prob else None
-    loss = _empty((rows,)) if want_loss else None
-    dz = _empty((rows, classes)) if want_dz else None
-    correct = _empty((rows,), torch.int32) if want_correct else None
+    h = host()
+    prob = h.empty((rows, classes)) if want_prob else None
+    loss = h.empty((rows,)) if want_loss else None
+    dz = h.empty((rows, classes)) if want_dz else None
+    correct = h.empty_i32((rows,)) if want_correct else None
     if labels is not None and labels.ndim == 2:
         if tuple(labels.shape) != (rows, classes):
             raise ValueError(f"targets have shape {tuple(labels.shape)}, expected {(rows, classes)}")
-        check(lib().aether_softmax_cce_targets(_ptr(z), _ptr(labels), _ptr(prob), _ptr(loss), _ptr(dz), _ptr(correct), rows,
-                                               classes, float(smooth_fwd), float(smooth_bwd), 1 if input_is_prob else 0,
-                                               _stream()), "aether_softmax_cce_targets")
+        h.aether_softmax_cce_targets(z, labels, prob, loss, dz, correct, rows, classes, smooth_fwd, smooth_bwd, 1 if input_is_prob else 0)
     else:
-        check(lib().aether_softmax_cce(_ptr(z), _ptr(labels), _ptr(prob), _ptr(loss), _ptr(dz), _ptr(correct), rows,
-                                       classes, float(smooth_fwd), float(smooth_bwd), 1 if input_is_prob else 0,
-                                       _stream()), "aether_softmax_cce")
+        h.aether_softmax_cce(z, labels, prob, loss, dz, correct, rows, classes, smooth_fwd, smooth_bwd, 1 if input_is_prob else 0)
     return prob, loss, dz, correct
 
 
@@ -974,9 +990,8 @@ class SoftMax(_Saved):
         dv = to_device(dvalues)
         if tuple(dv.shape) != tuple(self.output.shape):
             raise ValueError(f"dvalues has shape {tuple(dv.shape)}, expected {tuple(self.output.shape)}")
-        dx = torch.empty_like(dv)
-        check(lib().aether_softmax_bwd(_ptr(self.output), _ptr(dv), _ptr(dx), dv.shape[0], dv.shape[1], _stream()),
-              "aether_softmax_bwd")
+        dx = host().empty_like(dv)
+        host().aether_softmax_bwd(self.output, dv, dx, dv.shape[0], dv.shape[1])
         self.dinputs = dx
         return self.dinputs
 
@@ -1011,15 +1026,13 @@ class Loss(_Saved):
 
     def regularization_loss(self):
         out = None
-        L = lib()
         for layer in self.trainable_layers:
             for arr, l1, l2 in ((layer.weights, layer.weight_regularizer_l1, layer.weight_regularizer_l2),
                                 (layer.biases, layer.bias_regularizer_l1, layer.bias_regularizer_l2)):
                 if l1 > 0 or l2 > 0:
                     if out is None:
                         out = torch.zeros(1, dtype=torch.float32, device=_device())
-                    check(L.aether_regularizer_loss(_ptr(arr), arr.numel(), float(l1), float(l2), _ptr(out),
-                                                    _stream()), "aether_regularizer_loss")
+                    host().aether_regularizer_loss(arr, arr.numel(), l1, l2, out)
         return out[0] if out is not None else 0
 
 
@@ -1093,25 +1106,40 @@ class Optimizer_Adam(_Saved):
 
     def _step(self, p, g, m, v):
         if self.step_dev is not None:   # iterations, decay and bias corrections evaluated on the device
-            check(lib().aether_adam_step_dev(_ptr(p), _ptr(g), _ptr(m), _ptr(v), p.numel(), float(self.learning_rate),
-                                             float(self.decay), float(self.beta_1), float(self.beta_2),
-                                             float(self.epsilon), float(self.grad_scale), _ptr(self.step_dev),
-                                             _stream()), "aether_adam_step_dev")
+            host().aether_adam_step_dev(p, g, m, v, p.numel(), self.learning_rate, self.decay, self.beta_1, self.beta_2,
+                                        self.epsilon, self.grad_scale, self.step_dev)
             return
         t = self.iterations + 1
-        check(lib().aether_adam_step(_ptr(p), _ptr(g), _ptr(m), _ptr(v), p.numel(), float(self.current_learning_rate),
-                                     float(self.beta_1), float(self.beta_2), float(self.epsilon),
-                                     float(1 - self.beta_1 ** t), float(1 - self.beta_2 ** t), float(self.grad_scale),
-                                     _stream()), "aether_adam_step")
+        host().aether_adam_step(p, g, m, v, p.numel(), self.current_learning_rate, self.beta_1, self.beta_2, self.epsilon,
+                                1 - self.beta_1 ** t, 1 - self.beta_2 ** t, self.grad_scale)
 
-    def update_parameters(self, layer):
+    @staticmethod
+    def _ensure_state(layer):
         if not hasattr(layer, "weight_cache"):
             layer.weight_momentums = torch.zeros_like(layer.weights)
             layer.weight_cache = torch.zeros_like(layer.weights)
             layer.bias_momentums = torch.zeros_like(layer.biases)
             layer.bias_cache = torch.zeros_like(layer.biases)
+
+    def update_parameters(self, layer):
+        self._ensure_state(layer)
         self._step(layer.weights, layer.dweights, layer.weight_momentums, layer.weight_cache)
         self._step(layer.biases, layer.dbiases, layer.bias_momentums, layer.bias_cache)
+
+    def update_layers(self, layers):
+        """``update_parameters`` of every layer in one launch (a layer by itself is two launches of a few microseconds)."""
+        if self.step_dev is not None:
+            for layer in layers:
+                self.update_parameters(layer)
+            return
+        arrays = []
+        for layer in layers:
+            self._ensure_state(layer)
+            arrays += (layer.weights, layer.dweights, layer.weight_momentums, layer.weight_cache,
+                       layer.biases, layer.dbiases, layer.bias_momentums, layer.bias_cache)
+        t = self.iterations + 1
+        host().aether_adam_steps(arrays, self.current_learning_rate, self.beta_1, self.beta_2, self.epsilon,
+                                 1 - self.beta_1 ** t, 1 - self.beta_2 ** t, self.grad_scale)
 
     def update_flat(self, params, grads, m, v):
         """One launch over a flat parameter buffer (used by the data-parallel trainer)."""

@@ -17,7 +17,7 @@ import numpy as np
 import torch
 
 from .layers import (Activation_Softmax_Loss_CategoricalCrossEntropy, Batch_Norm, Conv_Layer, Flatten, Layer_Dropout_Spatial,
-                     Loss_CategoricalCrossEntropy, Pooling, ReLU, SoftMax, to_device, _labels_i32, _softmax_cce, _Saved)
+                     Loss_CategoricalCrossEntropy, Optimizer_Adam, Pooling, ReLU, SoftMax, to_device, _labels_i32, _softmax_cce, _Saved)
 
 
 class Layer_Input:
@@ -327,6 +327,8 @@ class Model:
             self._updated_early = set()
         elif self.flat_params is not None and hasattr(opt, "update_flat"):
             opt.update_flat(self.flat_params, self.flat_grads, self.flat_m, self.flat_v)
+        elif type(opt).update_parameters is Optimizer_Adam.update_parameters:
+            opt.update_layers(self.trainable_layers)
         else:
             for layer in self.trainable_layers:
                 opt.update_parameters(layer)

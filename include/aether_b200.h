@@ -273,6 +273,17 @@ int aether_mul(const float* a, const float* b, float* y, int64_t n, void* stream
  *      data-parallel average). */
 int aether_adam_step(float* p, const float* g, float* m, float* v, int64_t n, float lr, float beta1, float beta2,
                      float eps, float bias_corr1, float bias_corr2, float grad_scale, void* stream);
+/* The same update of several tensors in one launch (Model's loop over the trainable layers, CNN_model_cupy.py:124-125):
+ * `tensors` is a HOST array of `count` entries. */
+typedef struct AetherAdamTensor {
+    float* p;
+    const float* g;
+    float* m;
+    float* v;
+    int64_t n;
+} AetherAdamTensor;
+int aether_adam_steps(const AetherAdamTensor* tensors, int count, float lr, float beta1, float beta2, float eps,
+                      float bias_corr1, float bias_corr2, float grad_scale, void* stream);
 /* ---- Variants for a train step captured in a CUDA graph.  A replayed graph cannot change kernel arguments, so
  *      whatever the reference changes on the host from step to step is read from device memory instead: one int64
  *      counter that the caller increments once per step (a device-side add inside the graph).
