@@ -42,6 +42,7 @@ int* device_status_word() {
 // One thread waits on a barrier that nothing ever completes, with the same bounded wait the convolution kernels
 // use, gives up after `limit` cycles, records its code and returns: the give-up path of every kernel, run alone.
 __global__ void selftest_bounded_wait_kernel(int* status, long long limit) {
+    pdl_wait();
     __shared__ __align__(8) unsigned long long bar;
     if (threadIdx.x == 0) {
         const uint32_t b = smem_u32(&bar);
@@ -128,7 +129,7 @@ extern "C" int aether_selftest_bounded_wait(int64_t limit_cycles, void* stream) 
         return set_error(AE_BAD_ARG, "aether_selftest_bounded_wait: limit_cycles must be in [1, 2e9] (about a second at most)");
     int* status = device_status_word();
     if (!status) return set_error(AE_CUDA, "aether_selftest_bounded_wait: no status word (pinned allocation failed)");
-    selftest_bounded_wait_kernel<<<1, 32, 0, static_cast<cudaStream_t>(stream)>>>(status, (long long)limit_cycles);
+    launch(selftest_bounded_wait_kernel, 1, 32, 0, static_cast<cudaStream_t>(stream), status, (long long)limit_cycles);
     count_launch();
     return check_launch("selftest_bounded_wait_kernel");
 }

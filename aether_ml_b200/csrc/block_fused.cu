@@ -41,6 +41,7 @@ __global__ void __launch_bounds__(256) bn_act_pool_fwd_kernel(const float* __res
                                                               unsigned total, int W, int C4, int fH_, int fW_, int Wo,
                                                               __nv_bfloat16* __restrict__ copy, int copy_ld,
                                                               float* __restrict__ xsel) {
+    pdl_wait();
     const int fH = F ? F : fH_, fW = F ? F : fW_;
     for (unsigned idx = blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += gridDim.x * blockDim.x) {
         const unsigned cv = idx % (unsigned)C4;
@@ -91,6 +92,7 @@ __global__ void __launch_bounds__(256) bn_act_pool_bwd_reduce_sel_kernel(
     const float* __restrict__ xsel, const float* __restrict__ dpool, const float* __restrict__ gamma,
     const float* __restrict__ beta, const float* __restrict__ mean, const float* __restrict__ var, float eps, float alpha,
     long long windows, long long win_per_block, int C, float* __restrict__ part) {
+    pdl_wait();
     const long long w0 = blockIdx.x * win_per_block;
     long long w1 = w0 + win_per_block;
     if (w1 > windows) w1 = windows;
@@ -152,6 +154,7 @@ __global__ void __launch_bounds__(256) bn_act_pool_bwd_reduce_kernel(
     const float* __restrict__ gamma, const float* __restrict__ beta, const float* __restrict__ mean,
     const float* __restrict__ var, float eps, float alpha, long long windows, long long win_per_block, int W, int C, int fH,
     int fW, int Wo, float* __restrict__ part) {
+    pdl_wait();
     const long long w0 = blockIdx.x * win_per_block;
     long long w1 = w0 + win_per_block;
     if (w1 > windows) w1 = windows;
@@ -219,6 +222,7 @@ __global__ void __launch_bounds__(256) bn_act_pool_bwd_apply_kernel(
     const float* __restrict__ var, float eps, float alpha, const float* __restrict__ coeff, float* __restrict__ dx,
     unsigned total, int W, int C, int fH_, int fW_, int Wo, __nv_bfloat16* __restrict__ copy, int copy_ld,
     float* __restrict__ colsum_part) {
+    pdl_wait();
     const int fH = F ? F : fH_, fW = F ? F : fW_;
     const int C4 = C >> 2;
     // column sums of dx (the bias gradient of the convolution in front): only with grids whose stride keeps a thread on
@@ -341,11 +345,11 @@ extern "C" int aether_bn_act_pool_fwd_copy(const float* x, const float* partials
     const int fb = fused_blocks(windows4, 256, 16);
     __nv_bfloat16* copy = static_cast<__nv_bfloat16*>(operand_copy);
     if (fH == 2 && fW == 2)
-        bn_act_pool_fwd_kernel<2><<<fb, 256, 0, st>>>(x, coeff, coeff + C, alpha, pooled, argmax, (unsigned)windows4, W, C / 4,
-                                                     fH, fW, W / fW, copy, copy_ld, selected_x);
+        launch(bn_act_pool_fwd_kernel<2>, fb, 256, 0, st, x, coeff, coeff + C, alpha, pooled, argmax, (unsigned)windows4, W, C / 4, fH, fW,
+               W / fW, copy, copy_ld, selected_x);
     else
-        bn_act_pool_fwd_kernel<0><<<fb, 256, 0, st>>>(x, coeff, coeff + C, alpha, pooled, argmax, (unsigned)windows4, W, C / 4,
-                                                     fH, fW, W / fW, copy, copy_ld, selected_x);
+        launch(bn_act_pool_fwd_kernel<0>, fb, 256, 0, st, x, coeff, coeff + C, alpha, pooled, argmax, (unsigned)windows4, W, C / 4, fH, fW,
+               W / fW, copy, copy_ld, selected_x);
     count_launch();
     return check_launch("aether_bn_act_pool_fwd");
 }
@@ -391,11 +395,11 @@ extern "C" int aether_bn_act_pool_bwd_copy(const float* x, const float* dpooled,
     float* coeff = part + (size_t)bn_partial_blocks(rows) * 3 * C;
     if (selected_x) {
         if (!aligned16(selected_x)) return set_error(AE_BAD_ARG, "aether_bn_act_pool_bwd_copy: selected_x must be 16-byte aligned");
-        bn_act_pool_bwd_reduce_sel_kernel<<<nb, 256, 0, st>>>(selected_x, dpooled, gamma, beta, batch_mean, batch_var, eps, alpha,
-                                                              windows, (windows + nb - 1) / nb, C, part);
+        launch(bn_act_pool_bwd_reduce_sel_kernel, nb, 256, 0, st, selected_x, dpooled, gamma, beta, batch_mean, batch_var, eps, alpha,
+               windows, (windows + nb - 1) / nb, C, part);
     } else {
-        bn_act_pool_bwd_reduce_kernel<<<nb, 256, 0, st>>>(x, dpooled, argmax, gamma, beta, batch_mean, batch_var, eps, alpha, windows,
-                                                          (windows + nb - 1) / nb, W, C, fH, fW, W / fW, part);
+        launch(bn_act_pool_bwd_reduce_kernel, nb, 256, 0, st, x, dpooled, argmax, gamma, beta, batch_mean, batch_var, eps, alpha, windows,
+               (windows + nb - 1) / nb, W, C, fH, fW, W / fW, part);
     }
     count_launch();
     bn_backward_coeffs(part, nb, C, rows, gamma, batch_mean, batch_var, eps, dgamma, dbeta, coeff, channel_scale, st);
@@ -406,13 +410,11 @@ extern "C" int aether_bn_act_pool_bwd_copy(const float* x, const float* dpooled,
         *colsum_rows = fb;
     }
     if (fH == 2 && fW == 2)
-        bn_act_pool_bwd_apply_kernel<2><<<fb, 256, 0, st>>>(x, dpooled, argmax, gamma, beta, batch_mean, batch_var, eps, alpha,
-                                                           coeff, dx, (unsigned)windows4, W, C, fH, fW, W / fW, copy, copy_ld,
-                                                           copy ? colsum_part : nullptr);
+        launch(bn_act_pool_bwd_apply_kernel<2>, fb, 256, 0, st, x, dpooled, argmax, gamma, beta, batch_mean, batch_var, eps, alpha, coeff,
+               dx, (unsigned)windows4, W, C, fH, fW, W / fW, copy, copy_ld, copy ? colsum_part : nullptr);
     else
-        bn_act_pool_bwd_apply_kernel<0><<<fb, 256, 0, st>>>(x, dpooled, argmax, gamma, beta, batch_mean, batch_var, eps, alpha,
-                                                           coeff, dx, (unsigned)windows4, W, C, fH, fW, W / fW, copy, copy_ld,
-                                                           copy ? colsum_part : nullptr);
+        launch(bn_act_pool_bwd_apply_kernel<0>, fb, 256, 0, st, x, dpooled, argmax, gamma, beta, batch_mean, batch_var, eps, alpha, coeff,
+               dx, (unsigned)windows4, W, C, fH, fW, W / fW, copy, copy_ld, copy ? colsum_part : nullptr);
     count_launch();
     return check_launch("aether_bn_act_pool_bwd");
 }

@@ -9,6 +9,7 @@
 #include <atomic>
 
 #include "../../include/aether_b200.h"
+#include "launch.cuh"
 
 namespace aether {
 

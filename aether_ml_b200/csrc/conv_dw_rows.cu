@@ -87,8 +87,10 @@ __global__ void __launch_bounds__(DWR_THREADS, 1) dw_rows_kernel(const __grid_co
         tmem_alloc(sTmemPtr, 512);
         tmem_relinquish();
     }
+    pdl_wait();                       // set-up done; from here on global memory is touched
     tc_fence_before();
     __syncthreads();
+
     tc_fence_after();
     const uint32_t tmem_base = *tmem_ptr_generic;
 
@@ -289,7 +291,7 @@ int run_rows_dw(const void* x_sh, int Cin_p, int H, int W, int S, const void* dy
     static PerDeviceSmem configured;
     if ((rc = ensure_dynamic_smem(dw_rows_kernel, smem_max, configured, "dw_rows"))) return rc;
     prof_begin(PK_DW, st);
-    dw_rows_kernel<<<units * (sa + sb), DWR_THREADS, smem, st>>>(p);
+    launch(dw_rows_kernel, units * (sa + sb), DWR_THREADS, smem, st, p);
     prof_end(PK_DW, st);
     count_launch();
     *used = true;

@@ -97,7 +97,6 @@ __global__ void __launch_bounds__(FirstCfg<STATS>::THREADS, 1) first_conv_kernel
         }
         mbar_fence_init();
     }
-    for (int i = threadIdx.x; i < NT; i += blockDim.x) bias_s[i] = (p.bias != nullptr && i < p.Cout) ? p.bias[i] : 0.f;
     for (int k = threadIdx.x; k < 64; k += blockDim.x) {
         const int kk = k < p.K ? k : 0;
         const int tap = kk / p.Cin, c = kk - tap * p.Cin;
@@ -106,6 +105,12 @@ __global__ void __launch_bounds__(FirstCfg<STATS>::THREADS, 1) first_conv_kernel
         kj_s[k] = j;
         koff_s[k] = (i * p.W + j) * p.Cin + c;
     }
+    if (warp == FT_PROD_WARPS) {
+        tmem_alloc(sTmemPtr, tmem_cols);
+        tmem_relinquish();
+    }
+    pdl_wait();                       // set-up done; from here on global memory is touched
+    for (int i = threadIdx.x; i < NT; i += blockDim.x) bias_s[i] = (p.bias != nullptr && i < p.Cout) ? p.bias[i] : 0.f;
     // filter operand: row n = output channel, element k at byte (k/8 ^ n%8)*16 + (k%8)*2 of the row
     for (int it = threadIdx.x; it < NT * (p.KP >> 3); it += blockDim.x) {
         const int n = it / (p.KP >> 3), ch = it - n * (p.KP >> 3);
@@ -119,12 +124,9 @@ __global__ void __launch_bounds__(FirstCfg<STATS>::THREADS, 1) first_conv_kernel
         *reinterpret_cast<uint4*>(gen_base + (sW - smem_base) + n * 128 + ((ch ^ (n & 7)) << 4)) = q;
     }
     fence_proxy_async_smem();
-    if (warp == FT_PROD_WARPS) {
-        tmem_alloc(sTmemPtr, tmem_cols);
-        tmem_relinquish();
-    }
     tc_fence_before();
     __syncthreads();
+
     tc_fence_after();
     const uint32_t tmem_base = *tmem_ptr_generic;
     const int grid = (int)gridDim.x;
@@ -465,8 +467,10 @@ __global__ void __launch_bounds__(FD_THREADS, 1) first_dw_kernel(const __grid_co
         tmem_alloc(sTmemPtr, tmem_cols);
         tmem_relinquish();
     }
+    pdl_wait();                       // set-up done; from here on global memory is touched
     tc_fence_before();
     __syncthreads();
+
     tc_fence_after();
     const uint32_t tmem_base = *tmem_ptr_generic;
     const int grid = (int)gridDim.x;
@@ -695,8 +699,8 @@ int first_tc_fwd(const AetherConvDesc& d, const float* x, const float* w, const 
                        : ensure_dynamic_smem(first_conv_kernel<false>, 232448, configured[0], "first_conv"))
         return rc;
     const int grid = first_tc_grid(p.ntiles);
-    if (stats) first_conv_kernel<true><<<grid, FirstCfg<true>::THREADS, smem, st>>>(p);
-    else first_conv_kernel<false><<<grid, FirstCfg<false>::THREADS, smem, st>>>(p);
+    if (stats) launch(first_conv_kernel<true>, grid, FirstCfg<true>::THREADS, smem, st, p);
+    else launch(first_conv_kernel<false>, grid, FirstCfg<false>::THREADS, smem, st, p);
     count_launch();
     return check_launch("first_conv_kernel");
 }
@@ -776,7 +780,7 @@ int first_tc_bwd_filter(const AetherConvDesc& d, const float* x, const float* dy
     const int smem = 1024 + p.stages * p.stage_bytes + tail;
     static PerDeviceSmem configured;
     if (int rc0 = ensure_dynamic_smem(first_dw_kernel, 232448, configured, "first_dw")) return rc0;
-    first_dw_kernel<<<grid, FD_THREADS, smem, st>>>(p);
+    launch(first_dw_kernel, grid, FD_THREADS, smem, st, p);
     count_launch();
     int rc = check_launch("first_dw_kernel");
     if (rc) return rc;

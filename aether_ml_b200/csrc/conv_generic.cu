@@ -25,6 +25,7 @@ template <int MAXD>
 __global__ void __launch_bounds__(256) gen_fwd_pointwise_few_kernel(const float* __restrict__ x, const float* __restrict__ w,
                                                                     const float* __restrict__ b, float* __restrict__ y,
                                                                     long long rows, int Cin, int Cout) {
+    pdl_wait();
     extern __shared__ __align__(16) float head_wT[];
     head_load_filter_T(w, head_wT, Cin, Cout);
     const int lane = threadIdx.x & 31;
@@ -70,6 +71,7 @@ template <int CIN>
 __global__ void __launch_bounds__(256) gen_dx_fewc_kernel(const float* __restrict__ dy, const float* __restrict__ w,
                                                           float* __restrict__ dx, int S, int H, int W, int Cout, int fH,
                                                           int fW, int sH, int sW, int pH, int pW, int Ho, int Wo) {
+    pdl_wait();
     const long long total = 1LL * S * H * W;
     const int C4 = Cout >> 2;
     for (long long pix = blockIdx.x * (long long)blockDim.x + threadIdx.x; pix < total;
@@ -112,6 +114,7 @@ __global__ void __launch_bounds__(256) gen_dx_fewc_kernel(const float* __restric
 // ---------------------------------------------------------------------------------- dW, dB of classifier heads: partials added in fixed order
 __global__ void gen_dw_reduce_kernel(const float* __restrict__ part, int nblocks, int entries, int Cout,
                                      float* __restrict__ dw, float* __restrict__ db) {
+    pdl_wait();
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= entries + Cout) return;
     float s = 0.f;
@@ -129,6 +132,7 @@ __global__ void gen_dw_reduce_kernel(const float* __restrict__ part, int nblocks
 template <int MAXD>
 __global__ void __launch_bounds__(256) head_dx_kernel(const float* __restrict__ dy, const float* __restrict__ w,
                                                       float* __restrict__ dx, long long rows, int Cin, int Cout) {
+    pdl_wait();
     extern __shared__ __align__(16) float head_wT[];
     head_load_filter_T(w, head_wT, Cin, Cout);
     const int C4 = Cin >> 2;
@@ -165,6 +169,7 @@ template <int MAXD>
 __global__ void __launch_bounds__(256) head_dw_partial_kernel(const float* __restrict__ x, const float* __restrict__ dy,
                                                               float* __restrict__ part, long long rows, int Cin, int Cout,
                                                               long long rows_per_block) {
+    pdl_wait();
     const long long r0 = blockIdx.x * rows_per_block;
     long long r1 = r0 + rows_per_block;
     if (r1 > rows) r1 = rows;
@@ -228,7 +233,7 @@ int generic_conv_fwd(const AetherConvDesc& d, const float* x, const float* w, co
         if (int rc = ensure_dynamic_smem(gen_fwd_pointwise_few_kernel<16>, 96 * 1024, configured, "head forward")) return rc;
         long long nb = (rows + 7) / 8;                        // a warp per row, 8 rows per block and pass
         if (nb > 2LL * num_sms()) nb = 2LL * num_sms();       // every block loads the filter once
-        gen_fwd_pointwise_few_kernel<16><<<(int)nb, 256, smem, st>>>(x, w, b, y, rows, d.Cin, d.Cout);
+        launch(gen_fwd_pointwise_few_kernel<16>, (int)nb, 256, smem, st, x, w, b, y, rows, d.Cin, d.Cout);
         count_launch();
         return check_launch("gen_fwd_pointwise_few_kernel");
     }
@@ -241,8 +246,7 @@ int generic_conv_bwd_data(const AetherConvDesc& d, const float* dy, const float*
     if (d.Cin <= 4 && d.Cout % 4 == 0 && (reinterpret_cast<uintptr_t>(dy) & 15u) == 0 && (reinterpret_cast<uintptr_t>(w) & 15u) == 0) {
         const int nb = gen_blocks(1LL * d.S * d.H * d.W, 256);
 #define AETHER_DX_FEWC(CIN)                                                                                          \
-    gen_dx_fewc_kernel<CIN><<<nb, 256, 0, st>>>(dy, w, dx, d.S, d.H, d.W, d.Cout, d.fH, d.fW, d.sH, d.sW, d.padH, d.padW, \
-                                               Ho, Wo)
+    launch(gen_dx_fewc_kernel<CIN>, nb, 256, 0, st, dy, w, dx, d.S, d.H, d.W, d.Cout, d.fH, d.fW, d.sH, d.sW, d.padH, d.padW, Ho, Wo)
         switch (d.Cin) {
             case 1: AETHER_DX_FEWC(1); break;
             case 2: AETHER_DX_FEWC(2); break;
@@ -259,7 +263,7 @@ int generic_conv_bwd_data(const AetherConvDesc& d, const float* dy, const float*
         static PerDeviceSmem configured;
         if (int rc = ensure_dynamic_smem(head_dx_kernel<16>, 96 * 1024, configured, "head dX")) return rc;
         long long nb = rows < 2LL * num_sms() ? rows : 2LL * num_sms();
-        head_dx_kernel<16><<<(int)nb, 256, smem, st>>>(dy, w, dx, rows, d.Cin, d.Cout);
+        launch(head_dx_kernel<16>, (int)nb, 256, smem, st, dy, w, dx, rows, d.Cin, d.Cout);
         count_launch();
         return check_launch("head_dx_kernel");
     }
@@ -293,11 +297,11 @@ int generic_conv_bwd_filter(const AetherConvDesc& d, const float* x, const float
     const long long ppb = (npix + nb - 1) / nb;
     const int entries = d.Cin * d.Cout;
     float* part = static_cast<float*>(ws);
-    head_dw_partial_kernel<16><<<dim3(nb, ceil_div(d.Cin / 4, 256)), 256, 0, st>>>(x, dy, part, npix, d.Cin, d.Cout, ppb);
+    launch(head_dw_partial_kernel<16>, dim3(nb, ceil_div(d.Cin / 4, 256)), 256, 0, st, x, dy, part, npix, d.Cin, d.Cout, ppb);
     count_launch();
     int rc = check_launch("head_dw_partial_kernel");
     if (rc) return rc;
-    gen_dw_reduce_kernel<<<ceil_div(entries + d.Cout, 256), 256, 0, st>>>(part, nb, entries, d.Cout, dw, db);
+    launch(gen_dw_reduce_kernel, ceil_div(entries + d.Cout, 256), 256, 0, st, part, nb, entries, d.Cout, dw, db);
     count_launch();
     return check_launch("gen_dw_reduce_kernel");
 }

@@ -140,7 +140,6 @@ __global__ void __launch_bounds__(HALO_THREADS, 1) halo_conv_kernel(const __grid
         tma_prefetch_desc(&p.tm_in);
         tma_prefetch_desc(&p.tm_w);
     }
-    for (int i = threadIdx.x; i < NT; i += blockDim.x) bias_s[i] = (p.bias != nullptr && i < p.n_out) ? p.bias[i] : 0.f;
     if (warp == 1) {
         if (PAIR) {
             tmem_alloc_pair(sTmemPtr, tmem_cols);
@@ -150,9 +149,12 @@ __global__ void __launch_bounds__(HALO_THREADS, 1) halo_conv_kernel(const __grid
             tmem_relinquish();
         }
     }
+    pdl_wait();                       // set-up done; from here on global memory is touched
+    for (int i = threadIdx.x; i < NT; i += blockDim.x) bias_s[i] = (p.bias != nullptr && i < p.n_out) ? p.bias[i] : 0.f;
     tc_fence_before();
     if (PAIR) cluster_sync_all();
     else __syncthreads();
+
     tc_fence_after();
     const uint32_t tmem_base = *tmem_ptr_generic;
 
@@ -554,23 +556,9 @@ int run_halo_igemm(bool tf32, const void* in, int in_C, int in_H, int in_W, int 
     if ((rc = ensure_dynamic_smem(kernels[ki], smem_max, configured[ki], "halo_conv"))) return rc;
     prof_begin(prof_kind, st);
     if (g.pair) {
-        cudaLaunchConfig_t cfg;
-        memset(&cfg, 0, sizeof(cfg));
-        cfg.gridDim = dim3(g.grid, 1, 1);
-        cfg.blockDim = dim3(HALO_THREADS, 1, 1);
-        cfg.dynamicSmemBytes = smem;
-        cfg.stream = st;
-        cudaLaunchAttribute attr;
-        attr.id = cudaLaunchAttributeClusterDimension;
-        attr.val.clusterDim.x = 2;
-        attr.val.clusterDim.y = 1;
-        attr.val.clusterDim.z = 1;
-        cfg.attrs = &attr;
-        cfg.numAttrs = 1;
-        const cudaError_t e = cudaLaunchKernelEx(&cfg, kernels[ki], p);
-        if (e != cudaSuccess) return set_error(AE_CUDA, "halo_conv_kernel (CTA pairs): %s", cudaGetErrorString(e));
+        launch_cluster(kernels[ki], 2, g.grid, HALO_THREADS, smem, st, p);
     } else {
-        kernels[ki]<<<g.grid, HALO_THREADS, smem, st>>>(p);
+        launch(kernels[ki], g.grid, HALO_THREADS, smem, st, p);
     }
     prof_end(prof_kind, st);
     count_launch();

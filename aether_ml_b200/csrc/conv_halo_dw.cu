@@ -72,8 +72,10 @@ __global__ void __launch_bounds__(DWH_THREADS, 1) dw_halo_kernel(const __grid_co
         tmem_alloc(sTmemPtr, 512);
         tmem_relinquish();
     }
+    pdl_wait();                       // set-up done; from here on global memory is touched
     tc_fence_before();
     __syncthreads();
+
     tc_fence_after();
     const uint32_t tmem_base = *tmem_ptr_generic;
 
@@ -252,7 +254,7 @@ int run_halo_dw(const void* x_sh, int Cin_p, int H, int W, int S, const void* dy
     static PerDeviceSmem configured;
     if (int rc0 = ensure_dynamic_smem(dw_halo_kernel, smem_max, configured, "dw_halo")) return rc0;
     prof_begin(PK_DW, st);
-    dw_halo_kernel<<<dim3((unsigned)splits, gy), DWH_THREADS, smem, st>>>(p);
+    launch(dw_halo_kernel, dim3((unsigned)splits, gy), DWH_THREADS, smem, st, p);
     prof_end(PK_DW, st);
     count_launch();
     *used = true;

@@ -99,6 +99,7 @@ __device__ __forceinline__ float acc_elem(unsigned long long v, int hi) {
 template <int BM, int BN, int TM, int TN, bool DX, bool VEC>
 __global__ void __launch_bounds__((BM / TM) * (BN / TN), 512 / ((BM / TM) * (BN / TN)))
 simt_conv_kernel(const SimtGemm g, int n_tiles_n) {
+    pdl_wait();
     constexpr int THREADS = (BM / TM) * (BN / TN);
     constexpr int BK = SIMT_BK;
     using LA = SimtLoad<BM, THREADS>;
@@ -322,6 +323,7 @@ struct SimtDw {
 template <int BM, int BN, int TM, int TN, bool VEC>
 __global__ void __launch_bounds__((BM / TM) * (BN / TN), (BM == 128 && BN == 64) ? 3 : 512 / ((BM / TM) * (BN / TN)))
 simt_dw_kernel(const SimtDw g, int n_tiles_n) {
+    pdl_wait();
     constexpr int THREADS = (BM / TM) * (BN / TN);
     constexpr int BK = SIMT_BK;
     constexpr int MV = BM / 4, NV = BN / 4;                  // loads per pixel
@@ -496,8 +498,8 @@ static int launch_simt_conv(const SimtGemm& g, long long M, int classes, bool ve
     if (mt * ntn > 0x7fffffffLL) return set_error(AE_UNSUPPORTED, "convolution of %lld pixels and %d channels is too large", M, g.N);
     const dim3 grid((unsigned)(mt * ntn), 1, (unsigned)classes);
     constexpr int THREADS = (BM / TM) * (BN / TN);
-    if (vec) simt_conv_kernel<BM, BN, TM, TN, DX, true><<<grid, THREADS, 0, st>>>(g, ntn);
-    else simt_conv_kernel<BM, BN, TM, TN, DX, false><<<grid, THREADS, 0, st>>>(g, ntn);
+    if (vec) launch(simt_conv_kernel<BM, BN, TM, TN, DX, true>, grid, THREADS, 0, st, g, ntn);
+    else launch(simt_conv_kernel<BM, BN, TM, TN, DX, false>, grid, THREADS, 0, st, g, ntn);
     count_launch();
     return check_launch("simt_conv_kernel");
 }
@@ -578,8 +580,8 @@ template <int BM, int BN, int TM, int TN>
 static void launch_simt_dw(const SimtDw& g, const SimtDwPlan& p, bool vec, cudaStream_t st) {
     const dim3 grid((unsigned)(p.tiles_k * p.tiles_n), (unsigned)p.splits);
     constexpr int THREADS = (BM / TM) * (BN / TN);
-    if (vec) simt_dw_kernel<BM, BN, TM, TN, true><<<grid, THREADS, 0, st>>>(g, p.tiles_n);
-    else simt_dw_kernel<BM, BN, TM, TN, false><<<grid, THREADS, 0, st>>>(g, p.tiles_n);
+    if (vec) launch(simt_dw_kernel<BM, BN, TM, TN, true>, grid, THREADS, 0, st, g, p.tiles_n);
+    else launch(simt_dw_kernel<BM, BN, TM, TN, false>, grid, THREADS, 0, st, g, p.tiles_n);
     count_launch();
 }
 

@@ -80,6 +80,7 @@ __global__ void __launch_bounds__(SC_THREADS) smallc_fwd_kernel(const SmallcGeom
                                                                 const float* __restrict__ w, const float* __restrict__ b,
                                                                 float* __restrict__ y, float* __restrict__ stats,
                                                                 long long ntiles) {
+    pdl_wait();
     extern __shared__ float sm[];
     __shared__ SmallcTables tab;
     __shared__ __align__(16) float red_s[SC_THREADS * 4];    // statistics, used once at the end of the kernel
@@ -173,6 +174,7 @@ template <int KPG>
 __global__ void __launch_bounds__(SC_THREADS) smallc_dw_kernel(const SmallcGeom g, const float* __restrict__ x,
                                                                const float* __restrict__ dy, float* __restrict__ part,
                                                                long long ntiles) {
+    pdl_wait();
     extern __shared__ float sm[];
     __shared__ SmallcTables tab;
     float* colT = sm;                         // [K][TP]
@@ -233,6 +235,7 @@ __global__ void __launch_bounds__(SC_THREADS) smallc_dw_kernel(const SmallcGeom 
 // dw[e] / db[d] = sum over CTAs of the partials, 8 lanes per output combined in fixed order.
 __global__ void __launch_bounds__(256) smallc_reduce_kernel(const float* __restrict__ part, int nblocks, int K, int Cout,
                                                             float* __restrict__ dw, float* __restrict__ db) {
+    pdl_wait();
     __shared__ float red[8][32];
     const int el = threadIdx.x & 31, ln = threadIdx.x >> 5;
     const int e = blockIdx.x * 32 + el;
@@ -308,7 +311,7 @@ static int launch_smallc_fwd(const SmallcGeom& g, const float* x, const float* w
     static PerDeviceSmem configured;
     int rc = smallc_smem(smallc_fwd_kernel<R>, smem, configured, "smallc_fwd");
     if (rc) return rc;
-    smallc_fwd_kernel<R><<<nb, SC_THREADS, smem, st>>>(g, x, w, b, y, stats, ntiles);
+    launch(smallc_fwd_kernel<R>, nb, SC_THREADS, smem, st, g, x, w, b, y, stats, ntiles);
     count_launch();
     return check_launch("smallc_fwd_kernel");
 }
@@ -344,7 +347,7 @@ static int launch_smallc_dw(const SmallcGeom& g, const float* x, const float* dy
     static PerDeviceSmem configured;
     int rc = smallc_smem(smallc_dw_kernel<KPG>, smem, configured, "smallc_dw");
     if (rc) return rc;
-    smallc_dw_kernel<KPG><<<nb, SC_THREADS, smem, st>>>(g, x, dy, part, ntiles);
+    launch(smallc_dw_kernel<KPG>, nb, SC_THREADS, smem, st, g, x, dy, part, ntiles);
     count_launch();
     return check_launch("smallc_dw_kernel");
 }
@@ -367,14 +370,14 @@ int smallc_conv_bwd_filter(const AetherConvDesc& d, const float* x, const float*
     else if (g.KPG <= 8) rc = launch_smallc_dw<8>(g, xs, dy, part, nb, ntiles, smem, st);
     else rc = launch_smallc_dw<16>(g, xs, dy, part, nb, ntiles, smem, st);
     if (rc) return rc;
-    smallc_reduce_kernel<<<ceil_div((g.K + 1) * g.Cout, 32), 256, 0, st>>>(part, nb, g.K, g.Cout, dw, db);
+    launch(smallc_reduce_kernel, ceil_div((g.K + 1) * g.Cout, 32), 256, 0, st, part, nb, g.K, g.Cout, dw, db);
     count_launch();
     return check_launch("smallc_reduce_kernel");
 }
 
 // Sums nb partials of [K + 1][Cout] floats (row K = dB) into dw / db in fixed order (also used by conv_first_tc.cu).
 int smallc_reduce_partials(const float* part, int nb, int K, int Cout, float* dw, float* db, cudaStream_t st) {
-    smallc_reduce_kernel<<<ceil_div((K + 1) * Cout, 32), 256, 0, st>>>(part, nb, K, Cout, dw, db);
+    launch(smallc_reduce_kernel, ceil_div((K + 1) * Cout, 32), 256, 0, st, part, nb, K, Cout, dw, db);
     count_launch();
     return check_launch("smallc_reduce_kernel");
 }

@@ -197,9 +197,11 @@ __global__ void __launch_bounds__(IGEMM_THREADS, 1) igemm_conv_kernel(const __gr
             tmem_relinquish();
         }
     }
+    pdl_wait();                       // set-up done; from here on global memory is touched
     tc_fence_before();
     if (PAIR) cluster_sync_all();     // the other CTA's barriers exist before anything is sent to them
     else __syncthreads();
+
     tc_fence_after();
     const uint32_t tmem_base = *tmem_ptr_generic;
 
@@ -576,9 +578,11 @@ __global__ void __launch_bounds__(DW_THREADS, 1) dw_conv_kernel(const __grid_con
             tmem_relinquish();
         }
     }
+    pdl_wait();                       // set-up done; from here on global memory is touched
     tc_fence_before();
     if (PAIR) cluster_sync_all();
     else __syncthreads();
+
     tc_fence_after();
     const uint32_t tmem_base = *tmem_ptr_generic;
 
@@ -720,6 +724,7 @@ __global__ void __launch_bounds__(DW_THREADS, 1) dw_conv_kernel(const __grid_con
 __global__ void __launch_bounds__(256) dw_reduce_kernel(const float* __restrict__ part, float* __restrict__ dw, int splits,
                                                         int U, int UC, int ldn, int cblocks, int taps, int Cin, int Cout,
                                                         int tap_split, int splits2) {
+    pdl_wait();
     __shared__ float red[8][32];
     __shared__ float4 red4[8][32];
     const int el = threadIdx.x & 31, ln = threadIdx.x >> 5;
@@ -795,6 +800,7 @@ template <bool COLSUM>
 __global__ void __launch_bounds__(256) cast_bf16_kernel(const float* __restrict__ src, __nv_bfloat16* __restrict__ dst,
                                                         long long rows, int C, int Cp, float* __restrict__ colsum_part,
                                                         long long rows_per_block) {
+    pdl_wait();
     const int G = Cp / 8;                 // 8-channel groups per row
     const long long r_begin = blockIdx.x * rows_per_block;
     long long r_end = r_begin + rows_per_block;
@@ -856,6 +862,7 @@ __global__ void __launch_bounds__(256) cast_bf16_kernel(const float* __restrict_
 // Column sums of an fp32 [rows][C] matrix into part[block][C] (used for dB when no cast pass runs).
 __global__ void __launch_bounds__(256) colsum_kernel(const float* __restrict__ src, long long rows, int C,
                                                      float* __restrict__ part, long long rows_per_block) {
+    pdl_wait();
     const long long r_begin = blockIdx.x * rows_per_block;
     long long r_end = r_begin + rows_per_block;
     if (r_end > rows) r_end = rows;
@@ -883,6 +890,7 @@ __global__ void __launch_bounds__(256) colsum_kernel(const float* __restrict__ s
 // out[c] = sum over blocks of part[block][C]: 32 columns x 8 row lanes per CTA, lanes combined in fixed order.
 __global__ void __launch_bounds__(256) colsum_finish_kernel(const float* __restrict__ part, int nblocks, int C,
                                                             float* __restrict__ out) {
+    pdl_wait();
     // 8 columns x 32 lanes per CTA: short serial chains, lanes combined in fixed order
     __shared__ float red[32][8];
     const int cl = threadIdx.x & 7, lane = threadIdx.x >> 3;
@@ -901,7 +909,7 @@ __global__ void __launch_bounds__(256) colsum_finish_kernel(const float* __restr
 }
 
 int colsum_finish(const float* part, int rows, int C, float* out, cudaStream_t st) {
-    colsum_finish_kernel<<<ceil_div(C, 8), 256, 0, st>>>(part, rows, C, out);
+    launch(colsum_finish_kernel, ceil_div(C, 8), 256, 0, st, part, rows, C, out);
     count_launch();
     return check_launch("colsum_finish_kernel");
 }
@@ -917,6 +925,7 @@ template <typename OutT>
 __global__ void __launch_bounds__(256) filter_shadow_tiled_kernel(const float* __restrict__ w, OutT* __restrict__ fwd,
                                                                   OutT* __restrict__ dx, int Cin, int Cout, int Cin_p,
                                                                   int Cout_p) {
+    pdl_wait();
     __shared__ float tile[32][33];
     const int tap = blockIdx.z;
     const int n0 = blockIdx.x * 32, k0 = blockIdx.y * 32;       // n: output channel, k: input channel
@@ -941,7 +950,7 @@ template <typename OutT>
 static int launch_filter_shadows(const float* w, OutT* fwd, OutT* dx, int taps, int Cin, int Cout, int Cin_p, int Cout_p,
                                  cudaStream_t st) {
     const dim3 grid((unsigned)ceil_div(Cout_p, 32), (unsigned)ceil_div(Cin_p, 32), (unsigned)taps);
-    filter_shadow_tiled_kernel<OutT><<<grid, dim3(32, 8), 0, st>>>(w, fwd, dx, Cin, Cout, Cin_p, Cout_p);
+    launch(filter_shadow_tiled_kernel<OutT>, grid, dim3(32, 8), 0, st, w, fwd, dx, Cin, Cout, Cin_p, Cout_p);
     count_launch();
     return check_launch("filter_shadow_tiled_kernel");
 }
@@ -979,7 +988,8 @@ int num_sms() {
 }
 
 // A stand-in with the pair kernels' launch shape for the occupancy query below.
-__global__ void __launch_bounds__(IGEMM_THREADS, 1) pair_probe_kernel() {}
+__global__ void __launch_bounds__(IGEMM_THREADS, 1) pair_probe_kernel() {
+    pdl_wait(); }
 
 bool cta_pairs_available() {
     static std::atomic<int> cache[AE_MAX_DEVICES];       // 0 = not asked yet, 1 = yes, 2 = no
@@ -1167,23 +1177,9 @@ static int launch_igemm_k(const IgemmParams& p, cudaStream_t st) {
     const int pk = p.sgn > 0 ? PK_IGEMM_FWD : PK_IGEMM_DX;
     prof_begin(pk, st);
     if (PAIR) {
-        cudaLaunchConfig_t cfg;
-        memset(&cfg, 0, sizeof(cfg));
-        cfg.gridDim = dim3(grid, 1, 1);
-        cfg.blockDim = dim3(IGEMM_THREADS, 1, 1);
-        cfg.dynamicSmemBytes = Cfg::SMEM_BYTES;
-        cfg.stream = st;
-        cudaLaunchAttribute attr;
-        attr.id = cudaLaunchAttributeClusterDimension;
-        attr.val.clusterDim.x = 2;
-        attr.val.clusterDim.y = 1;
-        attr.val.clusterDim.z = 1;
-        cfg.attrs = &attr;
-        cfg.numAttrs = 1;
-        const cudaError_t e = cudaLaunchKernelEx(&cfg, igemm_conv_kernel<TF32, NT, STATS, PAIR>, p);
-        if (e != cudaSuccess) return set_error(AE_CUDA, "igemm_conv_kernel (CTA pairs): %s", cudaGetErrorString(e));
+        launch_cluster(igemm_conv_kernel<TF32, NT, STATS, PAIR>, 2, grid, IGEMM_THREADS, Cfg::SMEM_BYTES, st, p);
     } else {
-        igemm_conv_kernel<TF32, NT, STATS, PAIR><<<grid, IGEMM_THREADS, Cfg::SMEM_BYTES, st>>>(p);
+        launch(igemm_conv_kernel<TF32, NT, STATS, PAIR>, grid, IGEMM_THREADS, Cfg::SMEM_BYTES, st, p);
     }
     prof_end(pk, st);
     count_launch();
@@ -1261,7 +1257,7 @@ static int launch_cast(const float* src, __nv_bfloat16* dst, long long rows, int
     prof_begin(PK_SHADOW, st);
     if (colsum_part) {
         const long long rpb = (rows + colsum_blocks - 1) / colsum_blocks;
-        cast_bf16_kernel<true><<<colsum_blocks, 256, 0, st>>>(src, dst, rows, C, Cp, colsum_part, rpb);
+        launch(cast_bf16_kernel<true>, colsum_blocks, 256, 0, st, src, dst, rows, C, Cp, colsum_part, rpb);
     } else {
         long long blocks = 8LL * num_sms();
         const int G = Cp / 8;
@@ -1269,7 +1265,7 @@ static int launch_cast(const float* src, __nv_bfloat16* dst, long long rows, int
         if (blocks * planes > rows) blocks = (rows + planes - 1) / planes;
         if (blocks < 1) blocks = 1;
         const long long rpb = (rows + blocks - 1) / blocks;
-        cast_bf16_kernel<false><<<(int)blocks, 256, 0, st>>>(src, dst, rows, C, Cp, nullptr, rpb);
+        launch(cast_bf16_kernel<false>, (int)blocks, 256, 0, st, src, dst, rows, C, Cp, nullptr, rpb);
     }
     prof_end(PK_SHADOW, st);
     count_launch();
@@ -1328,23 +1324,9 @@ static int launch_dw(const DwParams& p, int splits, int grid_y, cudaStream_t st)
     if (int rc = ensure_dynamic_smem(dw_conv_kernel<TF32, NB, PAIR>, Cfg::SMEM_BYTES, configured, "dw_conv")) return rc;
     prof_begin(PK_DW, st);
     if (PAIR) {
-        cudaLaunchConfig_t cfg;
-        memset(&cfg, 0, sizeof(cfg));
-        cfg.gridDim = dim3(2 * splits, grid_y, 1);
-        cfg.blockDim = dim3(DW_THREADS, 1, 1);
-        cfg.dynamicSmemBytes = Cfg::SMEM_BYTES;
-        cfg.stream = st;
-        cudaLaunchAttribute attr;
-        attr.id = cudaLaunchAttributeClusterDimension;
-        attr.val.clusterDim.x = 2;
-        attr.val.clusterDim.y = 1;
-        attr.val.clusterDim.z = 1;
-        cfg.attrs = &attr;
-        cfg.numAttrs = 1;
-        const cudaError_t e = cudaLaunchKernelEx(&cfg, dw_conv_kernel<TF32, NB, PAIR>, p);
-        if (e != cudaSuccess) return set_error(AE_CUDA, "dw_conv_kernel (CTA pairs): %s", cudaGetErrorString(e));
+        launch_cluster(dw_conv_kernel<TF32, NB, PAIR>, 2, dim3(2 * splits, grid_y), DW_THREADS, Cfg::SMEM_BYTES, st, p);
     } else {
-        dw_conv_kernel<TF32, NB, PAIR><<<dim3(splits, grid_y), DW_THREADS, Cfg::SMEM_BYTES, st>>>(p);
+        launch(dw_conv_kernel<TF32, NB, PAIR>, dim3(splits, grid_y), DW_THREADS, Cfg::SMEM_BYTES, st, p);
     }
     prof_end(PK_DW, st);
     count_launch();
@@ -1376,7 +1358,7 @@ int tc_conv_bwd(const AetherConvDesc& d, const float* x, const float* dy, const 
     if (pl.tf32) {
         if (db) {
             const long long rpb = (out_rows + pl.db_blocks - 1) / pl.db_blocks;
-            colsum_kernel<<<pl.db_blocks, 256, 0, st>>>(dy, out_rows, d.Cout, dbpart, rpb);
+            launch(colsum_kernel, pl.db_blocks, 256, 0, st, dy, out_rows, d.Cout, dbpart, rpb);
             count_launch();
             if ((rc = check_launch("colsum_kernel"))) return rc;
         }
@@ -1391,7 +1373,7 @@ int tc_conv_bwd(const AetherConvDesc& d, const float* x, const float* dy, const 
         dy_op = dysh;
     }
     if (db) {
-        colsum_finish_kernel<<<ceil_div(d.Cout, 8), 256, 0, st>>>(dbpart, db_rows, d.Cout, db);
+        launch(colsum_finish_kernel, ceil_div(d.Cout, 8), 256, 0, st, dbpart, db_rows, d.Cout, db);
         count_launch();
         if ((rc = check_launch("colsum_finish_kernel"))) return rc;
     }
@@ -1429,8 +1411,8 @@ int tc_conv_bwd(const AetherConvDesc& d, const float* x, const float* dy, const 
                               &sa, &sb, &tap_split, st, &dw_done)))
             return rc;
         if (dw_done) {
-            dw_reduce_kernel<<<dw_reduce_grid(pl.taps, d.Cin, d.Cout), 256, 0, st>>>(part, dw, sa, pl.dw_U, pl.KC, pl.Cout_p, pl.dw_cblocks, pl.taps,
-                                                            d.Cin, d.Cout, tap_split, sb);
+            launch(dw_reduce_kernel, dw_reduce_grid(pl.taps, d.Cin, d.Cout), 256, 0, st, part, dw, sa, pl.dw_U, pl.KC, pl.Cout_p,
+                   pl.dw_cblocks, pl.taps, d.Cin, d.Cout, tap_split, sb);
             count_launch();
             if ((rc = check_launch("dw_reduce_kernel"))) return rc;
         }
@@ -1439,8 +1421,8 @@ int tc_conv_bwd(const AetherConvDesc& d, const float* x, const float* dy, const 
                                   part, pl.dw_halo_splits, &splits, st, &dw_done)))
                 return rc;
             if (dw_done) {
-                dw_reduce_kernel<<<dw_reduce_grid(pl.taps, d.Cin, d.Cout), 256, 0, st>>>(part, dw, splits, pl.dw_U, pl.KC, pl.Cout_p, pl.dw_cblocks,
-                                                                pl.taps, d.Cin, d.Cout, pl.taps, splits);
+                launch(dw_reduce_kernel, dw_reduce_grid(pl.taps, d.Cin, d.Cout), 256, 0, st, part, dw, splits, pl.dw_U, pl.KC, pl.Cout_p,
+                       pl.dw_cblocks, pl.taps, d.Cin, d.Cout, pl.taps, splits);
                 count_launch();
                 if ((rc = check_launch("dw_reduce_kernel"))) return rc;
             }
@@ -1474,8 +1456,8 @@ int tc_conv_bwd(const AetherConvDesc& d, const float* x, const float* dy, const 
         else rc = (pl.dw_nb == 2) ? launch_dw<false, 2, false>(p, pl.dw_splits, gy, st) : launch_dw<false, 1, false>(p, pl.dw_splits, gy, st);
         if (rc) return rc;
         if (!direct) {
-            dw_reduce_kernel<<<dw_reduce_grid(pl.taps, d.Cin, d.Cout), 256, 0, st>>>(p.part, dw, pl.dw_splits, pl.dw_U, pl.KC, pl.Cout_p,
-                                                            pl.dw_cblocks, pl.taps, d.Cin, d.Cout, pl.taps, pl.dw_splits);
+            launch(dw_reduce_kernel, dw_reduce_grid(pl.taps, d.Cin, d.Cout), 256, 0, st, p.part, dw, pl.dw_splits, pl.dw_U, pl.KC,
+                   pl.Cout_p, pl.dw_cblocks, pl.taps, d.Cin, d.Cout, pl.taps, pl.dw_splits);
             count_launch();
             if ((rc = check_launch("dw_reduce_kernel"))) return rc;
         }

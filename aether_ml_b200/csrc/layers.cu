@@ -33,6 +33,7 @@ __global__ void __launch_bounds__(256) bn_reduce_kernel(const float* __restrict_
                                                         float eps, long long rows, int C, float* __restrict__ part,
                                                         long long rows_per_block, const float* __restrict__ act_gamma,
                                                         const float* __restrict__ act_beta, float alpha) {
+    pdl_wait();
     const long long r0 = blockIdx.x * rows_per_block;
     long long r1 = r0 + rows_per_block;
     if (r1 > rows) r1 = rows;
@@ -117,6 +118,7 @@ __global__ void __launch_bounds__(256) bn_reduce_vec4_kernel(const float* __rest
                                                              float eps, long long rows, int C, float* __restrict__ part,
                                                              long long rows_per_block, const float* __restrict__ act_gamma,
                                                              const float* __restrict__ act_beta, float alpha) {
+    pdl_wait();
     const long long r0 = blockIdx.x * rows_per_block;
     long long r1 = r0 + rows_per_block;
     if (r1 > rows) r1 = rows;
@@ -224,8 +226,8 @@ static void launch_bn_reduce(int nb, cudaStream_t st, const float* x, const floa
     const bool vec = (C & 3) == 0 && (reinterpret_cast<uintptr_t>(x) & 15u) == 0 &&
                      (MODE == 0 || (reinterpret_cast<uintptr_t>(dy) & 15u) == 0) &&
                      (act_gamma == nullptr || ((reinterpret_cast<uintptr_t>(act_gamma) | reinterpret_cast<uintptr_t>(act_beta)) & 15u) == 0);
-    if (vec) bn_reduce_vec4_kernel<MODE><<<nb, 256, 0, st>>>(x, dy, mean, var, eps, rows, C, part, rpb, act_gamma, act_beta, alpha);
-    else bn_reduce_kernel<MODE><<<nb, 256, 0, st>>>(x, dy, mean, var, eps, rows, C, part, rpb, act_gamma, act_beta, alpha);
+    if (vec) launch(bn_reduce_vec4_kernel<MODE>, nb, 256, 0, st, x, dy, mean, var, eps, rows, C, part, rpb, act_gamma, act_beta, alpha);
+    else launch(bn_reduce_kernel<MODE>, nb, 256, 0, st, x, dy, mean, var, eps, rows, C, part, rpb, act_gamma, act_beta, alpha);
 }
 
 // Merges the per-block (n, mean, M2) triples in double precision, writes batch mean / biased variance,
@@ -240,6 +242,7 @@ __global__ void __launch_bounds__(FIN_THREADS) bn_finalize_fwd_kernel(const floa
                                        float momentum, float* __restrict__ running_mean,
                                        float* __restrict__ running_var, float* __restrict__ batch_mean,
                                        float* __restrict__ batch_var, float* __restrict__ scale_shift) {
+    pdl_wait();
     // One pass over the per-block triples, all in double: N = sum n, S = sum n * mean, Q = sum (M2 + n * mean^2); then
     // M2 = Q - N * M^2.  The subtraction loses log2(mean^2 / var) of double's 53 bits, harmless for any ratio a float
     // tensor can show (the per-block M2 themselves carry 24 bits).  Lanes are combined in fixed order.
@@ -280,6 +283,7 @@ __global__ void __launch_bounds__(FIN_THREADS) bn_finalize_fwd_kernel(const floa
 __global__ void bn_eval_coeff_kernel(int C, const float* __restrict__ gamma, const float* __restrict__ beta, float eps,
                                      const float* __restrict__ running_mean, const float* __restrict__ running_var,
                                      float* __restrict__ scale_shift) {
+    pdl_wait();
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= C) return;
     const float sc = gamma[c] / sqrtf(running_var[c] + eps);
@@ -292,6 +296,7 @@ __global__ void __launch_bounds__(256) affine_channels_kernel(const float* __res
                                                               const float* __restrict__ scale,
                                                               const float* __restrict__ shift, long long n, int C,
                                                               float act_alpha) {
+    pdl_wait();
     const long long stride = (long long)gridDim.x * blockDim.x;
     const bool act = act_alpha >= 0.f;
     if ((C & 3) == 0) {
@@ -337,6 +342,7 @@ __global__ void __launch_bounds__(FIN_THREADS) bn_finalize_bwd_kernel(const floa
                                        const float* __restrict__ var, float eps, float* __restrict__ dgamma,
                                        float* __restrict__ dbeta, float* __restrict__ coeff,
                                        const float* __restrict__ pscale) {
+    pdl_wait();
     // pscale (nullable): per-channel factor that multiplied the layer's output (a fused spatial-dropout mask).  The
     // upstream gradient is that factor times what the kernels summed, so it scales both sums and the dy coefficient.
     __shared__ double red_a[FIN_LANES][FIN_CH], red_b[FIN_LANES][FIN_CH];
@@ -382,6 +388,7 @@ __global__ void __launch_bounds__(256) bn_bwd_apply_kernel(const float* __restri
                                                            const float* __restrict__ act_beta,
                                                            const float* __restrict__ mean, const float* __restrict__ var,
                                                            float eps, float alpha) {
+    pdl_wait();
     const long long stride = (long long)gridDim.x * blockDim.x;
     if ((C & 3) == 0) {
         const long long n4 = n >> 2;
@@ -433,6 +440,7 @@ static int bn_blocks(long long rows) {
 }
 
 __global__ void coeff_scale_kernel(float* __restrict__ scale_shift, const float* __restrict__ m, int C) {
+    pdl_wait();
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= C) return;
     scale_shift[c] *= m[c];
@@ -457,11 +465,11 @@ float* bn_forward_coeffs(const float* x, const float* partials, long long nblock
     } else {
         nb = (int)nblocks;
     }
-    bn_finalize_fwd_kernel<<<ceil_div(C, FIN_CH), FIN_THREADS, 0, st>>>(src, nb, C, gamma, beta, eps, momentum, running_mean, running_var,
-                                                            batch_mean, batch_var, coeff);
+    launch(bn_finalize_fwd_kernel, ceil_div(C, FIN_CH), FIN_THREADS, 0, st, src, nb, C, gamma, beta, eps, momentum, running_mean,
+           running_var, batch_mean, batch_var, coeff);
     count_launch();
     if (channel_scale) {
-        coeff_scale_kernel<<<ceil_div(C, 128), 128, 0, st>>>(coeff, channel_scale, C);
+        launch(coeff_scale_kernel, ceil_div(C, 128), 128, 0, st, coeff, channel_scale, C);
         count_launch();
     }
     return coeff;
@@ -470,7 +478,7 @@ float* bn_forward_coeffs(const float* x, const float* partials, long long nblock
 // Inference coefficients from the running statistics into ws (2*C floats).
 float* bn_eval_coeffs(const float* gamma, const float* beta, const float* running_mean, const float* running_var, int C,
                       float eps, float* ws, cudaStream_t st) {
-    bn_eval_coeff_kernel<<<ceil_div(C, 128), 128, 0, st>>>(C, gamma, beta, eps, running_mean, running_var, ws);
+    launch(bn_eval_coeff_kernel, ceil_div(C, 128), 128, 0, st, C, gamma, beta, eps, running_mean, running_var, ws);
     count_launch();
     return ws;
 }
@@ -479,8 +487,7 @@ float* bn_eval_coeffs(const float* gamma, const float* beta, const float* runnin
 void bn_backward_coeffs(const float* part, int nb, int C, long long rows, const float* gamma, const float* mean,
                         const float* var, float eps, float* dgamma, float* dbeta, float* coeff, const float* pscale,
                         cudaStream_t st) {
-    bn_finalize_bwd_kernel<<<ceil_div(C, FIN_CH), FIN_THREADS, 0, st>>>(part, nb, C, rows, gamma, mean, var, eps, dgamma, dbeta, coeff,
-                                                            pscale);
+    launch(bn_finalize_bwd_kernel, ceil_div(C, FIN_CH), FIN_THREADS, 0, st, part, nb, C, rows, gamma, mean, var, eps, dgamma, dbeta, coeff, pscale);
     count_launch();
 }
 
@@ -506,10 +513,10 @@ extern "C" int aether_bn_fwd_train(const float* x, const float* gamma, const flo
     float* part = static_cast<float*>(ws);
     float* coeff = part + (size_t)nb * 3 * C;
     launch_bn_reduce<0>(nb, st, x, nullptr, nullptr, nullptr, eps, rows, C, part);
-    bn_finalize_fwd_kernel<<<ceil_div(C, FIN_CH), FIN_THREADS, 0, st>>>(part, nb, C, gamma, beta, eps, momentum, running_mean,
-                                                            running_var, batch_mean, batch_var, coeff);
+    launch(bn_finalize_fwd_kernel, ceil_div(C, FIN_CH), FIN_THREADS, 0, st, part, nb, C, gamma, beta, eps, momentum, running_mean,
+           running_var, batch_mean, batch_var, coeff);
     const long long n = rows * C;
-    affine_channels_kernel<<<blocks_for(n / 4 + 1, 256), 256, 0, st>>>(x, y, coeff, coeff + C, n, C, -1.f);
+    launch(affine_channels_kernel, blocks_for(n / 4 + 1, 256), 256, 0, st, x, y, coeff, coeff + C, n, C, -1.f);
     count_launch(3);
     return check_launch("aether_bn_fwd_train");
 }
@@ -529,10 +536,10 @@ extern "C" int aether_bn_fwd_train_partials(const float* x, const float* partial
     if ((C & 3) == 0 && (!aligned16(x) || !aligned16(y))) return set_error(AE_BAD_ARG, "aether_bn_fwd_train_partials: arrays must be 16-byte aligned");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     float* coeff = static_cast<float*>(ws);
-    bn_finalize_fwd_kernel<<<ceil_div(C, FIN_CH), FIN_THREADS, 0, st>>>(partials, (int)nblocks, C, gamma, beta, eps, momentum, running_mean,
-                                                            running_var, batch_mean, batch_var, coeff);
+    launch(bn_finalize_fwd_kernel, ceil_div(C, FIN_CH), FIN_THREADS, 0, st, partials, (int)nblocks, C, gamma, beta, eps, momentum,
+           running_mean, running_var, batch_mean, batch_var, coeff);
     const long long n = rows * C;
-    affine_channels_kernel<<<blocks_for(n / 4 + 1, 256), 256, 0, st>>>(x, y, coeff, coeff + C, n, C, -1.f);
+    launch(affine_channels_kernel, blocks_for(n / 4 + 1, 256), 256, 0, st, x, y, coeff, coeff + C, n, C, -1.f);
     count_launch(2);
     return check_launch("aether_bn_fwd_train_partials");
 }
@@ -589,10 +596,10 @@ extern "C" int aether_bn_fwd_train_static(const float* x, const float* gamma, co
     // partials, the finalize kernel stores all coefficients), so stale contents of a previous call never matter
     // and nothing has to be cleared.
     launch_bn_reduce<0>(nb, st, x, nullptr, nullptr, nullptr, eps, rows, C, part);
-    bn_finalize_fwd_kernel<<<ceil_div(C, FIN_CH), FIN_THREADS, 0, st>>>(part, nb, C, gamma, beta, eps, momentum, running_mean,
-                                                            running_var, batch_mean, batch_var, coeff);
+    launch(bn_finalize_fwd_kernel, ceil_div(C, FIN_CH), FIN_THREADS, 0, st, part, nb, C, gamma, beta, eps, momentum, running_mean,
+           running_var, batch_mean, batch_var, coeff);
     const long long n = rows * C;
-    affine_channels_kernel<<<blocks_for(n / 4 + 1, 256), 256, 0, st>>>(x, y, coeff, coeff + C, n, C, -1.f);
+    launch(affine_channels_kernel, blocks_for(n / 4 + 1, 256), 256, 0, st, x, y, coeff, coeff + C, n, C, -1.f);
     count_launch(3);
     return check_launch("aether_bn_fwd_train_static");
 }
@@ -606,9 +613,9 @@ extern "C" int aether_bn_fwd_eval(const float* x, const float* gamma, const floa
     if (ws_bytes < 2 * (size_t)C * sizeof(float)) return set_error(AE_BAD_ARG, "aether_bn_fwd_eval: workspace too small");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     float* coeff = static_cast<float*>(ws);
-    bn_eval_coeff_kernel<<<ceil_div(C, 128), 128, 0, st>>>(C, gamma, beta, eps, running_mean, running_var, coeff);
+    launch(bn_eval_coeff_kernel, ceil_div(C, 128), 128, 0, st, C, gamma, beta, eps, running_mean, running_var, coeff);
     const long long n = rows * C;
-    affine_channels_kernel<<<blocks_for(n / 4 + 1, 256), 256, 0, st>>>(x, y, coeff, coeff + C, n, C, -1.f);
+    launch(affine_channels_kernel, blocks_for(n / 4 + 1, 256), 256, 0, st, x, y, coeff, coeff + C, n, C, -1.f);
     count_launch(2);
     return check_launch("aether_bn_fwd_eval");
 }
@@ -627,10 +634,10 @@ extern "C" int aether_bn_bwd(const float* x, const float* dy, const float* gamma
     float* part = static_cast<float*>(ws);
     float* coeff = part + (size_t)nb * 3 * C;
     launch_bn_reduce<1>(nb, st, x, dy, batch_mean, batch_var, eps, rows, C, part);
-    bn_finalize_bwd_kernel<<<ceil_div(C, FIN_CH), FIN_THREADS, 0, st>>>(part, nb, C, rows, gamma, batch_mean, batch_var, eps, dgamma,
-                                                            dbeta, coeff, nullptr);
+    launch(bn_finalize_bwd_kernel, ceil_div(C, FIN_CH), FIN_THREADS, 0, st, part, nb, C, rows, gamma, batch_mean, batch_var, eps, dgamma,
+           dbeta, coeff, nullptr);
     const long long n = rows * C;
-    bn_bwd_apply_kernel<<<blocks_for(n / 4 + 1, 256), 256, 0, st>>>(x, dy, dx, coeff, n, C, nullptr, nullptr, nullptr, nullptr, eps, 0.f);
+    launch(bn_bwd_apply_kernel, blocks_for(n / 4 + 1, 256), 256, 0, st, x, dy, dx, coeff, n, C, nullptr, nullptr, nullptr, nullptr, eps, 0.f);
     count_launch(3);
     return check_launch("aether_bn_bwd");
 }
@@ -669,16 +676,16 @@ extern "C" int aether_bn_act_fwd_train(const float* x, const float* partials, in
     } else {
         nb = (int)nblocks;
     }
-    bn_finalize_fwd_kernel<<<ceil_div(C, FIN_CH), FIN_THREADS, 0, st>>>(src, nb, C, gamma, beta, eps, momentum, running_mean, running_var,
-                                                            batch_mean, batch_var, coeff);
+    launch(bn_finalize_fwd_kernel, ceil_div(C, FIN_CH), FIN_THREADS, 0, st, src, nb, C, gamma, beta, eps, momentum, running_mean,
+           running_var, batch_mean, batch_var, coeff);
     if (channel_scale) {
         // act(v) * m = act(m * v) for m >= 0 (ReLU and Leaky_ReLU are positively homogeneous): a spatial-dropout
         // mask behind the activation is folded into the affine coefficients, at no cost per element
-        coeff_scale_kernel<<<ceil_div(C, 128), 128, 0, st>>>(coeff, channel_scale, C);
+        launch(coeff_scale_kernel, ceil_div(C, 128), 128, 0, st, coeff, channel_scale, C);
         count_launch();
     }
     const long long n = rows * C;
-    affine_channels_kernel<<<blocks_for(n / 4 + 1, 256), 256, 0, st>>>(x, y, coeff, coeff + C, n, C, alpha);
+    launch(affine_channels_kernel, blocks_for(n / 4 + 1, 256), 256, 0, st, x, y, coeff, coeff + C, n, C, alpha);
     count_launch(2);
     return check_launch("aether_bn_act_fwd_train");
 }
@@ -693,9 +700,9 @@ extern "C" int aether_bn_act_fwd_eval(const float* x, const float* gamma, const 
     if (ws_bytes < 2 * (size_t)C * sizeof(float)) return set_error(AE_BAD_ARG, "aether_bn_act_fwd_eval: workspace too small");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     float* coeff = static_cast<float*>(ws);
-    bn_eval_coeff_kernel<<<ceil_div(C, 128), 128, 0, st>>>(C, gamma, beta, eps, running_mean, running_var, coeff);
+    launch(bn_eval_coeff_kernel, ceil_div(C, 128), 128, 0, st, C, gamma, beta, eps, running_mean, running_var, coeff);
     const long long n = rows * C;
-    affine_channels_kernel<<<blocks_for(n / 4 + 1, 256), 256, 0, st>>>(x, y, coeff, coeff + C, n, C, alpha);
+    launch(affine_channels_kernel, blocks_for(n / 4 + 1, 256), 256, 0, st, x, y, coeff, coeff + C, n, C, alpha);
     count_launch(2);
     return check_launch("aether_bn_act_fwd_eval");
 }
@@ -714,13 +721,13 @@ extern "C" int aether_bn_act_bwd(const float* x, const float* beta, const float*
     float* part = static_cast<float*>(ws);
     float* coeff = part + (size_t)nb * 3 * C;
     launch_bn_reduce<1>(nb, st, x, dy, batch_mean, batch_var, eps, rows, C, part, gamma, beta, alpha);
-    bn_finalize_bwd_kernel<<<ceil_div(C, FIN_CH), FIN_THREADS, 0, st>>>(part, nb, C, rows, gamma, batch_mean, batch_var, eps, dgamma,
-                                                            dbeta, coeff, channel_scale);
+    launch(bn_finalize_bwd_kernel, ceil_div(C, FIN_CH), FIN_THREADS, 0, st, part, nb, C, rows, gamma, batch_mean, batch_var, eps, dgamma,
+           dbeta, coeff, channel_scale);
     const long long n = rows * C;
     // the four per-channel vectors are read as float4 when C % 4 == 0
     if ((C & 3) == 0 && (!aligned16(gamma) || !aligned16(beta) || !aligned16(batch_mean) || !aligned16(batch_var)))
         return set_error(AE_BAD_ARG, "aether_bn_act_bwd: gamma, beta, batch_mean and batch_var must be 16-byte aligned");
-    bn_bwd_apply_kernel<<<blocks_for(n / 4 + 1, 256), 256, 0, st>>>(x, dy, dx, coeff, n, C, gamma, beta, batch_mean, batch_var, eps, alpha);
+    launch(bn_bwd_apply_kernel, blocks_for(n / 4 + 1, 256), 256, 0, st, x, dy, dx, coeff, n, C, gamma, beta, batch_mean, batch_var, eps, alpha);
     count_launch(3);
     return check_launch("aether_bn_act_bwd");
 }
@@ -737,6 +744,7 @@ template <bool MAX, typename I, int F>
 __global__ void __launch_bounds__(256) pool_fwd_kernel(const float* __restrict__ x, float* __restrict__ y,
                                                        uint8_t* __restrict__ arg, int S, int H, int W, int C, int fH_,
                                                        int fW_, int sH, int sW, int Ho, int Wo, int vec) {
+    pdl_wait();
     const int fH = F ? F : fH_, fW = F ? F : fW_;
     const int Cv = C / vec;
     const I total = (I)(1LL * S * Ho * Wo * Cv);
@@ -808,6 +816,7 @@ template <bool MAX>
 __global__ void __launch_bounds__(256) pool_bwd_tiled_kernel(const float* __restrict__ dy, const uint8_t* __restrict__ arg,
                                                              float* __restrict__ dx, unsigned total, int W, int C4,
                                                              int fH, int fW, int Ho, int Wo) {
+    pdl_wait();
     const float inv = 1.f / (float)(fH * fW);
     for (unsigned idx = blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += gridDim.x * blockDim.x) {
         const unsigned cv = idx % (unsigned)C4;
@@ -840,6 +849,7 @@ template <bool MAX, int VEC, typename I>
 __global__ void __launch_bounds__(256) pool_bwd_kernel(const float* __restrict__ dy, const uint8_t* __restrict__ arg,
                                                        float* __restrict__ dx, int S, int H, int W, int C, int fH,
                                                        int fW, int sH, int sW, int Ho, int Wo) {
+    pdl_wait();
     const int Cv = C / VEC;
     const I total = (I)(1LL * S * H * W * Cv);
     const float inv = 1.f / (float)(fH * fW);
@@ -891,6 +901,7 @@ __global__ void __launch_bounds__(256) pool_bwd_kernel(const float* __restrict__
 // y = x > 0 ? x : alpha * x   (alpha = 0 gives ReLU)
 __global__ void __launch_bounds__(256) lrelu_fwd_kernel(const float* __restrict__ x, float* __restrict__ y, long long n,
                                                         float alpha) {
+    pdl_wait();
     const long long stride = (long long)gridDim.x * blockDim.x;
     const long long n4 = n >> 2;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n4; i += stride) {
@@ -907,6 +918,7 @@ __global__ void __launch_bounds__(256) lrelu_fwd_kernel(const float* __restrict_
 // dx = x < 0 ? alpha * dy : dy   (the gradient passes where x == 0, as in the reference)
 __global__ void __launch_bounds__(256) lrelu_bwd_kernel(const float* __restrict__ x, const float* __restrict__ dy,
                                                         float* __restrict__ dx, long long n, float alpha) {
+    pdl_wait();
     const long long stride = (long long)gridDim.x * blockDim.x;
     const long long n4 = n >> 2;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n4; i += stride) {
@@ -940,6 +952,7 @@ __global__ void __launch_bounds__(256) dropout_fwd_kernel(const float* __restric
                                                           float* __restrict__ mask, long long n, float keep,
                                                           unsigned long long seed, unsigned long long offset,
                                                           const long long* __restrict__ calls_dev) {
+    pdl_wait();
     const long long stride = (long long)gridDim.x * blockDim.x;
     const float scale = 1.f / keep;
     // a call counter kept in device memory (replayed CUDA graphs cannot change kernel arguments) selects the stream
@@ -964,6 +977,7 @@ __global__ void __launch_bounds__(256) dropout_fwd_kernel(const float* __restric
 // Channel mask of Layer_Dropout_Spatial drawn on the device: mask[c] = Bernoulli(keep) / keep, one Philox stream per call.
 __global__ void channel_mask_kernel(float* __restrict__ mask, int C, float keep, unsigned long long seed,
                                     const long long* __restrict__ calls_dev) {
+    pdl_wait();
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= C) return;
     const unsigned long long ctr = (unsigned long long)c + (((unsigned long long)*calls_dev) << 40);
@@ -974,6 +988,7 @@ __global__ void channel_mask_kernel(float* __restrict__ mask, int C, float keep,
 }
 __global__ void __launch_bounds__(256) mul_kernel(const float* __restrict__ a, const float* __restrict__ b,
                                                   float* __restrict__ y, long long n) {
+    pdl_wait();
     const long long stride = (long long)gridDim.x * blockDim.x;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += stride) y[i] = a[i] * b[i];
 }
@@ -1013,6 +1028,7 @@ __device__ __forceinline__ void adam_range(const AdamScalars& a, float* __restri
 }
 __global__ void __launch_bounds__(256) adam_kernel(float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m,
                                                    float* __restrict__ v, long long n, const AdamScalars a) {
+    pdl_wait();
     adam_range(a, p, g, m, v, n, blockIdx.x * (long long)blockDim.x + threadIdx.x, (long long)gridDim.x * blockDim.x);
 }
 
@@ -1024,6 +1040,7 @@ struct AdamList {
     int count;
 };
 __global__ void __launch_bounds__(256) adam_list_kernel(const __grid_constant__ AdamList l, const AdamScalars a) {
+    pdl_wait();
     int t = 0;
     while (t + 1 < l.count && (int)blockIdx.x >= l.first_block[t + 1]) ++t;
     const int blocks = l.first_block[t + 1] - l.first_block[t];
@@ -1038,6 +1055,7 @@ __global__ void __launch_bounds__(256) adam_dev_kernel(float* __restrict__ p, co
                                                        float* __restrict__ m, float* __restrict__ v, long long n, float lr0,
                                                        float decay, float b1, float b2, float eps, float gscale,
                                                        const long long* __restrict__ iterations) {
+    pdl_wait();
     // two powers in double precision, once per block (every thread computing them cost the small networks 5 us)
     __shared__ AdamScalars a;
     if (threadIdx.x == 0) {
@@ -1055,6 +1073,7 @@ __global__ void __launch_bounds__(256) adam_dev_kernel(float* __restrict__ p, co
 // g += l1 * sign(w) + 2 * l2 * w   (Layer_Dense.backward regulariser terms, :337-351; sign(0) = +1)
 __global__ void __launch_bounds__(256) reg_grad_kernel(const float* __restrict__ w, float* __restrict__ g, long long n,
                                                        float l1, float l2) {
+    pdl_wait();
     const long long stride = (long long)gridDim.x * blockDim.x;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += stride) {
         const float wi = w[i];
@@ -1065,6 +1084,7 @@ __global__ void __launch_bounds__(256) reg_grad_kernel(const float* __restrict__
 // out[0] += l1 * sum|w| + l2 * sum w^2   (Loss.regularization_loss, :593-609); single block, fixed order.
 __global__ void __launch_bounds__(256) reg_loss_kernel(const float* __restrict__ w, long long n, float l1, float l2,
                                                        float* __restrict__ out) {
+    pdl_wait();
     __shared__ double sh[256];
     double acc = 0.0;
     for (long long i = threadIdx.x; i < n; i += blockDim.x) {
@@ -1088,6 +1108,7 @@ __global__ void __launch_bounds__(256) softmax_cce_kernel(const float* __restric
                                                           float* __restrict__ dz, int* __restrict__ correct, int rows,
                                                           int classes, float smooth_fwd, float smooth_bwd,
                                                           int input_is_prob, const float* __restrict__ targets) {
+    pdl_wait();
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (warp >= rows) return;
@@ -1151,6 +1172,7 @@ __global__ void __launch_bounds__(256) softmax_cce_kernel(const float* __restric
 // One warp per sample, the dot product reduced with shuffles in a fixed order.
 __global__ void __launch_bounds__(256) softmax_bwd_kernel(const float* __restrict__ p, const float* __restrict__ dv,
                                                           float* __restrict__ dx, int rows, int classes) {
+    pdl_wait();
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (warp >= rows) return;
@@ -1167,7 +1189,7 @@ __global__ void __launch_bounds__(256) softmax_bwd_kernel(const float* __restric
 // ====================================================================================== C ABI
 extern "C" int aether_softmax_bwd(const float* p, const float* dvalues, float* dinputs, int rows, int classes, void* stream) {
     if (!p || !dvalues || !dinputs || rows <= 0 || classes <= 0) return set_error(AE_BAD_ARG, "aether_softmax_bwd: bad argument");
-    softmax_bwd_kernel<<<ceil_div(rows * 32, 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(p, dvalues, dinputs, rows, classes);
+    launch(softmax_bwd_kernel, ceil_div(rows * 32, 256), 256, 0, static_cast<cudaStream_t>(stream), p, dvalues, dinputs, rows, classes);
     count_launch();
     return check_launch("aether_softmax_bwd");
 }
@@ -1187,8 +1209,8 @@ extern "C" int aether_pool_fwd(const float* x, float* y, uint8_t* argmax, int S,
     const bool two = vec == 4 && fH == 2 && fW == 2;
 #define AETHER_POOL_FWD(MAXK, I, ARG)                                                                                  \
     do {                                                                                                               \
-        if (two) pool_fwd_kernel<MAXK, I, 2><<<nb, 256, 0, st>>>(x, y, ARG, S, H, W, C, fH, fW, sH, sW, Ho, Wo, vec);  \
-        else pool_fwd_kernel<MAXK, I, 0><<<nb, 256, 0, st>>>(x, y, ARG, S, H, W, C, fH, fW, sH, sW, Ho, Wo, vec);      \
+        if (two) launch(pool_fwd_kernel<MAXK, I, 2>, nb, 256, 0, st, x, y, ARG, S, H, W, C, fH, fW, sH, sW, Ho, Wo, vec);  \
+        else launch(pool_fwd_kernel<MAXK, I, 0>, nb, 256, 0, st, x, y, ARG, S, H, W, C, fH, fW, sH, sW, Ho, Wo, vec);      \
     } while (0)
     if (kind == AETHER_POOL_MAX) {
         if (small) AETHER_POOL_FWD(true, unsigned, argmax);
@@ -1217,14 +1239,14 @@ extern "C" int aether_pool_bwd(const float* dy, const uint8_t* argmax, float* dx
     if (vec && sH == fH && sW == fW && H == Ho * fH && W == Wo * fW && windows4 < (1LL << 32) - (1LL << 22)) {
         const int nbt = blocks_for(windows4, 256, 16);
         if (kind == AETHER_POOL_MAX)
-            pool_bwd_tiled_kernel<true><<<nbt, 256, 0, st>>>(dy, argmax, dx, (unsigned)windows4, W, C / 4, fH, fW, Ho, Wo);
+            launch(pool_bwd_tiled_kernel<true>, nbt, 256, 0, st, dy, argmax, dx, (unsigned)windows4, W, C / 4, fH, fW, Ho, Wo);
         else
-            pool_bwd_tiled_kernel<false><<<nbt, 256, 0, st>>>(dy, nullptr, dx, (unsigned)windows4, W, C / 4, fH, fW, Ho, Wo);
+            launch(pool_bwd_tiled_kernel<false>, nbt, 256, 0, st, dy, nullptr, dx, (unsigned)windows4, W, C / 4, fH, fW, Ho, Wo);
         count_launch();
         return check_launch("aether_pool_bwd");
     }
 #define AETHER_POOL_BWD(MAXK, V, I, ARG) \
-    pool_bwd_kernel<MAXK, V, I><<<nb, 256, 0, st>>>(dy, ARG, dx, S, H, W, C, fH, fW, sH, sW, Ho, Wo)
+    launch(pool_bwd_kernel<MAXK, V, I>, nb, 256, 0, st, dy, ARG, dx, S, H, W, C, fH, fW, sH, sW, Ho, Wo)
     const bool small = total < (1LL << 31);
     if (kind == AETHER_POOL_MAX) {
         if (vec && small) AETHER_POOL_BWD(true, 4, unsigned, argmax);
@@ -1245,7 +1267,7 @@ extern "C" int aether_pool_bwd(const float* dy, const uint8_t* argmax, float* dx
 extern "C" int aether_leaky_relu_fwd(const float* x, float* y, int64_t n, float alpha, void* stream) {
     if (!x || !y || n <= 0) return set_error(AE_BAD_ARG, "aether_leaky_relu_fwd: bad argument");
     if (!aligned16(x) || !aligned16(y)) return set_error(AE_BAD_ARG, "aether_leaky_relu_fwd: arrays must be 16-byte aligned");
-    lrelu_fwd_kernel<<<blocks_for(n / 4 + 1, 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(x, y, n, alpha);
+    launch(lrelu_fwd_kernel, blocks_for(n / 4 + 1, 256), 256, 0, static_cast<cudaStream_t>(stream), x, y, n, alpha);
     count_launch();
     return check_launch("aether_leaky_relu_fwd");
 }
@@ -1253,7 +1275,7 @@ extern "C" int aether_leaky_relu_fwd(const float* x, float* y, int64_t n, float 
 extern "C" int aether_leaky_relu_bwd(const float* x, const float* dy, float* dx, int64_t n, float alpha, void* stream) {
     if (!x || !dy || !dx || n <= 0) return set_error(AE_BAD_ARG, "aether_leaky_relu_bwd: bad argument");
     if (!aligned16(x) || !aligned16(dy) || !aligned16(dx)) return set_error(AE_BAD_ARG, "aether_leaky_relu_bwd: arrays must be 16-byte aligned");
-    lrelu_bwd_kernel<<<blocks_for(n / 4 + 1, 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(x, dy, dx, n, alpha);
+    launch(lrelu_bwd_kernel, blocks_for(n / 4 + 1, 256), 256, 0, static_cast<cudaStream_t>(stream), x, dy, dx, n, alpha);
     count_launch();
     return check_launch("aether_leaky_relu_bwd");
 }
@@ -1262,7 +1284,7 @@ extern "C" int aether_channel_scale(const float* x, const float* scale, float* y
     if (!x || !scale || !y || n <= 0 || C <= 0 || n % C) return set_error(AE_BAD_ARG, "aether_channel_scale: bad argument");
     if ((C & 3) == 0 && (!aligned16(x) || !aligned16(y) || !aligned16(scale)))
         return set_error(AE_BAD_ARG, "aether_channel_scale: arrays must be 16-byte aligned");
-    affine_channels_kernel<<<blocks_for(n / 4 + 1, 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(x, y, scale, nullptr, n, C, -1.f);
+    launch(affine_channels_kernel, blocks_for(n / 4 + 1, 256), 256, 0, static_cast<cudaStream_t>(stream), x, y, scale, nullptr, n, C, -1.f);
     count_launch();
     return check_launch("aether_channel_scale");
 }
@@ -1271,8 +1293,8 @@ extern "C" int aether_dropout_fwd(const float* x, float* y, float* mask, int64_t
                                   uint64_t offset, void* stream) {
     if (!x || !y || !mask || n <= 0 || !(keep_prob > 0.f) || keep_prob > 1.f)
         return set_error(AE_BAD_ARG, "aether_dropout_fwd: bad argument");
-    dropout_fwd_kernel<<<blocks_for(n / 4 + 1, 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(x, y, mask, n, keep_prob, seed, offset,
-                                                                                                  nullptr);
+    launch(dropout_fwd_kernel, blocks_for(n / 4 + 1, 256), 256, 0, static_cast<cudaStream_t>(stream), x, y, mask, n, keep_prob, seed,
+           offset, nullptr);
     count_launch();
     return check_launch("aether_dropout_fwd");
 }
@@ -1282,8 +1304,8 @@ extern "C" int aether_dropout_fwd_dev(const float* x, float* y, float* mask, int
                                       uint64_t offset, const int64_t* calls_dev, void* stream) {
     if (!x || !y || !mask || !calls_dev || n <= 0 || !(keep_prob > 0.f) || keep_prob > 1.f)
         return set_error(AE_BAD_ARG, "aether_dropout_fwd_dev: bad argument");
-    dropout_fwd_kernel<<<blocks_for(n / 4 + 1, 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-        x, y, mask, n, keep_prob, seed, offset, reinterpret_cast<const long long*>(calls_dev));
+    launch(dropout_fwd_kernel, blocks_for(n / 4 + 1, 256), 256, 0, static_cast<cudaStream_t>(stream),  x, y, mask, n, keep_prob, seed,
+           offset, reinterpret_cast<const long long*>(calls_dev));
     count_launch();
     return check_launch("aether_dropout_fwd_dev");
 }
@@ -1292,8 +1314,8 @@ extern "C" int aether_channel_mask_dev(float* mask, int C, float keep_prob, uint
                                        void* stream) {
     if (!mask || !calls_dev || C <= 0 || !(keep_prob > 0.f) || keep_prob > 1.f)
         return set_error(AE_BAD_ARG, "aether_channel_mask_dev: bad argument");
-    channel_mask_kernel<<<ceil_div(C, 128), 128, 0, static_cast<cudaStream_t>(stream)>>>(
-        mask, C, keep_prob, seed, reinterpret_cast<const long long*>(calls_dev));
+    launch(channel_mask_kernel, ceil_div(C, 128), 128, 0, static_cast<cudaStream_t>(stream),  mask, C, keep_prob, seed,
+           reinterpret_cast<const long long*>(calls_dev));
     count_launch();
     return check_launch("aether_channel_mask_dev");
 }
@@ -1304,15 +1326,15 @@ extern "C" int aether_adam_step_dev(float* p, const float* g, float* m, float* v
     if (!p || !g || !m || !v || !iterations_dev || n <= 0) return set_error(AE_BAD_ARG, "aether_adam_step_dev: bad argument");
     if (!(beta1 >= 0.f && beta1 < 1.f) || !(beta2 >= 0.f && beta2 < 1.f))
         return set_error(AE_BAD_ARG, "aether_adam_step_dev: betas must be in [0, 1)");
-    adam_dev_kernel<<<blocks_for(n / 4 + 1, 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-        p, g, m, v, n, lr0, decay, beta1, beta2, eps, grad_scale, reinterpret_cast<const long long*>(iterations_dev));
+    launch(adam_dev_kernel, blocks_for(n / 4 + 1, 256), 256, 0, static_cast<cudaStream_t>(stream),  p, g, m, v, n, lr0, decay, beta1,
+           beta2, eps, grad_scale, reinterpret_cast<const long long*>(iterations_dev));
     count_launch();
     return check_launch("aether_adam_step_dev");
 }
 
 extern "C" int aether_mul(const float* a, const float* b, float* y, int64_t n, void* stream) {
     if (!a || !b || !y || n <= 0) return set_error(AE_BAD_ARG, "aether_mul: bad argument");
-    mul_kernel<<<blocks_for(n, 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(a, b, y, n);
+    launch(mul_kernel, blocks_for(n, 256), 256, 0, static_cast<cudaStream_t>(stream), a, b, y, n);
     count_launch();
     return check_launch("aether_mul");
 }
@@ -1323,7 +1345,7 @@ extern "C" int aether_adam_step(float* p, const float* g, float* m, float* v, in
     if (!p || !g || !m || !v || n <= 0) return set_error(AE_BAD_ARG, "aether_adam_step: bad argument");
     if (!(bias_corr1 > 0.f) || !(bias_corr2 > 0.f)) return set_error(AE_BAD_ARG, "aether_adam_step: bias corrections must be > 0");
     const AdamScalars a = {lr, beta1, beta2, eps, 1.f / bias_corr1, 1.f / bias_corr2, grad_scale};
-    adam_kernel<<<blocks_for(n / 4 + 1, 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(p, g, m, v, n, a);
+    launch(adam_kernel, blocks_for(n / 4 + 1, 256), 256, 0, static_cast<cudaStream_t>(stream), p, g, m, v, n, a);
     count_launch();
     return check_launch("aether_adam_step");
 }
@@ -1344,7 +1366,7 @@ extern "C" int aether_adam_steps(const AetherAdamTensor* tensors, int count, flo
             l.t[i] = tensors[begin + i];
             l.first_block[i + 1] = l.first_block[i] + blocks_for(l.t[i].n / 4 + 1, 256);
         }
-        adam_list_kernel<<<l.first_block[l.count], 256, 0, static_cast<cudaStream_t>(stream)>>>(l, a);
+        launch(adam_list_kernel, l.first_block[l.count], 256, 0, static_cast<cudaStream_t>(stream), l, a);
         count_launch();
         if (int rc = check_launch("aether_adam_steps")) return rc;
     }
@@ -1353,14 +1375,14 @@ extern "C" int aether_adam_steps(const AetherAdamTensor* tensors, int count, flo
 
 extern "C" int aether_regularizer_grad(const float* w, float* g, int64_t n, float l1, float l2, void* stream) {
     if (!w || !g || n <= 0) return set_error(AE_BAD_ARG, "aether_regularizer_grad: bad argument");
-    reg_grad_kernel<<<blocks_for(n, 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(w, g, n, l1, l2);
+    launch(reg_grad_kernel, blocks_for(n, 256), 256, 0, static_cast<cudaStream_t>(stream), w, g, n, l1, l2);
     count_launch();
     return check_launch("aether_regularizer_grad");
 }
 
 extern "C" int aether_regularizer_loss(const float* w, int64_t n, float l1, float l2, float* out, void* stream) {
     if (!w || !out || n <= 0) return set_error(AE_BAD_ARG, "aether_regularizer_loss: bad argument");
-    reg_loss_kernel<<<1, 256, 0, static_cast<cudaStream_t>(stream)>>>(w, n, l1, l2, out);
+    launch(reg_loss_kernel, 1, 256, 0, static_cast<cudaStream_t>(stream), w, n, l1, l2, out);
     count_launch();
     return check_launch("aether_regularizer_loss");
 }
@@ -1372,7 +1394,8 @@ extern "C" int aether_softmax_cce(const float* z, const int32_t* labels, float* 
     if (!labels && (loss || dz || correct)) return set_error(AE_BAD_ARG, "aether_softmax_cce: labels required for loss/gradient");
     const int threads = 256;
     const int blocks = ceil_div(rows * 32, threads);
-    softmax_cce_kernel<<<blocks, threads, 0, static_cast<cudaStream_t>(stream)>>>(z, labels, prob, loss, dz, correct, rows, classes, smooth_fwd, smooth_bwd, input_is_prob, nullptr);
+    launch(softmax_cce_kernel, blocks, threads, 0, static_cast<cudaStream_t>(stream), z, labels, prob, loss, dz, correct, rows, classes,
+           smooth_fwd, smooth_bwd, input_is_prob, nullptr);
     count_launch();
     return check_launch("aether_softmax_cce");
 }
@@ -1383,7 +1406,8 @@ extern "C" int aether_softmax_cce_targets(const float* z, const float* targets, 
     if (!z || !targets || rows <= 0 || classes <= 0) return set_error(AE_BAD_ARG, "aether_softmax_cce_targets: bad argument");
     const int threads = 256;
     const int blocks = ceil_div(rows * 32, threads);
-    softmax_cce_kernel<<<blocks, threads, 0, static_cast<cudaStream_t>(stream)>>>(z, nullptr, prob, loss, dz, correct, rows, classes, smooth_fwd, smooth_bwd, input_is_prob, targets);
+    launch(softmax_cce_kernel, blocks, threads, 0, static_cast<cudaStream_t>(stream), z, nullptr, prob, loss, dz, correct, rows, classes,
+           smooth_fwd, smooth_bwd, input_is_prob, targets);
     count_launch();
     return check_launch("aether_softmax_cce_targets");
 }

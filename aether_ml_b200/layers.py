@@ -11,6 +11,7 @@ NumPy arrays (copied to the device).  Outputs are torch CUDA tensors.
 """
 import ctypes as C
 import os
+import weakref
 
 import numpy as np
 import torch
@@ -46,11 +47,38 @@ def to_device(a, dtype=torch.float32):
     return t if t.is_contiguous() else t.contiguous()
 
 
+class _Neighbour:
+    """An attribute that refers to another layer without keeping it alive.  The layer list of a model owns its layers;
+    with owning links between neighbours a dropped model, its workspaces and its activations stayed in device memory
+    until Python's cycle collector happened to run, and the next model paid for fresh allocations."""
+
+    def __set_name__(self, owner, name):
+        self.name, self.slot = name, "_link_" + name
+
+    def __get__(self, obj, owner=None):
+        if obj is None:
+            return self
+        try:
+            ref = obj.__dict__[self.slot]
+        except KeyError:
+            raise AttributeError(self.name) from None
+        return ref() if ref is not None else None
+
+    def __set__(self, obj, value):
+        try:
+            obj.__dict__[self.slot] = weakref.ref(value) if value is not None else None
+        except TypeError:                       # an object that takes no weak references (a caller's own class)
+            obj.__dict__[self.slot] = lambda: value
+
+
 class _Saved:
     """Pickling of a layer / loss / optimizer for ``Model.save`` (the reference pickles the whole model after
     stripping the per-step arrays, CNN_model_cupy.py:291-309): device arrays travel as NumPy arrays, everything that
     belongs to one forward/backward pass (activations, gradients, workspaces, operand-copy bookkeeping, links to the
     neighbouring layers) is left out and rebuilt empty on loading."""
+
+    prev = _Neighbour()
+    next = _Neighbour()
 
     _TRANSIENT = ("inputs", "output", "dinputs", "dweights", "dbiases", "prev", "next", "bn_partials", "binary_mask",
                   "channel_mask", "batch_mean", "batch_var", "running_mean", "running_var", "inputs_shape",
@@ -383,13 +411,14 @@ class Pooling(_Saved):
     """Drop-in for ``Pooling`` (CNN_classes_cupy.py:204-312), 'valid' padding, max or average.
     The argmax is kept as one byte per output (window-local index of the first maximum);
     ``max_indicies`` reconstructs the reference's (rows, cols) pair on demand."""
+    fused_bn = _Neighbour()
 
     def __init__(self, filter_size=(2, 2), strides=(2, 2), padding="valid", pooling_type="max"):
         self.filter_size = filter_size
         self.strides = strides
         self.padding = padding
         self.pooling_type = pooling_type
-        self.fused_bn = None            # a Batch_Norm that pools inside its own kernels (Model.finalize(fuse=True))
+        self.fused_bn = None            # (a weak link) a Batch_Norm that pools inside its own kernels (Model.finalize(fuse=True))
 
     def _restore_transient(self):
         self.fused_bn = None
