@@ -68,6 +68,8 @@ SIGNATURES = {
     "aether_bn_act_pool_fwd": (_I, [_P, _P, _I64, _P, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _F, _F, _F, _P, _I,
                                     _P, _SZ, _P]),
     "aether_bn_act_pool_bwd": (_I, [_P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _F, _F, _P, _P, _SZ, _P]),
+    "aether_chain_fwd": (_I, [_P, _P, _I64] + [_P] * 11 + [_I] * 6 + [_F, _F, _F, _P, _I, _P, _I, _P, _SZ, _P]),
+    "aether_chain_bwd": (_I, [_P] * 12 + [_I] * 6 + [_F, _F, _P, _P, _I, _P, _I, C.POINTER(C.c_int), _P, _SZ, _P]),
     "aether_bn_fwd_train_partials": (_I, [_P, _P, _I64, _P, _P, _P, _P, _P, _P, _P, _I64, _I, _F, _F, _P, _SZ, _P]),
     "aether_bn_workspace_bytes": (_SZ, [_I64, _I]),
     "aether_bn_fwd_train": (_I, [_P, _P, _P, _P, _P, _P, _P, _P, _I64, _I, _F, _F, _P, _SZ, _P]),
@@ -80,6 +82,8 @@ SIGNATURES = {
     "aether_leaky_relu_bwd": (_I, [_P, _P, _P, _I64, _F, _P]),
     "aether_channel_scale": (_I, [_P, _P, _P, _I64, _I, _P]),
     "aether_dropout_fwd": (_I, [_P, _P, _P, _I64, _F, _U64, _U64, _P]),
+    "aether_copy": (_I, [_P, _P, _I64, _P]),
+    "aether_upload": (_I, [_P, _P, _I, _P]),
     "aether_mul": (_I, [_P, _P, _P, _I64, _P]),
     "aether_adam_step": (_I, [_P, _P, _P, _P, _I64, _F, _F, _F, _F, _F, _F, _F, _P]),
     "aether_adam_steps": (_I, [_P, _I, _F, _F, _F, _F, _F, _F, _F, _P]),
@@ -89,6 +93,7 @@ SIGNATURES = {
     "aether_regularizer_grad": (_I, [_P, _P, _I64, _F, _F, _P]),
     "aether_regularizer_loss": (_I, [_P, _I64, _F, _F, _P, _P]),
     "aether_softmax_cce": (_I, [_P, _P, _P, _P, _P, _P, _I, _I, _F, _F, _I, _P]),
+    "aether_softmax_cce_i64": (_I, [_P, _P, _P, _P, _P, _P, _I, _I, _F, _F, _I, _P]),
     "aether_softmax_bwd": (_I, [_P, _P, _P, _I, _I, _P]),
     "aether_softmax_cce_targets": (_I, [_P, _P, _P, _P, _P, _P, _I, _I, _F, _F, _I, _P]),
 }

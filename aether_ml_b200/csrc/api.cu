@@ -206,7 +206,7 @@ extern "C" int aether_conv2d_fwd_ex(const AetherConvDesc* d, const float* x, con
                                     float* stats, size_t stats_bytes, void* ws, size_t ws_bytes, int flags, void* stream) {
     int rc = validate_desc(d, "aether_conv2d_fwd_ex");
     if (rc) return rc;
-    if (flags & ~AETHER_CONV_X_COPY_READY) return set_error(AE_BAD_ARG, "aether_conv2d_fwd_ex: unknown flag bits 0x%x", flags);
+    if (flags & ~(AETHER_CONV_X_COPY_READY | AETHER_CONV_W_COPY_READY)) return set_error(AE_BAD_ARG, "aether_conv2d_fwd_ex: unknown flag bits 0x%x", flags);
     if ((flags & AETHER_CONV_X_COPY_READY) && !(tc_conv_eligible(*d) && d->math_mode == AETHER_MATH_BF16))
         return set_error(AE_UNSUPPORTED, "aether_conv2d_fwd_ex: this shape / math mode reads no operand copy of x "
                                          "(aether_conv2d_operand_layout returned 0)");

@@ -284,6 +284,233 @@ __global__ void __launch_bounds__(256) bn_act_pool_bwd_apply_kernel(
     }
 }
 
+// ====================================================================================== block tail, every layer's output kept
+// The same chain for a model whose layers each keep their own output (no fusion asked for): Batch_Norm, activation,
+// optional spatial dropout, optional max pooling in one pass, writing the output of EVERY layer from registers.  Layer by
+// layer the chain reads what the layer before has just written: 4 reads and 3.3 writes of |x| forward against 1 read here,
+// 6 reads and 4 writes backward against 3 reads; bound by HBM / L2 bandwidth on large tensors, by launches on small ones
+// (five and six launches become one or two and three).
+//   forward : bn = x * scale + shift;  act = lrelu(bn);  drop = act * mask (a copy in inference);  pooled, arg
+// A thread owns one window (1x1 without pooling) and four channels; cells no window covers (H, W no multiples of the
+// window) belong to ragged windows that are not pooled.
+template <int F>
+__global__ void __launch_bounds__(256) chain_fwd_kernel(const float* __restrict__ x, const float* __restrict__ scale,
+                                                        const float* __restrict__ shift, const float* __restrict__ gamma,
+                                                        const float* __restrict__ beta, const float* __restrict__ rmean,
+                                                        const float* __restrict__ rvar, float eps, float alpha,
+                                                        const float* __restrict__ mask, float* __restrict__ bn,
+                                                        float* __restrict__ act, float* __restrict__ drop,
+                                                        float* __restrict__ pooled, uint8_t* __restrict__ arg, unsigned total, int H,
+                                                        int W, int C4, int fH_, int fW_, int Hc, int Wc,
+                                                        __nv_bfloat16* __restrict__ copy, int copy_ld) {
+    pdl_wait();
+    const int fH = F ? F : fH_, fW = F ? F : fW_;
+    const int Ho = H / fH, Wo = W / fW;
+    for (unsigned idx = blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += gridDim.x * blockDim.x) {
+        const unsigned cv = idx % (unsigned)C4;
+        unsigned pix = idx / (unsigned)C4;
+        const int wo = (int)(pix % (unsigned)Wc);
+        pix /= (unsigned)Wc;
+        const int ho = (int)(pix % (unsigned)Hc);
+        const unsigned smp = pix / (unsigned)Hc;
+        float4 s, t;
+        if (scale != nullptr) {
+            s = *reinterpret_cast<const float4*>(scale + cv * 4);
+            t = *reinterpret_cast<const float4*>(shift + cv * 4);
+        } else {                                              // inference: the coefficients of bn_eval_coeff_kernel
+            const float4 g = *reinterpret_cast<const float4*>(gamma + cv * 4), b = *reinterpret_cast<const float4*>(beta + cv * 4);
+            const float4 m = *reinterpret_cast<const float4*>(rmean + cv * 4), v = *reinterpret_cast<const float4*>(rvar + cv * 4);
+            s = make_float4(g.x / sqrtf(v.x + eps), g.y / sqrtf(v.y + eps), g.z / sqrtf(v.z + eps), g.w / sqrtf(v.w + eps));
+            t = make_float4(b.x - m.x * s.x, b.y - m.y * s.y, b.z - m.z * s.z, b.w - m.w * s.w);
+        }
+        const float4 k4 = mask != nullptr ? *reinterpret_cast<const float4*>(mask + cv * 4) : make_float4(1.f, 1.f, 1.f, 1.f);
+        const size_t first = (((size_t)smp * H + (size_t)ho * fH) * W + (size_t)wo * fW) * C4 + cv;
+        const bool whole = ho < Ho && wo < Wo;                // a ragged window covers cells outside the image, too
+        float4 pre[F ? F * F : 1];
+        if (F) {
+#pragma unroll
+            for (int k = 0; k < F * F; ++k)
+                if (whole || (ho * F + k / (F ? F : 1) < H && wo * F + k % (F ? F : 1) < W))
+                    pre[k] = reinterpret_cast<const float4*>(x)[first + ((size_t)(k / (F ? F : 1)) * W + k % (F ? F : 1)) * C4];
+        }
+        float4 best = make_float4(0.f, 0.f, 0.f, 0.f);
+        uchar4 code = make_uchar4(0, 0, 0, 0);
+#pragma unroll
+        for (int i = 0; i < fH; ++i)
+#pragma unroll
+            for (int j = 0; j < fW; ++j) {
+                if (!whole && (ho * fH + i >= H || wo * fW + j >= W)) continue;
+                const size_t cell = first + ((size_t)i * W + j) * C4;
+                const float4 v = F ? pre[F ? i * F + j : 0] : reinterpret_cast<const float4*>(x)[cell];
+                float4 o = make_float4(fmaf(v.x, s.x, t.x), fmaf(v.y, s.y, t.y), fmaf(v.z, s.z, t.z), fmaf(v.w, s.w, t.w));
+                reinterpret_cast<float4*>(bn)[cell] = o;
+                o = make_float4(lrelu(o.x, alpha), lrelu(o.y, alpha), lrelu(o.z, alpha), lrelu(o.w, alpha));
+                reinterpret_cast<float4*>(act)[cell] = o;
+                if (drop != nullptr) {
+                    if (mask != nullptr) o = make_float4(o.x * k4.x, o.y * k4.y, o.z * k4.z, o.w * k4.w);
+                    reinterpret_cast<float4*>(drop)[cell] = o;
+                }
+                const unsigned char k = (unsigned char)(i * fW + j);
+                if (k == 0) {
+                    best = o;
+                } else {                                      // first maximum in row-major window order, as Pooling
+                    if (o.x > best.x) { best.x = o.x; code.x = k; }
+                    if (o.y > best.y) { best.y = o.y; code.y = k; }
+                    if (o.z > best.z) { best.z = o.z; code.z = k; }
+                    if (o.w > best.w) { best.w = o.w; code.w = k; }
+                }
+            }
+        if (pooled != nullptr && whole) {
+            const size_t opix = ((size_t)smp * Ho + ho) * Wo + wo;
+            reinterpret_cast<float4*>(pooled)[opix * C4 + cv] = best;
+            reinterpret_cast<uchar4*>(arg)[opix * C4 + cv] = code;
+            if (copy != nullptr) store_operand_copy(copy, copy_ld, opix, (int)cv, C4, best);
+        } else if (pooled == nullptr && copy != nullptr) {
+            store_operand_copy(copy, copy_ld, first / C4, (int)cv, C4, best);
+        }
+    }
+}
+
+//   backward: the gradients of every layer's input, and Batch_Norm's sums over the activation's
+//     pool_dx = dy at the selected cell;  drop_dx = pool_dx * mask;  act_dx = drop_dx * act'(bn);  sum act_dx, sum act_dx * xhat
+// bn = x * scale + shift is recomputed (the same fma, so the same sign as the stored tensor).  Thread = (channel group,
+// window lane) over a slab of windows, partials [block][2][C] as in the other statistics passes.
+template <int F>
+__global__ void __launch_bounds__(256) chain_bwd_kernel(const float* __restrict__ x, const float* __restrict__ dy,
+                                                        const uint8_t* __restrict__ arg, const float* __restrict__ scale,
+                                                        const float* __restrict__ shift, const float* __restrict__ mean,
+                                                        const float* __restrict__ var, float eps, float alpha,
+                                                        const float* __restrict__ mask, float* __restrict__ pool_dx,
+                                                        float* __restrict__ drop_dx, float* __restrict__ act_dx,
+                                                        long long windows, long long win_per_block, int H, int W, int C, int fH_,
+                                                        int fW_, int Hc, int Wc, float* __restrict__ part) {
+    pdl_wait();
+    const int fH = F ? F : fH_, fW = F ? F : fW_;
+    const int Ho = H / fH, Wo = W / fW;
+    const long long w0 = blockIdx.x * win_per_block;
+    long long w1 = w0 + win_per_block;
+    if (w1 > windows) w1 = windows;
+    const int CV = C >> 2;
+    const int cols = CV < 256 ? CV : 256;
+    const int lanes = 256 / cols;
+    __shared__ float4 sh_a4[256], sh_b4[256];
+    for (int cbase = 0; cbase < CV; cbase += cols) {
+        const int cv = cbase + threadIdx.x % cols;
+        const int rl = threadIdx.x / cols;
+        float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
+        if (rl < lanes && cv < CV) {
+            const int c = cv * 4;
+            const float4 mu = make_float4(mean[c], mean[c + 1], mean[c + 2], mean[c + 3]);
+            const float4 inv = make_float4(rsqrtf(var[c] + eps), rsqrtf(var[c + 1] + eps), rsqrtf(var[c + 2] + eps),
+                                           rsqrtf(var[c + 3] + eps));
+            const float4 s = *reinterpret_cast<const float4*>(scale + c), t = *reinterpret_cast<const float4*>(shift + c);
+            const float4 k4 = mask != nullptr ? *reinterpret_cast<const float4*>(mask + c) : make_float4(1.f, 1.f, 1.f, 1.f);
+            for (long long wdx = w0 + rl; wdx < w1; wdx += lanes) {
+                unsigned pix = (unsigned)wdx;
+                const int wo = (int)(pix % (unsigned)Wc);
+                pix /= (unsigned)Wc;
+                const int ho = (int)(pix % (unsigned)Hc);
+                const unsigned smp = pix / (unsigned)Hc;
+                const bool whole = ho < Ho && wo < Wo;
+                const size_t first = (((size_t)smp * H + (size_t)ho * fH) * W + (size_t)wo * fW) * CV + cv;
+                float4 g = make_float4(0.f, 0.f, 0.f, 0.f);
+                uchar4 cd = make_uchar4(0, 0, 0, 0);
+                if (arg == nullptr) {
+                    g = reinterpret_cast<const float4*>(dy)[first];
+                } else if (whole) {
+                    const size_t o = (((size_t)smp * Ho + ho) * Wo + wo) * CV + cv;
+                    g = reinterpret_cast<const float4*>(dy)[o];
+                    cd = reinterpret_cast<const uchar4*>(arg)[o];
+                }
+                float4 pre[F ? F * F : 1];
+                if (F) {
+#pragma unroll
+                    for (int k = 0; k < F * F; ++k)
+                        if (whole || (ho * F + k / (F ? F : 1) < H && wo * F + k % (F ? F : 1) < W))
+                            pre[k] = reinterpret_cast<const float4*>(x)[first + ((size_t)(k / (F ? F : 1)) * W + k % (F ? F : 1)) * CV];
+                }
+#pragma unroll
+                for (int i = 0; i < fH; ++i)
+#pragma unroll
+                    for (int j = 0; j < fW; ++j) {
+                        if (!whole && (ho * fH + i >= H || wo * fW + j >= W)) continue;
+                        const size_t cell = first + ((size_t)i * W + j) * CV;
+                        const float4 v = F ? pre[F ? i * F + j : 0] : reinterpret_cast<const float4*>(x)[cell];
+                        const unsigned char k = (unsigned char)(i * fW + j);
+                        float4 d = make_float4(cd.x == k ? g.x : 0.f, cd.y == k ? g.y : 0.f, cd.z == k ? g.z : 0.f, cd.w == k ? g.w : 0.f);
+                        if (pool_dx != nullptr) reinterpret_cast<float4*>(pool_dx)[cell] = d;
+                        if (drop_dx != nullptr) {
+                            d = make_float4(d.x * k4.x, d.y * k4.y, d.z * k4.z, d.w * k4.w);
+                            reinterpret_cast<float4*>(drop_dx)[cell] = d;
+                        }
+                        d.x = fmaf(v.x, s.x, t.x) < 0.f ? alpha * d.x : d.x; d.y = fmaf(v.y, s.y, t.y) < 0.f ? alpha * d.y : d.y;
+                        d.z = fmaf(v.z, s.z, t.z) < 0.f ? alpha * d.z : d.z; d.w = fmaf(v.w, s.w, t.w) < 0.f ? alpha * d.w : d.w;
+                        reinterpret_cast<float4*>(act_dx)[cell] = d;
+                        a.x += d.x; a.y += d.y; a.z += d.z; a.w += d.w;
+                        b.x = fmaf(d.x, (v.x - mu.x) * inv.x, b.x); b.y = fmaf(d.y, (v.y - mu.y) * inv.y, b.y);
+                        b.z = fmaf(d.z, (v.z - mu.z) * inv.z, b.z); b.w = fmaf(d.w, (v.w - mu.w) * inv.w, b.w);
+                    }
+            }
+        }
+        sh_a4[threadIdx.x] = a;
+        sh_b4[threadIdx.x] = b;
+        __syncthreads();
+        if (threadIdx.x < cols && cv < CV) {
+            float* out = part + (size_t)blockIdx.x * 2 * C + cv * 4;
+            const float* pa = reinterpret_cast<const float*>(sh_a4);
+            const float* pb = reinterpret_cast<const float*>(sh_b4);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                float sa = 0.f, sb = 0.f;
+                for (int l = 0; l < lanes; ++l) {
+                    sa += pa[(l * cols + threadIdx.x) * 4 + k];
+                    sb += pb[(l * cols + threadIdx.x) * 4 + k];
+                }
+                out[k] = sa;
+                out[C + k] = sb;
+            }
+        }
+        __syncthreads();
+    }
+}
+
+// dx = k1 * g + k2 * x + k3, with the bf16 operand copy of dx and its column sums for the convolution in front
+// (C / 4 divides 256: a thread keeps its four channels).
+__global__ void __launch_bounds__(256) chain_apply_copy_kernel(const float* __restrict__ x, const float* __restrict__ g_,
+                                                               const float* __restrict__ coeff, float* __restrict__ dx, long long n4,
+                                                               int C, __nv_bfloat16* __restrict__ copy, int copy_ld,
+                                                               float* __restrict__ colsum_part) {
+    pdl_wait();
+    const int C4 = C >> 2;
+    const int cv = threadIdx.x % C4, c = cv * 4;
+    const float4 k1 = *reinterpret_cast<const float4*>(coeff + c);
+    const float4 k2 = *reinterpret_cast<const float4*>(coeff + C + c);
+    const float4 k3 = *reinterpret_cast<const float4*>(coeff + 2 * C + c);
+    float4 csum = make_float4(0.f, 0.f, 0.f, 0.f);
+    const long long stride = (long long)gridDim.x * 256;
+#pragma unroll 2
+    for (long long i = blockIdx.x * 256LL + threadIdx.x; i < n4; i += stride) {
+        const float4 v = reinterpret_cast<const float4*>(x)[i];
+        const float4 g = reinterpret_cast<const float4*>(g_)[i];
+        float4 o;
+        o.x = fmaf(k1.x, g.x, fmaf(k2.x, v.x, k3.x));
+        o.y = fmaf(k1.y, g.y, fmaf(k2.y, v.y, k3.y));
+        o.z = fmaf(k1.z, g.z, fmaf(k2.z, v.z, k3.z));
+        o.w = fmaf(k1.w, g.w, fmaf(k2.w, v.w, k3.w));
+        reinterpret_cast<float4*>(dx)[i] = o;
+        store_operand_copy(copy, copy_ld, (size_t)((unsigned long long)i / (unsigned)C4), cv, C4, o);
+        csum.x += o.x; csum.y += o.y; csum.z += o.z; csum.w += o.w;
+    }
+    __shared__ float4 red[256];
+    red[threadIdx.x] = csum;
+    __syncthreads();
+    if ((int)threadIdx.x < C4) {
+        float4 t = red[threadIdx.x];
+        for (int l = threadIdx.x + C4; l < 256; l += C4) { const float4 v = red[l]; t.x += v.x; t.y += v.y; t.z += v.z; t.w += v.w; }
+        *reinterpret_cast<float4*>(colsum_part + (size_t)blockIdx.x * C + threadIdx.x * 4) = t;
+    }
+}
+
 static int fused_blocks(long long items, int threads, int per_sm) {
     long long b = (items + threads - 1) / threads;
     const long long cap = 148LL * per_sm;
@@ -417,4 +644,91 @@ extern "C" int aether_bn_act_pool_bwd_copy(const float* x, const float* dpooled,
                dx, (unsigned)windows4, W, C, fH, fW, W / fW, copy, copy_ld, copy ? colsum_part : nullptr);
     count_launch();
     return check_launch("aether_bn_act_pool_bwd");
+}
+
+extern "C" int aether_chain_fwd(const float* x, const float* partials, int64_t nblocks, const float* gamma, const float* beta,
+                                float* running_mean, float* running_var, float* batch_mean, float* batch_var, float* bn_out,
+                                float* act_out, float* drop_out, float* pooled, uint8_t* argmax, int S, int H, int W, int C, int fH,
+                                int fW, float eps, float momentum, float alpha, const float* mask, int training, void* operand_copy,
+                                int copy_ld, void* ws, size_t ws_bytes, void* stream) {
+    if (!x || !gamma || !beta || !running_mean || !running_var || !bn_out || !act_out || (pooled && !argmax) || !ws ||
+        (training && (!batch_mean || !batch_var)) || (mask && !drop_out))
+        return set_error(AE_BAD_ARG, "aether_chain_fwd: null pointer");
+    if (S <= 0 || H <= 0 || W <= 0 || C <= 0 || fH <= 0 || fW <= 0 || (!pooled && (fH != 1 || fW != 1)))
+        return set_error(AE_BAD_ARG, "aether_chain_fwd: bad dimension");
+    if (!(alpha >= 0.f && alpha < 1.f)) return set_error(AE_BAD_ARG, "aether_chain_fwd: alpha must be in [0, 1)");
+    const long long items = 1LL * S * ceil_div(H, fH) * ceil_div(W, fW) * (C / 4);
+    if (C % 4 || fH * fW > 255 || items >= (1LL << 32) - (1LL << 22))
+        return set_error(AE_UNSUPPORTED, "aether_chain_fwd: needs C %% 4 == 0, windows of at most 255 cells, 32-bit window indices");
+    if (!aligned16(x) || !aligned16(bn_out) || !aligned16(act_out) || (drop_out && !aligned16(drop_out)) || (pooled && !aligned16(pooled)) ||
+        !aligned16(gamma) || !aligned16(beta) || !aligned16(running_mean) || !aligned16(running_var) || (mask && !aligned16(mask)) || !aligned16(ws) ||
+        (argmax && (reinterpret_cast<uintptr_t>(argmax) & 3)))
+        return set_error(AE_BAD_ARG, "aether_chain_fwd: arrays must be 16-byte aligned (argmax: 4)");
+    if (operand_copy && (copy_ld < C || copy_ld % 4 || (reinterpret_cast<uintptr_t>(operand_copy) & 7)))
+        return set_error(AE_BAD_ARG, "aether_chain_fwd: operand copy needs ld >= C, ld %% 4 == 0, 8-byte alignment");
+    const long long rows = 1LL * S * H * W;
+    if (ws_bytes < aether_bn_workspace_bytes(rows, C)) return set_error(AE_BAD_ARG, "aether_chain_fwd: workspace too small");
+    if (partials && (nblocks <= 0 || nblocks > (1 << 30))) return set_error(AE_BAD_ARG, "aether_chain_fwd: nblocks");
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    const float* coeff = nullptr;
+    if (training)
+        coeff = bn_forward_coeffs(x, partials, nblocks, gamma, beta, running_mean, running_var, batch_mean, batch_var, rows, C, eps,
+                                  momentum, nullptr, static_cast<float*>(ws), st);
+    const float* shift = coeff ? coeff + C : nullptr;
+    const int fb = fused_blocks(items, 256, 16);
+    const auto kernel = fH == 2 && fW == 2 ? chain_fwd_kernel<2> : fH == 1 && fW == 1 ? chain_fwd_kernel<1> : chain_fwd_kernel<0>;
+    launch(kernel, fb, 256, 0, st, x, coeff, shift, gamma, beta, running_mean, running_var, eps, alpha, mask, bn_out, act_out, drop_out,
+           pooled, argmax, (unsigned)items, H, W, C / 4, fH, fW, ceil_div(H, fH), ceil_div(W, fW), static_cast<__nv_bfloat16*>(operand_copy),
+           copy_ld);
+    count_launch();
+    return check_launch("aether_chain_fwd");
+}
+
+extern "C" int aether_chain_bwd(const float* x, const float* dy, const uint8_t* argmax, const float* gamma, const float* batch_mean,
+                                const float* batch_var, float* pool_dx, float* drop_dx, float* act_dx, float* dx, float* dgamma,
+                                float* dbeta, int S, int H, int W, int C, int fH, int fW, float eps, float alpha, const float* mask,
+                                void* operand_copy, int copy_ld, float* colsum_part, int colsum_rows_max, int* colsum_rows, void* ws,
+                                size_t ws_bytes, void* stream) {
+    if (!x || !dy || !gamma || !batch_mean || !batch_var || !act_dx || !dx || !dgamma || !dbeta || !ws || (argmax && !pool_dx) ||
+        (mask && !drop_dx))
+        return set_error(AE_BAD_ARG, "aether_chain_bwd: null pointer");
+    if (S <= 0 || H <= 0 || W <= 0 || C <= 0 || fH <= 0 || fW <= 0 || (!argmax && (fH != 1 || fW != 1)))
+        return set_error(AE_BAD_ARG, "aether_chain_bwd: bad dimension");
+    if (!(alpha >= 0.f && alpha < 1.f)) return set_error(AE_BAD_ARG, "aether_chain_bwd: alpha must be in [0, 1)");
+    const long long windows = 1LL * S * ceil_div(H, fH) * ceil_div(W, fW);
+    if (C % 4 || fH * fW > 255 || windows >= (1LL << 32))
+        return set_error(AE_UNSUPPORTED, "aether_chain_bwd: needs C %% 4 == 0, windows of at most 255 cells, 32-bit window indices");
+    if (!aligned16(x) || !aligned16(dy) || !aligned16(act_dx) || !aligned16(dx) || (pool_dx && !aligned16(pool_dx)) ||
+        (drop_dx && !aligned16(drop_dx)) || (mask && !aligned16(mask)) || !aligned16(ws) || (argmax && (reinterpret_cast<uintptr_t>(argmax) & 3)))
+        return set_error(AE_BAD_ARG, "aether_chain_bwd: arrays must be 16-byte aligned (argmax: 4)");
+    if (operand_copy) {
+        if (copy_ld < C || copy_ld % 4 || (reinterpret_cast<uintptr_t>(operand_copy) & 7) || !colsum_part || !colsum_rows ||
+            colsum_rows_max < 1 || !aligned16(colsum_part))
+            return set_error(AE_BAD_ARG, "aether_chain_bwd: operand copy needs ld >= C, ld %% 4 == 0, 8-byte alignment and a column-sum buffer");
+        if (C / 4 > 256 || 256 % (C / 4)) return set_error(AE_UNSUPPORTED, "aether_chain_bwd: the column sums need C / 4 to divide 256 (C = %d)", C);
+    }
+    const long long rows = 1LL * S * H * W;
+    if (ws_bytes < aether_bn_workspace_bytes(rows, C)) return set_error(AE_BAD_ARG, "aether_chain_bwd: workspace too small");
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    float* part = static_cast<float*>(ws);
+    float* coeff = part + (size_t)bn_partial_blocks(rows) * 3 * C;        // still the forward pass's scale and shift
+    int nb = bn_partial_blocks(rows);
+    if (nb > windows) nb = (int)windows;
+    const auto kernel = fH == 2 && fW == 2 ? chain_bwd_kernel<2> : fH == 1 && fW == 1 ? chain_bwd_kernel<1> : chain_bwd_kernel<0>;
+    launch(kernel, nb, 256, 0, st, x, dy, argmax, coeff, coeff + C, batch_mean, batch_var, eps, alpha, mask, pool_dx, drop_dx, act_dx, windows,
+           (windows + nb - 1) / nb, H, W, C, fH, fW, ceil_div(H, fH), ceil_div(W, fW), part);
+    count_launch();
+    bn_backward_coeffs(part, nb, C, rows, gamma, batch_mean, batch_var, eps, dgamma, dbeta, coeff, nullptr, st);
+    const long long n4 = rows * (C / 4);
+    if (operand_copy) {
+        int fb = fused_blocks(n4, 256, 8);
+        if (fb > colsum_rows_max) fb = colsum_rows_max;
+        *colsum_rows = fb;
+        launch(chain_apply_copy_kernel, fb, 256, 0, st, x, act_dx, coeff, dx, n4, C, static_cast<__nv_bfloat16*>(operand_copy), copy_ld,
+               colsum_part);
+        count_launch();
+    } else {
+        bn_backward_apply(x, act_dx, dx, coeff, rows * C, C, st);
+    }
+    return check_launch("aether_chain_bwd");
 }

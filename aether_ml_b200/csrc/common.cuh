@@ -122,6 +122,8 @@ void bn_backward_coeffs(const float* part, int nb, int C, long long rows, const 
                         const float* var, float eps, float* dgamma, float* dbeta, float* coeff, const float* pscale,
                         cudaStream_t st);
 
+void bn_backward_apply(const float* x, const float* dy, float* dx, const float* coeff, long long n, int C, cudaStream_t st);
+
 static inline void conv_out_hw(const AetherConvDesc& d, int& Ho, int& Wo) {
     Ho = (d.H + 2 * d.padH - d.fH) / d.sH + 1;
     Wo = (d.W + 2 * d.padW - d.fW) / d.sW + 1;

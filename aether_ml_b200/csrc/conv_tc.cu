@@ -717,23 +717,49 @@ __global__ void __launch_bounds__(DW_THREADS, 1) dw_conv_kernel(const __grid_con
     }
 }
 
+// out[c] = sum over blocks of part[block][C] for the eight columns of CTA `cta` (256 threads): 32 lanes per column, so
+// the serial chains are short, combined in fixed order.
+__device__ __forceinline__ void finish_columns(const float* __restrict__ part, int nblocks, int C, float* __restrict__ out, int cta,
+                                               float (*red)[8]) {
+    const int cl = threadIdx.x & 7, lane = threadIdx.x >> 3;
+    const int c = cta * 8 + cl;
+    float s = 0.f;
+    if (c < C)
+#pragma unroll 4
+        for (int b = lane; b < nblocks; b += 32) s += part[(size_t)b * C + c];
+    red[lane][cl] = s;
+    __syncthreads();
+    if (lane == 0 && c < C) {
+        float t = 0.f;
+#pragma unroll
+        for (int l = 0; l < 32; ++l) t += red[l][cl];
+        out[c] = t;
+    }
+}
+
 // dW[tap][c][d] = sum over splits of part[split][tap*cblocks + c/UC][c%UC][d]
 // Taps from tap_split on have splits2 partials instead of splits (kernels whose CTA classes differ in number).
 // A block of 256 threads handles 32 consecutive outputs with 8 lanes each: lane l adds splits l, l+8, ... and the
 // lanes are combined in fixed order through shared memory (bit-reproducible; many loads in flight per output).
+// `nred` CTAs do that; the CTAs behind them finish dB, which saves a launch of its own.
 __global__ void __launch_bounds__(256) dw_reduce_kernel(const float* __restrict__ part, float* __restrict__ dw, int splits,
                                                         int U, int UC, int ldn, int cblocks, int taps, int Cin, int Cout,
-                                                        int tap_split, int splits2) {
+                                                        int tap_split, int splits2, int nred, const float* __restrict__ dbpart,
+                                                        int db_rows, float* __restrict__ db) {
     pdl_wait();
     __shared__ float red[8][32];
     __shared__ float4 red4[8][32];
+    if ((int)blockIdx.x >= nred) {                     // the blocks behind: dB from the column sums that came with dy's copy
+        finish_columns(dbpart, db_rows, Cout, db, (int)blockIdx.x - nred, reinterpret_cast<float (*)[8]>(red));
+        return;
+    }
     const int el = threadIdx.x & 31, ln = threadIdx.x >> 5;
     const long long total = 1LL * taps * Cin * Cout;
     const size_t split_stride = (size_t)U * UC * ldn;
     if ((Cout & 3) == 0 && (ldn & 3) == 0) {           // four consecutive output channels per thread
         const int Cq = Cout >> 2;
         const long long total4 = total >> 2;
-        for (long long base = blockIdx.x * 32LL; base < total4; base += gridDim.x * 32LL) {
+        for (long long base = blockIdx.x * 32LL; base < total4; base += nred * 32LL) {
             const long long i4 = base + el;
             float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
             if (i4 < total4) {
@@ -762,7 +788,7 @@ __global__ void __launch_bounds__(256) dw_reduce_kernel(const float* __restrict_
         }
         return;
     }
-    for (long long base = blockIdx.x * 32LL; base < total; base += gridDim.x * 32LL) {
+    for (long long base = blockIdx.x * 32LL; base < total; base += nred * 32LL) {
         const long long idx = base + el;
         float acc = 0.f;
         if (idx < total) {
@@ -887,25 +913,11 @@ __global__ void __launch_bounds__(256) colsum_kernel(const float* __restrict__ s
     }
 }
 
-// out[c] = sum over blocks of part[block][C]: 32 columns x 8 row lanes per CTA, lanes combined in fixed order.
 __global__ void __launch_bounds__(256) colsum_finish_kernel(const float* __restrict__ part, int nblocks, int C,
                                                             float* __restrict__ out) {
     pdl_wait();
-    // 8 columns x 32 lanes per CTA: short serial chains, lanes combined in fixed order
     __shared__ float red[32][8];
-    const int cl = threadIdx.x & 7, lane = threadIdx.x >> 3;
-    const int c = blockIdx.x * 8 + cl;
-    float s = 0.f;
-    if (c < C)
-        for (int b = lane; b < nblocks; b += 32) s += part[(size_t)b * C + c];
-    red[lane][cl] = s;
-    __syncthreads();
-    if (lane == 0 && c < C) {
-        float t = 0.f;
-#pragma unroll
-        for (int l = 0; l < 32; ++l) t += red[l][cl];
-        out[c] = t;
-    }
+    finish_columns(part, nblocks, C, out, (int)blockIdx.x, red);
 }
 
 int colsum_finish(const float* part, int rows, int C, float* out, cudaStream_t st) {
@@ -1073,10 +1085,11 @@ static TcPlan compute_plan(const AetherConvDesc& d) {
     size_t off = 0;
     auto take = [&](size_t bytes) { size_t o = off; off = align_up(off + bytes, 1024); return o; };
     const size_t in_rows = (size_t)d.S * d.H * d.W;
-    pl.off_xsh = take(pl.tf32 ? 0 : in_rows * pl.Cin_p * 2);
-    pl.off_dysh = take(pl.tf32 ? 0 : (size_t)out_rows * pl.Cout_p * 2);
+    // the filter operands first: their place does not depend on the batch size, so they stay valid across batches
     pl.off_wf = take((size_t)pl.taps * pl.Cout_p * pl.Cin_p * pl.elt);
     pl.off_wd = take(pl.tf32 ? 0 : (size_t)pl.taps * pl.Cin_p * pl.Cout_p * pl.elt);
+    pl.off_xsh = take(pl.tf32 ? 0 : in_rows * pl.Cin_p * 2);
+    pl.off_dysh = take(pl.tf32 ? 0 : (size_t)out_rows * pl.Cout_p * 2);
     int part_splits = pl.dw_splits > pl.dw_halo_splits ? pl.dw_splits : pl.dw_halo_splits;
     if (!pl.tf32) {
         const int rs = rows_dw_max_splits(pl.Cin_p, pl.Cout_p, pl.Ho, pl.Wo, d.S, d.fH, d.fW);
@@ -1299,7 +1312,9 @@ int tc_conv_fwd(const AetherConvDesc& d, const float* x, const float* w, const f
     int rc;
     if (pl.tf32) {
         float* wf = reinterpret_cast<float*>(wsb + pl.off_wf);
-        if ((rc = launch_filter_shadows<float>(w, wf, nullptr, pl.taps, d.Cin, d.Cout, pl.Cin_p, pl.Cout_p, st))) return rc;
+        if (!(flags & AETHER_CONV_W_COPY_READY) &&
+            (rc = launch_filter_shadows<float>(w, wf, nullptr, pl.taps, d.Cin, d.Cout, pl.Cin_p, pl.Cout_p, st)))
+            return rc;
         return run_igemm(true, x, d.Cin, d.H, d.W, d.S, wf, pl.Cin_p, pl.Cout_p, pl.taps, y, d.Cout, pl.Ho, pl.Wo,
                          pl.til_out, pl.Cout_p, d.fH, d.fW, +1, -d.padH, -d.padW, b, stats, st);
     }
@@ -1312,7 +1327,9 @@ int tc_conv_fwd(const AetherConvDesc& d, const float* x, const float* w, const f
     // both filter operands (forward: transposed, dX: as stored) from one read of w; a backward call that is told
     // the weights have not changed since (x_shadow_valid bit 1) reuses the second one
     __nv_bfloat16* wd = reinterpret_cast<__nv_bfloat16*>(wsb + pl.off_wd);
-    if ((rc = launch_filter_shadows<__nv_bfloat16>(w, wf, wd, pl.taps, d.Cin, d.Cout, pl.Cin_p, pl.Cout_p, st))) return rc;
+    if (!(flags & AETHER_CONV_W_COPY_READY) &&
+        (rc = launch_filter_shadows<__nv_bfloat16>(w, wf, wd, pl.taps, d.Cin, d.Cout, pl.Cin_p, pl.Cout_p, st)))
+        return rc;
     return run_igemm(false, xsh, pl.Cin_p, d.H, d.W, d.S, wf, pl.Cin_p, pl.Cout_p, pl.taps, y, d.Cout, pl.Ho, pl.Wo,
                      pl.til_out, pl.Cout_p, d.fH, d.fW, +1, -d.padH, -d.padW, b, stats, st);
 }
@@ -1372,12 +1389,6 @@ int tc_conv_bwd(const AetherConvDesc& d, const float* x, const float* dy, const 
         x_op = xsh;
         dy_op = dysh;
     }
-    if (db) {
-        launch(colsum_finish_kernel, ceil_div(d.Cout, 8), 256, 0, st, dbpart, db_rows, d.Cout, db);
-        count_launch();
-        if ((rc = check_launch("colsum_finish_kernel"))) return rc;
-    }
-
     // ---- dX: gather over dy with the filter read as (rows = Cin, K = Cout)
     if (dx) {
         if (pl.tf32) {
@@ -1396,7 +1407,15 @@ int tc_conv_bwd(const AetherConvDesc& d, const float* x, const float* dy, const 
     }
 
     // ---- dW: split over pixel tiles, fixed-order reduction of the partials
-    bool dw_done = false;
+    bool dw_done = false, db_done = db == nullptr;
+    auto reduce_dw = [&](const float* part, int splits, int tap_split, int splits2) {
+        const int nred = dw_reduce_grid(pl.taps, d.Cin, d.Cout);
+        launch(dw_reduce_kernel, nred + (db ? ceil_div(d.Cout, 8) : 0), 256, 0, st, part, dw, splits, pl.dw_U, pl.KC, pl.Cout_p,
+               pl.dw_cblocks, pl.taps, d.Cin, d.Cout, tap_split, splits2, nred, dbpart, db_rows, db);
+        db_done = true;
+        count_launch();
+        return check_launch("dw_reduce_kernel");
+    };
     // Which dW kernel (bf16).  The kernels that reuse a shared-memory window across the taps win on wide images; on
     // 16..20-pixel rows the per-tap kernel on CTA pairs is faster (a fifth of such a window is halo).  Measured on B200,
     // 128 -> 256 channels, window kernel / pair kernel in ms: 32x32 (batch 1024) 0.518 / 0.545, 24x24 (2048) 0.556 /
@@ -1411,20 +1430,14 @@ int tc_conv_bwd(const AetherConvDesc& d, const float* x, const float* dy, const 
                               &sa, &sb, &tap_split, st, &dw_done)))
             return rc;
         if (dw_done) {
-            launch(dw_reduce_kernel, dw_reduce_grid(pl.taps, d.Cin, d.Cout), 256, 0, st, part, dw, sa, pl.dw_U, pl.KC, pl.Cout_p,
-                   pl.dw_cblocks, pl.taps, d.Cin, d.Cout, tap_split, sb);
-            count_launch();
-            if ((rc = check_launch("dw_reduce_kernel"))) return rc;
+            if ((rc = reduce_dw(part, sa, tap_split, sb))) return rc;
         }
         if (!dw_done) {
             if ((rc = run_halo_dw(x_op, pl.Cin_p, d.H, d.W, d.S, dy_op, pl.Cout_p, pl.Ho, pl.Wo, d.fH, d.fW, d.padH, d.padW,
                                   part, pl.dw_halo_splits, &splits, st, &dw_done)))
                 return rc;
             if (dw_done) {
-                launch(dw_reduce_kernel, dw_reduce_grid(pl.taps, d.Cin, d.Cout), 256, 0, st, part, dw, splits, pl.dw_U, pl.KC, pl.Cout_p,
-                       pl.dw_cblocks, pl.taps, d.Cin, d.Cout, pl.taps, splits);
-                count_launch();
-                if ((rc = check_launch("dw_reduce_kernel"))) return rc;
+                if ((rc = reduce_dw(part, splits, pl.taps, splits))) return rc;
             }
         }
     }
@@ -1456,12 +1469,10 @@ int tc_conv_bwd(const AetherConvDesc& d, const float* x, const float* dy, const 
         else rc = (pl.dw_nb == 2) ? launch_dw<false, 2, false>(p, pl.dw_splits, gy, st) : launch_dw<false, 1, false>(p, pl.dw_splits, gy, st);
         if (rc) return rc;
         if (!direct) {
-            launch(dw_reduce_kernel, dw_reduce_grid(pl.taps, d.Cin, d.Cout), 256, 0, st, p.part, dw, pl.dw_splits, pl.dw_U, pl.KC,
-                   pl.Cout_p, pl.dw_cblocks, pl.taps, d.Cin, d.Cout, pl.taps, pl.dw_splits);
-            count_launch();
-            if ((rc = check_launch("dw_reduce_kernel"))) return rc;
+            if ((rc = reduce_dw(p.part, pl.dw_splits, pl.taps, pl.dw_splits))) return rc;
         }
     }
+    if (!db_done) return colsum_finish(dbpart, db_rows, d.Cout, db, st);
     return AE_OK;
 }
 

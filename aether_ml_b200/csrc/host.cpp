@@ -15,10 +15,12 @@
 #include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAStream.h>
 #include <dlfcn.h>
+#include <string.h>
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <tuple>
+#include <type_traits>
 #include <utility>
 #include <vector>
 
@@ -136,10 +138,10 @@ struct Entry<int (*)(A...)> {
 #define ENTRY_POINTS(X)                                                                                                \
     X(aether_conv2d_fwd_ex) X(aether_conv2d_bwd_ex) X(aether_bn_fwd_train) X(aether_bn_fwd_train_partials)             \
     X(aether_bn_fwd_eval) X(aether_bn_bwd) X(aether_bn_act_fwd_train) X(aether_bn_act_fwd_eval) X(aether_bn_act_bwd)   \
-    X(aether_bn_act_pool_fwd_copy) X(aether_pool_fwd) X(aether_pool_bwd) X(aether_leaky_relu_fwd)                      \
+    X(aether_bn_act_pool_fwd_copy) X(aether_chain_fwd) X(aether_pool_fwd) X(aether_pool_bwd) X(aether_leaky_relu_fwd)                      \
     X(aether_leaky_relu_bwd) X(aether_channel_scale) X(aether_dropout_fwd) X(aether_mul) X(aether_adam_step)           \
     X(aether_adam_step_dev) X(aether_dropout_fwd_dev) X(aether_channel_mask_dev) X(aether_regularizer_grad)            \
-    X(aether_regularizer_loss) X(aether_softmax_cce) X(aether_softmax_bwd) X(aether_softmax_cce_targets)
+    X(aether_regularizer_loss) X(aether_copy) X(aether_softmax_cce) X(aether_softmax_cce_i64) X(aether_softmax_bwd) X(aether_softmax_cce_targets)
 
 #define DECLARE(name)                                                                                                  \
     void* fn_##name = nullptr;                                                                                         \
@@ -148,43 +150,58 @@ struct Entry<int (*)(A...)> {
     }
 ENTRY_POINTS(DECLARE)
 
-// The block tail's backward pass also reports how many rows of column sums it wrote: returned as a number instead of
-// through the `int* colsum_rows` argument, which the Python function does not have.
-void* fn_bwd_copy = nullptr;
-PyObject* py_bwd_copy(PyObject*, PyObject* const* args, Py_ssize_t n) {
-    HANDLE_TH_ERRORS
-    static const char* name = "aether_bn_act_pool_bwd_copy";
-    if (fn_bwd_copy == nullptr || n != 25) {
-        PyErr_Format(PyExc_TypeError, "%s takes 25 arguments (%zd given) and a bound library", name, n);
-        return nullptr;
+// Entry points that report a number through an `int*` argument (the rows of column sums a backward pass wrote): the Python
+// function does not have that argument and returns the number.
+template <typename Sig>
+struct EntryOut;
+template <typename... A>
+struct EntryOut<int (*)(A...)> {
+    using Fn = int (*)(A...);
+    using Args = std::tuple<A...>;
+    static constexpr size_t N = sizeof...(A) - 1;
+
+    template <size_t I>
+    static bool get(Args& a, PyObject* const* args, int& next, int* out) {
+        if constexpr (std::is_same_v<std::tuple_element_t<I, Args>, int*>) {
+            std::get<I>(a) = out;
+            return true;
+        } else {
+            return Arg<std::tuple_element_t<I, Args>>::from(args[next++], std::get<I>(a));
+        }
     }
-    const float *x, *dp, *gamma, *beta, *bm, *bv, *scale, *sel;
-    const uint8_t* arg;
-    float *dx, *dg, *db, *cs, eps, alpha;
-    void *copy, *ws;
-    int S, H, W, C, fH, fW, ld, rows_max, rows = 0, i = 0;
-    size_t ws_bytes;
-    auto get = [&](auto& v) { return Arg<std::decay_t<decltype(v)>>::from(args[i++], v); };
-    if (!(get(x) && get(dp) && get(arg) && get(gamma) && get(beta) && get(bm) && get(bv) && get(dx) && get(dg) && get(db) && get(S) &&
-          get(H) && get(W) && get(C) && get(fH) && get(fW) && get(eps) && get(alpha) && get(scale) && get(copy) && get(ld) && get(cs) &&
-          get(rows_max) && get(sel) && get(ws)))
-        return nullptr;
-    ws_bytes = THPVariable_Check(args[24]) ? (size_t)THPVariable_Unpack(args[24]).nbytes() : 0;
-    void* st = current_stream();
-    int rc;
-    Py_BEGIN_ALLOW_THREADS
-    rc = reinterpret_cast<decltype(&aether_bn_act_pool_bwd_copy)>(fn_bwd_copy)(x, dp, arg, gamma, beta, bm, bv, dx, dg, db, S, H, W, C, fH,
-                                                                               fW, eps, alpha, scale, copy, ld, cs, rows_max, &rows, sel,
-                                                                               ws, ws_bytes, st);
-    Py_END_ALLOW_THREADS
-    if (rc != 0) return fail(rc, name);
-    return PyLong_FromLong(rows);
-    END_HANDLE_TH_ERRORS
-}
+    template <size_t... I>
+    static PyObject* call(Fn fn, const char* name, PyObject* const* args, std::index_sequence<I...>) {
+        Args a;
+        int next = 0, out = 0, rc;
+        if (!(get<I>(a, args, next, &out) && ...)) return nullptr;
+        std::get<N>(a) = current_stream();
+        Py_BEGIN_ALLOW_THREADS
+        rc = std::apply(fn, a);
+        Py_END_ALLOW_THREADS
+        return rc != 0 ? fail(rc, name) : PyLong_FromLong(out);
+    }
+    static PyObject* run(void* fn, const char* name, PyObject* const* args, Py_ssize_t n) {
+        if (fn == nullptr || n != (Py_ssize_t)N - 1) {
+            PyErr_Format(PyExc_TypeError, "%s takes %zd arguments (%zd given) and a bound library", name, (Py_ssize_t)N - 1, n);
+            return nullptr;
+        }
+        HANDLE_TH_ERRORS
+        return call(reinterpret_cast<Fn>(fn), name, args, std::make_index_sequence<N>{});
+        END_HANDLE_TH_ERRORS
+    }
+};
+#define ENTRY_POINTS_OUT(X) X(aether_bn_act_pool_bwd_copy) X(aether_chain_bwd)
+#define DECLARE_OUT(name)                                                                                              \
+    void* fn_##name = nullptr;                                                                                         \
+    PyObject* py_##name(PyObject*, PyObject* const* args, Py_ssize_t n) {                                              \
+        return EntryOut<decltype(&name)>::run(fn_##name, #name, args, n);                                              \
+    }
+ENTRY_POINTS_OUT(DECLARE_OUT)
 
 // aether_adam_steps(arrays, lr, beta1, beta2, eps, bias_corr1, bias_corr2, grad_scale): `arrays` is a flat list of
 // (parameters, gradients, momentums, cache) per tensor.
 void* fn_adam_steps = nullptr;
+void* fn_upload = nullptr;
 PyObject* py_adam_steps(PyObject*, PyObject* const* args, Py_ssize_t n) {
     HANDLE_TH_ERRORS
     static const char* name = "aether_adam_steps";
@@ -233,8 +250,9 @@ PyObject* py_bind(PyObject*, PyObject* args) {
         return nullptr;                                                                        \
     }
     ENTRY_POINTS(RESOLVE)
-    fn_bwd_copy = dlsym(h, "aether_bn_act_pool_bwd_copy");
+    ENTRY_POINTS_OUT(RESOLVE)
     fn_adam_steps = dlsym(h, "aether_adam_steps");
+    fn_upload = dlsym(h, "aether_upload");
     g_last_error = reinterpret_cast<const char* (*)()>(dlsym(h, "aether_last_error"));
     Py_XDECREF(g_error);
     Py_INCREF(error);
@@ -289,6 +307,32 @@ PyObject* py_empty_like(PyObject*, PyObject* o) {
     return new_array(t.sizes(), t.scalar_type());
 }
 
+// upload(values, like_shape): a new array of that shape with the fp32 values of a contiguous host buffer.
+PyObject* py_upload(PyObject*, PyObject* const* args, Py_ssize_t n) {
+    if (fn_upload == nullptr || n != 2) {
+        PyErr_SetString(PyExc_TypeError, "upload takes a host array and a shape, and needs a bound library");
+        return nullptr;
+    }
+    Py_buffer b;
+    if (PyObject_GetBuffer(args[0], &b, PyBUF_C_CONTIGUOUS | PyBUF_FORMAT) != 0) return nullptr;
+    PyObject* t = nullptr;
+    if (b.format == nullptr || strcmp(b.format, "f") != 0) {
+        PyErr_SetString(PyExc_TypeError, "upload: expected fp32 values");
+    } else if ((t = py_empty<at::kFloat>(nullptr, args[1])) != nullptr) {
+        const at::Tensor& a = THPVariable_Unpack(t);
+        int rc = AETHER_E_BAD_ARG;
+        if (a.numel() == b.len / 4 && a.numel() < (1 << 30))
+            rc = reinterpret_cast<decltype(&aether_upload)>(fn_upload)(static_cast<const float*>(b.buf), a.data_ptr<float>(), (int)a.numel(),
+                                                                       current_stream());
+        if (rc != 0) {
+            Py_DECREF(t);
+            t = fail(rc, "aether_upload");
+        }
+    }
+    PyBuffer_Release(&b);
+    return t;
+}
+
 // Identity of an array's contents as far as the host can tell: address, elements, in-place changes so far, row length.
 PyObject* py_tag(PyObject*, PyObject* o) {
     if (!THPVariable_Check(o)) {
@@ -303,8 +347,9 @@ PyObject* py_tag(PyObject*, PyObject* o) {
 #define METHOD(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_##name)), METH_FASTCALL, nullptr},
 PyMethodDef methods[] = {
     ENTRY_POINTS(METHOD)
-    {"aether_bn_act_pool_bwd_copy", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_bwd_copy)), METH_FASTCALL, nullptr},
+    ENTRY_POINTS_OUT(METHOD)
     {"aether_adam_steps", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_adam_steps)), METH_FASTCALL, nullptr},
+    {"upload", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_upload)), METH_FASTCALL, "upload(host fp32 buffer, shape): a new array with those values"},
     {"device", py_device, METH_NOARGS, "index of the current device"},
     {"bind", py_bind, METH_VARARGS, "bind(path, AetherError): resolve the entry points in the library at `path`"},
     {"ready", py_ready, METH_O, "the argument when it is a contiguous fp32 CUDA tensor, else None"},

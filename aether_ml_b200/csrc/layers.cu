@@ -4,6 +4,7 @@
 // :685-736, SoftMax + categorical cross-entropy :541-680.  All arrays are fp32 with the channel
 // (last) axis contiguous; kernels use 128-bit accesses along it whenever the channel count allows.
 #include <math.h>
+#include <string.h>
 
 #include "common.cuh"
 
@@ -291,6 +292,46 @@ __global__ void bn_eval_coeff_kernel(int C, const float* __restrict__ gamma, con
     scale_shift[C + c] = beta[c] - running_mean[c] * sc;
 }
 
+// Batch_Norm with the running statistics (and the activation behind it, act_alpha >= 0) in one launch: the coefficients of
+// bn_eval_coeff_kernel, operation for operation, from the four vectors.  The grid's stride keeps a thread on its four
+// channels whenever it is a multiple of C / 4 (the host sees to that for the usual channel counts), so they are computed
+// once per thread; a launch of its own for them cost a batch of 128 as much as the pass over the data.
+__device__ __forceinline__ void eval_coeff4(const float* gamma, const float* beta, const float* rm, const float* rv, float eps, int c,
+                                            float4& s, float4& t) {
+    const float4 g = *reinterpret_cast<const float4*>(gamma + c), b = *reinterpret_cast<const float4*>(beta + c);
+    const float4 m = *reinterpret_cast<const float4*>(rm + c), v = *reinterpret_cast<const float4*>(rv + c);
+    s = make_float4(g.x / sqrtf(v.x + eps), g.y / sqrtf(v.y + eps), g.z / sqrtf(v.z + eps), g.w / sqrtf(v.w + eps));
+    t = make_float4(b.x - m.x * s.x, b.y - m.y * s.y, b.z - m.z * s.z, b.w - m.w * s.w);
+}
+__global__ void __launch_bounds__(256) bn_eval_apply_kernel(const float* __restrict__ x, float* __restrict__ y,
+                                                            const float* __restrict__ gamma, const float* __restrict__ beta,
+                                                            const float* __restrict__ rm, const float* __restrict__ rv, float eps,
+                                                            long long n4, int C4, float act_alpha) {
+    pdl_wait();
+    const long long stride = (long long)gridDim.x * blockDim.x;
+    const bool act = act_alpha >= 0.f;
+    const long long i0 = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    const int cstep = (int)(stride % C4);
+    int cq = (int)(i0 % C4);
+    float4 s, t;
+    if (i0 < n4) eval_coeff4(gamma, beta, rm, rv, eps, cq * 4, s, t);
+#pragma unroll 2
+    for (long long i = i0; i < n4; i += stride) {
+        const float4 v = reinterpret_cast<const float4*>(x)[i];
+        float4 o = make_float4(fmaf(v.x, s.x, t.x), fmaf(v.y, s.y, t.y), fmaf(v.z, s.z, t.z), fmaf(v.w, s.w, t.w));
+        if (act) {
+            o.x = o.x > 0.f ? o.x : act_alpha * o.x; o.y = o.y > 0.f ? o.y : act_alpha * o.y;
+            o.z = o.z > 0.f ? o.z : act_alpha * o.z; o.w = o.w > 0.f ? o.w : act_alpha * o.w;
+        }
+        reinterpret_cast<float4*>(y)[i] = o;
+        if (cstep != 0) {
+            cq += cstep;
+            if (cq >= C4) cq -= C4;
+            if (i + stride < n4) eval_coeff4(gamma, beta, rm, rv, eps, cq * 4, s, t);
+        }
+    }
+}
+
 // y = x * scale[c] + shift[c], optionally followed by y = y > 0 ? y : act_alpha * y (act_alpha < 0: no activation)
 __global__ void __launch_bounds__(256) affine_channels_kernel(const float* __restrict__ x, float* __restrict__ y,
                                                               const float* __restrict__ scale,
@@ -447,6 +488,20 @@ __global__ void coeff_scale_kernel(float* __restrict__ scale_shift, const float*
     scale_shift[C + c] *= m[c];
 }
 
+// Inference forward of [rows][C], C % 4 == 0 and everything 16-byte aligned; false: the caller takes the two-launch path.
+static bool launch_bn_eval(const float* x, const float* gamma, const float* beta, const float* rm, const float* rv, float* y, long long n,
+                           int C, float eps, float act_alpha, cudaStream_t st) {
+    if (C % 4 || !aligned16(x) || !aligned16(y) || !aligned16(gamma) || !aligned16(beta) || !aligned16(rm) || !aligned16(rv)) return false;
+    const int C4 = C / 4;
+    int nb = blocks_for(n / 4, 256);
+    int step = C4;                                       // CTAs whose threads together cover whole rows: C4 / gcd(C4, 256)
+    while (step % 2 == 0 && C4 / step < 256) step /= 2;
+    if (nb >= step) nb -= nb % step;
+    launch(bn_eval_apply_kernel, nb, 256, 0, st, x, y, gamma, beta, rm, rv, eps, n / 4, C4, act_alpha);
+    count_launch();
+    return true;
+}
+
 // ---- pieces of Batch_Norm shared with block_fused.cu ----------------------------------------------------------
 int bn_partial_blocks(long long rows) { return bn_blocks(rows); }
 
@@ -488,6 +543,12 @@ void bn_backward_coeffs(const float* part, int nb, int C, long long rows, const 
                         const float* var, float eps, float* dgamma, float* dbeta, float* coeff, const float* pscale,
                         cudaStream_t st) {
     launch(bn_finalize_bwd_kernel, ceil_div(C, FIN_CH), FIN_THREADS, 0, st, part, nb, C, rows, gamma, mean, var, eps, dgamma, dbeta, coeff, pscale);
+    count_launch();
+}
+
+// dx = k1 * dy + k2 * x + k3 with the coefficients of bn_backward_coeffs.
+void bn_backward_apply(const float* x, const float* dy, float* dx, const float* coeff, long long n, int C, cudaStream_t st) {
+    launch(bn_bwd_apply_kernel, blocks_for(n / 4 + 1, 256), 256, 0, st, x, dy, dx, coeff, n, C, nullptr, nullptr, nullptr, nullptr, 0.f, 0.f);
     count_launch();
 }
 
@@ -612,6 +673,7 @@ extern "C" int aether_bn_fwd_eval(const float* x, const float* gamma, const floa
     if (rows <= 0 || C <= 0) return set_error(AE_BAD_ARG, "aether_bn_fwd_eval: rows=%lld C=%d", (long long)rows, C);
     if (ws_bytes < 2 * (size_t)C * sizeof(float)) return set_error(AE_BAD_ARG, "aether_bn_fwd_eval: workspace too small");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if (launch_bn_eval(x, gamma, beta, running_mean, running_var, y, rows * C, C, eps, -1.f, st)) return check_launch("aether_bn_fwd_eval");
     float* coeff = static_cast<float*>(ws);
     launch(bn_eval_coeff_kernel, ceil_div(C, 128), 128, 0, st, C, gamma, beta, eps, running_mean, running_var, coeff);
     const long long n = rows * C;
@@ -699,6 +761,7 @@ extern "C" int aether_bn_act_fwd_eval(const float* x, const float* gamma, const 
     if (rc) return rc;
     if (ws_bytes < 2 * (size_t)C * sizeof(float)) return set_error(AE_BAD_ARG, "aether_bn_act_fwd_eval: workspace too small");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if (launch_bn_eval(x, gamma, beta, running_mean, running_var, y, rows * C, C, eps, alpha, st)) return check_launch("aether_bn_act_fwd_eval");
     float* coeff = static_cast<float*>(ws);
     launch(bn_eval_coeff_kernel, ceil_div(C, 128), 128, 0, st, C, gamma, beta, eps, running_mean, running_var, coeff);
     const long long n = rows * C;
@@ -986,6 +1049,16 @@ __global__ void channel_mask_kernel(float* __restrict__ mask, int C, float keep,
     const float u = (float)(r.x >> 8) * (1.0f / 16777216.0f);
     mask[c] = u < keep ? 1.f / keep : 0.f;
 }
+// Values that travel as kernel arguments (aether_upload).
+static constexpr int UPLOAD_FLOATS = 512;
+struct UploadValues {
+    float f[UPLOAD_FLOATS];
+};
+__global__ void __launch_bounds__(256) upload_kernel(const __grid_constant__ UploadValues v, float* __restrict__ y, int n) {
+    pdl_wait();
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) y[i] = v.f[i];
+}
 __global__ void __launch_bounds__(256) mul_kernel(const float* __restrict__ a, const float* __restrict__ b,
                                                   float* __restrict__ y, long long n) {
     pdl_wait();
@@ -1107,7 +1180,8 @@ __global__ void __launch_bounds__(256) softmax_cce_kernel(const float* __restric
                                                           float* __restrict__ prob, float* __restrict__ loss,
                                                           float* __restrict__ dz, int* __restrict__ correct, int rows,
                                                           int classes, float smooth_fwd, float smooth_bwd,
-                                                          int input_is_prob, const float* __restrict__ targets) {
+                                                          int input_is_prob, const float* __restrict__ targets,
+                                                          const long long* __restrict__ labels64) {
     pdl_wait();
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
@@ -1131,7 +1205,7 @@ __global__ void __launch_bounds__(256) softmax_cce_kernel(const float* __restric
     }
     // targets: class indices (labels) or rows of target probabilities (one-hot or soft, :625-637); for the accuracy a
     // row of targets stands for its arg-max (CNN_model_cupy.py:383-385)
-    int label = labels ? labels[warp] : -1;
+    int label = labels ? labels[warp] : labels64 ? (int)labels64[warp] : -1;
     if (targets) {
         const float* tr = targets + (size_t)warp * classes;
         float tm = -INFINITY;
@@ -1152,7 +1226,7 @@ __global__ void __launch_bounds__(256) softmax_cce_kernel(const float* __restric
     for (int k = lane; k < classes; k += 32) {
         const float pk = input_is_prob ? zr[k] : expf(zr[k] - mx) / sum;
         if (prob) prob[(size_t)warp * classes + k] = pk;
-        if (labels || targets) {
+        if (labels || labels64 || targets) {
             const float onehot = targets ? targets[(size_t)warp * classes + k] : ((k == label) ? 1.f : 0.f);
             const float tf = onehot * (1.f - smooth_fwd) + smooth_fwd / classes;
             const float tb = onehot * (1.f - smooth_bwd) + smooth_bwd / classes;
@@ -1395,7 +1469,7 @@ extern "C" int aether_softmax_cce(const float* z, const int32_t* labels, float* 
     const int threads = 256;
     const int blocks = ceil_div(rows * 32, threads);
     launch(softmax_cce_kernel, blocks, threads, 0, static_cast<cudaStream_t>(stream), z, labels, prob, loss, dz, correct, rows, classes,
-           smooth_fwd, smooth_bwd, input_is_prob, nullptr);
+           smooth_fwd, smooth_bwd, input_is_prob, nullptr, nullptr);
     count_launch();
     return check_launch("aether_softmax_cce");
 }
@@ -1407,7 +1481,34 @@ extern "C" int aether_softmax_cce_targets(const float* z, const float* targets, 
     const int threads = 256;
     const int blocks = ceil_div(rows * 32, threads);
     launch(softmax_cce_kernel, blocks, threads, 0, static_cast<cudaStream_t>(stream), z, nullptr, prob, loss, dz, correct, rows, classes,
-           smooth_fwd, smooth_bwd, input_is_prob, targets);
+           smooth_fwd, smooth_bwd, input_is_prob, targets, nullptr);
     count_launch();
     return check_launch("aether_softmax_cce_targets");
+}
+
+extern "C" int aether_softmax_cce_i64(const float* z, const int64_t* labels, float* prob, float* loss, float* dz, int32_t* correct,
+                                      int rows, int classes, float smooth_fwd, float smooth_bwd, int input_is_prob, void* stream) {
+    if (!z || !labels || rows <= 0 || classes <= 0) return set_error(AE_BAD_ARG, "aether_softmax_cce_i64: bad argument");
+    launch(softmax_cce_kernel, ceil_div(rows * 32, 256), 256, 0, static_cast<cudaStream_t>(stream), z, nullptr, prob, loss, dz, correct, rows,
+           classes, smooth_fwd, smooth_bwd, input_is_prob, nullptr, reinterpret_cast<const long long*>(labels));
+    count_launch();
+    return check_launch("aether_softmax_cce_i64");
+}
+
+extern "C" int aether_copy(const float* x, float* y, int64_t n, void* stream) {
+    if (!x || !y || n <= 0) return set_error(AE_BAD_ARG, "aether_copy: bad argument");
+    const cudaError_t e = cudaMemcpyAsync(y, x, (size_t)n * sizeof(float), cudaMemcpyDeviceToDevice, static_cast<cudaStream_t>(stream));
+    return e == cudaSuccess ? AE_OK : set_error(AE_CUDA, "aether_copy: %s", cudaGetErrorString(e));
+}
+
+extern "C" int aether_upload(const float* values, float* y, int n, void* stream) {
+    if (!values || !y || n <= 0) return set_error(AE_BAD_ARG, "aether_upload: bad argument");
+    for (int begin = 0; begin < n; begin += UPLOAD_FLOATS) {
+        UploadValues v;
+        const int m = n - begin < UPLOAD_FLOATS ? n - begin : UPLOAD_FLOATS;
+        memcpy(v.f, values + begin, (size_t)m * sizeof(float));
+        launch(upload_kernel, ceil_div(m, 256), 256, 0, static_cast<cudaStream_t>(stream), v, y + begin, m);
+        count_launch();
+    }
+    return check_launch("aether_upload");
 }

@@ -104,6 +104,13 @@ class _Saved:
         pass
 
 
+def _copied(x):
+    y = host().empty_like(x)
+    if x.numel():
+        host().aether_copy(x, y, x.numel())
+    return y
+
+
 class _Workspace:
     """Grow-only byte buffer owned by a layer and handed to the library as scratch."""
 
@@ -135,6 +142,10 @@ class _OperandCopies:
         tag = host().tag
         self.x = tag(x)
         self.w = tag(w)
+
+    def weights_valid(self, ws, w):
+        """Whether the copies of the weights that the last forward pass left describe `w` still."""
+        return self.ws_ptr is not None and ws.data_ptr() == self.ws_ptr and host().tag(w) == self.w
 
     def flags(self, ws, x, w):
         """Bit 0: the copy of x is valid; bit 1: the copies of the weights are (aether_conv2d_bwd's x_shadow_valid)."""
@@ -219,6 +230,7 @@ class Conv_Layer(_Saved):
     reference's CUDA scatter kernel produces (:4-35), returned contiguous instead of as a sliced view.
     One extra keyword, ``math_mode`` in {"bf16", "tf32", "fp32"}, selects the operand precision of
     the tensor-core kernels (default from $AETHER_MATH_MODE, else bf16)."""
+    _weights_fixed = False      # Model.predict / evaluate: the weights do not change between the batches of the call
 
     def __init__(self, input_shape, num_filters=1, filter_size=(3, 3), strides=(1, 1), padding="same",
                  math_mode=None):
@@ -336,17 +348,19 @@ class Conv_Layer(_Saved):
         H = host()
         ws = self._ws.get(p.ws_bytes)
         y = H.empty(p.y_shape)
+        w = self.filter_weights
         flags = 0
         if self._handed.x is not None:
             flags = _lib.CONV_X_COPY_READY if self._handed.x_ready(ws, x) else 0
             self._handed.x = None
         if not flags:
             _require_written(x, "Conv_Layer.forward")
+        if self._weights_fixed and p.layout is not None and self._copies.weights_valid(ws, w):
+            flags |= _lib.CONV_W_COPY_READY
         # With emit_bn_stats the kernel's epilogue also writes the per-channel partial statistics that the
         # Batch_Norm behind this layer would otherwise compute in a pass of its own over y (:467-470).
         nblk = p.stats_blocks if (training and self.emit_bn_stats) else 0
         self.bn_partials = None
-        w = self.filter_weights
         if nblk > 0:
             stats = self._stats_ws.get(nblk * 3 * self.num_filters * 4)
             H.aether_conv2d_fwd_ex(p.raw, x, w, self.biases, y, stats, self._stats_ws.size, ws, self._ws.size, flags)
@@ -549,10 +563,10 @@ class Layer_Dropout_Spatial(_Saved):
             host().aether_channel_mask_dev(self.channel_mask, Cc, self.keep_prob, self.seed, self.step_dev)
         else:
             if self.fixed_mask is not None:
-                mask = np.asarray(self.fixed_mask, dtype=np.float32).reshape(1, 1, 1, Cc)
+                mask = np.ascontiguousarray(self.fixed_mask, dtype=np.float32).reshape(1, 1, 1, Cc)
             else:
                 mask = (np.random.binomial(1, self.keep_prob, size=(1, 1, 1, Cc)) / self.keep_prob).astype(np.float32)
-            self.channel_mask = to_device(mask)
+            self.channel_mask = host().upload(mask, (1, 1, 1, Cc))
         return self.channel_mask
 
     def forward(self, inputs, training):
@@ -562,7 +576,7 @@ class Layer_Dropout_Spatial(_Saved):
             self.output = x
             return self.output
         if not training:
-            self.output = x.clone()
+            self.output = _copied(x)
             return self.output
         Cc = x.shape[-1]
         self.draw_mask(Cc)
@@ -607,7 +621,7 @@ class Layer_Dropout(_Saved):
         x = to_device(inputs)
         self.inputs = x
         if not training:
-            self.output = x.clone()
+            self.output = _copied(x)
             return self.output
         h = host()
         y = h.empty_like(x)
@@ -821,7 +835,7 @@ class Batch_Norm(_Saved):
                                                  fH, fW, self.epsilon, self.fused_alpha, getattr(self, "_fused_mask", None),
                                                  target[0] if target else None, target[1] if target else 0,
                                                  target[2] if target else None, target[3] if target else 0,
-                                                 getattr(self, "_xsel", None), ws)
+                                                 getattr(self, "_xsel", None), ws, self._ws.size)
             if target:
                 if self.lean:
                     _mark_unwritten(dx)
@@ -870,6 +884,7 @@ class Layer_Dense(_Saved):
     convolution kernels as a 1x1 convolution on a 1x1 image (x (S,n_in) is NHWC with H=W=1; weights
     (n_in,n_out) are a (1,1,Cin,Cout) filter), so they use the same tensor-core path.  Parameters are
     fp32 (the reference's are fp64 because ``randn`` is); biases keep the (1, n_out) shape."""
+    _weights_fixed = False
 
     def __init__(self, n_inputs, n_neurons, weight_regularizer_l1=0, bias_regularizer_l1=0,
                  weight_regularizer_l2=0, bias_regularizer_l2=0, math_mode=None):
@@ -939,6 +954,8 @@ class Layer_Dense(_Saved):
             self._handed.x = None
         if not flags:
             _require_written(x, "Layer_Dense.forward")
+        if self._weights_fixed and p.layout is not None and self._copies.weights_valid(ws, w):
+            flags |= _lib.CONV_W_COPY_READY
         H.aether_conv2d_fwd_ex(p.raw, x, w, self.biases, y, None, 0, ws, self._ws.size, flags)
         self.inputs = x
         self.output = y
@@ -988,6 +1005,13 @@ def _labels_i32(y_true):
     return to_device(y, torch.int32)
 
 
+def _labels(y_true):
+    """``_labels_i32`` without the conversion of 64-bit class indices that are on the device already: the kernel takes them."""
+    if isinstance(y_true, torch.Tensor) and y_true.dtype is torch.int64 and y_true.ndim == 1 and y_true.is_cuda and y_true.is_contiguous():
+        return y_true
+    return _labels_i32(y_true)
+
+
 def _softmax_cce(z, labels, want_prob, want_loss, want_dz, want_correct, smooth_fwd, smooth_bwd, input_is_prob=False):
     rows, classes = z.shape
     h = host()
@@ -999,6 +1023,8 @@ def _softmax_cce(z, labels, want_prob, want_loss, want_dz, want_correct, smooth_
         if tuple(labels.shape) != (rows, classes):
             raise ValueError(f"targets have shape {tuple(labels.shape)}, expected {(rows, classes)}")
         h.aether_softmax_cce_targets(z, labels, prob, loss, dz, correct, rows, classes, smooth_fwd, smooth_bwd, 1 if input_is_prob else 0)
+    elif labels is not None and labels.dtype is torch.int64:
+        h.aether_softmax_cce_i64(z, labels, prob, loss, dz, correct, rows, classes, smooth_fwd, smooth_bwd, 1 if input_is_prob else 0)
     else:
         h.aether_softmax_cce(z, labels, prob, loss, dz, correct, rows, classes, smooth_fwd, smooth_bwd, 1 if input_is_prob else 0)
     return prob, loss, dz, correct
@@ -1075,12 +1101,12 @@ class Loss_CategoricalCrossEntropy(Loss):
     def forward(self, y_pred, y_true, training=True):
         p = to_device(y_pred)
         smooth = self.label_smoothing if training else 0.0
-        _, loss, _, _ = _softmax_cce(p, _labels_i32(y_true), False, True, False, False, smooth, 0.0, input_is_prob=True)
+        _, loss, _, _ = _softmax_cce(p, _labels(y_true), False, True, False, False, smooth, 0.0, input_is_prob=True)
         return loss
 
     def backward(self, dvalues, y_true):
         p = to_device(dvalues)
-        _, _, dz, _ = _softmax_cce(p, _labels_i32(y_true), False, False, True, False, 0.0, self.label_smoothing,
+        _, _, dz, _ = _softmax_cce(p, _labels(y_true), False, False, True, False, 0.0, self.label_smoothing,
                                    input_is_prob=True)
         self.dinputs = dz
         return self.dinputs
@@ -1103,7 +1129,7 @@ class Activation_Softmax_Loss_CategoricalCrossEntropy:
     def backward(self, dvalues, y_true, training=True):
         p = to_device(dvalues)
         smooth = self.label_smoothing if training else 0.0
-        _, _, dz, _ = _softmax_cce(p, _labels_i32(y_true), False, False, True, False, 0.0, smooth, input_is_prob=True)
+        _, _, dz, _ = _softmax_cce(p, _labels(y_true), False, False, True, False, 0.0, smooth, input_is_prob=True)
         self.dinputs = dz
         return self.dinputs
 

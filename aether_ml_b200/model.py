@@ -16,8 +16,9 @@ import pickle
 import numpy as np
 import torch
 
-from .layers import (Activation_Softmax_Loss_CategoricalCrossEntropy, Batch_Norm, Conv_Layer, Flatten, Layer_Dropout_Spatial,
-                     Loss_CategoricalCrossEntropy, Optimizer_Adam, Pooling, ReLU, SoftMax, to_device, _labels_i32, _softmax_cce, _Saved)
+from ._lib import host
+from .layers import (Activation_Softmax_Loss_CategoricalCrossEntropy, Batch_Norm, Conv_Layer, Flatten, Layer_Dropout_Spatial, Leaky_ReLU,
+                     Loss_CategoricalCrossEntropy, Optimizer_Adam, Pooling, ReLU, SoftMax, to_device, _labels, _labels_i32, _softmax_cce, _Saved)
 
 
 class Layer_Input:
@@ -80,6 +81,152 @@ def _batches(n, batch_size):
     return [slice(k * batch_size, (k + 1) * batch_size) for k in range(steps)]
 
 
+class _Chain:
+    """A Batch_Norm and the layers right behind it -- (Leaky_)ReLU, optional Layer_Dropout_Spatial, optional max Pooling whose
+    stride is its window -- that a model with unfused layers runs in one pass each way (aether_chain_fwd / _bwd): every
+    layer keeps the inputs, outputs and gradients it would have produced by itself, written from registers instead of
+    one layer after the other.  Decided anew on each pass: anything out of the ordinary (a subclass, a patched method,
+    replaced layers, shapes the kernels do not take) runs layer by layer."""
+
+    def __init__(self, parts, conv, consumer):
+        self.parts = parts                      # (bn, act[, drop][, pool])
+        self.length = len(parts)
+        self.bn, self.act = parts[0], parts[1]
+        self.drop = next((l for l in parts if isinstance(l, Layer_Dropout_Spatial)), None)
+        self.pool = next((l for l in parts if isinstance(l, Pooling)), None)
+        self.conv = conv                        # the Conv_Layer in front: takes the bf16 copy of dx
+        self.consumer = consumer                # the layer behind: takes the bf16 copy of the last output
+        self.live = None                        # the arrays of the last training pass, while they stand
+
+    @staticmethod
+    def find(layers, i):
+        """The chain that starts at layers[i], or None."""
+        def at(k):
+            return layers[k] if k < len(layers) else None
+        bn, act = at(i), at(i + 1)
+        if type(bn) is not Batch_Norm or type(act) not in (ReLU, Leaky_ReLU):
+            return None
+        parts, k = [bn, act], i + 2
+        if type(at(k)) is Layer_Dropout_Spatial:
+            parts.append(at(k))
+            k += 1
+        pool = at(k)
+        if (type(pool) is Pooling and pool.pooling_type == "max" and pool.padding == "valid" and tuple(pool.strides) == tuple(pool.filter_size)
+                and pool.filter_size[0] * pool.filter_size[1] <= 255):
+            parts.append(pool)
+            k += 1
+        conv = layers[i - 1] if i > 0 and type(layers[i - 1]) is Conv_Layer else None
+        behind = at(k)
+        if isinstance(behind, Flatten):
+            behind = at(k + 1)
+        return _Chain(tuple(parts), conv, behind if hasattr(behind, "x_copy_target") else None)
+
+    def _intact(self, layers, i):
+        for k, part in enumerate(self.parts):
+            if i + k >= len(layers) or layers[i + k] is not part or "forward" in part.__dict__ or "backward" in part.__dict__:
+                return False
+        pool = self.pool
+        return (self.bn.fused_alpha is None and not self.act.fused_into_prev and (self.drop is None or not self.drop.fused_into_prev)
+                and (pool is None or (pool.fused_bn is None and pool.pooling_type == "max" and pool.padding == "valid"
+                                      and tuple(pool.strides) == tuple(pool.filter_size))))
+
+    def forward(self, layers, i, inputs, training):
+        """Runs the chain's layers; False when they have to run one by one."""
+        self.live = None
+        if not self._intact(layers, i):
+            return False
+        x = to_device(inputs)
+        bn, act, drop, pool = self.bn, self.act, self.drop, self.pool
+        shape = x.shape
+        Cc = shape[-1]
+        if Cc % 4 or x.ndim not in (2, 4) or (pool is not None and x.ndim != 4) or x.numel() == 0:
+            return False
+        S, H, W = (shape[0], shape[1], shape[2]) if x.ndim == 4 else (shape[0], 1, 1)
+        fH, fW = pool.filter_size if pool is not None else (1, 1)
+        alpha = act._alpha
+        if H < fH or W < fW or not 0.0 <= alpha < 1.0 or x.numel() >= 1 << 32:
+            return False
+        if bn.gamma is None:
+            bn._create(Cc)
+        h = host()
+        ws = bn._workspace(S * H * W, Cc)
+        keep = (1,) * (x.ndim - 1) + (Cc,)
+        part = mask = None
+        if training:
+            bn._bm, bn._bv = h.empty(keep), h.empty(keep)
+            part = bn.stats_from.bn_partials if bn.stats_from is not None else None
+            if part is not None and part[2] != x.data_ptr():
+                part = None
+            if drop is not None:
+                mask = drop.draw_mask(Cc)
+        bn_out, act_out = h.empty(shape), h.empty(shape)
+        last = act_out
+        drop_out = pooled = arg = None
+        if drop is not None:
+            last = drop_out = h.empty(shape)
+        if pool is not None:
+            pshape = (S, H // fH, W // fW, Cc)
+            last = pooled = h.empty(pshape)
+            arg = h.empty_u8(pshape)
+        target = self.consumer.x_copy_target(tuple(last.shape)) if self.consumer is not None else None
+        h.aether_chain_fwd(x, part[0] if part else None, part[1] if part else 0, bn.gamma, bn.beta, bn._rm, bn._rv,
+                           bn._bm if training else None, bn._bv if training else None, bn_out, act_out, drop_out, pooled, arg, S, H, W,
+                           Cc, fH, fW, bn.epsilon, bn.momentum, alpha, mask, 1 if training else 0, target[0] if target else None,
+                           target[1] if target else 0, ws, bn._ws.size)
+        if training:
+            bn._expose_statistics(keep)
+        bn.pooled_now = False
+        bn.inputs, bn.output = x, bn_out
+        act.inputs, act.output = bn_out, act_out
+        if drop is not None:
+            drop.inputs, drop.output = act_out, drop_out
+        if pool is not None:
+            pool.inputs, pool.output, pool._argmax = (act_out if drop is None else drop_out), pooled, arg
+        if target:
+            self.consumer.x_copy_written(last)
+        if training:
+            self.live = (x, bn_out, bn_out._version, ws, mask, S, H, W, Cc, fH, fW, alpha)
+        return True
+
+    def backward(self, layers, i, dvalues):
+        """Runs the chain's backward passes; False when they have to run one by one."""
+        live, self.live = self.live, None
+        bn, act, drop, pool = self.bn, self.act, self.drop, self.pool
+        if live is None or not self._intact(layers, i):
+            return False
+        x, bn_out, version, ws, mask, S, H, W, Cc, fH, fW, alpha = live
+        if (bn.inputs is not x or act.inputs is not bn_out or bn_out._version != version or bn._ws.buf is not ws or act._alpha != alpha
+                or (drop is not None and drop.channel_mask is not mask)):
+            return False
+        dy = to_device(dvalues)
+        if pool is None and dy.shape != x.shape:
+            return False
+        h = host()
+        shape = x.shape
+        pool_dx = h.empty(shape) if pool is not None else None
+        drop_dx = h.empty(shape) if drop is not None else None
+        act_dx, dx = h.empty(shape), h.empty(shape)
+        if getattr(bn, "_grad_views", None) is not None:
+            bn.dweights, bn.dbiases = bn._grad_views
+        else:
+            bn.dweights, bn.dbiases = h.empty((Cc,)), h.empty((Cc,))
+        conv = self.conv
+        target = None
+        if conv is not None and conv.output is x and Cc // 4 <= 256 and 256 % (Cc // 4) == 0:
+            target = conv.dy_copy_target()
+        rows = h.aether_chain_bwd(x, dy, pool._argmax if pool is not None else None, bn.gamma, bn._bm, bn._bv, pool_dx, drop_dx, act_dx, dx,
+                                  bn.dweights, bn.dbiases, S, H, W, Cc, fH, fW, bn.epsilon, alpha, mask, target[0] if target else None,
+                                  target[1] if target else 0, target[2] if target else None, target[3] if target else 0, ws, bn._ws.size)
+        if pool is not None:
+            pool.dinputs = pool_dx
+        if drop is not None:
+            drop.dinputs = drop_dx
+        act.dinputs, bn.dinputs = act_dx, dx
+        if target:
+            conv.dy_copy_written(dx, rows)
+        return True
+
+
 class Model:
     def __init__(self):
         self.layers = []
@@ -96,6 +243,8 @@ class Model:
         self._bucket_of_layer = {}
         self._update_stream = None # side stream on which finished buckets are updated while backward goes on
         self._updated_early = set()
+        self._chains = {}          # position of a Batch_Norm -> the _Chain that starts there
+        self._chain_ends = {}      # position of a chain's last layer -> where it starts
 
     def add(self, layer):
         self.layers.append(layer)
@@ -206,6 +355,10 @@ class Model:
                     a.lean = bool(lean)
                     if isinstance(getattr(a, "prev", None), Conv_Layer):
                         a.copy_dy_consumer = a.prev
+        self._chains = {}
+        if not fuse:
+            self._chains = {i: c for i in range(len(self.layers)) if (c := _Chain.find(self.layers, i)) is not None}
+        self._chain_ends = {i + c.length - 1: i for i, c in self._chains.items()}
         self.trainable_layers = [l for l in self.layers if hasattr(l, "weights")]
         if self.loss is not None:
             self.loss.remember_trainable_layers(self.trainable_layers)
@@ -265,9 +418,16 @@ class Model:
     # ------------------------------------------------------------------ passes
     def forward(self, X, training):
         self.input_layer.forward(X, training)
-        for layer in self.layers:
+        layers, chains, i = self.layers, self._chains, 0
+        while i < len(layers):
+            layer = layers[i]
+            chain = chains.get(i)
+            if chain is not None and chain.forward(layers, i, layer.prev.output, training):
+                i += chain.length
+                continue
             layer.forward(layer.prev.output, training)
-        return layer.output
+            i += 1
+        return layers[-1].output
 
     def backward(self, output, y):
         if self.softmax_classifier_output is not None:
@@ -278,11 +438,18 @@ class Model:
             self.loss.backward(output, y)
             upstream = self.layers
         first = self.layers[0]
-        for layer in reversed(upstream):
-            if layer is first and hasattr(layer, "_desc"):
+        i = len(upstream) - 1
+        while i >= 0:
+            layer = upstream[i]
+            start = self._chain_ends.get(i)
+            if start is not None and self._chains[start].backward(self.layers, start, layer.next.dinputs):
+                layer = upstream[start]         # the chain's only trainable layer is its Batch_Norm
+                i = start
+            elif layer is first and hasattr(layer, "_desc"):
                 layer.backward(layer.next.dinputs, need_dinputs=False)   # nobody consumes d(loss)/d(images)
             else:
                 layer.backward(layer.next.dinputs)
+            i -= 1
             b = self._bucket_of_layer.get(id(layer))
             if b is not None:                   # this layer's gradients complete a bucket: start reducing it
                 self.bucket_reducer.start(b)
@@ -493,7 +660,7 @@ class Model:
         if getattr(self, "_graph", None) is None:
             raise RuntimeError("train_step_graph called before capture_train_step")
         self._g_X.copy_(to_device(X), non_blocking=True)
-        self._g_y.copy_(_labels_i32(y), non_blocking=True)
+        self._g_y.copy_(_labels(y), non_blocking=True)
         self._graph.replay()
         if self._graph_opt is not None:
             if self.grad_hook is not None:
@@ -577,11 +744,24 @@ class Model:
         if validation_data is not None:
             self.evaluate(*validation_data, batch_size=batch_size)
 
+    def _inference(self, X, batch_size):
+        """Slices and outputs of the forward passes over X.  The weights stay as they are between the batches of one call,
+        so from the second on the tensor-core layers use the operand copies of them that the first one made."""
+        fixed = [l for l in self.layers if hasattr(l, "_weights_fixed")]
+        try:
+            for k, sl in enumerate(_batches(len(X), batch_size)):
+                if k == 1:
+                    for l in fixed:
+                        l._weights_fixed = True
+                yield sl, self.forward(X[sl], training=False)
+        finally:
+            for l in fixed:
+                l._weights_fixed = False
+
     def evaluate(self, X_val, y_val, *, batch_size=None):
         self.loss.new_pass()
         self.accuracy.new_pass()
-        for sl in _batches(len(X_val), batch_size):
-            output = self.forward(X_val[sl], training=False)
+        for sl, output in self._inference(X_val, batch_size):
             self.loss.calculate(output, y_val[sl], training=False)
             self.accuracy.calculate(self.output_layer_activation.predictions(output), y_val[sl])
         validation_loss = self.loss.calculate_accumulated()
@@ -590,7 +770,9 @@ class Model:
         return float(validation_accuracy), float(validation_loss)
 
     def predict(self, X, *, batch_size=None):
-        outs = [self.forward(X[sl], training=False).clone() for sl in _batches(len(X), batch_size)]
+        # (SoftMax writes a new array every time; an output layer of the caller's may not)
+        own = type(self.layers[-1]) is SoftMax
+        outs = [output if own else output.clone() for _, output in self._inference(X, batch_size)]
         return torch.vstack(outs)
 
     # ------------------------------------------------------------------ parameters

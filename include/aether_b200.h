@@ -121,7 +121,8 @@ int aether_conv2d_bwd(const AetherConvDesc* desc, const float* x, const float* d
  *     [S*Ho*Wo][dy_copy_ld] bf16 (padding channels zero); with the copy of dy the producer also hands in per-block
  *     column sums of dy for the bias gradient (:132), float [rows][Cout] at dy_colsum_offset, rows <= dy_colsum_rows_max.
  *   aether_conv2d_fwd_ex: aether_conv2d_fwd (stats == NULL) / aether_conv2d_fwd_bnstats (stats given) with flags:
- *     AETHER_CONV_X_COPY_READY = the copy of x is already in ws.
+ *     AETHER_CONV_X_COPY_READY = the copy of x is already in ws; AETHER_CONV_W_COPY_READY = w has not changed since the last
+ *     forward call with this ws, layer and math mode (any batch size), whose copies of the filter are used again.
  *   aether_conv2d_bwd_ex: aether_conv2d_bwd whose bit mask may also carry AETHER_CONV_DY_COPY_READY = the copy of dy
  *     and dy_colsum_rows rows of column sums are already in ws.
  * These entry points have no counterpart in the reference. */
@@ -245,6 +246,25 @@ int aether_bn_act_pool_bwd_copy(const float* x, const float* dpooled, const uint
                                 int colsum_rows_max, int* colsum_rows, const float* selected_x, void* ws, size_t ws_bytes,
                                 void* stream);
 
+/* The same chain where every layer keeps its own output (Model runs it for layers that follow each other and are not
+ * fused): one pass writes Batch_Norm's output, the activation's, the spatial dropout's (drop_out, may be NULL when there
+ * is no such layer; mask = its channel mask in training, NULL in inference where it copies) and, when `pooled` is given,
+ * those of a max Pooling with fH x fW windows of stride (fH, fW) -- H and W need not be multiples of them; without
+ * pooling fH = fW = 1.  The numbers are those of the layers by themselves.  operand_copy as in ..._fwd_copy, of the last
+ * tensor of the chain.  aether_chain_bwd: dy is the gradient of the last tensor; writes the input gradient of every layer
+ * (pool_dx, drop_dx: NULL where there is no such layer) and, with operand_copy, what ..._bwd_copy writes beside dx.  It
+ * reads the coefficients the training forward pass left in the same `ws`.  C % 4 == 0. */
+int aether_chain_fwd(const float* x, const float* partials, int64_t nblocks, const float* gamma, const float* beta,
+                     float* running_mean, float* running_var, float* batch_mean, float* batch_var, float* bn_out, float* act_out,
+                     float* drop_out, float* pooled, uint8_t* argmax, int S, int H, int W, int C, int fH, int fW, float eps,
+                     float momentum, float alpha, const float* mask, int training, void* operand_copy, int copy_ld, void* ws,
+                     size_t ws_bytes, void* stream);
+int aether_chain_bwd(const float* x, const float* dy, const uint8_t* argmax, const float* gamma, const float* batch_mean,
+                     const float* batch_var, float* pool_dx, float* drop_dx, float* act_dx, float* dx, float* dgamma, float* dbeta,
+                     int S, int H, int W, int C, int fH, int fW, float eps, float alpha, const float* mask, void* operand_copy,
+                     int copy_ld, float* colsum_part, int colsum_rows_max, int* colsum_rows, void* ws, size_t ws_bytes,
+                     void* stream);
+
 /* ---- Pooling, 'valid' padding (CNN_classes_cupy.py:204-312) ---------------------------------- */
 /* Forward :212-273.  argmax (uint8, same shape as y; max pooling only) receives i*fW+j of the first
  * maximum of each window in row-major order (:259-265). */
@@ -266,6 +286,11 @@ int aether_channel_scale(const float* x, const float* scale, float* y, int64_t n
  *      y = x * mask; the mask is stored for the backward (aether_mul(dy, mask)). */
 int aether_dropout_fwd(const float* x, float* y, float* mask, int64_t n, float keep_prob, uint64_t seed, uint64_t offset,
                        void* stream);
+/* y = x (Layer_Dropout* in inference, :372-374, :393-395). */
+int aether_copy(const float* x, float* y, int64_t n, void* stream);
+/* n floats from HOST memory to the device array y, carried as kernel arguments: a channel mask (:392-397) is a few hundred
+ * bytes, and a copy from pageable memory costs the host several times a launch.  `values` may be reused at once. */
+int aether_upload(const float* values, float* y, int n, void* stream);
 int aether_mul(const float* a, const float* b, float* y, int64_t n, void* stream);
 
 /* ---- Optimizer_Adam.update_parameters :702-734 over one flat buffer.  bias_corr = 1 - beta^(it+1);
@@ -310,6 +335,9 @@ int aether_regularizer_loss(const float* w, int64_t n, float l1, float l2, float
  *      (the reference's loss classes take the softmax OUTPUT), so the softmax itself is skipped. */
 int aether_softmax_cce(const float* z, const int32_t* labels, float* prob, float* loss, float* dz, int32_t* correct,
                        int rows, int classes, float smooth_fwd, float smooth_bwd, int input_is_prob, void* stream);
+/* The same with 64-bit class indices, the integer type index arrays usually have. */
+int aether_softmax_cce_i64(const float* z, const int64_t* labels, float* prob, float* loss, float* dz, int32_t* correct,
+                           int rows, int classes, float smooth_fwd, float smooth_bwd, int input_is_prob, void* stream);
 /* The same with rows of target probabilities, float [rows][classes], instead of class indices: one-hot rows or soft
  * targets, used as they are (after label smoothing) by the loss and its gradient (:625-637, :644-650, :672-680);
  * `correct` compares arg-maxes. */
