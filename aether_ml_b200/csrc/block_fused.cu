@@ -13,24 +13,9 @@
 #include <cuda_bf16.h>
 
 #include "common.cuh"
+#include "tail.cuh"
 
 namespace aether {
-
-// Operand copy hand-off.  The tensor these passes write (the pooled activation going forward, dx going back) is the
-// next convolution's x, respectively the previous convolution's dy, whose tensor-core kernels read a bf16 copy with
-// the channels padded to `ld`.  When the consumer's workspace is known the copy is written here, from the values
-// already in registers, instead of by a cast pass that reads the fp32 tensor again: 4 channels = 8 bytes per thread,
-// and the threads of the first channel groups also zero the padding [C, ld) of their pixel.
-__device__ __forceinline__ void store_operand_copy(__nv_bfloat16* copy, int ld, size_t pixel, int cv, int C4, float4 v) {
-    __nv_bfloat162 o[2] = {__floats2bfloat162_rn(v.x, v.y), __floats2bfloat162_rn(v.z, v.w)};
-    __nv_bfloat16* row = copy + pixel * (size_t)ld;
-    *reinterpret_cast<uint2*>(row + cv * 4) = *reinterpret_cast<uint2*>(o);
-    for (int pg = C4 + cv; pg * 4 < ld; pg += C4) *reinterpret_cast<uint2*>(row + pg * 4) = make_uint2(0u, 0u);
-}
-
-__device__ __forceinline__ float lrelu(float v, float alpha) { return v > 0.f ? v : alpha * v; }
-// derivative of the activation at pre-activation v (the reference passes the gradient at v == 0, :412-428)
-__device__ __forceinline__ float lrelu_grad(float v, float alpha) { return v < 0.f ? alpha : 1.f; }
 
 // F > 0: square F x F windows known at compile time -- the window's loads are issued together (one load in flight
 // per thread does not cover the HBM latency); F == 0: any window, cells one after the other.
@@ -566,6 +551,25 @@ extern "C" int aether_bn_act_pool_fwd_copy(const float* x, const float* partials
     if (ws_bytes < aether_bn_workspace_bytes(rows, C)) return set_error(AE_BAD_ARG, "aether_bn_act_pool_fwd: workspace too small");
     if (partials && (nblocks <= 0 || nblocks > (1 << 30))) return set_error(AE_BAD_ARG, "aether_bn_act_pool_fwd: nblocks");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if (training && bn_small(rows * C, C)) {
+        BnSmallFwd p = {};
+        p.x = x;
+        p.part = partials;
+        p.nblocks = (int)nblocks;
+        if (!partials) {
+            p.part = static_cast<float*>(ws);
+            p.nblocks = bn_reduce_partials(x, rows, C, static_cast<float*>(ws), 148, st);
+        }
+        p.gamma = gamma; p.beta = beta; p.running_mean = running_mean; p.running_var = running_var;
+        p.batch_mean = batch_mean; p.batch_var = batch_var; p.eps = eps; p.momentum = momentum; p.alpha = alpha;
+        p.mask = channel_scale;
+        p.fold = 1;
+        p.pooled = pooled; p.arg = argmax; p.xsel = selected_x; p.copy = static_cast<__nv_bfloat16*>(operand_copy); p.copy_ld = copy_ld;
+        p.H = H; p.W = W; p.C = C; p.fH = fH; p.fW = fW; p.Hc = H / fH; p.Wc = W / fW;
+        p.windows = (unsigned)(windows4 / (C / 4));
+        bn_small_forward(p, st);
+        return check_launch("aether_bn_act_pool_fwd");
+    }
     float* coeff = training ? bn_forward_coeffs(x, partials, nblocks, gamma, beta, running_mean, running_var, batch_mean,
                                                 batch_var, rows, C, eps, momentum, channel_scale, static_cast<float*>(ws), st)
                             : bn_eval_coeffs(gamma, beta, running_mean, running_var, C, eps, static_cast<float*>(ws), st);
@@ -616,8 +620,10 @@ extern "C" int aether_bn_act_pool_bwd_copy(const float* x, const float* dpooled,
     if (ws_bytes < aether_bn_workspace_bytes(rows, C)) return set_error(AE_BAD_ARG, "aether_bn_act_pool_bwd: workspace too small");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const long long windows = windows4 / (C / 4);
+    const bool small = bn_small(rows * C, C);
     int nb = bn_partial_blocks(rows);
     if (nb > windows) nb = (int)windows;
+    if (small && nb > 148) nb = 148;
     float* part = static_cast<float*>(ws);
     float* coeff = part + (size_t)bn_partial_blocks(rows) * 3 * C;
     if (selected_x) {
@@ -629,6 +635,18 @@ extern "C" int aether_bn_act_pool_bwd_copy(const float* x, const float* dpooled,
                (windows + nb - 1) / nb, W, C, fH, fW, W / fW, part);
     }
     count_launch();
+    if (small) {
+        BnSmallBwd p = {};
+        p.x = x; p.dy = dpooled; p.arg = argmax; p.part = part; p.nblocks = nb; p.gamma = gamma; p.beta = beta; p.mean = batch_mean;
+        p.var = batch_var; p.pscale = channel_scale; p.eps = eps; p.alpha = alpha; p.dgamma = dgamma; p.dbeta = dbeta; p.dx = dx;
+        p.copy = static_cast<__nv_bfloat16*>(operand_copy); p.copy_ld = copy_ld; p.colsum_part = operand_copy ? colsum_part : nullptr;
+        p.W = W; p.C = C; p.fH = fH; p.fW = fW;
+        p.windows = (unsigned)windows;
+        p.rows = rows;
+        const int sums = bn_small_backward(p, operand_copy ? colsum_rows_max : 0, st);
+        if (operand_copy) *colsum_rows = sums;
+        return check_launch("aether_bn_act_pool_bwd");
+    }
     bn_backward_coeffs(part, nb, C, rows, gamma, batch_mean, batch_var, eps, dgamma, dbeta, coeff, channel_scale, st);
     int fb = fused_blocks(windows4, 256, 16);
     __nv_bfloat16* copy = static_cast<__nv_bfloat16*>(operand_copy);
@@ -670,6 +688,25 @@ extern "C" int aether_chain_fwd(const float* x, const float* partials, int64_t n
     if (ws_bytes < aether_bn_workspace_bytes(rows, C)) return set_error(AE_BAD_ARG, "aether_chain_fwd: workspace too small");
     if (partials && (nblocks <= 0 || nblocks > (1 << 30))) return set_error(AE_BAD_ARG, "aether_chain_fwd: nblocks");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if (training && bn_small(rows * C, C)) {
+        BnSmallFwd p = {};
+        p.x = x;
+        p.part = partials;
+        p.nblocks = (int)nblocks;
+        if (!partials) {
+            p.part = static_cast<float*>(ws);
+            p.nblocks = bn_reduce_partials(x, rows, C, static_cast<float*>(ws), 148, st);
+        }
+        p.gamma = gamma; p.beta = beta; p.running_mean = running_mean; p.running_var = running_var;
+        p.batch_mean = batch_mean; p.batch_var = batch_var; p.eps = eps; p.momentum = momentum; p.alpha = alpha; p.mask = mask;
+        p.coeff = static_cast<float*>(ws) + (size_t)bn_partial_blocks(rows) * 3 * C;
+        p.bn_out = bn_out; p.act_out = act_out; p.drop_out = drop_out; p.pooled = pooled; p.arg = argmax;
+        p.copy = static_cast<__nv_bfloat16*>(operand_copy); p.copy_ld = copy_ld;
+        p.H = H; p.W = W; p.C = C; p.fH = fH; p.fW = fW; p.Hc = ceil_div(H, fH); p.Wc = ceil_div(W, fW);
+        p.windows = (unsigned)(items / (C / 4));
+        bn_small_forward(p, st);
+        return check_launch("aether_chain_fwd");
+    }
     const float* coeff = nullptr;
     if (training)
         coeff = bn_forward_coeffs(x, partials, nblocks, gamma, beta, running_mean, running_var, batch_mean, batch_var, rows, C, eps,
@@ -712,12 +749,26 @@ extern "C" int aether_chain_bwd(const float* x, const float* dy, const uint8_t* 
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     float* part = static_cast<float*>(ws);
     float* coeff = part + (size_t)bn_partial_blocks(rows) * 3 * C;        // still the forward pass's scale and shift
+    const bool small = bn_small(rows * C, C);
     int nb = bn_partial_blocks(rows);
     if (nb > windows) nb = (int)windows;
+    if (small && nb > 148 * 2) nb = 148 * 2;
     const auto kernel = fH == 2 && fW == 2 ? chain_bwd_kernel<2> : fH == 1 && fW == 1 ? chain_bwd_kernel<1> : chain_bwd_kernel<0>;
     launch(kernel, nb, 256, 0, st, x, dy, argmax, coeff, coeff + C, batch_mean, batch_var, eps, alpha, mask, pool_dx, drop_dx, act_dx, windows,
            (windows + nb - 1) / nb, H, W, C, fH, fW, ceil_div(H, fH), ceil_div(W, fW), part);
     count_launch();
+    if (small) {
+        BnSmallBwd p = {};
+        p.x = x; p.dy = act_dx; p.part = part; p.nblocks = nb; p.gamma = gamma; p.mean = batch_mean; p.var = batch_var; p.eps = eps;
+        p.alpha = -1.f; p.dgamma = dgamma; p.dbeta = dbeta; p.dx = dx; p.copy = static_cast<__nv_bfloat16*>(operand_copy); p.copy_ld = copy_ld;
+        p.colsum_part = operand_copy ? colsum_part : nullptr;
+        p.W = p.fH = p.fW = 1; p.C = C;
+        p.windows = (unsigned)rows;
+        p.rows = rows;
+        const int sums = bn_small_backward(p, operand_copy ? colsum_rows_max : 0, st);
+        if (operand_copy) *colsum_rows = sums;
+        return check_launch("aether_chain_bwd");
+    }
     bn_backward_coeffs(part, nb, C, rows, gamma, batch_mean, batch_var, eps, dgamma, dbeta, coeff, nullptr, st);
     const long long n4 = rows * (C / 4);
     if (operand_copy) {

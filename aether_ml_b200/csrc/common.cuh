@@ -113,6 +113,8 @@ int tc_conv_bwd(const AetherConvDesc& d, const float* x, const float* dy, const 
 
 // ---- layers.cu : pieces of Batch_Norm shared with block_fused.cu
 int bn_partial_blocks(long long rows);
+// (count, mean, M2) partials of x into part, in at most `most` rows; returns their number
+int bn_reduce_partials(const float* x, long long rows, int C, float* part, int most, cudaStream_t st);
 float* bn_forward_coeffs(const float* x, const float* partials, long long nblocks, const float* gamma, const float* beta,
                          float* running_mean, float* running_var, float* batch_mean, float* batch_var, long long rows,
                          int C, float eps, float momentum, const float* channel_scale, float* ws, cudaStream_t st);

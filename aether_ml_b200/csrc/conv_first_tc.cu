@@ -26,7 +26,7 @@ struct FirstParams {
     const float* w;      // (fH, fW, Cin, Cout) = [K][Cout]
     const float* bias;   // nullable
     float* y;
-    float* stats;        // nullable: [cta][4][3][Cout] (count, mean, M2) partials
+    float* stats;        // nullable: [cta][3][Cout] (count, mean, M2) partials
     int* status;
     int H, W, Cin, Cout, NT, fH, fW, sH, sW, pH, pW, Ho, Wo, K, KP;
     long long P;         // output pixels
@@ -67,7 +67,7 @@ __global__ void __launch_bounds__(FirstCfg<STATS>::THREADS, 1) first_conv_kernel
     uint8_t* gen_base = smem_raw + (smem_base - smem_u32(smem_raw));
     const int NT = p.NT, S = p.stages;
     const uint32_t sW = smem_base;                                  // filter: NT rows of 128 bytes
-    const uint32_t sA = sW + (uint32_t)NT * 128u;                   // NT is a multiple of 64: stays 1024-byte aligned
+    const uint32_t sA = sW + (uint32_t)NT * 128u;                   // NT is a multiple of 32: stays 1024-byte aligned
     const uint32_t sBar = sA + (uint32_t)S * FT_STAGE_BYTES;
     auto full_bar = [&](int s) { return sBar + 8u * s; };
     auto empty_bar = [&](int s) { return sBar + 8u * (S + s); };
@@ -365,22 +365,9 @@ __global__ void __launch_bounds__(FirstCfg<STATS>::THREADS, 1) first_conv_kernel
             if (++buf == NB) { buf = 0; aph ^= 1u; }
         }
         if (STATS && persist) flush_stats(0, false, 0.f);
-        if (STATS && lane < 4) {
-            float* sp = p.stats + ((size_t)blockIdx.x * 4 + q) * 3 * (size_t)p.Cout;
-            for (int cc = 0; cc < ncols; cc += 16) {
-#pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    const int col = col_begin + tcol4 + cc + k;
-                    if (col < p.Cout) {
-                        float m, m2;
-                        stats_result(stat_w, cc + tcol4 + k, st_rows, m, m2);
-                        sp[col] = st_rows;
-                        sp[p.Cout + col] = m + bias_s[col];
-                        sp[2 * p.Cout + col] = m2;
-                    }
-                }
-            }
-        }
+        if (STATS)
+            stats_merge_store(reinterpret_cast<float*>(gen_base + (sBar - smem_base) + FT_TAIL), ew, lane, st_rows, ncols, 0, p.Cout, bias_s,
+                              p.stats + (size_t)blockIdx.x * 3 * p.Cout);
     }
 
     tc_fence_before();
@@ -660,7 +647,7 @@ static bool first_tc_shape(const AetherConvDesc& d, int& K, int& KP, int& NT, in
     if (d.Cin > 4 || K > 64) return false;
     if (d.Cout % 4 || d.Cout < 16 || d.Cout > 256) return false;
     KP = (K + 15) / 16 * 16;
-    NT = (d.Cout + 63) / 64 * 64;              // two column halves of 16-column groups; filter rows fill whole 8-row atoms
+    NT = (d.Cout + 31) / 32 * 32;              // two column halves of 16-column groups; filter rows fill whole 8-row atoms
     conv_out_hw(d, Ho, Wo);
     if (Ho < 1 || Wo < 1) return false;
     const long long P = 1LL * d.S * Ho * Wo;
@@ -678,7 +665,7 @@ long long first_tc_stats_blocks(const AetherConvDesc& d) {
     int K, KP, NT, Ho, Wo;
     if (!first_tc_shape(d, K, KP, NT, Ho, Wo)) return 0;
     const long long P = 1LL * d.S * Ho * Wo;
-    return 4LL * first_tc_grid((P + 127) / 128);
+    return first_tc_grid((P + 127) / 128);
 }
 
 int first_tc_fwd(const AetherConvDesc& d, const float* x, const float* w, const float* b, float* y, float* stats,

@@ -13,10 +13,11 @@ namespace aether {
 // sums each and combine them with shuffles in a fixed order.
 // The filter is kept transposed in shared memory, wT[d][Cin], so a lane's four channels of output d are one 16-byte
 // shared-memory read (4 * Cout scalar global loads per four channels before).
+// (rows of Cin + 4 floats: with Cin a multiple of 32 the outputs of one channel would all fall on one bank)
 __device__ __forceinline__ void head_load_filter_T(const float* __restrict__ w, float* wT, int Cin, int Cout) {
     for (int i = threadIdx.x; i < Cin * Cout; i += blockDim.x) {
         const int c = i / Cout, d = i - c * Cout;
-        wT[d * Cin + c] = w[i];
+        wT[d * (Cin + 4) + c] = w[i];
     }
     __syncthreads();
 }
@@ -42,7 +43,7 @@ __global__ void __launch_bounds__(256) gen_fwd_pointwise_few_kernel(const float*
 #pragma unroll
             for (int d = 0; d < MAXD; ++d) {
                 if (d < Cout) {
-                    const float4 k = *reinterpret_cast<const float4*>(head_wT + d * Cin + 4 * c4);
+                    const float4 k = *reinterpret_cast<const float4*>(head_wT + d * (Cin + 4) + 4 * c4);
                     acc[d] = fmaf(v.x, k.x, fmaf(v.y, k.y, fmaf(v.z, k.z, fmaf(v.w, k.w, acc[d]))));
                 }
             }
@@ -111,21 +112,6 @@ __global__ void __launch_bounds__(256) gen_dx_fewc_kernel(const float* __restric
     }
 }
 
-// ---------------------------------------------------------------------------------- dW, dB of classifier heads: partials added in fixed order
-__global__ void gen_dw_reduce_kernel(const float* __restrict__ part, int nblocks, int entries, int Cout,
-                                     float* __restrict__ dw, float* __restrict__ db) {
-    pdl_wait();
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= entries + Cout) return;
-    float s = 0.f;
-    for (int b = 0; b < nblocks; ++b) s += part[(size_t)b * (entries + Cout) + e];
-    if (e < entries) {
-        if (dw) dw[e] = s;
-    } else if (db) {
-        db[e - entries] = s;
-    }
-}
-
 // ---------------------------------------------------------------------------------- classifier heads, backward
 // dx[p][c] = sum_d dy[p][d] * w[c][d] for a pointwise layer with few outputs: a block takes a row at a time, a thread
 // four channels; the filter is read transposed from shared memory, the row of dy is the same address for every thread.
@@ -153,7 +139,7 @@ __global__ void __launch_bounds__(256) head_dx_kernel(const float* __restrict__ 
 #pragma unroll
             for (int d = 0; d < MAXD; ++d) {
                 if (d < Cout) {
-                    const float4 k = *reinterpret_cast<const float4*>(head_wT + d * Cin + 4 * c4);
+                    const float4 k = *reinterpret_cast<const float4*>(head_wT + d * (Cin + 4) + 4 * c4);
                     a.x = fmaf(g[d], k.x, a.x); a.y = fmaf(g[d], k.y, a.y); a.z = fmaf(g[d], k.z, a.z); a.w = fmaf(g[d], k.w, a.w);
                 }
             }
@@ -162,28 +148,31 @@ __global__ void __launch_bounds__(256) head_dx_kernel(const float* __restrict__ 
     }
 }
 
-// dw[c][d] = sum_p x[p][c] * dy[p][d], db[d] = sum_p dy[p][d] over this block's rows, written as the partials
-// gen_dw_reduce_kernel adds up ([block][Cin * Cout + Cout]).  A thread keeps four channels x Cout sums; x is read once,
-// coalesced; the row of dy is the same address for every thread.  blockIdx.y walks the channels in groups of 1024.
+// dw[c][d] = sum_p x[p][c] * dy[p][d], db[d] = sum_p dy[p][d] over a part of the rows: partials [part][Cin * Cout + Cout]
+// that smallc_reduce_kernel adds up.  A thread keeps four channels x Cout sums; x is read once, coalesced; the row of dy
+// is the same address for every thread of a row.  A block is row lanes x four-channel groups (blockIdx.y walks the
+// groups beyond 256) and every row lane writes a part of its own.  Few rows per thread: the loop is a chain of load
+// latencies (4 blocks of 32 rows at batch 128 took 17 us, of which the sums themselves are a small part).
 template <int MAXD>
 __global__ void __launch_bounds__(256) head_dw_partial_kernel(const float* __restrict__ x, const float* __restrict__ dy,
                                                               float* __restrict__ part, long long rows, int Cin, int Cout,
-                                                              long long rows_per_block) {
+                                                              int lanes, int parts) {
     pdl_wait();
-    const long long r0 = blockIdx.x * rows_per_block;
-    long long r1 = r0 + rows_per_block;
-    if (r1 > rows) r1 = rows;
     const int C4 = Cin >> 2;
-    const int c4 = blockIdx.y * blockDim.x + threadIdx.x;
+    const int groups = 256 / lanes;
+    const int rl = threadIdx.x / groups, gi = threadIdx.x - rl * groups;
+    const int c4 = blockIdx.y * groups + gi;
+    const int mine = blockIdx.x * lanes + rl;             // this row lane's part: rows mine, mine + parts, ...
+    if (rl >= lanes || mine >= parts) return;
     const int entries = Cin * Cout;
-    float* out = part + (size_t)blockIdx.x * (entries + Cout);
+    float* out = part + (size_t)mine * (entries + Cout);
     if (c4 < C4) {
         float4 acc[MAXD];
 #pragma unroll
         for (int d = 0; d < MAXD; ++d) acc[d] = make_float4(0.f, 0.f, 0.f, 0.f);
         const float4* xp = reinterpret_cast<const float4*>(x) + c4;
 #pragma unroll 2
-        for (long long r = r0; r < r1; ++r) {
+        for (long long r = mine; r < rows; r += parts) {
             const float4 v = xp[(size_t)r * C4];
             const float* gr = dy + (size_t)r * Cout;
 #pragma unroll
@@ -203,17 +192,18 @@ __global__ void __launch_bounds__(256) head_dw_partial_kernel(const float* __res
             }
         }
     }
-    if (blockIdx.y == 0 && (int)threadIdx.x < Cout) {
+    if (blockIdx.y == 0 && gi < Cout) {
         float sdy = 0.f;
-        for (long long r = r0; r < r1; ++r) sdy += dy[(size_t)r * Cout + threadIdx.x];
-        out[entries + threadIdx.x] = sdy;
+#pragma unroll 4
+        for (long long r = mine; r < rows; r += parts) sdy += dy[(size_t)r * Cout + gi];
+        out[entries + gi] = sdy;
     }
 }
 
 // Pointwise layer with at most 16 outputs whose transposed filter fits in shared memory (a classifier head).
 static bool head_shape(const AetherConvDesc& d) {
     return d.fH == 1 && d.fW == 1 && d.sH == 1 && d.sW == 1 && d.padH == 0 && d.padW == 0 && d.Cout <= 16 && d.Cin >= 128 &&
-           (d.Cin & 3) == 0 && (size_t)d.Cin * d.Cout * sizeof(float) <= 96 * 1024;
+           (d.Cin & 3) == 0 && (size_t)(d.Cin + 4) * d.Cout * sizeof(float) <= 96 * 1024;
 }
 
 // ---------------------------------------------------------------------------------- host
@@ -228,7 +218,7 @@ static int gen_blocks(long long total, int threads) {
 int generic_conv_fwd(const AetherConvDesc& d, const float* x, const float* w, const float* b, float* y, cudaStream_t st) {
     if (head_shape(d) && (reinterpret_cast<uintptr_t>(x) & 15u) == 0) {
         const long long rows = 1LL * d.S * d.H * d.W;
-        const int smem = d.Cin * d.Cout * (int)sizeof(float);
+        const int smem = (d.Cin + 4) * d.Cout * (int)sizeof(float);
         static PerDeviceSmem configured;
         if (int rc = ensure_dynamic_smem(gen_fwd_pointwise_few_kernel<16>, 96 * 1024, configured, "head forward")) return rc;
         long long nb = (rows + 7) / 8;                        // a warp per row, 8 rows per block and pass
@@ -259,7 +249,7 @@ int generic_conv_bwd_data(const AetherConvDesc& d, const float* dy, const float*
     }
     if (head_shape(d) && (reinterpret_cast<uintptr_t>(dx) & 15u) == 0) {
         const long long rows = 1LL * d.S * d.H * d.W;
-        const int smem = d.Cin * d.Cout * (int)sizeof(float);
+        const int smem = (d.Cin + 4) * d.Cout * (int)sizeof(float);
         static PerDeviceSmem configured;
         if (int rc = ensure_dynamic_smem(head_dx_kernel<16>, 96 * 1024, configured, "head dX")) return rc;
         long long nb = rows < 2LL * num_sms() ? rows : 2LL * num_sms();
@@ -270,20 +260,16 @@ int generic_conv_bwd_data(const AetherConvDesc& d, const float* dy, const float*
     return simt_conv_bwd_data(d, dy, w, dx, st);
 }
 
-static int gen_dw_blocks(const AetherConvDesc& d) {
-    int Ho, Wo;
-    conv_out_hw(d, Ho, Wo);
-    const long long npix = 1LL * d.S * Ho * Wo;
-    long long nb = npix / 32;
-    if (nb > 148LL * 4) nb = 148LL * 4;
-    if (nb < 1) nb = 1;
-    return (int)nb;
+// Parts of the rows of a classifier head's dW: four rows each until there are 128 of them (their sum is a pass of its own).
+static int head_dw_parts(const AetherConvDesc& d) {
+    const long long rows = 1LL * d.S * d.H * d.W, n = (rows + 3) / 4;
+    return (int)(n < 128 ? n : 128);
 }
 
 size_t generic_conv_workspace_bytes(const AetherConvDesc& d) {
     const size_t simt = simt_conv_workspace_bytes(d);
     if (!head_shape(d)) return simt;
-    const size_t head = align_up((size_t)gen_dw_blocks(d) * ((size_t)d.Cin * d.Cout + d.Cout) * sizeof(float), 1024);
+    const size_t head = align_up((size_t)head_dw_parts(d) * ((size_t)d.Cin * d.Cout + d.Cout) * sizeof(float), 1024);
     return head > simt ? head : simt;
 }
 
@@ -292,18 +278,16 @@ int generic_conv_bwd_filter(const AetherConvDesc& d, const float* x, const float
     if (!head_shape(d) || x == nullptr || (reinterpret_cast<uintptr_t>(x) & 15u)) return simt_conv_bwd_filter(d, x, dy, dw, db, ws, ws_bytes, st);
     if (!ws || ws_bytes < generic_conv_workspace_bytes(d))
         return set_error(AE_BAD_ARG, "conv workspace too small: %zu < %zu", ws_bytes, generic_conv_workspace_bytes(d));
-    const int nb = gen_dw_blocks(d);
-    const long long npix = 1LL * d.S * d.H * d.W;
-    const long long ppb = (npix + nb - 1) / nb;
-    const int entries = d.Cin * d.Cout;
+    const int parts = head_dw_parts(d), C4 = d.Cin / 4;
+    int lanes = 1;                                       // row lanes per block: as many as whole channel rows fit 256 threads
+    while (lanes * 2 <= parts && C4 * lanes * 2 <= 256) lanes *= 2;
+    const int groups = 256 / lanes;
     float* part = static_cast<float*>(ws);
-    launch(head_dw_partial_kernel<16>, dim3(nb, ceil_div(d.Cin / 4, 256)), 256, 0, st, x, dy, part, npix, d.Cin, d.Cout, ppb);
+    launch(head_dw_partial_kernel<16>, dim3(ceil_div(parts, lanes), ceil_div(C4, groups)), 256, 0, st, x, dy, part, 1LL * d.S * d.H * d.W, d.Cin,
+           d.Cout, lanes, parts);
     count_launch();
-    int rc = check_launch("head_dw_partial_kernel");
-    if (rc) return rc;
-    launch(gen_dw_reduce_kernel, ceil_div(entries + d.Cout, 256), 256, 0, st, part, nb, entries, d.Cout, dw, db);
-    count_launch();
-    return check_launch("gen_dw_reduce_kernel");
+    if (int rc = check_launch("head_dw_partial_kernel")) return rc;
+    return smallc_reduce_partials(part, parts, d.Cin, d.Cout, dw, db, st);
 }
 
 }  // namespace aether

@@ -51,13 +51,17 @@ __global__ void __launch_bounds__(DWH_THREADS, 1) dw_halo_kernel(const __grid_co
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
 
-    // Rows that no TMA box ever writes (the tail of each dy region up to a multiple of 16 rows) must read as zero.
-    {
-        uint4* z = reinterpret_cast<uint4*>(gen_base);
-        const int n16 = S * p.stage_bytes / 16;
-        for (int i = threadIdx.x; i < n16; i += blockDim.x) z[i] = make_uint4(0, 0, 0, 0);
-        fence_proxy_async_smem();
+    // Rows that no TMA box ever writes (the tails of the two regions of a stage) are read by the MMAs and must be zero: the
+    // dy rows because they are part of the last reduction step, the x rows so that zero times them stays zero.  Only those
+    // few KB are cleared, not the stages.
+    for (int s = 0; s < S; ++s) {
+        uint8_t* st = gen_base + (size_t)s * p.stage_bytes;
+        for (int o = p.xr_rows * 128 + threadIdx.x * 16; o < p.xr_bytes; o += blockDim.x * 16)
+            *reinterpret_cast<uint4*>(st + o) = make_uint4(0, 0, 0, 0);
+        for (int o = p.xr_bytes + p.dyr_rows * 128 + threadIdx.x * 16; o < p.stage_bytes; o += blockDim.x * 16)
+            *reinterpret_cast<uint4*>(st + o) = make_uint4(0, 0, 0, 0);
     }
+    fence_proxy_async_smem();
     if (threadIdx.x == 0) {
         for (int s = 0; s < S; ++s) {
             mbar_init(full_bar(s), 1);

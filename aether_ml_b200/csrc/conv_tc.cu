@@ -109,7 +109,7 @@ struct IgemmParams {
     CUtensorMap tm_w;    // filter matrix, K contiguous: (K, taps * rows_per_tap), box (128 B of K, NT)
     float* out;          // fp32 output, NHWC (out_N, out_H, out_W, n_out), 16-byte aligned, n_out % 4 == 0
     const float* bias;   // nullable, n_out entries
-    float* stats;        // STATS only: [gridDim.x / n_tiles_n * 4][3][n_out] (count, mean, M2) partial blocks
+    float* stats;        // STATS only: [gridDim.x / n_tiles_n][3][n_out] (count, mean, M2) partial rows
     int* status;
     int n_out;
     int out_W, out_H, out_N;   // output extent: accumulator rows outside it are by-products
@@ -461,27 +461,14 @@ __global__ void __launch_bounds__(IGEMM_THREADS, 1) igemm_conv_kernel(const __gr
             }
             st_rows += tile_rows;
         }
-        if (STATS && lane < 4) {
-            // (count, mean, M2) of this warp's rows over all tiles of the CTA.  The grid is a multiple of
-            // n_tiles_n, so the CTA kept column tile blockIdx.x % n_tiles_n; the n_tiles_n CTAs of a group fill the
-            // disjoint column ranges of block (group * 4 + q) of [3][n_out].
-            // (PAIR: the same with pairs in the place of CTAs and one block group per CTA of the pair.)
+        if (STATS) {
+            // One (count, mean, M2) row per CTA group: the grid is a multiple of n_tiles_n, so the CTA kept column tile
+            // blockIdx.x % n_tiles_n, and the n_tiles_n CTAs of a group fill the disjoint column ranges of row `group` of
+            // [3][n_out].  (PAIR: the same with pairs in the place of CTAs and one row per CTA of the pair.)
             const int ntc = (int)(t_first % p.n_tiles_n);
             const size_t group = PAIR ? (size_t)(t_first / p.n_tiles_n) * 2 + cta_rank : (size_t)(t_first / p.n_tiles_n);
-            float* sp = p.stats + (group * 4 + q) * 3 * (size_t)p.n_out;
-            for (int cc = 0; cc < ncols; cc += 16) {
-#pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    const int col = ntc * NT + col_begin + tcol4 + cc + k;
-                    if (col < p.n_out) {
-                        float m, m2;
-                        stats_result(stat_w, cc + tcol4 + k, st_rows, m, m2);
-                        sp[col] = st_rows;
-                        sp[p.n_out + col] = m + (p.bias != nullptr ? __ldg(p.bias + col) : 0.f);
-                        sp[2 * p.n_out + col] = m2;
-                    }
-                }
-            }
+            stats_merge_store(reinterpret_cast<float*>(gen_base + (sBar - smem_base) + IGEMM_TAIL), ew, lane, st_rows, ncols, ntc * NT, p.n_out,
+                              p.bias, p.stats + group * 3 * (size_t)p.n_out);
         }
     }
 
@@ -552,11 +539,15 @@ __global__ void __launch_bounds__(DW_THREADS, 1) dw_conv_kernel(const __grid_con
     const int cta_rank = PAIR ? (int)cluster_cta_rank() : 0;
     const bool issuer = cta_rank == 0;
 
-    // Rows past p.rows are never written by TMA but are read by the MMAs: keep them zero.
+    // Rows of a box past p.rows are never written by TMA; those that belong to the last reduction step are read by the MMAs
+    // and must be zero.  Nothing to do when the box is whole steps (clearing all stages took 2 us of a small layer's 11).
     {
-        uint4* z = reinterpret_cast<uint4*>(gen_base);
-        const int n16 = STAGES * Cfg::STAGE_BYTES / 16;
-        for (int i = threadIdx.x; i < n16; i += blockDim.x) z[i] = make_uint4(0, 0, 0, 0);
+        const int k_end = (p.rows + Cfg::KROWS - 1) / Cfg::KROWS * Cfg::KROWS;
+        const int per_tile = (k_end - p.rows) * 8;                              // 16-byte pieces
+        for (int i = threadIdx.x; i < STAGES * (MB + NB) * per_tile; i += blockDim.x) {
+            const int tile = i / per_tile;
+            *reinterpret_cast<uint4*>(gen_base + (size_t)tile * TILE_A_BYTES + p.rows * 128 + (i - tile * per_tile) * 16) = make_uint4(0, 0, 0, 0);
+        }
         fence_proxy_async_smem();
     }
     if (threadIdx.x == 0) {
@@ -1063,6 +1054,30 @@ static TcPlan compute_plan(const AetherConvDesc& d) {
         if (want > ptiles) want = ptiles;
         return (int)want;
     };
+    // Small layers, whose operands stay in L2: the products are cheap, what counts is how many CTAs share them and how many
+    // partials they leave.  One M group per CTA and few splits against many groups and as many splits as SMs: estimated
+    // per candidate from what a stage (64 KB from L2), an accumulator's store and the partials' way through L2 take.
+    // (128 images 8x8 64->128: 128 CTAs x 64 partials of 295 KB -> 29 partials; Dense 784->128 at batch 128: 2 CTAs -> 7.)
+    auto decompose_small = [&]() {
+        pl.dw_MG = ceil_div(pl.dw_U, MB);
+        pl.dw_ntn = pl.Cout_p / pl.dw_nt;
+        const double t_stage = 0.45 * (MB + pl.dw_nb) / 4.0, t_store = 0.5;
+        const double dw_us = 2.0 * pl.dw_U * UC * pl.Cout_p * 4.0 / 4e6;        // a partial written and read at 4 TB/s
+        const int max_gpc = 512 / pl.dw_nt;
+        double best = 1e30;
+        int best_gpc = 1, best_splits = 1;
+        for (int g = 1; g <= max_gpc && g <= pl.dw_MG; ++g) {
+            const long long cols = 1LL * ceil_div(pl.dw_MG, g) * pl.dw_ntn;
+            for (long long s = 1; s <= ptiles && s * cols <= num_sms(); ++s) {
+                const double cost = (double)((ptiles + s - 1) / s) * g * t_stage + g * t_store + (s > 1 ? 1.5 + s * dw_us : 0.0);
+                if (cost < best - 1e-9) { best = cost; best_gpc = g; best_splits = (int)s; }
+            }
+        }
+        if (best == 1e30) return 0;
+        pl.dw_gpc = best_gpc;
+        pl.dw_ngc = ceil_div(pl.dw_MG, best_gpc);
+        return best_splits;
+    };
     // pairs: the channel counts must fill 256 rows and two column halves, and every pair needs a few pixel tiles
     pl.dw_halo_splits = decompose(1);
     if (pl.dw_halo_splits < 1) pl.dw_halo_splits = 1;
@@ -1076,6 +1091,11 @@ static TcPlan compute_plan(const AetherConvDesc& d) {
         } else {
             pl.dw_splits = ps;
         }
+    }
+    if (!pl.dw_pair && (1LL * d.S * d.H * d.W * pl.Cin_p + 1LL * d.S * pl.Ho * pl.Wo * pl.Cout_p) * pl.elt <= (32LL << 20)) {
+        const int s = decompose_small();
+        if (s > 0) pl.dw_splits = s;
+        else decompose(1);
     }
     const long long out_rows = 1LL * d.S * pl.Ho * pl.Wo;
     pl.db_blocks = (int)(out_rows < 4LL * num_sms() * 64 ? (out_rows + 63) / 64 : 4LL * num_sms());
@@ -1291,17 +1311,17 @@ long long tc_conv_stats_blocks(const AetherConvDesc& d) {
     const long long hb = halo_igemm_stats_blocks(pl.tf32, pl.tf32 ? d.Cin : pl.Cin_p, d.S, pl.taps, d.Cout, pl.Ho, pl.Wo,
                                                  pl.Cout_p, d.fH, d.fW);
     if (hb > 0) return hb;
-    // per-tap kernel: one block per CTA group (the CTAs of one set of pixel tiles) and 32-row quarter
+    // per-tap kernel: one row per CTA group (the CTAs of one set of pixel tiles)
     const int nt = pick_nt(pl.Cout_p);
     const int n_tiles_n = ceil_div(pl.Cout_p, nt);
     if (igemm_use_pairs(pl.til_out.total(), nt, n_tiles_n)) {       // one block group per CTA of a pair
         const int pairs = igemm_pair_grid(pl.til_out.total(), n_tiles_n, true) / 2;
         if (pairs % n_tiles_n) return 0;
-        return 4LL * 2 * (pairs / n_tiles_n);
+        return 2LL * (pairs / n_tiles_n);
     }
     const int grid = igemm_grid(pl.til_out.total(), n_tiles_n, true);
     if (grid % n_tiles_n) return 0;
-    return 4LL * (grid / n_tiles_n);
+    return grid / n_tiles_n;
 }
 
 int tc_conv_fwd(const AetherConvDesc& d, const float* x, const float* w, const float* b, float* y, float* stats, void* ws,

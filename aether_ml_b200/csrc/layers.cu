@@ -7,6 +7,7 @@
 #include <string.h>
 
 #include "common.cuh"
+#include "tail.cuh"
 
 namespace aether {
 
@@ -530,6 +531,14 @@ float* bn_forward_coeffs(const float* x, const float* partials, long long nblock
     return coeff;
 }
 
+int bn_reduce_partials(const float* x, long long rows, int C, float* part, int most, cudaStream_t st) {
+    int nb = bn_blocks(rows);
+    if (nb > most) nb = most;
+    launch_bn_reduce<0>(nb, st, x, nullptr, nullptr, nullptr, 0.f, rows, C, part);
+    count_launch();
+    return nb;
+}
+
 // Inference coefficients from the running statistics into ws (2*C floats).
 float* bn_eval_coeffs(const float* gamma, const float* beta, const float* running_mean, const float* running_var, int C,
                       float eps, float* ws, cudaStream_t st) {
@@ -544,6 +553,47 @@ void bn_backward_coeffs(const float* part, int nb, int C, long long rows, const 
                         cudaStream_t st) {
     launch(bn_finalize_bwd_kernel, ceil_div(C, FIN_CH), FIN_THREADS, 0, st, part, nb, C, rows, gamma, mean, var, eps, dgamma, dbeta, coeff, pscale);
     count_launch();
+}
+
+// Statistics partials of x for the one-pass forms of bn_small.cu: the producer's, or reduced here into ws (no more rows than
+// CTAs merge quickly).
+static const float* bn_small_partials(const float* x, const float* partials, int64_t* nblocks, long long rows, int C, float* ws,
+                                      cudaStream_t st) {
+    if (partials) return partials;
+    *nblocks = bn_reduce_partials(x, rows, C, ws, 148, st);
+    return ws;
+}
+// Batch_Norm (+ activation, alpha >= 0, + folded mask) of a small [rows][C] tensor.
+static void bn_small_rows(const float* x, const float* partials, int64_t nblocks, const float* gamma, const float* beta, float* running_mean,
+                          float* running_var, float* batch_mean, float* batch_var, float* y, long long rows, int C, float eps, float momentum,
+                          float alpha, const float* mask, float* ws, cudaStream_t st) {
+    BnSmallFwd p = {};
+    p.x = x;
+    p.part = bn_small_partials(x, partials, &nblocks, rows, C, ws, st);
+    p.nblocks = (int)nblocks;
+    p.gamma = gamma; p.beta = beta; p.running_mean = running_mean; p.running_var = running_var;
+    p.batch_mean = batch_mean; p.batch_var = batch_var; p.eps = eps; p.momentum = momentum; p.alpha = alpha;
+    p.mask = mask;
+    p.fold = 1;
+    (alpha >= 0.f ? p.act_out : p.bn_out) = y;
+    p.H = p.W = p.fH = p.fW = p.Hc = p.Wc = 1;
+    p.C = C;
+    p.windows = (unsigned)rows;
+    bn_small_forward(p, st);
+}
+static void bn_small_rows_bwd(const float* x, const float* dy, const float* gamma, const float* beta, const float* mean, const float* var,
+                              const float* pscale, float* dx, float* dgamma, float* dbeta, long long rows, int C, float eps, float alpha,
+                              float* ws, cudaStream_t st) {
+    int nb = bn_blocks(rows);
+    if (nb > 148) nb = 148;
+    launch_bn_reduce<1>(nb, st, x, dy, mean, var, eps, rows, C, ws, alpha >= 0.f ? gamma : nullptr, alpha >= 0.f ? beta : nullptr, alpha);
+    count_launch();
+    BnSmallBwd p = {};
+    p.x = x; p.dy = dy; p.part = ws; p.nblocks = nb; p.gamma = gamma; p.beta = beta; p.mean = mean; p.var = var; p.pscale = pscale;
+    p.eps = eps; p.alpha = alpha; p.dgamma = dgamma; p.dbeta = dbeta; p.dx = dx; p.W = p.fH = p.fW = 1; p.C = C;
+    p.windows = (unsigned)rows;
+    p.rows = rows;
+    bn_small_backward(p, 0, st);
 }
 
 // dx = k1 * dy + k2 * x + k3 with the coefficients of bn_backward_coeffs.
@@ -570,6 +620,11 @@ extern "C" int aether_bn_fwd_train(const float* x, const float* gamma, const flo
     if (ws_bytes < aether_bn_workspace_bytes(rows, C)) return set_error(AE_BAD_ARG, "aether_bn_fwd_train: workspace too small");
     if ((C & 3) == 0 && (!aligned16(x) || !aligned16(y))) return set_error(AE_BAD_ARG, "aether_bn_fwd_train: arrays must be 16-byte aligned");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if (bn_small(rows * C, C)) {
+        bn_small_rows(x, nullptr, 0, gamma, beta, running_mean, running_var, batch_mean, batch_var, y, rows, C, eps, momentum, -1.f, nullptr,
+                      static_cast<float*>(ws), st);
+        return check_launch("aether_bn_fwd_train");
+    }
     const int nb = bn_blocks(rows);
     float* part = static_cast<float*>(ws);
     float* coeff = part + (size_t)nb * 3 * C;
@@ -596,6 +651,11 @@ extern "C" int aether_bn_fwd_train_partials(const float* x, const float* partial
         return set_error(AE_BAD_ARG, "aether_bn_fwd_train_partials: workspace too small or misaligned (needs 2*C floats)");
     if ((C & 3) == 0 && (!aligned16(x) || !aligned16(y))) return set_error(AE_BAD_ARG, "aether_bn_fwd_train_partials: arrays must be 16-byte aligned");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if (bn_small(rows * C, C)) {
+        bn_small_rows(x, partials, nblocks, gamma, beta, running_mean, running_var, batch_mean, batch_var, y, rows, C, eps, momentum, -1.f,
+                      nullptr, nullptr, st);
+        return check_launch("aether_bn_fwd_train_partials");
+    }
     float* coeff = static_cast<float*>(ws);
     launch(bn_finalize_fwd_kernel, ceil_div(C, FIN_CH), FIN_THREADS, 0, st, partials, (int)nblocks, C, gamma, beta, eps, momentum,
            running_mean, running_var, batch_mean, batch_var, coeff);
@@ -692,6 +752,10 @@ extern "C" int aether_bn_bwd(const float* x, const float* dy, const float* gamma
     if ((C & 3) == 0 && (!aligned16(x) || !aligned16(dy) || !aligned16(dx)))
         return set_error(AE_BAD_ARG, "aether_bn_bwd: arrays must be 16-byte aligned");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if (bn_small(rows * C, C)) {
+        bn_small_rows_bwd(x, dy, gamma, nullptr, batch_mean, batch_var, nullptr, dx, dgamma, dbeta, rows, C, eps, -1.f, static_cast<float*>(ws), st);
+        return check_launch("aether_bn_bwd");
+    }
     const int nb = bn_blocks(rows);
     float* part = static_cast<float*>(ws);
     float* coeff = part + (size_t)nb * 3 * C;
@@ -727,6 +791,11 @@ extern "C" int aether_bn_act_fwd_train(const float* x, const float* partials, in
     if (ws_bytes < aether_bn_workspace_bytes(rows, C)) return set_error(AE_BAD_ARG, "aether_bn_act_fwd_train: workspace too small");
     if (partials && (nblocks <= 0 || nblocks > (1 << 30))) return set_error(AE_BAD_ARG, "aether_bn_act_fwd_train: nblocks");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if (bn_small(rows * C, C)) {
+        bn_small_rows(x, partials, nblocks, gamma, beta, running_mean, running_var, batch_mean, batch_var, y, rows, C, eps, momentum, alpha,
+                      channel_scale, static_cast<float*>(ws), st);
+        return check_launch("aether_bn_act_fwd_train");
+    }
     int nb = bn_blocks(rows);
     float* part = static_cast<float*>(ws);
     float* coeff = part + (size_t)nb * 3 * C;
@@ -780,6 +849,11 @@ extern "C" int aether_bn_act_bwd(const float* x, const float* beta, const float*
     if (rc) return rc;
     if (ws_bytes < aether_bn_workspace_bytes(rows, C)) return set_error(AE_BAD_ARG, "aether_bn_act_bwd: workspace too small");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if (bn_small(rows * C, C) && aligned16(gamma) && aligned16(beta) && aligned16(batch_mean) && aligned16(batch_var)) {
+        bn_small_rows_bwd(x, dy, gamma, beta, batch_mean, batch_var, channel_scale, dx, dgamma, dbeta, rows, C, eps, alpha,
+                          static_cast<float*>(ws), st);
+        return check_launch("aether_bn_act_bwd");
+    }
     const int nb = bn_blocks(rows);
     float* part = static_cast<float*>(ws);
     float* coeff = part + (size_t)nb * 3 * C;

@@ -11,9 +11,11 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include "sm100_ptx.cuh"
+
 namespace aether {
 
-static constexpr int STATS_WARP_FLOATS = 3 * 128;
+static constexpr int STATS_WARP_FLOATS = 3 * 128 + 4;   // (the last: the warp's row count, for the merge at the end)
 
 // Two fp32 values in one 64-bit register, and the packed arithmetic of sm_100 (one instruction for two results, each
 // rounded exactly like the scalar add / fma): the per-element work of the statistics is three such instructions per
@@ -79,6 +81,36 @@ __device__ __forceinline__ void stats_result(const float* stat_w, int c, float r
     const float m = rows > 0.f ? s / rows : 0.f;
     mean = stat_w[256 + c] + m;
     m2 = fmaxf(q - s * m, 0.f);
+}
+
+// The end of a statistics epilogue: the four 32-row quarters of each column half are merged (Chan's formula, fixed order), so
+// a CTA hands ONE (count, mean, M2) row to whoever adds the rows up, not four.  Called by all 256 epilogue threads; `ew` is
+// the warp's index (its half is ew / 4), `stats0` warp 0's area, `rows` the rows this warp has summed, `ncols` the columns
+// of a half; out[col], out[n_out + col], out[2 n_out + col] for col = col0 + half * ncols + c below n_out.
+__device__ __forceinline__ void stats_merge_store(float* stats0, int ew, int lane, float rows, int ncols, int col0, int n_out,
+                                                  const float* bias, float* out) {
+    if (lane == 0) stats0[ew * STATS_WARP_FLOATS + 3 * 128] = rows;
+    named_bar_sync(2, 256);
+    for (int t = ew * 32 + lane; t < 2 * ncols; t += 256) {
+        const int half = t >= ncols ? 1 : 0, c = t - half * ncols, col = col0 + t;
+        if (col >= n_out) continue;
+        float N = 0.f, M = 0.f, M2 = 0.f;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const float* w = stats0 + (half * 4 + k) * STATS_WARP_FLOATS;
+            const float n = w[3 * 128];
+            if (n == 0.f) continue;
+            float m, m2;
+            stats_result(w, c, n, m, m2);
+            const float tot = N + n, delta = m - M;
+            M2 += m2 + delta * delta * N * n / tot;
+            M += delta * n / tot;
+            N = tot;
+        }
+        out[col] = N;
+        out[n_out + col] = M + (bias != nullptr ? bias[col] : 0.f);
+        out[2 * n_out + col] = M2;
+    }
 }
 
 }  // namespace aether
