@@ -3,7 +3,7 @@
 //   y[p][d] = b[d] + sum_k col[p][k] * w[k][d]            (Conv_Layer.forward, CNN_classes_cupy.py:70-120)
 //
 // With 3 input channels a pixel's 12 bytes cannot be the inner extent of a TMA box and K = 27 is less than one
-// 128-byte operand row, so the im2col rows are built by threads: four producer warps gather the K input values of
+// 128-byte operand row, so the im2col rows are built by threads: producer warps gather the K input values of
 // 128 output pixels (one pixel per thread), convert them to bf16 and write them as a K-major, 128-byte-swizzled
 // operand tile (16-byte chunk c of row r is stored at chunk c ^ (r % 8)); the filter is laid out the same way once
 // per CTA.  One warp issues K/16 (two for a 3x3 RGB filter) 128 x Cout x 16 MMAs per tile into one of up to four
@@ -16,7 +16,6 @@
 #include "common.cuh"
 #include "sm100_ptx.cuh"
 #include "stats_epilogue.cuh"
-#include "tc_host.cuh"
 #include "tc_host.cuh"
 
 namespace aether {
@@ -33,12 +32,12 @@ struct FirstParams {
     int stages, ntiles;
 };
 
-// Producer warps: about two threads per pixel -- a lone producer warp per scheduler cannot hide the gather latency.
-// The kernel with the statistics epilogue runs 7 of them: 16 warps are four per scheduler and 128 registers per thread,
-// 17 warps put five on one scheduler and cap every thread at 96, which the statistics' running sums do not fit in.
+// Producer warps: one or two groups of four that build alternate tiles, a pixel per thread, the next tile's loads in flight
+// while the current one is stored.  One group in the kernel with the statistics epilogue: more than 16 warps would cap
+// every thread at 96 registers, which the statistics' running sums do not fit in.
 static constexpr int FT_EPI_WARPS = 8;
 template <bool STATS> struct FirstCfg {
-    static constexpr int PROD_WARPS = STATS ? 7 : 8;
+    static constexpr int PROD_WARPS = STATS ? 4 : 8;             // groups of four: a thread per pixel of a tile
     static constexpr int THREADS = 32 * (PROD_WARPS + 1 + FT_EPI_WARPS);   // producers, MMA issuer, epilogue
 };
 static constexpr int FT_STAGE_BYTES = 128 * 128;                             // 128 pixel rows of 128 bytes
@@ -59,7 +58,70 @@ __device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
     return *reinterpret_cast<const uint32_t*>(&v);
 }
 
-template <bool STATS>
+// ---- the im2col gather shared by the forward and the filter-gradient kernel.  A thread builds one operand row: the K input
+// values of one output pixel.  All of a row's loads are independent and issued together (a row is one load latency; in
+// pieces of eight values it was three or four of them, each behind a 64-bit division of the pixel index, and the gather
+// took 1.6 us per tile, twice the rest of the kernel).
+struct FirstTaps {                 // entry k of a row: element offset from the window's first value, filter row | column << 8
+    int2 t[64];
+};
+__device__ __forceinline__ void first_fill_taps(FirstTaps& tab, int K, int Cin, int fW, int W) {
+    for (int k = threadIdx.x; k < 64; k += blockDim.x) {
+        const int kk = k < K ? k : 0;
+        const int tap = kk / Cin, c = kk - tap * Cin;
+        const int i = tap / fW, j = tap - i * fW;
+        tab.t[k] = make_int2((i * W + j) * Cin + c, k < K ? i | (j << 8) : 0x3f3f);   // past K: bit 63 of the masks, never set
+    }
+}
+struct FirstPixel {
+    const float* base;             // the window's first value (may lie before the image: used with valid taps only)
+    unsigned long long rows, cols; // bit i / j: filter row i / column j falls inside the image
+};
+__device__ __forceinline__ FirstPixel first_pixel(const float* x, long long pix, long long P, int H, int W, int Cin, int fH, int fW, int sH, int sW,
+                                                  int pH, int pW, int Ho, int Wo) {
+    FirstPixel q;
+    q.rows = q.cols = 0ull;
+    q.base = x;
+    if (pix < P) {
+        int n, ho, wo;
+        if (P < (1LL << 31)) {                          // 32-bit divisions are several times cheaper
+            const unsigned u = (unsigned)pix, r = u / (unsigned)Wo;
+            wo = (int)(u - r * (unsigned)Wo);
+            n = (int)(r / (unsigned)Ho);
+            ho = (int)(r - (unsigned)n * (unsigned)Ho);
+        } else {
+            const long long r = pix / Wo, s = r / Ho;
+            wo = (int)(pix - r * Wo);
+            n = (int)s;
+            ho = (int)(r - s * Ho);
+        }
+        const int h0 = ho * sH - pH, w0 = wo * sW - pW;
+        q.base = x + (((long long)n * H + h0) * W + w0) * Cin;
+        // rows i with 0 <= h0 + i < H, columns alike (filters of at most 64 entries)
+        const int i0 = h0 < 0 ? -h0 : 0, i1 = min(fH, H - h0), j0 = w0 < 0 ? -w0 : 0, j1 = min(fW, W - w0);
+        if (i1 > i0) q.rows = (~0ull >> (64 - i1)) & ~((1ull << i0) - 1ull);
+        if (j1 > j0) q.cols = (~0ull >> (64 - j1)) & ~((1ull << j0) - 1ull);
+    }
+    return q;
+}
+template <int KP>
+__device__ __forceinline__ void first_gather(const FirstTaps& tab, const FirstPixel& q, float (&v)[KP]) {
+#pragma unroll
+    for (int k = 0; k < KP; ++k) {
+        const int2 t = tab.t[k];
+        v[k] = ((q.rows >> (t.y & 63)) & (q.cols >> (t.y >> 8)) & 1ull) ? __ldg(q.base + t.x) : 0.f;
+    }
+}
+template <int KP>
+__device__ __forceinline__ void first_store_row(uint8_t* tile, int r, const float (&v)[KP]) {
+#pragma unroll
+    for (int ch = 0; ch < KP / 8; ++ch)
+        *reinterpret_cast<uint4*>(tile + r * 128 + ((ch ^ (r & 7)) << 4)) =
+            make_uint4(pack_bf16(v[8 * ch], v[8 * ch + 1]), pack_bf16(v[8 * ch + 2], v[8 * ch + 3]), pack_bf16(v[8 * ch + 4], v[8 * ch + 5]),
+                       pack_bf16(v[8 * ch + 6], v[8 * ch + 7]));
+}
+
+template <bool STATS, int KP>
 __global__ void __launch_bounds__(FirstCfg<STATS>::THREADS, 1) first_conv_kernel(const __grid_constant__ FirstParams p) {
     constexpr int FT_PROD_WARPS = FirstCfg<STATS>::PROD_WARPS;
     extern __shared__ uint8_t smem_raw[];
@@ -76,9 +138,7 @@ __global__ void __launch_bounds__(FirstCfg<STATS>::THREADS, 1) first_conv_kernel
     const uint32_t sTmemPtr = sBar + 8u * (2 * S + 8);
     volatile uint32_t* tmem_ptr_generic = reinterpret_cast<volatile uint32_t*>(gen_base + (sTmemPtr - smem_base));
     float* bias_s = reinterpret_cast<float*>(gen_base + (sBar - smem_base) + 256);         // NT <= 256 floats
-    int* koff_s = reinterpret_cast<int*>(gen_base + (sBar - smem_base) + 256 + 1024);      // K <= 64 entries each
-    int* ki_s = koff_s + 64;
-    int* kj_s = ki_s + 64;
+    FirstTaps& taps = *reinterpret_cast<FirstTaps*>(gen_base + (sBar - smem_base) + 256 + 1024);
 
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
@@ -88,7 +148,7 @@ __global__ void __launch_bounds__(FirstCfg<STATS>::THREADS, 1) first_conv_kernel
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < S; ++s) {
-            mbar_init(full_bar(s), 32 * FT_PROD_WARPS);
+            mbar_init(full_bar(s), 128);
             mbar_init(empty_bar(s), 1);
         }
         for (int b = 0; b < 4; ++b) {
@@ -97,14 +157,7 @@ __global__ void __launch_bounds__(FirstCfg<STATS>::THREADS, 1) first_conv_kernel
         }
         mbar_fence_init();
     }
-    for (int k = threadIdx.x; k < 64; k += blockDim.x) {
-        const int kk = k < p.K ? k : 0;
-        const int tap = kk / p.Cin, c = kk - tap * p.Cin;
-        const int i = tap / p.fW, j = tap - i * p.fW;
-        ki_s[k] = k < p.K ? i : (1 << 20);                         // entries past K fail the bounds test: zero
-        kj_s[k] = j;
-        koff_s[k] = (i * p.W + j) * p.Cin + c;
-    }
+    first_fill_taps(taps, p.K, p.Cin, p.fW, p.W);
     if (warp == FT_PROD_WARPS) {
         tmem_alloc(sTmemPtr, tmem_cols);
         tmem_relinquish();
@@ -112,8 +165,8 @@ __global__ void __launch_bounds__(FirstCfg<STATS>::THREADS, 1) first_conv_kernel
     pdl_wait();                       // set-up done; from here on global memory is touched
     for (int i = threadIdx.x; i < NT; i += blockDim.x) bias_s[i] = (p.bias != nullptr && i < p.Cout) ? p.bias[i] : 0.f;
     // filter operand: row n = output channel, element k at byte (k/8 ^ n%8)*16 + (k%8)*2 of the row
-    for (int it = threadIdx.x; it < NT * (p.KP >> 3); it += blockDim.x) {
-        const int n = it / (p.KP >> 3), ch = it - n * (p.KP >> 3);
+    for (int it = threadIdx.x; it < NT * (KP / 8); it += blockDim.x) {
+        const int ch = it / NT, n = it - ch * NT;                  // neighbouring threads read neighbouring output channels
         float v[8];
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
@@ -133,46 +186,23 @@ __global__ void __launch_bounds__(FirstCfg<STATS>::THREADS, 1) first_conv_kernel
 
     if (warp < FT_PROD_WARPS) {
         // ------------------------------------------------------------------ producers
-        // A tile is 128 rows x (KP / 8) 16-byte chunks; the producer threads take the (row, chunk) pairs round robin.
-        constexpr int NPT = 32 * FT_PROD_WARPS;
+        constexpr int GROUPS = FT_PROD_WARPS / 4;
         uint8_t* tile_gen = gen_base + (sA - smem_base);
-        const int ntasks = (p.KP >> 3) << 7;
-        const long long HoWo = (long long)p.Ho * p.Wo;
-        int s = 0;
-        uint32_t ph = 0;
-        for (int t = blockIdx.x; t < p.ntiles; t += grid) {
-            if (!mbar_wait(empty_bar(s), ph ^ 1u, p.status, DS_TIMEOUT_EMPTY)) break;
-            uint8_t* stage_gen = tile_gen + s * FT_STAGE_BYTES;
-            int r_prev = -1, h0 = 0, w0 = 0;
-            long long base = 0;
-            for (int task = threadIdx.x; task < ntasks; task += NPT) {
-                const int r = task & 127, ch = task >> 7;
-                if (r != r_prev) {                                  // with 256 producer threads: once per thread and tile
-                    r_prev = r;
-                    const long long pix = (long long)t * 128 + r;
-                    h0 = -(1 << 20); w0 = 0; base = 0;
-                    if (pix < p.P) {
-                        const long long n = pix / HoWo;
-                        const int rem = (int)(pix - n * HoWo);
-                        const int ho = rem / p.Wo, wo = rem - ho * p.Wo;
-                        h0 = ho * p.sH - p.pH;
-                        w0 = wo * p.sW - p.pW;
-                        base = ((n * p.H + h0) * p.W + w0) * p.Cin;  // may point before the image: only used with valid taps
-                    }
-                }
-                float v[8];
-#pragma unroll
-                for (int e = 0; e < 8; ++e) {
-                    const int k = ch * 8 + e;
-                    const int hi = h0 + ki_s[k], wi = w0 + kj_s[k];
-                    v[e] = (hi >= 0 && hi < p.H && wi >= 0 && wi < p.W) ? __ldg(p.x + base + koff_s[k]) : 0.f;
-                }
-                const uint4 q = make_uint4(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]), pack_bf16(v[4], v[5]), pack_bf16(v[6], v[7]));
-                *reinterpret_cast<uint4*>(stage_gen + r * 128 + ((ch ^ (r & 7)) << 4)) = q;
-            }
+        const int grp = threadIdx.x >> 7, r = threadIdx.x & 127;
+        auto pixel = [&](int t) {
+            return first_pixel(p.x, (long long)t * 128 + r, p.P, p.H, p.W, p.Cin, p.fH, p.fW, p.sH, p.sW, p.pH, p.pW, p.Ho, p.Wo);
+        };
+        float v[KP];
+        int t = blockIdx.x + grp * grid;
+        if (t < p.ntiles) first_gather<KP>(taps, pixel(t), v);
+        for (int it = grp; t < p.ntiles; it += GROUPS) {
+            const int s = it % S;
+            if (!mbar_wait(empty_bar(s), ((uint32_t)(it / S) & 1u) ^ 1u, p.status, DS_TIMEOUT_EMPTY)) break;
+            first_store_row<KP>(tile_gen + s * FT_STAGE_BYTES, r, v);
             fence_proxy_async_smem();                               // generic-proxy writes -> visible to the tensor core
             mbar_arrive(full_bar(s));
-            if (++s == S) { s = 0; ph ^= 1u; }
+            t += GROUPS * grid;
+            if (t < p.ntiles) first_gather<KP>(taps, pixel(t), v);
         }
     } else if (warp == FT_PROD_WARPS) {
         // ------------------------------------------------------------------ MMA issuer
@@ -183,7 +213,7 @@ __global__ void __launch_bounds__(FirstCfg<STATS>::THREADS, 1) first_conv_kernel
         const uint32_t lo_proto = (uint32_t)proto;
         const uint32_t w_lo = lo_proto + ((sW & 0x3FFFFu) >> 4);
         const uint32_t a_lo0 = lo_proto + ((sA & 0x3FFFFu) >> 4);
-        const int ksteps = p.KP >> 4;
+        constexpr int ksteps = KP / 16;
         int s = 0;
         uint32_t ph = 0, buf = 0, aph = 0;
         bool ok = true;
@@ -413,6 +443,7 @@ static constexpr int FD_ROWS = 6;                                            // 
 static constexpr int FD_TAIL = 1024 + FD_NP * 8 * 4 + 1024;                  // barriers, k tables, dB staging
 static constexpr int FD_THREADS = 32 * (FD_PROD_WARPS + 1 + 4);              // producers, MMA issuer, 4 epilogue warps
 
+template <int KP>
 __global__ void __launch_bounds__(FD_THREADS, 1) first_dw_kernel(const __grid_constant__ FirstDwParams p) {
     extern __shared__ uint8_t smem_raw[];
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -424,9 +455,7 @@ __global__ void __launch_bounds__(FD_THREADS, 1) first_dw_kernel(const __grid_co
     const uint32_t done_bar = sBar + 8u * (2 * S);
     const uint32_t sTmemPtr = sBar + 8u * (2 * S + 1);
     volatile uint32_t* tmem_ptr_generic = reinterpret_cast<volatile uint32_t*>(gen_base + (sTmemPtr - smem_base));
-    int* koff_s = reinterpret_cast<int*>(gen_base + (sBar - smem_base) + 256);
-    int* ki_s = koff_s + 64;
-    int* kj_s = ki_s + 64;
+    FirstTaps& taps = *reinterpret_cast<FirstTaps*>(gen_base + (sBar - smem_base) + 256);
     float* dbsum_s = reinterpret_cast<float*>(gen_base + (sBar - smem_base) + 1024);      // [producer threads][8]
 
     const int warp = threadIdx.x >> 5;
@@ -442,14 +471,7 @@ __global__ void __launch_bounds__(FD_THREADS, 1) first_dw_kernel(const __grid_co
         mbar_fence_init();
         if (p.dy_bf16) tma_prefetch_desc(&p.tm_dy);
     }
-    for (int k = threadIdx.x; k < 64; k += blockDim.x) {
-        const int kk = k < p.K ? k : 0;
-        const int tap = kk / p.Cin, c = kk - tap * p.Cin;
-        const int i = tap / p.fW, j = tap - i * p.fW;
-        ki_s[k] = k < p.K ? i : (1 << 20);
-        kj_s[k] = j;
-        koff_s[k] = (i * p.W + j) * p.Cin + c;
-    }
+    first_fill_taps(taps, p.K, p.Cin, p.fW, p.W);
     if (warp == FD_PROD_WARPS) {
         tmem_alloc(sTmemPtr, tmem_cols);
         tmem_relinquish();
@@ -470,13 +492,10 @@ __global__ void __launch_bounds__(FD_THREADS, 1) first_dw_kernel(const __grid_co
         const int r = threadIdx.x;                                   // 0 .. FD_NP-1
         const int FD_GRP = FD_NP / p.groups;
         const int grp = r / FD_GRP, rg = r - grp * FD_GRP;
-        const int chunks = p.KP >> 3;
-        const int col_items = 128 * chunks;                          // item -> pixel = item % 128, 16-byte chunk = item / 128
         const int C8 = p.Cout >> 3;                                  // 8-channel chunks of a dy row (power of two <= 32)
         const int my_chunk = rg & (C8 - 1);                          // fixed for this thread: FD_GRP % C8 == 0
         const int prow0 = rg / C8, prow_step = FD_GRP / C8;
         const int dchunks = p.dblocks * 16;                          // 8-channel chunks the operand holds (zero padded)
-        const long long HoWo = (long long)p.Ho * p.Wo;
         float bs[8];
 #pragma unroll
         for (int e = 0; e < 8; ++e) bs[e] = 0.f;
@@ -532,28 +551,10 @@ __global__ void __launch_bounds__(FD_THREADS, 1) first_dw_kernel(const __grid_co
                 }
             }
             // col tile: row = pixel of the tile (the forward kernel's operand, read here as MN-major B)
-            for (int it = rg; it < col_items; it += FD_GRP) {
-                const int pr = it & 127, ch = it >> 7;
-                const long long pix = pix0 + pr;
-                int h0 = -(1 << 20), w0 = 0;
-                long long base = 0;
-                if (pix < p.P) {
-                    const long long n = pix / HoWo;
-                    const int rem = (int)(pix - n * HoWo);
-                    const int ho = rem / p.Wo, wo = rem - ho * p.Wo;
-                    h0 = ho * p.sH - p.pH;
-                    w0 = wo * p.sW - p.pW;
-                    base = ((n * p.H + h0) * p.W + w0) * p.Cin;
-                }
-                float v[8];
-#pragma unroll
-                for (int e = 0; e < 8; ++e) {
-                    const int k = ch * 8 + e;
-                    const int hi = h0 + ki_s[k], wi = w0 + kj_s[k];
-                    v[e] = (hi >= 0 && hi < p.H && wi >= 0 && wi < p.W) ? __ldg(p.x + base + koff_s[k]) : 0.f;
-                }
-                const uint4 q = make_uint4(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]), pack_bf16(v[4], v[5]), pack_bf16(v[6], v[7]));
-                *reinterpret_cast<uint4*>(stage + pr * 128 + ((ch ^ (pr & 7)) << 4)) = q;
+            for (int pr = rg; pr < 128; pr += FD_GRP) {
+                float v[KP];
+                first_gather<KP>(taps, first_pixel(p.x, pix0 + pr, p.P, p.H, p.W, p.Cin, p.fH, p.fW, p.sH, p.sW, p.pH, p.pW, p.Ho, p.Wo), v);
+                first_store_row<KP>(stage, pr, v);
             }
             fence_proxy_async_smem();
             mbar_arrive(full_bar(s));
@@ -571,7 +572,7 @@ __global__ void __launch_bounds__(FD_THREADS, 1) first_dw_kernel(const __grid_co
     } else if (warp == FD_PROD_WARPS) {
         // ------------------------------------------------------------------ MMA issuer
         const bool leader = elect_one();
-        const uint32_t idesc = make_idesc(1u, 1u, 1u, 128u, (uint32_t)p.KP);      // A and B MN-major
+        const uint32_t idesc = make_idesc(1u, 1u, 1u, 128u, (uint32_t)KP);      // A and B MN-major
         const uint32_t hi = (uint32_t)(make_smem_desc(0, 0, 1024) >> 32);          // SBO = 8 reduction rows
         const uint32_t a_lbo = ((uint32_t)FT_STAGE_BYTES >> 4) << 16;              // next 64-channel chunk of dy
         int s = 0;
@@ -613,7 +614,7 @@ __global__ void __launch_bounds__(FD_THREADS, 1) first_dw_kernel(const __grid_co
             float* out = p.part + (size_t)blockIdx.x * (p.K + 1) * p.Cout;
             for (int db = 0; db < p.dblocks; ++db) {
                 const int d = db * 128 + q * 32 + lane;
-                for (int cg = 0; cg < p.KP; cg += 32) {
+                for (int cg = 0; cg < KP; cg += 32) {
                     uint32_t v[32];
                     if (any) {
                         tmem_ld_32x32(tmem_base + ((uint32_t)(q * 32) << 16) + db * 64 + cg, v);
@@ -681,13 +682,13 @@ int first_tc_fwd(const AetherConvDesc& d, const float* x, const float* w, const 
     p.ntiles = (int)((p.P + 127) / 128);
     p.stages = 4;
     const int smem = 1024 + NT * 128 + p.stages * FT_STAGE_BYTES + FT_TAIL + FT_STATS_BYTES;
-    static PerDeviceSmem configured[2];
-    if (int rc = stats ? ensure_dynamic_smem(first_conv_kernel<true>, 232448, configured[1], "first_conv")
-                       : ensure_dynamic_smem(first_conv_kernel<false>, 232448, configured[0], "first_conv"))
-        return rc;
-    const int grid = first_tc_grid(p.ntiles);
-    if (stats) launch(first_conv_kernel<true>, grid, FirstCfg<true>::THREADS, smem, st, p);
-    else launch(first_conv_kernel<false>, grid, FirstCfg<false>::THREADS, smem, st, p);
+    using KernelFn = void (*)(const FirstParams);
+    static const KernelFn kernels[2][4] = {{first_conv_kernel<false, 16>, first_conv_kernel<false, 32>, first_conv_kernel<false, 48>, first_conv_kernel<false, 64>},
+                                           {first_conv_kernel<true, 16>, first_conv_kernel<true, 32>, first_conv_kernel<true, 48>, first_conv_kernel<true, 64>}};
+    static PerDeviceSmem configured[2][4];
+    const int ki = KP / 16 - 1, si = stats ? 1 : 0;
+    if (int rc = ensure_dynamic_smem(kernels[si][ki], 232448, configured[si][ki], "first_conv")) return rc;
+    launch(kernels[si][ki], first_tc_grid(p.ntiles), stats ? FirstCfg<true>::THREADS : FirstCfg<false>::THREADS, smem, st, p);
     count_launch();
     return check_launch("first_conv_kernel");
 }
@@ -765,9 +766,12 @@ int first_tc_bwd_filter(const AetherConvDesc& d, const float* x, const float* dy
         p.dy_bf16 = 1;
     }
     const int smem = 1024 + p.stages * p.stage_bytes + tail;
-    static PerDeviceSmem configured;
-    if (int rc0 = ensure_dynamic_smem(first_dw_kernel, 232448, configured, "first_dw")) return rc0;
-    launch(first_dw_kernel, grid, FD_THREADS, smem, st, p);
+    using KernelFn = void (*)(const FirstDwParams);
+    static const KernelFn kernels[4] = {first_dw_kernel<16>, first_dw_kernel<32>, first_dw_kernel<48>, first_dw_kernel<64>};
+    static PerDeviceSmem configured[4];
+    const int ki = KP / 16 - 1;
+    if (int rc0 = ensure_dynamic_smem(kernels[ki], 232448, configured[ki], "first_dw")) return rc0;
+    launch(kernels[ki], grid, FD_THREADS, smem, st, p);
     count_launch();
     int rc = check_launch("first_dw_kernel");
     if (rc) return rc;

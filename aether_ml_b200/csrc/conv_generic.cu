@@ -148,8 +148,8 @@ __global__ void __launch_bounds__(256) head_dx_kernel(const float* __restrict__ 
     }
 }
 
-// dw[c][d] = sum_p x[p][c] * dy[p][d], db[d] = sum_p dy[p][d] over a part of the rows: partials [part][Cin * Cout + Cout]
-// that smallc_reduce_kernel adds up.  A thread keeps four channels x Cout sums; x is read once, coalesced; the row of dy
+// dw[c][d] = sum_p x[p][c] * dy[p][d], db[d] = sum_p dy[p][d] over a part of the rows: partials [part][Cout + 1][Cin]
+// (row Cout: the column sums of dy), d-major so that the threads' stores are whole lines, that head_dw_reduce_kernel adds up.  A thread keeps four channels x Cout sums; x is read once, coalesced; the row of dy
 // is the same address for every thread of a row.  A block is row lanes x four-channel groups (blockIdx.y walks the
 // groups beyond 256) and every row lane writes a part of its own.  Few rows per thread: the loop is a chain of load
 // latencies (4 blocks of 32 rows at batch 128 took 17 us, of which the sums themselves are a small part).
@@ -164,14 +164,13 @@ __global__ void __launch_bounds__(256) head_dw_partial_kernel(const float* __res
     const int c4 = blockIdx.y * groups + gi;
     const int mine = blockIdx.x * lanes + rl;             // this row lane's part: rows mine, mine + parts, ...
     if (rl >= lanes || mine >= parts) return;
-    const int entries = Cin * Cout;
-    float* out = part + (size_t)mine * (entries + Cout);
+    float* out = part + (size_t)mine * (Cout + 1) * Cin;
     if (c4 < C4) {
         float4 acc[MAXD];
 #pragma unroll
         for (int d = 0; d < MAXD; ++d) acc[d] = make_float4(0.f, 0.f, 0.f, 0.f);
         const float4* xp = reinterpret_cast<const float4*>(x) + c4;
-#pragma unroll 2
+#pragma unroll 4
         for (long long r = mine; r < rows; r += parts) {
             const float4 v = xp[(size_t)r * C4];
             const float* gr = dy + (size_t)r * Cout;
@@ -185,18 +184,40 @@ __global__ void __launch_bounds__(256) head_dw_partial_kernel(const float* __res
             }
         }
 #pragma unroll
-        for (int d = 0; d < MAXD; ++d) {
-            if (d < Cout) {
-                out[(size_t)(4 * c4 + 0) * Cout + d] = acc[d].x; out[(size_t)(4 * c4 + 1) * Cout + d] = acc[d].y;
-                out[(size_t)(4 * c4 + 2) * Cout + d] = acc[d].z; out[(size_t)(4 * c4 + 3) * Cout + d] = acc[d].w;
-            }
-        }
+        for (int d = 0; d < MAXD; ++d)
+            if (d < Cout) *reinterpret_cast<float4*>(out + (size_t)d * Cin + 4 * c4) = acc[d];
     }
     if (blockIdx.y == 0 && gi < Cout) {
         float sdy = 0.f;
 #pragma unroll 4
         for (long long r = mine; r < rows; r += parts) sdy += dy[(size_t)r * Cout + gi];
-        out[entries + gi] = sdy;
+        out[(size_t)Cout * Cin + gi] = sdy;
+    }
+}
+
+// dw[c][d] = sum over parts of part[p][d][c], db[d] of part[p][Cout][d]: 32 outputs x 8 lanes per block, fixed order.
+__global__ void __launch_bounds__(256) head_dw_reduce_kernel(const float* __restrict__ part, int parts, int Cin, int Cout,
+                                                             float* __restrict__ dw, float* __restrict__ db) {
+    pdl_wait();
+    __shared__ float red[8][32];
+    const int el = threadIdx.x & 31, ln = threadIdx.x >> 5;
+    const int e = blockIdx.x * 32 + el, total = Cin * Cout + Cout;        // d-major, then the Cout column sums
+    float s = 0.f;
+    if (e < total)
+#pragma unroll 4
+        for (int p = ln; p < parts; p += 8) s += part[(size_t)p * (Cout + 1) * Cin + e];
+    red[ln][el] = s;
+    __syncthreads();
+    if (ln == 0 && e < total) {
+        float t = 0.f;
+#pragma unroll
+        for (int l = 0; l < 8; ++l) t += red[l][el];
+        if (e < Cin * Cout) {
+            const int d = e / Cin, c = e - d * Cin;
+            if (dw) dw[c * Cout + d] = t;
+        } else if (db) {
+            db[e - Cin * Cout] = t;
+        }
     }
 }
 
@@ -269,7 +290,7 @@ static int head_dw_parts(const AetherConvDesc& d) {
 size_t generic_conv_workspace_bytes(const AetherConvDesc& d) {
     const size_t simt = simt_conv_workspace_bytes(d);
     if (!head_shape(d)) return simt;
-    const size_t head = align_up((size_t)head_dw_parts(d) * ((size_t)d.Cin * d.Cout + d.Cout) * sizeof(float), 1024);
+    const size_t head = align_up((size_t)head_dw_parts(d) * (d.Cout + 1) * d.Cin * sizeof(float), 1024);
     return head > simt ? head : simt;
 }
 
@@ -287,7 +308,9 @@ int generic_conv_bwd_filter(const AetherConvDesc& d, const float* x, const float
            d.Cout, lanes, parts);
     count_launch();
     if (int rc = check_launch("head_dw_partial_kernel")) return rc;
-    return smallc_reduce_partials(part, parts, d.Cin, d.Cout, dw, db, st);
+    launch(head_dw_reduce_kernel, ceil_div((d.Cin + 1) * d.Cout, 32), 256, 0, st, part, parts, d.Cin, d.Cout, dw, db);
+    count_launch();
+    return check_launch("head_dw_reduce_kernel");
 }
 
 }  // namespace aether

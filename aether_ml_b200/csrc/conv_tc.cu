@@ -497,6 +497,7 @@ struct DwParams {
     int gpc;             // M groups per CTA
     int n_tiles_n;
     int ldn;
+    int Cin, Cout;       // real channels: rows and columns of padding are not stored
 };
 
 static constexpr int DW_THREADS = 192;
@@ -685,13 +686,14 @@ __global__ void __launch_bounds__(DW_THREADS, 1) dw_conv_kernel(const __grid_con
 #pragma unroll
                         for (int k = 0; k < 32; ++k) r[k] = 0u;
                     }
-                    if (u < p.U) {
+                    if (u < p.U && (u % p.cblocks) * UC + c_in < p.Cin) {
                         float4* dst = reinterpret_cast<float4*>(
                             p.part + (((size_t)split * p.U + u) * UC + c_in) * (size_t)p.ldn + nt * NTP + ch * 32);
 #pragma unroll
                         for (int k = 0; k < 8; ++k)
-                            dst[k] = make_float4(__uint_as_float(r[4 * k]), __uint_as_float(r[4 * k + 1]),
-                                                 __uint_as_float(r[4 * k + 2]), __uint_as_float(r[4 * k + 3]));
+                            if (nt * NTP + ch * 32 + 4 * k < p.Cout)            // (Cout % 4 == 0)
+                                dst[k] = make_float4(__uint_as_float(r[4 * k]), __uint_as_float(r[4 * k + 1]),
+                                                     __uint_as_float(r[4 * k + 2]), __uint_as_float(r[4 * k + 3]));
                     }
                 }
             }
@@ -970,6 +972,7 @@ struct TcPlan {
     // dW decomposition
     int dw_nb, dw_nt, dw_cblocks, dw_U, dw_MG, dw_gpc, dw_ngc, dw_ntn, dw_splits;
     bool dw_pair;     // per-tap dW kernel on CTA pairs: dw_MG / dw_gpc / dw_ntn count pair groups and pair column tiles
+    bool dw_small;    // operands in L2: the per-tap dW kernel with the decomposition chosen for few partials
     int dw_halo_splits;   // most splits the halo dW kernel may write (sizes the partial buffer with dw_splits)
     int db_blocks, db_rows_max;
     PixelTiling til_out;   // tiles over output pixels (forward, dW)
@@ -1092,10 +1095,15 @@ static TcPlan compute_plan(const AetherConvDesc& d) {
             pl.dw_splits = ps;
         }
     }
+    pl.dw_small = false;
     if (!pl.dw_pair && (1LL * d.S * d.H * d.W * pl.Cin_p + 1LL * d.S * pl.Ho * pl.Wo * pl.Cout_p) * pl.elt <= (32LL << 20)) {
         const int s = decompose_small();
-        if (s > 0) pl.dw_splits = s;
-        else decompose(1);
+        if (s > 0) {
+            pl.dw_splits = s;
+            pl.dw_small = true;
+        } else {
+            decompose(1);
+        }
     }
     const long long out_rows = 1LL * d.S * pl.Ho * pl.Wo;
     pl.db_blocks = (int)(out_rows < 4LL * num_sms() * 64 ? (out_rows + 63) / 64 : 4LL * num_sms());
@@ -1442,7 +1450,9 @@ int tc_conv_bwd(const AetherConvDesc& d, const float* x, const float* dy, const 
     // 0.654, 20x20 (2048) 0.474 / 0.452, 16x16 (4096) 0.597 / 0.531, 16x16 256 -> 256 (2048) 0.656 / 0.486,
     // 12x12 (4096) 0.296 / 0.326.
     const bool per_tap_pairs = pl.dw_pair && pl.Wo >= 16 && pl.Wo <= 20;
-    if (dw && !pl.tf32 && !per_tap_pairs) {   // wide images: halo-reuse kernel (every tap re-reads one shared-memory window)
+    // Small layers take the per-tap kernel, too: the window kernels spread one strip per CTA over as many splits as there are
+    // SMs, and the partials cost more than the products (128 images 16x16 32->64: 17 + 7 us against 9 + 4).
+    if (dw && !pl.tf32 && !per_tap_pairs && !pl.dw_small) {   // wide images: halo-reuse kernel (every tap re-reads one shared-memory window)
         int splits = 0;
         float* part = reinterpret_cast<float*>(wsb + pl.off_part);
         int sa = 0, sb = 0, tap_split = 0;
@@ -1482,7 +1492,7 @@ int tc_conv_bwd(const AetherConvDesc& d, const float* x, const float* dy, const 
         p.tiles_w = til.tiles_w; p.tiles_h = til.tiles_h; p.tiles_n = til.tiles_n;
         p.fH = d.fH; p.fW = d.fW; p.padH = d.padH; p.padW = d.padW;
         p.cblocks = pl.dw_cblocks; p.U = pl.dw_U; p.MG = pl.dw_MG; p.gpc = pl.dw_gpc;
-        p.n_tiles_n = pl.dw_ntn; p.ldn = pl.Cout_p;
+        p.n_tiles_n = pl.dw_ntn; p.ldn = pl.Cout_p; p.Cin = d.Cin; p.Cout = d.Cout;
         const int gy = pl.dw_ngc * pl.dw_ntn;
         if (pl.dw_pair) rc = pl.tf32 ? launch_dw<true, 2, true>(p, pl.dw_splits, gy, st) : launch_dw<false, 2, true>(p, pl.dw_splits, gy, st);
         else if (pl.tf32) rc = (pl.dw_nb == 2) ? launch_dw<true, 2, false>(p, pl.dw_splits, gy, st) : launch_dw<true, 1, false>(p, pl.dw_splits, gy, st);
