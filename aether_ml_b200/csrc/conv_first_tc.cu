@@ -4,12 +4,15 @@
 //
 // With 3 input channels a pixel's 12 bytes cannot be the inner extent of a TMA box and K = 27 is less than one
 // 128-byte operand row, so the im2col rows are built by threads: producer warps gather the K input values of
-// 128 output pixels (one pixel per thread), convert them to bf16 and write them as a K-major, 128-byte-swizzled
-// operand tile (16-byte chunk c of row r is stored at chunk c ^ (r % 8)); the filter is laid out the same way once
-// per CTA.  One warp issues K/16 (two for a 3x3 RGB filter) 128 x Cout x 16 MMAs per tile into one of up to four
-// TMEM accumulators; eight epilogue warps add the bias and write 64-byte row segments straight from registers, and
-// optionally accumulate the per-channel statistics the following Batch_Norm needs.  The layer is bound by the HBM
-// write of its output (the CUDA-core version of the same layer, conv_smallc.cu, is bound by its FMAs).
+// 128 output pixels (one pixel per thread, all of a row's loads in flight together), convert them to bf16 and write them
+// as a K-major, 128-byte-swizzled operand tile (16-byte chunk c of row r is stored at chunk c ^ (r % 8)); the filter is
+// laid out the same way once per CTA.  One thread issues K/16 (two for a 3x3 RGB filter) 128 x Cout x 16 MMAs per tile into
+// one of up to four TMEM accumulators.  Two epilogue teams of four warps take alternate tiles: a thread reads 32 columns of
+// its accumulator row, adds the bias and writes them to a swizzled staging tile that TMA stores to global memory; the
+// statistics the following Batch_Norm needs are summed from the staged tile, a column per lane, so neither the exchange of
+// columns between lanes nor their reduction across lanes is left.  A tile costs about 1700 warp instructions at 32 filters
+// (6900 when every value went through shuffles and 64-byte register stores), the layer is bound by the HBM write of its
+// output.
 #include <cuda_bf16.h>
 #include <string.h>
 
@@ -20,29 +23,12 @@
 
 namespace aether {
 
-struct FirstParams {
-    const float* x;
-    const float* w;      // (fH, fW, Cin, Cout) = [K][Cout]
-    const float* bias;   // nullable
-    float* y;
-    float* stats;        // nullable: [cta][3][Cout] (count, mean, M2) partials
-    int* status;
-    int H, W, Cin, Cout, NT, fH, fW, sH, sW, pH, pW, Ho, Wo, K, KP;
-    long long P;         // output pixels
-    int stages, ntiles;
-};
-
-// Producer warps: one or two groups of four that build alternate tiles, a pixel per thread, the next tile's loads in flight
-// while the current one is stored.  One group in the kernel with the statistics epilogue: more than 16 warps would cap
-// every thread at 96 registers, which the statistics' running sums do not fit in.
-static constexpr int FT_EPI_WARPS = 8;
-template <bool STATS> struct FirstCfg {
-    static constexpr int PROD_WARPS = STATS ? 4 : 8;             // groups of four: a thread per pixel of a tile
-    static constexpr int THREADS = 32 * (PROD_WARPS + 1 + FT_EPI_WARPS);   // producers, MMA issuer, epilogue
-};
+static constexpr int FT_PROD_WARPS = 8;                                      // two groups of four that build alternate tiles
+static constexpr int FT_EPI_WARPS = 8;                                       // two teams of four
+static constexpr int FT_THREADS = 32 * (FT_PROD_WARPS + 1 + FT_EPI_WARPS);   // producers, MMA issuer, epilogue
 static constexpr int FT_STAGE_BYTES = 128 * 128;                             // 128 pixel rows of 128 bytes
-static constexpr int FT_TAIL = 2048;                                         // barriers, TMEM pointer, bias, k tables
-static constexpr int FT_STATS_BYTES = FT_EPI_WARPS * STATS_WARP_FLOATS * 4;
+static constexpr int FT_TAIL = 2048;                                         // barriers, TMEM pointer, bias, tap table
+static constexpr int FT_OUT_BYTES = 2 * 2 * FT_STAGE_BYTES;                  // two staging tiles (128 rows x 32 floats) per team
 
 __device__ __forceinline__ void ft_umma(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t hi, uint32_t idesc,
                                         uint32_t accumulate) {
@@ -60,8 +46,8 @@ __device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
 
 // ---- the im2col gather shared by the forward and the filter-gradient kernel.  A thread builds one operand row: the K input
 // values of one output pixel.  All of a row's loads are independent and issued together (a row is one load latency; in
-// pieces of eight values it was three or four of them, each behind a 64-bit division of the pixel index, and the gather
-// took 1.6 us per tile, twice the rest of the kernel).
+// pieces of eight values it was three or four of them, each behind a 64-bit division of the pixel index).  3x3 filters on
+// 1 or 3 channels, the usual first layers, have their offsets at compile time (CIN = 1, 3): two instructions per value.
 struct FirstTaps {                 // entry k of a row: element offset from the window's first value, filter row | column << 8
     int2 t[64];
 };
@@ -70,46 +56,45 @@ __device__ __forceinline__ void first_fill_taps(FirstTaps& tab, int K, int Cin, 
         const int kk = k < K ? k : 0;
         const int tap = kk / Cin, c = kk - tap * Cin;
         const int i = tap / fW, j = tap - i * fW;
-        tab.t[k] = make_int2((i * W + j) * Cin + c, k < K ? i | (j << 8) : 0x3f3f);   // past K: bit 63 of the masks, never set
+        tab.t[k] = make_int2((i * W + j) * Cin + c, k < K ? i | (j << 8) : 0x1f1f);   // past K: bit 31 of the masks, never set
     }
 }
-struct FirstPixel {
-    const float* base;             // the window's first value (may lie before the image: used with valid taps only)
-    unsigned long long rows, cols; // bit i / j: filter row i / column j falls inside the image
+struct FirstGeom {
+    const float* x;
+    int P;                         // output pixels
+    int H, W, Cin, fH, fW, sH, sW, pH, pW, Ho, Wo;
 };
-__device__ __forceinline__ FirstPixel first_pixel(const float* x, long long pix, long long P, int H, int W, int Cin, int fH, int fW, int sH, int sW,
-                                                  int pH, int pW, int Ho, int Wo) {
-    FirstPixel q;
-    q.rows = q.cols = 0ull;
-    q.base = x;
-    if (pix < P) {
-        int n, ho, wo;
-        if (P < (1LL << 31)) {                          // 32-bit divisions are several times cheaper
-            const unsigned u = (unsigned)pix, r = u / (unsigned)Wo;
-            wo = (int)(u - r * (unsigned)Wo);
-            n = (int)(r / (unsigned)Ho);
-            ho = (int)(r - (unsigned)n * (unsigned)Ho);
-        } else {
-            const long long r = pix / Wo, s = r / Ho;
-            wo = (int)(pix - r * Wo);
-            n = (int)s;
-            ho = (int)(r - s * Ho);
-        }
-        const int h0 = ho * sH - pH, w0 = wo * sW - pW;
-        q.base = x + (((long long)n * H + h0) * W + w0) * Cin;
-        // rows i with 0 <= h0 + i < H, columns alike (filters of at most 64 entries)
-        const int i0 = h0 < 0 ? -h0 : 0, i1 = min(fH, H - h0), j0 = w0 < 0 ? -w0 : 0, j1 = min(fW, W - w0);
-        if (i1 > i0) q.rows = (~0ull >> (64 - i1)) & ~((1ull << i0) - 1ull);
-        if (j1 > j0) q.cols = (~0ull >> (64 - j1)) & ~((1ull << j0) - 1ull);
+template <int KP, int CIN>
+__device__ __forceinline__ void first_gather(const FirstGeom& g, const FirstTaps& tab, long long pixel, float (&v)[KP]) {
+    unsigned rows = 0u, cols = 0u;                       // bit i / j: filter row i / column j falls inside the image
+    const float* base = g.x;
+    if (pixel < g.P) {
+        const unsigned u = (unsigned)pixel, r = u / (unsigned)g.Wo, n = r / (unsigned)g.Ho;
+        const int w0 = (int)(u - r * (unsigned)g.Wo) * g.sW - g.pW, h0 = (int)(r - n * (unsigned)g.Ho) * g.sH - g.pH;
+        base = g.x + (((long long)n * g.H + h0) * g.W + w0) * (CIN ? CIN : g.Cin);     // may lie before the image
+        const int i0 = h0 < 0 ? -h0 : 0, i1 = min(g.fH, g.H - h0), j0 = w0 < 0 ? -w0 : 0, j1 = min(g.fW, g.W - w0);
+        if (i1 > i0) rows = (0xffffffffu >> (32 - i1)) & ~((1u << i0) - 1u);           // filters of at most 31 x 31
+        if (j1 > j0) cols = (0xffffffffu >> (32 - j1)) & ~((1u << j0) - 1u);
     }
-    return q;
-}
-template <int KP>
-__device__ __forceinline__ void first_gather(const FirstTaps& tab, const FirstPixel& q, float (&v)[KP]) {
+    if constexpr (CIN > 0) {
+        const long long pitch = (long long)g.W * CIN;
 #pragma unroll
-    for (int k = 0; k < KP; ++k) {
-        const int2 t = tab.t[k];
-        v[k] = ((q.rows >> (t.y & 63)) & (q.cols >> (t.y >> 8)) & 1ull) ? __ldg(q.base + t.x) : 0.f;
+        for (int i = 0; i < 3; ++i) {
+            const float* row = base + i * pitch;
+            const unsigned m = ((rows >> i) & 1u) ? cols : 0u;
+#pragma unroll
+            for (int j = 0; j < 3; ++j)
+#pragma unroll
+                for (int c = 0; c < CIN; ++c) v[(i * 3 + j) * CIN + c] = ((m >> j) & 1u) ? __ldg(row + j * CIN + c) : 0.f;
+        }
+#pragma unroll
+        for (int k = 9 * CIN; k < KP; ++k) v[k] = 0.f;
+    } else {
+#pragma unroll
+        for (int k = 0; k < KP; ++k) {
+            const int2 t = tab.t[k];
+            v[k] = ((rows >> (t.y & 31)) & (cols >> (t.y >> 8)) & 1u) ? __ldg(base + t.x) : 0.f;
+        }
     }
 }
 template <int KP>
@@ -121,16 +106,29 @@ __device__ __forceinline__ void first_store_row(uint8_t* tile, int r, const floa
                        pack_bf16(v[8 * ch + 6], v[8 * ch + 7]));
 }
 
-template <bool STATS, int KP>
-__global__ void __launch_bounds__(FirstCfg<STATS>::THREADS, 1) first_conv_kernel(const __grid_constant__ FirstParams p) {
-    constexpr int FT_PROD_WARPS = FirstCfg<STATS>::PROD_WARPS;
+struct FirstParams {
+    CUtensorMap tm_y;    // output (Cout, P) fp32, box (32 channels, 128 pixels), 128-byte swizzle
+    FirstGeom g;
+    const float* w;      // (fH, fW, Cin, Cout) = [K][Cout]
+    const float* bias;   // nullable
+    float* stats;        // nullable: [cta][3][Cout] (count, mean, M2) partials
+    int* status;
+    int Cout, NT, K;
+    int stages, ntiles;
+};
+
+// Statistics of a column over the rows one thread sums: about the mean of its first tile (no cancellation where a channel's
+// mean is far from zero), running sums in shared memory, [3][chunks][256 epilogue threads].
+template <bool STATS, int KP, int CIN>
+__global__ void __launch_bounds__(FT_THREADS, 1) first_conv_kernel(const __grid_constant__ FirstParams p) {
     extern __shared__ uint8_t smem_raw[];
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t* gen_base = smem_raw + (smem_base - smem_u32(smem_raw));
     const int NT = p.NT, S = p.stages;
     const uint32_t sW = smem_base;                                  // filter: NT rows of 128 bytes
     const uint32_t sA = sW + (uint32_t)NT * 128u;                   // NT is a multiple of 32: stays 1024-byte aligned
-    const uint32_t sBar = sA + (uint32_t)S * FT_STAGE_BYTES;
+    const uint32_t sOut = sA + (uint32_t)S * FT_STAGE_BYTES;
+    const uint32_t sBar = sOut + FT_OUT_BYTES;
     auto full_bar = [&](int s) { return sBar + 8u * s; };
     auto empty_bar = [&](int s) { return sBar + 8u * (S + s); };
     auto tfull_bar = [&](int b) { return sBar + 8u * (2 * S + b); };
@@ -139,12 +137,13 @@ __global__ void __launch_bounds__(FirstCfg<STATS>::THREADS, 1) first_conv_kernel
     volatile uint32_t* tmem_ptr_generic = reinterpret_cast<volatile uint32_t*>(gen_base + (sTmemPtr - smem_base));
     float* bias_s = reinterpret_cast<float*>(gen_base + (sBar - smem_base) + 256);         // NT <= 256 floats
     FirstTaps& taps = *reinterpret_cast<FirstTaps*>(gen_base + (sBar - smem_base) + 256 + 1024);
+    float* stat_s = reinterpret_cast<float*>(gen_base + (sBar - smem_base) + FT_TAIL);     // STATS: 3 * (NT / 32) * 256 + 256 floats
 
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
-    const uint32_t NB = (4 * NT <= 512) ? 4u : (3 * NT <= 512) ? 3u : 2u;
-    const uint32_t need_cols = NB * (uint32_t)NT;
-    const uint32_t tmem_cols = (need_cols <= 32) ? 32u : (need_cols <= 64) ? 64u : (need_cols <= 128) ? 128u : (need_cols <= 256) ? 256u : 512u;
+    const int NB = (4 * NT <= 512) ? 4 : (3 * NT <= 512) ? 3 : 2;
+    const uint32_t need_cols = (uint32_t)(NB * NT);
+    const uint32_t tmem_cols = (need_cols <= 128) ? 128u : (need_cols <= 256) ? 256u : 512u;
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < S; ++s) {
@@ -153,11 +152,12 @@ __global__ void __launch_bounds__(FirstCfg<STATS>::THREADS, 1) first_conv_kernel
         }
         for (int b = 0; b < 4; ++b) {
             mbar_init(tfull_bar(b), 1);
-            mbar_init(tempty_bar(b), FT_EPI_WARPS);
+            mbar_init(tempty_bar(b), 4);
         }
         mbar_fence_init();
+        tma_prefetch_desc(&p.tm_y);
     }
-    first_fill_taps(taps, p.K, p.Cin, p.fW, p.W);
+    if (CIN == 0) first_fill_taps(taps, p.K, p.g.Cin, p.g.fW, p.g.W);
     if (warp == FT_PROD_WARPS) {
         tmem_alloc(sTmemPtr, tmem_cols);
         tmem_relinquish();
@@ -179,7 +179,6 @@ __global__ void __launch_bounds__(FirstCfg<STATS>::THREADS, 1) first_conv_kernel
     fence_proxy_async_smem();
     tc_fence_before();
     __syncthreads();
-
     tc_fence_after();
     const uint32_t tmem_base = *tmem_ptr_generic;
     const int grid = (int)gridDim.x;
@@ -189,215 +188,151 @@ __global__ void __launch_bounds__(FirstCfg<STATS>::THREADS, 1) first_conv_kernel
         constexpr int GROUPS = FT_PROD_WARPS / 4;
         uint8_t* tile_gen = gen_base + (sA - smem_base);
         const int grp = threadIdx.x >> 7, r = threadIdx.x & 127;
-        auto pixel = [&](int t) {
-            return first_pixel(p.x, (long long)t * 128 + r, p.P, p.H, p.W, p.Cin, p.fH, p.fW, p.sH, p.sW, p.pH, p.pW, p.Ho, p.Wo);
-        };
         float v[KP];
         int t = blockIdx.x + grp * grid;
-        if (t < p.ntiles) first_gather<KP>(taps, pixel(t), v);
+        if (t < p.ntiles) first_gather<KP, CIN>(p.g, taps, (long long)t * 128 + r, v);
         for (int it = grp; t < p.ntiles; it += GROUPS) {
             const int s = it % S;
             if (!mbar_wait(empty_bar(s), ((uint32_t)(it / S) & 1u) ^ 1u, p.status, DS_TIMEOUT_EMPTY)) break;
             first_store_row<KP>(tile_gen + s * FT_STAGE_BYTES, r, v);
             fence_proxy_async_smem();                               // generic-proxy writes -> visible to the tensor core
             mbar_arrive(full_bar(s));
-            t += GROUPS * grid;
-            if (t < p.ntiles) first_gather<KP>(taps, pixel(t), v);
+            t += GROUPS * grid;                                     // the next tile's loads are in flight meanwhile
+            if (t < p.ntiles) first_gather<KP, CIN>(p.g, taps, (long long)t * 128 + r, v);
         }
     } else if (warp == FT_PROD_WARPS) {
-        // ------------------------------------------------------------------ MMA issuer
-        const bool leader = elect_one();
-        const uint32_t idesc = make_idesc(1u, 0u, 0u, 128u, (uint32_t)NT);
-        const uint64_t proto = make_smem_desc(0, 16, 1024);
-        const uint32_t hi = (uint32_t)(proto >> 32);
-        const uint32_t lo_proto = (uint32_t)proto;
-        const uint32_t w_lo = lo_proto + ((sW & 0x3FFFFu) >> 4);
-        const uint32_t a_lo0 = lo_proto + ((sA & 0x3FFFFu) >> 4);
-        constexpr int ksteps = KP / 16;
-        int s = 0;
-        uint32_t ph = 0, buf = 0, aph = 0;
-        bool ok = true;
-        for (int t = blockIdx.x; t < p.ntiles && ok; t += grid) {
-            bool w_ok = mbar_wait_spin(tempty_bar(buf), aph ^ 1u, p.status, DS_TIMEOUT_TMEM_EMPTY);
-            w_ok = __all_sync(0xffffffffu, w_ok);
-            if (!w_ok) { ok = false; break; }
-            bool f_ok = mbar_wait_spin(full_bar(s), ph, p.status, DS_TIMEOUT_FULL);
-            f_ok = __all_sync(0xffffffffu, f_ok);
-            if (!f_ok) { ok = false; break; }
-            tc_fence_after();
-            const uint32_t d_tmem = tmem_base + buf * NT;
-            const uint32_t a_lo = a_lo0 + (uint32_t)s * (FT_STAGE_BYTES >> 4);
-            if (leader) {
+        // ------------------------------------------------------------------ MMA issuer (one thread)
+        if (lane == 0) {
+            const uint32_t idesc = make_idesc(1u, 0u, 0u, 128u, (uint32_t)NT);
+            const uint64_t proto = make_smem_desc(0, 16, 1024);
+            const uint32_t hi = (uint32_t)(proto >> 32);
+            const uint32_t lo_proto = (uint32_t)proto;
+            const uint32_t w_lo = lo_proto + ((sW & 0x3FFFFu) >> 4);
+            const uint32_t a_lo0 = lo_proto + ((sA & 0x3FFFFu) >> 4);
+            constexpr int ksteps = KP / 16;
+            int it = 0;
+            for (int t = blockIdx.x; t < p.ntiles; t += grid, ++it) {
+                const int s = it % S, buf = it % NB;
+                if (!mbar_wait(tempty_bar(buf), ((uint32_t)(it / NB) & 1u) ^ 1u, p.status, DS_TIMEOUT_TMEM_EMPTY)) break;
+                if (!mbar_wait(full_bar(s), (uint32_t)(it / S) & 1u, p.status, DS_TIMEOUT_FULL)) break;
+                tc_fence_after();
+                const uint32_t d_tmem = tmem_base + (uint32_t)(buf * NT);
+                const uint32_t a_lo = a_lo0 + (uint32_t)s * (FT_STAGE_BYTES >> 4);
+#pragma unroll
                 for (int ks = 0; ks < ksteps; ++ks) ft_umma(d_tmem, a_lo + 2u * ks, w_lo + 2u * ks, hi, idesc, ks ? 1u : 0u);
                 umma_commit(empty_bar(s));
                 umma_commit(tfull_bar(buf));
             }
-            if (++s == S) { s = 0; ph ^= 1u; }
-            if (++buf == NB) { buf = 0; aph ^= 1u; }
-            __syncwarp();
         }
     } else {
-        // ------------------------------------------------------------------ epilogue (same scheme as conv_halo.cu)
-        const int ew = warp - FT_PROD_WARPS - 1;
+        // ------------------------------------------------------------------ epilogue
+        const int et = threadIdx.x - 32 * (FT_PROD_WARPS + 1);       // 0 .. 255
+        const int team = et >> 7, tt = et & 127;
         const int q = warp & 3;                                      // TMEM lane quarter this warp may access
-        const int half = ew >> 2;
-        const int ncols = NT >> 1;
-        const int col_begin = half * ncols;
-        const int trow = lane >> 2, tcol4 = (lane & 3) * 4;
-        const bool lo2 = (lane & 2) == 0, odd = (lane & 1) != 0;
-        const bool all_cols = (p.Cout == NT);
-        float* stat_w = reinterpret_cast<float*>(gen_base + (sBar - smem_base) + FT_TAIL) + ew * STATS_WARP_FLOATS;
+        const int row = q * 32 + lane;                               // accumulator row of this thread
+        const int NC = NT >> 5;
+        // statistics: this thread sums column `lane` of every chunk over rows [32 * part, 32 * part + 32)
+        const int part = tt >> 5;
         float st_rows = 0.f;
-        if (STATS) {
-            for (int i = lane; i < STATS_WARP_FLOATS; i += 32) stat_w[i] = 0.f;
-            __syncwarp();
-        }
-        int row_in_tile[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) row_in_tile[j] = q * 32 + (j >> 1) * 16 + trow + (j & 1) * 8;
-        const float* bias4 = bias_s + col_begin + tcol4;
-        const f32x2 one2 = pack2(1.f, 1.f);
-        // Statistics: per-thread sums of its (4 rows x 4 columns) cells per 16-column group.  With one column batch
-        // per tile (ncols <= 64) they run over all tiles of the CTA and the lanes are combined once at the end --
-        // the epilogue is this kernel's critical path, and a per-tile lane reduction doubles its length.
-        const bool persist = ncols <= 64;
-        Stats4 st[4];                              // packed running sums of this thread's four 16-column groups
-#pragma unroll
-        for (int u = 0; u < 4; ++u) st[u].clear();
-        // adds the lanes with equal lane%4 (same 4 columns, 8 row groups) and accumulates into the warp's sums
-        // (about the columns' pivots, see stats_epilogue.cuh; `first`: the sums are the warp's first tile, taken
-        // without pivots, which are set from them)
-        auto flush_stats = [&](int cb, bool first, float rows) {
-            float4 st_s[4], st_q[4];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) { st_s[u] = st[u].sum(); st_q[u] = st[u].sumsq(); }
-#pragma unroll
-            for (int m = 4; m <= 16; m <<= 1) {
-#pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    st_s[u].x += __shfl_xor_sync(0xffffffffu, st_s[u].x, m); st_s[u].y += __shfl_xor_sync(0xffffffffu, st_s[u].y, m);
-                    st_s[u].z += __shfl_xor_sync(0xffffffffu, st_s[u].z, m); st_s[u].w += __shfl_xor_sync(0xffffffffu, st_s[u].w, m);
-                    st_q[u].x += __shfl_xor_sync(0xffffffffu, st_q[u].x, m); st_q[u].y += __shfl_xor_sync(0xffffffffu, st_q[u].y, m);
-                    st_q[u].z += __shfl_xor_sync(0xffffffffu, st_q[u].z, m); st_q[u].w += __shfl_xor_sync(0xffffffffu, st_q[u].w, m);
-                }
-            }
-            if (lane < 4) {
-#pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    const int cc = cb + u * 16;
-                    if (cc < ncols) stats_fold(stat_w, cc + tcol4, st_s[u], st_q[u], first, rows);
-                }
-            }
-            if (first) __syncwarp();               // the pivots must be visible to the whole warp before its next tile
-        };
-        uint32_t buf = 0, aph = 0;
+        float* st = stat_s + et;
+        uint8_t* out_gen = gen_base + (sOut - smem_base) + team * 2 * FT_STAGE_BYTES;
+        const uint32_t out_u = sOut + (uint32_t)(team * 2 * FT_STAGE_BYTES);
+        int cnt = 0, it = team;
         bool ok = true;
-        for (int t = blockIdx.x; t < p.ntiles && ok; t += grid) {
-            float* rowp[4];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const long long pix = (long long)t * 128 + row_in_tile[j];
-                rowp[j] = pix < p.P ? p.y + (size_t)pix * p.Cout + col_begin + tcol4 : nullptr;
-            }
-            float tile_rows = 0.f;                 // valid rows of this tile in this warp's quarter
-            if (STATS) {
-#pragma unroll
-                for (int j = 0; j < 4; ++j) tile_rows += (rowp[j] != nullptr) ? 1.f : 0.f;
-                tile_rows += __shfl_xor_sync(0xffffffffu, tile_rows, 4);
-                tile_rows += __shfl_xor_sync(0xffffffffu, tile_rows, 8);
-                tile_rows += __shfl_xor_sync(0xffffffffu, tile_rows, 16);
-            }
-            const bool first_stats = STATS && st_rows == 0.f && tile_rows > 0.f;      // the tile that sets the pivots
-            if (!mbar_wait(tfull_bar(buf), aph, p.status, DS_TIMEOUT_TMEM_FULL)) { ok = false; break; }
+        for (int t = blockIdx.x + team * grid; t < p.ntiles && ok; t += 2 * grid, it += 2) {
+            const int buf = it % NB;
+            bool mine = mbar_wait(tfull_bar(buf), (uint32_t)(it / NB) & 1u, p.status, DS_TIMEOUT_TMEM_FULL);
             tc_fence_after();
-            const uint32_t taddr0 = tmem_base + ((uint32_t)(q * 32) << 16) + buf * NT + col_begin;
-#pragma unroll 1
-            for (int cb0 = 0; cb0 < ncols; cb0 += 64) {
-                if (STATS && !persist) {
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) st[u].clear();
-                }
-                // two half batches of 2 x 16 columns: 32 accumulator registers in flight beside the running sums
-#pragma unroll
-                for (int hb = 0; hb < 2; ++hb) {
-                    const int cb = cb0 + hb * 32;
-                    if (cb >= ncols) break;
-                    uint32_t v[2][2][8];
-#pragma unroll
-                    for (int u = 0; u < 2; ++u) {
-                        if (cb + u * 16 < ncols) {
-                            tmem_ld_16x256b_x2(taddr0 + cb + u * 16, v[0][u]);
-                            tmem_ld_16x256b_x2(taddr0 + (16u << 16) + cb + u * 16, v[1][u]);
-                        }
-                    }
+            const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * NT);
+            const int left = p.g.P - t * 128;                        // rows of this tile
+            const int r0 = part * 32, nr = STATS ? max(0, min(32, left - r0)) : 0;
+            for (int ch = 0; ch < NC; ++ch, ++cnt) {
+                uint8_t* o = out_gen + (cnt & 1) * FT_STAGE_BYTES;
+                if (mine) {
+                    uint32_t v[32];
+                    tmem_ld_32x32(taddr + ch * 32, v);
                     tmem_ld_wait();
-                    if (cb + 32 >= ncols) {                       // accumulator fully read by this warp
+                    if (ch == NC - 1) {                               // accumulator fully read by this warp
                         tc_fence_before();
                         __syncwarp();
                         if (lane == 0) mbar_arrive(tempty_bar(buf));
                     }
 #pragma unroll
-                    for (int u = 0; u < 2; ++u) {
-                        if (cb + u * 16 < ncols) {
-                            const int cc = cb + u * 16;
-                            const int g = hb * 2 + u;             // 16-column group within the 64-column batch
-                            const float4 b4 = *reinterpret_cast<const float4*>(bias4 + cc);
-                            const bool cols_ok = all_cols || col_begin + tcol4 + cc < p.Cout;
-                            f32x2 npv01 = 0ull, npv23 = 0ull;             // minus the pivots of this lane's four columns
-                            if (STATS) {
-                                const float4 pv = *reinterpret_cast<const float4*>(stat_w + 256 + cc + tcol4);
-                                npv01 = pack2(-pv.x, -pv.y);
-                                npv23 = pack2(-pv.z, -pv.w);
-                            }
-#pragma unroll
-                            for (int j = 0; j < 4; ++j) {
-                                // quad exchange: 2+2 columns per lane -> 4 consecutive columns per lane (64-byte row segments)
-                                const uint32_t a0 = v[j >> 1][u][(j & 1) * 2 + 0], a1 = v[j >> 1][u][(j & 1) * 2 + 1];
-                                const uint32_t b0 = v[j >> 1][u][4 + (j & 1) * 2 + 0], b1 = v[j >> 1][u][4 + (j & 1) * 2 + 1];
-                                const uint32_t s0 = lo2 ? b0 : a0, s1 = lo2 ? b1 : a1;
-                                const uint32_t r0 = __shfl_xor_sync(0xffffffffu, s0, 2), r1 = __shfl_xor_sync(0xffffffffu, s1, 2);
-                                const uint32_t x0 = lo2 ? a0 : r0, x1 = lo2 ? a1 : r1;
-                                const uint32_t y0 = lo2 ? r0 : b0, y1 = lo2 ? r1 : b1;
-                                const uint32_t t0 = odd ? x0 : y0, t1 = odd ? x1 : y1;
-                                const uint32_t q0 = __shfl_xor_sync(0xffffffffu, t0, 1), q1 = __shfl_xor_sync(0xffffffffu, t1, 1);
-                                float4 a;
-                                a.x = __uint_as_float(odd ? q0 : x0);
-                                a.y = __uint_as_float(odd ? q1 : x1);
-                                a.z = __uint_as_float(odd ? y0 : q0);
-                                a.w = __uint_as_float(odd ? y1 : q1);
-                                const bool wr = cols_ok && rowp[j] != nullptr;
-                                if (wr)
-                                    __stcs(reinterpret_cast<float4*>(rowp[j] + cc),
-                                           make_float4(a.x + b4.x, a.y + b4.y, a.z + b4.z, a.w + b4.w));
-                                if (STATS) {
-                                    // rows past the last pixel hold zeros (their operand rows are zero): a product with
-                                    // the row's 0/1 factor removes them from the sums
-                                    const f32x2 m2 = (cols_ok && rowp[j] != nullptr) ? one2 : 0ull;
-                                    st[g].add(mul2(add2(pack2(a.x, a.y), npv01), m2), mul2(add2(pack2(a.z, a.w), npv23), m2));
-                                }
-                            }
-                        }
+                    for (int c4 = 0; c4 < 8; ++c4) {
+                        const float4 b = *reinterpret_cast<const float4*>(bias_s + ch * 32 + 4 * c4);
+                        *reinterpret_cast<float4*>(o + row * 128 + ((c4 ^ (row & 7)) << 4)) =
+                            make_float4(__uint_as_float(v[4 * c4]) + b.x, __uint_as_float(v[4 * c4 + 1]) + b.y,
+                                        __uint_as_float(v[4 * c4 + 2]) + b.z, __uint_as_float(v[4 * c4 + 3]) + b.w);
                     }
+                    fence_proxy_async_smem();
                 }
-                if (STATS) {
-                    // the first tile is always folded at once (it sets the pivots); with running per-thread sums the
-                    // other tiles are folded together after the last one
-                    if (!persist || first_stats) {
-                        flush_stats(cb0, first_stats, tile_rows);
-                        if (persist) {
+                if (tt == 0) tma_store_wait_read<0>();                   // the other staging tile is free again
+                ok = named_bar_and(1 + team, 128, mine);              // the tile is staged; a failed wait ends the whole team
+                if (!ok) break;
+                if (tt == 0) {
+                    tma_store_2d(&p.tm_y, out_u + (uint32_t)((cnt & 1) * FT_STAGE_BYTES), ch * 32, t * 128);
+                    tma_store_commit();
+                }
+                if (STATS && nr > 0) {
+                    const uint8_t* col = o + (lane & 3) * 4;
+                    float piv, s = 0.f, sq = 0.f;
+                    float* sp = st + ch * 256;
+                    if (st_rows == 0.f) {                             // first tile: its mean becomes the pivot
+                        float m = 0.f;
+                        for (int r = r0; r < r0 + nr; ++r) m += *reinterpret_cast<const float*>(col + r * 128 + (((lane >> 2) ^ (r & 7)) << 4));
+                        piv = m / (float)nr;
+                        sp[2 * NC * 256] = piv;
+                    } else {
+                        piv = sp[2 * NC * 256];
+                        s = sp[0];
+                        sq = sp[NC * 256];
+                    }
+                    if (nr == 32) {
 #pragma unroll
-                            for (int u = 0; u < 4; ++u) st[u].clear();
+                        for (int r = 0; r < 32; ++r) {
+                            const float d = *reinterpret_cast<const float*>(col + (r0 + r) * 128 + (((lane >> 2) ^ (r & 7)) << 4)) - piv;
+                            s += d;
+                            sq = fmaf(d, d, sq);
+                        }
+                    } else {
+                        for (int r = r0; r < r0 + nr; ++r) {
+                            const float d = *reinterpret_cast<const float*>(col + r * 128 + (((lane >> 2) ^ (r & 7)) << 4)) - piv;
+                            s += d;
+                            sq = fmaf(d, d, sq);
                         }
                     }
+                    sp[0] = s;
+                    sp[NC * 256] = sq;
                 }
             }
-            st_rows += tile_rows;
-            if (++buf == NB) { buf = 0; aph ^= 1u; }
+            st_rows += (float)nr;
         }
-        if (STATS && persist) flush_stats(0, false, 0.f);
-        if (STATS)
-            stats_merge_store(reinterpret_cast<float*>(gen_base + (sBar - smem_base) + FT_TAIL), ew, lane, st_rows, ncols, 0, p.Cout, bias_s,
-                              p.stats + (size_t)blockIdx.x * 3 * p.Cout);
+        if (tt == 0) tma_store_wait_all<0>();
+        if (STATS) {
+            // one (count, mean, M2) row per CTA: the eight threads of a column merged in fixed order
+            float* rows_s = stat_s + 3 * NC * 256;
+            rows_s[et] = st_rows;
+            named_bar_sync(3, 256);
+            float* sp = p.stats + (size_t)blockIdx.x * 3 * p.Cout;
+            for (int col = et; col < p.Cout; col += 256) {
+                float N = 0.f, M = 0.f, M2 = 0.f;
+#pragma unroll
+                for (int k = 0; k < 8; ++k) {
+                    const int th = k * 32 + (col & 31);
+                    const float n = rows_s[th];
+                    if (n == 0.f) continue;
+                    const float* a = stat_s + (col >> 5) * 256 + th;
+                    const float s = a[0], m = s / n, m2 = fmaxf(a[NC * 256] - s * m, 0.f), mean = a[2 * NC * 256] + m;
+                    const float tot = N + n, delta = mean - M;
+                    M2 += m2 + delta * delta * N * n / tot;
+                    M += delta * n / tot;
+                    N = tot;
+                }
+                sp[col] = N;
+                sp[p.Cout + col] = M;
+                sp[2 * p.Cout + col] = M2;
+            }
+        }
     }
 
     tc_fence_before();
@@ -416,11 +351,11 @@ __global__ void __launch_bounds__(FirstCfg<STATS>::THREADS, 1) first_conv_kernel
 // the dy tile converted from fp32 to bf16; they also keep the fp32 column sums of dy for db.  The accumulators stay
 // in TMEM for the CTA's whole life; one partial per CTA, summed in fixed order by smallc_reduce_kernel.
 struct FirstDwParams {
-    const float* x;
+    FirstGeom g;
     const float* dy;
     float* part;         // [cta][K + 1][Cout]
     int* status;
-    int H, W, Cin, Cout, fH, fW, sH, sW, pH, pW, Ho, Wo, K, KP;
+    int Cout, K, KP;
     int dblocks;         // 128-channel blocks of dy
     long long P;
     int stages, ntiles, stage_bytes;
@@ -443,7 +378,7 @@ static constexpr int FD_ROWS = 6;                                            // 
 static constexpr int FD_TAIL = 1024 + FD_NP * 8 * 4 + 1024;                  // barriers, k tables, dB staging
 static constexpr int FD_THREADS = 32 * (FD_PROD_WARPS + 1 + 4);              // producers, MMA issuer, 4 epilogue warps
 
-template <int KP>
+template <int KP, int CIN>
 __global__ void __launch_bounds__(FD_THREADS, 1) first_dw_kernel(const __grid_constant__ FirstDwParams p) {
     extern __shared__ uint8_t smem_raw[];
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -471,7 +406,7 @@ __global__ void __launch_bounds__(FD_THREADS, 1) first_dw_kernel(const __grid_co
         mbar_fence_init();
         if (p.dy_bf16) tma_prefetch_desc(&p.tm_dy);
     }
-    first_fill_taps(taps, p.K, p.Cin, p.fW, p.W);
+    if (CIN == 0) first_fill_taps(taps, p.K, p.g.Cin, p.g.fW, p.g.W);
     if (warp == FD_PROD_WARPS) {
         tmem_alloc(sTmemPtr, tmem_cols);
         tmem_relinquish();
@@ -553,7 +488,7 @@ __global__ void __launch_bounds__(FD_THREADS, 1) first_dw_kernel(const __grid_co
             // col tile: row = pixel of the tile (the forward kernel's operand, read here as MN-major B)
             for (int pr = rg; pr < 128; pr += FD_GRP) {
                 float v[KP];
-                first_gather<KP>(taps, first_pixel(p.x, pix0 + pr, p.P, p.H, p.W, p.Cin, p.fH, p.fW, p.sH, p.sW, p.pH, p.pW, p.Ho, p.Wo), v);
+                first_gather<KP, CIN>(p.g, taps, pix0 + pr, v);
                 first_store_row<KP>(stage, pr, v);
             }
             fence_proxy_async_smem();
@@ -645,14 +580,14 @@ __global__ void __launch_bounds__(FD_THREADS, 1) first_dw_kernel(const __grid_co
 static bool first_tc_shape(const AetherConvDesc& d, int& K, int& KP, int& NT, int& Ho, int& Wo) {
     if (d.math_mode != AETHER_MATH_BF16) return false;
     K = d.fH * d.fW * d.Cin;
-    if (d.Cin > 4 || K > 64) return false;
+    if (d.Cin > 4 || K > 64 || d.fH > 31 || d.fW > 31) return false;
     if (d.Cout % 4 || d.Cout < 16 || d.Cout > 256) return false;
     KP = (K + 15) / 16 * 16;
-    NT = (d.Cout + 31) / 32 * 32;              // two column halves of 16-column groups; filter rows fill whole 8-row atoms
+    NT = (d.Cout + 31) / 32 * 32;              // whole 32-column chunks
     conv_out_hw(d, Ho, Wo);
     if (Ho < 1 || Wo < 1) return false;
     const long long P = 1LL * d.S * Ho * Wo;
-    return (P + 127) / 128 < 0x7fffffffLL && 1LL * d.S * d.H * d.W * d.Cin < (1LL << 40);
+    return P < 0x7fffff00LL;                   // pixel indices and TMA coordinates are 32-bit
 }
 
 bool first_tc_eligible(const AetherConvDesc& d) {
@@ -669,26 +604,39 @@ long long first_tc_stats_blocks(const AetherConvDesc& d) {
     return first_tc_grid((P + 127) / 128);
 }
 
+static FirstGeom first_geom(const AetherConvDesc& d, const float* x, int Ho, int Wo) {
+    return FirstGeom{x, (int)(1LL * d.S * Ho * Wo), d.H, d.W, d.Cin, d.fH, d.fW, d.sH, d.sW, d.padH, d.padW, Ho, Wo};
+}
+// Kernel variant: 3x3 filters on 1 or 3 channels at compile time, else the tap table at K padded to 16, 32, 48, 64.
+static int first_variant(const AetherConvDesc& d, int KP) {
+    if (d.fH == 3 && d.fW == 3 && d.Cin == 1) return 4;
+    if (d.fH == 3 && d.fW == 3 && d.Cin == 3) return 5;
+    return KP / 16 - 1;
+}
+
 int first_tc_fwd(const AetherConvDesc& d, const float* x, const float* w, const float* b, float* y, float* stats,
                  cudaStream_t st) {
     int K, KP, NT, Ho, Wo;
     if (!first_tc_shape(d, K, KP, NT, Ho, Wo)) return set_error(AE_UNSUPPORTED, "first_tc_fwd: shape not supported");
     FirstParams p;
     memset(&p, 0, sizeof(p));
-    p.x = x; p.w = w; p.bias = b; p.y = y; p.stats = stats; p.status = device_status_word();
-    p.H = d.H; p.W = d.W; p.Cin = d.Cin; p.Cout = d.Cout; p.NT = NT; p.fH = d.fH; p.fW = d.fW; p.sH = d.sH; p.sW = d.sW;
-    p.pH = d.padH; p.pW = d.padW; p.Ho = Ho; p.Wo = Wo; p.K = K; p.KP = KP;
-    p.P = 1LL * d.S * Ho * Wo;
-    p.ntiles = (int)((p.P + 127) / 128);
+    p.g = first_geom(d, x, Ho, Wo);
+    p.w = w; p.bias = b; p.stats = stats; p.status = device_status_word();
+    p.Cout = d.Cout; p.NT = NT; p.K = K;
+    p.ntiles = (p.g.P + 127) / 128;
     p.stages = 4;
-    const int smem = 1024 + NT * 128 + p.stages * FT_STAGE_BYTES + FT_TAIL + FT_STATS_BYTES;
+    if (int rc = make_map_2d(&p.tm_y, y, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, d.Cout, p.g.P, 32, 128)) return rc;
+    const int stat_bytes = stats ? (3 * (NT / 32) * 256 + 256) * 4 : 0;
+    const int smem = 1024 + NT * 128 + p.stages * FT_STAGE_BYTES + FT_OUT_BYTES + FT_TAIL + stat_bytes;
     using KernelFn = void (*)(const FirstParams);
-    static const KernelFn kernels[2][4] = {{first_conv_kernel<false, 16>, first_conv_kernel<false, 32>, first_conv_kernel<false, 48>, first_conv_kernel<false, 64>},
-                                           {first_conv_kernel<true, 16>, first_conv_kernel<true, 32>, first_conv_kernel<true, 48>, first_conv_kernel<true, 64>}};
-    static PerDeviceSmem configured[2][4];
-    const int ki = KP / 16 - 1, si = stats ? 1 : 0;
+    static const KernelFn kernels[2][6] = {{first_conv_kernel<false, 16, 0>, first_conv_kernel<false, 32, 0>, first_conv_kernel<false, 48, 0>,
+                                            first_conv_kernel<false, 64, 0>, first_conv_kernel<false, 16, 1>, first_conv_kernel<false, 32, 3>},
+                                           {first_conv_kernel<true, 16, 0>, first_conv_kernel<true, 32, 0>, first_conv_kernel<true, 48, 0>,
+                                            first_conv_kernel<true, 64, 0>, first_conv_kernel<true, 16, 1>, first_conv_kernel<true, 32, 3>}};
+    static PerDeviceSmem configured[2][6];
+    const int ki = first_variant(d, KP), si = stats ? 1 : 0;
     if (int rc = ensure_dynamic_smem(kernels[si][ki], 232448, configured[si][ki], "first_conv")) return rc;
-    launch(kernels[si][ki], first_tc_grid(p.ntiles), stats ? FirstCfg<true>::THREADS : FirstCfg<false>::THREADS, smem, st, p);
+    launch(kernels[si][ki], first_tc_grid(p.ntiles), FT_THREADS, smem, st, p);
     count_launch();
     return check_launch("first_conv_kernel");
 }
@@ -742,9 +690,9 @@ int first_tc_bwd_filter(const AetherConvDesc& d, const float* x, const float* dy
         return set_error(AE_UNSUPPORTED, "first_tc_bwd_filter: shape not supported");
     FirstDwParams p;
     memset(&p, 0, sizeof(p));
-    p.x = x; p.dy = dy; p.part = static_cast<float*>(ws); p.status = device_status_word();
-    p.H = d.H; p.W = d.W; p.Cin = d.Cin; p.Cout = d.Cout; p.fH = d.fH; p.fW = d.fW; p.sH = d.sH; p.sW = d.sW;
-    p.pH = d.padH; p.pW = d.padW; p.Ho = Ho; p.Wo = Wo; p.K = K; p.KP = KP;
+    p.g = first_geom(d, x, Ho, Wo);
+    p.dy = dy; p.part = static_cast<float*>(ws); p.status = device_status_word();
+    p.Cout = d.Cout; p.K = K; p.KP = KP;
     p.dblocks = (d.Cout + 127) / 128;
     p.P = 1LL * d.S * Ho * Wo;
     p.ntiles = (int)((p.P + 127) / 128);
@@ -767,9 +715,10 @@ int first_tc_bwd_filter(const AetherConvDesc& d, const float* x, const float* dy
     }
     const int smem = 1024 + p.stages * p.stage_bytes + tail;
     using KernelFn = void (*)(const FirstDwParams);
-    static const KernelFn kernels[4] = {first_dw_kernel<16>, first_dw_kernel<32>, first_dw_kernel<48>, first_dw_kernel<64>};
-    static PerDeviceSmem configured[4];
-    const int ki = KP / 16 - 1;
+    static const KernelFn kernels[6] = {first_dw_kernel<16, 0>, first_dw_kernel<32, 0>, first_dw_kernel<48, 0>,
+                                        first_dw_kernel<64, 0>, first_dw_kernel<16, 1>, first_dw_kernel<32, 3>};
+    static PerDeviceSmem configured[6];
+    const int ki = first_variant(d, KP);
     if (int rc0 = ensure_dynamic_smem(kernels[ki], 232448, configured[ki], "first_dw")) return rc0;
     launch(kernels[ki], grid, FD_THREADS, smem, st, p);
     count_launch();
