@@ -328,9 +328,9 @@ __global__ void __launch_bounds__(256) chain_fwd_kernel(const float* __restrict_
                 const size_t cell = first + ((size_t)i * W + j) * C4;
                 const float4 v = F ? pre[F ? i * F + j : 0] : reinterpret_cast<const float4*>(x)[cell];
                 float4 o = make_float4(fmaf(v.x, s.x, t.x), fmaf(v.y, s.y, t.y), fmaf(v.z, s.z, t.z), fmaf(v.w, s.w, t.w));
-                reinterpret_cast<float4*>(bn)[cell] = o;
+                if (bn != nullptr) reinterpret_cast<float4*>(bn)[cell] = o;
                 o = make_float4(lrelu(o.x, alpha), lrelu(o.y, alpha), lrelu(o.z, alpha), lrelu(o.w, alpha));
-                reinterpret_cast<float4*>(act)[cell] = o;
+                if (act != nullptr) reinterpret_cast<float4*>(act)[cell] = o;
                 if (drop != nullptr) {
                     if (mask != nullptr) o = make_float4(o.x * k4.x, o.y * k4.y, o.z * k4.z, o.w * k4.w);
                     reinterpret_cast<float4*>(drop)[cell] = o;
@@ -348,7 +348,7 @@ __global__ void __launch_bounds__(256) chain_fwd_kernel(const float* __restrict_
         if (pooled != nullptr && whole) {
             const size_t opix = ((size_t)smp * Ho + ho) * Wo + wo;
             reinterpret_cast<float4*>(pooled)[opix * C4 + cv] = best;
-            reinterpret_cast<uchar4*>(arg)[opix * C4 + cv] = code;
+            if (arg != nullptr) reinterpret_cast<uchar4*>(arg)[opix * C4 + cv] = code;
             if (copy != nullptr) store_operand_copy(copy, copy_ld, opix, (int)cv, C4, best);
         } else if (pooled == nullptr && copy != nullptr) {
             store_operand_copy(copy, copy_ld, first / C4, (int)cv, C4, best);
@@ -669,8 +669,8 @@ extern "C" int aether_chain_fwd(const float* x, const float* partials, int64_t n
                                 float* act_out, float* drop_out, float* pooled, uint8_t* argmax, int S, int H, int W, int C, int fH,
                                 int fW, float eps, float momentum, float alpha, const float* mask, int training, void* operand_copy,
                                 int copy_ld, void* ws, size_t ws_bytes, void* stream) {
-    if (!x || !gamma || !beta || !running_mean || !running_var || !bn_out || !act_out || (pooled && !argmax) || !ws ||
-        (training && (!batch_mean || !batch_var)) || (mask && !drop_out))
+    if (!x || !gamma || !beta || !running_mean || !running_var || !ws || (mask && !drop_out) ||
+        (training ? (!batch_mean || !batch_var || !bn_out || !act_out || (pooled && !argmax)) : (!act_out && !drop_out && !pooled)))
         return set_error(AE_BAD_ARG, "aether_chain_fwd: null pointer");
     if (S <= 0 || H <= 0 || W <= 0 || C <= 0 || fH <= 0 || fW <= 0 || (!pooled && (fH != 1 || fW != 1)))
         return set_error(AE_BAD_ARG, "aether_chain_fwd: bad dimension");
@@ -678,8 +678,8 @@ extern "C" int aether_chain_fwd(const float* x, const float* partials, int64_t n
     const long long items = 1LL * S * ceil_div(H, fH) * ceil_div(W, fW) * (C / 4);
     if (C % 4 || fH * fW > 255 || items >= (1LL << 32) - (1LL << 22))
         return set_error(AE_UNSUPPORTED, "aether_chain_fwd: needs C %% 4 == 0, windows of at most 255 cells, 32-bit window indices");
-    if (!aligned16(x) || !aligned16(bn_out) || !aligned16(act_out) || (drop_out && !aligned16(drop_out)) || (pooled && !aligned16(pooled)) ||
-        !aligned16(gamma) || !aligned16(beta) || !aligned16(running_mean) || !aligned16(running_var) || (mask && !aligned16(mask)) || !aligned16(ws) ||
+    if (!aligned16(x) || (bn_out && !aligned16(bn_out)) || (act_out && !aligned16(act_out)) || (drop_out && !aligned16(drop_out)) ||
+        (pooled && !aligned16(pooled)) || !aligned16(gamma) || !aligned16(beta) || !aligned16(running_mean) || !aligned16(running_var) || (mask && !aligned16(mask)) || !aligned16(ws) ||
         (argmax && (reinterpret_cast<uintptr_t>(argmax) & 3)))
         return set_error(AE_BAD_ARG, "aether_chain_fwd: arrays must be 16-byte aligned (argmax: 4)");
     if (operand_copy && (copy_ld < C || copy_ld % 4 || (reinterpret_cast<uintptr_t>(operand_copy) & 7)))

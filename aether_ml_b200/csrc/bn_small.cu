@@ -19,20 +19,30 @@ namespace aether {
 static constexpr int BNS_THREADS = 512, BNS_WARPS = BNS_THREADS / 32, BNS_LANES = BNS_THREADS / 8;
 
 // Sums of NQ quantities over the partial rows for the 32 channels of this CTA: out[q][channel] in shared memory.
-// f(row, channel, values[NQ]) reads one partial row.
+// f(entries, values[NQ]) turns the NQ entries of one partial row into what is summed.
 template <int NQ, typename F>
-__device__ __forceinline__ void merge_partials(double (*red)[BNS_WARPS][32], int nblocks, int c, bool c_ok, F f) {
+__device__ __forceinline__ void merge_partials(double (*red)[BNS_WARPS][32], const float* __restrict__ part, int nblocks, int C, int c,
+                                               bool c_ok, F f) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    constexpr int U = 5;                                 // rows in flight per warp (148 rows: two round trips to L2)
     double s[NQ];
 #pragma unroll
     for (int q = 0; q < NQ; ++q) s[q] = 0.0;
     if (c_ok)
-#pragma unroll 4
-        for (int b = warp; b < nblocks; b += BNS_WARPS) {
-            double v[NQ];
-            f(b, c, v);
+        for (int b = warp; b < nblocks; b += U * BNS_WARPS) {
+            float t[U][NQ];
 #pragma unroll
-            for (int q = 0; q < NQ; ++q) s[q] += v[q];
+            for (int u = 0; u < U; ++u)
+#pragma unroll
+                for (int q = 0; q < NQ; ++q)
+                    t[u][q] = b + u * BNS_WARPS < nblocks ? part[((size_t)(b + u * BNS_WARPS) * NQ + q) * C + c] : 0.f;
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                double v[NQ];
+                f(t[u], v);
+#pragma unroll
+                for (int q = 0; q < NQ; ++q) s[q] += v[q];
+            }
         }
 #pragma unroll
     for (int q = 0; q < NQ; ++q) red[q][warp][lane] = s[q];
@@ -55,12 +65,11 @@ __global__ void __launch_bounds__(BNS_THREADS, 2) bn_small_fwd_kernel(const BnSm
     const int cb = blockIdx.x % ncb, chunk = blockIdx.x / ncb, chunks = gridDim.x / ncb;
     {
         const int c = cb * 32 + (threadIdx.x & 31);
-        merge_partials<3>(red, p.nblocks, c, c < p.C, [&](int b, int ch, double (&v)[3]) {
-            const float* q = p.part + (size_t)b * 3 * p.C + ch;
-            const double n = q[0], m = q[p.C];
+        merge_partials<3>(red, p.part, p.nblocks, p.C, c, c < p.C, [](const float (&q)[3], double (&v)[3]) {
+            const double n = q[0], m = q[1];
             v[0] = n;
             v[1] = n * m;
-            v[2] = (double)q[2 * p.C] + n * m * m;
+            v[2] = (double)q[2] + n * m * m;
         });
         if (threadIdx.x < 32) {                          // as bn_finalize_fwd_kernel
             float sc = 0.f, sh = 0.f, mk = 1.f;
@@ -161,10 +170,9 @@ __global__ void __launch_bounds__(BNS_THREADS, 2) bn_small_bwd_kernel(const BnSm
     const int cb = blockIdx.x % ncb, chunk = blockIdx.x / ncb, chunks = gridDim.x / ncb;
     {
         const int c = cb * 32 + (threadIdx.x & 31);
-        merge_partials<2>(red, p.nblocks, c, c < p.C, [&](int b, int ch, double (&v)[2]) {
-            const float* q = p.part + (size_t)b * 2 * p.C + ch;
+        merge_partials<2>(red, p.part, p.nblocks, p.C, c, c < p.C, [](const float (&q)[2], double (&v)[2]) {
             v[0] = q[0];
-            v[1] = q[p.C];
+            v[1] = q[1];
         });
         if (threadIdx.x < 32) {
             float k1 = 0.f, k2 = 0.f, k3 = 0.f;
@@ -243,14 +251,19 @@ __global__ void __launch_bounds__(BNS_THREADS, 2) bn_small_bwd_kernel(const BnSm
         }
     }
     if (p.colsum_part != nullptr) {                       // one row of column sums per chunk; this CTA's 32 columns of it
-        float4* sums = reinterpret_cast<float4*>(red);    // 512 x 16 bytes = the merge's staging, no longer needed
+        float4* sums = reinterpret_cast<float4*>(red);    // the merge's staging, no longer needed
+#pragma unroll
+        for (int o = 8; o <= 16; o *= 2) {
+            csum.x += __shfl_xor_sync(0xffffffffu, csum.x, o); csum.y += __shfl_xor_sync(0xffffffffu, csum.y, o);
+            csum.z += __shfl_xor_sync(0xffffffffu, csum.z, o); csum.w += __shfl_xor_sync(0xffffffffu, csum.w, o);
+        }
         __syncthreads();
-        sums[threadIdx.x] = csum;
+        if ((threadIdx.x & 31) < 8) sums[(threadIdx.x >> 5) * 8 + g8] = csum;
         __syncthreads();
         if (threadIdx.x < 8 && c_ok) {
             float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 8
-            for (int l = 0; l < BNS_LANES; ++l) { const float4 v = sums[l * 8 + threadIdx.x]; t.x += v.x; t.y += v.y; t.z += v.z; t.w += v.w; }
+#pragma unroll
+            for (int l = 0; l < BNS_WARPS; ++l) { const float4 v = sums[l * 8 + threadIdx.x]; t.x += v.x; t.y += v.y; t.z += v.z; t.w += v.w; }
             *reinterpret_cast<float4*>(p.colsum_part + (size_t)chunk * p.C + c) = t;
         }
     }

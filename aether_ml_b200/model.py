@@ -11,14 +11,16 @@ Additions that the reference does not have, all optional:
     parallelism -- one all-reduce cover the whole network;
   * ``train_step(X, y)`` runs one forward/backward/update without printing or host synchronisation.
 """
+import math
 import pickle
 
 import numpy as np
 import torch
 
 from ._lib import host
-from .layers import (Activation_Softmax_Loss_CategoricalCrossEntropy, Batch_Norm, Conv_Layer, Flatten, Layer_Dropout_Spatial, Leaky_ReLU,
-                     Loss_CategoricalCrossEntropy, Optimizer_Adam, Pooling, ReLU, SoftMax, to_device, _labels, _labels_i32, _softmax_cce, _Saved)
+from .layers import (Activation_Softmax_Loss_CategoricalCrossEntropy, Batch_Norm, Conv_Layer, Flatten, Layer_Dense, Layer_Dropout,
+                     Layer_Dropout_Spatial, Leaky_ReLU, Loss_CategoricalCrossEntropy, Optimizer_Adam, Pooling, ReLU, SoftMax, to_device, _labels,
+                     _labels_i32, _softmax_cce, _Saved)
 
 
 class Layer_Input:
@@ -89,7 +91,7 @@ class _Chain:
     replaced layers, shapes the kernels do not take) runs layer by layer."""
 
     def __init__(self, parts, conv, consumer):
-        self.parts = parts                      # (bn, act[, drop][, pool])
+        self.parts = parts                      # [bn, act[, drop][, pool]]
         self.length = len(parts)
         self.bn, self.act = parts[0], parts[1]
         self.drop = next((l for l in parts if isinstance(l, Layer_Dropout_Spatial)), None)
@@ -119,19 +121,23 @@ class _Chain:
         behind = at(k)
         if isinstance(behind, Flatten):
             behind = at(k + 1)
-        return _Chain(tuple(parts), conv, behind if hasattr(behind, "x_copy_target") else None)
+        return _Chain(parts, conv, behind if hasattr(behind, "x_copy_target") else None)
 
     def _intact(self, layers, i):
-        for k, part in enumerate(self.parts):
-            if i + k >= len(layers) or layers[i + k] is not part or "forward" in part.__dict__ or "backward" in part.__dict__:
+        if layers[i:i + self.length] != self.parts:
+            return False
+        for part in self.parts:
+            d = part.__dict__
+            if "forward" in d or "backward" in d:
                 return False
         pool = self.pool
         return (self.bn.fused_alpha is None and not self.act.fused_into_prev and (self.drop is None or not self.drop.fused_into_prev)
                 and (pool is None or (pool.fused_bn is None and pool.pooling_type == "max" and pool.padding == "valid"
                                       and tuple(pool.strides) == tuple(pool.filter_size))))
 
-    def forward(self, layers, i, inputs, training):
-        """Runs the chain's layers; False when they have to run one by one."""
+    def forward(self, layers, i, inputs, training, keep_all=True):
+        """Runs the chain's layers; False when they have to run one by one.  An inference pass with ``keep_all=False`` writes
+        the last layer's output only and leaves the attributes of the others alone."""
         self.live = None
         if not self._intact(layers, i):
             return False
@@ -159,15 +165,20 @@ class _Chain:
                 part = None
             if drop is not None:
                 mask = drop.draw_mask(Cc)
-        bn_out, act_out = h.empty(shape), h.empty(shape)
-        last = act_out
-        drop_out = pooled = arg = None
-        if drop is not None:
-            last = drop_out = h.empty(shape)
-        if pool is not None:
-            pshape = (S, H // fH, W // fW, Cc)
-            last = pooled = h.empty(pshape)
-            arg = h.empty_u8(pshape)
+        bn_out = act_out = drop_out = pooled = arg = None
+        if training or keep_all:
+            bn_out, last = h.empty(shape), h.empty(shape)
+            act_out = last
+            if drop is not None:
+                last = drop_out = h.empty(shape)
+            if pool is not None:
+                pshape = (S, H // fH, W // fW, Cc)
+                last = pooled = h.empty(pshape)
+                arg = h.empty_u8(pshape)
+        elif pool is not None:
+            last = pooled = h.empty((S, H // fH, W // fW, Cc))
+        else:                                   # (spatial dropout does nothing in inference)
+            last = act_out = h.empty(shape)
         target = self.consumer.x_copy_target(tuple(last.shape)) if self.consumer is not None else None
         h.aether_chain_fwd(x, part[0] if part else None, part[1] if part else 0, bn.gamma, bn.beta, bn._rm, bn._rv,
                            bn._bm if training else None, bn._bv if training else None, bn_out, act_out, drop_out, pooled, arg, S, H, W,
@@ -175,6 +186,11 @@ class _Chain:
                            target[1] if target else 0, ws, bn._ws.size)
         if training:
             bn._expose_statistics(keep)
+        if target:
+            self.consumer.x_copy_written(last)
+        if bn_out is None:
+            self.parts[-1].output = last
+            return True
         bn.pooled_now = False
         bn.inputs, bn.output = x, bn_out
         act.inputs, act.output = bn_out, act_out
@@ -182,8 +198,6 @@ class _Chain:
             drop.inputs, drop.output = act_out, drop_out
         if pool is not None:
             pool.inputs, pool.output, pool._argmax = (act_out if drop is None else drop_out), pooled, arg
-        if target:
-            self.consumer.x_copy_written(last)
         if training:
             self.live = (x, bn_out, bn_out._version, ws, mask, S, H, W, Cc, fH, fW, alpha)
         return True
@@ -416,16 +430,20 @@ class Model:
                 self._bucket_of_layer[id(self.trainable_layers[trigger])] = i
 
     # ------------------------------------------------------------------ passes
-    def forward(self, X, training):
+    def forward(self, X, training, *, keep=True):
+        """``keep=False`` (inference passes whose layers' attributes the next pass replaces): a chain of layers run in one
+        pass writes its last output only."""
         self.input_layer.forward(X, training)
-        layers, chains, i = self.layers, self._chains, 0
+        layers, chains, i, prev = self.layers, self._chains, 0, self.input_layer
         while i < len(layers):
             layer = layers[i]
             chain = chains.get(i)
-            if chain is not None and chain.forward(layers, i, layer.prev.output, training):
+            if chain is not None and chain.forward(layers, i, prev.output, training, keep):
                 i += chain.length
+                prev = layers[i - 1]
                 continue
-            layer.forward(layer.prev.output, training)
+            layer.forward(prev.output, training)
+            prev = layer
             i += 1
         return layers[-1].output
 
@@ -744,16 +762,56 @@ class Model:
         if validation_data is not None:
             self.evaluate(*validation_data, batch_size=batch_size)
 
+    # Bytes of layer outputs that an inference pass takes several batches together up to.  A batch of the reference's networks
+    # leaves most of the GPU idle in its deeper layers and takes longer to launch than to run (32x32 network, batch 128:
+    # 112 us of host work for 86 us on the GPU), so a pass takes as many whole batches as keep its outputs within a
+    # gigabyte, as much as a training batch of 512 of that network: 1000 images in batches of 128, 900 -> 295 us.
+    INFERENCE_PASS_BYTES = 1 << 30
+    _PER_SAMPLE = (Conv_Layer, Batch_Norm, ReLU, Leaky_ReLU, Layer_Dropout, Layer_Dropout_Spatial, Pooling, Flatten, Layer_Dense, SoftMax)
+
+    def _output_bytes(self, shape):
+        """Bytes of all layers' outputs for one sample of ``shape``; None when a layer is not one of this package's own,
+        which treat every sample by itself in inference, or does not take the shape."""
+        total = 0
+        for l in self.layers:
+            if type(l) not in self._PER_SAMPLE or "forward" in l.__dict__:
+                return None
+            if type(l) is Conv_Layer:
+                if len(shape) != 3:
+                    return None
+                shape = l._plan((1, *shape)).y_shape
+                if shape is None:
+                    return None
+                shape = shape[1:]
+            elif type(l) is Pooling:
+                if len(shape) != 3:
+                    return None
+                shape = tuple((n - f) // s + 1 for n, f, s in zip(shape, l.filter_size, l.strides)) + (shape[2],)
+            elif type(l) is Flatten:
+                shape = (math.prod(shape),)
+            elif type(l) is Layer_Dense:
+                shape = (l.weights.shape[1],)
+            total += 4 * math.prod(shape)
+        return total if total > 0 else None
+
     def _inference(self, X, batch_size):
-        """Slices and outputs of the forward passes over X.  The weights stay as they are between the batches of one call,
-        so from the second on the tensor-core layers use the operand copies of them that the first one made."""
+        """Slices and outputs of the forward passes over X: whole batches, several at once where they are small, then the
+        last batch by itself, whose inputs and outputs the layers keep.  The weights stay as they are between the passes of
+        one call, so from the second on the tensor-core layers use the operand copies of them that the first one made."""
+        passes = _batches(len(X), batch_size)
+        if len(passes) > 2 and hasattr(X, "shape"):
+            per_sample = self._output_bytes(tuple(X.shape[1:]))
+            if per_sample is not None:
+                step = batch_size * max(1, self.INFERENCE_PASS_BYTES // (per_sample * batch_size))
+                head = (len(passes) - 1) * batch_size
+                passes = [slice(k, min(k + step, head)) for k in range(0, head, step)] + passes[-1:]
         fixed = [l for l in self.layers if hasattr(l, "_weights_fixed")]
         try:
-            for k, sl in enumerate(_batches(len(X), batch_size)):
+            for k, sl in enumerate(passes):
                 if k == 1:
                     for l in fixed:
                         l._weights_fixed = True
-                yield sl, self.forward(X[sl], training=False)
+                yield sl, self.forward(X[sl], training=False, keep=k == len(passes) - 1)
         finally:
             for l in fixed:
                 l._weights_fixed = False
@@ -761,9 +819,11 @@ class Model:
     def evaluate(self, X_val, y_val, *, batch_size=None):
         self.loss.new_pass()
         self.accuracy.new_pass()
-        for sl, output in self._inference(X_val, batch_size):
-            self.loss.calculate(output, y_val[sl], training=False)
-            self.accuracy.calculate(self.output_layer_activation.predictions(output), y_val[sl])
+        for sl, outputs in self._inference(X_val, batch_size):
+            y_pass = y_val[sl]
+            for part in _batches(len(outputs), batch_size):
+                self.loss.calculate(outputs[part], y_pass[part], training=False)
+                self.accuracy.calculate(self.output_layer_activation.predictions(outputs[part]), y_pass[part])
         validation_loss = self.loss.calculate_accumulated()
         validation_accuracy = self.accuracy.calculate_accumulated()
         print(f'Valdiation, acc: {float(validation_accuracy):.3f}, loss: {float(validation_loss):.3f}')

@@ -250,7 +250,8 @@ int aether_bn_act_pool_bwd_copy(const float* x, const float* dpooled, const uint
  * fused): one pass writes Batch_Norm's output, the activation's, the spatial dropout's (drop_out, may be NULL when there
  * is no such layer; mask = its channel mask in training, NULL in inference where it copies) and, when `pooled` is given,
  * those of a max Pooling with fH x fW windows of stride (fH, fW) -- H and W need not be multiples of them; without
- * pooling fH = fW = 1.  The numbers are those of the layers by themselves.  operand_copy as in ..._fwd_copy, of the last
+ * pooling fH = fW = 1.  The numbers are those of the layers by themselves.  In inference (training = 0) any output but
+ * one may be NULL: what nobody will read is not written.  operand_copy as in ..._fwd_copy, of the last
  * tensor of the chain.  aether_chain_bwd: dy is the gradient of the last tensor; writes the input gradient of every layer
  * (pool_dx, drop_dx: NULL where there is no such layer) and, with operand_copy, what ..._bwd_copy writes beside dx.  It
  * reads the coefficients the training forward pass left in the same `ws`.  C % 4 == 0. */
