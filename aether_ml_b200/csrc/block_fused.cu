@@ -201,7 +201,7 @@ __global__ void __launch_bounds__(256) bn_act_pool_bwd_reduce_kernel(
 
 // dx = k1 * g + k2 * x + k3 for every cell of every window (g is non-zero only at the window's selected cell).
 template <int F>
-__global__ void __launch_bounds__(256) bn_act_pool_bwd_apply_kernel(
+__global__ void __launch_bounds__(256, 3) bn_act_pool_bwd_apply_kernel(
     const float* __restrict__ x, const float* __restrict__ dpool, const uint8_t* __restrict__ arg,
     const float* __restrict__ gamma, const float* __restrict__ beta, const float* __restrict__ mean,
     const float* __restrict__ var, float eps, float alpha, const float* __restrict__ coeff, float* __restrict__ dx,
@@ -213,6 +213,12 @@ __global__ void __launch_bounds__(256) bn_act_pool_bwd_apply_kernel(
     // column sums of dx (the bias gradient of the convolution in front): only with grids whose stride keeps a thread on
     // one channel group (gridDim.x * 256 a multiple of C4; the host checks), so four running sums per thread suffice
     float4 csum = make_float4(0.f, 0.f, 0.f, 0.f);
+    // Coefficients of this thread's channels, loaded once where the stride keeps it on them: seven vectors from L1 and four
+    // reciprocal roots per window made the L1 the limit (the three block tails of the 128/256/512-channel network
+    // at batch 4096: 1440 -> 1230 us).
+    const bool fixed = gridDim.x * blockDim.x % (unsigned)C4 == 0;
+    float4 k1 = csum, k2 = csum, k3 = csum, mu = csum, ga = csum, be = csum, inv = csum;
+    bool loaded = false;
     for (unsigned idx = blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += gridDim.x * blockDim.x) {
         const unsigned cv = idx % (unsigned)C4;
         unsigned pix = idx / (unsigned)C4;
@@ -221,14 +227,17 @@ __global__ void __launch_bounds__(256) bn_act_pool_bwd_apply_kernel(
         const int c = cv * 4;
         const float4 g = __ldcs(reinterpret_cast<const float4*>(dpool) + idx);
         const uchar4 cd = reinterpret_cast<const uchar4*>(arg)[idx];
-        const float4 k1 = *reinterpret_cast<const float4*>(coeff + c);
-        const float4 k2 = *reinterpret_cast<const float4*>(coeff + C + c);
-        const float4 k3 = *reinterpret_cast<const float4*>(coeff + 2 * C + c);
-        const float4 mu = *reinterpret_cast<const float4*>(mean + c);
-        const float4 vr = *reinterpret_cast<const float4*>(var + c);
-        const float4 ga = *reinterpret_cast<const float4*>(gamma + c);
-        const float4 be = *reinterpret_cast<const float4*>(beta + c);
-        const float4 inv = make_float4(rsqrtf(vr.x + eps), rsqrtf(vr.y + eps), rsqrtf(vr.z + eps), rsqrtf(vr.w + eps));
+        if (!loaded) {
+            k1 = *reinterpret_cast<const float4*>(coeff + c);
+            k2 = *reinterpret_cast<const float4*>(coeff + C + c);
+            k3 = *reinterpret_cast<const float4*>(coeff + 2 * C + c);
+            mu = *reinterpret_cast<const float4*>(mean + c);
+            ga = *reinterpret_cast<const float4*>(gamma + c);
+            be = *reinterpret_cast<const float4*>(beta + c);
+            const float4 vr = *reinterpret_cast<const float4*>(var + c);
+            inv = make_float4(rsqrtf(vr.x + eps), rsqrtf(vr.y + eps), rsqrtf(vr.z + eps), rsqrtf(vr.w + eps));
+            loaded = fixed;
+        }
         const size_t first = ((size_t)pix * fH * W + (size_t)wo * fW) * C4 + cv;
         float4 pre[F ? F * F : 1];
         if (F) {
@@ -648,7 +657,7 @@ extern "C" int aether_bn_act_pool_bwd_copy(const float* x, const float* dpooled,
         return check_launch("aether_bn_act_pool_bwd");
     }
     bn_backward_coeffs(part, nb, C, rows, gamma, batch_mean, batch_var, eps, dgamma, dbeta, coeff, channel_scale, st);
-    int fb = fused_blocks(windows4, 256, 16);
+    int fb = fused_blocks(windows4, 256, 3);     // what is resident at once: equal shares, coefficients loaded once per thread
     __nv_bfloat16* copy = static_cast<__nv_bfloat16*>(operand_copy);
     if (copy) {                                  // one row of column sums per CTA: no more CTAs than rows offered
         if (fb > colsum_rows_max) fb = colsum_rows_max;

@@ -55,7 +55,7 @@ __global__ void __launch_bounds__(DWR_THREADS, 1) dw_rows_kernel(const __grid_co
     const uint32_t sTmemPtr = sBar + 8u * (2 * S + 1);
     volatile uint32_t* tmem_ptr_generic = reinterpret_cast<volatile uint32_t*>(gen_base + (sTmemPtr - smem_base));
 
-    const int warp = threadIdx.x >> 5;
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);
     const int lane = threadIdx.x & 31;
 
     // Rows that no TMA box writes (the tails of the regions) are read by the MMAs and must be zero.
@@ -110,20 +110,20 @@ __global__ void __launch_bounds__(DWR_THREADS, 1) dw_rows_kernel(const __grid_co
     const uint32_t stage_tx = (uint32_t)(p.x_box_rows + 2 * p.dy_box_rows) * 128u;
 
     if (warp == 0) {
-        if (lane == 0) {
-            uint32_t it = 0;
-            for (long long st = split; st < total_strips; st += splits, ++it) {
+        if (elect_one()) {
+            int s = 0;
+            uint32_t ph = 0;
+            for (long long st = split; st < total_strips; st += splits) {
                 const int th = (int)(st % p.tiles_h);
                 const int n = (int)(st / p.tiles_h);
                 const int h0 = th * p.BH;
-                const int s = it % S;
-                const uint32_t ph = (it / S) & 1u;
                 if (!mbar_wait(empty_bar(s), ph ^ 1u, p.status, DS_TIMEOUT_EMPTY)) break;
                 mbar_arrive_expect_tx(full_bar(s), stage_tx);
                 const uint32_t base = smem_base + s * p.stage_bytes;
                 tma_load_4d(base, &p.tm_dy, full_bar(s), db * 128, 0, h0, n);
                 tma_load_4d(base + p.dyr_bytes, &p.tm_dy, full_bar(s), db * 128 + 64, 0, h0, n);
                 tma_load_4d(base + 2 * p.dyr_bytes, &p.tm_x, full_bar(s), cb * 64, -p.padL, h0 - p.padT + row0, n);
+                if (++s == S) { s = 0; ph ^= 1u; }
             }
         }
     } else if (warp == 1) {
@@ -134,12 +134,11 @@ __global__ void __launch_bounds__(DWR_THREADS, 1) dw_rows_kernel(const __grid_co
         const uint32_t a_lbo = ((uint32_t)p.dyr_bytes >> 4) << 16;              // second 64-channel block of dy
         const uint32_t b_lbo = 8u << 16;                                        // next tap = next pixel row (128 bytes)
         const uint32_t row_step = (uint32_t)p.Wp * 8u;                          // next filter row = Wp pixel rows
-        uint32_t it = 0;
+        int s = 0;
+        uint32_t ph = 0;
         bool ok = true;
         uint32_t acc = 0;
-        for (long long st = split; st < total_strips && ok; st += splits, ++it) {
-            const int s = it % S;
-            const uint32_t ph = (it / S) & 1u;
+        for (long long st = split; st < total_strips && ok; st += splits) {
             bool f_ok = mbar_wait_spin(full_bar(s), ph, p.status, DS_TIMEOUT_FULL);
             f_ok = __all_sync(0xffffffffu, f_ok);
             if (!f_ok) { ok = false; break; }
@@ -165,6 +164,7 @@ __global__ void __launch_bounds__(DWR_THREADS, 1) dw_rows_kernel(const __grid_co
                 b_k += 128u;
             }
             if (leader) umma_commit(empty_bar(s));
+            if (++s == S) { s = 0; ph ^= 1u; }
             __syncwarp();
         }
         if (leader) umma_commit(done_bar);

@@ -139,7 +139,7 @@ __global__ void __launch_bounds__(FT_THREADS, 1) first_conv_kernel(const __grid_
     FirstTaps& taps = *reinterpret_cast<FirstTaps*>(gen_base + (sBar - smem_base) + 256 + 1024);
     float* stat_s = reinterpret_cast<float*>(gen_base + (sBar - smem_base) + FT_TAIL);     // STATS: 3 * (NT / 32) * 256 + 256 floats
 
-    const int warp = threadIdx.x >> 5;
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);
     const int lane = threadIdx.x & 31;
     const int NB = (4 * NT <= 512) ? 4 : (3 * NT <= 512) ? 3 : 2;
     const uint32_t need_cols = (uint32_t)(NB * NT);
@@ -202,7 +202,7 @@ __global__ void __launch_bounds__(FT_THREADS, 1) first_conv_kernel(const __grid_
         }
     } else if (warp == FT_PROD_WARPS) {
         // ------------------------------------------------------------------ MMA issuer (one thread)
-        if (lane == 0) {
+        if (elect_one()) {
             const uint32_t idesc = make_idesc(1u, 0u, 0u, 128u, (uint32_t)NT);
             const uint64_t proto = make_smem_desc(0, 16, 1024);
             const uint32_t hi = (uint32_t)(proto >> 32);
@@ -393,7 +393,7 @@ __global__ void __launch_bounds__(FD_THREADS, 1) first_dw_kernel(const __grid_co
     FirstTaps& taps = *reinterpret_cast<FirstTaps*>(gen_base + (sBar - smem_base) + 256);
     float* dbsum_s = reinterpret_cast<float*>(gen_base + (sBar - smem_base) + 1024);      // [producer threads][8]
 
-    const int warp = threadIdx.x >> 5;
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);
     const int lane = threadIdx.x & 31;
     const uint32_t tmem_cols = 128;                                          // dblocks (<= 2) x KP (<= 64) columns
 

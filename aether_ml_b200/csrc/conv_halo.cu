@@ -115,7 +115,7 @@ __global__ void __launch_bounds__(HALO_THREADS, 1) halo_conv_kernel(const __grid
     volatile uint32_t* tmem_ptr_generic = reinterpret_cast<volatile uint32_t*>(gen_base + (sTmemPtr - smem_base));
     float* bias_s = reinterpret_cast<float*>(gen_base + (sBar - smem_base) + 256);     // NT floats
 
-    const int warp = threadIdx.x >> 5;
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);
     const int lane = threadIdx.x & 31;
     const int NT = p.NT;
     const int cta_rank = PAIR ? (int)cluster_cta_rank() : 0;
@@ -169,7 +169,7 @@ __global__ void __launch_bounds__(HALO_THREADS, 1) halo_conv_kernel(const __grid
 
     if (warp == 0) {
         // ------------------------------------------------------------------ TMA producer
-        if (lane == 0) {
+        if (elect_one()) {
             // resident filter: p.w_bytes per CTA; a pair's two halves are counted on the even CTA's barrier
             if (issuer) mbar_arrive_expect_tx(wfull_bar, (uint32_t)p.w_bytes * (uint32_t)PF);
             const uint32_t wbar = PAIR ? cluster_map_shared(wfull_bar, 0) : wfull_bar;

@@ -17,6 +17,7 @@
 
 #include "common.cuh"
 #include "sm100_ptx.cuh"
+#include "store_block.cuh"
 #include "tc_host.cuh"
 
 namespace aether {
@@ -48,7 +49,7 @@ __global__ void __launch_bounds__(DWH_THREADS, 1) dw_halo_kernel(const __grid_co
     const uint32_t sTmemPtr = sBar + 8u * (2 * S + 1);
     volatile uint32_t* tmem_ptr_generic = reinterpret_cast<volatile uint32_t*>(gen_base + (sTmemPtr - smem_base));
 
-    const int warp = threadIdx.x >> 5;
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);
     const int lane = threadIdx.x & 31;
 
     // Rows that no TMA box ever writes (the tails of the two regions of a stage) are read by the MMAs and must be zero: the
@@ -91,19 +92,19 @@ __global__ void __launch_bounds__(DWH_THREADS, 1) dw_halo_kernel(const __grid_co
     const uint32_t stage_tx = (uint32_t)(p.xr_rows + p.dyr_rows) * 128u;
 
     if (warp == 0) {
-        if (lane == 0) {
-            uint32_t it = 0;
-            for (long long st = split; st < total_strips; st += splits, ++it) {
+        if (elect_one()) {
+            int s = 0;
+            uint32_t ph = 0;
+            for (long long st = split; st < total_strips; st += splits) {
                 const int th = (int)(st % p.tiles_h);
                 const int n = (int)(st / p.tiles_h);
                 const int h0 = th * p.BH;
-                const int s = it % S;
-                const uint32_t ph = (it / S) & 1u;
                 if (!mbar_wait(empty_bar(s), ph ^ 1u, p.status, DS_TIMEOUT_EMPTY)) break;
                 mbar_arrive_expect_tx(full_bar(s), stage_tx);
                 const uint32_t base = smem_base + s * p.stage_bytes;
                 tma_load_4d(base, &p.tm_x, full_bar(s), cb * 64, -p.padL, h0 - p.padT, n);
                 tma_load_4d(base + p.xr_bytes, &p.tm_dy, full_bar(s), db * 64, 0, h0, n);
+                if (++s == S) { s = 0; ph ^= 1u; }
             }
         }
     } else if (warp == 1) {
@@ -123,12 +124,11 @@ __global__ void __launch_bounds__(DWH_THREADS, 1) dw_halo_kernel(const __grid_co
             const uint32_t offb = (uint32_t)((tb / p.fW) * p.Wp + (tb % p.fW));
             pair_lo[pr] = (offa * 8u) + (((offb - offa) * 8u) << 16);
         }
-        uint32_t it = 0;
+        int s = 0;
+        uint32_t ph = 0;
         bool ok = true;
         uint32_t acc = 0;
-        for (long long st = split; st < total_strips && ok; st += splits, ++it) {
-            const int s = it % S;
-            const uint32_t ph = (it / S) & 1u;
+        for (long long st = split; st < total_strips && ok; st += splits) {
             bool f_ok = mbar_wait_spin(full_bar(s), ph, p.status, DS_TIMEOUT_FULL);
             f_ok = __all_sync(0xffffffffu, f_ok);
             if (!f_ok) { ok = false; break; }
@@ -154,19 +154,20 @@ __global__ void __launch_bounds__(DWH_THREADS, 1) dw_halo_kernel(const __grid_co
                 b_lo += 128u;
             }
             if (leader) umma_commit(empty_bar(s));
+            if (++s == S) { s = 0; ph ^= 1u; }
             __syncwarp();
         }
         if (leader) umma_commit(done_bar);
         __syncwarp();
     } else {
         const int q = warp & 3;
-        const int row = q * 32 + lane;
         const bool any = split < total_strips;
         bool ok = true;
         if (any) ok = mbar_wait(done_bar, 0, p.status, DS_TIMEOUT_TMEM_FULL);
         tc_fence_after();
         if (ok) {
-            const int m = row >> 6, c_in = row & 63;
+            const int m = q >> 1, c_in0 = (q & 1) * 32;          // this warp's 32 rows: one tap, half a channel block
+            float* stage = reinterpret_cast<float*>(gen_base) + q * STORE_BLOCK_FLOATS;       // every MMA has read its operands
             for (int pr = 0; pr < p.npairs; ++pr) {
                 int ta = 2 * pr, tb = 2 * pr + 1;
                 bool dup = false;
@@ -183,15 +184,9 @@ __global__ void __launch_bounds__(DWH_THREADS, 1) dw_halo_kernel(const __grid_co
 #pragma unroll
                         for (int k = 0; k < 32; ++k) r[k] = 0u;
                     }
-                    if (write) {
-                        float4* dst = reinterpret_cast<float4*>(
-                            p.part + (((size_t)split * (taps * p.cblocks) + (size_t)tap * p.cblocks + cb) * 64 + c_in) * (size_t)p.ldn +
-                            db * 64 + ch * 32);
-#pragma unroll
-                        for (int k = 0; k < 8; ++k)
-                            dst[k] = make_float4(__uint_as_float(r[4 * k]), __uint_as_float(r[4 * k + 1]),
-                                                 __uint_as_float(r[4 * k + 2]), __uint_as_float(r[4 * k + 3]));
-                    }
+                    if (write)
+                        store_block_32x32(stage, r, p.part + (((size_t)split * (taps * p.cblocks) + (size_t)tap * p.cblocks + cb) * 64 + c_in0) *
+                                                     (size_t)p.ldn + db * 64 + ch * 32, p.ldn, 32, 32, lane);
                 }
             }
         }

@@ -20,6 +20,7 @@
 #include "common.cuh"
 #include "sm100_ptx.cuh"
 #include "stats_epilogue.cuh"
+#include "store_block.cuh"
 #include "tc_host.cuh"
 
 namespace aether {
@@ -133,11 +134,11 @@ template <int NT, bool PAIR = false>
 struct IgemmCfg {
     static constexpr int B_ROWS = PAIR ? NT / 2 : NT;           // filter rows this CTA stages
     static constexpr int TILE_B_BYTES = B_ROWS * 128;
-    // 128-byte K chunks per stage: one thread issues for both SMs of a pair, and with one chunk per stage its
+    // 128-byte K chunks per stage: one thread issues for both SMs of a pair (and the MMAs of narrow tiles are short), and with one chunk per stage its
     // per-stage work (barrier wait, four MMAs, two commits) is not hidden behind the MMAs; a pair's stage takes two
-    static constexpr int KS = PAIR ? 2 : 1;
+    static constexpr int KS = PAIR || NT <= 64 ? 2 : 1;
     static constexpr int STAGE_A_BYTES = KS * TILE_A_BYTES, STAGE_B_BYTES = KS * TILE_B_BYTES;
-    static constexpr int STAGES = PAIR ? (NT == 256 ? 3 : 4) : ((NT == 256) ? 4 : (NT == 128 ? 6 : 8));
+    static constexpr int STAGES = PAIR ? (NT == 256 ? 3 : 4) : ((NT == 256) ? 4 : (NT == 128 ? 6 : NT == 64 ? 4 : 5));
     static constexpr int SMEM_BYTES = 1024 + STAGES * (STAGE_A_BYTES + STAGE_B_BYTES) + IGEMM_TAIL + IGEMM_STATS_BYTES;
 };
 
@@ -170,7 +171,7 @@ __global__ void __launch_bounds__(IGEMM_THREADS, 1) igemm_conv_kernel(const __gr
     volatile uint32_t* tmem_ptr_generic =
         reinterpret_cast<volatile uint32_t*>(gen_base + (sTmemPtr - smem_base));
 
-    const int warp = threadIdx.x >> 5;
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);      // (warp-uniform for the compiler, too)
     const int lane = threadIdx.x & 31;
     const int cta_rank = PAIR ? (int)cluster_cta_rank() : 0;
     const bool issuer = cta_rank == 0;            // the CTA whose warp 1 issues the MMAs
@@ -230,41 +231,51 @@ __global__ void __launch_bounds__(IGEMM_THREADS, 1) igemm_conv_kernel(const __gr
 
     if (warp == 0) {
         // ------------------------------------------------------------------ TMA producer
-        if (lane == 0) {
-            uint32_t it = 0;
+        // One elected lane (elect.sync, not `lane == 0`: the compiler then knows that one thread issues, and a chunk's four
+        // MMAs and two copies go out in 130-160 ns instead of 290, less than a 128-column chunk takes to multiply); stages,
+        // phases and taps are counted on, not divided out.
+        if (elect_one()) {
+            uint32_t s = 0, ph = 0;
             bool ok = true;
             for (long long t = t_first; t < total_tiles && ok; t += t_step) {
                 int nt, w0, h0, n0;
                 decode(t, nt, w0, h0, n0);
-                int tap = 0, kc = 0;                       // the (tap, K chunk) of the next chunk to load
-                for (int k0 = 0; k0 < kiters && ok; k0 += KS, ++it) {
-                    const int s = it % STAGES;
-                    const uint32_t ph = (it / STAGES) & 1u;
+                int kc = 0, j = 0;                         // the (K chunk, filter column) of the next chunk to load
+                int cw = w0 + p.off_w, ch = h0 + p.off_h, wrow = nt * NT + (PAIR ? cta_rank * Cfg::B_ROWS : 0);
+                for (int k0 = 0; k0 < kiters; k0 += KS) {
                     const int nsub = kiters - k0 < KS ? kiters - k0 : KS;
                     if (!mbar_wait(empty_bar(s), ph ^ 1u, p.status, DS_TIMEOUT_EMPTY)) { ok = false; break; }
                     if (issuer) mbar_arrive_expect_tx(full_bar(s), chunk_tx * (uint32_t)nsub);
                     const uint32_t bar = PAIR ? cluster_map_shared(full_bar(s), 0) : full_bar(s);   // PAIR: the even CTA's
-                    for (int c = 0; c < nsub; ++c) {
-                        const int i = tap / p.fW, j = tap % p.fW;
-                        const uint32_t dA = sA + s * Cfg::STAGE_A_BYTES + c * TILE_A_BYTES;
-                        const uint32_t dB = sB + s * Cfg::STAGE_B_BYTES + c * Cfg::TILE_B_BYTES;
-                        if (PAIR) {
-                            tma_load_4d_pair(dA, &p.tm_in, bar, kc * KC, w0 + p.sgn * j + p.off_w, h0 + p.sgn * i + p.off_h, n0);
-                            tma_load_2d_pair(dB, &p.tm_w, bar, kc * KC, tap * p.rows_per_tap + nt * NT + cta_rank * Cfg::B_ROWS);
-                        } else {
-                            tma_load_4d(dA, &p.tm_in, bar, kc * KC, w0 + p.sgn * j + p.off_w, h0 + p.sgn * i + p.off_h, n0);
-                            tma_load_2d(dB, &p.tm_w, bar, kc * KC, tap * p.rows_per_tap + nt * NT);
+#pragma unroll
+                    for (int c = 0; c < KS; ++c) {
+                        if (c < nsub) {
+                            const uint32_t dA = sA + s * Cfg::STAGE_A_BYTES + c * TILE_A_BYTES;
+                            const uint32_t dB = sB + s * Cfg::STAGE_B_BYTES + c * Cfg::TILE_B_BYTES;
+                            if (PAIR) {
+                                tma_load_4d_pair(dA, &p.tm_in, bar, kc * KC, cw, ch, n0);
+                                tma_load_2d_pair(dB, &p.tm_w, bar, kc * KC, wrow);
+                            } else {
+                                tma_load_4d(dA, &p.tm_in, bar, kc * KC, cw, ch, n0);
+                                tma_load_2d(dB, &p.tm_w, bar, kc * KC, wrow);
+                            }
+                            if (++kc == p.kchunks) {
+                                kc = 0;
+                                wrow += p.rows_per_tap;
+                                cw += p.sgn;
+                                if (++j == p.fW) { j = 0; cw = w0 + p.off_w; ch += p.sgn; }
+                            }
                         }
-                        if (++kc == p.kchunks) { kc = 0; ++tap; }
                     }
+                    if (++s == STAGES) { s = 0; ph ^= 1u; }
                 }
             }
         }
     } else if (warp == 1) {
-        // ------------------------------------------------------------------ MMA issuer (one thread)
-        if (lane == 0 && issuer) {
+        // ------------------------------------------------------------------ MMA issuer (one elected thread)
+        if (issuer && elect_one()) {
             constexpr uint32_t idesc = make_idesc(TF32 ? 2u : 1u, 0u, 0u, PAIR ? 256u : 128u, (uint32_t)NT);
-            uint32_t it = 0;
+            uint32_t s = 0, ph = 0;
             uint32_t lt = 0;
             bool ok = true;
             for (long long t = t_first; t < total_tiles && ok; t += t_step, ++lt) {
@@ -273,26 +284,20 @@ __global__ void __launch_bounds__(IGEMM_THREADS, 1) igemm_conv_kernel(const __gr
                 if (!mbar_wait(tempty_bar(buf), aph ^ 1u, p.status, DS_TIMEOUT_TMEM_EMPTY)) { ok = false; break; }
                 tc_fence_after();
                 const uint32_t d_tmem = tmem_base + buf * NT;
-                for (int k0 = 0; k0 < kiters; k0 += KS, ++it) {
-                    const int s = it % STAGES;
-                    const uint32_t ph = (it / STAGES) & 1u;
+                for (int k0 = 0; k0 < kiters; k0 += KS) {
                     const int nsub = kiters - k0 < KS ? kiters - k0 : KS;
                     if (!mbar_wait(full_bar(s), ph, p.status, DS_TIMEOUT_FULL)) { ok = false; break; }
                     tc_fence_after();
 #pragma unroll
                     for (int c = 0; c < KS; ++c) {
                         if (c < nsub) {
-                            const uint32_t a0 = sA + s * Cfg::STAGE_A_BYTES + c * TILE_A_BYTES;
-                            const uint32_t b0 = sB + s * Cfg::STAGE_B_BYTES + c * Cfg::TILE_B_BYTES;
+                            const uint64_t da = make_smem_desc(sA + s * Cfg::STAGE_A_BYTES + c * TILE_A_BYTES, 16, 1024);
+                            const uint64_t db = make_smem_desc(sB + s * Cfg::STAGE_B_BYTES + c * Cfg::TILE_B_BYTES, 16, 1024);
 #pragma unroll
-                            for (int k = 0; k < 4; ++k) {
+                            for (int k = 0; k < 4; ++k) {                  // 32 bytes of K each: two 16-byte units further
                                 const uint32_t acc = (k0 + c > 0 || k > 0) ? 1u : 0u;
-                                if (PAIR)
-                                    umma_pair<TF32>(d_tmem, make_smem_desc(a0 + k * 32, 16, 1024),
-                                                    make_smem_desc(b0 + k * 32, 16, 1024), idesc, acc);
-                                else
-                                    umma<TF32>(d_tmem, make_smem_desc(a0 + k * 32, 16, 1024), make_smem_desc(b0 + k * 32, 16, 1024),
-                                               idesc, acc);
+                                if (PAIR) umma_pair<TF32>(d_tmem, da + 2u * k, db + 2u * k, idesc, acc);
+                                else umma<TF32>(d_tmem, da + 2u * k, db + 2u * k, idesc, acc);
                             }
                         }
                     }
@@ -303,6 +308,7 @@ __global__ void __launch_bounds__(IGEMM_THREADS, 1) igemm_conv_kernel(const __gr
                     } else {
                         umma_commit(empty_bar(s));
                     }
+                    if (++s == STAGES) { s = 0; ph ^= 1u; }
                 }
                 if (ok) {
                     if (PAIR) {
@@ -535,7 +541,7 @@ __global__ void __launch_bounds__(DW_THREADS, 1) dw_conv_kernel(const __grid_con
     const uint32_t sTmemPtr = sBar + 8u * (2 * STAGES + 1);
     volatile uint32_t* tmem_ptr_generic = reinterpret_cast<volatile uint32_t*>(gen_base + (sTmemPtr - smem_base));
 
-    const int warp = threadIdx.x >> 5;
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);      // (warp-uniform for the compiler, too)
     const int lane = threadIdx.x & 31;
     const int cta_rank = PAIR ? (int)cluster_cta_rank() : 0;
     const bool issuer = cta_rank == 0;
@@ -589,8 +595,19 @@ __global__ void __launch_bounds__(DW_THREADS, 1) dw_conv_kernel(const __grid_con
     const int ksteps = (p.rows + Cfg::KROWS - 1) / Cfg::KROWS;
 
     if (warp == 0) {
-        if (lane == 0) {
-            uint32_t it = 0;
+        if (elect_one()) {                            // (see igemm_conv_kernel)
+            struct Unit { int u, cb, i, j; };
+            auto unit = [&](int u) { const int tap = u / p.cblocks; return Unit{u, u - tap * p.cblocks, tap / p.fW, tap % p.fW}; };
+            auto advance = [&](Unit& x, int n) {
+                x.u += n;
+                x.cb += n;
+                while (x.cb >= p.cblocks) {
+                    x.cb -= p.cblocks;
+                    if (++x.j == p.fW) { x.j = 0; ++x.i; }
+                }
+            };
+            const Unit first = unit((g_begin * PF + cta_rank) * MB), last = unit(p.U - 1);
+            uint32_t s = 0, ph = 0;
             bool ok = true;
             for (long long pt = split; pt < total_ptiles && ok; pt += splits) {
                 long long r = pt;
@@ -599,56 +616,57 @@ __global__ void __launch_bounds__(DW_THREADS, 1) dw_conv_kernel(const __grid_con
                 const int th = (int)(r % p.tiles_h);
                 const int tn = (int)(r / p.tiles_h);
                 const int w0 = tw * p.BW, h0 = th * p.BH, n0 = tn * p.BN;
-                for (int g = g_begin; g < g_end; ++g, ++it) {
-                    const int s = it % STAGES;
-                    const uint32_t ph = (it / STAGES) & 1u;
+                Unit x = first;
+                for (int g = g_begin; g < g_end; ++g) {
                     if (!mbar_wait(empty_bar(s), ph ^ 1u, p.status, DS_TIMEOUT_EMPTY)) { ok = false; break; }
                     if (issuer) mbar_arrive_expect_tx(full_bar(s), stage_tx);
                     const uint32_t bar = PAIR ? cluster_map_shared(full_bar(s), 0) : full_bar(s);   // PAIR: the even CTA's
                     const uint32_t st = smem_base + s * Cfg::STAGE_BYTES;
-                    for (int m = 0; m < MB; ++m) {
-                        int u = (g * PF + cta_rank) * MB + m;
-                        if (u >= p.U) u = p.U - 1;       // padding unit of the last group: results are dropped
-                        const int tap = u / p.cblocks, cb = u % p.cblocks;
-                        const int i = tap / p.fW, j = tap % p.fW;
-                        if (PAIR) tma_load_4d_pair(st + m * TILE_A_BYTES, &p.tm_x, bar, cb * UC, w0 + j - p.padW, h0 + i - p.padH, n0);
-                        else tma_load_4d(st + m * TILE_A_BYTES, &p.tm_x, bar, cb * UC, w0 + j - p.padW, h0 + i - p.padH, n0);
-                    }
+#pragma unroll
                     for (int nb = 0; nb < NB; ++nb) {
                         const int dyc = ((nt * PF + cta_rank) * NB + nb) * UC;
                         if (PAIR) tma_load_4d_pair(st + (MB + nb) * TILE_A_BYTES, &p.tm_dy, bar, dyc, w0, h0, n0);
                         else tma_load_4d(st + (MB + nb) * TILE_A_BYTES, &p.tm_dy, bar, dyc, w0, h0, n0);
                     }
+#pragma unroll
+                    for (int m = 0; m < MB; ++m) {
+                        const Unit y = x.u < p.U ? x : last;       // padding unit of the last group: results are dropped
+                        const int cw = w0 + y.j - p.padW, chh = h0 + y.i - p.padH;
+                        if (PAIR) tma_load_4d_pair(st + m * TILE_A_BYTES, &p.tm_x, bar, y.cb * UC, cw, chh, n0);
+                        else tma_load_4d(st + m * TILE_A_BYTES, &p.tm_x, bar, y.cb * UC, cw, chh, n0);
+                        advance(x, 1);
+                    }
+                    if (PAIR) advance(x, MB);                      // the other CTA's units
+                    if (++s == STAGES) { s = 0; ph ^= 1u; }
                 }
             }
         }
     } else if (warp == 1) {
-        if (lane == 0 && issuer) {
+        if (issuer && elect_one()) {
             constexpr uint32_t idesc = make_idesc(TF32 ? 2u : 1u, 1u, 1u, 128u * PF, (uint32_t)NTP);
-            uint32_t it = 0;
+            // MN-major operands: 16-bit types use the plain 128-byte swizzle (8-row K groups); 32-bit types need the
+            // 32-byte-unit variant (4-row K groups).
+            constexpr uint32_t LT = TF32 ? 1u : 2u;
+            constexpr uint32_t SBO = TF32 ? 512u : 1024u;
+            uint32_t s = 0, ph = 0;
             bool ok = true;
-            bool first = true;
-            for (long long pt = split; pt < total_ptiles && ok; pt += splits, first = false) {
-                for (int g = 0; g < ngroups; ++g, ++it) {
-                    const int s = it % STAGES;
-                    const uint32_t ph = (it / STAGES) & 1u;
+            uint32_t acc0 = 0;
+            for (long long pt = split; pt < total_ptiles && ok; pt += splits) {
+                for (int g = 0; g < ngroups; ++g) {
                     if (!mbar_wait(full_bar(s), ph, p.status, DS_TIMEOUT_FULL)) { ok = false; break; }
                     tc_fence_after();
                     const uint32_t a0 = smem_base + s * Cfg::STAGE_BYTES;
-                    const uint32_t b0 = a0 + MB * TILE_A_BYTES;
+                    uint64_t da = make_smem_desc(a0, TILE_A_BYTES, SBO, LT);
+                    uint64_t db = make_smem_desc(a0 + MB * TILE_A_BYTES, TILE_A_BYTES, SBO, LT);
                     const uint32_t d_tmem = tmem_base + g * NTP;
+                    uint32_t acc = acc0;
+#pragma unroll 4
                     for (int kk = 0; kk < ksteps; ++kk) {
-                        const uint32_t koff = kk * Cfg::KROWS * 128;
-                        // MN-major operands: 16-bit types use the plain 128-byte swizzle (8-row K groups);
-                        // 32-bit types need the 32-byte-unit variant (4-row K groups).
-                        constexpr uint32_t LT = TF32 ? 1u : 2u;
-                        constexpr uint32_t SBO = TF32 ? 512u : 1024u;
-                        if (PAIR)
-                            umma_pair<TF32>(d_tmem, make_smem_desc(a0 + koff, TILE_A_BYTES, SBO, LT),
-                                            make_smem_desc(b0 + koff, TILE_A_BYTES, SBO, LT), idesc, (!first || kk > 0) ? 1u : 0u);
-                        else
-                            umma<TF32>(d_tmem, make_smem_desc(a0 + koff, TILE_A_BYTES, SBO, LT),
-                                       make_smem_desc(b0 + koff, TILE_A_BYTES, SBO, LT), idesc, (!first || kk > 0) ? 1u : 0u);
+                        if (PAIR) umma_pair<TF32>(d_tmem, da, db, idesc, acc);
+                        else umma<TF32>(d_tmem, da, db, idesc, acc);
+                        acc = 1u;
+                        da += Cfg::KROWS * 128 / 16;
+                        db += Cfg::KROWS * 128 / 16;
                     }
                     if (PAIR) {
                         umma_commit_pair(empty_bar(s));
@@ -656,7 +674,9 @@ __global__ void __launch_bounds__(DW_THREADS, 1) dw_conv_kernel(const __grid_con
                     } else {
                         umma_commit(empty_bar(s));
                     }
+                    if (++s == STAGES) { s = 0; ph ^= 1u; }
                 }
+                acc0 = 1u;
             }
             if (PAIR) {
                 umma_commit_pair(done_bar);
@@ -667,15 +687,18 @@ __global__ void __launch_bounds__(DW_THREADS, 1) dw_conv_kernel(const __grid_con
         }
     } else {
         const int q = warp & 3;
-        const int row = q * 32 + lane;
         const bool any_tiles = split < total_ptiles;
         bool ok = true;
         if (any_tiles) ok = mbar_wait(done_bar, 0, p.status, DS_TIMEOUT_TMEM_FULL);
         tc_fence_after();
         if (ok) {
-            const int m = row / UC, c_in = row % UC;
+            // this warp's 32 rows belong to one unit: rows c_in0 .. c_in0 + 31 of its channel block
+            const int m = q * 32 / UC, c_in0 = q * 32 % UC;
+            float* stage = reinterpret_cast<float*>(gen_base) + q * STORE_BLOCK_FLOATS;       // every MMA has read its operands
             for (int g = 0; g < ngroups; ++g) {
                 const int u = ((g_begin + g) * PF + cta_rank) * MB + m;
+                const int rows = u < p.U ? p.Cin - (u % p.cblocks) * UC - c_in0 : 0;
+                float* dst = p.part + (((size_t)split * p.U + u) * UC + c_in0) * (size_t)p.ldn + nt * NTP;
 #pragma unroll 1
                 for (int ch = 0; ch < NTP / 32; ++ch) {
                     uint32_t r[32];
@@ -686,15 +709,7 @@ __global__ void __launch_bounds__(DW_THREADS, 1) dw_conv_kernel(const __grid_con
 #pragma unroll
                         for (int k = 0; k < 32; ++k) r[k] = 0u;
                     }
-                    if (u < p.U && (u % p.cblocks) * UC + c_in < p.Cin) {
-                        float4* dst = reinterpret_cast<float4*>(
-                            p.part + (((size_t)split * p.U + u) * UC + c_in) * (size_t)p.ldn + nt * NTP + ch * 32);
-#pragma unroll
-                        for (int k = 0; k < 8; ++k)
-                            if (nt * NTP + ch * 32 + 4 * k < p.Cout)            // (Cout % 4 == 0)
-                                dst[k] = make_float4(__uint_as_float(r[4 * k]), __uint_as_float(r[4 * k + 1]),
-                                                     __uint_as_float(r[4 * k + 2]), __uint_as_float(r[4 * k + 3]));
-                    }
+                    store_block_32x32(stage, r, dst + ch * 32, p.ldn, rows, p.Cout - nt * NTP - ch * 32, lane);
                 }
             }
         }
@@ -732,84 +747,65 @@ __device__ __forceinline__ void finish_columns(const float* __restrict__ part, i
 
 // dW[tap][c][d] = sum over splits of part[split][tap*cblocks + c/UC][c%UC][d]
 // Taps from tap_split on have splits2 partials instead of splits (kernels whose CTA classes differ in number).
-// A block of 256 threads handles 32 consecutive outputs with 8 lanes each: lane l adds splits l, l+8, ... and the
-// lanes are combined in fixed order through shared memory (bit-reproducible; many loads in flight per output).
+// Four consecutive output channels per thread; 1 << lane_bits threads share an output, thread l of them adds splits l,
+// l + lanes, ... and they are combined in fixed order through shared memory (bit-reproducible).  Bound by L2: what counts is
+// loads in flight, so lanes are used only where there are few outputs (dw_reduce_lane_bits).
 // `nred` CTAs do that; the CTAs behind them finish dB, which saves a launch of its own.
 __global__ void __launch_bounds__(256) dw_reduce_kernel(const float* __restrict__ part, float* __restrict__ dw, int splits,
                                                         int U, int UC, int ldn, int cblocks, int taps, int Cin, int Cout,
-                                                        int tap_split, int splits2, int nred, const float* __restrict__ dbpart,
-                                                        int db_rows, float* __restrict__ db) {
+                                                        int tap_split, int splits2, int lane_bits, int nred,
+                                                        const float* __restrict__ dbpart, int db_rows, float* __restrict__ db) {
     pdl_wait();
-    __shared__ float red[8][32];
-    __shared__ float4 red4[8][32];
+    __shared__ float4 red4[256];
     if ((int)blockIdx.x >= nred) {                     // the blocks behind: dB from the column sums that came with dy's copy
-        finish_columns(dbpart, db_rows, Cout, db, (int)blockIdx.x - nred, reinterpret_cast<float (*)[8]>(red));
+        finish_columns(dbpart, db_rows, Cout, db, (int)blockIdx.x - nred, reinterpret_cast<float (*)[8]>(red4));
         return;
     }
-    const int el = threadIdx.x & 31, ln = threadIdx.x >> 5;
-    const long long total = 1LL * taps * Cin * Cout;
+    const int per = 256 >> lane_bits, lanes = 1 << lane_bits;       // outputs of a CTA, threads per output
+    const int el = threadIdx.x & (per - 1), ln = threadIdx.x >> (8 - lane_bits);
+    const int Cq = Cout >> 2;                          // (Cout % 4 == 0, ldn a multiple of 32)
+    const long long total4 = 1LL * taps * Cin * Cq;
     const size_t split_stride = (size_t)U * UC * ldn;
-    if ((Cout & 3) == 0 && (ldn & 3) == 0) {           // four consecutive output channels per thread
-        const int Cq = Cout >> 2;
-        const long long total4 = total >> 2;
-        for (long long base = blockIdx.x * 32LL; base < total4; base += nred * 32LL) {
-            const long long i4 = base + el;
-            float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (i4 < total4) {
-                const int d = (int)(i4 % Cq) * 4;
-                const long long tc = i4 / Cq;
-                const int c = (int)(tc % Cin);
-                const int tap = (int)(tc / Cin);
-                const int u = tap * cblocks + c / UC;
-                const float* src = part + ((size_t)u * UC + (c % UC)) * (size_t)ldn + d;
-                const int ns = tap < tap_split ? splits : splits2;
-#pragma unroll 4
-                for (int s = ln; s < ns; s += 8) {
-                    const float4 v = *reinterpret_cast<const float4*>(src + s * split_stride);
-                    acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
-                }
-            }
-            red4[ln][el] = acc;
-            __syncthreads();
-            if (ln == 0 && i4 < total4) {
-                float4 t = red4[0][el];
-#pragma unroll
-                for (int l = 1; l < 8; ++l) { const float4 v = red4[l][el]; t.x += v.x; t.y += v.y; t.z += v.z; t.w += v.w; }
-                *reinterpret_cast<float4*>(dw + i4 * 4) = t;
-            }
-            __syncthreads();
-        }
-        return;
-    }
-    for (long long base = blockIdx.x * 32LL; base < total; base += nred * 32LL) {
-        const long long idx = base + el;
-        float acc = 0.f;
-        if (idx < total) {
-            const int d = (int)(idx % Cout);
-            const long long tc = idx / Cout;
+    for (long long base = 1LL * blockIdx.x * per; base < total4; base += 1LL * nred * per) {
+        const long long i4 = base + el;
+        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (i4 < total4) {
+            const int d = (int)(i4 % Cq) * 4;
+            const long long tc = i4 / Cq;
             const int c = (int)(tc % Cin);
             const int tap = (int)(tc / Cin);
             const int u = tap * cblocks + c / UC;
             const float* src = part + ((size_t)u * UC + (c % UC)) * (size_t)ldn + d;
             const int ns = tap < tap_split ? splits : splits2;
-            for (int s = ln; s < ns; s += 8) acc += src[s * split_stride];
+#pragma unroll 8
+            for (int s = ln; s < ns; s += lanes) {
+                const float4 v = *reinterpret_cast<const float4*>(src + s * split_stride);
+                acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
+            }
         }
-        red[ln][el] = acc;
-        __syncthreads();
-        if (ln == 0 && idx < total) {
-            float t = 0.f;
-#pragma unroll
-            for (int l = 0; l < 8; ++l) t += red[l][el];
-            dw[idx] = t;
+        if (lanes > 1) {
+            red4[threadIdx.x] = acc;
+            __syncthreads();
+            if (ln == 0)
+                for (int l = 1; l < lanes; ++l) { const float4 v = red4[l * per + el]; acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w; }
+            __syncthreads();
         }
-        __syncthreads();
+        if (ln == 0 && i4 < total4) *reinterpret_cast<float4*>(dw + i4 * 4) = acc;
     }
 }
 
-static int dw_reduce_grid(int taps, int Cin, int Cout) {
-    const long long groups = (1LL * taps * Cin * Cout + 31) / 32;
-    const long long cap = 8LL * 148;
-    return (int)(groups < cap ? (groups < 1 ? 1 : groups) : cap);
+// Threads per output: enough for some 64K threads (128 blocks of 16 warps), at most eight and no more than splits.
+static int dw_reduce_lane_bits(int taps, int Cin, int Cout, int splits) {
+    const long long total4 = 1LL * taps * Cin * (Cout / 4);
+    int bits = 0;
+    while (bits < 3 && (total4 << bits) < 65536 && (2 << bits) <= splits) ++bits;
+    return bits;
+}
+static int dw_reduce_grid(int taps, int Cin, int Cout, int lane_bits) {
+    const long long per = 256 >> lane_bits;
+    const long long groups = (1LL * taps * Cin * (Cout / 4) + per - 1) / per;
+    const long long cap = 8LL * num_sms();
+    return (int)(groups < cap ? groups : cap);
 }
 
 // ====================================================================================== shadow copies
@@ -878,29 +874,35 @@ __global__ void __launch_bounds__(256) cast_bf16_kernel(const float* __restrict_
     }
 }
 
-// Column sums of an fp32 [rows][C] matrix into part[block][C] (used for dB when no cast pass runs).
+// Column sums of an fp32 [rows][C] matrix into part[block][C] (used for dB when no cast pass runs; C % 4 == 0, 16-byte
+// aligned).  Four channels per thread, eight rows in flight.
 __global__ void __launch_bounds__(256) colsum_kernel(const float* __restrict__ src, long long rows, int C,
                                                      float* __restrict__ part, long long rows_per_block) {
     pdl_wait();
     const long long r_begin = blockIdx.x * rows_per_block;
     long long r_end = r_begin + rows_per_block;
     if (r_end > rows) r_end = rows;
-    // thread -> (column group, row lane) so that a warp reads consecutive addresses when C <= 256
-    const int cols = C < 256 ? C : 256;
-    const int lanes = 256 / cols > 0 ? 256 / cols : 1;
-    __shared__ float red[256];
-    for (int cbase = 0; cbase < C; cbase += cols) {
+    const int C4 = C >> 2;
+    const int cols = C4 < 256 ? C4 : 256;
+    const int lanes = 256 / cols;
+    __shared__ float4 red[256];
+    for (int cbase = 0; cbase < C4; cbase += cols) {
         const int c = cbase + threadIdx.x % cols;
         const int rl = threadIdx.x / cols;
-        float acc = 0.f;
-        if (rl < lanes && c < C)
-            for (long long r = r_begin + rl; r < r_end; r += lanes) acc += src[r * C + c];
+        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (rl < lanes && c < C4) {
+            const float4* s = reinterpret_cast<const float4*>(src) + c;
+#pragma unroll 8
+            for (long long r = r_begin + rl; r < r_end; r += lanes) {
+                const float4 v = s[r * C4];
+                acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
+            }
+        }
         red[threadIdx.x] = acc;
         __syncthreads();
-        if (threadIdx.x < cols && c < C) {
-            float s = 0.f;
-            for (int l = 0; l < lanes; ++l) s += red[l * cols + threadIdx.x];
-            part[(size_t)blockIdx.x * C + c] = s;
+        if (threadIdx.x < cols && c < C4) {
+            for (int l = 1; l < lanes; ++l) { const float4 v = red[l * cols + threadIdx.x]; acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w; }
+            reinterpret_cast<float4*>(part + (size_t)blockIdx.x * C)[c] = acc;
         }
         __syncthreads();
     }
@@ -1181,6 +1183,16 @@ bool tc_conv_operand_layout(const AetherConvDesc& d, AetherOperandLayout* out) {
     return true;
 }
 
+// Column tile: the widest that divides the padded output channels (fewest reads of the pixel operand), halved while there
+// are tiles for less than half of the SMs: with few tiles a CTA waits for its own stream of operands out of L2 (some 145
+// GB/s per SM), and narrower tiles split the filter's part of that over idle SMs (128 rows of a
+// Dense layer 2048 -> 256: 15.7 -> 12.3 us; 64 images 7x7 128 -> 256: 12.0 -> 9.2 us).
+static int pick_nt(int n_padded, long long m_tiles) {
+    int nt = n_padded % 256 == 0 ? 256 : n_padded % 128 == 0 ? 128 : n_padded % 64 == 0 ? 64 : 32;
+    while (nt > 32 && m_tiles * (n_padded / nt) * 2 <= num_sms()) nt /= 2;
+    return nt;
+}
+
 // CTAs of the per-tap kernel.  With statistics the grid is a multiple of the number of column tiles, so that a
 // CTA (tiles blockIdx.x + k * grid, column tile = tile % n_tiles_n) keeps one column tile throughout.
 static int igemm_grid(long long m_tiles, int n_tiles_n, bool stats) {
@@ -1235,13 +1247,6 @@ static int launch_igemm(const IgemmParams& p, bool pair, cudaStream_t st) {
     return p.stats ? launch_igemm_k<TF32, NT, true, false>(p, st) : launch_igemm_k<TF32, NT, false, false>(p, st);
 }
 
-static int pick_nt(int n_padded) {
-    if (n_padded % 256 == 0) return 256;
-    if (n_padded % 128 == 0) return 128;
-    if (n_padded % 64 == 0) return 64;
-    return 32;
-}
-
 template <bool TF32>
 static int dispatch_igemm(IgemmParams& p, int nt, bool pair, cudaStream_t st) {
     switch (nt) {
@@ -1271,7 +1276,7 @@ static int run_igemm(bool tf32, const void* in, int in_C, int in_H, int in_W, in
     const int elt = tf32 ? 4 : 2;
     const int KC = 128 / elt;
     const CUtensorMapDataType dt = tf32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
-    const int nt = pick_nt(n_padded);
+    const int nt = pick_nt(n_padded, til.total());
     const bool pair = igemm_use_pairs(til.total(), nt, ceil_div(n_padded, nt));   // each CTA of a pair stages half the filter rows
     int rc;
     if ((rc = make_map_nhwc(&p.tm_in, in, dt, elt, in_C, in_W, in_H, S, KC, til.BW, til.BH, til.BN))) return rc;
@@ -1320,7 +1325,7 @@ long long tc_conv_stats_blocks(const AetherConvDesc& d) {
                                                  pl.Cout_p, d.fH, d.fW);
     if (hb > 0) return hb;
     // per-tap kernel: one row per CTA group (the CTAs of one set of pixel tiles)
-    const int nt = pick_nt(pl.Cout_p);
+    const int nt = pick_nt(pl.Cout_p, pl.til_out.total());
     const int n_tiles_n = ceil_div(pl.Cout_p, nt);
     if (igemm_use_pairs(pl.til_out.total(), nt, n_tiles_n)) {       // one block group per CTA of a pair
         const int pairs = igemm_pair_grid(pl.til_out.total(), n_tiles_n, true) / 2;
@@ -1437,9 +1442,10 @@ int tc_conv_bwd(const AetherConvDesc& d, const float* x, const float* dy, const 
     // ---- dW: split over pixel tiles, fixed-order reduction of the partials
     bool dw_done = false, db_done = db == nullptr;
     auto reduce_dw = [&](const float* part, int splits, int tap_split, int splits2) {
-        const int nred = dw_reduce_grid(pl.taps, d.Cin, d.Cout);
+        const int bits = dw_reduce_lane_bits(pl.taps, d.Cin, d.Cout, splits);
+        const int nred = dw_reduce_grid(pl.taps, d.Cin, d.Cout, bits);
         launch(dw_reduce_kernel, nred + (db ? ceil_div(d.Cout, 8) : 0), 256, 0, st, part, dw, splits, pl.dw_U, pl.KC, pl.Cout_p,
-               pl.dw_cblocks, pl.taps, d.Cin, d.Cout, tap_split, splits2, nred, dbpart, db_rows, db);
+               pl.dw_cblocks, pl.taps, d.Cin, d.Cout, tap_split, splits2, bits, nred, dbpart, db_rows, db);
         db_done = true;
         count_launch();
         return check_launch("dw_reduce_kernel");
