@@ -2,21 +2,23 @@
 // statistics partials runs inside the pass over the data instead of in a launch of its own.
 //
 // A small tensor's pass takes three to five microseconds, and the finalize kernels before it (layers.cu) five to seven: a
-// handful of CTAs on a chain of L2 round trips.  Here the grid is channel blocks of 32 x chunks of the pixels, two CTAs per
-// SM; every CTA merges the partials of its own 32 channels (the producers write at most one row of partials per CTA, 148:
-// 57 KB out of L2, sixteen warps side by side, double precision, fixed order -- the same bits in every CTA), and the
-// coefficients go straight from shared memory into its pass.  The first chunk's CTA writes the statistics.
+// handful of CTAs on a chain of L2 round trips.  Here the grid is channel blocks of 32 x chunks of the pixels, one CTA of 32
+// warps per SM; every CTA merges the partials of its own 32 channels (the producers write at most two rows of partials per
+// CTA, 296: 114 KB out of L2 per CTA, which is why there is one per SM and not two; double precision, fixed order -- the same
+// bits in every CTA), and the coefficients go straight from shared memory into its pass.  The first chunk's CTA writes the
+// statistics.  (Clusters of four CTAs that share the merge through distributed shared memory start later than they save.)
 // Only below BN_SMALL_ELEMENTS: a large tensor is a stream of HBM traffic, for which the CTAs' 128-byte pieces and the
 // repeated merge cost more than the 7 us they save.
 #include <cuda_bf16.h>
 
 #include "common.cuh"
+#include "stats_epilogue.cuh"
 #include "tail.cuh"
 #include "tc_host.cuh"
 
 namespace aether {
 
-static constexpr int BNS_THREADS = 512, BNS_WARPS = BNS_THREADS / 32, BNS_LANES = BNS_THREADS / 8;
+static constexpr int BNS_THREADS = 1024, BNS_WARPS = BNS_THREADS / 32, BNS_LANES = BNS_THREADS / 8;
 
 // Sums of NQ quantities over the partial rows for the 32 channels of this CTA: out[q][channel] in shared memory.
 // f(entries, values[NQ]) turns the NQ entries of one partial row into what is summed.
@@ -24,7 +26,7 @@ template <int NQ, typename F>
 __device__ __forceinline__ void merge_partials(double (*red)[BNS_WARPS][32], const float* __restrict__ part, int nblocks, int C, int c,
                                                bool c_ok, F f) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    constexpr int U = 5;                                 // rows in flight per warp (148 rows: two round trips to L2)
+    constexpr int U = 5;                                 // rows in flight per warp (296 rows: two round trips to L2)
     double s[NQ];
 #pragma unroll
     for (int q = 0; q < NQ; ++q) s[q] = 0.0;
@@ -57,7 +59,7 @@ __device__ __forceinline__ void merge_partials(double (*red)[BNS_WARPS][32], con
 }
 
 template <int F>
-__global__ void __launch_bounds__(BNS_THREADS, 2) bn_small_fwd_kernel(const BnSmallFwd p) {
+__global__ void __launch_bounds__(BNS_THREADS, 1) bn_small_fwd_kernel(const BnSmallFwd p) {
     pdl_wait();
     __shared__ double red[3][BNS_WARPS][32];
     __shared__ __align__(16) float sc_s[32], sh_s[32], mk_s[32];
@@ -66,10 +68,7 @@ __global__ void __launch_bounds__(BNS_THREADS, 2) bn_small_fwd_kernel(const BnSm
     {
         const int c = cb * 32 + (threadIdx.x & 31);
         merge_partials<3>(red, p.part, p.nblocks, p.C, c, c < p.C, [](const float (&q)[3], double (&v)[3]) {
-            const double n = q[0], m = q[1];
-            v[0] = n;
-            v[1] = n * m;
-            v[2] = (double)q[2] + n * m * m;
+            stats_row_terms(q[0], q[1], q[2], v[0], v[1], v[2]);
         });
         if (threadIdx.x < 32) {                          // as bn_finalize_fwd_kernel
             float sc = 0.f, sh = 0.f, mk = 1.f;
@@ -162,7 +161,7 @@ __global__ void __launch_bounds__(BNS_THREADS, 2) bn_small_fwd_kernel(const BnSm
 // dx = k1 * g + k2 * x + k3 with g = dy [* act'(gamma * xhat + beta)] at every cell, or at the selected cell of each pooling
 // window only; the merge is bn_finalize_bwd_kernel's.
 template <int F>
-__global__ void __launch_bounds__(BNS_THREADS, 2) bn_small_bwd_kernel(const BnSmallBwd p) {
+__global__ void __launch_bounds__(BNS_THREADS, 1) bn_small_bwd_kernel(const BnSmallBwd p) {
     pdl_wait();
     __shared__ double red[2][BNS_WARPS][32];
     __shared__ __align__(16) float k_s[3][32];
@@ -269,10 +268,10 @@ __global__ void __launch_bounds__(BNS_THREADS, 2) bn_small_bwd_kernel(const BnSm
     }
 }
 
-// CTAs of a pass: two per SM in whole channel blocks, no more chunks than there are rounds of windows.
+// CTAs of a pass: one per SM in whole channel blocks, no more chunks than there are rounds of windows.
 static int small_chunks(int C, unsigned windows, int most) {
     const int ncb = ceil_div(C, 32);
-    int chunks = 2 * num_sms() / ncb;
+    int chunks = num_sms() / ncb;
     const int rounds = (int)((windows + BNS_LANES - 1) / BNS_LANES);
     if (chunks > rounds) chunks = rounds;
     if (most > 0 && chunks > most) chunks = most;

@@ -16,6 +16,8 @@
 #include <cuda_bf16.h>
 #include <string.h>
 
+#include <type_traits>
+
 #include "common.cuh"
 #include "sm100_ptx.cuh"
 #include "stats_epilogue.cuh"
@@ -111,14 +113,28 @@ struct FirstParams {
     FirstGeom g;
     const float* w;      // (fH, fW, Cin, Cout) = [K][Cout]
     const float* bias;   // nullable
-    float* stats;        // nullable: [cta][3][Cout] (count, mean, M2) partials
+    float* stats;        // nullable: [2 * cta][3][Cout] (count, mean, M2) partials (stats_epilogue.cuh)
     int* status;
     int Cout, NT, K;
     int stages, ntiles;
 };
 
-// Statistics of a column over the rows one thread sums: about the mean of its first tile (no cancellation where a channel's
-// mean is far from zero), running sums in shared memory, [3][chunks][256 epilogue threads].
+// Statistics: a thread sums one column over 32 rows of a tile, as eight sums of four rows each that a fixed tree adds up,
+// about the mean of the CTA's first tile (no cancellation where a channel's mean is far from zero).  Up to 128 channels the
+// eight sums run on over the CTA's tiles, in shared memory, and the tree comes at the end.  The two epilogue teams take
+// every other tile and add to the running sums in tile order: a team waits for the other's statistics of the tile before
+// (turn barriers, one per team and 32-channel chunk) with the tile's values already in registers, so that the exclusive part
+// is short.  (128 channels at 4096 x 32x32: 423 us with sums of each team's own, 617 with both teams on every tile, 512 so;
+// the network's statistics then do not depend on how its tiles meet the teams.)
+// Shared memory: 16 turn barriers; float4[chunks][4][128] running sums (S, S, Q, Q; up to 128 channels); float[chunks][3][128]
+// (pivot, S, Q); float[256] rows of each thread.
+static constexpr int FT_TURN_BYTES = 128;
+static int ft_stats_bytes(int NT) {
+    const int NC = NT / 32;
+    return FT_TURN_BYTES + (NT <= 128 ? NC * 4 * 128 * 16 : 0) + NC * 3 * 128 * 4 + 256 * 4;
+}
+__device__ __forceinline__ float stats_tree(const float (&v)[8]) { return ((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7])); }
+
 template <bool STATS, int KP, int CIN>
 __global__ void __launch_bounds__(FT_THREADS, 1) first_conv_kernel(const __grid_constant__ FirstParams p) {
     extern __shared__ uint8_t smem_raw[];
@@ -137,7 +153,12 @@ __global__ void __launch_bounds__(FT_THREADS, 1) first_conv_kernel(const __grid_
     volatile uint32_t* tmem_ptr_generic = reinterpret_cast<volatile uint32_t*>(gen_base + (sTmemPtr - smem_base));
     float* bias_s = reinterpret_cast<float*>(gen_base + (sBar - smem_base) + 256);         // NT <= 256 floats
     FirstTaps& taps = *reinterpret_cast<FirstTaps*>(gen_base + (sBar - smem_base) + 256 + 1024);
-    float* stat_s = reinterpret_cast<float*>(gen_base + (sBar - smem_base) + FT_TAIL);     // STATS: 3 * (NT / 32) * 256 + 256 floats
+    const uint32_t sTurn = sBar + FT_TAIL;                                                 // STATS only, see above
+    auto turn_bar = [&](int team, int ch) { return sTurn + 8u * (team * 8 + ch); };
+    const bool persist = NT <= 128;
+    float4* run_s = reinterpret_cast<float4*>(gen_base + (sTurn - smem_base) + FT_TURN_BYTES);
+    float* stat_s = reinterpret_cast<float*>(run_s + (persist ? (NT >> 5) * 4 * 128 : 0));
+    float* rows_s = stat_s + (NT >> 5) * 3 * 128;
 
     const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);
     const int lane = threadIdx.x & 31;
@@ -154,6 +175,8 @@ __global__ void __launch_bounds__(FT_THREADS, 1) first_conv_kernel(const __grid_
             mbar_init(tfull_bar(b), 1);
             mbar_init(tempty_bar(b), 4);
         }
+        if (STATS)
+            for (int b = 0; b < 16; ++b) mbar_init(sTurn + 8u * b, 4);
         mbar_fence_init();
         tma_prefetch_desc(&p.tm_y);
     }
@@ -234,14 +257,13 @@ __global__ void __launch_bounds__(FT_THREADS, 1) first_conv_kernel(const __grid_
         // statistics: this thread sums column `lane` of every chunk over rows [32 * part, 32 * part + 32)
         const int part = tt >> 5;
         float st_rows = 0.f;
-        float* st = stat_s + et;
         uint8_t* out_gen = gen_base + (sOut - smem_base) + team * 2 * FT_STAGE_BYTES;
         const uint32_t out_u = sOut + (uint32_t)(team * 2 * FT_STAGE_BYTES);
         int cnt = 0, it = team;
-        bool ok = true;
+        bool ok = true, in_turn = true;
         for (int t = blockIdx.x + team * grid; t < p.ntiles && ok; t += 2 * grid, it += 2) {
             const int buf = it % NB;
-            bool mine = mbar_wait(tfull_bar(buf), (uint32_t)(it / NB) & 1u, p.status, DS_TIMEOUT_TMEM_FULL);
+            bool mine = in_turn && mbar_wait(tfull_bar(buf), (uint32_t)(it / NB) & 1u, p.status, DS_TIMEOUT_TMEM_FULL);
             tc_fence_after();
             const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * NT);
             const int left = p.g.P - t * 128;                        // rows of this tile
@@ -273,64 +295,99 @@ __global__ void __launch_bounds__(FT_THREADS, 1) first_conv_kernel(const __grid_
                     tma_store_2d(&p.tm_y, out_u + (uint32_t)((cnt & 1) * FT_STAGE_BYTES), ch * 32, t * 128);
                     tma_store_commit();
                 }
-                if (STATS && nr > 0) {
-                    const uint8_t* col = o + (lane & 3) * 4;
-                    float piv, s = 0.f, sq = 0.f;
-                    float* sp = st + ch * 256;
-                    if (st_rows == 0.f) {                             // first tile: its mean becomes the pivot
-                        float m = 0.f;
-                        for (int r = r0; r < r0 + nr; ++r) m += *reinterpret_cast<const float*>(col + r * 128 + (((lane >> 2) ^ (r & 7)) << 4));
-                        piv = m / (float)nr;
-                        sp[2 * NC * 256] = piv;
-                    } else {
-                        piv = sp[2 * NC * 256];
-                        s = sp[0];
-                        sq = sp[NC * 256];
-                    }
-                    if (nr == 32) {
+                if (STATS) {
+                    const bool first = it == 0;                       // sets the pivots
+                    const uint8_t* col = o + r0 * 128 + (lane & 3) * 4;
+                    float val[32];                                    // (rows past the last are never added)
 #pragma unroll
-                        for (int r = 0; r < 32; ++r) {
-                            const float d = *reinterpret_cast<const float*>(col + (r0 + r) * 128 + (((lane >> 2) ^ (r & 7)) << 4)) - piv;
-                            s += d;
-                            sq = fmaf(d, d, sq);
+                    for (int r = 0; r < 32; ++r) val[r] = *reinterpret_cast<const float*>(col + r * 128 + (((lane >> 2) ^ (r & 7)) << 4));
+                    if (!first)                                       // the other team has added the tile before
+                        in_turn = in_turn && mbar_wait(turn_bar(team, ch), (uint32_t)((it >> 1) - (team == 0 ? 1 : 0)) & 1u, p.status, DS_TIMEOUT_TMEM_FULL);
+                    if (in_turn && nr > 0) {
+                        float* base = stat_s + ch * 3 * 128 + tt;
+                        float4* run = run_s + ch * 4 * 128 + tt;
+                        const float npiv = first ? 0.f : -base[0];
+                        float s8[8], q8[8];
+                        if (persist && !first) {
+#pragma unroll
+                            for (int h = 0; h < 2; ++h) {
+                                *reinterpret_cast<float4*>(s8 + 4 * h) = run[h * 128];
+                                *reinterpret_cast<float4*>(q8 + 4 * h) = run[(2 + h) * 128];
+                            }
+                        } else {
+#pragma unroll
+                            for (int k = 0; k < 8; ++k) s8[k] = q8[k] = 0.f;
                         }
-                    } else {
-                        for (int r = r0; r < r0 + nr; ++r) {
-                            const float d = *reinterpret_cast<const float*>(col + r * 128 + (((lane >> 2) ^ (r & 7)) << 4)) - piv;
-                            s += d;
-                            sq = fmaf(d, d, sq);
+                        auto add_rows = [&](auto all) {
+#pragma unroll
+                            for (int r = 0; r < 32; ++r)
+                                if (decltype(all)::value || r < nr) {
+                                    const float d = val[r] + npiv;
+                                    s8[r & 7] += d;
+                                    q8[r & 7] = fmaf(d, d, q8[r & 7]);
+                                }
+                        };
+                        if (nr == 32) add_rows(std::true_type{});
+                        else add_rows(std::false_type{});
+                        if (!persist || first) {
+                            float s = stats_tree(s8), sq = stats_tree(q8);
+                            if (first) {
+                                const float piv = s * (1.f / (float)nr);
+                                base[0] = piv;
+                                base[128] = 0.f;
+                                base[256] = sq - s * piv;
+                            } else {
+                                base[128] += s;
+                                base[256] += sq;
+                            }
+#pragma unroll
+                            for (int k = 0; k < 8; ++k) s8[k] = q8[k] = 0.f;
+                        }
+                        if (persist) {
+#pragma unroll
+                            for (int h = 0; h < 2; ++h) {
+                                run[h * 128] = *reinterpret_cast<const float4*>(s8 + 4 * h);
+                                run[(2 + h) * 128] = *reinterpret_cast<const float4*>(q8 + 4 * h);
+                            }
                         }
                     }
-                    sp[0] = s;
-                    sp[NC * 256] = sq;
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(turn_bar(team ^ 1, ch));
                 }
             }
             st_rows += (float)nr;
         }
         if (tt == 0) tma_store_wait_all<0>();
         if (STATS) {
-            // one (count, mean, M2) row per CTA: the eight threads of a column merged in fixed order
-            float* rows_s = stat_s + 3 * NC * 256;
+            // two rows per CTA (stats_epilogue.cuh): the four threads of a column merged in fixed order
             rows_s[et] = st_rows;
             named_bar_sync(3, 256);
-            float* sp = p.stats + (size_t)blockIdx.x * 3 * p.Cout;
-            for (int col = et; col < p.Cout; col += 256) {
-                float N = 0.f, M = 0.f, M2 = 0.f;
+            float* sp = p.stats + (size_t)blockIdx.x * 6 * p.Cout;
+            for (int c = et; c < p.Cout; c += 256) {
+                double N = 0.0, S = 0.0, Q = 0.0;
 #pragma unroll
-                for (int k = 0; k < 8; ++k) {
-                    const int th = k * 32 + (col & 31);
-                    const float n = rows_s[th];
+                for (int k = 0; k < 4; ++k) {
+                    const int th = k * 32 + (c & 31);
+                    const float n = rows_s[th] + rows_s[128 + th];
                     if (n == 0.f) continue;
-                    const float* a = stat_s + (col >> 5) * 256 + th;
-                    const float s = a[0], m = s / n, m2 = fmaxf(a[NC * 256] - s * m, 0.f), mean = a[2 * NC * 256] + m;
-                    const float tot = N + n, delta = mean - M;
-                    M2 += m2 + delta * delta * N * n / tot;
-                    M += delta * n / tot;
-                    N = tot;
+                    const float* base = stat_s + (c >> 5) * 3 * 128 + th;
+                    float s = base[128], q = base[256];
+                    if (persist) {
+                        const float4* run = run_s + (c >> 5) * 4 * 128 + th;
+                        float v[8];
+                        *reinterpret_cast<float4*>(v) = run[0];
+                        *reinterpret_cast<float4*>(v + 4) = run[128];
+                        s += stats_tree(v);
+                        *reinterpret_cast<float4*>(v) = run[256];
+                        *reinterpret_cast<float4*>(v + 4) = run[384];
+                        q += stats_tree(v);
+                    }
+                    const float m = s / n, mean = base[0] + m, m2 = fmaxf(q - s * m, 0.f);
+                    double dn, ds, dq;
+                    stats_row_terms(n, mean, m2, dn, ds, dq);
+                    N += dn; S += ds; Q += dq;
                 }
-                sp[col] = N;
-                sp[p.Cout + col] = M;
-                sp[2 * p.Cout + col] = M2;
+                stats_store_rows(N, S, Q, sp, c, p.Cout);
             }
         }
     }
@@ -601,7 +658,7 @@ long long first_tc_stats_blocks(const AetherConvDesc& d) {
     int K, KP, NT, Ho, Wo;
     if (!first_tc_shape(d, K, KP, NT, Ho, Wo)) return 0;
     const long long P = 1LL * d.S * Ho * Wo;
-    return first_tc_grid((P + 127) / 128);
+    return 2LL * first_tc_grid((P + 127) / 128);
 }
 
 static FirstGeom first_geom(const AetherConvDesc& d, const float* x, int Ho, int Wo) {
@@ -626,7 +683,7 @@ int first_tc_fwd(const AetherConvDesc& d, const float* x, const float* w, const 
     p.ntiles = (p.g.P + 127) / 128;
     p.stages = 4;
     if (int rc = make_map_2d(&p.tm_y, y, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, d.Cout, p.g.P, 32, 128)) return rc;
-    const int stat_bytes = stats ? (3 * (NT / 32) * 256 + 256) * 4 : 0;
+    const int stat_bytes = stats ? ft_stats_bytes(NT) : 0;
     const int smem = 1024 + NT * 128 + p.stages * FT_STAGE_BYTES + FT_OUT_BYTES + FT_TAIL + stat_bytes;
     using KernelFn = void (*)(const FirstParams);
     static const KernelFn kernels[2][6] = {{first_conv_kernel<false, 16, 0>, first_conv_kernel<false, 32, 0>, first_conv_kernel<false, 48, 0>,

@@ -37,8 +37,8 @@ struct HaloParams {
     CUtensorMap tm_w;    // filter matrix (K, taps*rows_per_tap), box (128 B of K, NT)
     float* out;          // (N, Hout, Wout, n_out) fp32
     const float* bias;   // nullable
-    float* stats;        // nullable: per CTA (count, mean, M2) of every output channel,
-                         // [cta][3][n_out] -- the partials Batch_Norm's statistics are merged from
+    float* stats;        // nullable: per CTA two rows of (count, mean, M2) of every output channel,
+                         // [2 * cta][3][n_out] -- the partials Batch_Norm's statistics are merged from
     int* status;
     int n_out;           // real output channels
     int NT;              // accumulator columns (padded output channels), multiple of 32, <= 256
@@ -418,9 +418,9 @@ __global__ void __launch_bounds__(HALO_THREADS, 1) halo_conv_kernel(const __grid
             st_rows += tile_rows;
             if (++buf == NB) { buf = 0; aph ^= 1u; }
         }
-        if (do_stats)                             // one (count, mean, M2) row per CTA, [cta][3][n_out]
+        if (do_stats)                             // two rows per CTA, [2 * cta][3][n_out]
             stats_merge_store(reinterpret_cast<float*>(gen_base + (sBar - smem_base) + HALO_TAIL), ew, lane, st_rows, ncols, 0, p.n_out, bias_s,
-                              p.stats + (size_t)blockIdx.x * 3 * p.n_out);
+                              p.stats + (size_t)blockIdx.x * 6 * p.n_out);
     }
 
     tc_fence_before();
@@ -490,12 +490,12 @@ static bool halo_geometry(bool tf32, int in_C, int S, int taps, int out_C, int o
 }
 
 // Number of (count, mean, M2) partial blocks the kernel writes per output channel when asked for statistics
-// (one per CTA), or 0 when the halo kernel does not take this problem.
+// (two per CTA), or 0 when the halo kernel does not take this problem.
 long long halo_igemm_stats_blocks(bool tf32, int in_C, int S, int taps, int out_C, int out_H, int out_W, int n_padded,
                                   int fH, int fW) {
     HaloGeom g;
     if (!halo_geometry(tf32, in_C, S, taps, out_C, out_H, out_W, n_padded, fH, fW, g)) return 0;
-    return g.grid;             // one row per CTA
+    return 2LL * g.grid;       // two rows per CTA (stats_epilogue.cuh)
 }
 
 int run_halo_igemm(bool tf32, const void* in, int in_C, int in_H, int in_W, int S, const void* wmat, int w_inner,

@@ -110,7 +110,7 @@ struct IgemmParams {
     CUtensorMap tm_w;    // filter matrix, K contiguous: (K, taps * rows_per_tap), box (128 B of K, NT)
     float* out;          // fp32 output, NHWC (out_N, out_H, out_W, n_out), 16-byte aligned, n_out % 4 == 0
     const float* bias;   // nullable, n_out entries
-    float* stats;        // STATS only: [gridDim.x / n_tiles_n][3][n_out] (count, mean, M2) partial rows
+    float* stats;        // STATS only: [2 * gridDim.x / n_tiles_n][3][n_out] (count, mean, M2) partial rows
     int* status;
     int n_out;
     int out_W, out_H, out_N;   // output extent: accumulator rows outside it are by-products
@@ -468,13 +468,13 @@ __global__ void __launch_bounds__(IGEMM_THREADS, 1) igemm_conv_kernel(const __gr
             st_rows += tile_rows;
         }
         if (STATS) {
-            // One (count, mean, M2) row per CTA group: the grid is a multiple of n_tiles_n, so the CTA kept column tile
-            // blockIdx.x % n_tiles_n, and the n_tiles_n CTAs of a group fill the disjoint column ranges of row `group` of
-            // [3][n_out].  (PAIR: the same with pairs in the place of CTAs and one row per CTA of the pair.)
+            // Two rows (stats_epilogue.cuh) per CTA group: the grid is a multiple of n_tiles_n, so the CTA kept column tile
+            // blockIdx.x % n_tiles_n, and the n_tiles_n CTAs of a group fill the disjoint column ranges of rows 2 * group
+            // and 2 * group + 1 of [3][n_out].  (PAIR: the same with pairs in the place of CTAs and two rows per CTA of the pair.)
             const int ntc = (int)(t_first % p.n_tiles_n);
             const size_t group = PAIR ? (size_t)(t_first / p.n_tiles_n) * 2 + cta_rank : (size_t)(t_first / p.n_tiles_n);
             stats_merge_store(reinterpret_cast<float*>(gen_base + (sBar - smem_base) + IGEMM_TAIL), ew, lane, st_rows, ncols, ntc * NT, p.n_out,
-                              p.bias, p.stats + group * 3 * (size_t)p.n_out);
+                              p.bias, p.stats + group * 6 * (size_t)p.n_out);
         }
     }
 
@@ -1324,17 +1324,17 @@ long long tc_conv_stats_blocks(const AetherConvDesc& d) {
     const long long hb = halo_igemm_stats_blocks(pl.tf32, pl.tf32 ? d.Cin : pl.Cin_p, d.S, pl.taps, d.Cout, pl.Ho, pl.Wo,
                                                  pl.Cout_p, d.fH, d.fW);
     if (hb > 0) return hb;
-    // per-tap kernel: one row per CTA group (the CTAs of one set of pixel tiles)
+    // per-tap kernel: two rows per CTA group (the CTAs of one set of pixel tiles)
     const int nt = pick_nt(pl.Cout_p, pl.til_out.total());
     const int n_tiles_n = ceil_div(pl.Cout_p, nt);
     if (igemm_use_pairs(pl.til_out.total(), nt, n_tiles_n)) {       // one block group per CTA of a pair
         const int pairs = igemm_pair_grid(pl.til_out.total(), n_tiles_n, true) / 2;
         if (pairs % n_tiles_n) return 0;
-        return 2LL * (pairs / n_tiles_n);
+        return 4LL * (pairs / n_tiles_n);
     }
     const int grid = igemm_grid(pl.til_out.total(), n_tiles_n, true);
     if (grid % n_tiles_n) return 0;
-    return grid / n_tiles_n;
+    return 2LL * (grid / n_tiles_n);
 }
 
 int tc_conv_fwd(const AetherConvDesc& d, const float* x, const float* w, const float* b, float* y, float* stats, void* ws,

@@ -7,6 +7,7 @@
 #include <string.h>
 
 #include "common.cuh"
+#include "stats_epilogue.cuh"
 #include "tail.cuh"
 
 namespace aether {
@@ -308,10 +309,11 @@ __global__ void __launch_bounds__(FIN_THREADS) bn_finalize_fwd_kernel(const floa
             }
 #pragma unroll
             for (int u = 0; u < U; ++u) {
-                const double nl = t[u][0], ml = t[u][1];
-                v[0] += nl;
-                v[1] += nl * ml;
-                v[2] += (double)t[u][2] + nl * ml * ml;
+                double dn, ds, dq;
+                stats_row_terms(t[u][0], t[u][1], t[u][2], dn, ds, dq);
+                v[0] += dn;
+                v[1] += ds;
+                v[2] += dq;
             }
         }
     fin_sum<3>(v);

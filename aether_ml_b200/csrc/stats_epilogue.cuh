@@ -83,10 +83,33 @@ __device__ __forceinline__ void stats_result(const float* stat_w, int c, float r
     m2 = fmaxf(q - s * m, 0.f);
 }
 
-// The end of a statistics epilogue: the four 32-row quarters of each column half are merged (Chan's formula, fixed order), so
-// a CTA hands ONE (count, mean, M2) row to whoever adds the rows up, not four.  Called by all 256 epilogue threads; `ew` is
-// the warp's index (its half is ew / 4), `stats0` warp 0's area, `rows` the rows this warp has summed, `ncols` the columns
-// of a half; out[col], out[n_out + col], out[2 n_out + col] for col = col0 + half * ncols + c below n_out.
+// One CTA's sums of a column in double -- N rows, S = sum n * mean, Q = sum (M2 + n * mean^2) over its warps' triples -- as two
+// rows of (count, mean, M2): the rounded triple, and a row of count 0 that holds what the rounding took from S and Q.  Whoever
+// adds the rows up (in double, too) gets the sums of the warps' triples as if it had read those, from half as many rows.
+__device__ __forceinline__ void stats_store_rows(double N, double S, double Q, float* out, int col, int n_out) {
+    const float mean = N > 0.0 ? (float)(S / N) : 0.f;
+    const double nm2 = N * (double)mean * (double)mean;
+    const float m2 = fmaxf((float)(Q - nm2), 0.f);
+    out[col] = (float)N;
+    out[n_out + col] = mean;
+    out[2 * (size_t)n_out + col] = m2;
+    out += 3 * (size_t)n_out;
+    out[col] = 0.f;
+    out[n_out + col] = (float)(S - N * (double)mean);
+    out[2 * (size_t)n_out + col] = (float)(Q - nm2 - (double)m2);
+}
+// What a row (n, m, m2) adds to (N, S, Q).
+__device__ __forceinline__ void stats_row_terms(float n, float m, float m2, double& dn, double& ds, double& dq) {
+    const double nl = n, ml = m;
+    dn = nl;
+    ds = n > 0.f ? nl * ml : ml;
+    dq = (double)m2 + nl * ml * ml;
+}
+
+// The end of a statistics epilogue: the four 32-row quarters of each column half are merged in fixed order, so a CTA hands
+// two rows (above) to whoever adds the rows up, not four.  Called by all 256 epilogue threads; `ew` is the warp's index (its
+// half is ew / 4), `stats0` warp 0's area, `rows` the rows this warp has summed, `ncols` the columns of a half; the rows are
+// written for col = col0 + half * ncols + c below n_out.
 __device__ __forceinline__ void stats_merge_store(float* stats0, int ew, int lane, float rows, int ncols, int col0, int n_out,
                                                   const float* bias, float* out) {
     if (lane == 0) stats0[ew * STATS_WARP_FLOATS + 3 * 128] = rows;
@@ -94,7 +117,8 @@ __device__ __forceinline__ void stats_merge_store(float* stats0, int ew, int lan
     for (int t = ew * 32 + lane; t < 2 * ncols; t += 256) {
         const int half = t >= ncols ? 1 : 0, c = t - half * ncols, col = col0 + t;
         if (col >= n_out) continue;
-        float N = 0.f, M = 0.f, M2 = 0.f;
+        const float b = bias != nullptr ? bias[col] : 0.f;
+        double N = 0.0, S = 0.0, Q = 0.0;
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
             const float* w = stats0 + (half * 4 + k) * STATS_WARP_FLOATS;
@@ -102,14 +126,11 @@ __device__ __forceinline__ void stats_merge_store(float* stats0, int ew, int lan
             if (n == 0.f) continue;
             float m, m2;
             stats_result(w, c, n, m, m2);
-            const float tot = N + n, delta = m - M;
-            M2 += m2 + delta * delta * N * n / tot;
-            M += delta * n / tot;
-            N = tot;
+            double dn, ds, dq;
+            stats_row_terms(n, m + b, m2, dn, ds, dq);
+            N += dn; S += ds; Q += dq;
         }
-        out[col] = N;
-        out[n_out + col] = M + (bias != nullptr ? bias[col] : 0.f);
-        out[2 * n_out + col] = M2;
+        stats_store_rows(N, S, Q, out, col, n_out);
     }
 }
 

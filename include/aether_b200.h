@@ -93,7 +93,8 @@ int aether_conv2d_fwd(const AetherConvDesc* desc, const float* x, const float* w
 /* Conv_Layer.forward with the Batch_Norm statistics of its output taken in the kernel's epilogue: the reference
  * computes them in a separate pass over the layer output (Batch_Norm.forward, CNN_classes_cupy.py:467-470, mean and
  * var over all axes but the last).  `stats` receives aether_conv2d_bnstats_blocks(desc) blocks of [3][Cout] floats:
- * (count, mean, M2 = sum of squared deviations) of y over the rows each block covered; hand them to
+ * (count, mean, M2 = sum of squared deviations) of y over the rows each block covered -- a block of count 0 holds the
+ * rounding errors of the blocks beside it, to be added to sum(count * mean) and sum(M2 + count * mean^2); hand them to
  * aether_bn_fwd_train_partials.  aether_conv2d_bnstats_blocks returns 0 when the forward kernel that serves the
  * shape does not produce statistics; then aether_conv2d_fwd_bnstats fails with AETHER_E_UNSUPPORTED and the
  * caller uses aether_conv2d_fwd + aether_bn_fwd_train. */
