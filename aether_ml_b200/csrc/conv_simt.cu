@@ -13,9 +13,8 @@
 // splits the input pixels of dX into s*s classes (blockIdx.z) that each see only the taps which reach them; no tap is
 // visited that contributes nothing.  Sums run over k in order within a split, splits are added in fixed order.
 // Sums are kept in pairs along the output channels for fma.rn.f32x2 (5 % over scalar FMAs: half the issue slots).
-// Measured on B200 against one thread per output element: 96 x 28x28 32->64 3x3 fp32, forward + backward, 7.2 -> 0.24 ms
-// (forward 40 TFLOP/s; the FMA pipe is active 60 % of the cycles, the rest waits for shared memory); 100 x 57x45 48->72
-// stride 2, 6.3 -> 0.50 ms.
+// Measured on B200 against one thread per output element: 96 x 28x28 32->64 3x3 fp32, forward + backward, 7.2 -> 0.22 ms
+// (43 TFLOP/s, 50 to 63 where the tiles fill whole rounds of the SMs); 100 x 57x45 48->72 stride 2, 6.3 -> 0.46 ms.
 #include "common.cuh"
 #include "tc_host.cuh"
 
@@ -60,6 +59,23 @@ struct TapPos {
     }
 };
 
+// Thread (tx, ty) of a tile of TX x TY threads: a warp is four threads wide where the tile divides that way, so that the eight
+// lanes that a 16-byte shared-memory read serves together share its rows and columns (1-2 %).
+template <int TX, int TY>
+__device__ __forceinline__ void simt_thread(int tid, int& tx, int& ty) {
+    constexpr int WX = (TX % 4 == 0 && TY % 8 == 0) ? 4 : TX, NX = TX / WX;
+    if (WX == TX) {
+        tx = tid % TX;
+        ty = tid / TX;
+    } else {
+        const int warp = tid >> 5, lane = tid & 31;
+        tx = warp % NX * WX + lane % WX;
+        ty = warp / NX * (32 / WX) + lane / WX;
+    }
+}
+// CTAs per SM that the register file should hold.
+constexpr int simt_ctas(int sums, int threads) { return threads == 256 ? 2 : (sums >= 64 ? 384 : 512) / threads; }
+
 // Two sums at a time (fma.rn.f32x2: the same roundings as two fmaf).
 __device__ __forceinline__ void fma2(unsigned long long& d, unsigned long long a, unsigned long long b) {
     asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
@@ -97,7 +113,7 @@ __device__ __forceinline__ float acc_elem(unsigned long long v, int hi) {
 
 // ---------------------------------------------------------------------------------- forward and dX
 template <int BM, int BN, int TM, int TN, bool DX, bool VEC>
-__global__ void __launch_bounds__((BM / TM) * (BN / TN), 512 / ((BM / TM) * (BN / TN)))
+__global__ void __launch_bounds__((BM / TM) * (BN / TN), simt_ctas(TM * TN, (BM / TM) * (BN / TN)))
 simt_conv_kernel(const SimtGemm g, int n_tiles_n) {
     pdl_wait();
     constexpr int THREADS = (BM / TM) * (BN / TN);
@@ -109,7 +125,8 @@ simt_conv_kernel(const SimtGemm g, int n_tiles_n) {
     __shared__ __align__(16) float As[2][BK][BM + 4];
     __shared__ __align__(16) float Bs[2][BK][BN + 4];
     const int tid = threadIdx.x;
-    const int tx = tid % (BN / TN), ty = tid / (BN / TN);
+    int tx, ty;
+    simt_thread<BN / TN, BM / TM>(tid, tx, ty);
 
     // pixel class (dX of a strided layer): rows h = hs + a * sH, taps i = ph + sH * ti
     int ph = 0, pw = 0, nH = g.fH, nW = g.fW, hs = 0, ws = 0, hq = 0, wq = 0, MH = g.OH, MW = g.OW;
@@ -321,18 +338,19 @@ struct SimtDw {
 };
 
 template <int BM, int BN, int TM, int TN, bool VEC>
-__global__ void __launch_bounds__((BM / TM) * (BN / TN), (BM == 128 && BN == 64) ? 3 : 512 / ((BM / TM) * (BN / TN)))
+__global__ void __launch_bounds__((BM / TM) * (BN / TN), simt_ctas(TM * TN, (BM / TM) * (BN / TN)))
 simt_dw_kernel(const SimtDw g, int n_tiles_n) {
     pdl_wait();
     constexpr int THREADS = (BM / TM) * (BN / TN);
     constexpr int BK = SIMT_BK;
     constexpr int MV = BM / 4, NV = BN / 4;                  // loads per pixel
     constexpr int LA = (BK * MV + THREADS - 1) / THREADS, LB = (BK * NV + THREADS - 1) / THREADS;
-    static_assert(THREADS % MV == 0, "a thread keeps its filter entries");
+    static_assert(THREADS % MV == 0 && THREADS >= BN, "a thread keeps its filter entries; one thread per column for dB");
     __shared__ __align__(16) float As[2][BK][BM + 4];
     __shared__ __align__(16) float Bs[2][BK][BN + 4];
     const int tid = threadIdx.x;
-    const int tx = tid % (BN / TN), ty = tid / (BN / TN);
+    int tx, ty;
+    simt_thread<BN / TN, BM / TM>(tid, tx, ty);
     const int kt = blockIdx.x / n_tiles_n, nt = blockIdx.x - kt * n_tiles_n;
     const int k0 = kt * BM, n0 = nt * BN;
     const long long p_begin = blockIdx.y * g.per_split;
@@ -477,20 +495,6 @@ simt_dw_kernel(const SimtDw g, int n_tiles_n) {
 }
 
 // ---------------------------------------------------------------------------------- host
-// Columns of a tile: the width that pads N least; a narrower tile re-reads the other operand more often and pays more
-// shared-memory reads per FMA, which the factors stand for.
-static int simt_pick_bn(int N) {
-    const int widths[4] = {128, 64, 32, 16};
-    const double cost[4] = {1.0, 1.05, 1.25, 1.7};
-    int best = 128;
-    double best_cost = 1e30;
-    for (int i = 0; i < 4; ++i) {
-        const double c = cost[i] * ceil_div(N, widths[i]) * widths[i];
-        if (c < best_cost) { best_cost = c; best = widths[i]; }
-    }
-    return best;
-}
-
 template <int BM, int BN, int TM, int TN, bool DX>
 static int launch_simt_conv(const SimtGemm& g, long long M, int classes, bool vec, cudaStream_t st) {
     const int ntn = ceil_div(g.N, BN);
@@ -504,16 +508,36 @@ static int launch_simt_conv(const SimtGemm& g, long long M, int classes, bool ve
     return check_launch("simt_conv_kernel");
 }
 
+// Tile of the forward pass and dX: the one whose busiest SM is through first.  An SM takes as many CTAs at a time as its
+// registers hold (`ctas`) and works at `rate` then (relative, measured: 8x8 sums per thread reach up to 63 TFLOP/s over the chip, 4x4 28); with
+// fewer it waits for latency, which is why few pixels take the small tiles.
+struct SimtTile { int bm, bn, ctas; double rate; };
+static constexpr SimtTile SIMT_CONV_TILES[] = {{128, 128, 2, 0.8}, {128, 64, 3, 1.0},  {64, 64, 6, 0.95},
+                                               {128, 32, 4, 0.7}, {128, 16, 4, 0.42}, {64, 32, 4, 0.45}};
+static int simt_pick_tile(const SimtTile* tiles, int n, long long M, int N, long long copies) {
+    int best = 0;
+    double best_cost = 1e300;
+    for (int i = 0; i < n; ++i) {
+        const SimtTile& t = tiles[i];
+        const long long count = (M + t.bm - 1) / t.bm * ceil_div(N, t.bn) * copies;
+        const long long per_sm = (count + num_sms() - 1) / num_sms(), rest = per_sm % t.ctas;
+        double cost = (double)(per_sm - rest);
+        if (rest) cost += rest / (0.1 + 0.9 * rest / t.ctas);
+        cost *= t.bm * (double)t.bn / t.rate;
+        if (cost < best_cost) { best_cost = cost; best = i; }
+    }
+    return best;
+}
+
 template <bool DX>
 static int simt_conv(const SimtGemm& g, long long M, int classes, bool vec, cudaStream_t st) {
-    const int bn = simt_pick_bn(g.N);
-    // Too few 128-row tiles to give every SM two: quarter-size tiles spread the work over more of them.
-    if (bn >= 32 && (M + 127) / 128 * ceil_div(g.N, bn) * classes < 2LL * num_sms()) return launch_simt_conv<64, 32, 4, 4, DX>(g, M, classes, vec, st);
-    switch (bn) {
-        case 128: return launch_simt_conv<128, 128, 8, 8, DX>(g, M, classes, vec, st);
-        case 64: return launch_simt_conv<128, 64, 8, 8, DX>(g, M, classes, vec, st);
-        case 32: return launch_simt_conv<128, 32, 8, 4, DX>(g, M, classes, vec, st);
-        default: return launch_simt_conv<128, 16, 4, 4, DX>(g, M, classes, vec, st);
+    switch (simt_pick_tile(SIMT_CONV_TILES, 6, M, g.N, classes)) {
+        case 0: return launch_simt_conv<128, 128, 8, 8, DX>(g, M, classes, vec, st);
+        case 1: return launch_simt_conv<128, 64, 8, 8, DX>(g, M, classes, vec, st);
+        case 2: return launch_simt_conv<64, 64, 8, 8, DX>(g, M, classes, vec, st);
+        case 3: return launch_simt_conv<128, 32, 8, 4, DX>(g, M, classes, vec, st);
+        case 4: return launch_simt_conv<128, 16, 4, 4, DX>(g, M, classes, vec, st);
+        default: return launch_simt_conv<64, 32, 4, 4, DX>(g, M, classes, vec, st);
     }
 }
 
@@ -543,10 +567,12 @@ int simt_conv_bwd_data(const AetherConvDesc& d, const float* dy, const float* w,
     return simt_conv<true>(g, M, d.sH * d.sW, vec, st);
 }
 
-// Tile and split of dW.  Rows: 128 filter entries, or 32 where there are no more (first layers); enough splits of the
-// pixels for two CTAs per SM, each at least 16 steps long so that its partial is worth writing.
+// Tile and split of dW: the tile whose padded filter entries x output channels cost least at the rate of its thread tile, and
+// as many splits of the pixels as fill the chip, each at least 16 steps long so that its partial is worth writing.
+static constexpr SimtTile SIMT_DW_TILES[] = {{128, 128, 2, 1.0}, {128, 64, 3, 0.97}, {96, 64, 4, 0.9},
+                                             {64, 64, 6, 0.85},   {64, 32, 4, 0.6},  {32, 64, 4, 0.6}};
 struct SimtDwPlan {
-    int bm, bn, tiles_k, tiles_n, splits;
+    int tile, tiles_k, tiles_n, splits;
     long long per_split;
 };
 static SimtDwPlan simt_dw_plan(const AetherConvDesc& d) {
@@ -555,12 +581,15 @@ static SimtDwPlan simt_dw_plan(const AetherConvDesc& d) {
     SimtDwPlan p;
     const int KK = d.fH * d.fW * d.Cin;
     const long long P = 1LL * d.S * Ho * Wo;
-    p.bn = d.Cout <= 32 ? 32 : simt_pick_bn(d.Cout) == 128 ? 128 : 64;
-    p.bm = KK <= 32 ? 32 : (p.bn == 32 || KK <= 64) ? 64 : 128;
-    if (p.bm == 32 || (p.bm == 64 && p.bn == 128)) p.bn = 64;
-    p.tiles_k = ceil_div(KK, p.bm);
-    p.tiles_n = ceil_div(d.Cout, p.bn);
-    const int per_sm = p.bm == 128 ? (p.bn == 128 ? 2 : 3) : 4;
+    double best = 1e300;
+    for (int i = 0; i < (int)(sizeof(SIMT_DW_TILES) / sizeof(SimtTile)); ++i) {
+        const SimtTile& t = SIMT_DW_TILES[i];
+        const double cost = 1.0 * ceil_div(KK, t.bm) * t.bm * ceil_div(d.Cout, t.bn) * t.bn / t.rate;
+        if (cost < best) { best = cost; p.tile = i; }
+    }
+    p.tiles_k = ceil_div(KK, SIMT_DW_TILES[p.tile].bm);
+    p.tiles_n = ceil_div(d.Cout, SIMT_DW_TILES[p.tile].bn);
+    const int per_sm = SIMT_DW_TILES[p.tile].ctas;
     long long want = (long long)per_sm * num_sms() / (1LL * p.tiles_k * p.tiles_n);
     const long long most = (P + 16 * SIMT_BK - 1) / (16 * SIMT_BK);
     if (want > most) want = most;
@@ -599,11 +628,14 @@ int simt_conv_bwd_filter(const AetherConvDesc& d, const float* x, const float* d
     g.P = 1LL * d.S * g.Ho * g.Wo;
     g.per_split = p.per_split;
     const bool vec = d.Cin % 4 == 0 && d.Cout % 4 == 0 && aligned16(x) && aligned16(dy);
-    if (p.bm == 128 && p.bn == 128) launch_simt_dw<128, 128, 8, 8>(g, p, vec, st);
-    else if (p.bm == 128) launch_simt_dw<128, 64, 8, 8>(g, p, vec, st);
-    else if (p.bm == 64 && p.bn == 64) launch_simt_dw<64, 64, 8, 4>(g, p, vec, st);
-    else if (p.bm == 64) launch_simt_dw<64, 32, 4, 4>(g, p, vec, st);
-    else launch_simt_dw<32, 64, 4, 4>(g, p, vec, st);
+    switch (p.tile) {
+        case 0: launch_simt_dw<128, 128, 8, 8>(g, p, vec, st); break;
+        case 1: launch_simt_dw<128, 64, 8, 8>(g, p, vec, st); break;
+        case 2: launch_simt_dw<96, 64, 8, 8>(g, p, vec, st); break;
+        case 3: launch_simt_dw<64, 64, 8, 8>(g, p, vec, st); break;
+        case 4: launch_simt_dw<64, 32, 4, 4>(g, p, vec, st); break;
+        default: launch_simt_dw<32, 64, 4, 4>(g, p, vec, st); break;
+    }
     int rc = check_launch("simt_dw_kernel");
     if (rc) return rc;
     return smallc_reduce_partials(g.part, p.splits, g.KK, d.Cout, dw, db, st);
