@@ -26,7 +26,7 @@ template <int NQ, typename F>
 __device__ __forceinline__ void merge_partials(double (*red)[BNS_WARPS][32], const float* __restrict__ part, int nblocks, int C, int c,
                                                bool c_ok, F f) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    constexpr int U = 5;                                 // rows in flight per warp (296 rows: two round trips to L2)
+    constexpr int U = NQ == 3 ? 10 : 5;                                 // rows in flight per warp (296 rows: two round trips to L2)
     double s[NQ];
 #pragma unroll
     for (int q = 0; q < NQ; ++q) s[q] = 0.0;
@@ -50,10 +50,10 @@ __device__ __forceinline__ void merge_partials(double (*red)[BNS_WARPS][32], con
     for (int q = 0; q < NQ; ++q) red[q][warp][lane] = s[q];
     __syncthreads();
     if (warp < NQ) {                                     // one warp per quantity adds the warps' sums, in order
-        double t = 0.0;
+        double t[4] = {0.0, 0.0, 0.0, 0.0};              // (four chains: a double add takes long)
 #pragma unroll
-        for (int w = 0; w < BNS_WARPS; ++w) t += red[warp][w][lane];
-        red[warp][0][lane] = t;
+        for (int w = 0; w < BNS_WARPS; ++w) t[w & 3] += red[warp][w][lane];
+        red[warp][0][lane] = (t[0] + t[1]) + (t[2] + t[3]);
     }
     __syncthreads();
 }
@@ -74,11 +74,11 @@ __global__ void __launch_bounds__(BNS_THREADS, 1) bn_small_fwd_kernel(const BnSm
             float sc = 0.f, sh = 0.f, mk = 1.f;
             if (c < p.C) {
                 const double N = red[0][0][threadIdx.x], S1 = red[1][0][threadIdx.x], Q = red[2][0][threadIdx.x];
-                const double M = N > 0 ? S1 / N : 0.0;
+                const double rN = N > 0 ? 1.0 / N : 0.0, M = S1 * rN;
                 double M2 = Q - N * M * M;
                 if (M2 < 0.0) M2 = 0.0;
-                const double var = N > 0 ? M2 / N : 0.0;
-                const double s = (double)p.gamma[c] / sqrt(var + (double)p.eps);
+                const double var = M2 * rN;
+                const double s = (double)p.gamma[c] * rsqrt(var + (double)p.eps);
                 sc = (float)s;
                 sh = (float)((double)p.beta[c] - M * s);
                 if (p.mask != nullptr) mk = p.mask[c];
@@ -178,11 +178,11 @@ __global__ void __launch_bounds__(BNS_THREADS, 1) bn_small_bwd_kernel(const BnSm
             if (c < p.C) {
                 const double ms = p.pscale ? (double)p.pscale[c] : 1.0;
                 const double sdy = red[0][0][threadIdx.x] * ms, sdyx = red[1][0][threadIdx.x] * ms;
-                const double inv = 1.0 / sqrt((double)p.var[c] + (double)p.eps);
-                const double g = p.gamma[c], N = (double)p.rows, d2 = -g * inv * inv * sdyx / N;
+                const double inv = rsqrt((double)p.var[c] + (double)p.eps), rN = 1.0 / (double)p.rows;
+                const double g = p.gamma[c], d2 = -g * inv * inv * sdyx * rN;
                 k1 = (float)(g * inv * ms);
                 k2 = (float)d2;
-                k3 = (float)(-g * inv * sdy / N - d2 * (double)p.mean[c]);
+                k3 = (float)(-g * inv * sdy * rN - d2 * (double)p.mean[c]);
                 if (chunk == 0) {
                     p.dgamma[c] = (float)sdyx;
                     p.dbeta[c] = (float)sdy;

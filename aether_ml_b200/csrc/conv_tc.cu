@@ -832,20 +832,10 @@ __global__ void __launch_bounds__(256) cast_bf16_kernel(const float* __restrict_
         for (int k = 0; k < 8; ++k) acc[k] = 0.f;
         if (plane < planes) {
             const int c0 = g * 8;
-            for (long long r = r_begin + plane; r < r_end; r += planes) {
-                float v[8];
-                const float* s = src + r * C + c0;
-                if (vec && c0 + 8 <= C) {
-                    // streaming (evict-first) reads: the fp32 source is not needed again soon, the bf16 copy
-                    // written below is, so it should be what stays in L2
-                    const float4 a = __ldcs(reinterpret_cast<const float4*>(s));
-                    const float4 b = __ldcs(reinterpret_cast<const float4*>(s + 4));
-                    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
-                    v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
-                } else {
-#pragma unroll
-                    for (int k = 0; k < 8; ++k) v[k] = (c0 + k < C) ? s[k] : 0.f;
-                }
+            // streaming (evict-first) reads: the fp32 source is not needed again soon, the bf16 copy written here is, so it
+            // should be what stays in L2
+            const bool whole = vec && c0 + 8 <= C;
+            auto take = [&](long long r, const float (&v)[8]) {
                 if (COLSUM) {
 #pragma unroll
                     for (int k = 0; k < 8; ++k) acc[k] += v[k];
@@ -854,6 +844,37 @@ __global__ void __launch_bounds__(256) cast_bf16_kernel(const float* __restrict_
 #pragma unroll
                 for (int k = 0; k < 4; ++k) o[k] = __floats2bfloat162_rn(v[2 * k], v[2 * k + 1]);
                 *reinterpret_cast<uint4*>(dst + r * Cp + c0) = *reinterpret_cast<uint4*>(o);
+            };
+            long long r = r_begin + plane;
+            if (whole) {
+                constexpr int U = 4;                     // rows in flight: eight 16-byte loads per thread
+                for (; r + (U - 1) * planes < r_end; r += U * planes) {
+                    float4 t[U][2];
+#pragma unroll
+                    for (int u = 0; u < U; ++u) {
+                        const float4* s = reinterpret_cast<const float4*>(src + (r + u * planes) * C + c0);
+                        t[u][0] = __ldcs(s);
+                        t[u][1] = __ldcs(s + 1);
+                    }
+#pragma unroll
+                    for (int u = 0; u < U; ++u) {
+                        const float v[8] = {t[u][0].x, t[u][0].y, t[u][0].z, t[u][0].w, t[u][1].x, t[u][1].y, t[u][1].z, t[u][1].w};
+                        take(r + u * planes, v);
+                    }
+                }
+            }
+            for (; r < r_end; r += planes) {
+                float v[8];
+                const float* s = src + r * C + c0;
+                if (whole) {
+                    const float4 a = __ldcs(reinterpret_cast<const float4*>(s)), b = __ldcs(reinterpret_cast<const float4*>(s + 4));
+                    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+                    v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+                } else {
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) v[k] = (c0 + k < C) ? s[k] : 0.f;
+                }
+                take(r, v);
             }
         }
         if (COLSUM) {

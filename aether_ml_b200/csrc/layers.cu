@@ -319,15 +319,15 @@ __global__ void __launch_bounds__(FIN_THREADS) bn_finalize_fwd_kernel(const floa
     fin_sum<3>(v);
     if (ln != 0 || c >= C) return;
     const double N = v[0], S1 = v[1], Q = v[2];
-    const double M = N > 0 ? S1 / N : 0.0;
+    const double rN = N > 0 ? 1.0 / N : 0.0, M = S1 * rN;
     double M2 = Q - N * M * M;
     if (M2 < 0.0) M2 = 0.0;
-    const double var = N > 0 ? M2 / N : 0.0;
+    const double var = M2 * rN;
     batch_mean[c] = (float)M;
     batch_var[c] = (float)var;
     running_mean[c] = momentum * running_mean[c] + (1.f - momentum) * (float)M;
     running_var[c] = momentum * running_var[c] + (1.f - momentum) * (float)var;
-    const double sc = (double)gamma[c] / sqrt(var + (double)eps);
+    const double sc = (double)gamma[c] * rsqrt(var + (double)eps);
     scale_shift[c] = (float)sc;
     scale_shift[C + c] = (float)((double)beta[c] - M * sc);
 }
@@ -475,11 +475,11 @@ __global__ void __launch_bounds__(FIN_THREADS) bn_finalize_bwd_kernel(const floa
     dbeta[c] = (float)sdy;
     // dx = gamma*inv/N * (N*dy - sum(dy) - xhat * sum(dy*xhat)),  xhat = (x - mean) * inv
     //    = k1*dy + k2*x + k3
-    const double inv = 1.0 / sqrt((double)var[c] + (double)eps);
-    const double g = gamma[c], N = (double)rows, mu = mean[c];
+    const double inv = rsqrt((double)var[c] + (double)eps);
+    const double g = gamma[c], rN = 1.0 / (double)rows, mu = mean[c];
     const double k1 = g * inv * ms;
-    const double k2 = -g * inv * inv * sdyx / N;
-    const double k3 = -g * inv * sdy / N - k2 * mu;
+    const double k2 = -g * inv * inv * sdyx * rN;
+    const double k3 = -g * inv * sdy * rN - k2 * mu;
     coeff[c] = (float)k1;
     coeff[C + c] = (float)k2;
     coeff[2 * C + c] = (float)k3;
