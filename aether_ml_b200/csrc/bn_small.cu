@@ -26,7 +26,7 @@ template <int NQ, typename F>
 __device__ __forceinline__ void merge_partials(double (*red)[BNS_WARPS][32], const float* __restrict__ part, int nblocks, int C, int c,
                                                bool c_ok, F f) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    constexpr int U = NQ == 3 ? 10 : 5;                                 // rows in flight per warp (296 rows: two round trips to L2)
+    constexpr int U = 5;                                 // rows in flight per warp (296 rows: two round trips to L2)
     double s[NQ];
 #pragma unroll
     for (int q = 0; q < NQ; ++q) s[q] = 0.0;
@@ -67,21 +67,26 @@ __global__ void __launch_bounds__(BNS_THREADS, 1) bn_small_fwd_kernel(const BnSm
     const int cb = blockIdx.x % ncb, chunk = blockIdx.x / ncb, chunks = gridDim.x / ncb;
     {
         const int c = cb * 32 + (threadIdx.x & 31);
+        float ga = 0.f, be = 0.f, mk = 1.f;              // (loads that need not wait for the merge)
+        if (threadIdx.x < 32 && c < p.C) {
+            ga = p.gamma[c];
+            be = p.beta[c];
+            if (p.mask != nullptr) mk = p.mask[c];
+        }
         merge_partials<3>(red, p.part, p.nblocks, p.C, c, c < p.C, [](const float (&q)[3], double (&v)[3]) {
             stats_row_terms(q[0], q[1], q[2], v[0], v[1], v[2]);
         });
         if (threadIdx.x < 32) {                          // as bn_finalize_fwd_kernel
-            float sc = 0.f, sh = 0.f, mk = 1.f;
+            float sc = 0.f, sh = 0.f;
             if (c < p.C) {
                 const double N = red[0][0][threadIdx.x], S1 = red[1][0][threadIdx.x], Q = red[2][0][threadIdx.x];
                 const double rN = N > 0 ? 1.0 / N : 0.0, M = S1 * rN;
                 double M2 = Q - N * M * M;
                 if (M2 < 0.0) M2 = 0.0;
                 const double var = M2 * rN;
-                const double s = (double)p.gamma[c] * rsqrt(var + (double)p.eps);
+                const double s = (double)ga * rsqrt(var + (double)p.eps);
                 sc = (float)s;
-                sh = (float)((double)p.beta[c] - M * s);
-                if (p.mask != nullptr) mk = p.mask[c];
+                sh = (float)((double)be - M * s);
                 if (chunk == 0) {
                     p.batch_mean[c] = (float)M;
                     p.batch_var[c] = (float)var;
@@ -169,6 +174,13 @@ __global__ void __launch_bounds__(BNS_THREADS, 1) bn_small_bwd_kernel(const BnSm
     const int cb = blockIdx.x % ncb, chunk = blockIdx.x / ncb, chunks = gridDim.x / ncb;
     {
         const int c = cb * 32 + (threadIdx.x & 31);
+        float ga = 0.f, va = 0.f, me = 0.f, ps = 1.f;
+        if (threadIdx.x < 32 && c < p.C) {
+            ga = p.gamma[c];
+            va = p.var[c];
+            me = p.mean[c];
+            if (p.pscale != nullptr) ps = p.pscale[c];
+        }
         merge_partials<2>(red, p.part, p.nblocks, p.C, c, c < p.C, [](const float (&q)[2], double (&v)[2]) {
             v[0] = q[0];
             v[1] = q[1];
@@ -176,13 +188,13 @@ __global__ void __launch_bounds__(BNS_THREADS, 1) bn_small_bwd_kernel(const BnSm
         if (threadIdx.x < 32) {
             float k1 = 0.f, k2 = 0.f, k3 = 0.f;
             if (c < p.C) {
-                const double ms = p.pscale ? (double)p.pscale[c] : 1.0;
+                const double ms = ps;
                 const double sdy = red[0][0][threadIdx.x] * ms, sdyx = red[1][0][threadIdx.x] * ms;
-                const double inv = rsqrt((double)p.var[c] + (double)p.eps), rN = 1.0 / (double)p.rows;
-                const double g = p.gamma[c], d2 = -g * inv * inv * sdyx * rN;
+                const double inv = rsqrt((double)va + (double)p.eps), rN = 1.0 / (double)p.rows;
+                const double g = ga, d2 = -g * inv * inv * sdyx * rN;
                 k1 = (float)(g * inv * ms);
                 k2 = (float)d2;
-                k3 = (float)(-g * inv * sdy * rN - d2 * (double)p.mean[c]);
+                k3 = (float)(-g * inv * sdy * rN - d2 * (double)me);
                 if (chunk == 0) {
                     p.dgamma[c] = (float)sdyx;
                     p.dbeta[c] = (float)sdy;
