@@ -220,6 +220,32 @@ extern "C" int aether_conv2d_fwd_ex(const AetherConvDesc* d, const float* x, con
     return aether_conv2d_fwd(d, x, w, b, y, ws, ws_bytes, stream);
 }
 
+extern "C" int aether_conv2d_act_fwd(const AetherConvDesc* d, const float* x, const float* w, const float* b, float* y, float* act_out,
+                                     float alpha, void* act_copy, int copy_ld, void* ws, size_t ws_bytes, int flags, void* stream) {
+    int rc = validate_desc(d, "aether_conv2d_act_fwd");
+    if (rc) return rc;
+    if (!x || !w || !y || !act_out) return set_error(AE_BAD_ARG, "aether_conv2d_act_fwd: null pointer");
+    if (!aligned16(x) || !aligned16(w) || !aligned16(y) || !aligned16(act_out) || (ws && !aligned16(ws)))
+        return set_error(AE_BAD_ARG, "aether_conv2d_act_fwd: arrays must be 16-byte aligned");
+    if (act_copy && (copy_ld < d->Cout || copy_ld % 4 || (reinterpret_cast<uintptr_t>(act_copy) & 7)))
+        return set_error(AE_BAD_ARG, "aether_conv2d_act_fwd: operand copy needs ld >= Cout, ld %% 4 == 0, 8-byte alignment");
+    if (!tc_conv_eligible(*d) || (act_copy && copy_ld > (d->Cout + 63) / 64 * 64))
+        return set_error(AE_UNSUPPORTED, "aether_conv2d_act_fwd: needs the tensor-core path and copy rows of at most the padded channels");
+    if (flags & ~(AETHER_CONV_X_COPY_READY | AETHER_CONV_W_COPY_READY)) return set_error(AE_BAD_ARG, "aether_conv2d_act_fwd: unknown flag bits 0x%x", flags);
+    if ((flags & AETHER_CONV_X_COPY_READY) && d->math_mode != AETHER_MATH_BF16)
+        return set_error(AE_UNSUPPORTED, "aether_conv2d_act_fwd: this math mode reads no operand copy of x");
+    if ((rc = pending_timeout("aether_conv2d_act_fwd"))) return rc;
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    const ActEpilogue act = {act_out, alpha, act_copy, copy_ld};
+    bool done = false;
+    if ((rc = tc_conv_fwd(*d, x, w, b, y, nullptr, ws, ws_bytes, flags, st, &act, &done)) || done) return rc;
+    int Ho, Wo;                                          // a kernel without that epilogue: the passes by themselves
+    conv_out_hw(*d, Ho, Wo);
+    const int64_t rows = 1LL * d->S * Ho * Wo;
+    if ((rc = aether_leaky_relu_fwd(y, act_out, rows * d->Cout, alpha, stream)) || !act_copy) return rc;
+    return tc_cast_operand(act_out, act_copy, rows, d->Cout, copy_ld, st);
+}
+
 extern "C" int aether_conv2d_fwd(const AetherConvDesc* d, const float* x, const float* w, const float* b, float* y,
                                  void* ws, size_t ws_bytes, void* stream) {
     int rc = validate_desc(d, "aether_conv2d_fwd");

@@ -104,8 +104,17 @@ int smallc_reduce_partials(const float* part, int nb, int K, int Cout, float* dw
 bool tc_conv_eligible(const AetherConvDesc& d);
 size_t tc_conv_workspace_bytes(const AetherConvDesc& d);
 // `stats` (nullable): per-block (count, mean, M2) of every output channel, tc_conv_stats_blocks(d) blocks of [3][Cout]
+int tc_cast_operand(const float* src, void* dst, long long rows, int C, int ld, cudaStream_t st);   // fp32 rows -> bf16 rows of ld
+// A (leaky) ReLU that the forward kernel may apply in its epilogue: its output and, nullable, the bf16 copy of
+// that in rows of `ld`.
+struct ActEpilogue {
+    float* out;
+    float alpha;
+    void* copy;
+    int ld;
+};
 int tc_conv_fwd(const AetherConvDesc& d, const float* x, const float* w, const float* b, float* y, float* stats, void* ws,
-                size_t ws_bytes, int flags, cudaStream_t st);
+                size_t ws_bytes, int flags, cudaStream_t st, const ActEpilogue* act = nullptr, bool* act_done = nullptr);
 bool tc_conv_operand_layout(const AetherConvDesc& d, AetherOperandLayout* out);
 long long tc_conv_stats_blocks(const AetherConvDesc& d);
 int tc_conv_bwd(const AetherConvDesc& d, const float* x, const float* dy, const float* w, float* dx, float* dw,

@@ -119,6 +119,7 @@ struct IgemmParams {
     int rows_per_tap;
     int fH, fW, sgn, off_h, off_w;
     int kchunks;
+    ActEpilogue act;     // ACT only
 };
 
 static constexpr int TILE_A_BYTES = 128 * 128;  // 128 pixel rows x 128 B
@@ -151,7 +152,11 @@ struct IgemmCfg {
 // own shared memory, with the byte counts of both CTAs landing on the even CTA's full barrier.  The even CTA issues
 // M = 256 MMAs that read both CTAs' stages and write both CTAs' TMEM (rows of its own pixels, all NT columns), and
 // signals both CTAs' barriers; the epilogue warps of both CTAs release the accumulator on the even CTA's barrier.
-template <bool TF32, int NT, bool STATS, bool PAIR>
+//
+// ACT: the epilogue also writes the (leaky) ReLU of the output and, when asked, the bf16 operand copy of that for the layer
+// behind (zero in the padded columns): a Dense layer and its activation of a small network are two launches of two
+// microseconds otherwise, three with the cast.
+template <bool TF32, int NT, bool STATS, bool PAIR, bool ACT = false>
 __global__ void __launch_bounds__(IGEMM_THREADS, 1) igemm_conv_kernel(const __grid_constant__ IgemmParams p) {
     using Cfg = IgemmCfg<NT, PAIR>;
     constexpr int STAGES = Cfg::STAGES;
@@ -355,12 +360,13 @@ __global__ void __launch_bounds__(IGEMM_THREADS, 1) igemm_conv_kernel(const __gr
             decode(t, nt, w0, h0, n0);
             const int col0 = nt * NT + col_begin + tcol4;             // first of this thread's columns
             float* rowp[4];
+            size_t pix[ACT ? 4 : 1];
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
                 const int w = w0 + r_w[j], h = h0 + r_h[j], n = n0 + r_n[j];
-                rowp[j] = (w < p.out_W && h < p.out_H && n < p.out_N)
-                              ? p.out + (((size_t)n * p.out_H + h) * p.out_W + w) * p.n_out + col0
-                              : nullptr;
+                const size_t at = ((size_t)n * p.out_H + h) * p.out_W + w;
+                rowp[j] = (w < p.out_W && h < p.out_H && n < p.out_N) ? p.out + at * p.n_out + col0 : nullptr;
+                if (ACT) pix[ACT ? j : 0] = at;
             }
             float tile_rows = 0.f;                 // valid rows of this tile in this warp's quarter
             if (STATS) {
@@ -428,6 +434,19 @@ __global__ void __launch_bounds__(IGEMM_THREADS, 1) igemm_conv_kernel(const __gr
                             a.z = __uint_as_float(odd ? f0 : g0);
                             a.w = __uint_as_float(odd ? f1 : g1);
                             const bool wr = cols_ok && rowp[j] != nullptr;
+                            if (ACT && rowp[j] != nullptr) {
+                                const int col = col0 + cc;
+                                float4 z = make_float4(a.x + b4.x, a.y + b4.y, a.z + b4.z, a.w + b4.w);
+                                z = make_float4(z.x > 0.f ? z.x : p.act.alpha * z.x, z.y > 0.f ? z.y : p.act.alpha * z.y,
+                                                z.z > 0.f ? z.z : p.act.alpha * z.z, z.w > 0.f ? z.w : p.act.alpha * z.w);
+                                if (!cols_ok) z = make_float4(0.f, 0.f, 0.f, 0.f);
+                                else *reinterpret_cast<float4*>(p.act.out + pix[ACT ? j : 0] * p.n_out + col) = z;
+                                if (p.act.copy != nullptr && col < p.act.ld) {
+                                    const __nv_bfloat162 o[2] = {__floats2bfloat162_rn(z.x, z.y), __floats2bfloat162_rn(z.z, z.w)};
+                                    *reinterpret_cast<uint2*>(static_cast<__nv_bfloat16*>(p.act.copy) + pix[ACT ? j : 0] * p.act.ld + col) =
+                                        *reinterpret_cast<const uint2*>(o);
+                                }
+                            }
                             if (wr)
                                 __stcs(reinterpret_cast<float4*>(rowp[j] + cc),
                                        make_float4(a.x + b4.x, a.y + b4.y, a.z + b4.z, a.w + b4.w));
@@ -1239,11 +1258,11 @@ static int igemm_pair_grid(long long m_tiles, int n_tiles_n, bool stats) {
     return 2 * pairs;
 }
 
-template <bool TF32, int NT, bool STATS, bool PAIR>
+template <bool TF32, int NT, bool STATS, bool PAIR, bool ACT = false>
 static int launch_igemm_k(const IgemmParams& p, cudaStream_t st) {
     using Cfg = IgemmCfg<NT, PAIR>;
     static PerDeviceSmem configured;
-    if (int rc = ensure_dynamic_smem(igemm_conv_kernel<TF32, NT, STATS, PAIR>, Cfg::SMEM_BYTES, configured, "igemm_conv")) return rc;
+    if (int rc = ensure_dynamic_smem(igemm_conv_kernel<TF32, NT, STATS, PAIR, ACT>, Cfg::SMEM_BYTES, configured, "igemm_conv")) return rc;
     const long long m_tiles = 1LL * p.tiles_w * p.tiles_h * p.tiles_n;
     const int grid = PAIR ? igemm_pair_grid(m_tiles, p.n_tiles_n, STATS) : igemm_grid(m_tiles, p.n_tiles_n, STATS);
     if (STATS && (grid / (PAIR ? 2 : 1)) % p.n_tiles_n)
@@ -1251,9 +1270,9 @@ static int launch_igemm_k(const IgemmParams& p, cudaStream_t st) {
     const int pk = p.sgn > 0 ? PK_IGEMM_FWD : PK_IGEMM_DX;
     prof_begin(pk, st);
     if (PAIR) {
-        launch_cluster(igemm_conv_kernel<TF32, NT, STATS, PAIR>, 2, grid, IGEMM_THREADS, Cfg::SMEM_BYTES, st, p);
+        launch_cluster(igemm_conv_kernel<TF32, NT, STATS, PAIR, ACT>, 2, grid, IGEMM_THREADS, Cfg::SMEM_BYTES, st, p);
     } else {
-        launch(igemm_conv_kernel<TF32, NT, STATS, PAIR>, grid, IGEMM_THREADS, Cfg::SMEM_BYTES, st, p);
+        launch(igemm_conv_kernel<TF32, NT, STATS, PAIR, ACT>, grid, IGEMM_THREADS, Cfg::SMEM_BYTES, st, p);
     }
     prof_end(pk, st);
     count_launch();
@@ -1264,6 +1283,9 @@ template <bool TF32, int NT>
 static int launch_igemm(const IgemmParams& p, bool pair, cudaStream_t st) {
     if constexpr (NT == 256 || NT == 128) {
         if (pair) return p.stats ? launch_igemm_k<TF32, NT, true, true>(p, st) : launch_igemm_k<TF32, NT, false, true>(p, st);
+    }
+    if constexpr (!TF32) {
+        if (p.act.out) return launch_igemm_k<TF32, NT, false, false, true>(p, st);
     }
     return p.stats ? launch_igemm_k<TF32, NT, true, false>(p, st) : launch_igemm_k<TF32, NT, false, false>(p, st);
 }
@@ -1282,7 +1304,7 @@ static int dispatch_igemm(IgemmParams& p, int nt, bool pair, cudaStream_t st) {
 static int run_igemm(bool tf32, const void* in, int in_C, int in_H, int in_W, int S, const void* wmat, int w_inner,
                      int rows_per_tap, int taps, float* out, int out_C, int out_H, int out_W, const PixelTiling& til,
                      int n_padded, int fH, int fW, int sgn, int off_h, int off_w, const float* bias, float* stats,
-                     cudaStream_t st) {
+                     cudaStream_t st, const ActEpilogue* act = nullptr, bool* act_done = nullptr) {
     {   // wide images with a filter that fits in shared memory: halo-reuse kernel
         bool used = false;
         const int padT = sgn > 0 ? -off_h : fH - 1 - off_h;
@@ -1307,6 +1329,10 @@ static int run_igemm(bool tf32, const void* in, int in_C, int in_H, int in_W, in
     p.out = out;
     p.bias = bias;
     p.stats = stats;
+    if (act != nullptr && !tf32 && !pair && stats == nullptr) {
+        p.act = *act;
+        *act_done = true;
+    }
     p.status = device_status_word();
     p.n_out = out_C;
     p.out_W = out_W; p.out_H = out_H; p.out_N = S;
@@ -1339,6 +1365,10 @@ static int launch_cast(const float* src, __nv_bfloat16* dst, long long rows, int
     return check_launch("cast_bf16_kernel");
 }
 
+int tc_cast_operand(const float* src, void* dst, long long rows, int C, int ld, cudaStream_t st) {
+    return launch_cast(src, static_cast<__nv_bfloat16*>(dst), rows, C, ld, nullptr, 0, st);
+}
+
 long long tc_conv_stats_blocks(const AetherConvDesc& d) {
     if (!tc_conv_eligible(d)) return 0;
     const TcPlan& pl = make_plan(d);
@@ -1359,7 +1389,7 @@ long long tc_conv_stats_blocks(const AetherConvDesc& d) {
 }
 
 int tc_conv_fwd(const AetherConvDesc& d, const float* x, const float* w, const float* b, float* y, float* stats, void* ws,
-                size_t ws_bytes, int flags, cudaStream_t st) {
+                size_t ws_bytes, int flags, cudaStream_t st, const ActEpilogue* act, bool* act_done) {
     const TcPlan& pl = make_plan(d);
     if (ws_bytes < pl.total || !ws) return set_error(AE_BAD_ARG, "conv workspace too small: %zu < %zu", ws_bytes, pl.total);
     uint8_t* wsb = static_cast<uint8_t*>(ws);
@@ -1385,7 +1415,7 @@ int tc_conv_fwd(const AetherConvDesc& d, const float* x, const float* w, const f
         (rc = launch_filter_shadows<__nv_bfloat16>(w, wf, wd, pl.taps, d.Cin, d.Cout, pl.Cin_p, pl.Cout_p, st)))
         return rc;
     return run_igemm(false, xsh, pl.Cin_p, d.H, d.W, d.S, wf, pl.Cin_p, pl.Cout_p, pl.taps, y, d.Cout, pl.Ho, pl.Wo,
-                     pl.til_out, pl.Cout_p, d.fH, d.fW, +1, -d.padH, -d.padW, b, stats, st);
+                     pl.til_out, pl.Cout_p, d.fH, d.fW, +1, -d.padH, -d.padW, b, stats, st, act, act_done);
 }
 
 template <bool TF32, int NB, bool PAIR>

@@ -3,6 +3,7 @@
 // Leaky_ReLU :417-428, Layer_Dropout_Spatial :384-404, Layer_Dropout :364-382, Optimizer_Adam
 // :685-736, SoftMax + categorical cross-entropy :541-680.  All arrays are fp32 with the channel
 // (last) axis contiguous; kernels use 128-bit accesses along it whenever the channel count allows.
+#include <cuda_bf16.h>
 #include <math.h>
 #include <string.h>
 
@@ -1135,6 +1136,41 @@ __global__ void __launch_bounds__(256) lrelu_bwd_kernel(const float* __restrict_
         dx[i] = x[i] < 0.f ? alpha * dy[i] : dy[i];
 }
 
+// The activation's backward pass in front of a Dense layer's: dx as above, its bf16 operand copy (rows of ld, zero in the
+// padded columns) and its column sums, the layer's dB -- one launch instead of three for the few hundred rows of a small
+// network.  A CTA owns 32 columns and walks all rows, 32 at a time, so the sums need no second pass.
+__global__ void __launch_bounds__(256) act_bwd_copy_kernel(const float* __restrict__ x, const float* __restrict__ dy, float* __restrict__ dx,
+                                                           int rows, int C, float alpha, __nv_bfloat16* __restrict__ copy, int ld,
+                                                           float* __restrict__ db) {
+    pdl_wait();
+    __shared__ float4 red[256];
+    const int cg = threadIdx.x & 7, rl = threadIdx.x >> 3, c = blockIdx.x * 32 + cg * 4;
+    float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (c < C) {
+#pragma unroll 4
+        for (int r = rl; r < rows; r += 32) {
+            const size_t at = (size_t)r * C + c;
+            const float4 v = *reinterpret_cast<const float4*>(x + at);
+            float4 g = *reinterpret_cast<const float4*>(dy + at);
+            g.x = v.x < 0.f ? alpha * g.x : g.x; g.y = v.y < 0.f ? alpha * g.y : g.y;
+            g.z = v.z < 0.f ? alpha * g.z : g.z; g.w = v.w < 0.f ? alpha * g.w : g.w;
+            *reinterpret_cast<float4*>(dx + at) = g;
+            const __nv_bfloat162 o[2] = {__floats2bfloat162_rn(g.x, g.y), __floats2bfloat162_rn(g.z, g.w)};
+            *reinterpret_cast<uint2*>(copy + (size_t)r * ld + c) = *reinterpret_cast<const uint2*>(o);
+            sum.x += g.x; sum.y += g.y; sum.z += g.z; sum.w += g.w;
+        }
+    } else if (c < ld) {
+        for (int r = rl; r < rows; r += 32) *reinterpret_cast<uint2*>(copy + (size_t)r * ld + c) = make_uint2(0u, 0u);
+    }
+    red[threadIdx.x] = sum;
+    __syncthreads();
+    if (threadIdx.x < 8 && c < C) {
+#pragma unroll
+        for (int l = 1; l < 32; ++l) { const float4 v = red[l * 8 + cg]; sum.x += v.x; sum.y += v.y; sum.z += v.z; sum.w += v.w; }
+        *reinterpret_cast<float4*>(db + c) = sum;
+    }
+}
+
 // ====================================================================================== dropout
 // Counter-based generator (Philox-4x32-10, Salmon et al. 2011): 4 uniforms per (seed, index).
 __device__ __forceinline__ uint4 philox4x32_10(uint2 key, uint4 ctr) {
@@ -1490,6 +1526,18 @@ extern "C" int aether_leaky_relu_bwd(const float* x, const float* dy, float* dx,
     launch(lrelu_bwd_kernel, blocks_for(n / 4 + 1, 256), 256, 0, static_cast<cudaStream_t>(stream), x, dy, dx, n, alpha);
     count_launch();
     return check_launch("aether_leaky_relu_bwd");
+}
+
+extern "C" int aether_act_bwd_copy(const float* x, const float* dy, float* dx, int rows, int C, float alpha, void* operand_copy, int copy_ld,
+                                   float* db, void* stream) {
+    if (!x || !dy || !dx || !operand_copy || !db || rows <= 0 || C <= 0) return set_error(AE_BAD_ARG, "aether_act_bwd_copy: bad argument");
+    if (C % 4 || copy_ld < C || copy_ld % 4 || (reinterpret_cast<uintptr_t>(operand_copy) & 7) || !aligned16(x) || !aligned16(dy) ||
+        !aligned16(dx) || !aligned16(db))
+        return set_error(AE_BAD_ARG, "aether_act_bwd_copy: needs C %% 4 == 0, 16-byte aligned arrays and a copy of ld >= C, ld %% 4 == 0");
+    launch(act_bwd_copy_kernel, ceil_div(copy_ld, 32), 256, 0, static_cast<cudaStream_t>(stream), x, dy, dx, rows, C, alpha,
+           static_cast<__nv_bfloat16*>(operand_copy), copy_ld, db);
+    count_launch();
+    return check_launch("aether_act_bwd_copy");
 }
 
 extern "C" int aether_channel_scale(const float* x, const float* scale, float* y, int64_t n, int C, void* stream) {

@@ -938,47 +938,85 @@ class Layer_Dense(_Saved):
             p = self._plans[key] = _ConvPlan(AetherConvDesc(S, 1, 1, n_in, n_out, 1, 1, 1, 1, 0, 0, _lib.MATH_MODES[self.math_mode]), 1, 1)
         return p
 
-    def forward(self, inputs, training):
-        x = to_device(inputs)
-        w = self.weights
-        if x.ndim != 2 or x.shape[1] != w.shape[0]:
-            raise ValueError(f"Layer_Dense expects (samples, {w.shape[0]}), got {tuple(x.shape)}")
-        S = x.shape[0]
-        p = self._plan(S)
-        H = host()
+    def _operands(self, x):
+        """(plan, workspace, which operand copies in it are valid) for a forward pass over `x`."""
+        p = self._plan(x.shape[0])
         ws = self._ws.get(p.ws_bytes)
-        y = H.empty((S, w.shape[1]))
         flags = 0
         if self._handed.x is not None:
             flags = _lib.CONV_X_COPY_READY if self._handed.x_ready(ws, x) else 0
             self._handed.x = None
         if not flags:
             _require_written(x, "Layer_Dense.forward")
-        if self._weights_fixed and p.layout is not None and self._copies.weights_valid(ws, w):
+        if self._weights_fixed and p.layout is not None and self._copies.weights_valid(ws, self.weights):
             flags |= _lib.CONV_W_COPY_READY
+        return p, ws, flags
+
+    def forward(self, inputs, training):
+        x = to_device(inputs)
+        w = self.weights
+        if x.ndim != 2 or x.shape[1] != w.shape[0]:
+            raise ValueError(f"Layer_Dense expects (samples, {w.shape[0]}), got {tuple(x.shape)}")
+        p, ws, flags = self._operands(x)
+        H = host()
+        y = H.empty((x.shape[0], w.shape[1]))
         H.aether_conv2d_fwd_ex(p.raw, x, w, self.biases, y, None, 0, ws, self._ws.size, flags)
         self.inputs = x
         self.output = y
         self._copies.record(ws, x, w)
         return y
 
+    def forward_act(self, x, alpha, target):
+        """`forward` and the (leaky) ReLU behind it in one call (Model): (output, activation's output)."""
+        w = self.weights
+        p, ws, flags = self._operands(x)
+        H = host()
+        shape = (x.shape[0], w.shape[1])
+        y, z = H.empty(shape), H.empty(shape)
+        H.aether_conv2d_act_fwd(p.raw, x, w, self.biases, y, z, alpha, target[0] if target else None, target[1] if target else 0, ws,
+                                self._ws.size, flags)
+        self.inputs = x
+        self.output = y
+        self._copies.record(ws, x, w)
+        return y, z
+
+    def _gradients(self):
+        if getattr(self, "_grad_views", None) is not None:
+            self.dweights, self.dbiases = self._grad_views
+        else:
+            self.dweights = host().empty_like(self.weights)
+            self.dbiases = host().empty_like(self.biases)
+
     def backward(self, dvalues):
-        dy = to_device(dvalues)
+        self._gradients()
+        return self._backward(to_device(dvalues), False)
+
+    def backward_act(self, act_inputs, dvalues, alpha):
+        """`backward` of the (leaky) ReLU behind this layer and of the layer itself: (the activation's dinputs, dinputs)."""
+        self._gradients()
+        H = host()
+        p = self._plan(act_inputs.shape[0])
+        lay = p.layout
+        dy = H.empty_like(act_inputs)
+        H.aether_act_bwd_copy(act_inputs, dvalues, dy, dy.shape[0], dy.shape[1], alpha, self._ws.get(p.ws_bytes).data_ptr() + lay.dy_copy_offset,
+                              lay.dy_copy_ld, self.dbiases)
+        return dy, self._backward(dy, True)
+
+    def _backward(self, dy, dy_ready):
+        """``dy_ready``: the operand copy of dy and dbiases are there already."""
         x = self.inputs
         w = self.weights
         p = self._plan(x.shape[0])
         H = host()
         ws = self._ws.get(p.ws_bytes)
-        if getattr(self, "_grad_views", None) is not None:
-            self.dweights, self.dbiases = self._grad_views
-        else:
-            self.dweights = H.empty_like(w)
-            self.dbiases = H.empty_like(self.biases)
         dx = H.empty_like(x)
-        copy_flags = self._copies.flags(ws, x, w)
-        if not (copy_flags & _lib.CONV_X_COPY_READY):
+        flags = self._copies.flags(ws, x, w)
+        if not (flags & _lib.CONV_X_COPY_READY):
             _require_written(x, "Layer_Dense.backward")
-        H.aether_conv2d_bwd_ex(p.raw, x, dy, w, dx, self.dweights, self.dbiases, ws, self._ws.size, copy_flags, 0)
+        if dy_ready:
+            H.aether_conv2d_bwd_ex(p.raw, x, dy, w, dx, self.dweights, None, ws, self._ws.size, flags | _lib.CONV_DY_COPY_READY, 1)
+        else:
+            H.aether_conv2d_bwd_ex(p.raw, x, dy, w, dx, self.dweights, self.dbiases, ws, self._ws.size, flags, 0)
         if self.weight_regularizer_l1 > 0 or self.weight_regularizer_l2 > 0:
             H.aether_regularizer_grad(w, self.dweights, w.numel(), self.weight_regularizer_l1, self.weight_regularizer_l2)
         if self.bias_regularizer_l1 > 0 or self.bias_regularizer_l2 > 0:

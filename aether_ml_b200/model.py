@@ -241,6 +241,58 @@ class _Chain:
         return True
 
 
+class _DenseAct:
+    """A Layer_Dense and the (Leaky_)ReLU behind it, run in one call each way; every attribute of both layers is as the layers
+    leave it.  Same conditions as _Chain, and only where the library has one launch for it."""
+    length = 2
+    MOST_ROWS = 1024            # aether_act_bwd_copy: a CTA walks all rows
+
+    def __init__(self, dense, act, behind):
+        self.parts = [dense, act]
+        self.dense, self.act = dense, act
+        self.consumer = behind if type(behind) is Layer_Dense else None
+
+    @staticmethod
+    def find(layers, i):
+        if i + 1 < len(layers) and type(layers[i]) is Layer_Dense and type(layers[i + 1]) in (ReLU, Leaky_ReLU):
+            return _DenseAct(layers[i], layers[i + 1], layers[i + 2] if i + 2 < len(layers) else None)
+        return None
+
+    def _intact(self, layers, i):
+        if layers[i:i + 2] != self.parts or self.act.fused_into_prev:
+            return False
+        for part in self.parts:
+            d = part.__dict__
+            if "forward" in d or "backward" in d:
+                return False
+        return True
+
+    def forward(self, layers, i, inputs, training, keep_all=True):
+        if not self._intact(layers, i):
+            return False
+        x = to_device(inputs)
+        dense, act = self.dense, self.act
+        if x.ndim != 2 or x.shape[1] != dense.weights.shape[0] or dense._plan(x.shape[0]).layout is None:
+            return False
+        target = self.consumer.x_copy_target((x.shape[0], dense.weights.shape[1])) if self.consumer is not None else None
+        act.inputs, act.output = dense.forward_act(x, act._alpha, target)
+        if target:
+            self.consumer.x_copy_written(act.output)
+        return True
+
+    def backward(self, layers, i, dvalues):
+        dense, act = self.dense, self.act
+        y = act.__dict__.get("inputs")
+        if y is None or not self._intact(layers, i) or dense.__dict__.get("output") is not y or not 0 < y.shape[0] <= self.MOST_ROWS:
+            return False
+        dy = to_device(dvalues)
+        lay = dense._plan(y.shape[0]).layout
+        if lay is None or dy.shape != y.shape or y.shape[0] != dense.inputs.shape[0]:
+            return False
+        act.dinputs, _ = dense.backward_act(y, dy, act._alpha)
+        return True
+
+
 class Model:
     def __init__(self):
         self.layers = []
@@ -257,7 +309,7 @@ class Model:
         self._bucket_of_layer = {}
         self._update_stream = None # side stream on which finished buckets are updated while backward goes on
         self._updated_early = set()
-        self._chains = {}          # position of a Batch_Norm -> the _Chain that starts there
+        self._chains = {}          # position of a Batch_Norm or Layer_Dense -> the _Chain or _DenseAct that starts there
         self._chain_ends = {}      # position of a chain's last layer -> where it starts
 
     def add(self, layer):
@@ -369,9 +421,8 @@ class Model:
                     a.lean = bool(lean)
                     if isinstance(getattr(a, "prev", None), Conv_Layer):
                         a.copy_dy_consumer = a.prev
-        self._chains = {}
-        if not fuse:
-            self._chains = {i: c for i in range(len(self.layers)) if (c := _Chain.find(self.layers, i)) is not None}
+        self._chains = {i: c for i in range(len(self.layers))
+                        if (c := (None if fuse else _Chain.find(self.layers, i)) or _DenseAct.find(self.layers, i)) is not None}
         self._chain_ends = {i + c.length - 1: i for i, c in self._chains.items()}
         self.trainable_layers = [l for l in self.layers if hasattr(l, "weights")]
         if self.loss is not None:
@@ -461,7 +512,7 @@ class Model:
             layer = upstream[i]
             start = self._chain_ends.get(i)
             if start is not None and self._chains[start].backward(self.layers, start, layer.next.dinputs):
-                layer = upstream[start]         # the chain's only trainable layer is its Batch_Norm
+                layer = upstream[start]         # the chain's only trainable layer is its first
                 i = start
             elif layer is first and hasattr(layer, "_desc"):
                 layer.backward(layer.next.dinputs, need_dinputs=False)   # nobody consumes d(loss)/d(images)

@@ -139,6 +139,17 @@ enum { AETHER_CONV_X_COPY_READY = 1, AETHER_CONV_W_COPY_READY = 2, AETHER_CONV_D
 int aether_conv2d_operand_layout(const AetherConvDesc* desc, AetherOperandLayout* out);
 int aether_conv2d_fwd_ex(const AetherConvDesc* desc, const float* x, const float* w, const float* b, float* y, float* stats,
                          size_t stats_bytes, void* ws, size_t ws_bytes, int flags, void* stream);
+
+/* The forward pass and the (leaky) ReLU behind it (a Dense layer of a small network is a launch of its own for each): y as
+ * aether_conv2d_fwd_ex writes it, act_out = y > 0 ? y : alpha * y and, when given, the bf16 operand copy of act_out for the
+ * layer behind, in rows of copy_ld (Cout <= copy_ld <= Cout rounded up to 64; padded columns are zeroed).  Shapes of the
+ * tensor-core path only.  aether_act_bwd_copy is the way back: dx = x < 0 ? alpha * dy : dy, its operand copy (dy_copy of
+ * aether_conv2d_operand_layout) and its column sums db, which the layer's backward call then need not write.  One CTA walks
+ * all rows of 32 columns: meant for up to a thousand rows. */
+int aether_conv2d_act_fwd(const AetherConvDesc* desc, const float* x, const float* w, const float* b, float* y, float* act_out,
+                          float alpha, void* act_copy, int copy_ld, void* ws, size_t ws_bytes, int flags, void* stream);
+int aether_act_bwd_copy(const float* x, const float* dy, float* dx, int rows, int C, float alpha, void* operand_copy, int copy_ld,
+                        float* db, void* stream);
 int aether_conv2d_bwd_ex(const AetherConvDesc* desc, const float* x, const float* dy, const float* w, float* dx, float* dw,
                          float* db, void* ws, size_t ws_bytes, int x_shadow_valid, int dy_colsum_rows, void* stream);
 
