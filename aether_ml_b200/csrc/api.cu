@@ -246,6 +246,35 @@ extern "C" int aether_conv2d_act_fwd(const AetherConvDesc* d, const float* x, co
     return tc_cast_operand(act_out, act_copy, rows, d->Cout, copy_ld, st);
 }
 
+extern "C" int aether_head_supported(const AetherConvDesc* d) {
+    return !validate_desc(d, "aether_head_supported") && !tc_conv_eligible(*d) && !first_tc_eligible(*d) && !smallc_conv_eligible(*d) &&
+           generic_head_shape(*d);
+}
+
+static int head_check(const AetherConvDesc* d, const char* who) {
+    if (int rc = validate_desc(d, who)) return rc;
+    if (!aether_head_supported(d)) return set_error(AE_UNSUPPORTED, "%s: not a classifier head (aether_head_supported returned 0)", who);
+    return pending_timeout(who);
+}
+
+extern "C" int aether_head_softmax_fwd(const AetherConvDesc* d, const float* x, const float* w, const float* b, float* y, float* prob,
+                                       void* stream) {
+    if (int rc = head_check(d, "aether_head_softmax_fwd")) return rc;
+    if (!x || !w || !y || !prob) return set_error(AE_BAD_ARG, "aether_head_softmax_fwd: null pointer");
+    if (!aligned16(x) || !aligned16(w) || !aligned16(y)) return set_error(AE_BAD_ARG, "aether_head_softmax_fwd: arrays must be 16-byte aligned");
+    return generic_head_softmax_fwd(*d, x, w, b, y, prob, static_cast<cudaStream_t>(stream));
+}
+
+extern "C" int aether_head_cce_bwd(const AetherConvDesc* d, const float* prob, const int32_t* labels, const int64_t* labels64,
+                                   const float* targets, float smooth, const float* w, float* dz, float* dx, void* stream) {
+    if (int rc = head_check(d, "aether_head_cce_bwd")) return rc;
+    if (!prob || !w || !dz || !dx || (labels != nullptr) + (labels64 != nullptr) + (targets != nullptr) != 1)
+        return set_error(AE_BAD_ARG, "aether_head_cce_bwd: null pointer, or not one kind of labels");
+    if (!aligned16(w) || !aligned16(dx)) return set_error(AE_BAD_ARG, "aether_head_cce_bwd: arrays must be 16-byte aligned");
+    return generic_head_cce_bwd(*d, prob, labels, reinterpret_cast<const long long*>(labels64), targets, smooth, w, dz, dx,
+                                static_cast<cudaStream_t>(stream));
+}
+
 extern "C" int aether_conv2d_fwd(const AetherConvDesc* d, const float* x, const float* w, const float* b, float* y,
                                  void* ws, size_t ws_bytes, void* stream) {
     int rc = validate_desc(d, "aether_conv2d_fwd");

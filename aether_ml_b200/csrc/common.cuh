@@ -71,6 +71,11 @@ int simt_conv_bwd_filter(const AetherConvDesc& d, const float* x, const float* d
 size_t simt_conv_workspace_bytes(const AetherConvDesc& d);
 
 // ---- conv_generic.cu : classifier heads and dX of first layers on the CUDA cores; everything else goes to conv_simt.cu
+// classifier heads (pointwise, few outputs) with the softmax / the combined softmax and cross-entropy gradient in the kernel
+bool generic_head_shape(const AetherConvDesc& d);
+int generic_head_softmax_fwd(const AetherConvDesc& d, const float* x, const float* w, const float* b, float* y, float* prob, cudaStream_t st);
+int generic_head_cce_bwd(const AetherConvDesc& d, const float* prob, const int* labels, const long long* labels64, const float* targets,
+                         float smooth, const float* w, float* dz, float* dx, cudaStream_t st);
 int generic_conv_fwd(const AetherConvDesc& d, const float* x, const float* w, const float* b, float* y, cudaStream_t st);
 int generic_conv_bwd_data(const AetherConvDesc& d, const float* dy, const float* w, float* dx, cudaStream_t st);
 int generic_conv_bwd_filter(const AetherConvDesc& d, const float* x, const float* dy, float* dw, float* db, void* ws,

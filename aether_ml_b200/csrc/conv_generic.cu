@@ -24,7 +24,7 @@ __device__ __forceinline__ void head_load_filter_T(const float* __restrict__ w, 
 template <int MAXD>
 __global__ void __launch_bounds__(256) gen_fwd_pointwise_few_kernel(const float* __restrict__ x, const float* __restrict__ w,
                                                                     const float* __restrict__ b, float* __restrict__ y,
-                                                                    long long rows, int Cin, int Cout) {
+                                                                    long long rows, int Cin, int Cout, float* __restrict__ prob) {
     pdl_wait();
     extern __shared__ __align__(16) float head_wT[];
     head_load_filter_T(w, head_wT, Cin, Cout);
@@ -52,11 +52,23 @@ __global__ void __launch_bounds__(256) gen_fwd_pointwise_few_kernel(const float*
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) acc[d] += __shfl_xor_sync(0xffffffffu, acc[d], o);
         }
+        float z = -INFINITY;
         if (lane < Cout) {
             float r = 0.f;
 #pragma unroll
             for (int d = 0; d < MAXD; ++d) r = (d == lane) ? acc[d] : r;
-            y[(size_t)row * Cout + lane] = r + (b ? b[lane] : 0.f);
+            z = r + (b ? b[lane] : 0.f);
+            y[(size_t)row * Cout + lane] = z;
+        }
+        if (prob != nullptr) {                               // the softmax behind the head, as softmax_cce_kernel computes it
+            float mx = z;
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+            const float e = lane < Cout ? expf(z - mx) : 0.f;
+            float sum = e;
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+            if (lane < Cout) prob[(size_t)row * Cout + lane] = e / sum;
         }
     }
 }
@@ -192,23 +204,46 @@ __global__ void __launch_bounds__(256, 2) dx_fewc_kernel(const float* __restrict
 // ---------------------------------------------------------------------------------- classifier heads, backward
 // dx[p][c] = sum_d dy[p][d] * w[c][d] for a pointwise layer with few outputs: a block takes a row at a time, a thread
 // four channels; the filter is read transposed from shared memory, the row of dy is the same address for every thread.
-template <int MAXD>
+// CCE: dy is not there yet -- it is the combined softmax / cross-entropy gradient (prob - y_smooth) / rows, which is computed
+// from the probabilities and the labels of the row (as softmax_cce_kernel does) and written to dz on the way.
+struct HeadCce {
+    const float* prob;
+    const int* labels;             // one of the three
+    const long long* labels64;
+    const float* targets;
+    float* dz;
+    float smooth, inv_rows;
+};
+template <int MAXD, bool CCE>
 __global__ void __launch_bounds__(256) head_dx_kernel(const float* __restrict__ dy, const float* __restrict__ w,
-                                                      float* __restrict__ dx, long long rows, int Cin, int Cout) {
+                                                      float* __restrict__ dx, long long rows, int Cin, int Cout, const HeadCce cce) {
     pdl_wait();
     extern __shared__ __align__(16) float head_wT[];
     head_load_filter_T(w, head_wT, Cin, Cout);
     const int C4 = Cin >> 2;
+    const float* src = CCE ? cce.prob : dy;
     float gn[MAXD];                                     // the next row's dy values, requested one row ahead
 #pragma unroll
-    for (int d = 0; d < MAXD; ++d) gn[d] = (d < Cout && blockIdx.x < rows) ? __ldg(dy + (size_t)blockIdx.x * Cout + d) : 0.f;
+    for (int d = 0; d < MAXD; ++d) gn[d] = (d < Cout && blockIdx.x < rows) ? __ldg(src + (size_t)blockIdx.x * Cout + d) : 0.f;
     for (long long row = blockIdx.x; row < rows; row += gridDim.x) {
         float g[MAXD];
         const long long nrow = row + gridDim.x;
 #pragma unroll
         for (int d = 0; d < MAXD; ++d) {
             g[d] = gn[d];
-            gn[d] = (d < Cout && nrow < rows) ? __ldg(dy + (size_t)nrow * Cout + d) : 0.f;
+            gn[d] = (d < Cout && nrow < rows) ? __ldg(src + (size_t)nrow * Cout + d) : 0.f;
+        }
+        if (CCE) {
+            const int label = cce.labels ? cce.labels[row] : cce.labels64 ? (int)cce.labels64[row] : -1;
+#pragma unroll
+            for (int d = 0; d < MAXD; ++d) {
+                if (d < Cout) {
+                    const float onehot = cce.targets ? cce.targets[(size_t)row * Cout + d] : (d == label ? 1.f : 0.f);
+                    const float tb = onehot * (1.f - cce.smooth) + cce.smooth / Cout;
+                    g[d] = (g[d] - tb) * cce.inv_rows;
+                    if ((int)threadIdx.x == d) cce.dz[(size_t)row * Cout + d] = g[d];
+                }
+            }
         }
         float4* out = reinterpret_cast<float4*>(dx + (size_t)row * Cin);
         for (int c4 = threadIdx.x; c4 < C4; c4 += blockDim.x) {
@@ -305,19 +340,43 @@ static bool head_shape(const AetherConvDesc& d) {
 }
 
 // ---------------------------------------------------------------------------------- host
+static int head_fwd(const AetherConvDesc& d, const float* x, const float* w, const float* b, float* y, float* prob, cudaStream_t st) {
+    const long long rows = 1LL * d.S * d.H * d.W;
+    const int smem = (d.Cin + 4) * d.Cout * (int)sizeof(float);
+    static PerDeviceSmem configured;
+    if (int rc = ensure_dynamic_smem(gen_fwd_pointwise_few_kernel<16>, 96 * 1024, configured, "head forward")) return rc;
+    long long nb = (rows + 7) / 8;                        // a warp per row, 8 rows per block and pass
+    if (nb > 2LL * num_sms()) nb = 2LL * num_sms();       // every block loads the filter once
+    launch(gen_fwd_pointwise_few_kernel<16>, (int)nb, 256, smem, st, x, w, b, y, rows, d.Cin, d.Cout, prob);
+    count_launch();
+    return check_launch("gen_fwd_pointwise_few_kernel");
+}
+
 int generic_conv_fwd(const AetherConvDesc& d, const float* x, const float* w, const float* b, float* y, cudaStream_t st) {
-    if (head_shape(d) && (reinterpret_cast<uintptr_t>(x) & 15u) == 0) {
-        const long long rows = 1LL * d.S * d.H * d.W;
-        const int smem = (d.Cin + 4) * d.Cout * (int)sizeof(float);
-        static PerDeviceSmem configured;
-        if (int rc = ensure_dynamic_smem(gen_fwd_pointwise_few_kernel<16>, 96 * 1024, configured, "head forward")) return rc;
-        long long nb = (rows + 7) / 8;                        // a warp per row, 8 rows per block and pass
-        if (nb > 2LL * num_sms()) nb = 2LL * num_sms();       // every block loads the filter once
-        launch(gen_fwd_pointwise_few_kernel<16>, (int)nb, 256, smem, st, x, w, b, y, rows, d.Cin, d.Cout);
-        count_launch();
-        return check_launch("gen_fwd_pointwise_few_kernel");
-    }
+    if (head_shape(d) && (reinterpret_cast<uintptr_t>(x) & 15u) == 0) return head_fwd(d, x, w, b, y, nullptr, st);
     return simt_conv_fwd(d, x, w, b, y, st);
+}
+
+bool generic_head_shape(const AetherConvDesc& d) { return head_shape(d); }
+int generic_head_softmax_fwd(const AetherConvDesc& d, const float* x, const float* w, const float* b, float* y, float* prob, cudaStream_t st) {
+    return head_fwd(d, x, w, b, y, prob, st);
+}
+
+static int head_dx(const AetherConvDesc& d, const float* dy, const float* w, float* dx, const HeadCce* cce, cudaStream_t st) {
+    const long long rows = 1LL * d.S * d.H * d.W;
+    const int smem = (d.Cin + 4) * d.Cout * (int)sizeof(float);
+    static PerDeviceSmem configured[2];
+    const auto kernel = cce ? head_dx_kernel<16, true> : head_dx_kernel<16, false>;
+    if (int rc = ensure_dynamic_smem(kernel, 96 * 1024, configured[cce ? 1 : 0], "head dX")) return rc;
+    const long long nb = rows < 2LL * num_sms() ? rows : 2LL * num_sms();
+    launch(kernel, (int)nb, 256, smem, st, dy, w, dx, rows, d.Cin, d.Cout, cce ? *cce : HeadCce{});
+    count_launch();
+    return check_launch("head_dx_kernel");
+}
+int generic_head_cce_bwd(const AetherConvDesc& d, const float* prob, const int* labels, const long long* labels64, const float* targets,
+                         float smooth, const float* w, float* dz, float* dx, cudaStream_t st) {
+    const HeadCce cce = {prob, labels, labels64, targets, dz, smooth, 1.f / (float)(1LL * d.S * d.H * d.W)};
+    return head_dx(d, nullptr, w, dx, &cce, st);
 }
 
 template <int CIN, int FB>
@@ -352,16 +411,7 @@ int generic_conv_bwd_data(const AetherConvDesc& d, const float* dy, const float*
             default: return dx_fewc<4>(d, dy, w, dx, Ho, Wo, st);
         }
     }
-    if (head_shape(d) && (reinterpret_cast<uintptr_t>(dx) & 15u) == 0) {
-        const long long rows = 1LL * d.S * d.H * d.W;
-        const int smem = (d.Cin + 4) * d.Cout * (int)sizeof(float);
-        static PerDeviceSmem configured;
-        if (int rc = ensure_dynamic_smem(head_dx_kernel<16>, 96 * 1024, configured, "head dX")) return rc;
-        long long nb = rows < 2LL * num_sms() ? rows : 2LL * num_sms();
-        launch(head_dx_kernel<16>, (int)nb, 256, smem, st, dy, w, dx, rows, d.Cin, d.Cout);
-        count_launch();
-        return check_launch("head_dx_kernel");
-    }
+    if (head_shape(d) && (reinterpret_cast<uintptr_t>(dx) & 15u) == 0) return head_dx(d, dy, w, dx, nullptr, st);
     return simt_conv_bwd_data(d, dy, w, dx, st);
 }
 

@@ -213,11 +213,12 @@ class _ConvPlan:
         self.x_shape = (desc.S, desc.H, desc.W, desc.Cin)
         self.y_shape = (desc.S, Ho, Wo, desc.Cout) if Ho >= 1 and Wo >= 1 else None
         self.b_shape = (desc.Cout,)
-        self.layout, self.ws_bytes, self.stats_blocks = None, 0, 0
+        self.layout, self.ws_bytes, self.stats_blocks, self.head = None, 0, 0, False
         if self.y_shape is not None:
             self.ws_bytes = int(lib().aether_conv2d_workspace_bytes(d))
             self.stats_blocks = int(lib().aether_conv2d_bnstats_blocks(d))
             self.layout = _operand_layout(desc)
+            self.head = bool(lib().aether_head_supported(d))
 
 
 # ------------------------------------------------------------------------------------- Conv_Layer
@@ -980,6 +981,31 @@ class Layer_Dense(_Saved):
         self._copies.record(ws, x, w)
         return y, z
 
+    def forward_softmax(self, x):
+        """`forward` of a classifier head and the SoftMax behind it in one launch (Model): (output, probabilities)."""
+        w = self.weights
+        p, ws, _ = self._operands(x)
+        H = host()
+        shape = (x.shape[0], w.shape[1])
+        y, prob = H.empty(shape), H.empty(shape)
+        H.aether_head_softmax_fwd(p.raw, x, w, self.biases, y, prob)
+        self.inputs = x
+        self.output = y
+        self._copies.record(ws, x, w)
+        return y, prob
+
+    def backward_softmax(self, prob, labels, smooth):
+        """The combined softmax / cross-entropy gradient and this head's `backward`: the gradient with respect to the logits."""
+        self._gradients()
+        H = host()
+        p = self._plan(prob.shape[0])
+        dz, dx = H.empty_like(prob), H.empty_like(self.inputs)
+        kinds = [None, None, None]
+        kinds[2 if labels.ndim == 2 else 1 if labels.dtype is torch.int64 else 0] = labels
+        H.aether_head_cce_bwd(p.raw, prob, *kinds, smooth, self.weights, dz, dx)
+        self._backward(dz, False, dx)
+        return dz
+
     def _gradients(self):
         if getattr(self, "_grad_views", None) is not None:
             self.dweights, self.dbiases = self._grad_views
@@ -1002,21 +1028,23 @@ class Layer_Dense(_Saved):
                               lay.dy_copy_ld, self.dbiases)
         return dy, self._backward(dy, True)
 
-    def _backward(self, dy, dy_ready):
-        """``dy_ready``: the operand copy of dy and dbiases are there already."""
+    def _backward(self, dy, dy_ready, dx=None):
+        """``dy_ready``: the operand copy of dy and dbiases are there already; ``dx``: dinputs, when they are."""
         x = self.inputs
         w = self.weights
         p = self._plan(x.shape[0])
         H = host()
         ws = self._ws.get(p.ws_bytes)
-        dx = H.empty_like(x)
+        want = None
+        if dx is None:
+            dx = want = H.empty_like(x)
         flags = self._copies.flags(ws, x, w)
         if not (flags & _lib.CONV_X_COPY_READY):
             _require_written(x, "Layer_Dense.backward")
         if dy_ready:
-            H.aether_conv2d_bwd_ex(p.raw, x, dy, w, dx, self.dweights, None, ws, self._ws.size, flags | _lib.CONV_DY_COPY_READY, 1)
+            H.aether_conv2d_bwd_ex(p.raw, x, dy, w, want, self.dweights, None, ws, self._ws.size, flags | _lib.CONV_DY_COPY_READY, 1)
         else:
-            H.aether_conv2d_bwd_ex(p.raw, x, dy, w, dx, self.dweights, self.dbiases, ws, self._ws.size, flags, 0)
+            H.aether_conv2d_bwd_ex(p.raw, x, dy, w, want, self.dweights, self.dbiases, ws, self._ws.size, flags, 0)
         if self.weight_regularizer_l1 > 0 or self.weight_regularizer_l2 > 0:
             H.aether_regularizer_grad(w, self.dweights, w.numel(), self.weight_regularizer_l1, self.weight_regularizer_l2)
         if self.bias_regularizer_l1 > 0 or self.bias_regularizer_l2 > 0:

@@ -293,6 +293,53 @@ class _DenseAct:
         return True
 
 
+class _Head:
+    """The Layer_Dense and the SoftMax a classifier ends in: logits and probabilities in one launch and, with the combined
+    softmax / cross-entropy loss, the gradient of the logits and of the layer's inputs in one.  Conditions as for _Chain."""
+    length = 2
+
+    def __init__(self, dense, softmax):
+        self.parts = [dense, softmax]
+        self.dense, self.softmax = dense, softmax
+
+    @staticmethod
+    def find(layers, i):
+        return _Head(layers[i], layers[i + 1]) if len(layers) == i + 2 and type(layers[i]) is Layer_Dense and type(layers[i + 1]) is SoftMax else None
+
+    def _intact(self, layers, i):
+        if layers[i:] != self.parts:
+            return False
+        for part in self.parts:
+            d = part.__dict__
+            if "forward" in d or "backward" in d:
+                return False
+        return True
+
+    def forward(self, layers, i, inputs, training, keep_all=True):
+        if not self._intact(layers, i):
+            return False
+        x = to_device(inputs)
+        dense, softmax = self.dense, self.softmax
+        if x.ndim != 2 or x.shape[1] != dense.weights.shape[0] or x.shape[0] == 0 or not dense._plan(x.shape[0]).head:
+            return False
+        softmax.inputs, softmax.output = dense.forward_softmax(x)
+        return True
+
+    def backward(self, layers, combined, output, y):
+        """Both layers' backward passes for the combined loss; False when they have to run one by one."""
+        dense, softmax = self.dense, self.softmax
+        z = softmax.__dict__.get("inputs")
+        if (z is None or type(combined) is not Activation_Softmax_Loss_CategoricalCrossEntropy or "backward" in combined.__dict__
+                or softmax.output is not output or dense.__dict__.get("output") is not z or not self._intact(layers, len(layers) - 2)
+                or not dense._plan(z.shape[0]).head or z.shape[0] != dense.inputs.shape[0]):
+            return False
+        labels = _labels(y)
+        if labels.shape[0] != z.shape[0] or (labels.ndim == 2 and labels.shape != z.shape):
+            return False
+        combined.dinputs = softmax.dinputs = dense.backward_softmax(output, labels, combined.label_smoothing)
+        return True
+
+
 class Model:
     def __init__(self):
         self.layers = []
@@ -422,8 +469,8 @@ class Model:
                     if isinstance(getattr(a, "prev", None), Conv_Layer):
                         a.copy_dy_consumer = a.prev
         self._chains = {i: c for i in range(len(self.layers))
-                        if (c := (None if fuse else _Chain.find(self.layers, i)) or _DenseAct.find(self.layers, i)) is not None}
-        self._chain_ends = {i + c.length - 1: i for i, c in self._chains.items()}
+                        if (c := (None if fuse else _Chain.find(self.layers, i)) or _DenseAct.find(self.layers, i) or _Head.find(self.layers, i)) is not None}
+        self._chain_ends = {i + c.length - 1: i for i, c in self._chains.items() if type(c) is not _Head}
         self.trainable_layers = [l for l in self.layers if hasattr(l, "weights")]
         if self.loss is not None:
             self.loss.remember_trainable_layers(self.trainable_layers)
@@ -499,30 +546,39 @@ class Model:
         return layers[-1].output
 
     def backward(self, output, y):
+        layers = self.layers
+        i = len(layers) - 1
         if self.softmax_classifier_output is not None:
-            self.softmax_classifier_output.backward(output, y, training=True)
-            self.layers[-1].dinputs = self.softmax_classifier_output.dinputs
-            upstream = self.layers[:-1]
+            head = self._chains.get(i - 1)
+            if type(head) is _Head and head.backward(layers, self.softmax_classifier_output, output, y):
+                i -= 1
+                self._gradients_written(layers[i])
+            else:
+                self.softmax_classifier_output.backward(output, y, training=True)
+                layers[-1].dinputs = self.softmax_classifier_output.dinputs
+            i -= 1
         else:
             self.loss.backward(output, y)
-            upstream = self.layers
-        first = self.layers[0]
-        i = len(upstream) - 1
+        first = layers[0]
         while i >= 0:
-            layer = upstream[i]
+            layer = layers[i]
+            dvalues = layer.next.dinputs
             start = self._chain_ends.get(i)
-            if start is not None and self._chains[start].backward(self.layers, start, layer.next.dinputs):
-                layer = upstream[start]         # the chain's only trainable layer is its first
+            if start is not None and self._chains[start].backward(layers, start, dvalues):
+                layer = layers[start]           # the chain's only trainable layer is its first
                 i = start
             elif layer is first and hasattr(layer, "_desc"):
-                layer.backward(layer.next.dinputs, need_dinputs=False)   # nobody consumes d(loss)/d(images)
+                layer.backward(dvalues, need_dinputs=False)   # nobody consumes d(loss)/d(images)
             else:
-                layer.backward(layer.next.dinputs)
+                layer.backward(dvalues)
             i -= 1
-            b = self._bucket_of_layer.get(id(layer))
-            if b is not None:                   # this layer's gradients complete a bucket: start reducing it
-                self.bucket_reducer.start(b)
-                self._update_bucket_early(b)
+            self._gradients_written(layer)
+
+    def _gradients_written(self, layer):
+        b = self._bucket_of_layer.get(id(layer)) if self._bucket_of_layer else None
+        if b is not None:                       # this layer's gradients complete a bucket: start reducing it
+            self.bucket_reducer.start(b)
+            self._update_bucket_early(b)
 
     def _update_bucket_early(self, b):
         """Every bucket but the last is updated as soon as its all-reduce is through, on a side stream, while the
