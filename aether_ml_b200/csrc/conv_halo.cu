@@ -46,6 +46,7 @@ struct HaloParams {
     int tiles_h, n_images;
     int fH, fW, padT, padL, flip;
     int kchunks, rows_per_tap;
+    int last_ksteps;     // MMAs (32 bytes of K each) that the last chunk of channels needs: the rest of it is padding
     int region_rows;     // (BH+fH-1) * Wp
     int region_stride;   // bytes between stages (multiple of 1024)
     int stages;
@@ -96,7 +97,9 @@ __device__ __forceinline__ void umma_lohi(uint32_t d_tmem, uint32_t a_lo, uint32
 // [r * NT/2, (r+1) * NT/2) of every tap resident; the even CTA issues 256-row MMAs that read both CTAs' windows and
 // filter halves and write both CTAs' accumulators.  Half a filter per SM leaves room for more window stages (and lets a
 // TF32 filter of 9 x 128 x 64 fit at all), and each MMA reads half as many filter bytes from each SM's shared memory.
-template <bool TF32, bool STATS, bool PAIR>
+// TAIL: the last chunk of channels is partly padding and takes fewer MMAs (p.last_ksteps); a variant of its own because the
+// issuing loop of the others has no cycle to spare (3 % on 56x56 128->64).
+template <bool TF32, bool STATS, bool PAIR, bool TAIL>
 __global__ void __launch_bounds__(HALO_THREADS, 1) halo_conv_kernel(const __grid_constant__ HaloParams p) {
     constexpr int KC = TF32 ? 32 : 64;
     extern __shared__ uint8_t smem_raw[];
@@ -230,6 +233,7 @@ __global__ void __launch_bounds__(HALO_THREADS, 1) halo_conv_kernel(const __grid
                 f_ok = __all_sync(0xffffffffu, f_ok);
                 if (!f_ok) { ok = false; break; }
                 tc_fence_after();
+                const int nk = kc + 1 == p.kchunks ? p.last_ksteps : 4;
                 uint32_t a_row = r_lo + (uint32_t)s * rs16;
                 // filter tap that multiplies window shift (ti,tj): the same index, or the mirrored one for dX
                 uint32_t b_cur = w_lo + (uint32_t)kc * wt16 + (p.flip ? (uint32_t)(taps - 1) * bstep : 0u);
@@ -238,9 +242,9 @@ __global__ void __launch_bounds__(HALO_THREADS, 1) halo_conv_kernel(const __grid
                     for (int tj = 0; tj < p.fW; ++tj) {
                         if (leader) {
                             umma_lohi<TF32, PAIR>(d_tmem, a_tap, b_cur, hi, idesc, acc);
-                            umma_lohi<TF32, PAIR>(d_tmem, a_tap + 2, b_cur + 2, hi, idesc, 1u);
-                            umma_lohi<TF32, PAIR>(d_tmem, a_tap + 4, b_cur + 4, hi, idesc, 1u);
-                            umma_lohi<TF32, PAIR>(d_tmem, a_tap + 6, b_cur + 6, hi, idesc, 1u);
+                            if (!TAIL || nk > 1) umma_lohi<TF32, PAIR>(d_tmem, a_tap + 2, b_cur + 2, hi, idesc, 1u);
+                            if (!TAIL || nk > 2) umma_lohi<TF32, PAIR>(d_tmem, a_tap + 4, b_cur + 4, hi, idesc, 1u);
+                            if (!TAIL || nk > 3) umma_lohi<TF32, PAIR>(d_tmem, a_tap + 6, b_cur + 6, hi, idesc, 1u);
                         }
                         acc = 1u;
                         a_tap += 8u;
@@ -500,7 +504,7 @@ long long halo_igemm_stats_blocks(bool tf32, int in_C, int S, int taps, int out_
 
 int run_halo_igemm(bool tf32, const void* in, int in_C, int in_H, int in_W, int S, const void* wmat, int w_inner,
                    int rows_per_tap, int taps, float* out, int out_C, int out_H, int out_W, int n_padded, int fH, int fW,
-                   int padT, int padL, int flip, const float* bias, float* stats, int prof_kind, cudaStream_t st,
+                   int padT, int padL, int flip, int k_real, const float* bias, float* stats, int prof_kind, cudaStream_t st,
                    bool* used) {
     *used = false;
     const int elt = tf32 ? 4 : 2;
@@ -528,17 +532,21 @@ int run_halo_igemm(bool tf32, const void* in, int in_C, int in_H, int in_W, int 
     p.tiles_h = tiles_h; p.n_images = S;
     p.fH = fH; p.fW = fW; p.padT = padT; p.padL = padL; p.flip = flip;
     p.kchunks = kchunks; p.rows_per_tap = rows_per_tap;
+    p.last_ksteps = last_ksteps(k_real, kchunks, KC);
     p.region_rows = region_rows; p.region_stride = region_stride; p.stages = stages; p.w_bytes = w_bytes;
     const int smem = fixed + stages * region_stride;
 
-    // eight instantiations: operand type x (with / without the statistics epilogue) x (single CTAs / CTA pairs)
+    // operand type x (with / without the statistics epilogue) x (single CTAs / CTA pairs) x (whole / partial last chunk)
     using KernelFn = void (*)(const HaloParams);
-    static const KernelFn kernels[8] = {halo_conv_kernel<false, false, false>, halo_conv_kernel<true, false, false>,
-                                        halo_conv_kernel<false, true, false>,  halo_conv_kernel<true, true, false>,
-                                        halo_conv_kernel<false, false, true>,  halo_conv_kernel<true, false, true>,
-                                        halo_conv_kernel<false, true, true>,   halo_conv_kernel<true, true, true>};
-    static PerDeviceSmem configured[8];
-    const int ki = (tf32 ? 1 : 0) + (stats ? 2 : 0) + (g.pair ? 4 : 0);
+    static const KernelFn kernels[16] = {
+        halo_conv_kernel<false, false, false, false>, halo_conv_kernel<true, false, false, false>, halo_conv_kernel<false, true, false, false>,
+        halo_conv_kernel<true, true, false, false>,   halo_conv_kernel<false, false, true, false>, halo_conv_kernel<true, false, true, false>,
+        halo_conv_kernel<false, true, true, false>,   halo_conv_kernel<true, true, true, false>,   halo_conv_kernel<false, false, false, true>,
+        halo_conv_kernel<true, false, false, true>,   halo_conv_kernel<false, true, false, true>,  halo_conv_kernel<true, true, false, true>,
+        halo_conv_kernel<false, false, true, true>,   halo_conv_kernel<true, false, true, true>,   halo_conv_kernel<false, true, true, true>,
+        halo_conv_kernel<true, true, true, true>};
+    static PerDeviceSmem configured[16];
+    const int ki = (tf32 ? 1 : 0) + (stats ? 2 : 0) + (g.pair ? 4 : 0) + (p.last_ksteps < 4 ? 8 : 0);
     if ((rc = ensure_dynamic_smem(kernels[ki], smem_max, configured[ki], "halo_conv"))) return rc;
     prof_begin(prof_kind, st);
     if (g.pair) {

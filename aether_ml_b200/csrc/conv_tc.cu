@@ -33,6 +33,12 @@ struct PixelTiling {
     long long total() const { return 1LL * tiles_w * tiles_h * tiles_n; }
 };
 
+// Columns of the halo kernel's accumulator: the output channels to the next 32 (the per-tap kernel's tiles are powers of two).
+static int halo_n(int out_C, int n_padded) {
+    const int n = (out_C + 31) / 32 * 32;
+    return n < n_padded ? n : n_padded;
+}
+
 static PixelTiling choose_tiling(int S, int H, int W) {
     // Exhaustive search over box shapes with <=128 pixels: minimise the number of tiles (i.e. wasted
     // MMA rows), prefer wide boxes on ties (longer contiguous runs per TMA row).
@@ -119,6 +125,7 @@ struct IgemmParams {
     int rows_per_tap;
     int fH, fW, sgn, off_h, off_w;
     int kchunks;
+    int last_ksteps;     // MMAs that the last K chunk of a tap needs
     ActEpilogue act;     // ACT only
 };
 
@@ -289,6 +296,7 @@ __global__ void __launch_bounds__(IGEMM_THREADS, 1) igemm_conv_kernel(const __gr
                 if (!mbar_wait(tempty_bar(buf), aph ^ 1u, p.status, DS_TIMEOUT_TMEM_EMPTY)) { ok = false; break; }
                 tc_fence_after();
                 const uint32_t d_tmem = tmem_base + buf * NT;
+                int kc = 0;
                 for (int k0 = 0; k0 < kiters; k0 += KS) {
                     const int nsub = kiters - k0 < KS ? kiters - k0 : KS;
                     if (!mbar_wait(full_bar(s), ph, p.status, DS_TIMEOUT_FULL)) { ok = false; break; }
@@ -298,9 +306,12 @@ __global__ void __launch_bounds__(IGEMM_THREADS, 1) igemm_conv_kernel(const __gr
                         if (c < nsub) {
                             const uint64_t da = make_smem_desc(sA + s * Cfg::STAGE_A_BYTES + c * TILE_A_BYTES, 16, 1024);
                             const uint64_t db = make_smem_desc(sB + s * Cfg::STAGE_B_BYTES + c * Cfg::TILE_B_BYTES, 16, 1024);
+                            const int nk = ++kc == p.kchunks ? p.last_ksteps : 4;
+                            if (kc == p.kchunks) kc = 0;
 #pragma unroll
                             for (int k = 0; k < 4; ++k) {                  // 32 bytes of K each: two 16-byte units further
                                 const uint32_t acc = (k0 + c > 0 || k > 0) ? 1u : 0u;
+                                if (k >= nk) break;
                                 if (PAIR) umma_pair<TF32>(d_tmem, da + 2u * k, db + 2u * k, idesc, acc);
                                 else umma<TF32>(d_tmem, da + 2u * k, db + 2u * k, idesc, acc);
                             }
@@ -1303,14 +1314,14 @@ static int dispatch_igemm(IgemmParams& p, int nt, bool pair, cudaStream_t st) {
 // Runs out[p, n] = sum_{tap,k} in[p (+/-) tap, k] * Wm[tap][n][k] (+ bias).
 static int run_igemm(bool tf32, const void* in, int in_C, int in_H, int in_W, int S, const void* wmat, int w_inner,
                      int rows_per_tap, int taps, float* out, int out_C, int out_H, int out_W, const PixelTiling& til,
-                     int n_padded, int fH, int fW, int sgn, int off_h, int off_w, const float* bias, float* stats,
+                     int n_padded, int fH, int fW, int sgn, int off_h, int off_w, int k_real, const float* bias, float* stats,
                      cudaStream_t st, const ActEpilogue* act = nullptr, bool* act_done = nullptr) {
     {   // wide images with a filter that fits in shared memory: halo-reuse kernel
         bool used = false;
         const int padT = sgn > 0 ? -off_h : fH - 1 - off_h;
         const int padL = sgn > 0 ? -off_w : fW - 1 - off_w;
         int rc0 = run_halo_igemm(tf32, in, in_C, in_H, in_W, S, wmat, w_inner, rows_per_tap, taps, out, out_C, out_H, out_W,
-                                 n_padded, fH, fW, padT, padL, sgn > 0 ? 0 : 1, bias, stats,
+                                 halo_n(out_C, n_padded), fH, fW, padT, padL, sgn > 0 ? 0 : 1, k_real, bias, stats,
                                  sgn > 0 ? PK_IGEMM_FWD : PK_IGEMM_DX, st, &used);
         if (rc0 || used) return rc0;
     }
@@ -1342,6 +1353,7 @@ static int run_igemm(bool tf32, const void* in, int in_C, int in_H, int in_W, in
     p.rows_per_tap = rows_per_tap;
     p.fH = fH; p.fW = fW; p.sgn = sgn; p.off_h = off_h; p.off_w = off_w;
     p.kchunks = ceil_div(in_C, KC);
+    p.last_ksteps = last_ksteps(k_real, p.kchunks, KC);
     return tf32 ? dispatch_igemm<true>(p, nt, pair, st) : dispatch_igemm<false>(p, nt, pair, st);
 }
 
@@ -1373,7 +1385,7 @@ long long tc_conv_stats_blocks(const AetherConvDesc& d) {
     if (!tc_conv_eligible(d)) return 0;
     const TcPlan& pl = make_plan(d);
     const long long hb = halo_igemm_stats_blocks(pl.tf32, pl.tf32 ? d.Cin : pl.Cin_p, d.S, pl.taps, d.Cout, pl.Ho, pl.Wo,
-                                                 pl.Cout_p, d.fH, d.fW);
+                                                 halo_n(d.Cout, pl.Cout_p), d.fH, d.fW);
     if (hb > 0) return hb;
     // per-tap kernel: two rows per CTA group (the CTAs of one set of pixel tiles)
     const int nt = pick_nt(pl.Cout_p, pl.til_out.total());
@@ -1400,7 +1412,7 @@ int tc_conv_fwd(const AetherConvDesc& d, const float* x, const float* w, const f
             (rc = launch_filter_shadows<float>(w, wf, nullptr, pl.taps, d.Cin, d.Cout, pl.Cin_p, pl.Cout_p, st)))
             return rc;
         return run_igemm(true, x, d.Cin, d.H, d.W, d.S, wf, pl.Cin_p, pl.Cout_p, pl.taps, y, d.Cout, pl.Ho, pl.Wo,
-                         pl.til_out, pl.Cout_p, d.fH, d.fW, +1, -d.padH, -d.padW, b, stats, st);
+                         pl.til_out, pl.Cout_p, d.fH, d.fW, +1, -d.padH, -d.padW, d.Cin, b, stats, st);
     }
     __nv_bfloat16* xsh = reinterpret_cast<__nv_bfloat16*>(wsb + pl.off_xsh);
     __nv_bfloat16* wf = reinterpret_cast<__nv_bfloat16*>(wsb + pl.off_wf);
@@ -1415,7 +1427,7 @@ int tc_conv_fwd(const AetherConvDesc& d, const float* x, const float* w, const f
         (rc = launch_filter_shadows<__nv_bfloat16>(w, wf, wd, pl.taps, d.Cin, d.Cout, pl.Cin_p, pl.Cout_p, st)))
         return rc;
     return run_igemm(false, xsh, pl.Cin_p, d.H, d.W, d.S, wf, pl.Cin_p, pl.Cout_p, pl.taps, y, d.Cout, pl.Ho, pl.Wo,
-                     pl.til_out, pl.Cout_p, d.fH, d.fW, +1, -d.padH, -d.padW, b, stats, st, act, act_done);
+                     pl.til_out, pl.Cout_p, d.fH, d.fW, +1, -d.padH, -d.padW, d.Cin, b, stats, st, act, act_done);
 }
 
 template <bool TF32, int NB, bool PAIR>
@@ -1478,14 +1490,14 @@ int tc_conv_bwd(const AetherConvDesc& d, const float* x, const float* dy, const 
         if (pl.tf32) {
             // the caller's (taps, Cin, Cout) array already is the K-major matrix needed here
             rc = run_igemm(true, dy, d.Cout, pl.Ho, pl.Wo, d.S, w, d.Cout, d.Cin, pl.taps, dx, d.Cin, d.H, d.W,
-                           pl.til_in, pl.Cin_p, d.fH, d.fW, -1, d.padH, d.padW, nullptr, nullptr, st);
+                           pl.til_in, pl.Cin_p, d.fH, d.fW, -1, d.padH, d.padW, d.Cout, nullptr, nullptr, st);
         } else {
             __nv_bfloat16* wd = reinterpret_cast<__nv_bfloat16*>(wsb + pl.off_wd);
             if (!w_shadow_valid &&
                 (rc = launch_filter_shadows<__nv_bfloat16>(w, nullptr, wd, pl.taps, d.Cin, d.Cout, pl.Cin_p, pl.Cout_p, st)))
                 return rc;
             rc = run_igemm(false, dy_op, pl.Cout_p, pl.Ho, pl.Wo, d.S, wd, pl.Cout_p, pl.Cin_p, pl.taps, dx, d.Cin, d.H,
-                           d.W, pl.til_in, pl.Cin_p, d.fH, d.fW, -1, d.padH, d.padW, nullptr, nullptr, st);
+                           d.W, pl.til_in, pl.Cin_p, d.fH, d.fW, -1, d.padH, d.padW, d.Cout, nullptr, nullptr, st);
         }
         if (rc) return rc;
     }

@@ -18,7 +18,7 @@ int make_map_2d(CUtensorMap* m, const void* base, CUtensorMapDataType dt, int el
 // Halo-reuse kernel (conv_halo.cu): launches and sets *used when the problem fits it, else leaves *used false.
 int run_halo_igemm(bool tf32, const void* in, int in_C, int in_H, int in_W, int S, const void* wmat, int w_inner,
                    int rows_per_tap, int taps, float* out, int out_C, int out_H, int out_W, int n_padded, int fH, int fW,
-                   int padT, int padL, int flip, const float* bias, float* stats, int prof_kind, cudaStream_t st,
+                   int padT, int padL, int flip, int k_real, const float* bias, float* stats, int prof_kind, cudaStream_t st,
                    bool* used);
 // Partial-statistics blocks ([block][3][out_C]: count, mean, M2) the halo kernel writes when `stats` is given; 0 when
 // the halo kernel does not take the problem.
@@ -35,5 +35,11 @@ int rows_dw_max_splits(int Cin_p, int Cout_p, int Ho, int Wo, int S, int fH, int
 int run_rows_dw(const void* x_sh, int Cin_p, int H, int W, int S, const void* dy_sh, int Cout_p, int Ho, int Wo, int fH,
                 int fW, int padH, int padW, float* part, int* splits_a, int* splits_b, int* tap_split, cudaStream_t st,
                 bool* used);
+
+// MMAs (32 bytes of K each) that the last of `kchunks` 128-byte chunks needs when only k_real of the channels are not padding.
+static inline int last_ksteps(int k_real, int kchunks, int KC) {
+    const int rest = k_real - (kchunks - 1) * KC, step = KC / 4;
+    return rest >= KC ? 4 : rest <= step ? 1 : (rest + step - 1) / step;
+}
 
 }  // namespace aether
