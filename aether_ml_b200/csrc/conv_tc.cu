@@ -762,9 +762,16 @@ __device__ __forceinline__ void finish_columns(const float* __restrict__ part, i
     const int cl = threadIdx.x & 7, lane = threadIdx.x >> 3;
     const int c = cta * 8 + cl;
     float s = 0.f;
-    if (c < C)
-#pragma unroll 4
-        for (int b = lane; b < nblocks; b += 32) s += part[(size_t)b * C + c];
+    if (c < C) {
+        constexpr int U = 8;
+        for (int b = lane; b < nblocks; b += 32 * U) {
+            float v[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) v[u] = b + 32 * u < nblocks ? part[(size_t)(b + 32 * u) * C + c] : 0.f;
+#pragma unroll
+            for (int u = 0; u < U; ++u) s += v[u];
+        }
+    }
     red[lane][cl] = s;
     __syncthreads();
     if (lane == 0 && c < C) {
@@ -878,32 +885,30 @@ __global__ void __launch_bounds__(256) cast_bf16_kernel(const float* __restrict_
             long long r = r_begin + plane;
             if (whole) {
                 constexpr int U = 4;                     // rows in flight: eight 16-byte loads per thread
-                for (; r + (U - 1) * planes < r_end; r += U * planes) {
+                for (; r < r_end; r += U * planes) {
                     float4 t[U][2];
 #pragma unroll
                     for (int u = 0; u < U; ++u) {
-                        const float4* s = reinterpret_cast<const float4*>(src + (r + u * planes) * C + c0);
-                        t[u][0] = __ldcs(s);
-                        t[u][1] = __ldcs(s + 1);
+                        if (r + u * planes < r_end) {
+                            const float4* s = reinterpret_cast<const float4*>(src + (r + u * planes) * C + c0);
+                            t[u][0] = __ldcs(s);
+                            t[u][1] = __ldcs(s + 1);
+                        }
                     }
 #pragma unroll
                     for (int u = 0; u < U; ++u) {
-                        const float v[8] = {t[u][0].x, t[u][0].y, t[u][0].z, t[u][0].w, t[u][1].x, t[u][1].y, t[u][1].z, t[u][1].w};
-                        take(r + u * planes, v);
+                        if (r + u * planes < r_end) {
+                            const float v[8] = {t[u][0].x, t[u][0].y, t[u][0].z, t[u][0].w, t[u][1].x, t[u][1].y, t[u][1].z, t[u][1].w};
+                            take(r + u * planes, v);
+                        }
                     }
                 }
             }
-            for (; r < r_end; r += planes) {
+            for (; r < r_end; r += planes) {             // (channels of padding, rows that are no multiple of 16 bytes)
                 float v[8];
                 const float* s = src + r * C + c0;
-                if (whole) {
-                    const float4 a = __ldcs(reinterpret_cast<const float4*>(s)), b = __ldcs(reinterpret_cast<const float4*>(s + 4));
-                    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
-                    v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
-                } else {
 #pragma unroll
-                    for (int k = 0; k < 8; ++k) v[k] = (c0 + k < C) ? s[k] : 0.f;
-                }
+                for (int k = 0; k < 8; ++k) v[k] = (c0 + k < C) ? s[k] : 0.f;
                 take(r, v);
             }
         }
@@ -943,10 +948,13 @@ __global__ void __launch_bounds__(256) colsum_kernel(const float* __restrict__ s
         float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
         if (rl < lanes && c < C4) {
             const float4* s = reinterpret_cast<const float4*>(src) + c;
-#pragma unroll 8
-            for (long long r = r_begin + rl; r < r_end; r += lanes) {
-                const float4 v = s[r * C4];
-                acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
+            constexpr int U = 8;                         // (a rest taken one by one would be a round trip each)
+            for (long long r = r_begin + rl; r < r_end; r += U * lanes) {
+                float4 v[U];
+#pragma unroll
+                for (int u = 0; u < U; ++u) v[u] = r + u * lanes < r_end ? s[(r + u * lanes) * C4] : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+                for (int u = 0; u < U; ++u) { acc.x += v[u].x; acc.y += v[u].y; acc.z += v[u].z; acc.w += v[u].w; }
             }
         }
         red[threadIdx.x] = acc;

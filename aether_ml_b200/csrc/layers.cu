@@ -187,18 +187,18 @@ __global__ void __launch_bounds__(256) bn_reduce_vec4_kernel(const float* __rest
                     b.x = fmaf(g.x, xh.x, b.x); b.y = fmaf(g.y, xh.y, b.y);
                     b.z = fmaf(g.z, xh.z, b.z); b.w = fmaf(g.w, xh.w, b.w);
                 };
-                for (; r + (U - 1) * step < rows; r += U * step) {
+                for (; r < rows; r += U * step) {
                     float4 v[U], g[U];
 #pragma unroll
                     for (int u = 0; u < U; ++u) {
+                        const bool in = r + u * step < rows;
                         const size_t at = (size_t)(rows - 1 - r - u * step) * CV;
-                        g[u] = gr[at];
-                        v[u] = xr[at];
+                        g[u] = in ? gr[at] : z4;                         // (no gradient adds zero)
+                        v[u] = in ? xr[at] : mu;
                     }
 #pragma unroll
                     for (int u = 0; u < U; ++u) add(v[u], g[u]);
                 }
-                for (; r < rows; r += step) add(xr[(size_t)(rows - 1 - r) * CV], gr[(size_t)(rows - 1 - r) * CV]);
             }
         }
         sh_a4[threadIdx.x] = a;
