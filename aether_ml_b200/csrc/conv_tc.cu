@@ -111,6 +111,22 @@ int make_map_2d(CUtensorMap* m, const void* base, CUtensorMapDataType dt, int el
 }
 
 // ====================================================================================== igemm (forward and dX)
+// Pixel tile `t` as column, row and image tile.  32-bit divisions where the count allows (always in practice): four 64-bit
+// ones cost the one thread that issues copies 0.3 us per tile, as much as a small layer's tile takes to multiply.
+__device__ __forceinline__ void split_tile(long long t, long long total, int tiles_w, int tiles_h, int& tw, int& th, int& tn) {
+    if (total <= 0x7fffffffLL) {
+        const unsigned u = (unsigned)t, a = u / (unsigned)tiles_w;
+        tw = (int)(u - a * (unsigned)tiles_w);
+        tn = (int)(a / (unsigned)tiles_h);
+        th = (int)(a - (unsigned)tn * (unsigned)tiles_h);
+    } else {
+        const long long a = t / tiles_w;
+        tw = (int)(t - a * tiles_w);
+        tn = (int)(a / tiles_h);
+        th = (int)(a - (long long)tn * tiles_h);
+    }
+}
+
 struct IgemmParams {
     CUtensorMap tm_in;   // activations (C, W, H, N), box (128 B of channels, BW, BH, BN)
     CUtensorMap tm_w;    // filter matrix, K contiguous: (K, taps * rows_per_tap), box (128 B of K, NT)
@@ -226,13 +242,11 @@ __global__ void __launch_bounds__(IGEMM_THREADS, 1) igemm_conv_kernel(const __gr
     // pixel tile of this CTA in unit t; one past the last tile (odd tile count) decodes to an image index outside the
     // tensor: its loads are zero-filled and none of its rows is stored
     auto decode = [&](long long t, int& nt, int& w0, int& h0, int& n0) {
-        nt = (int)(t % p.n_tiles_n);
-        long long mt = t / p.n_tiles_n;
+        long long mt = total_tiles <= 0x7fffffffLL ? (long long)((unsigned)t / (unsigned)p.n_tiles_n) : t / p.n_tiles_n;
+        nt = (int)(t - mt * p.n_tiles_n);
         if (PAIR) mt = 2 * mt + cta_rank;
-        const int tw = (int)(mt % p.tiles_w);
-        mt /= p.tiles_w;
-        const int th = (int)(mt % p.tiles_h);
-        const int tn = (int)(mt / p.tiles_h);
+        int tw, th, tn;
+        split_tile(mt, m_tiles + 1, p.tiles_w, p.tiles_h, tw, th, tn);
         w0 = tw * p.BW; h0 = th * p.BH; n0 = tn * p.BN;
     };
     const int taps = p.fH * p.fW;
@@ -543,14 +557,20 @@ struct DwCfg {
     static constexpr int UC = TF32 ? 32 : 64;       // channels per 128-byte block
     static constexpr int MB = 128 / UC;             // x blocks per M=128
     static constexpr int NT = NB * UC;              // dy channels per CTA
-    static constexpr int STAGE_BYTES = (MB + NB) * TILE_A_BYTES;
-    static constexpr int STAGES = (200 * 1024) / STAGE_BYTES;
+    static constexpr int STAGE_BYTES = MB * TILE_A_BYTES;       // x of one M group
+    static constexpr int DY_BYTES = NB * TILE_A_BYTES;          // dy of one pixel tile
+    static constexpr int DY_STAGES = TF32 ? 2 : NB == 1 ? 4 : 3;        // (a CTA with one M group takes one per stage of x)
+    static constexpr int STAGES = (200 * 1024 - DY_STAGES * DY_BYTES) / STAGE_BYTES;
     static constexpr int KROWS = TF32 ? 8 : 16;     // pixel rows per MMA
-    static constexpr int SMEM_BYTES = 1024 + STAGES * STAGE_BYTES + 256;
+    static constexpr int SMEM_BYTES = 1024 + STAGES * STAGE_BYTES + DY_STAGES * DY_BYTES + 256;
     static constexpr int MAX_GPC = 512 / NT;
     static_assert(STAGES >= 2, "need at least two stages");
 };
 
+// The kernel is bound by what an SM can pull from L2 (some 100 GB/s of it), so a pixel tile's dy is brought in once, in
+// stages of its own, and stays for all M groups of the CTA: with one stage of x and dy per group the tf32 layer
+// 256 x 16x16 128->128 took 47 us, DWTXT.
+//
 // PAIR (clusters of two CTAs, cta_group::2): an M group is 256 rows -- each CTA stages the MB units of its own half --
 // and a column tile 2 * NT channels of dy, of which each CTA stages its own NT.  Per stage a CTA loads the same bytes as
 // a single CTA but the pair does four times one CTA's products with them: the kernel is bound by what an SM can pull
@@ -564,11 +584,15 @@ __global__ void __launch_bounds__(DW_THREADS, 1) dw_conv_kernel(const __grid_con
     extern __shared__ uint8_t smem_raw[];
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t* gen_base = smem_raw + (smem_base - smem_u32(smem_raw));
-    const uint32_t sBar = smem_base + STAGES * Cfg::STAGE_BYTES;
+    constexpr int D = Cfg::DY_STAGES;
+    const uint32_t sDy = smem_base + STAGES * Cfg::STAGE_BYTES;
+    const uint32_t sBar = sDy + D * Cfg::DY_BYTES;
     auto full_bar = [&](int s) { return sBar + 8u * s; };
     auto empty_bar = [&](int s) { return sBar + 8u * (STAGES + s); };
-    const uint32_t done_bar = sBar + 8u * (2 * STAGES);
-    const uint32_t sTmemPtr = sBar + 8u * (2 * STAGES + 1);
+    auto dfull_bar = [&](int s) { return sBar + 8u * (2 * STAGES + s); };
+    auto dempty_bar = [&](int s) { return sBar + 8u * (2 * STAGES + D + s); };
+    const uint32_t done_bar = sBar + 8u * (2 * STAGES + 2 * D);
+    const uint32_t sTmemPtr = sBar + 8u * (2 * STAGES + 2 * D + 1);
     volatile uint32_t* tmem_ptr_generic = reinterpret_cast<volatile uint32_t*>(gen_base + (sTmemPtr - smem_base));
 
     const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);      // (warp-uniform for the compiler, too)
@@ -581,7 +605,7 @@ __global__ void __launch_bounds__(DW_THREADS, 1) dw_conv_kernel(const __grid_con
     {
         const int k_end = (p.rows + Cfg::KROWS - 1) / Cfg::KROWS * Cfg::KROWS;
         const int per_tile = (k_end - p.rows) * 8;                              // 16-byte pieces
-        for (int i = threadIdx.x; i < STAGES * (MB + NB) * per_tile; i += blockDim.x) {
+        for (int i = threadIdx.x; i < (STAGES * MB + D * NB) * per_tile; i += blockDim.x) {
             const int tile = i / per_tile;
             *reinterpret_cast<uint4*>(gen_base + (size_t)tile * TILE_A_BYTES + p.rows * 128 + (i - tile * per_tile) * 16) = make_uint4(0, 0, 0, 0);
         }
@@ -591,6 +615,10 @@ __global__ void __launch_bounds__(DW_THREADS, 1) dw_conv_kernel(const __grid_con
         for (int s = 0; s < STAGES; ++s) {
             mbar_init(full_bar(s), 1);
             mbar_init(empty_bar(s), 1);
+        }
+        for (int s = 0; s < D; ++s) {
+            mbar_init(dfull_bar(s), 1);
+            mbar_init(dempty_bar(s), 1);
         }
         mbar_init(done_bar, 1);
         mbar_fence_init();
@@ -621,7 +649,7 @@ __global__ void __launch_bounds__(DW_THREADS, 1) dw_conv_kernel(const __grid_con
     const int g_end = min(p.MG, g_begin + p.gpc);
     const int ngroups = g_end - g_begin;
     const long long total_ptiles = 1LL * p.tiles_w * p.tiles_h * p.tiles_n;
-    const uint32_t stage_tx = (uint32_t)(MB + NB) * (uint32_t)p.rows * 128u * (uint32_t)PF;   // both CTAs' boxes
+    const uint32_t box_tx = (uint32_t)p.rows * 128u * (uint32_t)PF;                           // both CTAs' boxes
     const int ksteps = (p.rows + Cfg::KROWS - 1) / Cfg::KROWS;
 
     if (warp == 0) {
@@ -637,27 +665,28 @@ __global__ void __launch_bounds__(DW_THREADS, 1) dw_conv_kernel(const __grid_con
                 }
             };
             const Unit first = unit((g_begin * PF + cta_rank) * MB), last = unit(p.U - 1);
-            uint32_t s = 0, ph = 0;
+            uint32_t s = 0, ph = 0, ds = 0, dph = 0;
             bool ok = true;
             for (long long pt = split; pt < total_ptiles && ok; pt += splits) {
-                long long r = pt;
-                const int tw = (int)(r % p.tiles_w);
-                r /= p.tiles_w;
-                const int th = (int)(r % p.tiles_h);
-                const int tn = (int)(r / p.tiles_h);
+                int tw, th, tn;
+                split_tile(pt, total_ptiles, p.tiles_w, p.tiles_h, tw, th, tn);
                 const int w0 = tw * p.BW, h0 = th * p.BH, n0 = tn * p.BN;
+                if (!mbar_wait(dempty_bar(ds), dph ^ 1u, p.status, DS_TIMEOUT_EMPTY)) break;
+                if (issuer) mbar_arrive_expect_tx(dfull_bar(ds), box_tx * (uint32_t)NB);
+                const uint32_t dbar = PAIR ? cluster_map_shared(dfull_bar(ds), 0) : dfull_bar(ds);          // PAIR: the even CTA's
+#pragma unroll
+                for (int nb = 0; nb < NB; ++nb) {
+                    const int dyc = ((nt * PF + cta_rank) * NB + nb) * UC;
+                    if (PAIR) tma_load_4d_pair(sDy + ds * Cfg::DY_BYTES + nb * TILE_A_BYTES, &p.tm_dy, dbar, dyc, w0, h0, n0);
+                    else tma_load_4d(sDy + ds * Cfg::DY_BYTES + nb * TILE_A_BYTES, &p.tm_dy, dbar, dyc, w0, h0, n0);
+                }
+                if (++ds == D) { ds = 0; dph ^= 1u; }
                 Unit x = first;
                 for (int g = g_begin; g < g_end; ++g) {
                     if (!mbar_wait(empty_bar(s), ph ^ 1u, p.status, DS_TIMEOUT_EMPTY)) { ok = false; break; }
-                    if (issuer) mbar_arrive_expect_tx(full_bar(s), stage_tx);
-                    const uint32_t bar = PAIR ? cluster_map_shared(full_bar(s), 0) : full_bar(s);   // PAIR: the even CTA's
+                    if (issuer) mbar_arrive_expect_tx(full_bar(s), box_tx * (uint32_t)MB);
+                    const uint32_t bar = PAIR ? cluster_map_shared(full_bar(s), 0) : full_bar(s);
                     const uint32_t st = smem_base + s * Cfg::STAGE_BYTES;
-#pragma unroll
-                    for (int nb = 0; nb < NB; ++nb) {
-                        const int dyc = ((nt * PF + cta_rank) * NB + nb) * UC;
-                        if (PAIR) tma_load_4d_pair(st + (MB + nb) * TILE_A_BYTES, &p.tm_dy, bar, dyc, w0, h0, n0);
-                        else tma_load_4d(st + (MB + nb) * TILE_A_BYTES, &p.tm_dy, bar, dyc, w0, h0, n0);
-                    }
 #pragma unroll
                     for (int m = 0; m < MB; ++m) {
                         const Unit y = x.u < p.U ? x : last;       // padding unit of the last group: results are dropped
@@ -678,16 +707,18 @@ __global__ void __launch_bounds__(DW_THREADS, 1) dw_conv_kernel(const __grid_con
             // 32-byte-unit variant (4-row K groups).
             constexpr uint32_t LT = TF32 ? 1u : 2u;
             constexpr uint32_t SBO = TF32 ? 512u : 1024u;
-            uint32_t s = 0, ph = 0;
+            uint32_t s = 0, ph = 0, ds = 0, dph = 0;
             bool ok = true;
             uint32_t acc0 = 0;
             for (long long pt = split; pt < total_ptiles && ok; pt += splits) {
+                if (!mbar_wait(dfull_bar(ds), dph, p.status, DS_TIMEOUT_FULL)) break;
+                const uint64_t db0 = make_smem_desc(sDy + ds * Cfg::DY_BYTES, TILE_A_BYTES, SBO, LT);
                 for (int g = 0; g < ngroups; ++g) {
                     if (!mbar_wait(full_bar(s), ph, p.status, DS_TIMEOUT_FULL)) { ok = false; break; }
                     tc_fence_after();
                     const uint32_t a0 = smem_base + s * Cfg::STAGE_BYTES;
                     uint64_t da = make_smem_desc(a0, TILE_A_BYTES, SBO, LT);
-                    uint64_t db = make_smem_desc(a0 + MB * TILE_A_BYTES, TILE_A_BYTES, SBO, LT);
+                    uint64_t db = db0;
                     const uint32_t d_tmem = tmem_base + g * NTP;
                     uint32_t acc = acc0;
 #pragma unroll 4
@@ -706,6 +737,15 @@ __global__ void __launch_bounds__(DW_THREADS, 1) dw_conv_kernel(const __grid_con
                     }
                     if (++s == STAGES) { s = 0; ph ^= 1u; }
                 }
+                if (ok) {                                          // this tile's dy is free once all groups have used it
+                    if (PAIR) {
+                        umma_commit_pair(dempty_bar(ds));
+                        umma_commit_pair(cluster_map_shared(dempty_bar(ds), 1));
+                    } else {
+                        umma_commit(dempty_bar(ds));
+                    }
+                }
+                if (++ds == D) { ds = 0; dph ^= 1u; }
                 acc0 = 1u;
             }
             if (PAIR) {
@@ -1125,7 +1165,7 @@ static TcPlan compute_plan(const AetherConvDesc& d) {
     auto decompose_small = [&]() {
         pl.dw_MG = ceil_div(pl.dw_U, MB);
         pl.dw_ntn = pl.Cout_p / pl.dw_nt;
-        const double t_stage = 0.45 * (MB + pl.dw_nb) / 4.0, t_store = 0.5;
+        const double t_box = 0.45 / 4.0, t_store = 0.5;                         // a box of 16 KB from L2; an accumulator's store
         const double dw_us = 2.0 * pl.dw_U * UC * pl.Cout_p * 4.0 / 4e6;        // a partial written and read at 4 TB/s
         const int max_gpc = 512 / pl.dw_nt;
         double best = 1e30;
@@ -1133,7 +1173,7 @@ static TcPlan compute_plan(const AetherConvDesc& d) {
         for (int g = 1; g <= max_gpc && g <= pl.dw_MG; ++g) {
             const long long cols = 1LL * ceil_div(pl.dw_MG, g) * pl.dw_ntn;
             for (long long s = 1; s <= ptiles && s * cols <= num_sms(); ++s) {
-                const double cost = (double)((ptiles + s - 1) / s) * g * t_stage + g * t_store + (s > 1 ? 1.5 + s * dw_us : 0.0);
+                const double cost = (double)((ptiles + s - 1) / s) * (g * MB + pl.dw_nb) * t_box + g * t_store + (s > 1 ? 1.5 + s * dw_us : 0.0);
                 if (cost < best - 1e-9) { best = cost; best_gpc = g; best_splits = (int)s; }
             }
         }
