@@ -344,6 +344,23 @@ PyObject* py_tag(PyObject*, PyObject* o) {
                          (long long)t._version(), (long long)(t.dim() > 0 ? t.size(-1) : 1));
 }
 
+// same(tensor, tag): whether tag(tensor) starts with the values of `tag`, without building a tuple to compare.
+PyObject* py_same(PyObject*, PyObject* const* args, Py_ssize_t n) {
+    if (n != 2 || !THPVariable_Check(args[0]) || !PyTuple_Check(args[1]) || PyTuple_GET_SIZE(args[1]) > 4) {
+        PyErr_SetString(PyExc_TypeError, "expected a tensor and a tag");
+        return nullptr;
+    }
+    const at::Tensor& t = THPVariable_Unpack(args[0]);
+    const long long now[4] = {(long long)reinterpret_cast<intptr_t>(t.const_data_ptr()), (long long)t.numel(), (long long)t._version(),
+                              (long long)(t.dim() > 0 ? t.size(-1) : 1)};
+    for (Py_ssize_t i = 0; i < PyTuple_GET_SIZE(args[1]); ++i) {
+        long long v;
+        if (!integer(PyTuple_GET_ITEM(args[1], i), v)) return nullptr;
+        if (v != now[i]) Py_RETURN_FALSE;
+    }
+    Py_RETURN_TRUE;
+}
+
 #define METHOD(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_##name)), METH_FASTCALL, nullptr},
 PyMethodDef methods[] = {
     ENTRY_POINTS(METHOD)
@@ -358,6 +375,7 @@ PyMethodDef methods[] = {
     {"empty_i32", py_empty<at::kInt>, METH_O, "uninitialised int32 array on the current device"},
     {"empty_like", py_empty_like, METH_O, "uninitialised contiguous array of the argument's shape and type on the current device"},
     {"tag", py_tag, METH_O, "(address, elements, version, row length) of a tensor"},
+    {"same", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_same)), METH_FASTCALL, "whether a tensor still has the values of a tag"},
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_host", "native host path of aether_ml_b200", -1, methods};
 

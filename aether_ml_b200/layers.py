@@ -145,14 +145,14 @@ class _OperandCopies:
 
     def weights_valid(self, ws, w):
         """Whether the copies of the weights that the last forward pass left describe `w` still."""
-        return self.ws_ptr is not None and ws.data_ptr() == self.ws_ptr and host().tag(w) == self.w
+        return self.ws_ptr is not None and ws.data_ptr() == self.ws_ptr and host().same(w, self.w)
 
     def flags(self, ws, x, w):
         """Bit 0: the copy of x is valid; bit 1: the copies of the weights are (aether_conv2d_bwd's x_shadow_valid)."""
         if self.ws_ptr is None or ws.data_ptr() != self.ws_ptr:
             return 0
-        tag = host().tag
-        return (1 if tag(x) == self.x else 0) | (2 if tag(w) == self.w else 0)
+        same = host().same
+        return (1 if same(x, self.x) else 0) | (2 if same(w, self.w) else 0)
 
 
 _unwritten_exist = False        # whether any array has ever been marked (the check below is on every layer's path)
@@ -189,10 +189,10 @@ class _HandedIn:
         self.dy = None       # (workspace address, tag of dy, rows of column sums)
 
     def x_ready(self, ws, x):
-        return self.x is not None and self.x == (ws.data_ptr(), _array_tag(x))
+        return self.x is not None and self.x[0] == ws.data_ptr() and host().same(x, self.x[1])
 
     def dy_rows(self, ws, dy):
-        if self.dy is not None and self.dy[:2] == (ws.data_ptr(), _array_tag(dy)):
+        if self.dy is not None and self.dy[0] == ws.data_ptr() and host().same(dy, self.dy[1]):
             return self.dy[2]
         return 0
 
@@ -901,12 +901,14 @@ class Layer_Dense(_Saved):
         self._plans = {}
         self._copies = _OperandCopies()
         self._handed = _HandedIn()
+        self._used = (None, None)       # plan and weights of the last forward pass
 
     def _restore_transient(self):
         self._ws = _Workspace()
         self._plans = {}
         self._copies = _OperandCopies()
         self._handed = _HandedIn()
+        self._used = (None, None)       # plan and weights of the last forward pass
 
     def x_copy_target(self, shape):
         """(address, row length) where the bf16 copy of an input of `shape` (any shape that flattens to
@@ -939,9 +941,16 @@ class Layer_Dense(_Saved):
             p = self._plans[key] = _ConvPlan(AetherConvDesc(S, 1, 1, n_in, n_out, 1, 1, 1, 1, 0, 0, _lib.MATH_MODES[self.math_mode]), 1, 1)
         return p
 
-    def _operands(self, x):
-        """(plan, workspace, which operand copies in it are valid) for a forward pass over `x`."""
-        p = self._plan(x.shape[0])
+    def _current(self):
+        """The plan of the last forward pass (looked up again when its inputs or weights have been replaced since): looking
+        it up costs a microsecond, and a small network's step is bound by what its calls cost the host."""
+        p, w = self._used
+        if p is None or w is not self.weights or p.x_shape[0] != self.inputs.shape[0]:
+            p = self._plan(self.inputs.shape[0])
+        return p
+
+    def _operands(self, x, p):
+        """(workspace, which operand copies in it are valid) for a forward pass over `x` by plan `p`."""
         ws = self._ws.get(p.ws_bytes)
         flags = 0
         if self._handed.x is not None:
@@ -951,88 +960,90 @@ class Layer_Dense(_Saved):
             _require_written(x, "Layer_Dense.forward")
         if self._weights_fixed and p.layout is not None and self._copies.weights_valid(ws, self.weights):
             flags |= _lib.CONV_W_COPY_READY
-        return p, ws, flags
+        return ws, flags
 
     def forward(self, inputs, training):
         x = to_device(inputs)
         w = self.weights
         if x.ndim != 2 or x.shape[1] != w.shape[0]:
             raise ValueError(f"Layer_Dense expects (samples, {w.shape[0]}), got {tuple(x.shape)}")
-        p, ws, flags = self._operands(x)
+        p = self._plan(x.shape[0])
+        ws, flags = self._operands(x, p)
         H = host()
         y = H.empty((x.shape[0], w.shape[1]))
         H.aether_conv2d_fwd_ex(p.raw, x, w, self.biases, y, None, 0, ws, self._ws.size, flags)
         self.inputs = x
         self.output = y
+        self._used = (p, w)
         self._copies.record(ws, x, w)
         return y
 
-    def forward_act(self, x, alpha, target):
+    def forward_act(self, x, alpha, target, p):
         """`forward` and the (leaky) ReLU behind it in one call (Model): (output, activation's output)."""
         w = self.weights
-        p, ws, flags = self._operands(x)
+        ws, flags = self._operands(x, p)
         H = host()
-        shape = (x.shape[0], w.shape[1])
+        shape = (p.x_shape[0], p.b_shape[0])
         y, z = H.empty(shape), H.empty(shape)
         H.aether_conv2d_act_fwd(p.raw, x, w, self.biases, y, z, alpha, target[0] if target else None, target[1] if target else 0, ws,
                                 self._ws.size, flags)
         self.inputs = x
         self.output = y
+        self._used = (p, w)
         self._copies.record(ws, x, w)
         return y, z
 
-    def forward_softmax(self, x):
+    def forward_softmax(self, x, p):
         """`forward` of a classifier head and the SoftMax behind it in one launch (Model): (output, probabilities)."""
         w = self.weights
-        p, ws, _ = self._operands(x)
+        ws, _ = self._operands(x, p)
         H = host()
-        shape = (x.shape[0], w.shape[1])
+        shape = (p.x_shape[0], p.b_shape[0])
         y, prob = H.empty(shape), H.empty(shape)
         H.aether_head_softmax_fwd(p.raw, x, w, self.biases, y, prob)
         self.inputs = x
         self.output = y
+        self._used = (p, w)
         self._copies.record(ws, x, w)
         return y, prob
 
-    def backward_softmax(self, prob, labels, smooth):
+    def backward_softmax(self, prob, labels, smooth, p):
         """The combined softmax / cross-entropy gradient and this head's `backward`: the gradient with respect to the logits."""
         self._gradients()
         H = host()
-        p = self._plan(prob.shape[0])
         dz, dx = H.empty_like(prob), H.empty_like(self.inputs)
         kinds = [None, None, None]
         kinds[2 if labels.ndim == 2 else 1 if labels.dtype is torch.int64 else 0] = labels
         H.aether_head_cce_bwd(p.raw, prob, *kinds, smooth, self.weights, dz, dx)
-        self._backward(dz, False, dx)
+        self._backward(dz, False, p, dx)
         return dz
 
     def _gradients(self):
         if getattr(self, "_grad_views", None) is not None:
             self.dweights, self.dbiases = self._grad_views
         else:
-            self.dweights = host().empty_like(self.weights)
-            self.dbiases = host().empty_like(self.biases)
+            H = host()
+            self.dweights = H.empty_like(self.weights)
+            self.dbiases = H.empty_like(self.biases)
 
     def backward(self, dvalues):
         self._gradients()
-        return self._backward(to_device(dvalues), False)
+        return self._backward(to_device(dvalues), False, self._current())
 
-    def backward_act(self, act_inputs, dvalues, alpha):
+    def backward_act(self, act_inputs, dvalues, alpha, p):
         """`backward` of the (leaky) ReLU behind this layer and of the layer itself: (the activation's dinputs, dinputs)."""
         self._gradients()
         H = host()
-        p = self._plan(act_inputs.shape[0])
         lay = p.layout
         dy = H.empty_like(act_inputs)
-        H.aether_act_bwd_copy(act_inputs, dvalues, dy, dy.shape[0], dy.shape[1], alpha, self._ws.get(p.ws_bytes).data_ptr() + lay.dy_copy_offset,
+        H.aether_act_bwd_copy(act_inputs, dvalues, dy, p.x_shape[0], p.b_shape[0], alpha, self._ws.get(p.ws_bytes).data_ptr() + lay.dy_copy_offset,
                               lay.dy_copy_ld, self.dbiases)
-        return dy, self._backward(dy, True)
+        return dy, self._backward(dy, True, p)
 
-    def _backward(self, dy, dy_ready, dx=None):
+    def _backward(self, dy, dy_ready, p, dx=None):
         """``dy_ready``: the operand copy of dy and dbiases are there already; ``dx``: dinputs, when they are."""
         x = self.inputs
         w = self.weights
-        p = self._plan(x.shape[0])
         H = host()
         ws = self._ws.get(p.ws_bytes)
         want = None

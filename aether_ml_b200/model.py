@@ -272,10 +272,13 @@ class _DenseAct:
             return False
         x = to_device(inputs)
         dense, act = self.dense, self.act
-        if x.ndim != 2 or x.shape[1] != dense.weights.shape[0] or dense._plan(x.shape[0]).layout is None:
+        if x.ndim != 2 or x.shape[1] != dense.weights.shape[0]:
             return False
-        target = self.consumer.x_copy_target((x.shape[0], dense.weights.shape[1])) if self.consumer is not None else None
-        act.inputs, act.output = dense.forward_act(x, act._alpha, target)
+        p = dense._plan(x.shape[0])
+        if p.layout is None:
+            return False
+        target = self.consumer.x_copy_target((p.x_shape[0], p.b_shape[0])) if self.consumer is not None else None
+        act.inputs, act.output = dense.forward_act(x, act._alpha, target, p)
         if target:
             self.consumer.x_copy_written(act.output)
         return True
@@ -286,10 +289,10 @@ class _DenseAct:
         if y is None or not self._intact(layers, i) or dense.__dict__.get("output") is not y or not 0 < y.shape[0] <= self.MOST_ROWS:
             return False
         dy = to_device(dvalues)
-        lay = dense._plan(y.shape[0]).layout
-        if lay is None or dy.shape != y.shape or y.shape[0] != dense.inputs.shape[0]:
+        p = dense._current()
+        if p.layout is None or dy.shape != y.shape or y.shape[0] != dense.inputs.shape[0]:
             return False
-        act.dinputs, _ = dense.backward_act(y, dy, act._alpha)
+        act.dinputs, _ = dense.backward_act(y, dy, act._alpha, p)
         return True
 
 
@@ -320,9 +323,12 @@ class _Head:
             return False
         x = to_device(inputs)
         dense, softmax = self.dense, self.softmax
-        if x.ndim != 2 or x.shape[1] != dense.weights.shape[0] or x.shape[0] == 0 or not dense._plan(x.shape[0]).head:
+        if x.ndim != 2 or x.shape[1] != dense.weights.shape[0] or x.shape[0] == 0:
             return False
-        softmax.inputs, softmax.output = dense.forward_softmax(x)
+        p = dense._plan(x.shape[0])
+        if not p.head:
+            return False
+        softmax.inputs, softmax.output = dense.forward_softmax(x, p)
         return True
 
     def backward(self, layers, combined, output, y):
@@ -331,12 +337,15 @@ class _Head:
         z = softmax.__dict__.get("inputs")
         if (z is None or type(combined) is not Activation_Softmax_Loss_CategoricalCrossEntropy or "backward" in combined.__dict__
                 or softmax.output is not output or dense.__dict__.get("output") is not z or not self._intact(layers, len(layers) - 2)
-                or not dense._plan(z.shape[0]).head or z.shape[0] != dense.inputs.shape[0]):
+                or z.shape[0] != dense.inputs.shape[0]):
+            return False
+        p = dense._current()
+        if not p.head:
             return False
         labels = _labels(y)
         if labels.shape[0] != z.shape[0] or (labels.ndim == 2 and labels.shape != z.shape):
             return False
-        combined.dinputs = softmax.dinputs = dense.backward_softmax(output, labels, combined.label_smoothing)
+        combined.dinputs = softmax.dinputs = dense.backward_softmax(output, labels, combined.label_smoothing, p)
         return True
 
 
