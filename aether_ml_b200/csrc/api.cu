@@ -287,7 +287,7 @@ extern "C" int aether_conv2d_fwd(const AetherConvDesc* d, const float* x, const 
     if (tc_conv_eligible(*d)) return tc_conv_fwd(*d, x, w, b, y, nullptr, ws, ws_bytes, 0, st);
     if (first_tc_eligible(*d)) return first_tc_fwd(*d, x, w, b, y, nullptr, st);
     if (smallc_conv_eligible(*d) && (!b || aligned16(b))) return smallc_conv_fwd(*d, x, w, b, y, nullptr, st);
-    return generic_conv_fwd(*d, x, w, b, y, st);
+    return generic_conv_fwd(*d, x, w, b, y, ws, ws_bytes, st);
 }
 
 extern "C" int64_t aether_conv2d_bnstats_blocks(const AetherConvDesc* d) {
@@ -346,7 +346,7 @@ extern "C" int aether_conv2d_bwd_ex(const AetherConvDesc* d, const float* x, con
         return set_error(AE_UNSUPPORTED, "aether_conv2d_bwd_ex: this shape / math mode / request reads no operand copy of dy "
                                          "(aether_conv2d_operand_layout returned 0, or a first layer asked for dx)");
     if (tc_conv_eligible(*d)) return tc_conv_bwd(*d, x, dy, w, dx, dw, db, ws, ws_bytes, x_shadow_valid, dy_colsum_rows, st);
-    if (dx && (rc = generic_conv_bwd_data(*d, dy, w, dx, st))) return rc;
+    if (dx && (rc = generic_conv_bwd_data(*d, dy, w, dx, ws, ws_bytes, st))) return rc;
     if (dw && first_tc_bwd_eligible(*d))
         return first_tc_bwd_filter(*d, x, dy, dw, db, ws, ws_bytes, dy_ready ? dy_colsum_rows : 0, st);
     if ((dw || db) && smallc_conv_eligible(*d) && (!db || aligned16(db)))

@@ -64,8 +64,9 @@ static inline int ceil_div(int a, int b) { return (a + b - 1) / b; }
 static inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
 // ---- conv_simt.cu : fp32 CUDA-core convolution for any filter/stride/padding/channel count, tiled implicit GEMMs
-int simt_conv_fwd(const AetherConvDesc& d, const float* x, const float* w, const float* b, float* y, cudaStream_t st);
-int simt_conv_bwd_data(const AetherConvDesc& d, const float* dy, const float* w, float* dx, cudaStream_t st);
+// (`ws`: scratch, nullable; without it tiles that do not fill the SMs are not split)
+int simt_conv_fwd(const AetherConvDesc& d, const float* x, const float* w, const float* b, float* y, void* ws, size_t ws_bytes, cudaStream_t st);
+int simt_conv_bwd_data(const AetherConvDesc& d, const float* dy, const float* w, float* dx, void* ws, size_t ws_bytes, cudaStream_t st);
 int simt_conv_bwd_filter(const AetherConvDesc& d, const float* x, const float* dy, float* dw, float* db, void* ws,
                          size_t ws_bytes, cudaStream_t st);
 size_t simt_conv_workspace_bytes(const AetherConvDesc& d);
@@ -76,8 +77,9 @@ bool generic_head_shape(const AetherConvDesc& d);
 int generic_head_softmax_fwd(const AetherConvDesc& d, const float* x, const float* w, const float* b, float* y, float* prob, cudaStream_t st);
 int generic_head_cce_bwd(const AetherConvDesc& d, const float* prob, const int* labels, const long long* labels64, const float* targets,
                          float smooth, const float* w, float* dz, float* dx, cudaStream_t st);
-int generic_conv_fwd(const AetherConvDesc& d, const float* x, const float* w, const float* b, float* y, cudaStream_t st);
-int generic_conv_bwd_data(const AetherConvDesc& d, const float* dy, const float* w, float* dx, cudaStream_t st);
+int generic_conv_fwd(const AetherConvDesc& d, const float* x, const float* w, const float* b, float* y, void* ws, size_t ws_bytes,
+                     cudaStream_t st);
+int generic_conv_bwd_data(const AetherConvDesc& d, const float* dy, const float* w, float* dx, void* ws, size_t ws_bytes, cudaStream_t st);
 int generic_conv_bwd_filter(const AetherConvDesc& d, const float* x, const float* dy, float* dw, float* db, void* ws,
                             size_t ws_bytes, cudaStream_t st);
 size_t generic_conv_workspace_bytes(const AetherConvDesc& d);

@@ -352,9 +352,10 @@ static int head_fwd(const AetherConvDesc& d, const float* x, const float* w, con
     return check_launch("gen_fwd_pointwise_few_kernel");
 }
 
-int generic_conv_fwd(const AetherConvDesc& d, const float* x, const float* w, const float* b, float* y, cudaStream_t st) {
+int generic_conv_fwd(const AetherConvDesc& d, const float* x, const float* w, const float* b, float* y, void* ws, size_t ws_bytes,
+                     cudaStream_t st) {
     if (head_shape(d) && (reinterpret_cast<uintptr_t>(x) & 15u) == 0) return head_fwd(d, x, w, b, y, nullptr, st);
-    return simt_conv_fwd(d, x, w, b, y, st);
+    return simt_conv_fwd(d, x, w, b, y, ws, ws_bytes, st);
 }
 
 bool generic_head_shape(const AetherConvDesc& d) { return head_shape(d); }
@@ -399,7 +400,7 @@ static int dx_fewc(const AetherConvDesc& d, const float* dy, const float* w, flo
     return check_launch("dx_fewc_kernel");
 }
 
-int generic_conv_bwd_data(const AetherConvDesc& d, const float* dy, const float* w, float* dx, cudaStream_t st) {
+int generic_conv_bwd_data(const AetherConvDesc& d, const float* dy, const float* w, float* dx, void* ws, size_t ws_bytes, cudaStream_t st) {
     int Ho, Wo;
     conv_out_hw(d, Ho, Wo);
     // (Few input channels leave a GEMM tile's columns empty.  More than 65535 pixel classes do not fit a grid.)
@@ -412,7 +413,7 @@ int generic_conv_bwd_data(const AetherConvDesc& d, const float* dy, const float*
         }
     }
     if (head_shape(d) && (reinterpret_cast<uintptr_t>(dx) & 15u) == 0) return head_dx(d, dy, w, dx, nullptr, st);
-    return simt_conv_bwd_data(d, dy, w, dx, st);
+    return simt_conv_bwd_data(d, dy, w, dx, ws, ws_bytes, st);
 }
 
 // Parts of the rows of a classifier head's dW: four rows each until there are 128 of them (their sum is a pass of its own).

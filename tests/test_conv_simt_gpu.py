@@ -34,3 +34,14 @@ def test_tile_edges(shape):
     dxo, dwo, dbo = O.conv_backward(x.astype(np.float64), w.astype(np.float64), dy.astype(np.float64), st, pad)
     for got, want in ((y, yo), (dx, dxo), (layer.dweights, dwo), (layer.dbiases, dbo)):
         assert O.rel_l2(got.cpu().numpy(), want) <= 1e-5
+
+
+# Reductions cut into pieces: all tiles of a small layer, the tiles behind the full rounds of a larger one (whole rows of tiles:
+# 56 and 20 of 500 + 20), scalar and 16-byte rows, the classes of a strided layer's dX, pieces of unequal length.
+SPLIT = [(3, 9, 8, 130, 77, 3, (1, 1), "same"), (2, 7, 9, 256, 64, 3, (1, 1), "valid"), (5, 11, 10, 96, 52, 3, (2, 2), "same"),
+         (40, 40, 40, 64, 48, 3, (1, 1), "same"), (4, 8, 8, 200, 33, 5, (1, 1), "same"), (1, 6, 5, 260, 24, 1, (1, 1), "valid")]
+
+
+@pytest.mark.parametrize("shape", SPLIT)
+def test_split_reductions(shape):
+    test_tile_edges(shape)
