@@ -20,7 +20,7 @@ import torch
 from ._lib import host
 from .layers import (Activation_Softmax_Loss_CategoricalCrossEntropy, Batch_Norm, Conv_Layer, Flatten, Layer_Dense, Layer_Dropout,
                      Layer_Dropout_Spatial, Leaky_ReLU, Loss_CategoricalCrossEntropy, Optimizer_Adam, Pooling, ReLU, SoftMax, to_device, _labels,
-                     _labels_i32, _softmax_cce, _Saved)
+                     _labels_i32, _softmax_cce, _Saved, _Workspace)
 
 
 class Layer_Input:
@@ -359,6 +359,7 @@ class Model:
         self.flat_params = None
         self.grad_hook = None      # callable(flat_grads) run between backward and the optimizer (all-reduce)
         self._graph = self._graph_opt = None
+        self._graph_memory = None  # arrays that the captured kernels address but that the graph itself does not own
         self._graph_metrics = False
         self._m_last = self._m_sum = None
         self.bucket_reducer = None # dp.BucketReducer: all-reduces the flat gradients bucket by bucket during backward
@@ -686,6 +687,9 @@ class Model:
                 ts += [l._rm, l._rv]
         return ts
 
+    def _workspaces(self):
+        return [w for l in self.layers for w in vars(l).values() if isinstance(w, _Workspace)]
+
     def _all_ranks_agree(self, ok):
         """True when `ok` holds on every rank (one small eager all-reduce; single process: `ok` itself)."""
         import torch.distributed as dist
@@ -736,6 +740,9 @@ class Model:
         reducer = self.bucket_reducer if (self.bucket_reducer is not None and self.bucket_reducer.active) else None
         eager_between = self.grad_hook is not None or (reducer is not None and not collectives_in_graph)
         self._graph = self._graph_opt = None
+        # A replay addresses these whatever the layers do meanwhile: a layer that is given a larger batch (evaluation, say)
+        # replaces its workspace, whose memory would else go to other arrays that every replay then writes over.
+        self._graph_memory = [w.buf for w in self._workspaces()] + self._graph_state() + [self.flat_grads]
         self.capture_note = "one graph"
         if reducer is not None and not eager_between:
             graph, ok, err = torch.cuda.CUDAGraph(), True, ""
@@ -788,6 +795,7 @@ class Model:
         self._graph_metrics = False
         if torch.cuda.is_available():
             torch.cuda.synchronize()
+        self._graph_memory = None           # (a replay may have been running until here)
 
     def train_step_graph(self, X, y):
         """One training step by replaying the captured graph on a new batch of the captured shape."""
