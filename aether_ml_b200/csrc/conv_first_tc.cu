@@ -306,8 +306,16 @@ __global__ void __launch_bounds__(FT_THREADS, 1) first_conv_kernel(const __grid_
                     if (in_turn && nr > 0) {
                         float* base = stat_s + ch * 3 * 128 + tt;
                         float4* run = run_s + ch * 4 * 128 + tt;
-                        const float npiv = first ? 0.f : -base[0];
                         float s8[8], q8[8];
+                        if (first) {                                  // the mean first, then the squares about it
+#pragma unroll
+                            for (int k = 0; k < 8; ++k) s8[k] = 0.f;
+#pragma unroll
+                            for (int r = 0; r < 32; ++r) s8[r & 7] += r < nr ? val[r] : 0.f;
+                            base[0] = stats_tree(s8) * (1.f / (float)nr);
+                            base[128] = base[256] = 0.f;
+                        }
+                        const float npiv = -base[0];
                         if (persist && !first) {
 #pragma unroll
                             for (int h = 0; h < 2; ++h) {
@@ -329,19 +337,9 @@ __global__ void __launch_bounds__(FT_THREADS, 1) first_conv_kernel(const __grid_
                         };
                         if (nr == 32) add_rows(std::true_type{});
                         else add_rows(std::false_type{});
-                        if (!persist || first) {
-                            float s = stats_tree(s8), sq = stats_tree(q8);
-                            if (first) {
-                                const float piv = s * (1.f / (float)nr);
-                                base[0] = piv;
-                                base[128] = 0.f;
-                                base[256] = sq - s * piv;
-                            } else {
-                                base[128] += s;
-                                base[256] += sq;
-                            }
-#pragma unroll
-                            for (int k = 0; k < 8; ++k) s8[k] = q8[k] = 0.f;
+                        if (!persist) {
+                            base[128] += stats_tree(s8);
+                            base[256] += stats_tree(q8);
                         }
                         if (persist) {
 #pragma unroll
@@ -382,10 +380,9 @@ __global__ void __launch_bounds__(FT_THREADS, 1) first_conv_kernel(const __grid_
                         *reinterpret_cast<float4*>(v + 4) = run[384];
                         q += stats_tree(v);
                     }
-                    const float m = s / n, mean = base[0] + m, m2 = fmaxf(q - s * m, 0.f);
-                    double dn, ds, dq;
-                    stats_row_terms(n, mean, m2, dn, ds, dq);
-                    N += dn; S += ds; Q += dq;
+                    const float m2 = fmaxf(q - s * (s / n), 0.f);
+                    const double mean = (double)base[0] + (double)s / (double)n;       // (rounded once, with the sums of all rows)
+                    N += n; S += n * mean; Q += m2 + n * mean * mean;
                 }
                 stats_store_rows(N, S, Q, sp, c, p.Cout);
             }
