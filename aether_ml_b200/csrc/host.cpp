@@ -263,6 +263,7 @@ PyObject* py_bind(PyObject*, PyObject* args) {
 // ---------------------------------------------------------------------------------- arrays
 // The argument itself when it is a contiguous fp32 CUDA tensor, else None.
 PyObject* py_ready(PyObject*, PyObject* o) {
+    HANDLE_TH_ERRORS                              // (a sparse tensor has no contiguity to ask for)
     if (THPVariable_Check(o)) {
         const at::Tensor& t = THPVariable_Unpack(o);
         if (t.is_cuda() && t.scalar_type() == at::kFloat && t.is_contiguous()) {
@@ -271,6 +272,7 @@ PyObject* py_ready(PyObject*, PyObject* o) {
         }
     }
     Py_RETURN_NONE;
+    END_HANDLE_TH_ERRORS
 }
 
 PyObject* py_device(PyObject*, PyObject*) {
@@ -285,6 +287,8 @@ PyObject* new_array(at::IntArrayRef sizes, at::ScalarType type) {
     END_HANDLE_TH_ERRORS
 }
 
+// Every function below runs inside HANDLE_TH_ERRORS where torch may throw (a tensor of inference mode has no version counter, a
+// wrapped tensor no address): an exception that left a C callback would end the process.
 template <at::ScalarType TYPE>
 PyObject* py_empty(PyObject*, PyObject* shape) {
     if (!PyTuple_Check(shape) || PyTuple_GET_SIZE(shape) > 8) {
@@ -299,20 +303,24 @@ PyObject* py_empty(PyObject*, PyObject* shape) {
 }
 
 PyObject* py_empty_like(PyObject*, PyObject* o) {
+    HANDLE_TH_ERRORS
     if (!THPVariable_Check(o)) {
         PyErr_SetString(PyExc_TypeError, "expected a tensor");
         return nullptr;
     }
     const at::Tensor& t = THPVariable_Unpack(o);
     return new_array(t.sizes(), t.scalar_type());
+    END_HANDLE_TH_ERRORS
 }
 
 // upload(values, like_shape): a new array of that shape with the fp32 values of a contiguous host buffer.
 PyObject* py_upload(PyObject*, PyObject* const* args, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
     if (fn_upload == nullptr || n != 2) {
         PyErr_SetString(PyExc_TypeError, "upload takes a host array and a shape, and needs a bound library");
         return nullptr;
     }
+    void* const stream = current_stream();        // (nothing throws while the buffer is held)
     Py_buffer b;
     if (PyObject_GetBuffer(args[0], &b, PyBUF_C_CONTIGUOUS | PyBUF_FORMAT) != 0) return nullptr;
     PyObject* t = nullptr;
@@ -322,8 +330,8 @@ PyObject* py_upload(PyObject*, PyObject* const* args, Py_ssize_t n) {
         const at::Tensor& a = THPVariable_Unpack(t);
         int rc = AETHER_E_BAD_ARG;
         if (a.numel() == b.len / 4 && a.numel() < (1 << 30))
-            rc = reinterpret_cast<decltype(&aether_upload)>(fn_upload)(static_cast<const float*>(b.buf), a.data_ptr<float>(), (int)a.numel(),
-                                                                       current_stream());
+            rc = reinterpret_cast<decltype(&aether_upload)>(fn_upload)(static_cast<const float*>(b.buf), static_cast<float*>(a.mutable_data_ptr()),
+                                                                       (int)a.numel(), stream);
         if (rc != 0) {
             Py_DECREF(t);
             t = fail(rc, "aether_upload");
@@ -331,10 +339,12 @@ PyObject* py_upload(PyObject*, PyObject* const* args, Py_ssize_t n) {
     }
     PyBuffer_Release(&b);
     return t;
+    END_HANDLE_TH_ERRORS
 }
 
 // Identity of an array's contents as far as the host can tell: address, elements, in-place changes so far, row length.
 PyObject* py_tag(PyObject*, PyObject* o) {
+    HANDLE_TH_ERRORS
     if (!THPVariable_Check(o)) {
         PyErr_SetString(PyExc_TypeError, "expected a tensor");
         return nullptr;
@@ -342,10 +352,12 @@ PyObject* py_tag(PyObject*, PyObject* o) {
     const at::Tensor& t = THPVariable_Unpack(o);
     return Py_BuildValue("(nLLL)", (Py_ssize_t) reinterpret_cast<intptr_t>(t.const_data_ptr()), (long long)t.numel(),
                          (long long)t._version(), (long long)(t.dim() > 0 ? t.size(-1) : 1));
+    END_HANDLE_TH_ERRORS
 }
 
 // same(tensor, tag): whether tag(tensor) starts with the values of `tag`, without building a tuple to compare.
 PyObject* py_same(PyObject*, PyObject* const* args, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
     if (n != 2 || !THPVariable_Check(args[0]) || !PyTuple_Check(args[1]) || PyTuple_GET_SIZE(args[1]) > 4) {
         PyErr_SetString(PyExc_TypeError, "expected a tensor and a tag");
         return nullptr;
@@ -359,6 +371,7 @@ PyObject* py_same(PyObject*, PyObject* const* args, Py_ssize_t n) {
         if (v != now[i]) Py_RETURN_FALSE;
     }
     Py_RETURN_TRUE;
+    END_HANDLE_TH_ERRORS
 }
 
 #define METHOD(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_##name)), METH_FASTCALL, nullptr},
