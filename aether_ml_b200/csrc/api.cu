@@ -242,8 +242,8 @@ extern "C" int aether_conv2d_act_fwd(const AetherConvDesc* d, const float* x, co
     int Ho, Wo;                                          // a kernel without that epilogue: the passes by themselves
     conv_out_hw(*d, Ho, Wo);
     const int64_t rows = 1LL * d->S * Ho * Wo;
-    if ((rc = aether_leaky_relu_fwd(y, act_out, rows * d->Cout, alpha, stream)) || !act_copy) return rc;
-    return tc_cast_operand(act_out, act_copy, rows, d->Cout, copy_ld, st);
+    if (!act_copy) return aether_leaky_relu_fwd(y, act_out, rows * d->Cout, alpha, stream);
+    return act_fwd_copy(y, act_out, alpha, act_copy, rows, d->Cout, copy_ld, st);
 }
 
 extern "C" int aether_head_supported(const AetherConvDesc* d) {

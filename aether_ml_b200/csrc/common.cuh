@@ -111,7 +111,6 @@ int smallc_reduce_partials(const float* part, int nb, int K, int Cout, float* dw
 bool tc_conv_eligible(const AetherConvDesc& d);
 size_t tc_conv_workspace_bytes(const AetherConvDesc& d);
 // `stats` (nullable): per-block (count, mean, M2) of every output channel, tc_conv_stats_blocks(d) blocks of [3][Cout]
-int tc_cast_operand(const float* src, void* dst, long long rows, int C, int ld, cudaStream_t st);   // fp32 rows -> bf16 rows of ld
 // A (leaky) ReLU that the forward kernel may apply in its epilogue: its output and, nullable, the bf16 copy of
 // that in rows of `ld`.
 struct ActEpilogue {
@@ -139,6 +138,9 @@ float* bn_eval_coeffs(const float* gamma, const float* beta, const float* runnin
 void bn_backward_coeffs(const float* part, int nb, int C, long long rows, const float* gamma, const float* mean,
                         const float* var, float eps, float* dgamma, float* dbeta, float* coeff, const float* pscale,
                         cudaStream_t st);
+
+// a (leaky) ReLU over [rows][C] and the bf16 copy of its output in rows of `ld` (C % 4 == 0, ld % 4 == 0, copy 8-byte aligned)
+int act_fwd_copy(const float* x, float* out, float alpha, void* copy, long long rows, int C, int ld, cudaStream_t st);
 
 void bn_backward_apply(const float* x, const float* dy, float* dx, const float* coeff, long long n, int C, cudaStream_t st);
 

@@ -1425,10 +1425,6 @@ static int launch_cast(const float* src, __nv_bfloat16* dst, long long rows, int
     return check_launch("cast_bf16_kernel");
 }
 
-int tc_cast_operand(const float* src, void* dst, long long rows, int C, int ld, cudaStream_t st) {
-    return launch_cast(src, static_cast<__nv_bfloat16*>(dst), rows, C, ld, nullptr, 0, st);
-}
-
 long long tc_conv_stats_blocks(const AetherConvDesc& d) {
     if (!tc_conv_eligible(d)) return 0;
     const TcPlan& pl = make_plan(d);

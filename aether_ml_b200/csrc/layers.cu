@@ -1136,6 +1136,35 @@ __global__ void __launch_bounds__(256) lrelu_bwd_kernel(const float* __restrict_
         dx[i] = x[i] < 0.f ? alpha * dy[i] : dy[i];
 }
 
+// The activation's forward pass with the bf16 operand copy of its output, zero in the padded columns: for shapes whose
+// convolution kernel does not write both in its epilogue.  Four columns per thread: rows of the copy need be no longer than
+// the next multiple of four, and its 8-byte stores no more than 8-byte alignment.
+__global__ void __launch_bounds__(256) act_fwd_copy_kernel(const float* __restrict__ x, float* __restrict__ out, long long rows, int C,
+                                                           float alpha, __nv_bfloat16* __restrict__ copy, int ld) {
+    pdl_wait();
+    const int L4 = ld >> 2;
+    const long long n = rows * L4, stride = (long long)gridDim.x * blockDim.x;
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += stride) {
+        const long long r = i / L4;
+        const int c = (int)(i - r * L4) * 4;
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (c < C) {
+            v = *reinterpret_cast<const float4*>(x + r * C + c);
+            v.x = v.x > 0.f ? v.x : alpha * v.x; v.y = v.y > 0.f ? v.y : alpha * v.y;
+            v.z = v.z > 0.f ? v.z : alpha * v.z; v.w = v.w > 0.f ? v.w : alpha * v.w;
+            *reinterpret_cast<float4*>(out + r * C + c) = v;
+        }
+        const __nv_bfloat162 o[2] = {__floats2bfloat162_rn(v.x, v.y), __floats2bfloat162_rn(v.z, v.w)};
+        *reinterpret_cast<uint2*>(copy + r * ld + c) = *reinterpret_cast<const uint2*>(o);
+    }
+}
+
+int act_fwd_copy(const float* x, float* out, float alpha, void* copy, long long rows, int C, int ld, cudaStream_t st) {
+    launch(act_fwd_copy_kernel, blocks_for(rows * (ld / 4), 256), 256, 0, st, x, out, rows, C, alpha, static_cast<__nv_bfloat16*>(copy), ld);
+    count_launch();
+    return check_launch("act_fwd_copy_kernel");
+}
+
 // The activation's backward pass in front of a Dense layer's: dx as above, its bf16 operand copy (rows of ld, zero in the
 // padded columns) and its column sums, the layer's dB -- one launch instead of three for the few hundred rows of a small
 // network.  A CTA owns 32 columns and walks all rows, 32 at a time, so the sums need no second pass.
