@@ -1258,6 +1258,14 @@ class Optimizer_Adam(_Saved):
         self._step(layer.weights, layer.dweights, layer.weight_momentums, layer.weight_cache)
         self._step(layer.biases, layer.dbiases, layer.bias_momentums, layer.bias_cache)
 
+    def updates_as_adam(self):
+        """Whether ``update_layers`` does what calling ``update_parameters`` for each layer does: not where a subclass or a
+        patched method updates in its own way."""
+        cls, own = type(self), self.__dict__
+        return (cls.update_parameters is Optimizer_Adam.update_parameters and cls._step is Optimizer_Adam._step
+                and cls._ensure_state is Optimizer_Adam._ensure_state
+                and not ("update_parameters" in own or "_step" in own or "_ensure_state" in own))
+
     def update_layers(self, layers):
         """``update_parameters`` of every layer in one launch (a layer by itself is two launches of a few microseconds)."""
         if self.step_dev is not None:

@@ -629,7 +629,7 @@ class Model:
             self._updated_early = set()
         elif self.flat_params is not None and hasattr(opt, "update_flat"):
             opt.update_flat(self.flat_params, self.flat_grads, self.flat_m, self.flat_v)
-        elif type(opt).update_parameters is Optimizer_Adam.update_parameters:
+        elif isinstance(opt, Optimizer_Adam) and opt.updates_as_adam():
             opt.update_layers(self.trainable_layers)
         else:
             for layer in self.trainable_layers:
