@@ -1647,13 +1647,22 @@ extern "C" int aether_adam_steps(const AetherAdamTensor* tensors, int count, flo
         if (!tensors[i].p || !tensors[i].g || !tensors[i].m || !tensors[i].v || tensors[i].n <= 0)
             return set_error(AE_BAD_ARG, "aether_adam_steps: bad tensor %d", i);
     const AdamScalars a = {lr, beta1, beta2, eps, 1.f / bias_corr1, 1.f / bias_corr2, grad_scale};
-    for (int begin = 0; begin < count; begin += ADAM_LIST) {
+    // Tensors of one launch are updated side by side: one that shares memory with an earlier one (weights of two tied layers,
+    // a layer listed twice) begins the next launch, so that the updates follow each other as in the caller's list.
+    auto overlap = [](const float* a, int64_t na, const float* b, int64_t nb) { return a < b + nb && b < a + na; };
+    auto shares = [&](const AetherAdamTensor& a, const AetherAdamTensor& b) {
+        return overlap(a.p, a.n, b.p, b.n) || overlap(a.m, a.n, b.m, b.n) || overlap(a.v, a.n, b.v, b.n);
+    };
+    for (int begin = 0; begin < count;) {
         AdamList l;
-        l.count = count - begin < ADAM_LIST ? count - begin : ADAM_LIST;
         l.first_block[0] = 0;
-        for (int i = 0; i < l.count; ++i) {
-            l.t[i] = tensors[begin + i];
-            l.first_block[i + 1] = l.first_block[i] + blocks_for(l.t[i].n / 4 + 1, 256);
+        for (l.count = 0; l.count < ADAM_LIST && begin < count; ++l.count, ++begin) {
+            const AetherAdamTensor& t = tensors[begin];
+            bool apart = true;
+            for (int i = 0; i < l.count && apart; ++i) apart = !shares(t, l.t[i]);
+            if (!apart) break;
+            l.t[l.count] = t;
+            l.first_block[l.count + 1] = l.first_block[l.count] + blocks_for(t.n / 4 + 1, 256);
         }
         launch(adam_list_kernel, l.first_block[l.count], 256, 0, static_cast<cudaStream_t>(stream), l, a);
         count_launch();

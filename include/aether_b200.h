@@ -321,7 +321,8 @@ int aether_mul(const float* a, const float* b, float* y, int64_t n, void* stream
 int aether_adam_step(float* p, const float* g, float* m, float* v, int64_t n, float lr, float beta1, float beta2,
                      float eps, float bias_corr1, float bias_corr2, float grad_scale, void* stream);
 /* The same update of several tensors in one launch (Model's loop over the trainable layers, CNN_model_cupy.py:124-125):
- * `tensors` is a HOST array of `count` entries. */
+ * `tensors` is a HOST array of `count` entries.  Entries that share parameters or moments are updated one after the other, in
+ * the order of the array (a launch for each set of entries that share nothing). */
 typedef struct AetherAdamTensor {
     float* p;
     const float* g;
