@@ -930,15 +930,17 @@ class Model:
                 head = (len(passes) - 1) * batch_size
                 passes = [slice(k, min(k + step, head)) for k in range(0, head, step)] + passes[-1:]
         fixed = [l for l in self.layers if hasattr(l, "_weights_fixed")]
-        try:
-            for k, sl in enumerate(passes):
-                if k == 1:
+        for k, sl in enumerate(passes):
+            # (set for the pass only: a caller that leaves its loop by an exception does not resume this one, and may train next)
+            try:
+                if k > 0:
                     for l in fixed:
                         l._weights_fixed = True
-                yield sl, self.forward(X[sl], training=False, keep=k == len(passes) - 1)
-        finally:
-            for l in fixed:
-                l._weights_fixed = False
+                output = self.forward(X[sl], training=False, keep=k == len(passes) - 1)
+            finally:
+                for l in fixed:
+                    l._weights_fixed = False
+            yield sl, output
 
     def evaluate(self, X_val, y_val, *, batch_size=None):
         self.loss.new_pass()
