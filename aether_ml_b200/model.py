@@ -918,12 +918,17 @@ class Model:
             total += 4 * math.prod(shape)
         return total if total > 0 else None
 
+    def _own_forward(self):
+        """False where a subclass or a patched method runs the passes: it gets the batches and the arguments it knows."""
+        return type(self).forward is Model.forward and "forward" not in vars(self)
+
     def _inference(self, X, batch_size):
         """Slices and outputs of the forward passes over X: whole batches, several at once where they are small, then the
         last batch by itself, whose inputs and outputs the layers keep.  The weights stay as they are between the passes of
         one call, so from the second on the tensor-core layers use the operand copies of them that the first one made."""
         passes = _batches(len(X), batch_size)
-        if len(passes) > 2 and hasattr(X, "shape"):
+        own = self._own_forward()
+        if own and len(passes) > 2 and hasattr(X, "shape"):
             per_sample = self._output_bytes(tuple(X.shape[1:]))
             if per_sample is not None:
                 step = batch_size * max(1, self.INFERENCE_PASS_BYTES // (per_sample * batch_size))
@@ -936,7 +941,7 @@ class Model:
                 if k > 0:
                     for l in fixed:
                         l._weights_fixed = True
-                output = self.forward(X[sl], training=False, keep=k == len(passes) - 1)
+                output = self.forward(X[sl], training=False, **({"keep": k == len(passes) - 1} if own else {}))
             finally:
                 for l in fixed:
                     l._weights_fixed = False
@@ -956,9 +961,9 @@ class Model:
         return float(validation_accuracy), float(validation_loss)
 
     def predict(self, X, *, batch_size=None):
-        # (SoftMax writes a new array every time; an output layer of the caller's may not)
-        own = type(self.layers[-1]) is SoftMax
-        outs = [output if own else output.clone() for _, output in self._inference(X, batch_size)]
+        # (SoftMax writes a new array every time; an output layer or a forward pass of the caller's may not)
+        new = type(self.layers[-1]) is SoftMax and "forward" not in vars(self.layers[-1]) and self._own_forward()
+        outs = [output if new else output.clone() for _, output in self._inference(X, batch_size)]
         return torch.vstack(outs)
 
     # ------------------------------------------------------------------ parameters
