@@ -121,7 +121,7 @@ class _Workspace:
     def get(self, nbytes):
         if self.size < nbytes or self.buf is None:
             nbytes = max(int(nbytes), 256)
-            self.buf = torch.empty(nbytes, dtype=torch.uint8, device=_device())
+            self.buf = host().empty_u8((nbytes,))
             self.size = nbytes
         return self.buf
 
@@ -179,6 +179,14 @@ def _array_tag(t):
     return host().tag(t)[:3]
 
 
+class _TakesCopies:
+    """What the layers with bf16 operand copies in their workspace share."""
+
+    def _forget_copies(self):
+        """The workspace's contents are no longer what the last passes left there."""
+        self._copies.ws_ptr = self._handed.x = self._handed.dy = None
+
+
 class _HandedIn:
     """Operand copies that a neighbouring layer's kernel wrote into this layer's workspace (see
     aether_conv2d_operand_layout): which array each describes, so the layer skips its own cast pass only for
@@ -222,7 +230,7 @@ class _ConvPlan:
 
 
 # ------------------------------------------------------------------------------------- Conv_Layer
-class Conv_Layer(_Saved):
+class Conv_Layer(_TakesCopies, _Saved):
     """Drop-in for ``Conv_Layer`` (CNN_classes_cupy.py:37-161).
 
     Same constructor arguments and attributes (``filter_weights``/``weights`` alias, ``biases``, the
@@ -880,7 +888,7 @@ class Flatten(_Saved):
         return self.dinputs
 
 
-class Layer_Dense(_Saved):
+class Layer_Dense(_TakesCopies, _Saved):
     """Drop-in for ``Layer_Dense`` (CNN_classes_cupy.py:315-362).  The three products run through the
     convolution kernels as a 1x1 convolution on a 1x1 image (x (S,n_in) is NHWC with H=W=1; weights
     (n_in,n_out) are a (1,1,Cin,Cout) filter), so they use the same tensor-core path.  Parameters are

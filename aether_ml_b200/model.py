@@ -20,7 +20,7 @@ import torch
 from ._lib import host
 from .layers import (Activation_Softmax_Loss_CategoricalCrossEntropy, Batch_Norm, Conv_Layer, Flatten, Layer_Dense, Layer_Dropout,
                      Layer_Dropout_Spatial, Leaky_ReLU, Loss_CategoricalCrossEntropy, Optimizer_Adam, Pooling, ReLU, SoftMax, to_device, _labels,
-                     _labels_i32, _softmax_cce, _Saved, _Workspace)
+                     _labels_i32, _softmax_cce, _Saved, _TakesCopies, _Workspace)
 
 
 class Layer_Input:
@@ -688,7 +688,9 @@ class Model:
         return ts
 
     def _workspaces(self):
-        return [w for l in self.layers for w in vars(l).values() if isinstance(w, _Workspace)]
+        """(layer, workspace, its buffer, its size) of all layers' workspaces as they are."""
+        names = ("_ws", "_stats_ws")
+        return [(l, w, w.buf, w.size) for l in self.layers for w in map(l.__dict__.get, names) if type(w) is _Workspace]
 
     def _all_ranks_agree(self, ok):
         """True when `ok` holds on every rank (one small eager all-reduce; single process: `ok` itself)."""
@@ -742,7 +744,7 @@ class Model:
         self._graph = self._graph_opt = None
         # A replay addresses these whatever the layers do meanwhile: a layer that is given a larger batch (evaluation, say)
         # replaces its workspace, whose memory would else go to other arrays that every replay then writes over.
-        self._graph_memory = [w.buf for w in self._workspaces()] + self._graph_state() + [self.flat_grads]
+        self._graph_memory = [buf for _, _, buf, _ in self._workspaces()] + self._graph_state() + [self.flat_grads]
         self.capture_note = "one graph"
         if reducer is not None and not eager_between:
             graph, ok, err = torch.cuda.CUDAGraph(), True, ""
@@ -886,75 +888,125 @@ class Model:
         if validation_data is not None:
             self.evaluate(*validation_data, batch_size=batch_size)
 
-    # Bytes of layer outputs that an inference pass takes several batches together up to.  A batch of the reference's networks
-    # leaves most of the GPU idle in its deeper layers and takes longer to launch than to run (32x32 network, batch 128:
-    # 112 us of host work for 86 us on the GPU), so a pass takes as many whole batches as keep its outputs within a
-    # gigabyte, as much as a training batch of 512 of that network: 1000 images in batches of 128, 900 -> 295 us.
-    INFERENCE_PASS_BYTES = 1 << 30
-    _PER_SAMPLE = (Conv_Layer, Batch_Norm, ReLU, Leaky_ReLU, Layer_Dropout, Layer_Dropout_Spatial, Pooling, Flatten, Layer_Dense, SoftMax)
+    # Bytes of layer outputs and workspaces that an inference pass takes several batches together up to.  A batch of the
+    # reference's networks leaves most of the GPU idle in its deeper layers and takes longer to launch than to run (32x32 network,
+    # batch 128: 112 us of host work for 86 us on the GPU), so a pass takes as many whole batches as keep its arrays within
+    # what a training batch of 512 of that network needs with its gradients: 1000 images in batches of 128, 900 -> 260 us (in
+    # one pass and the last batch; in three of at most a gigabyte 436 us).  Workspaces that training has given the layers
+    # are theirs again when the call ends, and where the memory is not there the batches are run one by one.
+    INFERENCE_PASS_BYTES = 5 << 28
+    _PER_SAMPLE = frozenset((Conv_Layer, Batch_Norm, ReLU, Leaky_ReLU, Layer_Dropout, Layer_Dropout_Spatial, Pooling, Flatten, Layer_Dense, SoftMax))
 
     def _output_bytes(self, shape):
-        """Bytes of all layers' outputs for one sample of ``shape``; None when a layer is not one of this package's own,
-        which treat every sample by itself in inference, or does not take the shape."""
-        total = 0
+        """Bytes of all layers' outputs for one sample of ``shape``, and the layers with a workspace that grows with the batch,
+        each with the shape of its sample; None when a layer is not one of this package's own, which treat every sample by
+        itself in inference, or does not take the shape."""
+        total, working, n = 0, [], math.prod(shape)
         for l in self.layers:
-            if type(l) not in self._PER_SAMPLE or "forward" in l.__dict__:
+            kind = type(l)
+            if kind not in self._PER_SAMPLE or "forward" in l.__dict__:
                 return None
-            if type(l) is Conv_Layer:
+            if kind is Conv_Layer:
                 if len(shape) != 3:
                     return None
+                working.append((l, shape))
                 shape = l._plan((1, *shape)).y_shape
                 if shape is None:
                     return None
                 shape = shape[1:]
-            elif type(l) is Pooling:
+                n = math.prod(shape)
+            elif kind is Pooling:
                 if len(shape) != 3:
                     return None
-                shape = tuple((n - f) // s + 1 for n, f, s in zip(shape, l.filter_size, l.strides)) + (shape[2],)
-            elif type(l) is Flatten:
-                shape = (math.prod(shape),)
-            elif type(l) is Layer_Dense:
-                shape = (l.weights.shape[1],)
-            total += 4 * math.prod(shape)
-        return total if total > 0 else None
+                shape = tuple((m - f) // s + 1 for m, f, s in zip(shape, l.filter_size, l.strides)) + (shape[2],)
+                n = math.prod(shape)
+            elif kind is Flatten:
+                shape = (n,)
+            elif kind is Layer_Dense:
+                working.append((l, ()))
+                n = l.weights.shape[1]
+                shape = (n,)
+            total += 4 * n
+        return (total, working) if total > 0 else None
+
+    def _pass_samples(self, X, batch_size, most):
+        """Samples of a pass: whole batches, `most` at most, whose arrays stay within INFERENCE_PASS_BYTES (one batch always)."""
+        found = self._output_bytes(tuple(X.shape[1:]))
+        if found is None:
+            return batch_size
+        per_sample, working = found
+        limit = self.INFERENCE_PASS_BYTES
+        n = min(most, max(1, limit // (per_sample * batch_size)) * batch_size)
+        while n > batch_size:
+            need = n * per_sample + sum(l._plan((n, *shape) if shape else n).ws_bytes for l, shape in working)
+            if need <= limit:
+                break
+            n = max(1, min(n // batch_size - 1, n * limit // need // batch_size)) * batch_size
+        return n
+
+    def _restore_workspaces(self, held, all_of_them=False):
+        """The layers' workspaces are again those of ``held``.  A layer that had none keeps its first one, which the next call
+        of a program that only infers needs again; ``all_of_them``: it gives that up, too."""
+        for l, w, buf, size in held:
+            if w.buf is not buf and (buf is not None or all_of_them):
+                w.buf, w.size = buf, size
+                if isinstance(l, _TakesCopies):
+                    l._forget_copies()
 
     def _own_forward(self):
         """False where a subclass or a patched method runs the passes: it gets the batches and the arguments it knows."""
         return type(self).forward is Model.forward and "forward" not in vars(self)
 
-    def _inference(self, X, batch_size):
+    def _inference(self, X, batch_size, held=()):
         """Slices and outputs of the forward passes over X: whole batches, several at once where they are small, then the
         last batch by itself, whose inputs and outputs the layers keep.  The weights stay as they are between the passes of
-        one call, so from the second on the tensor-core layers use the operand copies of them that the first one made."""
-        passes = _batches(len(X), batch_size)
+        one call, so from the second on the tensor-core layers use the operand copies of them that the first one made.
+        ``held``: the workspaces to go back to where several batches at once find no memory."""
+        batches = passes = _batches(len(X), batch_size)
         own = self._own_forward()
-        if own and len(passes) > 2 and hasattr(X, "shape"):
-            per_sample = self._output_bytes(tuple(X.shape[1:]))
-            if per_sample is not None:
-                step = batch_size * max(1, self.INFERENCE_PASS_BYTES // (per_sample * batch_size))
-                head = (len(passes) - 1) * batch_size
-                passes = [slice(k, min(k + step, head)) for k in range(0, head, step)] + passes[-1:]
+        if own and len(batches) > 2 and hasattr(X, "shape"):
+            head = (len(batches) - 1) * batch_size
+            step = self._pass_samples(X, batch_size, head)
+            passes = [slice(k, min(k + step, head)) for k in range(0, head, step)] + batches[-1:]
         fixed = [l for l in self.layers if hasattr(l, "_weights_fixed")]
-        for k, sl in enumerate(passes):
+        k, copied = 0, False
+        while k < len(passes):
+            sl, done = passes[k], False
             # (set for the pass only: a caller that leaves its loop by an exception does not resume this one, and may train next)
             try:
-                if k > 0:
+                if copied:
                     for l in fixed:
                         l._weights_fixed = True
                 output = self.forward(X[sl], training=False, **({"keep": k == len(passes) - 1} if own else {}))
+                done = True
+            except torch.OutOfMemoryError:
+                if len(passes) == len(batches):
+                    raise
             finally:
                 for l in fixed:
                     l._weights_fixed = False
+            if not done:                            # one by one then, without what this pass has left in memory
+                output = None
+                self._restore_workspaces(held, all_of_them=True)
+                for l in [self.input_layer] + self.layers:
+                    l.inputs = l.output = None
+                k, passes, copied = sl.start // batch_size, batches, False
+                continue
             yield sl, output
+            k, copied = k + 1, True
 
     def evaluate(self, X_val, y_val, *, batch_size=None):
         self.loss.new_pass()
         self.accuracy.new_pass()
-        for sl, outputs in self._inference(X_val, batch_size):
-            y_pass = y_val[sl]
-            for part in _batches(len(outputs), batch_size):
-                self.loss.calculate(outputs[part], y_pass[part], training=False)
-                self.accuracy.calculate(self.output_layer_activation.predictions(outputs[part]), y_pass[part])
+        held = self._workspaces()
+        try:
+            for sl, outputs in self._inference(X_val, batch_size, held):
+                y_pass = y_val[sl]
+                for part in _batches(len(outputs), batch_size):
+                    self.loss.calculate(outputs[part], y_pass[part], training=False)
+                    self.accuracy.calculate(self.output_layer_activation.predictions(outputs[part]), y_pass[part])
+        finally:
+            self._restore_workspaces(held)
         validation_loss = self.loss.calculate_accumulated()
         validation_accuracy = self.accuracy.calculate_accumulated()
         print(f'Valdiation, acc: {float(validation_accuracy):.3f}, loss: {float(validation_loss):.3f}')
@@ -963,7 +1015,11 @@ class Model:
     def predict(self, X, *, batch_size=None):
         # (SoftMax writes a new array every time; an output layer or a forward pass of the caller's may not)
         new = type(self.layers[-1]) is SoftMax and "forward" not in vars(self.layers[-1]) and self._own_forward()
-        outs = [output if new else output.clone() for _, output in self._inference(X, batch_size)]
+        held = self._workspaces()
+        try:
+            outs = [output if new else output.clone() for _, output in self._inference(X, batch_size, held)]
+        finally:
+            self._restore_workspaces(held)
         return torch.vstack(outs)
 
     # ------------------------------------------------------------------ parameters

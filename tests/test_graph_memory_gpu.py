@@ -38,9 +38,10 @@ def test_replay_after_a_larger_batch():
     X, y = torch.as_tensor(rng.random((16, 12, 12, 3)).astype(np.float32)).cuda(), torch.as_tensor(rng.integers(0, 10, 16)).cuda()
     larger = torch.as_tensor(rng.random((300, 12, 12, 3)).astype(np.float32)).cuda()
     alone, m = captured(X, y), captured(X, y)
-    held = [(weakref.ref(w.buf), w.buf.data_ptr(), w.buf.numel()) for w in m._workspaces() if w.buf is not None]
+    spaces = [w for _, w, buf, _ in m._workspaces() if buf is not None]
+    held = [(weakref.ref(w.buf), w.buf.data_ptr(), w.buf.numel()) for w in spaces]
     m.forward(larger, training=False)
-    replaced = [(p, n) for (_, p, n), w in zip(held, [w for w in m._workspaces() if w.buf is not None]) if w.buf.data_ptr() != p]
+    replaced = [(p, n) for (_, p, n), w in zip(held, spaces) if w.buf.data_ptr() != p]
     assert replaced and all(ref() is not None for ref, _, _ in held)
     others = [torch.full((n,), 0x5A, dtype=torch.uint8, device="cuda") for _, n in replaced for _ in range(3)]
     for _ in range(3):

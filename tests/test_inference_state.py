@@ -67,3 +67,56 @@ def test_a_forward_that_reuses_its_output():
     m.forward = lambda X, training: buffer.copy_(torch.as_tensor(X))
     X = np.arange(18.0).reshape(6, 3)
     assert np.array_equal(m.predict(X, batch_size=2).numpy(), X)
+
+
+@pytest.mark.parametrize("room", [8, 6, 5, 2])
+def test_several_batches_without_the_memory(monkeypatch, room):
+    """A pass over several batches that runs out of memory is done batch by batch, from memory that the pass does not hold."""
+    import torch
+    from aether_ml_b200.layers import _Workspace
+    from aether_ml_b200.model import Model
+    seen = []
+
+    def forward(self, X, training, keep=True):
+        seen.append((len(X), self.layers[0]._weights_fixed, keep))
+        self.layers[0].output = X
+        self.layers[0]._ws.buf, self.layers[0]._ws.size = object(), len(X)
+        if len(X) > room:
+            raise torch.OutOfMemoryError("no room")
+        return X
+    monkeypatch.setattr(Model, "forward", forward)
+    monkeypatch.setattr(Model, "_pass_samples", lambda self, X, batch, most: 6)
+    m = Model()
+    m.layers = [Layer()]
+    m.input_layer = Layer()
+    ws = m.layers[0]._ws = _Workspace()
+    buf = ws.buf = object()
+    X = np.arange(21.0).reshape(21, 1)
+    outs = []
+    held = m._workspaces()
+    for sl, out in m._inference(X, 2, held):
+        assert np.array_equal(out, X[sl])
+        outs.append(out)
+    m._restore_workspaces(held)
+    assert np.array_equal(np.vstack(outs), X) and ws.buf is buf
+    assert not m.layers[0]._weights_fixed
+    if room >= 6:
+        assert [n for n, _, _ in seen] == [6, 6, 6, 2, 1] and [f for _, f, _ in seen] == [False] + [True] * 4
+    else:
+        assert [n for n, _, _ in seen] == [6] + [2] * 10 + [1] and [f for _, f, _ in seen] == [False, False] + [True] * 10
+    assert [k for _, _, k in seen] == [False] * (len(seen) - 1) + [True]
+
+
+def test_one_batch_without_the_memory(monkeypatch):
+    """The caller's own batch size not fitting is the caller's to know."""
+    import torch
+    from aether_ml_b200.model import Model
+
+    def forward(self, X, training, keep=True):
+        raise torch.OutOfMemoryError("no room")
+    monkeypatch.setattr(Model, "forward", forward)
+    monkeypatch.setattr(Model, "_pass_samples", lambda self, X, batch, most: batch)
+    m = Model()
+    m.layers = [Layer()]
+    with pytest.raises(torch.OutOfMemoryError):
+        list(m._inference(np.zeros((9, 1)), 2))
