@@ -261,9 +261,17 @@ PyObject* py_bind(PyObject*, PyObject* args) {
 }
 
 // ---------------------------------------------------------------------------------- arrays
+// Every function below translates what torch may throw (a tensor of inference mode has no version counter, a sparse one no
+// contiguity, a wrapped one no address): an exception that left a C callback would end the process.  The ones that every
+// layer calls several times set the translation up only where something is thrown.
+PyObject* translated() {                          // (from a catch block)
+    HANDLE_TH_ERRORS
+    throw;
+    END_HANDLE_TH_ERRORS
+}
+
 // The argument itself when it is a contiguous fp32 CUDA tensor, else None.
-PyObject* py_ready(PyObject*, PyObject* o) {
-    HANDLE_TH_ERRORS                              // (a sparse tensor has no contiguity to ask for)
+PyObject* py_ready(PyObject*, PyObject* o) try {
     if (THPVariable_Check(o)) {
         const at::Tensor& t = THPVariable_Unpack(o);
         if (t.is_cuda() && t.scalar_type() == at::kFloat && t.is_contiguous()) {
@@ -272,7 +280,8 @@ PyObject* py_ready(PyObject*, PyObject* o) {
         }
     }
     Py_RETURN_NONE;
-    END_HANDLE_TH_ERRORS
+} catch (...) {
+    return translated();
 }
 
 PyObject* py_device(PyObject*, PyObject*) {
@@ -287,8 +296,6 @@ PyObject* new_array(at::IntArrayRef sizes, at::ScalarType type) {
     END_HANDLE_TH_ERRORS
 }
 
-// Every function below runs inside HANDLE_TH_ERRORS where torch may throw (a tensor of inference mode has no version counter, a
-// wrapped tensor no address): an exception that left a C callback would end the process.
 template <at::ScalarType TYPE>
 PyObject* py_empty(PyObject*, PyObject* shape) {
     if (!PyTuple_Check(shape) || PyTuple_GET_SIZE(shape) > 8) {
@@ -343,8 +350,7 @@ PyObject* py_upload(PyObject*, PyObject* const* args, Py_ssize_t n) {
 }
 
 // Identity of an array's contents as far as the host can tell: address, elements, in-place changes so far, row length.
-PyObject* py_tag(PyObject*, PyObject* o) {
-    HANDLE_TH_ERRORS
+PyObject* py_tag(PyObject*, PyObject* o) try {
     if (!THPVariable_Check(o)) {
         PyErr_SetString(PyExc_TypeError, "expected a tensor");
         return nullptr;
@@ -352,12 +358,12 @@ PyObject* py_tag(PyObject*, PyObject* o) {
     const at::Tensor& t = THPVariable_Unpack(o);
     return Py_BuildValue("(nLLL)", (Py_ssize_t) reinterpret_cast<intptr_t>(t.const_data_ptr()), (long long)t.numel(),
                          (long long)t._version(), (long long)(t.dim() > 0 ? t.size(-1) : 1));
-    END_HANDLE_TH_ERRORS
+} catch (...) {
+    return translated();
 }
 
 // same(tensor, tag): whether tag(tensor) starts with the values of `tag`, without building a tuple to compare.
-PyObject* py_same(PyObject*, PyObject* const* args, Py_ssize_t n) {
-    HANDLE_TH_ERRORS
+PyObject* py_same(PyObject*, PyObject* const* args, Py_ssize_t n) try {
     if (n != 2 || !THPVariable_Check(args[0]) || !PyTuple_Check(args[1]) || PyTuple_GET_SIZE(args[1]) > 4) {
         PyErr_SetString(PyExc_TypeError, "expected a tensor and a tag");
         return nullptr;
@@ -371,7 +377,8 @@ PyObject* py_same(PyObject*, PyObject* const* args, Py_ssize_t n) {
         if (v != now[i]) Py_RETURN_FALSE;
     }
     Py_RETURN_TRUE;
-    END_HANDLE_TH_ERRORS
+} catch (...) {
+    return translated();
 }
 
 #define METHOD(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_##name)), METH_FASTCALL, nullptr},
