@@ -83,6 +83,19 @@ def _batches(n, batch_size):
     return [slice(k * batch_size, (k + 1) * batch_size) for k in range(steps)]
 
 
+def _links(parts):
+    """How layers that follow each other are wired: (layer, attribute, the weak reference it holds), one reference object for
+    all that refer to the same layer."""
+    return [(p, name, p.__dict__.get(name)) for name, some in (("_link_prev", parts[1:]), ("_link_next", parts[:-1])) for p in some]
+
+
+def _as_wired(links):
+    for part, name, ref in links:
+        if part.__dict__.get(name) is not ref:
+            return False
+    return True
+
+
 class _Chain:
     """A Batch_Norm and the layers right behind it -- (Leaky_)ReLU, optional Layer_Dropout_Spatial, optional max Pooling whose
     stride is its window -- that a model with unfused layers runs in one pass each way (aether_chain_fwd / _bwd): every
@@ -92,6 +105,7 @@ class _Chain:
 
     def __init__(self, parts, conv, consumer):
         self.parts = parts                      # [bn, act[, drop][, pool]]
+        self.links = _links(parts)
         self.length = len(parts)
         self.bn, self.act = parts[0], parts[1]
         self.drop = next((l for l in parts if isinstance(l, Layer_Dropout_Spatial)), None)
@@ -124,7 +138,7 @@ class _Chain:
         return _Chain(parts, conv, behind if hasattr(behind, "x_copy_target") else None)
 
     def _intact(self, layers, i):
-        if layers[i:i + self.length] != self.parts:
+        if layers[i:i + self.length] != self.parts or not _as_wired(self.links):
             return False
         for part in self.parts:
             d = part.__dict__
@@ -249,6 +263,7 @@ class _DenseAct:
 
     def __init__(self, dense, act, behind):
         self.parts = [dense, act]
+        self.links = _links(self.parts)
         self.dense, self.act = dense, act
         self.consumer = behind if type(behind) is Layer_Dense else None
 
@@ -259,7 +274,7 @@ class _DenseAct:
         return None
 
     def _intact(self, layers, i):
-        if layers[i:i + 2] != self.parts or self.act.fused_into_prev:
+        if layers[i:i + 2] != self.parts or self.act.fused_into_prev or not _as_wired(self.links):
             return False
         for part in self.parts:
             d = part.__dict__
@@ -303,6 +318,7 @@ class _Head:
 
     def __init__(self, dense, softmax):
         self.parts = [dense, softmax]
+        self.links = _links(self.parts)
         self.dense, self.softmax = dense, softmax
 
     @staticmethod
@@ -310,7 +326,7 @@ class _Head:
         return _Head(layers[i], layers[i + 1]) if len(layers) == i + 2 and type(layers[i]) is Layer_Dense and type(layers[i + 1]) is SoftMax else None
 
     def _intact(self, layers, i):
-        if layers[i:] != self.parts:
+        if layers[i:] != self.parts or not _as_wired(self.links):
             return False
         for part in self.parts:
             d = part.__dict__
@@ -542,16 +558,15 @@ class Model:
         """``keep=False`` (inference passes whose layers' attributes the next pass replaces): a chain of layers run in one
         pass writes its last output only."""
         self.input_layer.forward(X, training)
-        layers, chains, i, prev = self.layers, self._chains, 0, self.input_layer
+        layers, chains, i = self.layers, self._chains, 0
         while i < len(layers):
             layer = layers[i]
+            inputs = layer.prev.output              # (of the layer in front, unless the caller has wired it otherwise)
             chain = chains.get(i)
-            if chain is not None and chain.forward(layers, i, prev.output, training, keep):
+            if chain is not None and chain.forward(layers, i, inputs, training, keep):
                 i += chain.length
-                prev = layers[i - 1]
                 continue
-            layer.forward(prev.output, training)
-            prev = layer
+            layer.forward(inputs, training)
             i += 1
         return layers[-1].output
 
