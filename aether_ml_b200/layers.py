@@ -48,9 +48,10 @@ def to_device(a, dtype=torch.float32):
 
 
 class _Neighbour:
-    """An attribute that refers to another layer without keeping it alive.  The layer list of a model owns its layers;
-    with owning links between neighbours a dropped model, its workspaces and its activations stayed in device memory
-    until Python's cycle collector happened to run, and the next model paid for fresh allocations."""
+    """An attribute that refers to another layer: owned when it is assigned, like any attribute, and not when a model links its
+    layers (`_link`).  The layer list of a model owns its layers; with owning links between neighbours a dropped model, its
+    workspaces and its activations stayed in device memory until Python's cycle collector happened to run, and the next
+    model paid for fresh allocations."""
 
     def __set_name__(self, owner, name):
         self.name, self.slot = name, "_link_" + name
@@ -59,16 +60,24 @@ class _Neighbour:
         if obj is None:
             return self
         try:
-            ref = obj.__dict__[self.slot]
+            held = obj.__dict__[self.slot]
         except KeyError:
             raise AttributeError(self.name) from None
-        return ref() if ref is not None else None
+        return held() if type(held) is weakref.ref else held
 
     def __set__(self, obj, value):
+        obj.__dict__[self.slot] = value
+
+
+def _link(layer, name, other):
+    """Sets ``layer.name`` to another layer of the same model without owning it."""
+    if isinstance(getattr(type(layer), name, None), _Neighbour):
         try:
-            obj.__dict__[self.slot] = weakref.ref(value) if value is not None else None
+            layer.__dict__["_link_" + name] = weakref.ref(other) if other is not None else None
+            return
         except TypeError:                       # an object that takes no weak references (a caller's own class)
-            obj.__dict__[self.slot] = lambda: value
+            pass
+    setattr(layer, name, other)
 
 
 class _Saved:

@@ -20,7 +20,7 @@ import torch
 from ._lib import host
 from .layers import (Activation_Softmax_Loss_CategoricalCrossEntropy, Batch_Norm, Conv_Layer, Flatten, Layer_Dense, Layer_Dropout,
                      Layer_Dropout_Spatial, Leaky_ReLU, Loss_CategoricalCrossEntropy, Optimizer_Adam, Pooling, ReLU, SoftMax, to_device, _labels,
-                     _labels_i32, _softmax_cce, _Saved, _TakesCopies, _Workspace)
+                     _labels_i32, _link, _softmax_cce, _Saved, _TakesCopies, _Workspace)
 
 
 class Layer_Input:
@@ -452,8 +452,8 @@ class Model:
         self.input_layer = Layer_Input()
         chain = [self.input_layer] + self.layers + [self.loss]
         for pos, layer in enumerate(self.layers, start=1):
-            layer.prev = chain[pos - 1]
-            layer.next = chain[pos + 1]
+            _link(layer, "prev", chain[pos - 1])
+            _link(layer, "next", chain[pos + 1])
         self.output_layer_activation = self.layers[-1]
         if isinstance(self.layers[0], Conv_Layer):
             self.layers[0].first_in_model = True        # backward never asks it for dinputs
@@ -482,7 +482,7 @@ class Model:
                 if (isinstance(c, Pooling) and c.pooling_type == "max" and c.padding == "valid"
                         and tuple(c.strides) == tuple(c.filter_size)):
                     a.fused_pool = c
-                    c.fused_bn = a
+                    _link(c, "fused_bn", a)
                     # The pooled tensor is the x of the layer behind (through a Flatten, if any) and the dx of this
                     # block tail is the dvalues of the convolution in front: the tail's kernels write the bf16 copies
                     # those layers' tensor-core kernels read, so neither runs a cast pass over the fp32 tensor.
