@@ -213,7 +213,7 @@ class _Chain:
         if pool is not None:
             pool.inputs, pool.output, pool._argmax = (act_out if drop is None else drop_out), pooled, arg
         if training:
-            self.live = (x, bn_out, bn_out._version, ws, mask, S, H, W, Cc, fH, fW, alpha)
+            self.live = (x, x._version, bn_out, bn_out._version, ws, mask, S, H, W, Cc, fH, fW, alpha)
         return True
 
     def backward(self, layers, i, dvalues):
@@ -222,8 +222,8 @@ class _Chain:
         bn, act, drop, pool = self.bn, self.act, self.drop, self.pool
         if live is None or not self._intact(layers, i):
             return False
-        x, bn_out, version, ws, mask, S, H, W, Cc, fH, fW, alpha = live
-        if (bn.inputs is not x or act.inputs is not bn_out or bn_out._version != version or bn._ws.buf is not ws or act._alpha != alpha
+        x, x_version, bn_out, version, ws, mask, S, H, W, Cc, fH, fW, alpha = live
+        if (bn.inputs is not x or act.inputs is not bn_out or bn_out._version != version or x._version != x_version or bn._ws.buf is not ws or act._alpha != alpha
                 or (drop is not None and drop.channel_mask is not mask)):
             return False
         dy = to_device(dvalues)
