@@ -560,7 +560,7 @@ extern "C" int aether_bn_act_pool_fwd_copy(const float* x, const float* partials
     if (ws_bytes < aether_bn_workspace_bytes(rows, C)) return set_error(AE_BAD_ARG, "aether_bn_act_pool_fwd: workspace too small");
     if (partials && (nblocks <= 0 || nblocks > (1 << 30))) return set_error(AE_BAD_ARG, "aether_bn_act_pool_fwd: nblocks");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (training && bn_small(rows * C, C)) {
+    if (training && bn_small(rows, C)) {
         BnSmallFwd p = {};
         p.x = x;
         p.part = partials;
@@ -629,7 +629,7 @@ extern "C" int aether_bn_act_pool_bwd_copy(const float* x, const float* dpooled,
     if (ws_bytes < aether_bn_workspace_bytes(rows, C)) return set_error(AE_BAD_ARG, "aether_bn_act_pool_bwd: workspace too small");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const long long windows = windows4 / (C / 4);
-    const bool small = bn_small(rows * C, C);
+    const bool small = bn_small(rows, C);
     int nb = bn_partial_blocks(rows);
     if (nb > windows) nb = (int)windows;
     if (small && nb > 148) nb = 148;
@@ -697,7 +697,7 @@ extern "C" int aether_chain_fwd(const float* x, const float* partials, int64_t n
     if (ws_bytes < aether_bn_workspace_bytes(rows, C)) return set_error(AE_BAD_ARG, "aether_chain_fwd: workspace too small");
     if (partials && (nblocks <= 0 || nblocks > (1 << 30))) return set_error(AE_BAD_ARG, "aether_chain_fwd: nblocks");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (training && bn_small(rows * C, C)) {
+    if (training && bn_small(rows, C, BN_SMALL_CHAIN)) {
         BnSmallFwd p = {};
         p.x = x;
         p.part = partials;
@@ -758,7 +758,7 @@ extern "C" int aether_chain_bwd(const float* x, const float* dy, const uint8_t* 
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     float* part = static_cast<float*>(ws);
     float* coeff = part + (size_t)bn_partial_blocks(rows) * 3 * C;        // still the forward pass's scale and shift
-    const bool small = bn_small(rows * C, C);
+    const bool small = bn_small(rows, C, BN_SMALL_CHAIN);
     int nb = bn_partial_blocks(rows);
     if (nb > windows) nb = (int)windows;
     if (small && nb > 148 * 2) nb = 148 * 2;

@@ -7,7 +7,7 @@
 // CTA, 296: 114 KB out of L2 per CTA, which is why there is one per SM and not two; double precision, fixed order -- the same
 // bits in every CTA), and the coefficients go straight from shared memory into its pass.  The first chunk's CTA writes the
 // statistics.  (Clusters of four CTAs that share the merge through distributed shared memory start later than they save.)
-// Only below BN_SMALL_ELEMENTS: a large tensor is a stream of HBM traffic, for which the CTAs' 128-byte pieces and the
+// Only below BN_SMALL (tail.cuh): a large tensor is a stream of HBM traffic, for which the CTAs' 128-byte pieces and the
 // repeated merge cost more than the 7 us they save.
 #include <cuda_bf16.h>
 
@@ -290,7 +290,7 @@ static int small_chunks(int C, unsigned windows, int most) {
     return chunks < 1 ? 1 : chunks;
 }
 
-bool bn_small(long long elements, int C) { return C % 4 == 0 && elements <= BN_SMALL_ELEMENTS; }
+bool bn_small(long long rows, int C, long long most) { return C % 4 == 0 && rows * (ceil_div(C, 32) * 32LL) <= most; }
 
 void bn_small_forward(const BnSmallFwd& p, cudaStream_t st) {
     const int grid = small_chunks(p.C, p.windows, 0) * ceil_div(p.C, 32);

@@ -685,7 +685,7 @@ extern "C" int aether_bn_fwd_train(const float* x, const float* gamma, const flo
     if (ws_bytes < aether_bn_workspace_bytes(rows, C)) return set_error(AE_BAD_ARG, "aether_bn_fwd_train: workspace too small");
     if ((C & 3) == 0 && (!aligned16(x) || !aligned16(y))) return set_error(AE_BAD_ARG, "aether_bn_fwd_train: arrays must be 16-byte aligned");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (bn_small(rows * C, C)) {
+    if (bn_small(rows, C)) {
         bn_small_rows(x, nullptr, 0, gamma, beta, running_mean, running_var, batch_mean, batch_var, y, rows, C, eps, momentum, -1.f, nullptr,
                       static_cast<float*>(ws), st);
         return check_launch("aether_bn_fwd_train");
@@ -716,7 +716,7 @@ extern "C" int aether_bn_fwd_train_partials(const float* x, const float* partial
         return set_error(AE_BAD_ARG, "aether_bn_fwd_train_partials: workspace too small or misaligned (needs 2*C floats)");
     if ((C & 3) == 0 && (!aligned16(x) || !aligned16(y))) return set_error(AE_BAD_ARG, "aether_bn_fwd_train_partials: arrays must be 16-byte aligned");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (bn_small(rows * C, C)) {
+    if (bn_small(rows, C)) {
         bn_small_rows(x, partials, nblocks, gamma, beta, running_mean, running_var, batch_mean, batch_var, y, rows, C, eps, momentum, -1.f,
                       nullptr, nullptr, st);
         return check_launch("aether_bn_fwd_train_partials");
@@ -817,7 +817,7 @@ extern "C" int aether_bn_bwd(const float* x, const float* dy, const float* gamma
     if ((C & 3) == 0 && (!aligned16(x) || !aligned16(dy) || !aligned16(dx)))
         return set_error(AE_BAD_ARG, "aether_bn_bwd: arrays must be 16-byte aligned");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (bn_small(rows * C, C)) {
+    if (bn_small(rows, C)) {
         bn_small_rows_bwd(x, dy, gamma, nullptr, batch_mean, batch_var, nullptr, dx, dgamma, dbeta, rows, C, eps, -1.f, static_cast<float*>(ws), st);
         return check_launch("aether_bn_bwd");
     }
@@ -856,7 +856,7 @@ extern "C" int aether_bn_act_fwd_train(const float* x, const float* partials, in
     if (ws_bytes < aether_bn_workspace_bytes(rows, C)) return set_error(AE_BAD_ARG, "aether_bn_act_fwd_train: workspace too small");
     if (partials && (nblocks <= 0 || nblocks > (1 << 30))) return set_error(AE_BAD_ARG, "aether_bn_act_fwd_train: nblocks");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (bn_small(rows * C, C)) {
+    if (bn_small(rows, C)) {
         bn_small_rows(x, partials, nblocks, gamma, beta, running_mean, running_var, batch_mean, batch_var, y, rows, C, eps, momentum, alpha,
                       channel_scale, static_cast<float*>(ws), st);
         return check_launch("aether_bn_act_fwd_train");
@@ -914,7 +914,7 @@ extern "C" int aether_bn_act_bwd(const float* x, const float* beta, const float*
     if (rc) return rc;
     if (ws_bytes < aether_bn_workspace_bytes(rows, C)) return set_error(AE_BAD_ARG, "aether_bn_act_bwd: workspace too small");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (bn_small(rows * C, C) && aligned16(gamma) && aligned16(beta) && aligned16(batch_mean) && aligned16(batch_var)) {
+    if (bn_small(rows, C) && aligned16(gamma) && aligned16(beta) && aligned16(batch_mean) && aligned16(batch_var)) {
         bn_small_rows_bwd(x, dy, gamma, beta, batch_mean, batch_var, channel_scale, dx, dgamma, dbeta, rows, C, eps, alpha,
                           static_cast<float*>(ws), st);
         return check_launch("aether_bn_act_bwd");

@@ -21,8 +21,14 @@ __device__ __forceinline__ float lrelu(float v, float alpha) { return v > 0.f ? 
 // derivative of the activation at pre-activation v (the reference passes the gradient at v == 0, :412-428)
 __device__ __forceinline__ float lrelu_grad(float v, float alpha) { return v < 0.f ? alpha : 1.f; }
 
-// ---- bn_small.cu: one-pass forms for tensors up to this many elements (32 MB: with what the passes write they stay in L2)
-static constexpr long long BN_SMALL_ELEMENTS = 8LL << 20;
+// ---- bn_small.cu: one-pass forms for small tensors.  A CTA works on 32 channels, so what counts is the rows times the channels
+// filled up to whole blocks of 32.  Measured on B200, one-pass against three-launch form in us, forward + backward:
+//   Batch_Norm alone, with the activation or with pooling: 1M x 4 (32M filled) 59 + 36 / 27 + 17, 128K x 8 (4M) 18 + 10 / 18 + 10,
+//     512K x 8 (16M) 34 + 23 / 21 + 16, 128K x 16 (4M) 16 + 11 / 15 + 12, 128K x 32 (4M) 15 + 13 / 16 + 16, 192K x 32 (6M) 19 + 23 /
+//     18 + 20, 32K x 256 (8M) 26 + 31 / 23 + 29;
+//   every layer's output kept (the pass writes four times as much): 128K x 32 (4M) 18 + 22 / 19 + 25, 192K x 32 (6M) 26 + 33 / 25 + 35,
+//     256K x 32 (8M) 36 + 43 / 31 + 46, 256K x 8 (8M) 24 + 21 / 19 + 21.
+static constexpr long long BN_SMALL = 4LL << 20, BN_SMALL_CHAIN = 7LL << 20;
 
 struct BnSmallFwd {
     const float* x;
@@ -56,7 +62,7 @@ struct BnSmallBwd {
     unsigned windows;
     long long rows;
 };
-bool bn_small(long long elements, int C);
+bool bn_small(long long rows, int C, long long most = BN_SMALL);
 void bn_small_forward(const BnSmallFwd& p, cudaStream_t st);
 // Returns the rows of column sums written (at most rows_max, when that is positive).
 int bn_small_backward(const BnSmallBwd& p, int rows_max, cudaStream_t st);

@@ -1,6 +1,6 @@
 """Batch_Norm's reductions at their edges: fewer rows than CTAs, than row lanes and than loads in flight, channel counts
-that fill no warp, that end inside a round of 1024 channels, and the boundary between the merged and the three-launch
-form (8M elements).  Relative L2 <= 1e-5 against float64; the statistics of values far from zero keep the digits that the
+that fill no warp, that end inside a round of 1024 channels, and tensors of eight million elements (the line between the
+merged and the three-launch form is in test_bn_small_line_gpu.py).  Relative L2 <= 1e-5 against float64; the statistics of values far from zero keep the digits that the
 values have (mean 100, deviation 1: the variance loses log2(100) bits, 1e-4)."""
 import pytest
 
