@@ -403,7 +403,7 @@ static int dx_fewc(const AetherConvDesc& d, const float* dy, const float* w, flo
 int generic_conv_bwd_data(const AetherConvDesc& d, const float* dy, const float* w, float* dx, void* ws, size_t ws_bytes, cudaStream_t st) {
     int Ho, Wo;
     conv_out_hw(d, Ho, Wo);
-    // (Few input channels leave a GEMM tile's columns empty.  More than 65535 pixel classes do not fit a grid.)
+    // (Few input channels leave a GEMM tile's columns empty.  More than 65535 pixel classes do not fit one grid.)
     if (d.Cin <= 4 && 1LL * d.sH * d.sW <= 65535) {
         switch (d.Cin) {
             case 1: return dx_fewc<1>(d, dy, w, dx, Ho, Wo, st);

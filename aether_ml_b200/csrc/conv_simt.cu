@@ -51,6 +51,7 @@ struct SimtGemm {
     float* part;
     long long row0, part_rows;
     int full, parts;
+    int class0;           // pixel class of blockIdx.z = 0
 };
 
 // One side of a tile: BR rows x SIMT_BK reduction steps, four consecutive steps per load.
@@ -150,8 +151,9 @@ simt_conv_kernel(const SimtGemm g, int n_tiles_n) {
     // pixel class (dX of a strided layer): rows h = hs + a * sH, taps i = ph + sH * ti
     int ph = 0, pw = 0, nH = g.fH, nW = g.fW, hs = 0, ws = 0, hq = 0, wq = 0, MH = g.OH, MW = g.OW;
     if (DX) {
-        ph = blockIdx.z / g.sW;
-        pw = blockIdx.z - ph * g.sW;
+        const int cls = g.class0 + (int)blockIdx.z;
+        ph = cls / g.sW;
+        pw = cls - ph * g.sW;
         nH = ph < g.fH ? (g.fH - ph - 1) / g.sH + 1 : 0;
         nW = pw < g.fW ? (g.fW - pw - 1) / g.sW + 1 : 0;
         hs = ((ph - g.pH) % g.sH + g.sH) % g.sH;
@@ -324,7 +326,7 @@ simt_conv_kernel(const SimtGemm g, int n_tiles_n) {
     const bool vec_out = (g.N & 3) == 0;
     const bool split = SPLIT && pieces > 1;
     const float* bias = DX || split ? nullptr : g.bias;
-    float* const out = split ? g.part + ((size_t)(blockIdx.z * pieces + piece) * g.part_rows) * g.N : g.out;
+    float* const out = split ? g.part + (((size_t)g.class0 + blockIdx.z) * pieces + piece) * g.part_rows * g.N : g.out;
 #pragma unroll
     for (int qm = 0; qm < QM; ++qm)
 #pragma unroll
@@ -362,7 +364,7 @@ __global__ void __launch_bounds__(256) simt_finish_kernel(const SimtGemm g) {
     pdl_wait();
     int hs = 0, ws = 0, MH = g.OH, MW = g.OW;
     if (DX) {
-        const int ph = blockIdx.z / g.sW, pw = blockIdx.z - ph * g.sW;
+        const int cls = g.class0 + (int)blockIdx.z, ph = cls / g.sW, pw = cls - ph * g.sW;
         hs = ((ph - g.pH) % g.sH + g.sH) % g.sH;
         ws = ((pw - g.pW) % g.sW + g.sW) % g.sW;
         MH = hs < g.OH ? (g.OH - hs - 1) / g.sH + 1 : 0;
@@ -375,7 +377,7 @@ __global__ void __launch_bounds__(256) simt_finish_kernel(const SimtGemm g) {
     if (row >= g.part_rows || m >= M) return;
     const int n = (int)(i - row * NV) * V;
     const size_t step = (size_t)g.part_rows * g.N;
-    const float* p = g.part + (size_t)blockIdx.z * g.parts * step + (size_t)row * g.N + n;
+    const float* p = g.part + ((size_t)g.class0 + blockIdx.z) * g.parts * step + (size_t)row * g.N + n;
     float s[V];
 #pragma unroll
     for (int e = 0; e < V; ++e) s[e] = 0.f;
@@ -647,7 +649,7 @@ static SimtPick simt_pick(const AetherConvDesc& d, size_t ws_bytes) {
     conv_out_hw(d, Ho, Wo);
     SimtPick best{};
     const int N = DX ? d.Cin : d.Cout, sms = num_sms();
-    best.classes = DX ? d.sH * d.sW : 1;
+    best.classes = DX ? (int)(1LL * d.sH * d.sW < 0x7fffffffLL ? 1LL * d.sH * d.sW : 0x7fffffffLL) : 1;
     best.M = DX ? 1LL * d.S * ceil_div(d.H, d.sH) * ceil_div(d.W, d.sW) : 1LL * d.S * Ho * Wo;    // (pixels of the largest class)
     const double steps = (double)d.fH * d.fW * (DX ? d.Cout : d.Cin) / best.classes / SIMT_BK;
     double best_us = 1e300;
@@ -696,18 +698,22 @@ static int launch_simt_conv(SimtGemm g, const SimtPick& p, bool vec, void* ws, c
     const long long ctas = (p.full_mt + (p.mt - p.full_mt) * p.parts) * ntn;
     if (ctas > 0x7fffffffLL) return set_error(AE_UNSUPPORTED, "convolution of %lld pixels and %d channels is too large", p.M, g.N);
     g.full = (int)(p.full_mt * ntn);
-    const dim3 grid((unsigned)ctas, 1, (unsigned)p.classes);
-    constexpr int THREADS = (BM / TM) * (BN / TN);
-    if (split) launch(vec ? simt_conv_kernel<BM, BN, TM, TN, DX, true, true> : simt_conv_kernel<BM, BN, TM, TN, DX, false, true>, grid, THREADS, 0, st, g, ntn);
-    else launch(vec ? simt_conv_kernel<BM, BN, TM, TN, DX, true, false> : simt_conv_kernel<BM, BN, TM, TN, DX, false, false>, grid, THREADS, 0, st, g, ntn);
-    count_launch();
-    if (int rc = check_launch("simt_conv_kernel")) return rc;
-    if (!split) return AE_OK;
+    constexpr int THREADS = (BM / TM) * (BN / TN), MOST = 65535;       // (classes a grid takes along z)
     const bool v4 = g.N % 4 == 0 && aligned16(g.out) && aligned16(g.part);
     const long long items = g.part_rows * (v4 ? g.N / 4 : g.N);
-    launch(v4 ? simt_finish_kernel<DX, 4> : simt_finish_kernel<DX, 1>, dim3((unsigned)((items + 255) / 256), 1, (unsigned)p.classes), 256, 0, st, g);
-    count_launch();
-    return check_launch("simt_finish_kernel");
+    for (g.class0 = 0; g.class0 < p.classes; g.class0 += MOST) {
+        const unsigned classes = (unsigned)(p.classes - g.class0 < MOST ? p.classes - g.class0 : MOST);
+        const dim3 grid((unsigned)ctas, 1, classes);
+        if (split) launch(vec ? simt_conv_kernel<BM, BN, TM, TN, DX, true, true> : simt_conv_kernel<BM, BN, TM, TN, DX, false, true>, grid, THREADS, 0, st, g, ntn);
+        else launch(vec ? simt_conv_kernel<BM, BN, TM, TN, DX, true, false> : simt_conv_kernel<BM, BN, TM, TN, DX, false, false>, grid, THREADS, 0, st, g, ntn);
+        count_launch();
+        if (int rc = check_launch("simt_conv_kernel")) return rc;
+        if (!split) continue;
+        launch(v4 ? simt_finish_kernel<DX, 4> : simt_finish_kernel<DX, 1>, dim3((unsigned)((items + 255) / 256), 1, classes), 256, 0, st, g);
+        count_launch();
+        if (int rc = check_launch("simt_finish_kernel")) return rc;
+    }
+    return AE_OK;
 }
 
 template <bool DX>
@@ -722,10 +728,38 @@ static int simt_conv(const SimtGemm& g, const SimtPick& p, bool vec, void* ws, c
     }
 }
 
+// The kernels count the pixels of the gathered operand from a tile's first sample in 32 bits.  How many samples may go
+// into one launch for that: all of them, unless the 128 rows of a tile meet samples 2^31 pixels apart (strides of thousands).
+static constexpr long long SIMT_MOST_PIXELS = 0x7fffffffLL;
+static int simt_samples(const AetherConvDesc& d, bool dx, int Ho, int Wo) {
+    const long long pixels = dx ? 1LL * Ho * Wo : 1LL * d.H * d.W;
+    const long long rows = dx ? 1LL * (d.H / d.sH) * (d.W / d.sW) : 1LL * Ho * Wo;         // a sample's, of the smallest class
+    const long long met = 127 / (rows > 1 ? rows : 1) + 2;
+    if (met * pixels <= SIMT_MOST_PIXELS) return d.S;
+    const long long n = SIMT_MOST_PIXELS / pixels;
+    return (int)(n < d.S ? n : d.S);
+}
+
+// `n` samples per launch: f(descriptor, elements of the samples before in its input and in its output).
+template <typename F>
+static int simt_by_samples(const AetherConvDesc& d, int n, long long in_sample, long long out_sample, F f) {
+    if (n < 1) return set_error(AE_UNSUPPORTED, "convolution of %dx%d images: more than 2^31 pixels each", d.H, d.W);
+    for (int s = 0; s < d.S; s += n) {
+        AetherConvDesc c = d;
+        c.S = d.S - s < n ? d.S - s : n;
+        if (int rc = f(c, s * in_sample, s * out_sample)) return rc;
+    }
+    return AE_OK;
+}
+
 int simt_conv_fwd(const AetherConvDesc& d, const float* x, const float* w, const float* b, float* y, void* ws, size_t ws_bytes, cudaStream_t st) {
     SimtGemm g{};
     int Ho, Wo;
     conv_out_hw(d, Ho, Wo);
+    if (const int n = simt_samples(d, false, Ho, Wo); n < d.S)
+        return simt_by_samples(d, n, 1LL * d.H * d.W * d.Cin, 1LL * Ho * Wo * d.Cout, [&](const AetherConvDesc& c, long long in, long long out) {
+            return simt_conv_fwd(c, x + in, w, b, y + out, nullptr, 0, st);
+        });
     g.in = x; g.w = w; g.bias = b; g.out = y;
     g.IH = d.H; g.IW = d.W; g.IC = d.Cin; g.N = d.Cout;
     g.fH = d.fH; g.fW = d.fW; g.sH = d.sH; g.sW = d.sW; g.pH = d.padH; g.pW = d.padW;
@@ -738,12 +772,15 @@ int simt_conv_bwd_data(const AetherConvDesc& d, const float* dy, const float* w,
     SimtGemm g{};
     int Ho, Wo;
     conv_out_hw(d, Ho, Wo);
+    if (const int n = simt_samples(d, true, Ho, Wo); n < d.S)
+        return simt_by_samples(d, n, 1LL * Ho * Wo * d.Cout, 1LL * d.H * d.W * d.Cin, [&](const AetherConvDesc& c, long long in, long long out) {
+            return simt_conv_bwd_data(c, dy + in, w, dx + out, nullptr, 0, st);
+        });
     g.in = dy; g.w = w; g.out = dx;
     g.IH = Ho; g.IW = Wo; g.IC = d.Cout; g.N = d.Cin;
     g.fH = d.fH; g.fW = d.fW; g.sH = d.sH; g.sW = d.sW; g.pH = d.padH; g.pW = d.padW;
     g.OH = d.H; g.OW = d.W; g.S = d.S; g.Cin = d.Cin; g.Cout = d.Cout;
     const bool vec = d.Cin % 4 == 0 && d.Cout % 4 == 0 && aligned16(dy) && aligned16(w) && aligned16(dx);
-    if (1LL * d.sH * d.sW > 65535) return set_error(AE_UNSUPPORTED, "stride %dx%d is too large", d.sH, d.sW);
     return simt_conv<true>(g, simt_pick<true>(d, ws ? ws_bytes : 0), vec, ws, st);
 }
 
@@ -762,6 +799,11 @@ static SimtDwPlan simt_dw_plan(const AetherConvDesc& d) {
     SimtDwPlan best{};
     const int KK = d.fH * d.fW * d.Cin;
     const long long P = 1LL * d.S * Ho * Wo;
+    // (x pixels are counted from a split's first sample in 32 bits: the samples that a split may meet, and so its length)
+    const long long met = SIMT_MOST_PIXELS / (1LL * d.H * d.W);
+    long long longest = P + SIMT_BK;
+    if (met < d.S && met > 2) longest = (met - 2) * Ho * Wo;
+    if (longest < SIMT_BK) longest = SIMT_BK;
     double best_us = 1e300;
     for (int i = 0; i < (int)(sizeof(SIMT_DW_TILES) / sizeof(SimtTile)); ++i) {
         const SimtTile& t = SIMT_DW_TILES[i];
@@ -777,6 +819,7 @@ static SimtDwPlan simt_dw_plan(const AetherConvDesc& d) {
             if (want < 1) want = 1;
             if (want > 65535) want = 65535;
             p.per_split = ((P + want - 1) / want + SIMT_BK - 1) / SIMT_BK * SIMT_BK;
+            if (p.per_split > longest) p.per_split = longest / SIMT_BK * SIMT_BK;
             p.splits = (int)((P + p.per_split - 1) / p.per_split);
             const double us = simt_rounds((tiles * p.splits + num_sms() - 1) / num_sms(), t.ctas) * SIMT_STEP_US * t.bm * t.bn / (128.0 * 64) /
                                   t.rate * ((double)(p.per_split / SIMT_BK) + 4.0) +
@@ -820,6 +863,9 @@ int simt_conv_bwd_filter(const AetherConvDesc& d, const float* x, const float* d
     g.KK = d.fH * d.fW * d.Cin;
     g.P = 1LL * d.S * g.Ho * g.Wo;
     g.per_split = p.per_split;
+    const long long met = p.per_split / (1LL * g.Ho * g.Wo) + 2;
+    if ((met < d.S ? met : d.S) * d.H * d.W > SIMT_MOST_PIXELS)
+        return set_error(AE_UNSUPPORTED, "filter gradient of %d x %dx%d images: samples too large", d.S, d.H, d.W);
     const bool vec = d.Cin % 4 == 0 && d.Cout % 4 == 0 && aligned16(x) && aligned16(dy);
     switch (p.tile) {
         case 0: launch_simt_dw<128, 128, 8, 8>(g, p, vec, st); break;
