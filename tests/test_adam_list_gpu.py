@@ -1,5 +1,5 @@
 """The update of many tensors in one call against the update of each by itself, bit for bit (the same operations per element):
-tensors that share memory, whose updates have to follow each other."""
+tensors that share memory, whose updates have to follow each other, and more tensors than one launch takes (32)."""
 import pytest
 
 pytestmark = pytest.mark.gpu
@@ -49,4 +49,14 @@ def both_ways(sizes, tie, steps=3):
 def test_shared_memory(sizes, tie):
     import torch
     a, b = both_ways(sizes, tie)
+    assert all(torch.equal(x, y) for x, y in zip(a, b))
+
+
+@pytest.mark.parametrize("count", [1, 15, 16, 17, 32, 33])                  # two tensors each
+def test_more_than_one_launch(count):
+    import torch
+    from aether_ml_b200 import _lib
+    n0 = _lib.launch_count()
+    a, b = both_ways([1 + 977 * k for k in range(count)], [], steps=1)
+    assert _lib.launch_count() - n0 == -(-2 * count // 32) + 2 * count
     assert all(torch.equal(x, y) for x, y in zip(a, b))
