@@ -312,7 +312,8 @@ __global__ void __launch_bounds__(FT_THREADS, 1) first_conv_kernel(const __grid_
                             for (int k = 0; k < 8; ++k) s8[k] = 0.f;
 #pragma unroll
                             for (int r = 0; r < 32; ++r) s8[r & 7] += r < nr ? val[r] : 0.f;
-                            base[0] = stats_tree(s8) * (1.f / (float)nr);
+                            const float mean = stats_tree(s8) * (1.f / (float)nr);
+                            base[0] = isfinite(mean) ? mean : 0.f;        // (else every value would differ from it by no number)
                             base[128] = base[256] = 0.f;
                         }
                         const float npiv = -base[0];

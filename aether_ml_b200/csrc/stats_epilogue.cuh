@@ -94,9 +94,10 @@ __device__ __forceinline__ void stats_store_rows(double N, double S, double Q, f
     out[n_out + col] = mean;
     out[2 * (size_t)n_out + col] = m2;
     out += 3 * (size_t)n_out;
+    const bool finite = isfinite(mean) && isfinite(Q);      // (an infinite sum has no rest, and its mean stays infinite)
     out[col] = 0.f;
-    out[n_out + col] = (float)(S - N * (double)mean);
-    out[2 * (size_t)n_out + col] = (float)(Q - nm2 - (double)m2);
+    out[n_out + col] = finite ? (float)(S - N * (double)mean) : 0.f;
+    out[2 * (size_t)n_out + col] = finite ? (float)(Q - nm2 - (double)m2) : 0.f;
 }
 // What a row (n, m, m2) adds to (N, S, Q).
 __device__ __forceinline__ void stats_row_terms(float n, float m, float m2, double& dn, double& ds, double& dq) {
