@@ -7,7 +7,8 @@
 //   dW       dw[k][d] = sum_p col[p][k] dy[p][d]             M = taps * Cin, N = Cout, K = output pixels, split
 //
 // Bound by the FMA pipes (74 TFLOP/s): a thread keeps an 8x8 block of sums, so that 64 FMAs share four 16-byte
-// shared-memory reads; tiles of 128 x {128, 64, 32, 16} and 16 steps of the reduction are staged through registers into
+// shared-memory reads; tiles of 64 or 128 pixels by 16 to 128 channels (SIMT_CONV_TILES, SIMT_DW_TILES) and 16 steps of the
+// reduction are staged through registers into
 // two shared-memory buffers, the next tile's global loads in flight during the FMAs of the current one.  The reduction
 // index walks (filter row, filter column, channel) by mixed-radix steps, so the loop has no division.  A stride s
 // splits the input pixels of dX into s*s classes (blockIdx.z) that each see only the taps which reach them; no tap is
@@ -417,7 +418,8 @@ struct SimtDw {
 
 // VEC: both operands go straight into shared memory (cp.async, two steps ahead): no staging registers and no stores between the
 // FMAs (64 x 32x32 96->96 with the 64 x 64 tile 403 -> 311 us, 96 x 28x28 32->64 75 -> 67 us).  Rows that take four-byte
-// loads are staged through registers (457 x 26x26 3->93: 100 us, asynchronously 115), and so are the forward pass and dX: their gathered operand is transposed on the way, which four-byte copies do more slowly (dX 76 -> 83 us) and reading it
+// loads are staged through registers (457 x 26x26 3->93: 100 us, asynchronously 115), and so are the forward pass and dX: their
+// gathered operand is transposed on the way, which four-byte copies do more slowly (dX 76 -> 83 us) and reading it
 // untransposed no faster (66 us); they wait for FMA issue (pipe 64 % busy with three warps per scheduler), not for memory.
 template <int BM, int BN, int TM, int TN, bool VEC>
 __global__ void __launch_bounds__((BM / TM) * (BN / TN), simt_ctas(TM * TN, (BM / TM) * (BN / TN)))

@@ -158,8 +158,8 @@ template <int NT, bool PAIR = false>
 struct IgemmCfg {
     static constexpr int B_ROWS = PAIR ? NT / 2 : NT;           // filter rows this CTA stages
     static constexpr int TILE_B_BYTES = B_ROWS * 128;
-    // 128-byte K chunks per stage: one thread issues for both SMs of a pair (and the MMAs of narrow tiles are short), and with one chunk per stage its
-    // per-stage work (barrier wait, four MMAs, two commits) is not hidden behind the MMAs; a pair's stage takes two
+    // 128-byte K chunks per stage: one thread issues for both SMs of a pair (and the MMAs of narrow tiles are short), and
+    // with one chunk per stage its per-stage work (barrier wait, four MMAs, two commits) is not hidden behind the MMAs; a pair's stage takes two
     static constexpr int KS = PAIR || NT <= 64 ? 2 : 1;
     static constexpr int STAGE_A_BYTES = KS * TILE_A_BYTES, STAGE_B_BYTES = KS * TILE_B_BYTES;
     static constexpr int STAGES = PAIR ? (NT == 256 ? 3 : 4) : ((NT == 256) ? 4 : (NT == 128 ? 6 : NT == 64 ? 4 : 5));
@@ -568,8 +568,8 @@ struct DwCfg {
 };
 
 // The kernel is bound by what an SM can pull from L2 (some 100 GB/s of it), so a pixel tile's dy is brought in once, in
-// stages of its own, and stays for all M groups of the CTA: with one stage of x and dy per group the tf32 layer
-// 256 x 16x16 128->128 took 47 us, DWTXT.
+// stages of its own, and stays for all M groups of the CTA (tf32 256 x 16x16 128->128: 47.5 us with x and dy in one stage per
+// group, 44.6 so).
 //
 // PAIR (clusters of two CTAs, cta_group::2): an M group is 256 rows -- each CTA stages the MB units of its own half --
 // and a column tile 2 * NT channels of dy, of which each CTA stages its own NT.  Per stage a CTA loads the same bytes as
@@ -1095,8 +1095,7 @@ int num_sms() {
 }
 
 // A stand-in with the pair kernels' launch shape for the occupancy query below.
-__global__ void __launch_bounds__(IGEMM_THREADS, 1) pair_probe_kernel() {
-    pdl_wait(); }
+__global__ void __launch_bounds__(IGEMM_THREADS, 1) pair_probe_kernel() { pdl_wait(); }
 
 bool cta_pairs_available() {
     static std::atomic<int> cache[AE_MAX_DEVICES];       // 0 = not asked yet, 1 = yes, 2 = no

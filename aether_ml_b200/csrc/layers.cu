@@ -1593,7 +1593,7 @@ extern "C" int aether_dropout_fwd_dev(const float* x, float* y, float* mask, int
                                       uint64_t offset, const int64_t* calls_dev, void* stream) {
     if (!x || !y || !mask || !calls_dev || n <= 0 || !(keep_prob > 0.f) || keep_prob > 1.f)
         return set_error(AE_BAD_ARG, "aether_dropout_fwd_dev: bad argument");
-    launch(dropout_fwd_kernel, blocks_for(n / 4 + 1, 256), 256, 0, static_cast<cudaStream_t>(stream),  x, y, mask, n, keep_prob, seed,
+    launch(dropout_fwd_kernel, blocks_for(n / 4 + 1, 256), 256, 0, static_cast<cudaStream_t>(stream), x, y, mask, n, keep_prob, seed,
            offset, reinterpret_cast<const long long*>(calls_dev));
     count_launch();
     return check_launch("aether_dropout_fwd_dev");
@@ -1603,7 +1603,7 @@ extern "C" int aether_channel_mask_dev(float* mask, int C, float keep_prob, uint
                                        void* stream) {
     if (!mask || !calls_dev || C <= 0 || !(keep_prob > 0.f) || keep_prob > 1.f)
         return set_error(AE_BAD_ARG, "aether_channel_mask_dev: bad argument");
-    launch(channel_mask_kernel, ceil_div(C, 128), 128, 0, static_cast<cudaStream_t>(stream),  mask, C, keep_prob, seed,
+    launch(channel_mask_kernel, ceil_div(C, 128), 128, 0, static_cast<cudaStream_t>(stream), mask, C, keep_prob, seed,
            reinterpret_cast<const long long*>(calls_dev));
     count_launch();
     return check_launch("aether_channel_mask_dev");
@@ -1615,7 +1615,7 @@ extern "C" int aether_adam_step_dev(float* p, const float* g, float* m, float* v
     if (!p || !g || !m || !v || !iterations_dev || n <= 0) return set_error(AE_BAD_ARG, "aether_adam_step_dev: bad argument");
     if (!(beta1 >= 0.f && beta1 < 1.f) || !(beta2 >= 0.f && beta2 < 1.f))
         return set_error(AE_BAD_ARG, "aether_adam_step_dev: betas must be in [0, 1)");
-    launch(adam_dev_kernel, blocks_for(n / 4 + 1, 256), 256, 0, static_cast<cudaStream_t>(stream),  p, g, m, v, n, lr0, decay, beta1,
+    launch(adam_dev_kernel, blocks_for(n / 4 + 1, 256), 256, 0, static_cast<cudaStream_t>(stream), p, g, m, v, n, lr0, decay, beta1,
            beta2, eps, grad_scale, reinterpret_cast<const long long*>(iterations_dev));
     count_launch();
     return check_launch("aether_adam_step_dev");

@@ -718,8 +718,8 @@ class Model:
 
     def capture_train_step(self, X, y, warmup=2, collectives_in_graph=True, metrics=False):
         """Records ``train_step`` for batches shaped like (X, y) into a CUDA graph; ``train_step_graph`` replays
-        it with one launch.  A step of the small reference networks is ~130 kernel launches of a few microseconds
-        each, so the eager step is bound by launch overhead, not by the GPU.  Needs ``finalize(flat=True)``.
+        it with one launch.  A step of the small reference networks is some forty kernels of a few microseconds
+        each, so the eager step is bound by what its calls cost the host, not by the GPU.  Needs ``finalize(flat=True)``.
         Whatever the reference changes on the host per step (Adam's iteration count and decayed learning rate,
         the dropout draws) is read from one int64 device counter that the graph itself increments.  The warm-up
         steps (they size the workspaces) are undone, so capturing does not train.

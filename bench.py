@@ -73,13 +73,10 @@ def cpu_threads():
 
 
 def reference_checkout():
-    """Path of an Aether-ML checkout to time verbatim ($AETHER_REFERENCE_ROOT, else the build container's mount), or
-    None.  The reference is pure Python; it is never copied into this repository, so on a box without a checkout
-    only the NumPy restatement (oracle/) can be timed."""
-    for cand in (os.environ.get("AETHER_REFERENCE_ROOT"), "/root/reference"):
-        if cand and os.path.exists(os.path.join(cand, "CNN", "models", "CNN_classes.py")):
-            return cand
-    return None
+    """Path of an Aether-ML checkout to time verbatim ($AETHER_REFERENCE_ROOT), or None.  The reference is pure Python; it
+    is never copied into this repository, so without a checkout only the NumPy restatement (oracle/) can be timed."""
+    root = os.environ.get("AETHER_REFERENCE_ROOT")
+    return root if root and os.path.exists(os.path.join(root, "CNN", "models", "CNN_classes.py")) else None
 
 
 def cpu_conv_sample(images, threads=1, min_seconds=0.0, max_passes=1):
