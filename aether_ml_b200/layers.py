@@ -312,12 +312,17 @@ class Conv_Layer(_TakesCopies, _Saved):
             p = self._plans[key] = self._make_plan(*shape)
         return p
 
-    def _make_plan(self, S, H, W, Cin):
+    def _extent(self, H, W):
+        """(padding, output rows, output columns) for images of that size."""
         fH, fW = self.filter_size
         sH, sW = self.strides
         P = (fH - 1) // 2 if self.padding == "same" else 0      # :78-81, same amount on both axes
-        Ho = int((H + 2 * P - fH) / sH + 1)
-        Wo = int((W + 2 * P - fW) / sW + 1)
+        return P, int((H + 2 * P - fH) / sH + 1), int((W + 2 * P - fW) / sW + 1)
+
+    def _make_plan(self, S, H, W, Cin):
+        fH, fW = self.filter_size
+        sH, sW = self.strides
+        P, Ho, Wo = self._extent(H, W)
         return _ConvPlan(AetherConvDesc(S, H, W, Cin, self.num_filters, fH, fW, sH, sW, P, P, _lib.MATH_MODES[self.math_mode]), Ho, Wo)
 
     # -- operand-copy hand-off: the kernel that produces this layer's x (going forward) or dy (going back) may write

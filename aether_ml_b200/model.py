@@ -13,6 +13,7 @@ Additions that the reference does not have, all optional:
 """
 import math
 import pickle
+import weakref
 
 import numpy as np
 import torch
@@ -84,9 +85,9 @@ def _batches(n, batch_size):
 
 
 def _links(parts):
-    """How layers that follow each other are wired: (layer, attribute, the weak reference it holds), one reference object for
-    all that refer to the same layer."""
-    return [(p, name, p.__dict__.get(name)) for name, some in (("_link_prev", parts[1:]), ("_link_next", parts[:-1])) for p in some]
+    """How layers that follow each other are wired: (layer, attribute, the weak reference it holds) going forward and going
+    back, one reference object for all that refer to the same layer."""
+    return [[(p, name, p.__dict__.get(name)) for p in some] for name, some in (("_link_prev", parts[1:]), ("_link_next", parts[:-1]))]
 
 
 def _as_wired(links):
@@ -137,8 +138,8 @@ class _Chain:
             behind = at(k + 1)
         return _Chain(parts, conv, behind if hasattr(behind, "x_copy_target") else None)
 
-    def _intact(self, layers, i):
-        if layers[i:i + self.length] != self.parts or not _as_wired(self.links):
+    def _intact(self, layers, i, back):
+        if layers[i:i + self.length] != self.parts or not _as_wired(self.links[back]):
             return False
         for part in self.parts:
             d = part.__dict__
@@ -153,7 +154,7 @@ class _Chain:
         """Runs the chain's layers; False when they have to run one by one.  An inference pass with ``keep_all=False`` writes
         the last layer's output only and leaves the attributes of the others alone."""
         self.live = None
-        if not self._intact(layers, i):
+        if not self._intact(layers, i, False):
             return False
         x = to_device(inputs)
         bn, act, drop, pool = self.bn, self.act, self.drop, self.pool
@@ -220,7 +221,7 @@ class _Chain:
         """Runs the chain's backward passes; False when they have to run one by one."""
         live, self.live = self.live, None
         bn, act, drop, pool = self.bn, self.act, self.drop, self.pool
-        if live is None or not self._intact(layers, i):
+        if live is None or not self._intact(layers, i, True):
             return False
         x, x_version, bn_out, version, ws, mask, S, H, W, Cc, fH, fW, alpha = live
         if (bn.inputs is not x or act.inputs is not bn_out or bn_out._version != version or x._version != x_version or bn._ws.buf is not ws or act._alpha != alpha
@@ -273,8 +274,8 @@ class _DenseAct:
             return _DenseAct(layers[i], layers[i + 1], layers[i + 2] if i + 2 < len(layers) else None)
         return None
 
-    def _intact(self, layers, i):
-        if layers[i:i + 2] != self.parts or self.act.fused_into_prev or not _as_wired(self.links):
+    def _intact(self, layers, i, back):
+        if layers[i:i + 2] != self.parts or self.act.fused_into_prev or not _as_wired(self.links[back]):
             return False
         for part in self.parts:
             d = part.__dict__
@@ -283,7 +284,7 @@ class _DenseAct:
         return True
 
     def forward(self, layers, i, inputs, training, keep_all=True):
-        if not self._intact(layers, i):
+        if not self._intact(layers, i, False):
             return False
         x = to_device(inputs)
         dense, act = self.dense, self.act
@@ -301,7 +302,7 @@ class _DenseAct:
     def backward(self, layers, i, dvalues):
         dense, act = self.dense, self.act
         y = act.__dict__.get("inputs")
-        if y is None or not self._intact(layers, i) or dense.__dict__.get("output") is not y or not 0 < y.shape[0] <= self.MOST_ROWS:
+        if y is None or not self._intact(layers, i, True) or dense.__dict__.get("output") is not y or not 0 < y.shape[0] <= self.MOST_ROWS:
             return False
         dy = to_device(dvalues)
         p = dense._current()
@@ -325,8 +326,8 @@ class _Head:
     def find(layers, i):
         return _Head(layers[i], layers[i + 1]) if len(layers) == i + 2 and type(layers[i]) is Layer_Dense and type(layers[i + 1]) is SoftMax else None
 
-    def _intact(self, layers, i):
-        if layers[i:] != self.parts or not _as_wired(self.links):
+    def _intact(self, layers, i, back):
+        if layers[i:] != self.parts or not _as_wired(self.links[back]):
             return False
         for part in self.parts:
             d = part.__dict__
@@ -335,7 +336,7 @@ class _Head:
         return True
 
     def forward(self, layers, i, inputs, training, keep_all=True):
-        if not self._intact(layers, i):
+        if not self._intact(layers, i, False):
             return False
         x = to_device(inputs)
         dense, softmax = self.dense, self.softmax
@@ -352,7 +353,7 @@ class _Head:
         dense, softmax = self.dense, self.softmax
         z = softmax.__dict__.get("inputs")
         if (z is None or type(combined) is not Activation_Softmax_Loss_CategoricalCrossEntropy or "backward" in combined.__dict__
-                or softmax.output is not output or dense.__dict__.get("output") is not z or not self._intact(layers, len(layers) - 2)
+                or softmax.output is not output or dense.__dict__.get("output") is not z or not self._intact(layers, len(layers) - 2, True)
                 or z.shape[0] != dense.inputs.shape[0]):
             return False
         p = dense._current()
@@ -561,7 +562,8 @@ class Model:
         layers, chains, i = self.layers, self._chains, 0
         while i < len(layers):
             layer = layers[i]
-            inputs = layer.prev.output              # (of the layer in front, unless the caller has wired it otherwise)
+            link = layer.__dict__.get("_link_prev")       # (layer.prev, the layer in front unless the caller has wired it otherwise)
+            inputs = (link() if type(link) is weakref.ref else layer.prev).output
             chain = chains.get(i)
             if chain is not None and chain.forward(layers, i, inputs, training, keep):
                 i += chain.length
@@ -704,8 +706,15 @@ class Model:
 
     def _workspaces(self):
         """(layer, workspace, its buffer, its size) of all layers' workspaces as they are."""
-        names = ("_ws", "_stats_ws")
-        return [(l, w, w.buf, w.size) for l in self.layers for w in map(l.__dict__.get, names) if type(w) is _Workspace]
+        found = []
+        for l in self.layers:
+            w = l.__dict__.get("_ws")
+            if type(w) is _Workspace:
+                found.append((l, w, w.buf, w.size))
+                w = l.__dict__.get("_stats_ws")
+                if w is not None:
+                    found.append((l, w, w.buf, w.size))
+        return found
 
     def _all_ranks_agree(self, ok):
         """True when `ok` holds on every rank (one small eager all-reduce; single process: `ok` itself)."""
@@ -925,11 +934,11 @@ class Model:
                 if len(shape) != 3:
                     return None
                 working.append((l, shape))
-                shape = l._plan((1, *shape)).y_shape
-                if shape is None:
+                _, Ho, Wo = l._extent(shape[0], shape[1])
+                if Ho < 1 or Wo < 1:
                     return None
-                shape = shape[1:]
-                n = math.prod(shape)
+                shape = (Ho, Wo, l.num_filters)
+                n = Ho * Wo * l.num_filters
             elif kind is Pooling:
                 if len(shape) != 3:
                     return None
