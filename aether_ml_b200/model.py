@@ -260,7 +260,14 @@ class _DenseAct:
     """A Layer_Dense and the (Leaky_)ReLU behind it, run in one call each way; every attribute of both layers is as the layers
     leave it.  Same conditions as _Chain, and only where the library has one launch for it."""
     length = 2
-    MOST_ROWS = 1024            # aether_act_bwd_copy: a CTA walks all rows
+
+    @staticmethod
+    def _together(rows, columns):
+        """Whether the activation's backward pass goes with its operand copy and column sums (aether_act_bwd_copy: a CTA walks all
+        rows of 32 columns, so its time grows with the rows while the passes by themselves spread over the GPU).  Activation
+        and layer backward in us, together / apart: 128 columns 256 rows 11.4 / 12.6, 512 14.4 / 14.1, 1024 19.3 / 13.6; 512
+        columns 512 rows 16.2 / 18.3, 768 19.2 / 19.5, 1024 22.1 / 20.8; 1024 columns 1024 rows 24.4 / 26.5, 1536 31.8 / 30.5."""
+        return 0 < rows <= 384 + min(columns, 1024)
 
     def __init__(self, dense, act, behind):
         self.parts = [dense, act]
@@ -302,7 +309,7 @@ class _DenseAct:
     def backward(self, layers, i, dvalues):
         dense, act = self.dense, self.act
         y = act.__dict__.get("inputs")
-        if y is None or not self._intact(layers, i, True) or dense.__dict__.get("output") is not y or not 0 < y.shape[0] <= self.MOST_ROWS:
+        if y is None or not self._intact(layers, i, True) or dense.__dict__.get("output") is not y or not self._together(*y.shape):
             return False
         dy = to_device(dvalues)
         p = dense._current()
