@@ -223,6 +223,9 @@ class ClockSampler:
         if self.proc is None:
             return {"sm_mhz": None, "sm_max_mhz": None, "reasons": ["nvidia-smi unavailable"]}
         time.sleep(0.15)
+        limit = time.perf_counter() + 3.0        # (a timed region of ten milliseconds may end before nvidia-smi has started)
+        while not self.rows and time.perf_counter() < limit:
+            time.sleep(0.05)
         self.proc.terminate()
         rows = [r for t, r in self.rows if t_begin <= t <= t_end + 0.2 and len(r) >= 7] or [r for _, r in self.rows if len(r) >= 7]
         if not rows:
