@@ -975,6 +975,10 @@ class Model:
             n = max(1, min(n // batch_size - 1, n * limit // need // batch_size)) * batch_size
         return n
 
+    def _workspaces_to_keep(self, samples, batch_size):
+        """What an inference that may join batches goes back to (two batches are never joined)."""
+        return self._workspaces() if batch_size is not None and samples > 2 * batch_size else ()
+
     def _restore_workspaces(self, held, all_of_them=False):
         """The layers' workspaces are again those of ``held``.  A layer that had none keeps its first one, which the next call
         of a program that only infers needs again; ``all_of_them``: it gives that up, too."""
@@ -1029,7 +1033,7 @@ class Model:
     def evaluate(self, X_val, y_val, *, batch_size=None):
         self.loss.new_pass()
         self.accuracy.new_pass()
-        held = self._workspaces()
+        held = self._workspaces_to_keep(len(X_val), batch_size)
         try:
             for sl, outputs in self._inference(X_val, batch_size, held):
                 y_pass = y_val[sl]
@@ -1046,7 +1050,7 @@ class Model:
     def predict(self, X, *, batch_size=None):
         # (SoftMax writes a new array every time; an output layer or a forward pass of the caller's may not)
         new = type(self.layers[-1]) is SoftMax and "forward" not in vars(self.layers[-1]) and self._own_forward()
-        held = self._workspaces()
+        held = self._workspaces_to_keep(len(X), batch_size)
         try:
             outs = [output if new else output.clone() for _, output in self._inference(X, batch_size, held)]
         finally:
