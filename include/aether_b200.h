@@ -142,7 +142,7 @@ int aether_conv2d_fwd_ex(const AetherConvDesc* desc, const float* x, const float
 
 /* The forward pass and the (leaky) ReLU behind it (a Dense layer of a small network is a launch of its own for each): y as
  * aether_conv2d_fwd_ex writes it, act_out = y > 0 ? y : alpha * y and, when given, the bf16 operand copy of act_out for the
- * layer behind, in rows of copy_ld (Cout <= copy_ld <= Cout rounded up to 64; padded columns are zeroed).  Shapes of the
+ * layer behind, in rows of copy_ld (a multiple of four, Cout <= copy_ld <= Cout rounded up to 64; 8-byte aligned; padded columns are zeroed).  Shapes of the
  * tensor-core path only.  aether_act_bwd_copy is the way back: dx = x < 0 ? alpha * dy : dy, its operand copy (dy_copy of
  * aether_conv2d_operand_layout) and its column sums db, which the layer's backward call then need not write.  One CTA walks
  * all rows of 32 columns: meant for up to a thousand rows. */
