@@ -102,6 +102,11 @@ static int validate_desc(const AetherConvDesc* d, const char* fn) {
     return AE_OK;
 }
 
+// Shapes that no kernel on plain bf16 / TF32 operands, no first-layer and no classifier-head kernel serves.
+static bool split_route(const AetherConvDesc& d) {
+    return !tc_conv_eligible(d) && !first_tc_eligible(d) && !smallc_conv_eligible(d) && !generic_head_shape(d) && split_conv_eligible(d);
+}
+
 static int pending_timeout(const char* fn) {
     if (g_status_host && *reinterpret_cast<volatile int*>(g_status_host) != 0)
         return set_error(AE_DEVICE_TIMEOUT, "%s: an earlier kernel abandoned a bounded wait (status %d)", fn,
@@ -187,11 +192,8 @@ extern "C" size_t aether_conv2d_workspace_bytes(const AetherConvDesc* d) {
         size_t s = first_tc_bwd_workspace_bytes(*d);
         if (s > g) g = s;
     }
-    if (tc_conv_eligible(*d)) {
-        size_t t = tc_conv_workspace_bytes(*d);
-        return t > g ? t : g;
-    }
-    return g;
+    const size_t t = tc_conv_eligible(*d) ? tc_conv_workspace_bytes(*d) : split_route(*d) ? split_conv_workspace_bytes(*d) : 0;
+    return t > g ? t : g;
 }
 
 extern "C" int aether_conv2d_operand_layout(const AetherConvDesc* d, AetherOperandLayout* out) {
@@ -287,6 +289,7 @@ extern "C" int aether_conv2d_fwd(const AetherConvDesc* d, const float* x, const 
     if (tc_conv_eligible(*d)) return tc_conv_fwd(*d, x, w, b, y, nullptr, ws, ws_bytes, 0, st);
     if (first_tc_eligible(*d)) return first_tc_fwd(*d, x, w, b, y, nullptr, st);
     if (smallc_conv_eligible(*d) && (!b || aligned16(b))) return smallc_conv_fwd(*d, x, w, b, y, nullptr, st);
+    if (split_route(*d) && ws && ws_bytes >= split_conv_workspace_bytes(*d)) return split_conv_fwd(*d, x, w, b, y, ws, st);
     return generic_conv_fwd(*d, x, w, b, y, ws, ws_bytes, st);
 }
 
@@ -346,6 +349,8 @@ extern "C" int aether_conv2d_bwd_ex(const AetherConvDesc* d, const float* x, con
         return set_error(AE_UNSUPPORTED, "aether_conv2d_bwd_ex: this shape / math mode / request reads no operand copy of dy "
                                          "(aether_conv2d_operand_layout returned 0, or a first layer asked for dx)");
     if (tc_conv_eligible(*d)) return tc_conv_bwd(*d, x, dy, w, dx, dw, db, ws, ws_bytes, x_shadow_valid, dy_colsum_rows, st);
+    if ((dx || dw) && split_route(*d) && ws && ws_bytes >= split_conv_workspace_bytes(*d))
+        return split_conv_bwd(*d, x, dy, w, dx, dw, db, ws, x_shadow_valid, st);
     if (dx && (rc = generic_conv_bwd_data(*d, dy, w, dx, ws, ws_bytes, st))) return rc;
     if (dw && first_tc_bwd_eligible(*d))
         return first_tc_bwd_filter(*d, x, dy, dw, db, ws, ws_bytes, dy_ready ? dy_colsum_rows : 0, st);

@@ -71,6 +71,14 @@ int simt_conv_bwd_filter(const AetherConvDesc& d, const float* x, const float* d
                          size_t ws_bytes, cudaStream_t st);
 size_t simt_conv_workspace_bytes(const AetherConvDesc& d);
 
+// ---- conv_split.cu : fp32 convolution on the tensor cores, operands as sums of three bf16 numbers (any stride up to 8, any
+// channel counts from 8); which shapes gain from it: split_conv_eligible
+bool split_conv_eligible(const AetherConvDesc& d);
+size_t split_conv_workspace_bytes(const AetherConvDesc& d);
+int split_conv_fwd(const AetherConvDesc& d, const float* x, const float* w, const float* b, float* y, void* ws, cudaStream_t st);
+int split_conv_bwd(const AetherConvDesc& d, const float* x, const float* dy, const float* w, float* dx, float* dw, float* db, void* ws,
+                   int copies_valid, cudaStream_t st);
+
 // ---- conv_generic.cu : classifier heads and dX of first layers on the CUDA cores; everything else goes to conv_simt.cu
 // classifier heads (pointwise, few outputs) with the softmax / the combined softmax and cross-entropy gradient in the kernel
 bool generic_head_shape(const AetherConvDesc& d);

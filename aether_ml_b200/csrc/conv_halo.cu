@@ -60,38 +60,6 @@ static constexpr int HALO_THREADS = 64 + 32 * HALO_EPI_WARPS;
 static constexpr int HALO_TAIL = 2048;          // barriers, TMEM pointer, bias
 static constexpr int HALO_STATS_BYTES = HALO_EPI_WARPS * STATS_WARP_FLOATS * 4;   // per-warp running column sums and pivots
 
-// MMA with descriptors given as (low word, shared high word); K-major 128-byte-swizzle operands.
-// PAIR: the 256-row form issued by the even CTA of a CTA pair (cta_group::2).
-template <bool TF32, bool PAIR>
-__device__ __forceinline__ void umma_lohi(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t hi, uint32_t idesc,
-                                          uint32_t accumulate) {
-    if constexpr (PAIR && TF32) {
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\tsetp.ne.b32 p, %5, 0;\n\tmov.b64 da, {%1, %4};\n\tmov.b64 db, {%2, %4};\n\t"
-            "tcgen05.mma.cta_group::2.kind::tf32 [%0], da, db, %3, p;\n\t}"
-            ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(hi), "r"(accumulate)
-            : "memory");
-    } else if constexpr (PAIR) {
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\tsetp.ne.b32 p, %5, 0;\n\tmov.b64 da, {%1, %4};\n\tmov.b64 db, {%2, %4};\n\t"
-            "tcgen05.mma.cta_group::2.kind::f16 [%0], da, db, %3, p;\n\t}"
-            ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(hi), "r"(accumulate)
-            : "memory");
-    } else if constexpr (TF32) {
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\tsetp.ne.b32 p, %5, 0;\n\tmov.b64 da, {%1, %4};\n\tmov.b64 db, {%2, %4};\n\t"
-            "tcgen05.mma.cta_group::1.kind::tf32 [%0], da, db, %3, p;\n\t}"
-            ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(hi), "r"(accumulate)
-            : "memory");
-    } else {
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\tsetp.ne.b32 p, %5, 0;\n\tmov.b64 da, {%1, %4};\n\tmov.b64 db, {%2, %4};\n\t"
-            "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, p;\n\t}"
-            ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(hi), "r"(accumulate)
-            : "memory");
-    }
-}
-
 // STATS: the epilogue also accumulates per-channel statistics of the output (p.stats must be set).
 // PAIR (clusters of two CTAs, cta_group::2): CTA rank r of a pair takes tile 2u + r of unit u and keeps filter rows
 // [r * NT/2, (r+1) * NT/2) of every tap resident; the even CTA issues 256-row MMAs that read both CTAs' windows and

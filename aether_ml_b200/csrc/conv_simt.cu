@@ -1,6 +1,7 @@
 // fp32 convolution on the CUDA cores as tiled implicit GEMMs: every filter size, stride, padding and channel count
 // Conv_Layer accepts (CNN/models/CNN_classes_cupy.py:70-154).  It serves what the tensor-core kernels do not take --
-// AETHER_MATH_FP32, strided layers, channel counts that are no multiple of 4 -- always in single precision.
+// AETHER_MATH_FP32, strided layers, channel counts that are no multiple of 4 -- always in single precision, where the layer is
+// too small or has too few channels for conv_split.cu, or no workspace is given.
 //
 //   forward  y[p][d]  = b[d] + sum_k col[p][k] w[k][d]       M = output pixels, N = Cout, K = taps * Cin
 //   dX       dx[q][c] = sum_(tap,d) dy[q - tap][d] w[tap][c][d]   M = input pixels, N = Cin, K = taps * Cout

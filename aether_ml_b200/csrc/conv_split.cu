@@ -1,0 +1,893 @@
+// Single-precision convolution on the tensor cores: every fp32 operand is the sum of three bf16 numbers (8 + 8 + 8 bits of
+// mantissa, exponents of the same range), x = x0 + x1 + x2 with x0 = bf16(x), x1 = bf16(x - x0), x2 = bf16(x - x0 - x1), and a
+// product of two fp32 numbers the six products x0 w0, x0 w1, x1 w0, x0 w2, x1 w1, x2 w0 (what is left out is below 2^-25 of it).  It
+// serves what the kernels on plain bf16 / TF32 operands do not take and the CUDA cores took (conv_simt.cu): AETHER_MATH_FP32,
+// strided layers, channel counts that are no multiple of 4 -- forward, dX and dW as implicit GEMMs (CNN_classes_cupy.py:70-154).
+//
+// Accuracy.  tcgen05 adds in fp32 but truncates after every step of 16 products (measured: one step keeps 25 fractional bits; the
+// error of a plain bf16 sum of 2048 exact products is 2.1e-6 and biased, 18 times an FMA loop's), so a sum stays in TMEM for
+// GROUP_STEPS steps only: the x0 w0 products of each group go to an accumulator of their own that the epilogue warps add to their running
+// sums in registers (rounding to nearest) while the next groups are multiplied.  The products of second and third
+// order are 2^-8 and 2^-16 of that and stay in two accumulators of their own for up to EPOCH_STAGES stages.  Relative error against
+// float64, FMA kernels / this one: 96 x 28x28 32->64 y 3.0e-7 / 8.2e-8, dX 4.2e-7 / 9.6e-8, dW 3.8e-7 / 2.6e-7, and no larger in
+// any of forty drawn layers.  An
+// output that is not finite (an infinite or NaN operand has no meaningful remainder, one above 3.39e38 rounds to infinity) is
+// summed again by FMAs from the fp32 arrays.  Operands below 2^-109 keep fewer than 24 bits (the last part is subnormal).
+//
+// Time.  Six MMAs take the place of one, 1/6 of the bf16 rate is 3.7 times the FMA pipes'.  N columns of the filter (dy in dW) are
+// staged as [w0 | w1 | w2], so that x0 multiplies [w1 | w2] and x1 [w0 | w1] in one MMA of 2 N columns each: four MMAs
+// per step, of whose operands shared memory delivers 4 x 4 KB + 6 N x 32 B against 6 N / 2 tensor clocks.  The
+// parts are made by a pass over x and dy (split3_kernel: 4 bytes read, 6 written, dB on the way) and copied by TMA, rows of 64
+// channels with zeros behind the last: channel counts need not be multiples of anything.  A strided layer's x is stored by
+// phases, so that a tap's pixels lie side by side (element strides in the tensor map halve the copies' rate).
+// Measured on B200, forward + backward, CUDA cores / this file: 40 x 33x32 64->128 444 / 156 us, 96 x 28x28 32->64 209 / 156, 100 x 57x45
+// 48->72 stride 2 432 / 272.  Bound by the operands' way from L2 into shared memory (some 60 bytes a clock and SM).
+#include <string.h>
+
+#include <cuda_bf16.h>
+
+#include "common.cuh"
+#include "sm100_ptx.cuh"
+#include "tc_host.cuh"
+
+namespace aether {
+
+static constexpr int SPLIT_KC = 64;             // channels per row of a tile (128 bytes)
+static constexpr int GROUP_STEPS = 2;           // steps of 16 products whose sum may stay in TMEM; a stage is two groups
+static constexpr int EPOCH_STAGES = 32;         // stages after which the small products' sums leave TMEM, too
+static constexpr int SPLIT_EPI_WARPS = 8;       // 4 TMEM lane quarters x 2 (16-column blocks taken in turn)
+static constexpr int SPLIT_THREADS = 128 + 32 * SPLIT_EPI_WARPS;     // warps 0 and 1 copy, 2 and 3 multiply, the others add and store
+static constexpr int DW_PIXELS = 64;            // pixel rows per stage of dW
+
+struct SplitParams {
+    CUtensorMap tm_a;     // igemm: pixels (C, W, H, N, part x phase), box 64 x BW x BH x BN; dW: x
+    CUtensorMap tm_b;     // igemm: filter (K, columns, part x tap), box 64 x NT; dW: dy (C, W, H, N, part)
+    const float* in;      // the fp32 arrays behind them, for outputs that are not finite; dW: x
+    const float* w;       // filter (taps, Cin, Cout); dW: dy
+    const float* bias;    // nullable
+    float* out;           // dW: partial sums [split][U][64][ldn]
+    int* status;
+    int IH, IW, IC;       // extent of `in`
+    int OH, OW, S;        // extent of the output pixels (dW: of dy)
+    int N;                // output columns
+    int fH, fW, sH, sW, pH, pW, Cin, Cout;
+    int dx;               // gather over dy, a stride's input pixels in sH * sW classes
+    int BW, BH, BN, rows, tiles_w, tiles_h, tiles_n;
+    int NT, n_tiles_n;    // column tile (a multiple of 16; dW: 64)
+    int kchunks, last_ksteps;
+    int units;
+    int U, cblocks, splits, ksteps, ldn;      // dW: units of 64 filter rows (tap, 64 channels), pixel splits, steps per stage
+};
+
+template <int NTMAX, bool DW>
+struct SplitCfg {
+    static constexpr int A_PART = DW ? 2 * DW_PIXELS * 128 : 128 * 128;     // bytes of one part of the 128 accumulator rows' operand
+    static constexpr int STAGE_A = 3 * A_PART;
+    static constexpr int STAGE_B = 3 * NTMAX * (DW ? 2 * DW_PIXELS : 128);
+    static constexpr int STAGES = (216 * 1024) / (STAGE_A + STAGE_B);
+    static constexpr int SMEM_BYTES = 1024 + STAGES * (STAGE_A + STAGE_B) + 256;
+    static constexpr int NBG = NTMAX <= 64 ? 2 : 1;             // accumulators of a stage's two groups
+    static constexpr int NBC = NTMAX <= 64 ? 2 : 1;             // accumulator pairs of the small products
+    static constexpr int BLOCKS = NTMAX / 32;                   // 16-column blocks of an epilogue warp
+    static_assert((NBG + NBC) * 2 * NTMAX <= 512 && STAGES >= 2, "TMEM, shared memory");
+};
+
+// A pixel class of dX: output rows h = hs + a * sH see the taps i = ph + ti * sH at input row a + hq - ti.  (Forward: one class.)
+struct SplitClass {
+    int ph, pw, nH, nW, hs, ws, hq, wq, MH, MW;
+};
+__device__ __forceinline__ SplitClass split_class(const SplitParams& p, int cls) {
+    SplitClass c = {0, 0, p.fH, p.fW, 0, 0, 0, 0, p.OH, p.OW};
+    if (p.dx) {
+        c.ph = cls / p.sW;
+        c.pw = cls - c.ph * p.sW;
+        c.nH = c.ph < p.fH ? (p.fH - c.ph - 1) / p.sH + 1 : 0;
+        c.nW = c.pw < p.fW ? (p.fW - c.pw - 1) / p.sW + 1 : 0;
+        c.hs = ((c.ph - p.pH) % p.sH + p.sH) % p.sH;
+        c.ws = ((c.pw - p.pW) % p.sW + p.sW) % p.sW;
+        c.hq = (c.hs + p.pH - c.ph) / p.sH;
+        c.wq = (c.ws + p.pW - c.pw) / p.sW;
+        c.MH = c.hs < p.OH ? (p.OH - c.hs - 1) / p.sH + 1 : 0;
+        c.MW = c.ws < p.OW ? (p.OW - c.ws - 1) / p.sW + 1 : 0;
+    }
+    return c;
+}
+
+// Row (column) offset `a` of a tap against stride `s`: the phase of the input pixels it reads, and where in them.
+__device__ __forceinline__ void split_phase(int a, int s, int& phase, int& at) {
+    at = a >= 0 ? a / s : -((-a + s - 1) / s);
+    phase = a - at * s;
+}
+
+// One output by FMAs in the order of the reduction.
+__device__ float split_direct(const SplitParams& p, int n, int h, int w, int col) {
+    float s = 0.f;
+    for (int i = 0; i < p.fH; ++i)
+        for (int j = 0; j < p.fW; ++j) {
+            int a = h * p.sH - p.pH + i, b = w * p.sW - p.pW + j;
+            if (p.dx) {
+                a = h + p.pH - i;
+                b = w + p.pW - j;
+                if (a < 0 || b < 0 || a % p.sH || b % p.sW) continue;
+                a /= p.sH;
+                b /= p.sW;
+            }
+            if ((unsigned)a >= (unsigned)p.IH || (unsigned)b >= (unsigned)p.IW) continue;
+            const float* x = p.in + (((size_t)n * p.IH + a) * p.IW + b) * p.IC;
+            const float* f = p.w + (size_t)(i * p.fW + j) * p.Cin * p.Cout;
+            for (int k = 0; k < p.IC; ++k) s = fmaf(x[k], p.dx ? f[(size_t)col * p.Cout + k] : f[(size_t)k * p.Cout + col], s);
+        }
+    return s;
+}
+
+// Pixel tile `t` of p's tiling: first column, row and image.
+__device__ __forceinline__ void split_tile_origin(const SplitParams& p, int t, int& w0, int& h0, int& n0) {
+    const unsigned u = (unsigned)t, a = u / (unsigned)p.tiles_w, n = a / (unsigned)p.tiles_h;
+    w0 = (int)(u - a * (unsigned)p.tiles_w) * p.BW;
+    h0 = (int)(a - n * (unsigned)p.tiles_h) * p.BH;
+    n0 = (int)n * p.BN;
+}
+
+// The same for an entry (filter row i, column j, channel c; output channel d) of a split's partial filter gradient.
+__device__ float split_direct_dw(const SplitParams& p, int t0, int t1, int i, int j, int c, int d) {
+    float s = 0.f;
+    for (int t = t0; t < t1; ++t) {
+        int w0, h0, n0;
+        split_tile_origin(p, t, w0, h0, n0);
+        for (int r = 0; r < p.rows; ++r) {
+            const int w = w0 + r % p.BW, h = h0 + r / p.BW % p.BH, n = n0 + r / (p.BW * p.BH);
+            const int a = h * p.sH - p.pH + i, b = w * p.sW - p.pW + j;
+            if (w >= p.OW || h >= p.OH || n >= p.S || (unsigned)a >= (unsigned)p.IH || (unsigned)b >= (unsigned)p.IW) continue;
+            s = fmaf(p.in[(((size_t)n * p.IH + a) * p.IW + b) * p.Cin + c], p.w[(((size_t)n * p.OH + h) * p.OW + w) * p.Cout + d], s);
+        }
+    }
+    return s;
+}
+
+// Row `r` of a unit's 128, pixel (b, a, n) of its box: where it goes (null: nowhere) and what it is (igemm: output column, row, image;
+// dW: filter column, filter row, channel).
+template <bool DW>
+__device__ __forceinline__ float* split_row(const SplitParams& p, int mt, int cls, const SplitClass& c, int w0, int h0, int n0, int r, int b, int a,
+                                            int n, int& x_w, int& x_h, int& x_n) {
+    if (DW) {
+        const int unit = mt * 2 + r / 64, tap = unit / p.cblocks;
+        x_h = tap / p.fW;
+        x_w = tap - x_h * p.fW;
+        x_n = (unit - tap * p.cblocks) * 64 + r % 64;
+        return (unit < p.U && x_n < p.Cin) ? p.out + (((size_t)cls * p.U + unit) * 64 + r % 64) * p.ldn : nullptr;
+    }
+    const int w = w0 + b, h = h0 + a;
+    x_n = n0 + n;
+    x_h = p.dx ? c.hs + h * p.sH : h;
+    x_w = p.dx ? c.ws + w * p.sW : w;
+    return (r < p.rows && h < c.MH && w < c.MW && x_n < p.S) ? p.out + (((size_t)x_n * p.OH + x_h) * p.OW + x_w) * p.N : nullptr;
+}
+
+// What this lane stored for a unit and is not finite, again by FMAs.
+template <bool DW>
+__device__ __noinline__ void split_repair(const SplitParams& p, int nt, int mt, int cls, int t0, int t1, int q, int part, int lane) {
+    int w0 = 0, h0 = 0, n0 = 0, x_w, x_h, x_n;
+    const SplitClass c = split_class(p, cls);
+    if (!DW) split_tile_origin(p, mt, w0, h0, n0);
+    for (int j = 0; j < 4; ++j) {
+        const int r = q * 32 + (lane & ~3) + j;
+        float* row = split_row<DW>(p, mt, cls, c, w0, h0, n0, r, r % p.BW, r / p.BW % p.BH, r / (p.BW * p.BH), x_w, x_h, x_n);
+        if (row == nullptr) continue;
+        for (int b = part; b * 16 < p.NT; b += 2)
+            for (int e = 0; e < 4; ++e) {
+                const int col = nt * p.NT + b * 16 + (lane & 3) * 4 + e;
+                if (col >= p.N || fabsf(row[col]) <= 3.402823466e38f) continue;
+                row[col] = DW ? split_direct_dw(p, t0, t1, x_h, x_w, x_n, col)
+                              : split_direct(p, x_n, x_h, x_w, col) + (p.bias != nullptr ? p.bias[col] : 0.f);
+            }
+    }
+}
+
+// Persistent over units: igemm, a (pixel class, pixel tile, column tile); dW, a (pair of row units, column tile, range of pixel tiles).
+template <int NTMAX, bool DW>
+__global__ void __launch_bounds__(SPLIT_THREADS, 1) split_conv_kernel(const __grid_constant__ SplitParams p) {
+    using Cfg = SplitCfg<NTMAX, DW>;
+    constexpr int STAGES = Cfg::STAGES, NBG = Cfg::NBG, NBC = Cfg::NBC, STAGE = Cfg::STAGE_A + Cfg::STAGE_B;
+    constexpr int TILE = DW_PIXELS * 128;                          // dW: 64 channels of a box of pixels
+    extern __shared__ uint8_t smem_raw[];
+    const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+    const uint32_t sBar = smem_base + STAGES * STAGE;
+    auto full_bar = [&](int s) { return sBar + 8u * s; };
+    auto empty_bar = [&](int s) { return sBar + 8u * (STAGES + s); };
+    auto gfull_bar = [&](int b) { return sBar + 8u * (2 * STAGES + b); };                 // the sums of a stage's groups are complete / taken
+    auto gempty_bar = [&](int b) { return sBar + 8u * (2 * STAGES + NBG + b); };
+    auto cfull_bar = [&](int b) { return sBar + 8u * (2 * STAGES + 2 * NBG + b); };       // an epoch's small products
+    auto cempty_bar = [&](int b) { return sBar + 8u * (2 * STAGES + 2 * NBG + NBC + b); };
+    const uint32_t sTmemPtr = sBar + 8u * (2 * STAGES + 2 * NBG + 2 * NBC);
+    uint8_t* gen_base = smem_raw + (smem_base - smem_u32(smem_raw));
+    volatile uint32_t* tmem_ptr_generic = reinterpret_cast<volatile uint32_t*>(gen_base + (sTmemPtr - smem_base));
+
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);
+    const int lane = threadIdx.x & 31;
+
+    if (DW && p.rows < p.ksteps * 16) {
+        // rows of a box past p.rows are never written by TMA but read by the last step: zeros
+        const int per_tile = (p.ksteps * 16 - p.rows) * 8;                                // 16-byte pieces
+        for (int i = threadIdx.x; i < STAGES * STAGE / TILE * per_tile; i += SPLIT_THREADS) {
+            const int tile = i / per_tile;
+            *reinterpret_cast<uint4*>(gen_base + (size_t)tile * TILE + p.rows * 128 + (i - tile * per_tile) * 16) = make_uint4(0, 0, 0, 0);
+        }
+        fence_proxy_async_smem();
+    }
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < STAGES; ++s) { mbar_init(full_bar(s), 2); mbar_init(empty_bar(s), 2); }
+        for (int b = 0; b < NBG; ++b) { mbar_init(gfull_bar(b), 1); mbar_init(gempty_bar(b), SPLIT_EPI_WARPS); }
+        for (int b = 0; b < NBC; ++b) { mbar_init(cfull_bar(b), 1); mbar_init(cempty_bar(b), SPLIT_EPI_WARPS); }
+        mbar_fence_init();
+        tma_prefetch_desc(&p.tm_a);
+        tma_prefetch_desc(&p.tm_b);
+    }
+    if (warp == 3) {
+        tmem_alloc(sTmemPtr, 512);
+        tmem_relinquish();
+    }
+    pdl_wait();
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem_base = *tmem_ptr_generic;
+    const uint32_t tmem_c = tmem_base + NBG * 2 * NTMAX;           // accumulators of the small products
+
+    const int NT = p.NT;
+    const int ptiles = p.tiles_w * p.tiles_h * p.tiles_n;
+    const int b_part = DW ? TILE : NT * 128;                       // bytes of one part of the columns' operand
+    // unit -> column tile; igemm: pixel tile `mt` of class `cls`; dW: pair of row units `mt`, range of pixel tiles [t0, t1)
+    auto decode = [&](int u, int& nt, int& mt, int& cls, int& t0, int& t1) {
+        const unsigned a = (unsigned)u / (unsigned)p.n_tiles_n;
+        nt = u - (int)a * p.n_tiles_n;
+        if (DW) {
+            const unsigned groups = (unsigned)(p.U + 1) / 2, split = a / groups;
+            mt = (int)(a - split * groups);
+            cls = (int)split;
+            t0 = (int)((long long)ptiles * cls / p.splits);
+            t1 = (int)((long long)ptiles * (cls + 1) / p.splits);
+        } else {
+            cls = (int)(a / (unsigned)ptiles);
+            mt = (int)a - cls * ptiles;
+            t0 = t1 = 0;
+        }
+    };
+    // stages of a unit, and steps of one of them
+    auto unit_stages = [&](int cls, int t0, int t1) {
+        if (DW) return t1 - t0;
+        const SplitClass c = split_class(p, cls);
+        return c.nH * c.nW * p.kchunks;
+    };
+    auto stage_steps = [&](int kc) { return DW ? p.ksteps : kc == p.kchunks - 1 ? p.last_ksteps : 4; };
+
+    if (warp < 2) {
+        // ---- copies: warp 0 the rows' operand, warp 1 the columns'
+        if (elect_one()) {
+            const bool rows = warp == 0;
+            uint32_t s = 0, ph = 0;
+            bool ok = true;
+            const uint32_t tx = 3u * 128u * (DW ? (uint32_t)p.rows * (rows ? 2u : 1u) : (uint32_t)(rows ? p.rows : NT));
+            const int phases = p.dx ? 1 : p.sH * p.sW;
+            for (int u = blockIdx.x; u < p.units && ok; u += gridDim.x) {
+                int nt, mt, cls, t0, t1, w0, h0, n0;
+                decode(u, nt, mt, cls, t0, t1);
+                if (DW) {
+                    int uc[2], uw[2], uh[2], uf[2];               // channel, column, row and phase of the pair's units
+#pragma unroll
+                    for (int k = 0; k < 2; ++k) {
+                        int unit = mt * 2 + k, fh, fw;
+                        if (unit >= p.U) unit = p.U - 1;          // padding unit of the last pair: results are dropped
+                        const int tap = unit / p.cblocks, i = tap / p.fW;
+                        uc[k] = (unit - tap * p.cblocks) * SPLIT_KC;
+                        split_phase(tap - i * p.fW - p.pW, p.sW, fw, uw[k]);
+                        split_phase(i - p.pH, p.sH, fh, uh[k]);
+                        uf[k] = fh * p.sW + fw;
+                    }
+                    split_tile_origin(p, t0, w0, h0, n0);
+                    for (int t = t0; t < t1; ++t) {
+                        if (!mbar_wait(empty_bar(s), ph ^ 1u, p.status, DS_TIMEOUT_EMPTY)) { ok = false; break; }
+                        const uint32_t bar = full_bar(s), at = smem_base + s * STAGE + (rows ? 0 : Cfg::STAGE_A);
+                        mbar_arrive_expect_tx(bar, tx);
+#pragma unroll
+                        for (int q = 0; q < 3; ++q) {
+                            if (rows) {
+                                tma_load_5d(at + q * Cfg::A_PART, &p.tm_a, bar, uc[0], w0 + uw[0], h0 + uh[0], n0, q * phases + uf[0]);
+                                tma_load_5d(at + q * Cfg::A_PART + TILE, &p.tm_a, bar, uc[1], w0 + uw[1], h0 + uh[1], n0, q * phases + uf[1]);
+                            } else {
+                                tma_load_5d(at + q * TILE, &p.tm_b, bar, nt * NT, w0, h0, n0, q);
+                            }
+                        }
+                        if (++s == STAGES) { s = 0; ph ^= 1u; }
+                        w0 += p.BW;                               // the next tile
+                        if (w0 >= p.tiles_w * p.BW) { w0 = 0; h0 += p.BH; }
+                        if (h0 >= p.tiles_h * p.BH) { h0 = 0; n0 += p.BN; }
+                    }
+                } else {
+                    // taps in order; forward: phase (fh, fw) and offset (ch, cw) of the input pixels advance with them
+                    const SplitClass c = split_class(p, cls);
+                    split_tile_origin(p, mt, w0, h0, n0);
+                    const int iters = c.nH * c.nW * p.kchunks, taps = p.fH * p.fW;
+                    int fh = 0, fw = 0, ch = h0 + c.hq, cw = w0 + c.wq, fw0, cw0;
+                    if (!p.dx) {
+                        split_phase(-p.pH, p.sH, fh, ch);
+                        split_phase(-p.pW, p.sW, fw, cw);
+                        ch += h0;
+                        cw += w0;
+                    }
+                    fw0 = fw;
+                    cw0 = cw;
+                    int kc = 0, j = 0, row = c.ph * p.fW, tap = row + c.pw;
+                    for (int it = 0; it < iters; ++it) {
+                        if (!mbar_wait(empty_bar(s), ph ^ 1u, p.status, DS_TIMEOUT_EMPTY)) { ok = false; break; }
+                        const uint32_t bar = full_bar(s), at = smem_base + s * STAGE + (rows ? 0 : Cfg::STAGE_A);
+                        mbar_arrive_expect_tx(bar, tx);
+#pragma unroll
+                        for (int q = 0; q < 3; ++q) {
+                            if (rows) tma_load_5d(at + q * Cfg::A_PART, &p.tm_a, bar, kc * SPLIT_KC, cw, ch, n0, q * phases + fh * p.sW + fw);
+                            else tma_load_3d(at + q * b_part, &p.tm_b, bar, kc * SPLIT_KC, nt * NT, q * taps + tap);
+                        }
+                        if (++kc == p.kchunks) {
+                            kc = 0;
+                            if (p.dx) { --cw; tap += p.sW; }
+                            else { ++tap; if (++fw == p.sW) { fw = 0; ++cw; } }
+                            if (++j == c.nW) {
+                                j = 0;
+                                fw = fw0;
+                                cw = cw0;
+                                if (p.dx) { --ch; row += p.sH * p.fW; }
+                                else { row += p.fW; if (++fh == p.sH) { fh = 0; ++ch; } }
+                                tap = row + c.pw;
+                            }
+                        }
+                        if (++s == STAGES) { s = 0; ph ^= 1u; }
+                    }
+                }
+            }
+        }
+    } else if (warp < 4) {
+        // ---- products: warp 3 has x0 w0, warp 2 the small ones.  Issuing an MMA or a commit costs a thread about 50 clocks and each
+        // barrier it waits for 80, as much as 128 columns take to multiply: with two threads those run beside the MMAs.  The loops
+        // are warp-uniform (every lane polls, one issues): descriptors stay in uniform registers, where MMAs take them from.
+        const bool main = warp == 3, leader = elect_one();
+        const uint32_t idesc1 = make_idesc(1u, DW, DW, 128u, (uint32_t)NT), idesc2 = make_idesc(1u, DW, DW, 128u, 2u * (uint32_t)NT);
+        constexpr uint32_t ADV = DW ? 16 * 128 / 16 : 32 / 16;                            // a step of 16 in units of 16 bytes
+        const uint64_t proto = make_smem_desc(0, DW ? TILE : 16, 1024);
+        const uint32_t hi = (uint32_t)(proto >> 32), lo0 = (uint32_t)proto + (smem_base >> 4);
+        constexpr uint32_t A_NEXT = Cfg::A_PART / 16;
+        const uint32_t b_next = (uint32_t)b_part / 16;
+        auto wait = [&](uint32_t bar, uint32_t parity, int code) { return __all_sync(0xffffffffu, mbar_wait_spin(bar, parity, p.status, code)) != 0; };
+        uint32_t s = 0, ph = 0, gb = 0, gph = 0;          // gb: accumulator of the stage (main) or of the epoch
+        bool ok = true;
+        for (int u = blockIdx.x; u < p.units && ok; u += gridDim.x) {
+            int nt, mt, cls, t0, t1;
+            decode(u, nt, mt, cls, t0, t1);
+            const int iters = unit_stages(cls, t0, t1);
+            int kc = 0, left = 0;                             // stages that the epoch still takes; 0: start one
+            for (int it = 0; it < iters; ++it) {
+                const int steps = stage_steps(kc);
+                if (++kc == p.kchunks) kc = 0;
+                const uint32_t da = lo0 + s * (STAGE / 16), db = da + Cfg::STAGE_A / 16;
+                if (main) {
+                    if (!wait(gempty_bar(gb), gph ^ 1u, DS_TIMEOUT_TMEM_EMPTY)) { ok = false; break; }
+                    if (!wait(full_bar(s), ph, DS_TIMEOUT_FULL)) { ok = false; break; }
+                    tc_fence_after();
+                    const uint32_t dg = tmem_base + gb * (2 * NTMAX);
+                    if (leader) {
+                        umma_lohi<false, false>(dg, da, db, hi, idesc1, 0u);
+                        if (steps > 1) umma_lohi<false, false>(dg, da + ADV, db + ADV, hi, idesc1, 1u);
+                        if (steps > 2) umma_lohi<false, false>(dg + NTMAX, da + 2 * ADV, db + 2 * ADV, hi, idesc1, 0u);
+                        if (steps > 3) umma_lohi<false, false>(dg + NTMAX, da + 3 * ADV, db + 3 * ADV, hi, idesc1, 1u);
+                        umma_commit(gfull_bar(gb));
+                        umma_commit(empty_bar(s));
+                    }
+                    if (++gb == NBG) { gb = 0; gph ^= 1u; }
+                } else {
+                    uint32_t acc = 1u;
+                    if (left == 0) {
+                        if (!wait(cempty_bar(gb), gph ^ 1u, DS_TIMEOUT_TMEM_EMPTY)) { ok = false; break; }
+                        left = EPOCH_STAGES;
+                        acc = 0u;
+                    }
+                    if (!wait(full_bar(s), ph, DS_TIMEOUT_FULL)) { ok = false; break; }
+                    tc_fence_after();
+                    const uint32_t dc = tmem_c + gb * (2 * NTMAX);
+                    const bool last = --left == 0 || it == iters - 1;
+                    if (leader) {
+#pragma unroll
+                        for (int k = 0; k < 4; ++k) {
+                            if (k < steps) {
+                                umma_lohi<false, false>(dc, da + ADV * k, db + b_next + ADV * k, hi, idesc2, k > 0 ? 1u : acc);      // x0 [w1 | w2]
+                                umma_lohi<false, false>(dc, da + A_NEXT + ADV * k, db + ADV * k, hi, idesc2, 1u);                    // x1 [w0 | w1]
+                                umma_lohi<false, false>(dc + NT, da + 2 * A_NEXT + ADV * k, db + ADV * k, hi, idesc1, 1u);           // x2 w0
+                            }
+                        }
+                        if (last) umma_commit(cfull_bar(gb));
+                        umma_commit(empty_bar(s));
+                    }
+                    if (last) {
+                        left = 0;
+                        if (++gb == NBC) { gb = 0; gph ^= 1u; }
+                    }
+                }
+                if (++s == STAGES) { s = 0; ph ^= 1u; }
+            }
+        }
+        __syncwarp();
+    } else {
+        // ---- sums: warp (q, part) has accumulator rows [32q, 32q + 32), a row per lane, and the 16-column blocks part, part + 2, ...
+        constexpr int BLOCKS = Cfg::BLOCKS;
+        const int q = warp & 3, part = (warp - 4) >> 2;
+        const uint32_t lane0 = ((uint32_t)(q * 32) << 16) + part * 16;
+        int r_w[4], r_h[4], r_n[4];                               // the four rows in the box of pixels that this lane's quad stores
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int r = q * 32 + (lane & ~3) + j;
+            r_w[j] = r % p.BW;
+            r_h[j] = r / p.BW % p.BH;
+            r_n[j] = r / (p.BW * p.BH);
+        }
+        uint32_t gb = 0, gph = 0, cb = 0, cph = 0;
+        bool ok = true;
+        for (int u = blockIdx.x; u < p.units && ok; u += gridDim.x) {
+            int nt, mt, cls, t0, t1;
+            decode(u, nt, mt, cls, t0, t1);
+            const int iters = unit_stages(cls, t0, t1);
+            float acc[BLOCKS][16];
+#pragma unroll
+            for (int b = 0; b < BLOCKS; ++b)
+#pragma unroll
+                for (int k = 0; k < 16; ++k) acc[b][k] = 0.f;
+            // acc += accumulator at column t0, then, when asked for, the one at t1  (blocks past NT: other accumulators' columns, never stored)
+            auto add = [&](uint32_t ta, uint32_t tb, bool both) {
+#pragma unroll
+                for (int b = 0; b < BLOCKS; b += 2) {
+                    uint32_t v[2][16], w[2][16];
+                    tmem_ld_32x16(ta + lane0 + 32 * b, v[0]);
+                    tmem_ld_32x16(ta + lane0 + 32 * b + 32, v[1]);
+                    if (both) {
+                        tmem_ld_32x16(tb + lane0 + 32 * b, w[0]);
+                        tmem_ld_32x16(tb + lane0 + 32 * b + 32, w[1]);
+                    } else {
+#pragma unroll
+                        for (int k = 0; k < 16; ++k) w[0][k] = w[1][k] = 0u;
+                    }
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int k = 0; k < 16; ++k) {
+                        acc[b][k] = (acc[b][k] + __uint_as_float(v[0][k])) + __uint_as_float(w[0][k]);
+                        acc[b + 1][k] = (acc[b + 1][k] + __uint_as_float(v[1][k])) + __uint_as_float(w[1][k]);
+                    }
+                }
+            };
+            auto release = [&](uint32_t bar) {
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(bar);
+            };
+            int kc = 0, left = EPOCH_STAGES;
+            for (int it = 0; it < iters; ++it) {
+                const int steps = stage_steps(kc);
+                if (++kc == p.kchunks) kc = 0;
+                if (!mbar_wait_spin(gfull_bar(gb), gph, p.status, DS_TIMEOUT_TMEM_FULL)) { ok = false; break; }
+                tc_fence_after();
+                add(tmem_base + gb * (2 * NTMAX), tmem_base + gb * (2 * NTMAX) + NTMAX, steps > GROUP_STEPS);
+                release(gempty_bar(gb));
+                if (++gb == NBG) { gb = 0; gph ^= 1u; }
+                if (--left == 0 || it == iters - 1) {
+                    left = EPOCH_STAGES;
+                    if (!mbar_wait_spin(cfull_bar(cb), cph, p.status, DS_TIMEOUT_TMEM_FULL)) { ok = false; break; }
+                    tc_fence_after();
+                    add(tmem_c + cb * (2 * NTMAX) + NT, tmem_c + cb * (2 * NTMAX), true);       // third order, then second
+                    release(cempty_bar(cb));
+                    if (++cb == NBC) { cb = 0; cph ^= 1u; }
+                }
+            }
+            if (!ok) break;
+            int w0 = 0, h0 = 0, n0 = 0, x_w, x_h, x_n;
+            const SplitClass c = split_class(p, cls);
+            if (!DW) split_tile_origin(p, mt, w0, h0, n0);
+            float* rowp[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) rowp[j] = split_row<DW>(p, mt, cls, c, w0, h0, n0, q * 32 + (lane & ~3) + j, r_w[j], r_h[j], r_n[j], x_w, x_h, x_n);
+            bool bad = false;
+            const bool b1 = lane & 1, b2 = lane & 2;
+#pragma unroll
+            for (int b = 0; b < BLOCKS; ++b) {
+                if ((2 * b + part) * 16 < NT) {
+                    // The quad's 4 rows x 16 columns are exchanged so that lane i holds columns 4i .. 4i + 3 of all four rows and the
+                    // quad stores 64 bytes of a row at a time: bit 1 of the lane against bit 1 of the column group, then bit 0.
+                    float m[4][4];                                // [row][column of this lane's group]
+                    float t[2][2][4];                             // [row bit 1 of group .. ] after the first exchange
+#pragma unroll
+                    for (int g = 0; g < 2; ++g)
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) {
+                            const float lo = acc[b][4 * g + e], up = acc[b][8 + 4 * g + e];        // groups g and g + 2 of this lane's row
+                            const float got = __shfl_xor_sync(0xffffffffu, b2 ? lo : up, 2);
+                            t[0][g][e] = b2 ? got : lo;           // rows (lane & 1) and (lane & 1) + 2 of groups (lane & 2) + g
+                            t[1][g][e] = b2 ? up : got;
+                        }
+#pragma unroll
+                    for (int h = 0; h < 2; ++h)
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) {
+                            const float got = __shfl_xor_sync(0xffffffffu, b1 ? t[h][0][e] : t[h][1][e], 1);
+                            m[2 * h][e] = b1 ? got : t[h][0][e];
+                            m[2 * h + 1][e] = b1 ? t[h][1][e] : got;
+                        }
+                    const int col = nt * NT + (2 * b + part) * 16 + (lane & 3) * 4;
+                    float bias[4] = {0.f, 0.f, 0.f, 0.f};
+                    if (!DW && p.bias != nullptr) {
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) bias[e] = col + e < p.N ? __ldg(p.bias + col + e) : 0.f;
+                    }
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        if (rowp[j] == nullptr) continue;
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) {
+                            bad |= !(fabsf(m[j][e]) <= 3.402823466e38f);
+                            m[j][e] += bias[e];
+                        }
+                        if ((DW ? p.ldn : p.N) % 4 == 0) {
+                            if (col < p.N) *reinterpret_cast<float4*>(rowp[j] + col) = make_float4(m[j][0], m[j][1], m[j][2], m[j][3]);
+                        } else {
+#pragma unroll
+                            for (int e = 0; e < 4; ++e)
+                                if (col + e < p.N) rowp[j][col + e] = m[j][e];
+                        }
+                    }
+                }
+            }
+            if (bad) split_repair<DW>(p, nt, mt, cls, t0, t1, q, part, lane);
+        }
+    }
+
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 3) {
+        tc_fence_after();
+        tmem_dealloc(tmem_base, 512);
+    }
+}
+
+// ====================================================================================== operands
+__device__ __forceinline__ void split3(float v, __nv_bfloat16& a, __nv_bfloat16& b, __nv_bfloat16& c) {
+    a = __float2bfloat16_rn(v);
+    const float r = v - __bfloat162float(a);             // exact
+    b = __float2bfloat16_rn(r);
+    c = __float2bfloat16_rn(r - __bfloat162float(b));
+}
+
+// A strided layer's x by phases: [sH * sW][S][ceil(H / sH)][ceil(W / sW)] pixels (those outside the image are zero), so that the pixels a tap
+// sees lie side by side.
+struct SplitPhases {
+    int H, W, sH, sW, PH, PW;
+    long long images;                                    // S * PH * PW
+    // source row of row `r`, or -1
+    __device__ __forceinline__ long long source(long long r) const {
+        const long long f = r / images;
+        const unsigned i = (unsigned)(r - f * images), a = i / (unsigned)PW, n = a / (unsigned)PH;
+        const int w = (int)(i - a * PW) * sW + (int)f % sW, h = (int)(a - n * PH) * sH + (int)f / sW;
+        return w < W && h < H ? ((long long)n * H + h) * W + w : -1;
+    }
+};
+
+// fp32 [rows][C] -> three bf16 arrays [3][rows][Cp] (channels padded with zeros to a multiple of 8) and, when asked for, each block's
+// column sums of the fp32 input (for dB).  Bound by HBM: 4 bytes read, 6 written.
+template <bool COLSUM, bool STRIDED>
+__global__ void __launch_bounds__(256) split3_kernel(const float* __restrict__ src, __nv_bfloat16* __restrict__ dst, long long rows, int C,
+                                                     int Cp, float* __restrict__ colsum_part, long long rows_per_block, const SplitPhases f) {
+    pdl_wait();
+    const int G = Cp / 8;                                // groups of eight channels
+    const long long r_begin = blockIdx.x * rows_per_block;
+    const long long r_end = r_begin + rows_per_block < rows ? r_begin + rows_per_block : rows;
+    const size_t plane = (size_t)rows * Cp;
+    __shared__ float red[COLSUM ? 256 * 8 : 8];
+    for (int gbase = 0; gbase < G; gbase += 256) {
+        const int Gc = (G - gbase) < 256 ? (G - gbase) : 256, lanes = 256 / Gc;
+        const int g = gbase + threadIdx.x % Gc, rl = threadIdx.x / Gc, c0 = g * 8;
+        float acc[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) acc[k] = 0.f;
+        if (rl < lanes) {
+            const bool whole = C % 4 == 0 && c0 + 8 <= C;
+            constexpr int U = 4;                         // rows in flight
+            for (long long r0 = r_begin + rl; r0 < r_end; r0 += U * lanes) {
+                float v[U][8];
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    const long long r = r0 + u * lanes;
+                    const long long at = STRIDED && r < r_end ? f.source(r) : r;
+                    const float* s = src + at * C + c0;
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) v[u][k] = 0.f;
+                    if (r < r_end && at >= 0) {
+                        if (whole) {
+                            *reinterpret_cast<float4*>(v[u]) = __ldcs(reinterpret_cast<const float4*>(s));
+                            *reinterpret_cast<float4*>(v[u] + 4) = __ldcs(reinterpret_cast<const float4*>(s + 4));
+                        } else {
+#pragma unroll
+                            for (int k = 0; k < 8; ++k)
+                                if (c0 + k < C) v[u][k] = __ldg(s + k);
+                        }
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    const long long r = r0 + u * lanes;
+                    if (r < r_end) {
+                        __align__(16) __nv_bfloat16 o[3][8];
+#pragma unroll
+                        for (int k = 0; k < 8; ++k) {
+                            if (COLSUM) acc[k] += v[u][k];
+                            split3(v[u][k], o[0][k], o[1][k], o[2][k]);
+                        }
+#pragma unroll
+                        for (int q = 0; q < 3; ++q) *reinterpret_cast<uint4*>(dst + q * plane + (size_t)r * Cp + c0) = *reinterpret_cast<const uint4*>(o[q]);
+                    }
+                }
+            }
+        }
+        if (COLSUM) {
+#pragma unroll
+            for (int k = 0; k < 8; ++k) red[threadIdx.x * 8 + k] = acc[k];
+            __syncthreads();
+            for (int cc = threadIdx.x; cc < Gc * 8; cc += 256) {
+                const int c = gbase * 8 + cc;
+                if (c < C) {
+                    float s = 0.f;
+                    for (int l = 0; l < lanes; ++l) s += red[(l * Gc + cc / 8) * 8 + cc % 8];
+                    colsum_part[(size_t)blockIdx.x * C + c] = s;
+                }
+            }
+            __syncthreads();
+        }
+    }
+}
+
+// The filter's operands from one read of w (taps, Cin, Cout): fwd [3][taps][Cout][Cin_p] (transposed), dx [3][taps][Cin][Cout_p].
+// grid (ceil(Cout_p / 32), ceil(Cin_p / 32), taps), block (32, 8).
+__global__ void __launch_bounds__(256) split3_filter_kernel(const float* __restrict__ w, __nv_bfloat16* __restrict__ fwd,
+                                                            __nv_bfloat16* __restrict__ dx, int Cin, int Cout, int Cin_p, int Cout_p) {
+    pdl_wait();
+    __shared__ float tile[32][33];
+    const int tap = blockIdx.z, taps = gridDim.z;
+    const int n0 = blockIdx.x * 32, k0 = blockIdx.y * 32;
+    auto put = [&](__nv_bfloat16* dst, size_t plane, size_t at, float v) {
+        __nv_bfloat16 a, b, c;
+        split3(v, a, b, c);
+        dst[at] = a;
+        dst[at + plane] = b;
+        dst[at + 2 * plane] = c;
+    };
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+        const int k = k0 + threadIdx.y + 8 * r, n = n0 + threadIdx.x;
+        const float v = (k < Cin && n < Cout) ? w[((size_t)tap * Cin + k) * Cout + n] : 0.f;
+        tile[threadIdx.y + 8 * r][threadIdx.x] = v;
+        if (dx != nullptr && k < Cin && n < Cout_p) put(dx, (size_t)taps * Cin * Cout_p, ((size_t)tap * Cin + k) * Cout_p + n, v);
+    }
+    if (fwd == nullptr) return;
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+        const int n = n0 + threadIdx.y + 8 * r, k = k0 + threadIdx.x;
+        if (n < Cout && k < Cin_p) put(fwd, (size_t)taps * Cout * Cin_p, ((size_t)tap * Cout + n) * Cin_p + k, tile[threadIdx.x][threadIdx.y + 8 * r]);
+    }
+}
+
+// ====================================================================================== host side
+struct SplitPlan {
+    bool use;
+    int Ho, Wo, taps, Cin_p, Cout_p, PH, PW;      // PH, PW: a phase's extent
+    PixelTiling til_fwd, til_dx, til_dw;
+    int nt_fwd, nt_dx, splits, cblocks, U, ldn, db_blocks;
+    size_t off_wf, off_wd, off_x, off_dy, off_part, off_dbpart, total;
+};
+
+// The box of at most `most` pixels with the fewest reduction rows (tiles times rows to the next `unit`).
+static PixelTiling split_tiling(int S, int H, int W, int most, int unit) {
+    PixelTiling best{};
+    long long best_cost = -1;
+    for (int bw = 1; bw <= W && bw <= most; ++bw)
+        for (int bh = 1; bh <= H && bw * bh <= most; ++bh) {
+            int bn = bh < H ? 1 : most / (bw * bh);
+            if (bn > S) bn = S;
+            const PixelTiling t = {bw, bh, bn, bw * bh * bn, ceil_div(W, bw), ceil_div(H, bh), ceil_div(S, bn)};
+            const long long cost = t.total() * ((t.rows + unit - 1) / unit);
+            if (best_cost < 0 || cost < best_cost || (cost == best_cost && bw > best.BW)) {
+                best_cost = cost;
+                best = t;
+            }
+        }
+    return best;
+}
+
+// Column tile: the one whose rounds over the SMs are through first (a unit's time goes with its columns, but for what the
+// 128 rows' copies take).
+static int split_nt(int N, long long tiles) {
+    int best = 16;
+    double best_cost = 1e300;
+    for (int nt = 16; nt <= 128; nt += 16) {
+        const long long units = tiles * ceil_div(N, nt);
+        const double cost = (double)((units + num_sms() - 1) / num_sms()) * (48.0 + nt);
+        if (cost < best_cost - 1e-9) { best_cost = cost; best = nt; }
+    }
+    return best;
+}
+
+static SplitPlan compute_split_plan(const AetherConvDesc& d) {
+    SplitPlan pl{};
+    conv_out_hw(d, pl.Ho, pl.Wo);
+    pl.taps = d.fH * d.fW;
+    pl.Cin_p = (d.Cin + 7) / 8 * 8;
+    pl.Cout_p = (d.Cout + 7) / 8 * 8;
+    if (d.sH > 4 || d.sW > 4 || pl.taps > 64) return pl;
+    // Fewer channels leave most of a 64-channel row empty, and a small layer is through on the CUDA cores before the passes that make
+    // the parts are (forward and backward on B200, CUDA cores / split, us: 208 x 53x48 16->64 stride 2 254 / 271, 209 x 23x18
+    // 36->16 stride 2 60 / 95, 6 x 16x16 32->165 5x5, 0.7 GFLOP, 71 / 83; 24 x 18x18 48->208 stride 2, 1.05 GFLOP, 98 / 47).
+    const double flops = 6.0 * d.S * pl.Ho * pl.Wo * pl.taps * d.Cin * d.Cout;
+    if (d.Cin < 32 || d.Cout < 32 || flops < 1e9) return pl;
+    // Short reductions: nothing to gain in accuracy over the FMA kernels' (their error grows with the reduction, this one's does not).
+    if (pl.taps * d.Cin < 64 || pl.taps * d.Cout < 64) return pl;
+    pl.PH = ceil_div(d.H, d.sH);
+    pl.PW = ceil_div(d.W, d.sW);
+    const size_t in_rows = (size_t)d.sH * d.sW * d.S * pl.PH * pl.PW, out_rows = (size_t)d.S * pl.Ho * pl.Wo;
+    if ((in_rows * pl.Cin_p + out_rows * pl.Cout_p) * 6 > (2ull << 30)) return pl;      // (the parts are scratch of the caller's)
+    if (1LL * d.S * d.H * d.W * ceil_div(d.Cin > d.Cout ? d.Cin : d.Cout, 16) > 0x7fffffffLL) return pl;       // units in 32 bits
+    pl.use = true;
+    pl.til_fwd = split_tiling(d.S, pl.Ho, pl.Wo, 128, 128);
+    pl.til_dx = split_tiling(d.S, pl.PH, pl.PW, 128, 128);
+    pl.til_dw = split_tiling(d.S, pl.Ho, pl.Wo, DW_PIXELS, 16);
+    pl.nt_fwd = split_nt(d.Cout, pl.til_fwd.total());
+    pl.nt_dx = split_nt(d.Cin, pl.til_dx.total() * d.sH * d.sW);
+    pl.cblocks = ceil_div(d.Cin, SPLIT_KC);
+    pl.U = pl.taps * pl.cblocks;
+    pl.ldn = (d.Cout + 3) / 4 * 4;
+    const long long cols = 1LL * ceil_div(pl.U, 2) * ceil_div(d.Cout, 64), ptiles = pl.til_dw.total();
+    long long splits = num_sms() / cols;
+    if (splits > ptiles / 4) splits = ptiles / 4;
+    pl.splits = (int)(splits < 1 ? 1 : splits);
+    pl.db_blocks = (int)(out_rows < 4ull * num_sms() * 64 ? (out_rows + 63) / 64 : 4ull * num_sms());
+    size_t off = 0;
+    auto take = [&](size_t bytes) { size_t o = off; off = align_up(off + bytes, 1024); return o; };
+    pl.off_wf = take((size_t)3 * pl.taps * d.Cout * pl.Cin_p * 2);
+    pl.off_wd = take((size_t)3 * pl.taps * d.Cin * pl.Cout_p * 2);
+    pl.off_x = take(3 * in_rows * pl.Cin_p * 2);
+    pl.off_dy = take(3 * out_rows * pl.Cout_p * 2);
+    pl.off_part = take((size_t)pl.splits * pl.U * 64 * pl.ldn * 4);
+    pl.off_dbpart = take((size_t)pl.db_blocks * d.Cout * 4);
+    pl.total = off;
+    return pl;
+}
+static const SplitPlan& split_plan(const AetherConvDesc& d) { return cached_plan<SplitPlan, compute_split_plan>(d); }
+
+bool split_conv_eligible(const AetherConvDesc& d) { return split_plan(d).use; }
+size_t split_conv_workspace_bytes(const AetherConvDesc& d) { return split_plan(d).total; }
+
+// (C, W, H, N, part x phase) bf16, box 64 channels x the pixels of `t`.
+static int split_pixel_map(CUtensorMap* m, const void* base, int Cp, int W, int H, int N, int phases, const PixelTiling& t) {
+    const cuuint64_t row = (cuuint64_t)Cp * 2;
+    const cuuint64_t dims[5] = {(cuuint64_t)Cp, (cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)N, (cuuint64_t)3 * phases};
+    const cuuint64_t strides[4] = {row, row * W, row * W * H, row * W * H * N};
+    const cuuint32_t box[5] = {SPLIT_KC, (cuuint32_t)t.BW, (cuuint32_t)t.BH, (cuuint32_t)t.BN, 1};
+    const cuuint32_t es[5] = {1, 1, 1, 1, 1};
+    return make_map(m, base, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, dims, strides, box, es, CU_TENSOR_MAP_SWIZZLE_128B);
+}
+
+template <int NTMAX, bool DW>
+static int launch_split(const SplitParams& p, int prof, cudaStream_t st) {
+    using Cfg = SplitCfg<NTMAX, DW>;
+    static PerDeviceSmem configured;
+    if (int rc = ensure_dynamic_smem(split_conv_kernel<NTMAX, DW>, Cfg::SMEM_BYTES, configured, "split_conv")) return rc;
+    const int grid = (int)(p.units < num_sms() ? p.units : num_sms());
+    prof_begin(prof, st);
+    launch(split_conv_kernel<NTMAX, DW>, grid, SPLIT_THREADS, Cfg::SMEM_BYTES, st, p);
+    prof_end(prof, st);
+    count_launch();
+    return check_launch("split_conv_kernel");
+}
+
+static void split_geometry(SplitParams& p, const AetherConvDesc& d, const PixelTiling& t) {
+    p.S = d.S; p.fH = d.fH; p.fW = d.fW; p.sH = d.sH; p.sW = d.sW; p.pH = d.padH; p.pW = d.padW; p.Cin = d.Cin; p.Cout = d.Cout;
+    p.BW = t.BW; p.BH = t.BH; p.BN = t.BN; p.rows = t.rows; p.tiles_w = t.tiles_w; p.tiles_h = t.tiles_h; p.tiles_n = t.tiles_n;
+    p.status = device_status_word();
+}
+
+// Forward (dx false: in = x, copies of it at `cp`) and dX (in = dy).
+static int run_split_igemm(const AetherConvDesc& d, const SplitPlan& pl, bool dx, const float* in, const void* cp, const float* w, const void* wcp,
+                           const float* bias, float* out, cudaStream_t st) {
+    SplitParams p;
+    memset(&p, 0, sizeof(p));
+    const PixelTiling& t = dx ? pl.til_dx : pl.til_fwd;
+    split_geometry(p, d, t);
+    p.in = in; p.w = w; p.bias = bias; p.out = out; p.dx = dx;
+    p.IH = dx ? pl.Ho : d.H; p.IW = dx ? pl.Wo : d.W; p.IC = dx ? d.Cout : d.Cin;
+    p.OH = dx ? d.H : pl.Ho; p.OW = dx ? d.W : pl.Wo; p.N = dx ? d.Cin : d.Cout;
+    p.NT = dx ? pl.nt_dx : pl.nt_fwd;
+    p.n_tiles_n = ceil_div(p.N, p.NT);
+    p.kchunks = ceil_div(p.IC, SPLIT_KC);
+    p.last_ksteps = ceil_div(p.IC - (p.kchunks - 1) * SPLIT_KC, 16);
+    p.units = (int)(t.total() * p.n_tiles_n * (dx ? d.sH * d.sW : 1));
+    const int Cp = dx ? pl.Cout_p : pl.Cin_p;
+    if (int rc = split_pixel_map(&p.tm_a, cp, Cp, dx ? pl.Wo : pl.PW, dx ? pl.Ho : pl.PH, d.S, dx ? 1 : d.sH * d.sW, t)) return rc;
+    const cuuint64_t dims[3] = {(cuuint64_t)Cp, (cuuint64_t)p.N, (cuuint64_t)3 * pl.taps};
+    const cuuint64_t strides[2] = {(cuuint64_t)Cp * 2, (cuuint64_t)Cp * 2 * p.N};
+    const cuuint32_t box[3] = {SPLIT_KC, (cuuint32_t)p.NT, 1}, es[3] = {1, 1, 1};
+    if (int rc = make_map(&p.tm_b, wcp, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, dims, strides, box, es, CU_TENSOR_MAP_SWIZZLE_128B)) return rc;
+    const int prof = dx ? PK_IGEMM_DX : PK_IGEMM_FWD;
+    return p.NT <= 64 ? launch_split<64, false>(p, prof, st) : launch_split<128, false>(p, prof, st);
+}
+
+static int launch_split3(const float* src, void* dst, long long rows, int C, int Cp, const SplitPhases& f, float* colsum, int blocks, cudaStream_t st) {
+    const int lanes = Cp / 8 >= 256 ? 1 : 256 / (Cp / 8);
+    __nv_bfloat16* out = static_cast<__nv_bfloat16*>(dst);
+    prof_begin(PK_SHADOW, st);
+    if (colsum) {
+        launch(split3_kernel<true, false>, blocks, 256, 0, st, src, out, rows, C, Cp, colsum, (rows + blocks - 1) / blocks, f);
+    } else {
+        long long nb = 8LL * num_sms();
+        if (nb * lanes > rows) nb = (rows + lanes - 1) / lanes;
+        const long long per = (rows + nb - 1) / nb;
+        launch(f.sH * f.sW > 1 ? split3_kernel<false, true> : split3_kernel<false, false>, (int)nb, 256, 0, st, src, out, rows, C, Cp, nullptr, per, f);
+    }
+    prof_end(PK_SHADOW, st);
+    count_launch();
+    return check_launch("split3_kernel");
+}
+// The parts of x, by phases.
+static int split_x(const AetherConvDesc& d, const SplitPlan& pl, const float* x, void* dst, cudaStream_t st) {
+    const SplitPhases f = {d.H, d.W, d.sH, d.sW, pl.PH, pl.PW, 1LL * d.S * pl.PH * pl.PW};
+    return launch_split3(x, dst, f.images * d.sH * d.sW, d.Cin, pl.Cin_p, f, nullptr, 0, st);
+}
+
+static int launch_split3_filter(const AetherConvDesc& d, const SplitPlan& pl, const float* w, void* fwd, void* dx, cudaStream_t st) {
+    const dim3 grid((unsigned)ceil_div(pl.Cout_p, 32), (unsigned)ceil_div(pl.Cin_p, 32), (unsigned)pl.taps);
+    launch(split3_filter_kernel, grid, dim3(32, 8), 0, st, w, static_cast<__nv_bfloat16*>(fwd), static_cast<__nv_bfloat16*>(dx), d.Cin, d.Cout,
+           pl.Cin_p, pl.Cout_p);
+    count_launch();
+    return check_launch("split3_filter_kernel");
+}
+
+int split_conv_fwd(const AetherConvDesc& d, const float* x, const float* w, const float* b, float* y, void* ws, cudaStream_t st) {
+    const SplitPlan& pl = split_plan(d);
+    uint8_t* wsb = static_cast<uint8_t*>(ws);
+    if (int rc = split_x(d, pl, x, wsb + pl.off_x, st)) return rc;
+    if (int rc = launch_split3_filter(d, pl, w, wsb + pl.off_wf, wsb + pl.off_wd, st)) return rc;
+    return run_split_igemm(d, pl, false, x, wsb + pl.off_x, w, wsb + pl.off_wf, b, y, st);
+}
+
+int split_conv_bwd(const AetherConvDesc& d, const float* x, const float* dy, const float* w, float* dx, float* dw, float* db, void* ws,
+                   int copies_valid, cudaStream_t st) {
+    const SplitPlan& pl = split_plan(d);
+    uint8_t* wsb = static_cast<uint8_t*>(ws);
+    float* dbpart = reinterpret_cast<float*>(wsb + pl.off_dbpart);
+    int rc;
+    if ((rc = launch_split3(dy, wsb + pl.off_dy, 1LL * d.S * pl.Ho * pl.Wo, d.Cout, pl.Cout_p, SplitPhases{0, 0, 1, 1, 0, 0, 0}, db ? dbpart : nullptr, pl.db_blocks, st))) return rc;
+    if (dx) {
+        if (!(copies_valid & AETHER_CONV_W_COPY_READY) && (rc = launch_split3_filter(d, pl, w, nullptr, wsb + pl.off_wd, st))) return rc;
+        if ((rc = run_split_igemm(d, pl, true, dy, wsb + pl.off_dy, w, wsb + pl.off_wd, nullptr, dx, st))) return rc;
+    }
+    if (!dw) return db ? colsum_finish(dbpart, pl.db_blocks, d.Cout, db, st) : AE_OK;
+    if (!(copies_valid & AETHER_CONV_X_COPY_READY) && (rc = split_x(d, pl, x, wsb + pl.off_x, st)))
+        return rc;
+    SplitParams p;
+    memset(&p, 0, sizeof(p));
+    const PixelTiling& t = pl.til_dw;
+    split_geometry(p, d, t);
+    p.in = x; p.w = dy; p.out = reinterpret_cast<float*>(wsb + pl.off_part);
+    p.IH = d.H; p.IW = d.W; p.IC = d.Cin; p.OH = pl.Ho; p.OW = pl.Wo; p.N = d.Cout;
+    p.NT = 64;
+    p.n_tiles_n = ceil_div(d.Cout, p.NT);
+    p.U = pl.U; p.cblocks = pl.cblocks; p.splits = pl.splits; p.ldn = pl.ldn;
+    p.ksteps = ceil_div(t.rows, 16);
+    p.kchunks = 1;
+    p.units = ceil_div(p.U, 2) * p.n_tiles_n * p.splits;
+    if ((rc = split_pixel_map(&p.tm_a, wsb + pl.off_x, pl.Cin_p, pl.PW, pl.PH, d.S, d.sH * d.sW, t))) return rc;
+    if ((rc = split_pixel_map(&p.tm_b, wsb + pl.off_dy, pl.Cout_p, pl.Wo, pl.Ho, d.S, 1, t))) return rc;
+    if ((rc = launch_split<64, true>(p, PK_DW, st))) return rc;
+    return dw_reduce(p.out, dw, p.splits, p.U, 64, p.ldn, p.cblocks, pl.taps, d.Cin, d.Cout, pl.taps, p.splits, dbpart, pl.db_blocks, db, st);
+}
+
+}  // namespace aether

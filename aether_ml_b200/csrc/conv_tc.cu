@@ -26,13 +26,6 @@
 namespace aether {
 
 // ====================================================================================== tiling
-// One M tile is a box of BN images x BH rows x BW columns of output pixels, at most 128 of them.
-struct PixelTiling {
-    int BW, BH, BN, rows;
-    int tiles_w, tiles_h, tiles_n;
-    long long total() const { return 1LL * tiles_w * tiles_h * tiles_n; }
-};
-
 // Columns of the halo kernel's accumulator: the output channels to the next 32 (the per-tap kernel's tiles are powers of two).
 static int halo_n(int out_C, int n_padded) {
     const int n = (out_C + 31) / 32 * 32;
@@ -77,37 +70,34 @@ static EncodeTiledFn encode_fn() {
     return fn;
 }
 
+int make_map(CUtensorMap* m, const void* base, CUtensorMapDataType dt, int rank, const cuuint64_t* dims, const cuuint64_t* strides,
+             const cuuint32_t* box, const cuuint32_t* estr, CUtensorMapSwizzle swz) {
+    EncodeTiledFn fn = encode_fn();
+    if (!fn) return set_error(AE_CUDA, "cuTensorMapEncodeTiled entry point not available");
+    CUresult r = fn(m, dt, rank, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swz,
+                    CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS)
+        return set_error(AE_CUDA, "cuTensorMapEncodeTiled(rank %d, %llu x %llu.., box %u x %u..) failed: %d", rank,
+                         (unsigned long long)dims[0], (unsigned long long)dims[1], box[0], box[1], (int)r);
+    return AE_OK;
+}
 // NHWC tensor seen as 4-D (C, W, H, N), 128-byte swizzle, box (box_c, BW, BH, BN).
 int make_map_nhwc(CUtensorMap* m, const void* base, CUtensorMapDataType dt, int elt, int C, int W, int H, int N, int box_c,
                   int BW, int BH, int BN, CUtensorMapSwizzle swz) {
-    EncodeTiledFn fn = encode_fn();
-    if (!fn) return set_error(AE_CUDA, "cuTensorMapEncodeTiled entry point not available");
-    cuuint64_t dims[4] = {(cuuint64_t)C, (cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)N};
-    cuuint64_t strides[3] = {(cuuint64_t)C * elt, (cuuint64_t)C * elt * W, (cuuint64_t)C * elt * W * H};
-    cuuint32_t box[4] = {(cuuint32_t)box_c, (cuuint32_t)BW, (cuuint32_t)BH, (cuuint32_t)BN};
-    cuuint32_t es[4] = {1, 1, 1, 1};
-    CUresult r = fn(m, dt, 4, const_cast<void*>(base), dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, swz,
-                    CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS)
-        return set_error(AE_CUDA, "cuTensorMapEncodeTiled(4d C=%d W=%d H=%d N=%d box %d,%d,%d,%d) failed: %d", C, W, H,
-                         N, box_c, BW, BH, BN, (int)r);
-    return AE_OK;
+    const cuuint64_t dims[4] = {(cuuint64_t)C, (cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)N};
+    const cuuint64_t strides[3] = {(cuuint64_t)C * elt, (cuuint64_t)C * elt * W, (cuuint64_t)C * elt * W * H};
+    const cuuint32_t box[4] = {(cuuint32_t)box_c, (cuuint32_t)BW, (cuuint32_t)BH, (cuuint32_t)BN};
+    const cuuint32_t es[4] = {1, 1, 1, 1};
+    return make_map(m, base, dt, 4, dims, strides, box, es, swz);
 }
 // Row-major matrix (inner = K elements contiguous, `rows` rows), box (box_k, box_rows).
 int make_map_2d(CUtensorMap* m, const void* base, CUtensorMapDataType dt, int elt, int inner, long long rows, int box_k,
                 int box_rows) {
-    EncodeTiledFn fn = encode_fn();
-    if (!fn) return set_error(AE_CUDA, "cuTensorMapEncodeTiled entry point not available");
-    cuuint64_t dims[2] = {(cuuint64_t)inner, (cuuint64_t)rows};
-    cuuint64_t strides[1] = {(cuuint64_t)inner * elt};
-    cuuint32_t box[2] = {(cuuint32_t)box_k, (cuuint32_t)box_rows};
-    cuuint32_t es[2] = {1, 1};
-    CUresult r = fn(m, dt, 2, const_cast<void*>(base), dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                    CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS)
-        return set_error(AE_CUDA, "cuTensorMapEncodeTiled(2d inner=%d rows=%lld box %d,%d) failed: %d", inner, rows,
-                         box_k, box_rows, (int)r);
-    return AE_OK;
+    const cuuint64_t dims[2] = {(cuuint64_t)inner, (cuuint64_t)rows};
+    const cuuint64_t strides[1] = {(cuuint64_t)inner * elt};
+    const cuuint32_t box[2] = {(cuuint32_t)box_k, (cuuint32_t)box_rows};
+    const cuuint32_t es[2] = {1, 1};
+    return make_map(m, base, dt, 2, dims, strides, box, es, CU_TENSOR_MAP_SWIZZLE_128B);
 }
 
 // ====================================================================================== igemm (forward and dX)
@@ -824,10 +814,11 @@ __device__ __forceinline__ void finish_columns(const float* __restrict__ part, i
 
 // dW[tap][c][d] = sum over splits of part[split][tap*cblocks + c/UC][c%UC][d]
 // Taps from tap_split on have splits2 partials instead of splits (kernels whose CTA classes differ in number).
-// Four consecutive output channels per thread; 1 << lane_bits threads share an output, thread l of them adds splits l,
+// V consecutive output channels per thread; 1 << lane_bits threads share an output, thread l of them adds splits l,
 // l + lanes, ... and they are combined in fixed order through shared memory (bit-reproducible).  Bound by L2: what counts is
 // loads in flight, so lanes are used only where there are few outputs (dw_reduce_lane_bits).
 // `nred` CTAs do that; the CTAs behind them finish dB, which saves a launch of its own.
+template <int V>
 __global__ void __launch_bounds__(256) dw_reduce_kernel(const float* __restrict__ part, float* __restrict__ dw, int splits,
                                                         int U, int UC, int ldn, int cblocks, int taps, int Cin, int Cout,
                                                         int tap_split, int splits2, int lane_bits, int nred,
@@ -840,14 +831,14 @@ __global__ void __launch_bounds__(256) dw_reduce_kernel(const float* __restrict_
     }
     const int per = 256 >> lane_bits, lanes = 1 << lane_bits;       // outputs of a CTA, threads per output
     const int el = threadIdx.x & (per - 1), ln = threadIdx.x >> (8 - lane_bits);
-    const int Cq = Cout >> 2;                          // (Cout % 4 == 0, ldn a multiple of 32)
+    const int Cq = Cout / V;                           // (V == 4: Cout % 4 == 0; ldn a multiple of 4)
     const long long total4 = 1LL * taps * Cin * Cq;
     const size_t split_stride = (size_t)U * UC * ldn;
     for (long long base = 1LL * blockIdx.x * per; base < total4; base += 1LL * nred * per) {
         const long long i4 = base + el;
         float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
         if (i4 < total4) {
-            const int d = (int)(i4 % Cq) * 4;
+            const int d = (int)(i4 % Cq) * V;
             const long long tc = i4 / Cq;
             const int c = (int)(tc % Cin);
             const int tap = (int)(tc / Cin);
@@ -856,8 +847,12 @@ __global__ void __launch_bounds__(256) dw_reduce_kernel(const float* __restrict_
             const int ns = tap < tap_split ? splits : splits2;
 #pragma unroll 8
             for (int s = ln; s < ns; s += lanes) {
-                const float4 v = *reinterpret_cast<const float4*>(src + s * split_stride);
-                acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
+                if constexpr (V == 4) {
+                    const float4 v = *reinterpret_cast<const float4*>(src + s * split_stride);
+                    acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
+                } else {
+                    acc.x += src[s * split_stride];
+                }
             }
         }
         if (lanes > 1) {
@@ -867,22 +862,30 @@ __global__ void __launch_bounds__(256) dw_reduce_kernel(const float* __restrict_
                 for (int l = 1; l < lanes; ++l) { const float4 v = red4[l * per + el]; acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w; }
             __syncthreads();
         }
-        if (ln == 0 && i4 < total4) *reinterpret_cast<float4*>(dw + i4 * 4) = acc;
+        if (ln == 0 && i4 < total4) {
+            if constexpr (V == 4) *reinterpret_cast<float4*>(dw + i4 * 4) = acc;
+            else dw[i4] = acc.x;
+        }
     }
 }
 
 // Threads per output: enough for some 64K threads (128 blocks of 16 warps), at most eight and no more than splits.
-static int dw_reduce_lane_bits(int taps, int Cin, int Cout, int splits) {
-    const long long total4 = 1LL * taps * Cin * (Cout / 4);
+static int dw_reduce_lane_bits(long long outputs, int splits) {
     int bits = 0;
-    while (bits < 3 && (total4 << bits) < 65536 && (2 << bits) <= splits) ++bits;
+    while (bits < 3 && (outputs << bits) < 65536 && (2 << bits) <= splits) ++bits;
     return bits;
 }
-static int dw_reduce_grid(int taps, int Cin, int Cout, int lane_bits) {
-    const long long per = 256 >> lane_bits;
-    const long long groups = (1LL * taps * Cin * (Cout / 4) + per - 1) / per;
-    const long long cap = 8LL * num_sms();
-    return (int)(groups < cap ? groups : cap);
+int dw_reduce(const float* part, float* dw, int splits, int U, int UC, int ldn, int cblocks, int taps, int Cin, int Cout, int tap_split,
+              int splits2, const float* dbpart, int db_rows, float* db, cudaStream_t st) {
+    const bool v4 = Cout % 4 == 0;
+    const long long outputs = 1LL * taps * Cin * (v4 ? Cout / 4 : Cout);
+    const int bits = dw_reduce_lane_bits(outputs, splits);
+    const long long per = 256 >> bits, groups = (outputs + per - 1) / per, cap = 8LL * num_sms();
+    const int nred = (int)(groups < cap ? groups : cap);
+    launch(v4 ? dw_reduce_kernel<4> : dw_reduce_kernel<1>, nred + (db ? ceil_div(Cout, 8) : 0), 256, 0, st, part, dw, splits, U, UC, ldn, cblocks,
+           taps, Cin, Cout, tap_split, splits2, bits, nred, dbpart, db_rows, db);
+    count_launch();
+    return check_launch("dw_reduce_kernel");
 }
 
 // ====================================================================================== shadow copies
@@ -1232,28 +1235,7 @@ static TcPlan compute_plan(const AetherConvDesc& d) {
     return pl;
 }
 
-// The tile search above costs some ten microseconds of host time, as much as the launches of a small layer, and a
-// network asks for the same few shapes again on every pass (workspace size, operand layout, statistics blocks, forward,
-// backward): each host thread keeps the plans it used last, direct-mapped.  A plan depends on the shape and the device only.
-static const TcPlan& make_plan(const AetherConvDesc& d) {
-    struct Slot {
-        AetherConvDesc key;
-        int dev = -1;
-        TcPlan plan;
-    };
-    static thread_local Slot slots[64];
-    const int dev = current_device();
-    uint32_t h = 2166136261u;
-    const int32_t* f = reinterpret_cast<const int32_t*>(&d);
-    for (size_t i = 0; i < sizeof(d) / sizeof(int32_t); ++i) h = (h ^ (uint32_t)f[i]) * 16777619u;
-    Slot& s = slots[(h ^ (h >> 16)) & 63u];
-    if (s.dev != dev || memcmp(&s.key, &d, sizeof(d)) != 0) {
-        s.plan = compute_plan(d);
-        s.key = d;
-        s.dev = dev;
-    }
-    return s.plan;
-}
+static const TcPlan& make_plan(const AetherConvDesc& d) { return cached_plan<TcPlan, compute_plan>(d); }
 
 bool tc_conv_eligible(const AetherConvDesc& d) {
     if (d.math_mode != AETHER_MATH_BF16 && d.math_mode != AETHER_MATH_TF32) return false;
@@ -1548,13 +1530,9 @@ int tc_conv_bwd(const AetherConvDesc& d, const float* x, const float* dy, const 
     // ---- dW: split over pixel tiles, fixed-order reduction of the partials
     bool dw_done = false, db_done = db == nullptr;
     auto reduce_dw = [&](const float* part, int splits, int tap_split, int splits2) {
-        const int bits = dw_reduce_lane_bits(pl.taps, d.Cin, d.Cout, splits);
-        const int nred = dw_reduce_grid(pl.taps, d.Cin, d.Cout, bits);
-        launch(dw_reduce_kernel, nred + (db ? ceil_div(d.Cout, 8) : 0), 256, 0, st, part, dw, splits, pl.dw_U, pl.KC, pl.Cout_p,
-               pl.dw_cblocks, pl.taps, d.Cin, d.Cout, tap_split, splits2, bits, nred, dbpart, db_rows, db);
         db_done = true;
-        count_launch();
-        return check_launch("dw_reduce_kernel");
+        return dw_reduce(part, dw, splits, pl.dw_U, pl.KC, pl.Cout_p, pl.dw_cblocks, pl.taps, d.Cin, d.Cout, tap_split, splits2, dbpart,
+                         db_rows, db, st);
     };
     // Which dW kernel (bf16).  The kernels that reuse a shared-memory window across the taps win on wide images; on
     // 16..20-pixel rows the per-tap kernel on CTA pairs is faster (a fifth of such a window is halo).  Measured on B200,

@@ -2,8 +2,42 @@
 #pragma once
 #include <cuda.h>
 #include <cuda_runtime.h>
+#include <string.h>
+
+#include "common.cuh"
 
 namespace aether {
+
+// One M tile is a box of BN images x BH rows x BW columns of output pixels.
+struct PixelTiling {
+    int BW, BH, BN, rows;
+    int tiles_w, tiles_h, tiles_n;
+    long long total() const { return 1LL * tiles_w * tiles_h * tiles_n; }
+};
+
+// The plan of a shape: working one out costs some ten microseconds of host time, as much as the launches of a small layer,
+// and a network asks for the same few shapes again on every pass (workspace size, operand layout, statistics blocks, forward,
+// backward): each host thread keeps the plans it used last, direct-mapped.  A plan depends on the shape and the device only.
+template <typename Plan, Plan (*COMPUTE)(const AetherConvDesc&)>
+const Plan& cached_plan(const AetherConvDesc& d) {
+    struct Slot {
+        AetherConvDesc key;
+        int dev = -1;
+        Plan plan;
+    };
+    static thread_local Slot slots[64];
+    const int dev = current_device();
+    uint32_t h = 2166136261u;
+    const int32_t* f = reinterpret_cast<const int32_t*>(&d);
+    for (size_t i = 0; i < sizeof(d) / sizeof(int32_t); ++i) h = (h ^ (uint32_t)f[i]) * 16777619u;
+    Slot& s = slots[(h ^ (h >> 16)) & 63u];
+    if (s.dev != dev || memcmp(&s.key, &d, sizeof(d)) != 0) {
+        s.plan = COMPUTE(d);
+        s.key = d;
+        s.dev = dev;
+    }
+    return s.plan;
+}
 
 int num_sms();
 // Whether this device can co-schedule the CTA pairs (clusters of two CTAs with ~210 KB of shared memory each) the
@@ -12,6 +46,9 @@ bool cta_pairs_available();
 // NHWC tensor seen as 4-D (C, W, H, N), box (box_c, BW, BH, BN); 128-byte swizzle unless told otherwise.
 int make_map_nhwc(CUtensorMap* m, const void* base, CUtensorMapDataType dt, int elt, int C, int W, int H, int N,
                   int box_c, int BW, int BH, int BN, CUtensorMapSwizzle swz = CU_TENSOR_MAP_SWIZZLE_128B);
+// Tensor map of any rank: sizes, byte strides of all dimensions but the innermost, box and element strides.
+int make_map(CUtensorMap* m, const void* base, CUtensorMapDataType dt, int rank, const cuuint64_t* dims, const cuuint64_t* strides,
+             const cuuint32_t* box, const cuuint32_t* estr, CUtensorMapSwizzle swz);
 // Row-major matrix (inner = K elements contiguous, `rows` rows), box (box_k, box_rows), 128-byte swizzle.
 int make_map_2d(CUtensorMap* m, const void* base, CUtensorMapDataType dt, int elt, int inner, long long rows, int box_k,
                 int box_rows);
@@ -35,6 +72,11 @@ int rows_dw_max_splits(int Cin_p, int Cout_p, int Ho, int Wo, int S, int fH, int
 int run_rows_dw(const void* x_sh, int Cin_p, int H, int W, int S, const void* dy_sh, int Cout_p, int Ho, int Wo, int fH,
                 int fW, int padH, int padW, float* part, int* splits_a, int* splits_b, int* tap_split, cudaStream_t st,
                 bool* used);
+
+// dw[tap][c][d] = sum over splits of part[split][tap * cblocks + c / UC][c % UC][d] (rows of `ldn`, a multiple of 4) and, when
+// asked for, db from `db_rows` rows of column sums (conv_tc.cu).
+int dw_reduce(const float* part, float* dw, int splits, int U, int UC, int ldn, int cblocks, int taps, int Cin, int Cout, int tap_split,
+              int splits2, const float* dbpart, int db_rows, float* db, cudaStream_t st);
 
 // MMAs (32 bytes of K each) that the last of `kchunks` 128-byte chunks needs when only k_real of the channels are not padding.
 static inline int last_ksteps(int k_real, int kchunks, int KC) {

@@ -37,8 +37,10 @@ extern "C" {
 /* Operand precision of the convolution GEMMs (accumulation is always fp32). */
 #define AETHER_MATH_BF16 0 /* bf16 operands on the tensor cores (tcgen05 kind::f16)            */
 #define AETHER_MATH_TF32 1 /* tf32 operands on the tensor cores (tcgen05 kind::tf32)           */
-#define AETHER_MATH_FP32 2 /* fp32 FMA on the CUDA cores (also used for shapes the tensor path   */
-                           /* does not take: stride > 1, Cin or Cout < 16 or not a multiple of 4) */
+#define AETHER_MATH_FP32 2 /* single precision (also used for shapes the tensor path does not    */
+                           /* take: stride > 1, Cin or Cout < 16 or not a multiple of 4): FMAs   */
+                           /* on the CUDA cores or, for larger layers with a workspace, tensor   */
+                           /* cores on operands split into three bf16 numbers, which is closer   */
 
 #define AETHER_POOL_MAX 0
 #define AETHER_POOL_AVG 1
