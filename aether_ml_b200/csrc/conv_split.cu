@@ -6,11 +6,11 @@
 //
 // Accuracy.  tcgen05 adds in fp32 but truncates after every step of 16 products (measured: one step keeps 25 fractional bits; the
 // error of a plain bf16 sum of 2048 exact products is 2.1e-6 and biased, 18 times an FMA loop's), so a sum stays in TMEM for
-// GROUP_STEPS steps only: the x0 w0 products of each group go to an accumulator of their own that the epilogue warps add to their running
-// sums in registers (rounding to nearest) while the next groups are multiplied.  The products of second and third
+// four steps only: the x0 w0 products of each stage go to an accumulator of their own that the epilogue warps add to their running
+// sums in registers (rounding to nearest) while the next stages are multiplied.  The products of second and third
 // order are 2^-8 and 2^-16 of that and stay in two accumulators of their own for up to EPOCH_STAGES stages.  Relative error against
-// float64, FMA kernels / this one: 96 x 28x28 32->64 y 3.0e-7 / 8.2e-8, dX 4.2e-7 / 9.6e-8, dW 3.8e-7 / 2.6e-7, and no larger in
-// any of forty drawn layers.  An
+// float64, FMA kernels / this one: 96 x 28x28 32->64 y 3.0e-7 / 8.2e-8, dX 4.2e-7 / 9.5e-8, dW 3.8e-7 / 1.4e-7, and smaller in
+// all of forty drawn layers.  An
 // output that is not finite (an infinite or NaN operand has no meaningful remainder, one above 3.39e38 rounds to infinity) is
 // summed again by FMAs from the fp32 arrays.  Operands below 2^-109 keep fewer than 24 bits (the last part is subnormal).
 //
@@ -20,11 +20,14 @@
 // parts are made by a pass over x and dy (split3_kernel: 4 bytes read, 6 written, dB on the way) and copied by TMA, rows of 64
 // channels with zeros behind the last: channel counts need not be multiples of anything.  A strided layer's x is stored by
 // phases, so that a tap's pixels lie side by side (element strides in the tensor map halve the copies' rate).
-// Measured on B200, forward + backward, CUDA cores / this file: 40 x 33x32 64->128 444 / 156 us, 96 x 28x28 32->64 209 / 156, 100 x 57x45
-// 48->72 stride 2 432 / 272.  Bound by the operands' way from L2 into shared memory (some 60 bytes a clock and SM).
+// Measured on B200, forward + backward, CUDA cores / this file: 40 x 33x32 64->128 444 / 118 us, 96 x 28x28 32->64 209 / 105, 100 x 57x45
+// 48->72 stride 2 432 / 199.  Bound by shared memory: the MMAs' operand reads (28 KB per step of 64 columns, 219 clocks) and the copies'
+// writes (16-18 KB) share its 128 bytes a clock.
 #include <string.h>
 
 #include <cuda_bf16.h>
+
+#include <type_traits>
 
 #include "common.cuh"
 #include "sm100_ptx.cuh"
@@ -32,20 +35,38 @@
 
 namespace aether {
 
-static constexpr int SPLIT_KC = 64;             // channels per row of a tile (128 bytes)
-static constexpr int GROUP_STEPS = 2;           // steps of 16 products whose sum may stay in TMEM; a stage is two groups
+static constexpr int SPLIT_KC = 64;             // most channels per row of a tile (128 bytes)
 static constexpr int EPOCH_STAGES = 32;         // stages after which the small products' sums leave TMEM, too
 static constexpr int SPLIT_EPI_WARPS = 8;       // 4 TMEM lane quarters x 2 (16-column blocks taken in turn)
 static constexpr int SPLIT_THREADS = 128 + 32 * SPLIT_EPI_WARPS;     // warps 0 and 1 copy, 2 and 3 multiply, the others add and store
 static constexpr int DW_PIXELS = 64;            // pixel rows per stage of dW
 
+// Quotients by a number known at launch (multiplication and shift; dividends below 2^31): the roles of the kernel decode their units by them
+// again and again, and an integer division is some 40 instructions.
+struct SplitDiv {
+    uint32_t d, mul, shift;
+};
+static SplitDiv split_div(uint32_t d) {
+    uint32_t shift = 0;
+    while ((1ull << shift) < d) ++shift;
+    return {d, (uint32_t)((((1ull << shift) - d) << 32) / d + 1), shift};
+}
+__device__ __forceinline__ int split_quot(int n, const SplitDiv& d) { return (int)((__umulhi((uint32_t)n, d.mul) + (uint32_t)n) >> d.shift); }
+
+// A pixel class of dX: output rows h = hs + a * sH see the taps i = ph + ti * sH at input row a + hq - ti.  (Forward: one class.)
+struct SplitClass {
+    int16_t ph, pw, nH, nW, hs, ws, hq, wq;
+    int MH, MW;
+};
+static constexpr int SPLIT_MOST_STRIDE = 4;
+
 struct SplitParams {
-    CUtensorMap tm_a;     // igemm: pixels (C, W, H, N, part x phase), box 64 x BW x BH x BN; dW: x
-    CUtensorMap tm_b;     // igemm: filter (K, columns, part x tap), box 64 x NT; dW: dy (C, W, H, N, part)
+    CUtensorMap tm_a;     // igemm: pixels (C, W, H, N, part x phase), box KC x BW x BH x BN; dW: x
+    CUtensorMap tm_b;     // igemm: filter (K, columns, part x tap), box KC x NT; dW: dy (C, W, H, N, part)
     const float* in;      // the fp32 arrays behind them, for outputs that are not finite; dW: x
     const float* w;       // filter (taps, Cin, Cout); dW: dy
     const float* bias;    // nullable
-    float* out;           // dW: partial sums [split][U][64][ldn]
+    float* out;           // dW: partial sums [split][U][KC][ldn]
     int* status;
     int IH, IW, IC;       // extent of `in`
     int OH, OW, S;        // extent of the output pixels (dW: of dy)
@@ -56,42 +77,27 @@ struct SplitParams {
     int NT, n_tiles_n;    // column tile (a multiple of 16; dW: 64)
     int kchunks, last_ksteps;
     int units;
-    int U, cblocks, splits, ksteps, ldn;      // dW: units of 64 filter rows (tap, 64 channels), pixel splits, steps per stage
+    SplitDiv by_ntn, by_tiles, by_tw, by_th, by_groups;     // column tiles, pixel tiles, tile columns, tile rows, groups of row units
+    SplitClass cls[SPLIT_MOST_STRIDE * SPLIT_MOST_STRIDE];
+    int U, cblocks, splits, ksteps, ldn;      // dW: units of KC filter rows (tap, KC channels), pixel splits, steps per stage
 };
 
-template <int NTMAX, bool DW>
+// KC: channels per row of a tile, 64 or 32 (64-byte swizzle).  A stage is KC channels of a tap or, in dW, a box of pixels: at most four steps
+// of 16 products, whose x0 w0 sum leaves TMEM then.
+template <int NTMAX, bool DW, int KC>
 struct SplitCfg {
-    static constexpr int A_PART = DW ? 2 * DW_PIXELS * 128 : 128 * 128;     // bytes of one part of the 128 accumulator rows' operand
+    static constexpr int ROW = KC * 2;                                      // bytes
+    static constexpr int UNITS = 128 / KC;                                  // dW: row units of the 128 accumulator rows
+    static constexpr int A_PART = DW ? UNITS * DW_PIXELS * ROW : 128 * ROW; // one part of the 128 accumulator rows' operand
     static constexpr int STAGE_A = 3 * A_PART;
-    static constexpr int STAGE_B = 3 * NTMAX * (DW ? 2 * DW_PIXELS : 128);
-    static constexpr int STAGES = (216 * 1024) / (STAGE_A + STAGE_B);
+    static constexpr int STAGE_B = 3 * NTMAX * (DW ? 2 * DW_PIXELS : ROW);  // (dW: 64 channels of dy per row)
+    static constexpr int FIT = (216 * 1024) / (STAGE_A + STAGE_B), STAGES = FIT < 6 ? FIT : 6;
     static constexpr int SMEM_BYTES = 1024 + STAGES * (STAGE_A + STAGE_B) + 256;
-    static constexpr int NBG = NTMAX <= 64 ? 2 : 1;             // accumulators of a stage's two groups
+    static constexpr int NBG = NTMAX <= 64 ? 4 : 2;             // accumulators of a stage's x0 w0
     static constexpr int NBC = NTMAX <= 64 ? 2 : 1;             // accumulator pairs of the small products
     static constexpr int BLOCKS = NTMAX / 32;                   // 16-column blocks of an epilogue warp
-    static_assert((NBG + NBC) * 2 * NTMAX <= 512 && STAGES >= 2, "TMEM, shared memory");
+    static_assert((NBG + NBC * 2) * NTMAX <= 512 && STAGES >= 2, "TMEM, shared memory");
 };
-
-// A pixel class of dX: output rows h = hs + a * sH see the taps i = ph + ti * sH at input row a + hq - ti.  (Forward: one class.)
-struct SplitClass {
-    int ph, pw, nH, nW, hs, ws, hq, wq, MH, MW;
-};
-__device__ __forceinline__ SplitClass split_class(const SplitParams& p, int cls) {
-    SplitClass c = {0, 0, p.fH, p.fW, 0, 0, 0, 0, p.OH, p.OW};
-    if (p.dx) {
-        c.ph = cls / p.sW;
-        c.pw = cls - c.ph * p.sW;
-        c.nH = c.ph < p.fH ? (p.fH - c.ph - 1) / p.sH + 1 : 0;
-        c.nW = c.pw < p.fW ? (p.fW - c.pw - 1) / p.sW + 1 : 0;
-        c.hs = ((c.ph - p.pH) % p.sH + p.sH) % p.sH;
-        c.ws = ((c.pw - p.pW) % p.sW + p.sW) % p.sW;
-        c.hq = (c.hs + p.pH - c.ph) / p.sH;
-        c.wq = (c.ws + p.pW - c.pw) / p.sW;
-        c.MH = c.hs < p.OH ? (p.OH - c.hs - 1) / p.sH + 1 : 0;
-        c.MW = c.ws < p.OW ? (p.OW - c.ws - 1) / p.sW + 1 : 0;
-    }
-    return c;
-}
 
 // Row (column) offset `a` of a tap against stride `s`: the phase of the input pixels it reads, and where in them.
 __device__ __forceinline__ void split_phase(int a, int s, int& phase, int& at) {
@@ -122,10 +128,10 @@ __device__ float split_direct(const SplitParams& p, int n, int h, int w, int col
 
 // Pixel tile `t` of p's tiling: first column, row and image.
 __device__ __forceinline__ void split_tile_origin(const SplitParams& p, int t, int& w0, int& h0, int& n0) {
-    const unsigned u = (unsigned)t, a = u / (unsigned)p.tiles_w, n = a / (unsigned)p.tiles_h;
-    w0 = (int)(u - a * (unsigned)p.tiles_w) * p.BW;
-    h0 = (int)(a - n * (unsigned)p.tiles_h) * p.BH;
-    n0 = (int)n * p.BN;
+    const int a = split_quot(t, p.by_tw), n = split_quot(a, p.by_th);
+    w0 = (t - a * p.tiles_w) * p.BW;
+    h0 = (a - n * p.tiles_h) * p.BH;
+    n0 = n * p.BN;
 }
 
 // The same for an entry (filter row i, column j, channel c; output channel d) of a split's partial filter gradient.
@@ -146,15 +152,15 @@ __device__ float split_direct_dw(const SplitParams& p, int t0, int t1, int i, in
 
 // Row `r` of a unit's 128, pixel (b, a, n) of its box: where it goes (null: nowhere) and what it is (igemm: output column, row, image;
 // dW: filter column, filter row, channel).
-template <bool DW>
+template <bool DW, int KC>
 __device__ __forceinline__ float* split_row(const SplitParams& p, int mt, int cls, const SplitClass& c, int w0, int h0, int n0, int r, int b, int a,
                                             int n, int& x_w, int& x_h, int& x_n) {
     if (DW) {
-        const int unit = mt * 2 + r / 64, tap = unit / p.cblocks;
+        const int unit = mt * (128 / KC) + r / KC, tap = unit / p.cblocks;
         x_h = tap / p.fW;
         x_w = tap - x_h * p.fW;
-        x_n = (unit - tap * p.cblocks) * 64 + r % 64;
-        return (unit < p.U && x_n < p.Cin) ? p.out + (((size_t)cls * p.U + unit) * 64 + r % 64) * p.ldn : nullptr;
+        x_n = (unit - tap * p.cblocks) * KC + r % KC;
+        return (unit < p.U && x_n < p.Cin) ? p.out + (((size_t)cls * p.U + unit) * KC + r % KC) * p.ldn : nullptr;
     }
     const int w = w0 + b, h = h0 + a;
     x_n = n0 + n;
@@ -164,14 +170,14 @@ __device__ __forceinline__ float* split_row(const SplitParams& p, int mt, int cl
 }
 
 // What this lane stored for a unit and is not finite, again by FMAs.
-template <bool DW>
+template <bool DW, int KC>
 __device__ __noinline__ void split_repair(const SplitParams& p, int nt, int mt, int cls, int t0, int t1, int q, int part, int lane) {
     int w0 = 0, h0 = 0, n0 = 0, x_w, x_h, x_n;
-    const SplitClass c = split_class(p, cls);
+    const SplitClass& c = p.cls[DW ? 0 : cls];
     if (!DW) split_tile_origin(p, mt, w0, h0, n0);
     for (int j = 0; j < 4; ++j) {
         const int r = q * 32 + (lane & ~3) + j;
-        float* row = split_row<DW>(p, mt, cls, c, w0, h0, n0, r, r % p.BW, r / p.BW % p.BH, r / (p.BW * p.BH), x_w, x_h, x_n);
+        float* row = split_row<DW, KC>(p, mt, cls, c, w0, h0, n0, r, r % p.BW, r / p.BW % p.BH, r / (p.BW * p.BH), x_w, x_h, x_n);
         if (row == nullptr) continue;
         for (int b = part; b * 16 < p.NT; b += 2)
             for (int e = 0; e < 4; ++e) {
@@ -183,18 +189,19 @@ __device__ __noinline__ void split_repair(const SplitParams& p, int nt, int mt, 
     }
 }
 
-// Persistent over units: igemm, a (pixel class, pixel tile, column tile); dW, a (pair of row units, column tile, range of pixel tiles).
-template <int NTMAX, bool DW>
+// Persistent over units: igemm, a (pixel class, pixel tile, column tile); dW, a (group of row units, column tile, range of pixel tiles).
+template <int NTMAX, bool DW, int KC>
 __global__ void __launch_bounds__(SPLIT_THREADS, 1) split_conv_kernel(const __grid_constant__ SplitParams p) {
-    using Cfg = SplitCfg<NTMAX, DW>;
+    using Cfg = SplitCfg<NTMAX, DW, KC>;
     constexpr int STAGES = Cfg::STAGES, NBG = Cfg::NBG, NBC = Cfg::NBC, STAGE = Cfg::STAGE_A + Cfg::STAGE_B;
-    constexpr int TILE = DW_PIXELS * 128;                          // dW: 64 channels of a box of pixels
+    constexpr int UNITS = Cfg::UNITS;
+    constexpr int TILE = DW_PIXELS * Cfg::ROW, DY_TILE = DW_PIXELS * 128;      // dW: KC channels of x, 64 channels of dy of a box of pixels
     extern __shared__ uint8_t smem_raw[];
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     const uint32_t sBar = smem_base + STAGES * STAGE;
     auto full_bar = [&](int s) { return sBar + 8u * s; };
     auto empty_bar = [&](int s) { return sBar + 8u * (STAGES + s); };
-    auto gfull_bar = [&](int b) { return sBar + 8u * (2 * STAGES + b); };                 // the sums of a stage's groups are complete / taken
+    auto gfull_bar = [&](int b) { return sBar + 8u * (2 * STAGES + b); };                 // the x0 w0 sum of a stage is complete / taken
     auto gempty_bar = [&](int b) { return sBar + 8u * (2 * STAGES + NBG + b); };
     auto cfull_bar = [&](int b) { return sBar + 8u * (2 * STAGES + 2 * NBG + b); };       // an epoch's small products
     auto cempty_bar = [&](int b) { return sBar + 8u * (2 * STAGES + 2 * NBG + NBC + b); };
@@ -207,10 +214,16 @@ __global__ void __launch_bounds__(SPLIT_THREADS, 1) split_conv_kernel(const __gr
 
     if (DW && p.rows < p.ksteps * 16) {
         // rows of a box past p.rows are never written by TMA but read by the last step: zeros
-        const int per_tile = (p.ksteps * 16 - p.rows) * 8;                                // 16-byte pieces
-        for (int i = threadIdx.x; i < STAGES * STAGE / TILE * per_tile; i += SPLIT_THREADS) {
-            const int tile = i / per_tile;
-            *reinterpret_cast<uint4*>(gen_base + (size_t)tile * TILE + p.rows * 128 + (i - tile * per_tile) * 16) = make_uint4(0, 0, 0, 0);
+        auto clear = [&](int first, int tiles, int tile_bytes, int row) {
+            const int per_tile = (p.ksteps * 16 - p.rows) * (row / 16);                   // 16-byte pieces
+            for (int i = threadIdx.x; i < tiles * per_tile; i += SPLIT_THREADS) {
+                const int tile = i / per_tile;
+                *reinterpret_cast<uint4*>(gen_base + first + (size_t)tile * tile_bytes + p.rows * row + (i - tile * per_tile) * 16) = make_uint4(0, 0, 0, 0);
+            }
+        };
+        for (int s = 0; s < STAGES; ++s) {
+            clear(s * STAGE, Cfg::STAGE_A / TILE, TILE, Cfg::ROW);
+            clear(s * STAGE + Cfg::STAGE_A, Cfg::STAGE_B / DY_TILE, DY_TILE, 128);
         }
         fence_proxy_async_smem();
     }
@@ -231,70 +244,73 @@ __global__ void __launch_bounds__(SPLIT_THREADS, 1) split_conv_kernel(const __gr
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_ptr_generic;
-    const uint32_t tmem_c = tmem_base + NBG * 2 * NTMAX;           // accumulators of the small products
+    const uint32_t tmem_c = tmem_base + NBG * NTMAX;           // accumulators of the small products
 
     const int NT = p.NT;
     const int ptiles = p.tiles_w * p.tiles_h * p.tiles_n;
-    const int b_part = DW ? TILE : NT * 128;                       // bytes of one part of the columns' operand
-    // unit -> column tile; igemm: pixel tile `mt` of class `cls`; dW: pair of row units `mt`, range of pixel tiles [t0, t1)
+    const int b_part = DW ? DY_TILE : NT * Cfg::ROW;                       // bytes of one part of the columns' operand
+    // unit -> column tile; igemm: pixel tile `mt` of class `cls`; dW: group of row units `mt`, range of pixel tiles [t0, t1)
     auto decode = [&](int u, int& nt, int& mt, int& cls, int& t0, int& t1) {
-        const unsigned a = (unsigned)u / (unsigned)p.n_tiles_n;
-        nt = u - (int)a * p.n_tiles_n;
+        const int a = split_quot(u, p.by_ntn);
+        nt = u - a * p.n_tiles_n;
         if (DW) {
-            const unsigned groups = (unsigned)(p.U + 1) / 2, split = a / groups;
-            mt = (int)(a - split * groups);
-            cls = (int)split;
+            cls = split_quot(a, p.by_groups);
+            mt = a - cls * (int)p.by_groups.d;
             t0 = (int)((long long)ptiles * cls / p.splits);
             t1 = (int)((long long)ptiles * (cls + 1) / p.splits);
         } else {
-            cls = (int)(a / (unsigned)ptiles);
-            mt = (int)a - cls * ptiles;
+            cls = split_quot(a, p.by_tiles);
+            mt = a - cls * ptiles;
             t0 = t1 = 0;
         }
     };
     // stages of a unit, and steps of one of them
     auto unit_stages = [&](int cls, int t0, int t1) {
         if (DW) return t1 - t0;
-        const SplitClass c = split_class(p, cls);
+        const SplitClass& c = p.cls[DW ? 0 : cls];
         return c.nH * c.nW * p.kchunks;
     };
-    auto stage_steps = [&](int kc) { return DW ? p.ksteps : kc == p.kchunks - 1 ? p.last_ksteps : 4; };
+    auto stage_steps = [&](int kc) { return DW ? p.ksteps : kc == p.kchunks - 1 ? p.last_ksteps : KC / 16; };
 
     if (warp < 2) {
-        // ---- copies: warp 0 the rows' operand, warp 1 the columns'
-        if (elect_one()) {
-            const bool rows = warp == 0;
+        // ---- copies: warp 0 the rows' operand, warp 1 the columns' (warp-uniform loops, one lane issues: see the products)
+        const bool leader = elect_one();
+        auto copies = [&](auto rows_tag) {
+            constexpr bool ROWS = decltype(rows_tag)::value;
             uint32_t s = 0, ph = 0;
-            bool ok = true;
-            const uint32_t tx = 3u * 128u * (DW ? (uint32_t)p.rows * (rows ? 2u : 1u) : (uint32_t)(rows ? p.rows : NT));
+            const uint32_t tx = 3u * (DW ? (uint32_t)p.rows * (ROWS ? 256u : 128u) : (uint32_t)(ROWS ? p.rows : NT) * Cfg::ROW);
             const int phases = p.dx ? 1 : p.sH * p.sW;
-            for (int u = blockIdx.x; u < p.units && ok; u += gridDim.x) {
+            auto free_stage = [&] { return __all_sync(0xffffffffu, mbar_wait_spin(empty_bar(s), ph ^ 1u, p.status, DS_TIMEOUT_EMPTY)) != 0; };
+            for (int u = blockIdx.x; u < p.units; u += gridDim.x) {
                 int nt, mt, cls, t0, t1, w0, h0, n0;
                 decode(u, nt, mt, cls, t0, t1);
                 if (DW) {
-                    int uc[2], uw[2], uh[2], uf[2];               // channel, column, row and phase of the pair's units
+                    int uc[UNITS], uw[UNITS], uh[UNITS], uf[UNITS];       // channel, column, row and phase of the group's units
 #pragma unroll
-                    for (int k = 0; k < 2; ++k) {
-                        int unit = mt * 2 + k, fh, fw;
-                        if (unit >= p.U) unit = p.U - 1;          // padding unit of the last pair: results are dropped
+                    for (int k = 0; k < UNITS; ++k) {
+                        int unit = mt * UNITS + k, fh, fw;
+                        if (unit >= p.U) unit = p.U - 1;          // padding unit of the last group: results are dropped
                         const int tap = unit / p.cblocks, i = tap / p.fW;
-                        uc[k] = (unit - tap * p.cblocks) * SPLIT_KC;
+                        uc[k] = (unit - tap * p.cblocks) * KC;
                         split_phase(tap - i * p.fW - p.pW, p.sW, fw, uw[k]);
                         split_phase(i - p.pH, p.sH, fh, uh[k]);
                         uf[k] = fh * p.sW + fw;
                     }
                     split_tile_origin(p, t0, w0, h0, n0);
                     for (int t = t0; t < t1; ++t) {
-                        if (!mbar_wait(empty_bar(s), ph ^ 1u, p.status, DS_TIMEOUT_EMPTY)) { ok = false; break; }
-                        const uint32_t bar = full_bar(s), at = smem_base + s * STAGE + (rows ? 0 : Cfg::STAGE_A);
-                        mbar_arrive_expect_tx(bar, tx);
+                        if (!free_stage()) return;
+                        const uint32_t bar = full_bar(s), at = smem_base + s * STAGE + (ROWS ? 0 : Cfg::STAGE_A);
+                        if (leader) {
+                            mbar_arrive_expect_tx(bar, tx);
 #pragma unroll
-                        for (int q = 0; q < 3; ++q) {
-                            if (rows) {
-                                tma_load_5d(at + q * Cfg::A_PART, &p.tm_a, bar, uc[0], w0 + uw[0], h0 + uh[0], n0, q * phases + uf[0]);
-                                tma_load_5d(at + q * Cfg::A_PART + TILE, &p.tm_a, bar, uc[1], w0 + uw[1], h0 + uh[1], n0, q * phases + uf[1]);
-                            } else {
-                                tma_load_5d(at + q * TILE, &p.tm_b, bar, nt * NT, w0, h0, n0, q);
+                            for (int q = 0; q < 3; ++q) {
+                                if (ROWS) {
+#pragma unroll
+                                    for (int k = 0; k < UNITS; ++k)
+                                        tma_load_5d(at + q * Cfg::A_PART + k * TILE, &p.tm_a, bar, uc[k], w0 + uw[k], h0 + uh[k], n0, q * phases + uf[k]);
+                                } else {
+                                    tma_load_5d(at + q * DY_TILE, &p.tm_b, bar, nt * NT, w0, h0, n0, q);
+                                }
                             }
                         }
                         if (++s == STAGES) { s = 0; ph ^= 1u; }
@@ -304,7 +320,7 @@ __global__ void __launch_bounds__(SPLIT_THREADS, 1) split_conv_kernel(const __gr
                     }
                 } else {
                     // taps in order; forward: phase (fh, fw) and offset (ch, cw) of the input pixels advance with them
-                    const SplitClass c = split_class(p, cls);
+                    const SplitClass& c = p.cls[DW ? 0 : cls];
                     split_tile_origin(p, mt, w0, h0, n0);
                     const int iters = c.nH * c.nW * p.kchunks, taps = p.fH * p.fW;
                     int fh = 0, fw = 0, ch = h0 + c.hq, cw = w0 + c.wq, fw0, cw0;
@@ -318,13 +334,15 @@ __global__ void __launch_bounds__(SPLIT_THREADS, 1) split_conv_kernel(const __gr
                     cw0 = cw;
                     int kc = 0, j = 0, row = c.ph * p.fW, tap = row + c.pw;
                     for (int it = 0; it < iters; ++it) {
-                        if (!mbar_wait(empty_bar(s), ph ^ 1u, p.status, DS_TIMEOUT_EMPTY)) { ok = false; break; }
-                        const uint32_t bar = full_bar(s), at = smem_base + s * STAGE + (rows ? 0 : Cfg::STAGE_A);
-                        mbar_arrive_expect_tx(bar, tx);
+                        if (!free_stage()) return;
+                        const uint32_t bar = full_bar(s), at = smem_base + s * STAGE + (ROWS ? 0 : Cfg::STAGE_A);
+                        if (leader) {
+                            mbar_arrive_expect_tx(bar, tx);
 #pragma unroll
-                        for (int q = 0; q < 3; ++q) {
-                            if (rows) tma_load_5d(at + q * Cfg::A_PART, &p.tm_a, bar, kc * SPLIT_KC, cw, ch, n0, q * phases + fh * p.sW + fw);
-                            else tma_load_3d(at + q * b_part, &p.tm_b, bar, kc * SPLIT_KC, nt * NT, q * taps + tap);
+                            for (int q = 0; q < 3; ++q) {
+                                if (ROWS) tma_load_5d(at + q * Cfg::A_PART, &p.tm_a, bar, kc * KC, cw, ch, n0, q * phases + fh * p.sW + fw);
+                                else tma_load_3d(at + q * b_part, &p.tm_b, bar, kc * KC, nt * NT, q * taps + tap);
+                            }
                         }
                         if (++kc == p.kchunks) {
                             kc = 0;
@@ -343,16 +361,22 @@ __global__ void __launch_bounds__(SPLIT_THREADS, 1) split_conv_kernel(const __gr
                     }
                 }
             }
-        }
+        };
+        if (warp == 0) copies(std::true_type{});
+        else copies(std::false_type{});
+        __syncwarp();
     } else if (warp < 4) {
         // ---- products: warp 3 has x0 w0, warp 2 the small ones.  Issuing an MMA or a commit costs a thread about 50 clocks and each
         // barrier it waits for 80, as much as 128 columns take to multiply: with two threads those run beside the MMAs.  The loops
         // are warp-uniform (every lane polls, one issues): descriptors stay in uniform registers, where MMAs take them from.
         const bool main = warp == 3, leader = elect_one();
         const uint32_t idesc1 = make_idesc(1u, DW, DW, 128u, (uint32_t)NT), idesc2 = make_idesc(1u, DW, DW, 128u, 2u * (uint32_t)NT);
-        constexpr uint32_t ADV = DW ? 16 * 128 / 16 : 32 / 16;                            // a step of 16 in units of 16 bytes
-        const uint64_t proto = make_smem_desc(0, DW ? TILE : 16, 1024);
-        const uint32_t hi = (uint32_t)(proto >> 32), lo0 = (uint32_t)proto + (smem_base >> 4);
+        // a step of 16 in units of 16 bytes: 32 bytes along the rows; dW: 16 rows
+        constexpr uint32_t ADV = DW ? Cfg::ROW : 2, ADVB = DW ? 128 : 2;
+        constexpr uint32_t SBO = 8 * Cfg::ROW, SBOB = DW ? 1024 : SBO;
+        const uint64_t pa = make_smem_desc(0, DW ? TILE : 16, SBO, KC == 64 ? 2 : 4), pb = make_smem_desc(0, DW ? DY_TILE : 16, SBOB, DW || KC == 64 ? 2 : 4);
+        const uint32_t hi = (uint32_t)(pa >> 32), hib = (uint32_t)(pb >> 32), lo0 = (uint32_t)pa + (smem_base >> 4);
+        const uint32_t lob0 = (uint32_t)pb + ((smem_base + Cfg::STAGE_A) >> 4);
         constexpr uint32_t A_NEXT = Cfg::A_PART / 16;
         const uint32_t b_next = (uint32_t)b_part / 16;
         auto wait = [&](uint32_t bar, uint32_t parity, int code) { return __all_sync(0xffffffffu, mbar_wait_spin(bar, parity, p.status, code)) != 0; };
@@ -366,17 +390,16 @@ __global__ void __launch_bounds__(SPLIT_THREADS, 1) split_conv_kernel(const __gr
             for (int it = 0; it < iters; ++it) {
                 const int steps = stage_steps(kc);
                 if (++kc == p.kchunks) kc = 0;
-                const uint32_t da = lo0 + s * (STAGE / 16), db = da + Cfg::STAGE_A / 16;
+                const uint32_t da = lo0 + s * (STAGE / 16), db = lob0 + s * (STAGE / 16);
                 if (main) {
                     if (!wait(gempty_bar(gb), gph ^ 1u, DS_TIMEOUT_TMEM_EMPTY)) { ok = false; break; }
                     if (!wait(full_bar(s), ph, DS_TIMEOUT_FULL)) { ok = false; break; }
                     tc_fence_after();
-                    const uint32_t dg = tmem_base + gb * (2 * NTMAX);
+                    const uint32_t dg = tmem_base + gb * NTMAX;
                     if (leader) {
-                        umma_lohi<false, false>(dg, da, db, hi, idesc1, 0u);
-                        if (steps > 1) umma_lohi<false, false>(dg, da + ADV, db + ADV, hi, idesc1, 1u);
-                        if (steps > 2) umma_lohi<false, false>(dg + NTMAX, da + 2 * ADV, db + 2 * ADV, hi, idesc1, 0u);
-                        if (steps > 3) umma_lohi<false, false>(dg + NTMAX, da + 3 * ADV, db + 3 * ADV, hi, idesc1, 1u);
+#pragma unroll
+                        for (int k = 0; k < KC / 16 || (DW && k < 4); ++k)
+                            if (k < steps) umma_2hi(dg, da + ADV * k, hi, db + ADVB * k, hib, idesc1, k > 0);
                         umma_commit(gfull_bar(gb));
                         umma_commit(empty_bar(s));
                     }
@@ -394,11 +417,11 @@ __global__ void __launch_bounds__(SPLIT_THREADS, 1) split_conv_kernel(const __gr
                     const bool last = --left == 0 || it == iters - 1;
                     if (leader) {
 #pragma unroll
-                        for (int k = 0; k < 4; ++k) {
+                        for (int k = 0; k < KC / 16 || (DW && k < 4); ++k) {
                             if (k < steps) {
-                                umma_lohi<false, false>(dc, da + ADV * k, db + b_next + ADV * k, hi, idesc2, k > 0 ? 1u : acc);      // x0 [w1 | w2]
-                                umma_lohi<false, false>(dc, da + A_NEXT + ADV * k, db + ADV * k, hi, idesc2, 1u);                    // x1 [w0 | w1]
-                                umma_lohi<false, false>(dc + NT, da + 2 * A_NEXT + ADV * k, db + ADV * k, hi, idesc1, 1u);           // x2 w0
+                                umma_2hi(dc, da + ADV * k, hi, db + b_next + ADVB * k, hib, idesc2, k > 0 ? 1u : acc);       // x0 [w1 | w2]
+                                umma_2hi(dc, da + A_NEXT + ADV * k, hi, db + ADVB * k, hib, idesc2, 1u);                     // x1 [w0 | w1]
+                                umma_2hi(dc + NT, da + 2 * A_NEXT + ADV * k, hi, db + ADVB * k, hib, idesc1, 1u);            // x2 w0
                             }
                         }
                         if (last) umma_commit(cfull_bar(gb));
@@ -437,58 +460,45 @@ __global__ void __launch_bounds__(SPLIT_THREADS, 1) split_conv_kernel(const __gr
             for (int b = 0; b < BLOCKS; ++b)
 #pragma unroll
                 for (int k = 0; k < 16; ++k) acc[b][k] = 0.f;
-            // acc += accumulator at column t0, then, when asked for, the one at t1  (blocks past NT: other accumulators' columns, never stored)
-            auto add = [&](uint32_t ta, uint32_t tb, bool both) {
+            auto add = [&](uint32_t t) {          // acc += accumulator at column t  (blocks past NT: other accumulators' columns, never stored)
+                uint32_t v[BLOCKS][16];
 #pragma unroll
-                for (int b = 0; b < BLOCKS; b += 2) {
-                    uint32_t v[2][16], w[2][16];
-                    tmem_ld_32x16(ta + lane0 + 32 * b, v[0]);
-                    tmem_ld_32x16(ta + lane0 + 32 * b + 32, v[1]);
-                    if (both) {
-                        tmem_ld_32x16(tb + lane0 + 32 * b, w[0]);
-                        tmem_ld_32x16(tb + lane0 + 32 * b + 32, w[1]);
-                    } else {
+                for (int b = 0; b < BLOCKS; ++b) tmem_ld_32x16(t + lane0 + 32 * b, v[b]);
+                tmem_ld_wait();
 #pragma unroll
-                        for (int k = 0; k < 16; ++k) w[0][k] = w[1][k] = 0u;
-                    }
-                    tmem_ld_wait();
+                for (int b = 0; b < BLOCKS; ++b)
 #pragma unroll
-                    for (int k = 0; k < 16; ++k) {
-                        acc[b][k] = (acc[b][k] + __uint_as_float(v[0][k])) + __uint_as_float(w[0][k]);
-                        acc[b + 1][k] = (acc[b + 1][k] + __uint_as_float(v[1][k])) + __uint_as_float(w[1][k]);
-                    }
-                }
+                    for (int k = 0; k < 16; ++k) acc[b][k] += __uint_as_float(v[b][k]);
             };
             auto release = [&](uint32_t bar) {
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(bar);
             };
-            int kc = 0, left = EPOCH_STAGES;
+            int left = EPOCH_STAGES;
             for (int it = 0; it < iters; ++it) {
-                const int steps = stage_steps(kc);
-                if (++kc == p.kchunks) kc = 0;
                 if (!mbar_wait_spin(gfull_bar(gb), gph, p.status, DS_TIMEOUT_TMEM_FULL)) { ok = false; break; }
                 tc_fence_after();
-                add(tmem_base + gb * (2 * NTMAX), tmem_base + gb * (2 * NTMAX) + NTMAX, steps > GROUP_STEPS);
+                add(tmem_base + gb * NTMAX);
                 release(gempty_bar(gb));
                 if (++gb == NBG) { gb = 0; gph ^= 1u; }
                 if (--left == 0 || it == iters - 1) {
                     left = EPOCH_STAGES;
                     if (!mbar_wait_spin(cfull_bar(cb), cph, p.status, DS_TIMEOUT_TMEM_FULL)) { ok = false; break; }
                     tc_fence_after();
-                    add(tmem_c + cb * (2 * NTMAX) + NT, tmem_c + cb * (2 * NTMAX), true);       // third order, then second
+                    add(tmem_c + cb * (2 * NTMAX) + NT);          // third order, then second
+                    add(tmem_c + cb * (2 * NTMAX));
                     release(cempty_bar(cb));
                     if (++cb == NBC) { cb = 0; cph ^= 1u; }
                 }
             }
             if (!ok) break;
             int w0 = 0, h0 = 0, n0 = 0, x_w, x_h, x_n;
-            const SplitClass c = split_class(p, cls);
+            const SplitClass& c = p.cls[DW ? 0 : cls];
             if (!DW) split_tile_origin(p, mt, w0, h0, n0);
             float* rowp[4];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) rowp[j] = split_row<DW>(p, mt, cls, c, w0, h0, n0, q * 32 + (lane & ~3) + j, r_w[j], r_h[j], r_n[j], x_w, x_h, x_n);
+            for (int j = 0; j < 4; ++j) rowp[j] = split_row<DW, KC>(p, mt, cls, c, w0, h0, n0, q * 32 + (lane & ~3) + j, r_w[j], r_h[j], r_n[j], x_w, x_h, x_n);
             bool bad = false;
             const bool b1 = lane & 1, b2 = lane & 2;
 #pragma unroll
@@ -539,7 +549,7 @@ __global__ void __launch_bounds__(SPLIT_THREADS, 1) split_conv_kernel(const __gr
                     }
                 }
             }
-            if (bad) split_repair<DW>(p, nt, mt, cls, t0, t1, q, part, lane);
+            if (bad) split_repair<DW, KC>(p, nt, mt, cls, t0, t1, q, part, lane);
         }
     }
 
@@ -573,7 +583,7 @@ struct SplitPhases {
     }
 };
 
-// fp32 [rows][C] -> three bf16 arrays [3][rows][Cp] (channels padded with zeros to a multiple of 8) and, when asked for, each block's
+// fp32 [rows][C] -> three bf16 arrays [3][rows][Cp] (channels padded with zeros) and, when asked for, each block's
 // column sums of the fp32 input (for dB).  Bound by HBM: 4 bytes read, 6 written.
 template <bool COLSUM, bool STRIDED>
 __global__ void __launch_bounds__(256) split3_kernel(const float* __restrict__ src, __nv_bfloat16* __restrict__ dst, long long rows, int C,
@@ -682,11 +692,12 @@ struct SplitPlan {
     bool use;
     int Ho, Wo, taps, Cin_p, Cout_p, PH, PW;      // PH, PW: a phase's extent
     PixelTiling til_fwd, til_dx, til_dw;
-    int nt_fwd, nt_dx, splits, cblocks, U, ldn, db_blocks;
+    int nt_fwd, nt_dx, kc_in, kc_out, splits, cblocks, U, ldn, db_blocks;
     size_t off_wf, off_wd, off_x, off_dy, off_part, off_dbpart, total;
 };
 
-// The box of at most `most` pixels with the fewest reduction rows (tiles times rows to the next `unit`).
+// The box of at most `most` pixels with the least to do: tiles times rows to the next `unit`, and half a unit for each tile (28x28 in boxes
+// of 16 pixels has no rows of padding, but a stage of one step takes 650 clocks and one of three 970).
 static PixelTiling split_tiling(int S, int H, int W, int most, int unit) {
     PixelTiling best{};
     long long best_cost = -1;
@@ -695,7 +706,7 @@ static PixelTiling split_tiling(int S, int H, int W, int most, int unit) {
             int bn = bh < H ? 1 : most / (bw * bh);
             if (bn > S) bn = S;
             const PixelTiling t = {bw, bh, bn, bw * bh * bn, ceil_div(W, bw), ceil_div(H, bh), ceil_div(S, bn)};
-            const long long cost = t.total() * ((t.rows + unit - 1) / unit);
+            const long long cost = t.total() * (2 * ((t.rows + unit - 1) / unit) + 1);
             if (best_cost < 0 || cost < best_cost || (cost == best_cost && bw > best.BW)) {
                 best_cost = cost;
                 best = t;
@@ -717,24 +728,35 @@ static int split_nt(int N, long long tiles) {
     return best;
 }
 
+// Channels per row: 32 where the last 64 would be half empty and few are in front of it.
+static int split_kc(int C) { return C <= 96 && ceil_div(C, 32) % 2 == 1 ? 32 : 64; }
+
 static SplitPlan compute_split_plan(const AetherConvDesc& d) {
     SplitPlan pl{};
     conv_out_hw(d, pl.Ho, pl.Wo);
     pl.taps = d.fH * d.fW;
-    pl.Cin_p = (d.Cin + 7) / 8 * 8;
-    pl.Cout_p = (d.Cout + 7) / 8 * 8;
-    if (d.sH > 4 || d.sW > 4 || pl.taps > 64) return pl;
-    // Fewer channels leave most of a 64-channel row empty, and a small layer is through on the CUDA cores before the passes that make
-    // the parts are (forward and backward on B200, CUDA cores / split, us: 208 x 53x48 16->64 stride 2 254 / 271, 209 x 23x18
-    // 36->16 stride 2 60 / 95, 6 x 16x16 32->165 5x5, 0.7 GFLOP, 71 / 83; 24 x 18x18 48->208 stride 2, 1.05 GFLOP, 98 / 47).
-    const double flops = 6.0 * d.S * pl.Ho * pl.Wo * pl.taps * d.Cin * d.Cout;
-    if (d.Cin < 32 || d.Cout < 32 || flops < 1e9) return pl;
+    // Rows of the parts: whole tile rows of 64 or 128 bytes, or a tap's copies take up to twice as long (dX of 100 x 57x45 48->72 stride 2
+    // 103 -> 62 us with rows of 128 channels instead of 72); a pointwise layer copies each row once and is better off with less to write.
+    pl.kc_in = split_kc(d.Cin);
+    pl.kc_out = split_kc(d.Cout);
+    const int ui = pl.taps > 1 ? pl.kc_in : 8, uo = pl.taps > 1 ? pl.kc_out : 8;
+    pl.Cin_p = (d.Cin + ui - 1) / ui * ui;
+    pl.Cout_p = (d.Cout + uo - 1) / uo * uo;
+    if (d.sH > SPLIT_MOST_STRIDE || d.sW > SPLIT_MOST_STRIDE || pl.taps > 64 || d.padH > 16384 || d.padW > 16384) return pl;
+    if (d.Cin < 16 || d.Cout < 16) return pl;
     // Short reductions: nothing to gain in accuracy over the FMA kernels' (their error grows with the reduction, this one's does not).
     if (pl.taps * d.Cin < 64 || pl.taps * d.Cout < 64) return pl;
     pl.PH = ceil_div(d.H, d.sH);
     pl.PW = ceil_div(d.W, d.sW);
     const size_t in_rows = (size_t)d.sH * d.sW * d.S * pl.PH * pl.PW, out_rows = (size_t)d.S * pl.Ho * pl.Wo;
     if ((in_rows * pl.Cin_p + out_rows * pl.Cout_p) * 6 > (2ull << 30)) return pl;      // (the parts are scratch of the caller's)
+    // What the FMA kernels take for a layer (33 TFLOP/s) must be worth the passes that make the parts (5 TB/s) and the longer way
+    // through the kernels.  Forward and backward on B200, CUDA cores / split, us: 209 x 23x18 36->16 stride 2 60 / 65, 17 x 13x21
+    // 32->16 5x5 36 / 42 and 2 x 9x10 65->130 36 / 47 stay; 6 x 16x16 32->165 5x5 71 / 71, 12 x 24x24 16->146 71 / 50, 6 x 43x43
+    // 88->188 1x1 53 / 46, 208 x 53x48 16->64 stride 2 254 / 235, 24 x 18x18 48->208 stride 2 98 / 43, 123 x 18x18 36->46 5x5 532 / 154 go.
+    const double fma_us = 6.0 * d.S * pl.Ho * pl.Wo * pl.taps * d.Cin * d.Cout / 33e6;
+    const double parts_us = (1.0 * in_rows * (4.0 * d.Cin / (d.sH * d.sW) + 6.0 * pl.Cin_p) + 1.0 * out_rows * (4.0 * d.Cout + 6.0 * pl.Cout_p)) / 5e6;
+    if (fma_us < 12.0 + 1.6 * parts_us) return pl;
     if (1LL * d.S * d.H * d.W * ceil_div(d.Cin > d.Cout ? d.Cin : d.Cout, 16) > 0x7fffffffLL) return pl;       // units in 32 bits
     pl.use = true;
     pl.til_fwd = split_tiling(d.S, pl.Ho, pl.Wo, 128, 128);
@@ -742,10 +764,10 @@ static SplitPlan compute_split_plan(const AetherConvDesc& d) {
     pl.til_dw = split_tiling(d.S, pl.Ho, pl.Wo, DW_PIXELS, 16);
     pl.nt_fwd = split_nt(d.Cout, pl.til_fwd.total());
     pl.nt_dx = split_nt(d.Cin, pl.til_dx.total() * d.sH * d.sW);
-    pl.cblocks = ceil_div(d.Cin, SPLIT_KC);
+    pl.cblocks = ceil_div(d.Cin, pl.kc_in);
     pl.U = pl.taps * pl.cblocks;
     pl.ldn = (d.Cout + 3) / 4 * 4;
-    const long long cols = 1LL * ceil_div(pl.U, 2) * ceil_div(d.Cout, 64), ptiles = pl.til_dw.total();
+    const long long cols = 1LL * ceil_div(pl.U, 128 / pl.kc_in) * ceil_div(d.Cout, 64), ptiles = pl.til_dw.total();
     long long splits = num_sms() / cols;
     if (splits > ptiles / 4) splits = ptiles / 4;
     pl.splits = (int)(splits < 1 ? 1 : splits);
@@ -756,7 +778,7 @@ static SplitPlan compute_split_plan(const AetherConvDesc& d) {
     pl.off_wd = take((size_t)3 * pl.taps * d.Cin * pl.Cout_p * 2);
     pl.off_x = take(3 * in_rows * pl.Cin_p * 2);
     pl.off_dy = take(3 * out_rows * pl.Cout_p * 2);
-    pl.off_part = take((size_t)pl.splits * pl.U * 64 * pl.ldn * 4);
+    pl.off_part = take((size_t)pl.splits * pl.U * pl.kc_in * pl.ldn * 4);
     pl.off_dbpart = take((size_t)pl.db_blocks * d.Cout * 4);
     pl.total = off;
     return pl;
@@ -766,33 +788,54 @@ static const SplitPlan& split_plan(const AetherConvDesc& d) { return cached_plan
 bool split_conv_eligible(const AetherConvDesc& d) { return split_plan(d).use; }
 size_t split_conv_workspace_bytes(const AetherConvDesc& d) { return split_plan(d).total; }
 
-// (C, W, H, N, part x phase) bf16, box 64 channels x the pixels of `t`.
-static int split_pixel_map(CUtensorMap* m, const void* base, int Cp, int W, int H, int N, int phases, const PixelTiling& t) {
+// (C, W, H, N, part x phase) bf16, box kc channels x the pixels of `t`.
+static int split_pixel_map(CUtensorMap* m, const void* base, int Cp, int W, int H, int N, int phases, const PixelTiling& t, int kc) {
     const cuuint64_t row = (cuuint64_t)Cp * 2;
     const cuuint64_t dims[5] = {(cuuint64_t)Cp, (cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)N, (cuuint64_t)3 * phases};
     const cuuint64_t strides[4] = {row, row * W, row * W * H, row * W * H * N};
-    const cuuint32_t box[5] = {SPLIT_KC, (cuuint32_t)t.BW, (cuuint32_t)t.BH, (cuuint32_t)t.BN, 1};
+    const cuuint32_t box[5] = {(cuuint32_t)kc, (cuuint32_t)t.BW, (cuuint32_t)t.BH, (cuuint32_t)t.BN, 1};
     const cuuint32_t es[5] = {1, 1, 1, 1, 1};
-    return make_map(m, base, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, dims, strides, box, es, CU_TENSOR_MAP_SWIZZLE_128B);
+    return make_map(m, base, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, dims, strides, box, es, kc == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B);
 }
 
-template <int NTMAX, bool DW>
+template <int NTMAX, bool DW, int KC>
 static int launch_split(const SplitParams& p, int prof, cudaStream_t st) {
-    using Cfg = SplitCfg<NTMAX, DW>;
+    using Cfg = SplitCfg<NTMAX, DW, KC>;
     static PerDeviceSmem configured;
-    if (int rc = ensure_dynamic_smem(split_conv_kernel<NTMAX, DW>, Cfg::SMEM_BYTES, configured, "split_conv")) return rc;
+    if (int rc = ensure_dynamic_smem(split_conv_kernel<NTMAX, DW, KC>, Cfg::SMEM_BYTES, configured, "split_conv")) return rc;
     const int grid = (int)(p.units < num_sms() ? p.units : num_sms());
     prof_begin(prof, st);
-    launch(split_conv_kernel<NTMAX, DW>, grid, SPLIT_THREADS, Cfg::SMEM_BYTES, st, p);
+    launch(split_conv_kernel<NTMAX, DW, KC>, grid, SPLIT_THREADS, Cfg::SMEM_BYTES, st, p);
     prof_end(prof, st);
     count_launch();
     return check_launch("split_conv_kernel");
+}
+
+static SplitClass split_class(const AetherConvDesc& d, int cls) {
+    const int ph = cls / d.sW, pw = cls % d.sW;
+    SplitClass c;
+    c.ph = (int16_t)ph;
+    c.pw = (int16_t)pw;
+    c.nH = (int16_t)(ph < d.fH ? (d.fH - ph - 1) / d.sH + 1 : 0);
+    c.nW = (int16_t)(pw < d.fW ? (d.fW - pw - 1) / d.sW + 1 : 0);
+    const int hs = ((ph - d.padH) % d.sH + d.sH) % d.sH, ws = ((pw - d.padW) % d.sW + d.sW) % d.sW;
+    c.hs = (int16_t)hs;
+    c.ws = (int16_t)ws;
+    c.hq = (int16_t)((hs + d.padH - ph) / d.sH);             // exact (hs + padH = ph mod sH), not negative (ph < sH)
+    c.wq = (int16_t)((ws + d.padW - pw) / d.sW);
+    c.MH = hs < d.H ? (d.H - hs - 1) / d.sH + 1 : 0;
+    c.MW = ws < d.W ? (d.W - ws - 1) / d.sW + 1 : 0;
+    return c;
 }
 
 static void split_geometry(SplitParams& p, const AetherConvDesc& d, const PixelTiling& t) {
     p.S = d.S; p.fH = d.fH; p.fW = d.fW; p.sH = d.sH; p.sW = d.sW; p.pH = d.padH; p.pW = d.padW; p.Cin = d.Cin; p.Cout = d.Cout;
     p.BW = t.BW; p.BH = t.BH; p.BN = t.BN; p.rows = t.rows; p.tiles_w = t.tiles_w; p.tiles_h = t.tiles_h; p.tiles_n = t.tiles_n;
     p.status = device_status_word();
+    p.by_tw = split_div(t.tiles_w);
+    p.by_th = split_div(t.tiles_h);
+    p.by_tiles = split_div((uint32_t)t.total());
+    p.by_ntn = split_div(p.n_tiles_n);
 }
 
 // Forward (dx false: in = x, copies of it at `cp`) and dX (in = dy).
@@ -801,23 +844,26 @@ static int run_split_igemm(const AetherConvDesc& d, const SplitPlan& pl, bool dx
     SplitParams p;
     memset(&p, 0, sizeof(p));
     const PixelTiling& t = dx ? pl.til_dx : pl.til_fwd;
+    p.NT = dx ? pl.nt_dx : pl.nt_fwd;
+    p.n_tiles_n = ceil_div(dx ? d.Cin : d.Cout, p.NT);
     split_geometry(p, d, t);
     p.in = in; p.w = w; p.bias = bias; p.out = out; p.dx = dx;
     p.IH = dx ? pl.Ho : d.H; p.IW = dx ? pl.Wo : d.W; p.IC = dx ? d.Cout : d.Cin;
     p.OH = dx ? d.H : pl.Ho; p.OW = dx ? d.W : pl.Wo; p.N = dx ? d.Cin : d.Cout;
-    p.NT = dx ? pl.nt_dx : pl.nt_fwd;
-    p.n_tiles_n = ceil_div(p.N, p.NT);
-    p.kchunks = ceil_div(p.IC, SPLIT_KC);
-    p.last_ksteps = ceil_div(p.IC - (p.kchunks - 1) * SPLIT_KC, 16);
+    for (int k = 0; k < (dx ? d.sH * d.sW : 1); ++k) p.cls[k] = dx ? split_class(d, k) : SplitClass{0, 0, (int16_t)d.fH, (int16_t)d.fW, 0, 0, 0, 0, p.OH, p.OW};
+    const int kc = dx ? pl.kc_out : pl.kc_in;
+    p.kchunks = ceil_div(p.IC, kc);
+    p.last_ksteps = ceil_div(p.IC - (p.kchunks - 1) * kc, 16);
     p.units = (int)(t.total() * p.n_tiles_n * (dx ? d.sH * d.sW : 1));
     const int Cp = dx ? pl.Cout_p : pl.Cin_p;
-    if (int rc = split_pixel_map(&p.tm_a, cp, Cp, dx ? pl.Wo : pl.PW, dx ? pl.Ho : pl.PH, d.S, dx ? 1 : d.sH * d.sW, t)) return rc;
+    if (int rc = split_pixel_map(&p.tm_a, cp, Cp, dx ? pl.Wo : pl.PW, dx ? pl.Ho : pl.PH, d.S, dx ? 1 : d.sH * d.sW, t, kc)) return rc;
     const cuuint64_t dims[3] = {(cuuint64_t)Cp, (cuuint64_t)p.N, (cuuint64_t)3 * pl.taps};
     const cuuint64_t strides[2] = {(cuuint64_t)Cp * 2, (cuuint64_t)Cp * 2 * p.N};
-    const cuuint32_t box[3] = {SPLIT_KC, (cuuint32_t)p.NT, 1}, es[3] = {1, 1, 1};
-    if (int rc = make_map(&p.tm_b, wcp, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, dims, strides, box, es, CU_TENSOR_MAP_SWIZZLE_128B)) return rc;
+    const cuuint32_t box[3] = {(cuuint32_t)kc, (cuuint32_t)p.NT, 1}, es[3] = {1, 1, 1};
+    if (int rc = make_map(&p.tm_b, wcp, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, dims, strides, box, es, kc == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B)) return rc;
     const int prof = dx ? PK_IGEMM_DX : PK_IGEMM_FWD;
-    return p.NT <= 64 ? launch_split<64, false>(p, prof, st) : launch_split<128, false>(p, prof, st);
+    if (kc == 32) return p.NT <= 64 ? launch_split<64, false, 32>(p, prof, st) : launch_split<128, false, 32>(p, prof, st);
+    return p.NT <= 64 ? launch_split<64, false, 64>(p, prof, st) : launch_split<128, false, 64>(p, prof, st);
 }
 
 static int launch_split3(const float* src, void* dst, long long rows, int C, int Cp, const SplitPhases& f, float* colsum, int blocks, cudaStream_t st) {
@@ -875,19 +921,21 @@ int split_conv_bwd(const AetherConvDesc& d, const float* x, const float* dy, con
     SplitParams p;
     memset(&p, 0, sizeof(p));
     const PixelTiling& t = pl.til_dw;
+    p.NT = 64;
+    p.n_tiles_n = ceil_div(d.Cout, p.NT);
     split_geometry(p, d, t);
     p.in = x; p.w = dy; p.out = reinterpret_cast<float*>(wsb + pl.off_part);
     p.IH = d.H; p.IW = d.W; p.IC = d.Cin; p.OH = pl.Ho; p.OW = pl.Wo; p.N = d.Cout;
-    p.NT = 64;
-    p.n_tiles_n = ceil_div(d.Cout, p.NT);
     p.U = pl.U; p.cblocks = pl.cblocks; p.splits = pl.splits; p.ldn = pl.ldn;
     p.ksteps = ceil_div(t.rows, 16);
     p.kchunks = 1;
-    p.units = ceil_div(p.U, 2) * p.n_tiles_n * p.splits;
-    if ((rc = split_pixel_map(&p.tm_a, wsb + pl.off_x, pl.Cin_p, pl.PW, pl.PH, d.S, d.sH * d.sW, t))) return rc;
-    if ((rc = split_pixel_map(&p.tm_b, wsb + pl.off_dy, pl.Cout_p, pl.Wo, pl.Ho, d.S, 1, t))) return rc;
-    if ((rc = launch_split<64, true>(p, PK_DW, st))) return rc;
-    return dw_reduce(p.out, dw, p.splits, p.U, 64, p.ldn, p.cblocks, pl.taps, d.Cin, d.Cout, pl.taps, p.splits, dbpart, pl.db_blocks, db, st);
+    const int groups = ceil_div(p.U, 128 / pl.kc_in);
+    p.by_groups = split_div(groups);
+    p.units = groups * p.n_tiles_n * p.splits;
+    if ((rc = split_pixel_map(&p.tm_a, wsb + pl.off_x, pl.Cin_p, pl.PW, pl.PH, d.S, d.sH * d.sW, t, pl.kc_in))) return rc;
+    if ((rc = split_pixel_map(&p.tm_b, wsb + pl.off_dy, pl.Cout_p, pl.Wo, pl.Ho, d.S, 1, t, 64))) return rc;
+    if ((rc = pl.kc_in == 32 ? launch_split<64, true, 32>(p, PK_DW, st) : launch_split<64, true, 64>(p, PK_DW, st))) return rc;
+    return dw_reduce(p.out, dw, p.splits, p.U, pl.kc_in, p.ldn, p.cblocks, pl.taps, d.Cin, d.Cout, pl.taps, p.splits, dbpart, pl.db_blocks, db, st);
 }
 
 }  // namespace aether

@@ -13,7 +13,7 @@ pytestmark = pytest.mark.gpu
 # (S, H, W, Cin, Cout, f, stride, pad, mode)
 SHAPES = [(9, 19, 17, 65, 130, 3, (1, 1), "same", "fp32"), (60, 15, 13, 37, 71, 3, (1, 1), "valid", "bf16"), (40, 21, 18, 72, 48, 3, (2, 2), "same", "bf16"),
           (61, 8, 8, 128, 33, 3, (1, 1), "same", "fp32"), (30, 23, 20, 64, 64, 5, (3, 2), "valid", "tf32"), (70, 30, 31, 96, 32, 1, (1, 1), "same", "fp32"),
-          (120, 12, 11, 100, 129, 1, (2, 2), "same", "fp32"), (16, 7, 7, 256, 256, 3, (1, 1), "same", "fp32"), (90, 9, 10, 32, 144, 3, (1, 4), "same", "tf32")]
+          (120, 12, 11, 100, 129, 1, (2, 2), "same", "fp32"), (60, 20, 21, 16, 50, 5, (1, 1), "same", "fp32"), (40, 33, 20, 90, 17, 3, (2, 1), "valid", "bf16"), (16, 7, 7, 256, 256, 3, (1, 1), "same", "fp32"), (90, 9, 10, 32, 144, 3, (1, 4), "same", "tf32")]
 
 
 def _layer(shape, x, b):
