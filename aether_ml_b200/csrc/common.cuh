@@ -113,7 +113,8 @@ size_t first_tc_bwd_workspace_bytes(const AetherConvDesc& d);
 bool first_tc_operand_layout(const AetherConvDesc& d, AetherOperandLayout* out);
 // out[c] = sum over `rows` rows of part[row][C] in fixed order (conv_tc.cu)
 int colsum_finish(const float* part, int rows, int C, float* out, cudaStream_t st);
-int smallc_reduce_partials(const float* part, int nb, int K, int Cout, float* dw, float* db, cudaStream_t st);
+int smallc_reduce_partials(const float* part, int nb, int K, int Cout, float* dw, float* db, cudaStream_t st, const float* colsum = nullptr,
+                           int rows = 0);
 
 // ---- conv_tc.cu : tcgen05 implicit-GEMM convolution (stride 1)
 bool tc_conv_eligible(const AetherConvDesc& d);

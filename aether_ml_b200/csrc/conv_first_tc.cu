@@ -779,12 +779,9 @@ int first_tc_bwd_filter(const AetherConvDesc& d, const float* x, const float* dy
     count_launch();
     int rc = check_launch("first_dw_kernel");
     if (rc) return rc;
-    if (p.dy_bf16) {
-        if ((rc = smallc_reduce_partials(p.part, grid, K, d.Cout, dw, nullptr, st))) return rc;
-        return db ? colsum_finish(reinterpret_cast<const float*>(static_cast<uint8_t*>(ws) + lay.colsum_off), dy_colsum_rows,
-                                  d.Cout, db, st)
-                  : AE_OK;
-    }
+    if (p.dy_bf16 && db)
+        return smallc_reduce_partials(p.part, grid, K, d.Cout, dw, db, st,
+                                      reinterpret_cast<const float*>(static_cast<uint8_t*>(ws) + lay.colsum_off), dy_colsum_rows);
     return smallc_reduce_partials(p.part, grid, K, d.Cout, dw, db, st);
 }
 

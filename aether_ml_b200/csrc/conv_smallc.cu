@@ -12,6 +12,7 @@
 // gather itself has no divisions.  dW keeps its accumulators in registers across all tiles of the CTA and
 // writes one partial per CTA; a second kernel adds the partials in fixed order (bit-reproducible, no atomics).
 #include "common.cuh"
+#include "finish_columns.cuh"
 
 namespace aether {
 
@@ -232,16 +233,23 @@ __global__ void __launch_bounds__(SC_THREADS) smallc_dw_kernel(const SmallcGeom 
     if (kg == 0) *reinterpret_cast<float4*>(out + (size_t)g.K * g.Cout + cg * 4) = bsum;
 }
 
-// dw[e] / db[d] = sum over CTAs of the partials, 8 lanes per output combined in fixed order.
+// dw[e] / db[d] = sum over CTAs of the partials, 8 lanes per output combined in fixed order.  Where dB comes from column sums that
+// were handed in with dy's copy (`colsum`, `rows` of them), the CTAs from `nred` on add those up.
 __global__ void __launch_bounds__(256) smallc_reduce_kernel(const float* __restrict__ part, int nblocks, int K, int Cout,
-                                                            float* __restrict__ dw, float* __restrict__ db) {
+                                                            float* __restrict__ dw, float* __restrict__ db, int nred,
+                                                            const float* __restrict__ colsum, int rows) {
     pdl_wait();
     __shared__ float red[8][32];
+    if ((int)blockIdx.x >= nred) {
+        finish_columns(colsum, rows, Cout, db, (int)blockIdx.x - nred, reinterpret_cast<float (*)[8]>(red));
+        return;
+    }
     const int el = threadIdx.x & 31, ln = threadIdx.x >> 5;
     const int e = blockIdx.x * 32 + el;
     const int total = (K + 1) * Cout;
     float s = 0.f;
     if (e < total)
+#pragma unroll 8
         for (int b = ln; b < nblocks; b += 8) s += part[(size_t)b * total + e];
     red[ln][el] = s;
     __syncthreads();
@@ -251,7 +259,7 @@ __global__ void __launch_bounds__(256) smallc_reduce_kernel(const float* __restr
         for (int l = 0; l < 8; ++l) t += red[l][el];
         if (e < K * Cout) {
             if (dw) dw[e] = t;
-        } else if (db) {
+        } else if (db && !colsum) {
             db[e - K * Cout] = t;
         }
     }
@@ -371,6 +379,13 @@ int smallc_conv_fwd(const AetherConvDesc& d, const float* x, const float* w, con
     return launch_smallc_fwd<4>(g, x, w, b, y, stats, nb, ntiles, smem, st);
 }
 
+static int launch_smallc_reduce(const float* part, int nb, int K, int Cout, float* dw, float* db, const float* colsum, int rows, cudaStream_t st) {
+    const int nred = ceil_div((K + 1) * Cout, 32);
+    launch(smallc_reduce_kernel, nred + (colsum ? ceil_div(Cout, 8) : 0), 256, 0, st, part, nb, K, Cout, dw, db, nred, colsum, rows);
+    count_launch();
+    return check_launch("smallc_reduce_kernel");
+}
+
 template <int KPG>
 static int launch_smallc_dw(const SmallcGeom& g, const float* x, const float* dy, float* part, int nb, long long ntiles,
                             size_t smem, cudaStream_t st) {
@@ -400,13 +415,13 @@ int smallc_conv_bwd_filter(const AetherConvDesc& d, const float* x, const float*
     else if (g.KPG <= 8) rc = launch_smallc_dw<8>(g, xs, dy, part, nb, ntiles, smem, st);
     else rc = launch_smallc_dw<16>(g, xs, dy, part, nb, ntiles, smem, st);
     if (rc) return rc;
-    launch(smallc_reduce_kernel, ceil_div((g.K + 1) * g.Cout, 32), 256, 0, st, part, nb, g.K, g.Cout, dw, db);
-    count_launch();
-    return check_launch("smallc_reduce_kernel");
+    return launch_smallc_reduce(part, nb, g.K, g.Cout, dw, db, nullptr, 0, st);
 }
 
-// Sums nb partials of [K + 1][Cout] floats (row K = dB) into dw / db in fixed order (also used by conv_first_tc.cu).
-int smallc_reduce_partials(const float* part, int nb, int K, int Cout, float* dw, float* db, cudaStream_t st) {
+// Sums nb partials of [K + 1][Cout] floats (row K = dB) into dw / db in fixed order (also used by conv_first_tc.cu).  `colsum`: dB is the
+// sum of these `rows` rows of column sums instead.
+int smallc_reduce_partials(const float* part, int nb, int K, int Cout, float* dw, float* db, cudaStream_t st, const float* colsum, int rows) {
+    if (colsum) return launch_smallc_reduce(part, nb, K, Cout, dw, db, colsum, rows, st);
     const int total = (K + 1) * Cout;
     if (nb <= 8 || (nb <= 24 && total >= 1 << 16)) {
         const bool v4 = Cout % 4 == 0 && aligned16(part) && aligned16(dw);
@@ -414,9 +429,7 @@ int smallc_reduce_partials(const float* part, int nb, int K, int Cout, float* dw
         count_launch();
         return check_launch("partial_sums_kernel");
     }
-    launch(smallc_reduce_kernel, ceil_div((K + 1) * Cout, 32), 256, 0, st, part, nb, K, Cout, dw, db);
-    count_launch();
-    return check_launch("smallc_reduce_kernel");
+    return launch_smallc_reduce(part, nb, K, Cout, dw, db, nullptr, 0, st);
 }
 
 }  // namespace aether

@@ -586,14 +586,12 @@ struct SplitPhases {
 // fp32 [rows][C] -> three bf16 arrays [3][rows][Cp] (channels padded with zeros) and, when asked for, each block's
 // column sums of the fp32 input (for dB).  Bound by HBM: 4 bytes read, 6 written.
 template <bool COLSUM, bool STRIDED>
-__global__ void __launch_bounds__(256) split3_kernel(const float* __restrict__ src, __nv_bfloat16* __restrict__ dst, long long rows, int C,
-                                                     int Cp, float* __restrict__ colsum_part, long long rows_per_block, const SplitPhases f) {
-    pdl_wait();
+__device__ __forceinline__ void split3_rows(const float* __restrict__ src, __nv_bfloat16* __restrict__ dst, long long rows, int C, int Cp,
+                                            float* __restrict__ colsum_part, long long rows_per_block, const SplitPhases& f, int block, float* red) {
     const int G = Cp / 8;                                // groups of eight channels
-    const long long r_begin = blockIdx.x * rows_per_block;
+    const long long r_begin = block * rows_per_block;
     const long long r_end = r_begin + rows_per_block < rows ? r_begin + rows_per_block : rows;
     const size_t plane = (size_t)rows * Cp;
-    __shared__ float red[COLSUM ? 256 * 8 : 8];
     for (int gbase = 0; gbase < G; gbase += 256) {
         const int Gc = (G - gbase) < 256 ? (G - gbase) : 256, lanes = 256 / Gc;
         const int g = gbase + threadIdx.x % Gc, rl = threadIdx.x / Gc, c0 = g * 8;
@@ -648,7 +646,7 @@ __global__ void __launch_bounds__(256) split3_kernel(const float* __restrict__ s
                 if (c < C) {
                     float s = 0.f;
                     for (int l = 0; l < lanes; ++l) s += red[(l * Gc + cc / 8) * 8 + cc % 8];
-                    colsum_part[(size_t)blockIdx.x * C + c] = s;
+                    colsum_part[(size_t)block * C + c] = s;
                 }
             }
             __syncthreads();
@@ -657,34 +655,47 @@ __global__ void __launch_bounds__(256) split3_kernel(const float* __restrict__ s
 }
 
 // The filter's operands from one read of w (taps, Cin, Cout): fwd [3][taps][Cout][Cin_p] (transposed), dx [3][taps][Cin][Cout_p].
-// grid (ceil(Cout_p / 32), ceil(Cin_p / 32), taps), block (32, 8).
-__global__ void __launch_bounds__(256) split3_filter_kernel(const float* __restrict__ w, __nv_bfloat16* __restrict__ fwd,
-                                                            __nv_bfloat16* __restrict__ dx, int Cin, int Cout, int Cin_p, int Cout_p) {
-    pdl_wait();
-    __shared__ float tile[32][33];
-    const int tap = blockIdx.z, taps = gridDim.z;
-    const int n0 = blockIdx.x * 32, k0 = blockIdx.y * 32;
+// Tile `b` of 32 x 32 channels: output channels fastest, then input channels, then taps.
+__device__ __forceinline__ void split3_filter_tile(const float* __restrict__ w, __nv_bfloat16* __restrict__ fwd, __nv_bfloat16* __restrict__ dx,
+                                                   int taps, int Cin, int Cout, int Cin_p, int Cout_p, int b, float (*tile)[33]) {
+    const int nt = (Cout_p + 31) / 32, kt = (Cin_p + 31) / 32, q = b / nt, tap = q / kt;
+    const int n0 = (b - q * nt) * 32, k0 = (q - tap * kt) * 32, tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
     auto put = [&](__nv_bfloat16* dst, size_t plane, size_t at, float v) {
-        __nv_bfloat16 a, b, c;
-        split3(v, a, b, c);
-        dst[at] = a;
-        dst[at + plane] = b;
-        dst[at + 2 * plane] = c;
+        __nv_bfloat16 x, y, z;
+        split3(v, x, y, z);
+        dst[at] = x;
+        dst[at + plane] = y;
+        dst[at + 2 * plane] = z;
     };
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
-        const int k = k0 + threadIdx.y + 8 * r, n = n0 + threadIdx.x;
+        const int k = k0 + ty + 8 * r, n = n0 + tx;
         const float v = (k < Cin && n < Cout) ? w[((size_t)tap * Cin + k) * Cout + n] : 0.f;
-        tile[threadIdx.y + 8 * r][threadIdx.x] = v;
+        tile[ty + 8 * r][tx] = v;
         if (dx != nullptr && k < Cin && n < Cout_p) put(dx, (size_t)taps * Cin * Cout_p, ((size_t)tap * Cin + k) * Cout_p + n, v);
     }
     if (fwd == nullptr) return;
     __syncthreads();
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
-        const int n = n0 + threadIdx.y + 8 * r, k = k0 + threadIdx.x;
-        if (n < Cout && k < Cin_p) put(fwd, (size_t)taps * Cout * Cin_p, ((size_t)tap * Cout + n) * Cin_p + k, tile[threadIdx.x][threadIdx.y + 8 * r]);
+        const int n = n0 + ty + 8 * r, k = k0 + tx;
+        if (n < Cout && k < Cin_p) put(fwd, (size_t)taps * Cout * Cin_p, ((size_t)tap * Cout + n) * Cin_p + k, tile[tx][ty + 8 * r]);
     }
+}
+
+// The parts of an array and, by the first `filter_blocks` CTAs, of the filter (one launch for what a forward pass needs).
+template <bool COLSUM, bool STRIDED>
+__global__ void __launch_bounds__(256) split3_kernel(const float* __restrict__ src, __nv_bfloat16* __restrict__ dst, long long rows, int C,
+                                                     int Cp, float* __restrict__ colsum_part, long long rows_per_block, const SplitPhases f,
+                                                     const float* __restrict__ w, __nv_bfloat16* __restrict__ fwd, __nv_bfloat16* __restrict__ dx,
+                                                     int taps, int Cin, int Cout, int Cin_p, int Cout_p, int filter_blocks) {
+    pdl_wait();
+    __shared__ float red[COLSUM ? 256 * 8 : 32 * 33];
+    if ((int)blockIdx.x < filter_blocks) {
+        split3_filter_tile(w, fwd, dx, taps, Cin, Cout, Cin_p, Cout_p, (int)blockIdx.x, reinterpret_cast<float (*)[33]>(red));
+        return;
+    }
+    split3_rows<COLSUM, STRIDED>(src, dst, rows, C, Cp, colsum_part, rows_per_block, f, (int)blockIdx.x - filter_blocks, red);
 }
 
 // ====================================================================================== host side
@@ -866,41 +877,31 @@ static int run_split_igemm(const AetherConvDesc& d, const SplitPlan& pl, bool dx
     return p.NT <= 64 ? launch_split<64, false, 64>(p, prof, st) : launch_split<128, false, 64>(p, prof, st);
 }
 
-static int launch_split3(const float* src, void* dst, long long rows, int C, int Cp, const SplitPhases& f, float* colsum, int blocks, cudaStream_t st) {
+// The parts of src and, when w is given, of the filter's operands (fwd nullable).
+static int launch_split3(const AetherConvDesc& d, const SplitPlan& pl, const float* src, void* dst, long long rows, int C, int Cp, const SplitPhases& f,
+                         float* colsum, const float* w, void* fwd, void* dx, cudaStream_t st) {
     const int lanes = Cp / 8 >= 256 ? 1 : 256 / (Cp / 8);
-    __nv_bfloat16* out = static_cast<__nv_bfloat16*>(dst);
+    long long nb = colsum ? pl.db_blocks : 8LL * num_sms();
+    if (!colsum && nb * lanes > rows) nb = (rows + lanes - 1) / lanes;
+    const int filter = w ? ceil_div(pl.Cout_p, 32) * ceil_div(pl.Cin_p, 32) * pl.taps : 0;
+    const auto kernel = colsum ? split3_kernel<true, false> : f.sH * f.sW > 1 ? split3_kernel<false, true> : split3_kernel<false, false>;
     prof_begin(PK_SHADOW, st);
-    if (colsum) {
-        launch(split3_kernel<true, false>, blocks, 256, 0, st, src, out, rows, C, Cp, colsum, (rows + blocks - 1) / blocks, f);
-    } else {
-        long long nb = 8LL * num_sms();
-        if (nb * lanes > rows) nb = (rows + lanes - 1) / lanes;
-        const long long per = (rows + nb - 1) / nb;
-        launch(f.sH * f.sW > 1 ? split3_kernel<false, true> : split3_kernel<false, false>, (int)nb, 256, 0, st, src, out, rows, C, Cp, nullptr, per, f);
-    }
+    launch(kernel, (int)nb + filter, 256, 0, st, src, static_cast<__nv_bfloat16*>(dst), rows, C, Cp, colsum, (rows + nb - 1) / nb, f, w,
+           static_cast<__nv_bfloat16*>(fwd), static_cast<__nv_bfloat16*>(dx), pl.taps, d.Cin, d.Cout, pl.Cin_p, pl.Cout_p, filter);
     prof_end(PK_SHADOW, st);
     count_launch();
     return check_launch("split3_kernel");
 }
 // The parts of x, by phases.
-static int split_x(const AetherConvDesc& d, const SplitPlan& pl, const float* x, void* dst, cudaStream_t st) {
+static int split_x(const AetherConvDesc& d, const SplitPlan& pl, const float* x, void* dst, const float* w, void* fwd, void* dx, cudaStream_t st) {
     const SplitPhases f = {d.H, d.W, d.sH, d.sW, pl.PH, pl.PW, 1LL * d.S * pl.PH * pl.PW};
-    return launch_split3(x, dst, f.images * d.sH * d.sW, d.Cin, pl.Cin_p, f, nullptr, 0, st);
-}
-
-static int launch_split3_filter(const AetherConvDesc& d, const SplitPlan& pl, const float* w, void* fwd, void* dx, cudaStream_t st) {
-    const dim3 grid((unsigned)ceil_div(pl.Cout_p, 32), (unsigned)ceil_div(pl.Cin_p, 32), (unsigned)pl.taps);
-    launch(split3_filter_kernel, grid, dim3(32, 8), 0, st, w, static_cast<__nv_bfloat16*>(fwd), static_cast<__nv_bfloat16*>(dx), d.Cin, d.Cout,
-           pl.Cin_p, pl.Cout_p);
-    count_launch();
-    return check_launch("split3_filter_kernel");
+    return launch_split3(d, pl, x, dst, f.images * d.sH * d.sW, d.Cin, pl.Cin_p, f, nullptr, w, fwd, dx, st);
 }
 
 int split_conv_fwd(const AetherConvDesc& d, const float* x, const float* w, const float* b, float* y, void* ws, cudaStream_t st) {
     const SplitPlan& pl = split_plan(d);
     uint8_t* wsb = static_cast<uint8_t*>(ws);
-    if (int rc = split_x(d, pl, x, wsb + pl.off_x, st)) return rc;
-    if (int rc = launch_split3_filter(d, pl, w, wsb + pl.off_wf, wsb + pl.off_wd, st)) return rc;
+    if (int rc = split_x(d, pl, x, wsb + pl.off_x, w, wsb + pl.off_wf, wsb + pl.off_wd, st)) return rc;
     return run_split_igemm(d, pl, false, x, wsb + pl.off_x, w, wsb + pl.off_wf, b, y, st);
 }
 
@@ -910,13 +911,16 @@ int split_conv_bwd(const AetherConvDesc& d, const float* x, const float* dy, con
     uint8_t* wsb = static_cast<uint8_t*>(ws);
     float* dbpart = reinterpret_cast<float*>(wsb + pl.off_dbpart);
     int rc;
-    if ((rc = launch_split3(dy, wsb + pl.off_dy, 1LL * d.S * pl.Ho * pl.Wo, d.Cout, pl.Cout_p, SplitPhases{0, 0, 1, 1, 0, 0, 0}, db ? dbpart : nullptr, pl.db_blocks, st))) return rc;
+    // (dX's filter operand too, where the forward pass has not left it)
+    const bool make_w = dx && !(copies_valid & AETHER_CONV_W_COPY_READY);
+    if ((rc = launch_split3(d, pl, dy, wsb + pl.off_dy, 1LL * d.S * pl.Ho * pl.Wo, d.Cout, pl.Cout_p, SplitPhases{0, 0, 1, 1, 0, 0, 0},
+                            db ? dbpart : nullptr, make_w ? w : nullptr, nullptr, wsb + pl.off_wd, st)))
+        return rc;
     if (dx) {
-        if (!(copies_valid & AETHER_CONV_W_COPY_READY) && (rc = launch_split3_filter(d, pl, w, nullptr, wsb + pl.off_wd, st))) return rc;
         if ((rc = run_split_igemm(d, pl, true, dy, wsb + pl.off_dy, w, wsb + pl.off_wd, nullptr, dx, st))) return rc;
     }
     if (!dw) return db ? colsum_finish(dbpart, pl.db_blocks, d.Cout, db, st) : AE_OK;
-    if (!(copies_valid & AETHER_CONV_X_COPY_READY) && (rc = split_x(d, pl, x, wsb + pl.off_x, st)))
+    if (!(copies_valid & AETHER_CONV_X_COPY_READY) && (rc = split_x(d, pl, x, wsb + pl.off_x, nullptr, nullptr, nullptr, st)))
         return rc;
     SplitParams p;
     memset(&p, 0, sizeof(p));

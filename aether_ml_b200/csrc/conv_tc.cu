@@ -18,6 +18,7 @@
 #include <cuda_bf16.h>
 
 #include "common.cuh"
+#include "finish_columns.cuh"
 #include "sm100_ptx.cuh"
 #include "stats_epilogue.cuh"
 #include "store_block.cuh"
@@ -782,33 +783,6 @@ __global__ void __launch_bounds__(DW_THREADS, 1) dw_conv_kernel(const __grid_con
         tc_fence_after();
         if (PAIR) tmem_dealloc_pair(tmem_base, 512);
         else tmem_dealloc(tmem_base, 512);
-    }
-}
-
-// out[c] = sum over blocks of part[block][C] for the eight columns of CTA `cta` (256 threads): 32 lanes per column, so
-// the serial chains are short, combined in fixed order.
-__device__ __forceinline__ void finish_columns(const float* __restrict__ part, int nblocks, int C, float* __restrict__ out, int cta,
-                                               float (*red)[8]) {
-    const int cl = threadIdx.x & 7, lane = threadIdx.x >> 3;
-    const int c = cta * 8 + cl;
-    float s = 0.f;
-    if (c < C) {
-        constexpr int U = 8;
-        for (int b = lane; b < nblocks; b += 32 * U) {
-            float v[U];
-#pragma unroll
-            for (int u = 0; u < U; ++u) v[u] = b + 32 * u < nblocks ? part[(size_t)(b + 32 * u) * C + c] : 0.f;
-#pragma unroll
-            for (int u = 0; u < U; ++u) s += v[u];
-        }
-    }
-    red[lane][cl] = s;
-    __syncthreads();
-    if (lane == 0 && c < C) {
-        float t = 0.f;
-#pragma unroll
-        for (int l = 0; l < 32; ++l) t += red[l][cl];
-        out[c] = t;
     }
 }
 
