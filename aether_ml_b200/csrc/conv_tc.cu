@@ -93,12 +93,12 @@ int make_map_nhwc(CUtensorMap* m, const void* base, CUtensorMapDataType dt, int 
 }
 // Row-major matrix (inner = K elements contiguous, `rows` rows), box (box_k, box_rows).
 int make_map_2d(CUtensorMap* m, const void* base, CUtensorMapDataType dt, int elt, int inner, long long rows, int box_k,
-                int box_rows) {
+                int box_rows, CUtensorMapSwizzle swz) {
     const cuuint64_t dims[2] = {(cuuint64_t)inner, (cuuint64_t)rows};
     const cuuint64_t strides[1] = {(cuuint64_t)inner * elt};
     const cuuint32_t box[2] = {(cuuint32_t)box_k, (cuuint32_t)box_rows};
     const cuuint32_t es[2] = {1, 1};
-    return make_map(m, base, dt, 2, dims, strides, box, es, CU_TENSOR_MAP_SWIZZLE_128B);
+    return make_map(m, base, dt, 2, dims, strides, box, es, swz);
 }
 
 // ====================================================================================== igemm (forward and dX)
@@ -145,15 +145,18 @@ static constexpr int IGEMM_STATS_BYTES = IGEMM_EPI_WARPS * STATS_WARP_FLOATS * 4
 
 // PAIR: two CTAs of a cluster share one 256-row MMA (cta_group::2).  Each holds its own 128 pixel rows and HALF of the
 // filter tile (NT/2 rows), so a stage is smaller and every SM pulls a third less from L2 per FLOP.
-template <int NT, bool PAIR = false>
+// RB: bytes of K per tile row; 64 (64-byte swizzle, four taps per stage) for layers of at most 32 channels, whose 128-byte rows would be
+// half zeros on their way from L2 (896 x 16x16 32->64 31.8 -> 26.2 us, 128 of them 9.5 -> 9.1).
+template <int NT, bool PAIR = false, int RB = 128>
 struct IgemmCfg {
     static constexpr int B_ROWS = PAIR ? NT / 2 : NT;           // filter rows this CTA stages
-    static constexpr int TILE_B_BYTES = B_ROWS * 128;
+    static constexpr int TILE_A_BYTES = 128 * RB;               // 128 pixel rows
+    static constexpr int TILE_B_BYTES = B_ROWS * RB;
     // 128-byte K chunks per stage: one thread issues for both SMs of a pair (and the MMAs of narrow tiles are short), and
     // with one chunk per stage its per-stage work (barrier wait, four MMAs, two commits) is not hidden behind the MMAs; a pair's stage takes two
-    static constexpr int KS = PAIR || NT <= 64 ? 2 : 1;
+    static constexpr int KS = RB == 64 ? 4 : PAIR || NT <= 64 ? 2 : 1;
     static constexpr int STAGE_A_BYTES = KS * TILE_A_BYTES, STAGE_B_BYTES = KS * TILE_B_BYTES;
-    static constexpr int STAGES = PAIR ? (NT == 256 ? 3 : 4) : ((NT == 256) ? 4 : (NT == 128 ? 6 : NT == 64 ? 4 : 5));
+    static constexpr int STAGES = RB == 64 ? (NT == 128 ? 3 : 4) : PAIR ? (NT == 256 ? 3 : 4) : ((NT == 256) ? 4 : (NT == 128 ? 6 : NT == 64 ? 4 : 5));
     static constexpr int SMEM_BYTES = 1024 + STAGES * (STAGE_A_BYTES + STAGE_B_BYTES) + IGEMM_TAIL + IGEMM_STATS_BYTES;
 };
 
@@ -170,11 +173,11 @@ struct IgemmCfg {
 // ACT: the epilogue also writes the (leaky) ReLU of the output and, when asked, the bf16 operand copy of that for the layer
 // behind (zero in the padded columns): a Dense layer and its activation of a small network are two launches of two
 // microseconds otherwise, three with the cast.
-template <bool TF32, int NT, bool STATS, bool PAIR, bool ACT = false>
+template <bool TF32, int NT, bool STATS, bool PAIR, bool ACT = false, int RB = 128>
 __global__ void __launch_bounds__(IGEMM_THREADS, 1) igemm_conv_kernel(const __grid_constant__ IgemmParams p) {
-    using Cfg = IgemmCfg<NT, PAIR>;
-    constexpr int STAGES = Cfg::STAGES;
-    constexpr int KC = TF32 ? 32 : 64;            // K elements per 128-byte row
+    using Cfg = IgemmCfg<NT, PAIR, RB>;
+    constexpr int STAGES = Cfg::STAGES, TILE_A_BYTES = Cfg::TILE_A_BYTES;
+    constexpr int KC = TF32 ? RB / 4 : RB / 2;    // K elements per row
     extern __shared__ uint8_t smem_raw[];
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     const uint32_t sA = smem_base;
@@ -243,7 +246,7 @@ __global__ void __launch_bounds__(IGEMM_THREADS, 1) igemm_conv_kernel(const __gr
     const int taps = p.fH * p.fW;
     const int kiters = taps * p.kchunks;
     // bytes per stage on the full barrier: this CTA's two boxes, in a pair those of both CTAs
-    const uint32_t chunk_tx = ((uint32_t)p.rows * 128u + (uint32_t)Cfg::B_ROWS * 128u) * (PAIR ? 2u : 1u);
+    const uint32_t chunk_tx = ((uint32_t)p.rows + (uint32_t)Cfg::B_ROWS) * (uint32_t)RB * (PAIR ? 2u : 1u);
     constexpr int KS = Cfg::KS;
 
     if (warp == 0) {
@@ -309,12 +312,12 @@ __global__ void __launch_bounds__(IGEMM_THREADS, 1) igemm_conv_kernel(const __gr
 #pragma unroll
                     for (int c = 0; c < KS; ++c) {
                         if (c < nsub) {
-                            const uint64_t da = make_smem_desc(sA + s * Cfg::STAGE_A_BYTES + c * TILE_A_BYTES, 16, 1024);
-                            const uint64_t db = make_smem_desc(sB + s * Cfg::STAGE_B_BYTES + c * Cfg::TILE_B_BYTES, 16, 1024);
-                            const int nk = ++kc == p.kchunks ? p.last_ksteps : 4;
+                            const uint64_t da = make_smem_desc(sA + s * Cfg::STAGE_A_BYTES + c * TILE_A_BYTES, 16, 8 * RB, RB == 128 ? 2 : 4);
+                            const uint64_t db = make_smem_desc(sB + s * Cfg::STAGE_B_BYTES + c * Cfg::TILE_B_BYTES, 16, 8 * RB, RB == 128 ? 2 : 4);
+                            const int nk = ++kc == p.kchunks ? p.last_ksteps : RB / 32;
                             if (kc == p.kchunks) kc = 0;
 #pragma unroll
-                            for (int k = 0; k < 4; ++k) {                  // 32 bytes of K each: two 16-byte units further
+                            for (int k = 0; k < RB / 32; ++k) {            // 32 bytes of K each: two 16-byte units further
                                 const uint32_t acc = (k0 + c > 0 || k > 0) ? 1u : 0u;
                                 if (k >= nk) break;
                                 if (PAIR) umma_pair<TF32>(d_tmem, da + 2u * k, db + 2u * k, idesc, acc);
@@ -1272,11 +1275,11 @@ static int igemm_pair_grid(long long m_tiles, int n_tiles_n, bool stats) {
     return 2 * pairs;
 }
 
-template <bool TF32, int NT, bool STATS, bool PAIR, bool ACT = false>
+template <bool TF32, int NT, bool STATS, bool PAIR, bool ACT = false, int RB = 128>
 static int launch_igemm_k(const IgemmParams& p, cudaStream_t st) {
-    using Cfg = IgemmCfg<NT, PAIR>;
+    using Cfg = IgemmCfg<NT, PAIR, RB>;
     static PerDeviceSmem configured;
-    if (int rc = ensure_dynamic_smem(igemm_conv_kernel<TF32, NT, STATS, PAIR, ACT>, Cfg::SMEM_BYTES, configured, "igemm_conv")) return rc;
+    if (int rc = ensure_dynamic_smem(igemm_conv_kernel<TF32, NT, STATS, PAIR, ACT, RB>, Cfg::SMEM_BYTES, configured, "igemm_conv")) return rc;
     const long long m_tiles = 1LL * p.tiles_w * p.tiles_h * p.tiles_n;
     const int grid = PAIR ? igemm_pair_grid(m_tiles, p.n_tiles_n, STATS) : igemm_grid(m_tiles, p.n_tiles_n, STATS);
     if (STATS && (grid / (PAIR ? 2 : 1)) % p.n_tiles_n)
@@ -1284,9 +1287,9 @@ static int launch_igemm_k(const IgemmParams& p, cudaStream_t st) {
     const int pk = p.sgn > 0 ? PK_IGEMM_FWD : PK_IGEMM_DX;
     prof_begin(pk, st);
     if (PAIR) {
-        launch_cluster(igemm_conv_kernel<TF32, NT, STATS, PAIR, ACT>, 2, grid, IGEMM_THREADS, Cfg::SMEM_BYTES, st, p);
+        launch_cluster(igemm_conv_kernel<TF32, NT, STATS, PAIR, ACT, RB>, 2, grid, IGEMM_THREADS, Cfg::SMEM_BYTES, st, p);
     } else {
-        launch(igemm_conv_kernel<TF32, NT, STATS, PAIR, ACT>, grid, IGEMM_THREADS, Cfg::SMEM_BYTES, st, p);
+        launch(igemm_conv_kernel<TF32, NT, STATS, PAIR, ACT, RB>, grid, IGEMM_THREADS, Cfg::SMEM_BYTES, st, p);
     }
     prof_end(pk, st);
     count_launch();
@@ -1294,7 +1297,10 @@ static int launch_igemm_k(const IgemmParams& p, cudaStream_t st) {
 }
 
 template <bool TF32, int NT>
-static int launch_igemm(const IgemmParams& p, bool pair, cudaStream_t st) {
+static int launch_igemm(const IgemmParams& p, bool pair, bool narrow, cudaStream_t st) {
+    if constexpr (!TF32 && NT <= 128) {
+        if (narrow) return p.stats ? launch_igemm_k<false, NT, true, false, false, 64>(p, st) : launch_igemm_k<false, NT, false, false, false, 64>(p, st);
+    }
     if constexpr (NT == 256 || NT == 128) {
         if (pair) return p.stats ? launch_igemm_k<TF32, NT, true, true>(p, st) : launch_igemm_k<TF32, NT, false, true>(p, st);
     }
@@ -1305,12 +1311,12 @@ static int launch_igemm(const IgemmParams& p, bool pair, cudaStream_t st) {
 }
 
 template <bool TF32>
-static int dispatch_igemm(IgemmParams& p, int nt, bool pair, cudaStream_t st) {
+static int dispatch_igemm(IgemmParams& p, int nt, bool pair, bool narrow, cudaStream_t st) {
     switch (nt) {
-        case 256: return launch_igemm<TF32, 256>(p, pair, st);
-        case 128: return launch_igemm<TF32, 128>(p, pair, st);
-        case 64: return launch_igemm<TF32, 64>(p, false, st);
-        default: return launch_igemm<TF32, 32>(p, false, st);
+        case 256: return launch_igemm<TF32, 256>(p, pair, narrow, st);
+        case 128: return launch_igemm<TF32, 128>(p, pair, narrow, st);
+        case 64: return launch_igemm<TF32, 64>(p, false, narrow, st);
+        default: return launch_igemm<TF32, 32>(p, false, narrow, st);
     }
 }
 
@@ -1331,13 +1337,15 @@ static int run_igemm(bool tf32, const void* in, int in_C, int in_H, int in_W, in
     IgemmParams p;
     memset(&p, 0, sizeof(p));
     const int elt = tf32 ? 4 : 2;
-    const int KC = 128 / elt;
     const CUtensorMapDataType dt = tf32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
     const int nt = pick_nt(n_padded, til.total());
     const bool pair = igemm_use_pairs(til.total(), nt, ceil_div(n_padded, nt));   // each CTA of a pair stages half the filter rows
+    const bool narrow = !tf32 && !pair && k_real <= 32 && nt <= 128 && (act == nullptr || stats != nullptr);
+    const int KC = narrow ? 32 : 128 / elt;
+    const CUtensorMapSwizzle swz = narrow ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B;
     int rc;
-    if ((rc = make_map_nhwc(&p.tm_in, in, dt, elt, in_C, in_W, in_H, S, KC, til.BW, til.BH, til.BN))) return rc;
-    if ((rc = make_map_2d(&p.tm_w, wmat, dt, elt, w_inner, 1LL * taps * rows_per_tap, KC, pair ? nt / 2 : nt))) return rc;
+    if ((rc = make_map_nhwc(&p.tm_in, in, dt, elt, in_C, in_W, in_H, S, KC, til.BW, til.BH, til.BN, swz))) return rc;
+    if ((rc = make_map_2d(&p.tm_w, wmat, dt, elt, w_inner, 1LL * taps * rows_per_tap, KC, pair ? nt / 2 : nt, swz))) return rc;
     if ((reinterpret_cast<uintptr_t>(out) & 15u) || (out_C & 3))
         return set_error(AE_BAD_ARG, "conv output must be 16-byte aligned with a channel count that is a multiple of 4");
     p.out = out;
@@ -1355,9 +1363,9 @@ static int run_igemm(bool tf32, const void* in, int in_C, int in_H, int in_W, in
     p.n_tiles_n = ceil_div(n_padded, nt);
     p.rows_per_tap = rows_per_tap;
     p.fH = fH; p.fW = fW; p.sgn = sgn; p.off_h = off_h; p.off_w = off_w;
-    p.kchunks = ceil_div(in_C, KC);
-    p.last_ksteps = last_ksteps(k_real, p.kchunks, KC);
-    return tf32 ? dispatch_igemm<true>(p, nt, pair, st) : dispatch_igemm<false>(p, nt, pair, st);
+    p.kchunks = narrow ? 1 : ceil_div(in_C, KC);
+    p.last_ksteps = narrow ? ceil_div(k_real, 16) : last_ksteps(k_real, p.kchunks, KC);
+    return tf32 ? dispatch_igemm<true>(p, nt, pair, false, st) : dispatch_igemm<false>(p, nt, pair, narrow, st);
 }
 
 static int launch_cast(const float* src, __nv_bfloat16* dst, long long rows, int C, int Cp, float* colsum_part,

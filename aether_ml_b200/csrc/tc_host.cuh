@@ -49,9 +49,9 @@ int make_map_nhwc(CUtensorMap* m, const void* base, CUtensorMapDataType dt, int 
 // Tensor map of any rank: sizes, byte strides of all dimensions but the innermost, box and element strides.
 int make_map(CUtensorMap* m, const void* base, CUtensorMapDataType dt, int rank, const cuuint64_t* dims, const cuuint64_t* strides,
              const cuuint32_t* box, const cuuint32_t* estr, CUtensorMapSwizzle swz);
-// Row-major matrix (inner = K elements contiguous, `rows` rows), box (box_k, box_rows), 128-byte swizzle.
+// Row-major matrix (inner = K elements contiguous, `rows` rows), box (box_k, box_rows); 128-byte swizzle unless told otherwise.
 int make_map_2d(CUtensorMap* m, const void* base, CUtensorMapDataType dt, int elt, int inner, long long rows, int box_k,
-                int box_rows);
+                int box_rows, CUtensorMapSwizzle swz = CU_TENSOR_MAP_SWIZZLE_128B);
 // Halo-reuse kernel (conv_halo.cu): launches and sets *used when the problem fits it, else leaves *used false.
 int run_halo_igemm(bool tf32, const void* in, int in_C, int in_H, int in_W, int S, const void* wmat, int w_inner,
                    int rows_per_tap, int taps, float* out, int out_C, int out_H, int out_W, int n_padded, int fH, int fW,
