@@ -71,8 +71,8 @@ int simt_conv_bwd_filter(const AetherConvDesc& d, const float* x, const float* d
                          size_t ws_bytes, cudaStream_t st);
 size_t simt_conv_workspace_bytes(const AetherConvDesc& d);
 
-// ---- conv_split.cu : fp32 convolution on the tensor cores, operands as sums of three bf16 numbers (any stride up to 8, any
-// channel counts from 8); which shapes gain from it: split_conv_eligible
+// ---- conv_split.cu : fp32 convolution on the tensor cores, operands as sums of three bf16 numbers (strides up to 4, any
+// channel counts from 16); which shapes gain from it: split_conv_eligible
 bool split_conv_eligible(const AetherConvDesc& d);
 size_t split_conv_workspace_bytes(const AetherConvDesc& d);
 int split_conv_fwd(const AetherConvDesc& d, const float* x, const float* w, const float* b, float* y, void* ws, cudaStream_t st);

@@ -20,9 +20,9 @@
 // parts are made by a pass over x and dy (split3_kernel: 4 bytes read, 6 written, dB on the way) and copied by TMA, rows of 64
 // channels with zeros behind the last: channel counts need not be multiples of anything.  A strided layer's x is stored by
 // phases, so that a tap's pixels lie side by side (element strides in the tensor map halve the copies' rate).
-// Measured on B200, forward + backward, CUDA cores / this file: 40 x 33x32 64->128 444 / 118 us, 96 x 28x28 32->64 209 / 105, 100 x 57x45
-// 48->72 stride 2 432 / 199.  Bound by shared memory: the MMAs' operand reads (28 KB per step of 64 columns, 219 clocks) and the copies'
-// writes (16-18 KB) share its 128 bytes a clock.
+// Measured on B200, forward + backward, CUDA cores / this file: 40 x 33x32 64->128 444 / 132 us, 96 x 28x28 32->64 211 / 100, 100 x 57x45
+// 48->72 stride 2 432 / 196 (three sets of inputs in turn).  Bound by shared memory: the MMAs' operand reads (28 KB per step of 64
+// columns, 219 clocks) and the copies' writes (16-18 KB) share its 128 bytes a clock, the tensor pipe is 42-47 % busy, DRAM 5-14 %.
 #include <string.h>
 
 #include <cuda_bf16.h>
@@ -763,8 +763,8 @@ static SplitPlan compute_split_plan(const AetherConvDesc& d) {
     if ((in_rows * pl.Cin_p + out_rows * pl.Cout_p) * 6 > (2ull << 30)) return pl;      // (the parts are scratch of the caller's)
     // What the FMA kernels take for a layer (33 TFLOP/s) must be worth the passes that make the parts (5 TB/s) and the longer way
     // through the kernels.  Forward and backward on B200, CUDA cores / split, us: 209 x 23x18 36->16 stride 2 60 / 65, 17 x 13x21
-    // 32->16 5x5 36 / 42 and 2 x 9x10 65->130 36 / 47 stay; 6 x 16x16 32->165 5x5 71 / 71, 12 x 24x24 16->146 71 / 50, 6 x 43x43
-    // 88->188 1x1 53 / 46, 208 x 53x48 16->64 stride 2 254 / 235, 24 x 18x18 48->208 stride 2 98 / 43, 123 x 18x18 36->46 5x5 532 / 154 go.
+    // 32->16 5x5 36 / 42 and 2 x 9x10 65->130 36 / 47 stay; 6 x 16x16 32->165 5x5 88 / 74, 12 x 24x24 16->146 70 / 50, 6 x 43x43
+    // 88->188 1x1 53 / 44, 208 x 53x48 16->64 stride 2 255 / 203, 24 x 18x18 48->208 stride 2 98 / 40, 123 x 18x18 36->46 5x5 532 / 152 go.
     const double fma_us = 6.0 * d.S * pl.Ho * pl.Wo * pl.taps * d.Cin * d.Cout / 33e6;
     const double parts_us = (1.0 * in_rows * (4.0 * d.Cin / (d.sH * d.sW) + 6.0 * pl.Cin_p) + 1.0 * out_rows * (4.0 * d.Cout + 6.0 * pl.Cout_p)) / 5e6;
     if (fma_us < 12.0 + 1.6 * parts_us) return pl;
