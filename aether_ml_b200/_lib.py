@@ -61,6 +61,7 @@ SIGNATURES = {
     "aether_head_supported": (_I, [_D]),
     "aether_head_softmax_fwd": (_I, [_D, _P, _P, _P, _P, _P, _P]),
     "aether_head_cce_bwd": (_I, [_D, _P, _P, _P, _P, _F, _P, _P, _P, _P]),
+    "aether_head_cce_bwd_ex": (_I, [_D, _P, _P, _P, _P, _F, _P, _P, _P, _P, _P, _P, _P, _SZ, _P]),
     "aether_act_bwd_copy": (_I, [_P, _P, _P, _I, _I, _F, _P, _I, _P, _P]),
     "aether_conv2d_bwd_ex": (_I, [_D, _P, _P, _P, _P, _P, _P, _P, _SZ, _I, _I, _P]),
     "aether_bn_act_pool_fwd_copy": (_I, [_P, _P, _I64, _P, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _F, _F, _F, _P,

@@ -269,11 +269,17 @@ extern "C" int aether_head_softmax_fwd(const AetherConvDesc* d, const float* x, 
 
 extern "C" int aether_head_cce_bwd(const AetherConvDesc* d, const float* prob, const int32_t* labels, const int64_t* labels64,
                                    const float* targets, float smooth, const float* w, float* dz, float* dx, void* stream) {
+    return aether_head_cce_bwd_ex(d, prob, labels, labels64, targets, smooth, nullptr, w, dz, dx, nullptr, nullptr, nullptr, 0, stream);
+}
+
+extern "C" int aether_head_cce_bwd_ex(const AetherConvDesc* d, const float* prob, const int32_t* labels, const int64_t* labels64,
+                                      const float* targets, float smooth, const float* x, const float* w, float* dz, float* dx, float* dw,
+                                      float* db, void* ws, size_t ws_bytes, void* stream) {
     if (int rc = head_check(d, "aether_head_cce_bwd")) return rc;
-    if (!prob || !w || !dz || !dx || (labels != nullptr) + (labels64 != nullptr) + (targets != nullptr) != 1)
+    if (!prob || !w || !dz || !dx || (dw && !x) || (labels != nullptr) + (labels64 != nullptr) + (targets != nullptr) != 1)
         return set_error(AE_BAD_ARG, "aether_head_cce_bwd: null pointer, or not one kind of labels");
-    if (!aligned16(w) || !aligned16(dx)) return set_error(AE_BAD_ARG, "aether_head_cce_bwd: arrays must be 16-byte aligned");
-    return generic_head_cce_bwd(*d, prob, labels, reinterpret_cast<const long long*>(labels64), targets, smooth, w, dz, dx,
+    if (!aligned16(x) || !aligned16(w) || !aligned16(dx) || !aligned16(ws)) return set_error(AE_BAD_ARG, "aether_head_cce_bwd: arrays must be 16-byte aligned");
+    return generic_head_cce_bwd(*d, prob, labels, reinterpret_cast<const long long*>(labels64), targets, smooth, x, w, dz, dx, dw, db, ws, ws_bytes,
                                 static_cast<cudaStream_t>(stream));
 }
 
@@ -351,6 +357,11 @@ extern "C" int aether_conv2d_bwd_ex(const AetherConvDesc* d, const float* x, con
     if (tc_conv_eligible(*d)) return tc_conv_bwd(*d, x, dy, w, dx, dw, db, ws, ws_bytes, x_shadow_valid, dy_colsum_rows, st);
     if ((dx || dw) && split_route(*d) && ws && ws_bytes >= split_conv_workspace_bytes(*d))
         return split_conv_bwd(*d, x, dy, w, dx, dw, db, ws, x_shadow_valid, st);
+    if (generic_head_shape(*d) && (x || dx)) {           // (without x: dX alone; dB goes the general way)
+        rc = generic_head_bwd(*d, x, dy, w, dx, x ? dw : nullptr, x ? db : nullptr, ws, ws_bytes, st);
+        if (rc || x || !db) return rc;
+        dx = nullptr;
+    }
     if (dx && (rc = generic_conv_bwd_data(*d, dy, w, dx, ws, ws_bytes, st))) return rc;
     if (dw && first_tc_bwd_eligible(*d))
         return first_tc_bwd_filter(*d, x, dy, dw, db, ws, ws_bytes, dy_ready ? dy_colsum_rows : 0, st);

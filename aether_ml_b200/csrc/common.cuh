@@ -83,8 +83,11 @@ int split_conv_bwd(const AetherConvDesc& d, const float* x, const float* dy, con
 // classifier heads (pointwise, few outputs) with the softmax / the combined softmax and cross-entropy gradient in the kernel
 bool generic_head_shape(const AetherConvDesc& d);
 int generic_head_softmax_fwd(const AetherConvDesc& d, const float* x, const float* w, const float* b, float* y, float* prob, cudaStream_t st);
+int generic_head_bwd(const AetherConvDesc& d, const float* x, const float* dy, const float* w, float* dx, float* dw, float* db, void* ws,
+                     size_t ws_bytes, cudaStream_t st);
 int generic_head_cce_bwd(const AetherConvDesc& d, const float* prob, const int* labels, const long long* labels64, const float* targets,
-                         float smooth, const float* w, float* dz, float* dx, cudaStream_t st);
+                         float smooth, const float* x, const float* w, float* dz, float* dx, float* dw, float* db, void* ws, size_t ws_bytes,
+                         cudaStream_t st);
 int generic_conv_fwd(const AetherConvDesc& d, const float* x, const float* w, const float* b, float* y, void* ws, size_t ws_bytes,
                      cudaStream_t st);
 int generic_conv_bwd_data(const AetherConvDesc& d, const float* dy, const float* w, float* dx, void* ws, size_t ws_bytes, cudaStream_t st);

@@ -11,34 +11,66 @@ namespace aether {
 // Here a warp takes a row: the lanes split the channels (float4 loads of x, the row is read once), keep Cout partial
 // sums each and combine them with shuffles in a fixed order.
 // The filter is kept transposed in shared memory, wT[d][Cin], so a lane's four channels of output d are one 16-byte
-// shared-memory read (4 * Cout scalar global loads per four channels before).
+// shared-memory read (4 * Cout scalar global loads per four channels before).  Its 16-byte loads are all in flight before the first
+// store: with scalar ones in a loop of their own the copy was a third of a small layer's time.
 // (rows of Cin + 4 floats: with Cin a multiple of 32 the outputs of one channel would all fall on one bank)
 __device__ __forceinline__ void head_load_filter_T(const float* __restrict__ w, float* wT, int Cin, int Cout) {
-    for (int i = threadIdx.x; i < Cin * Cout; i += blockDim.x) {
-        const int c = i / Cout, d = i - c * Cout;
-        wT[d * (Cin + 4) + c] = w[i];
+    constexpr int U = 4;
+    const int n4 = (Cin * Cout) >> 2;
+    for (int i0 = threadIdx.x; i0 < n4; i0 += U * blockDim.x) {
+        float4 v[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (i0 + u * (int)blockDim.x < n4) v[u] = __ldg(reinterpret_cast<const float4*>(w) + i0 + u * (int)blockDim.x);
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int i = i0 + u * (int)blockDim.x;
+            if (i >= n4) break;
+            int c = (int)(4u * (unsigned)i / (unsigned)Cout), d = 4 * i - c * Cout;
+            const float e[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                wT[d * (Cin + 4) + c] = e[k];
+                if (++d == Cout) { d = 0; ++c; }
+            }
+        }
     }
     __syncthreads();
 }
 
+// Bound by latency: a batch of 128 rows of 256 channels is 16 blocks and one row per warp.  The first row is requested before the
+// filter is copied, and the lanes' sums of 16 outputs meet in four halving exchanges (the lane's output is lane / 2) and one that
+// adds: 16 shuffles, in the order of the 80 that a butterfly per output takes.  With its softmax, as
+// a train of launches, before / after: 128 x 256->10 4.9 / 3.5 us, 1024 x 1024->10 14.9 / 9.9, 4096 x 1024->10 23.0 / 18.5.
 template <int MAXD>
 __global__ void __launch_bounds__(256) gen_fwd_pointwise_few_kernel(const float* __restrict__ x, const float* __restrict__ w,
                                                                     const float* __restrict__ b, float* __restrict__ y,
                                                                     long long rows, int Cin, int Cout, float* __restrict__ prob) {
+    static_assert(MAXD == 16, "the halving exchange below");
     pdl_wait();
     extern __shared__ __align__(16) float head_wT[];
-    head_load_filter_T(w, head_wT, Cin, Cout);
-    const int lane = threadIdx.x & 31;
+    const int lane = threadIdx.x & 31, out = lane >> 1;
     const long long warp0 = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
     const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
     const int C4 = Cin >> 2;
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 next[2];                                          // the next row's first channels, requested a row ahead
+#pragma unroll
+    for (int u = 0; u < 2; ++u)
+        next[u] = warp0 < rows && lane + 32 * u < C4 ? reinterpret_cast<const float4*>(x + (size_t)warp0 * Cin)[lane + 32 * u] : zero;
+    const float bias = b != nullptr && out < Cout ? b[out] : 0.f;
+    head_load_filter_T(w, head_wT, Cin, Cout);
     for (long long row = warp0; row < rows; row += nwarps) {
         float acc[MAXD];
 #pragma unroll
         for (int d = 0; d < MAXD; ++d) acc[d] = 0.f;
         const float4* xr = reinterpret_cast<const float4*>(x + (size_t)row * Cin);
+        const float4 v0 = next[0], v1 = next[1];
+#pragma unroll
+        for (int u = 0; u < 2; ++u)
+            next[u] = row + nwarps < rows && lane + 32 * u < C4 ? reinterpret_cast<const float4*>(x + (size_t)(row + nwarps) * Cin)[lane + 32 * u] : zero;
         for (int c4 = lane; c4 < C4; c4 += 32) {
-            const float4 v = xr[c4];
+            const float4 v = c4 < 32 ? v0 : c4 < 64 ? v1 : xr[c4];
 #pragma unroll
             for (int d = 0; d < MAXD; ++d) {
                 if (d < Cout) {
@@ -48,27 +80,29 @@ __global__ void __launch_bounds__(256) gen_fwd_pointwise_few_kernel(const float*
             }
         }
 #pragma unroll
-        for (int d = 0; d < MAXD; ++d) {
+        for (int n = MAXD / 2; n > 0; n >>= 1) {             // partner 2 n lanes on: each keeps n of the 2 n outputs
+            const bool hi = lane & (2 * n);
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) acc[d] += __shfl_xor_sync(0xffffffffu, acc[d], o);
+            for (int d = 0; d < n; ++d) {
+                const float give = hi ? acc[d] : acc[d + n], keep = hi ? acc[d + n] : acc[d];
+                acc[d] = keep + __shfl_xor_sync(0xffffffffu, give, 2 * n);
+            }
         }
+        const float sum_x = acc[0] + __shfl_xor_sync(0xffffffffu, acc[0], 1);
         float z = -INFINITY;
-        if (lane < Cout) {
-            float r = 0.f;
-#pragma unroll
-            for (int d = 0; d < MAXD; ++d) r = (d == lane) ? acc[d] : r;
-            z = r + (b ? b[lane] : 0.f);
-            y[(size_t)row * Cout + lane] = z;
+        if (out < Cout) {
+            z = sum_x + bias;
+            if (!(lane & 1)) y[(size_t)row * Cout + out] = z;
         }
         if (prob != nullptr) {                               // the softmax behind the head, as softmax_cce_kernel computes it
             float mx = z;
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-            const float e = lane < Cout ? expf(z - mx) : 0.f;
+            for (int o = 16; o > 1; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+            const float e = out < Cout ? expf(z - mx) : 0.f;
             float sum = e;
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-            if (lane < Cout) prob[(size_t)row * Cout + lane] = e / sum;
+            for (int o = 16; o > 1; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+            if (out < Cout && !(lane & 1)) prob[(size_t)row * Cout + out] = e / sum;
         }
     }
 }
@@ -202,10 +236,16 @@ __global__ void __launch_bounds__(256, 2) dx_fewc_kernel(const float* __restrict
 }
 
 // ---------------------------------------------------------------------------------- classifier heads, backward
-// dx[p][c] = sum_d dy[p][d] * w[c][d] for a pointwise layer with few outputs: a block takes a row at a time, a thread
-// four channels; the filter is read transposed from shared memory, the row of dy is the same address for every thread.
+// All of a head's backward pass in one launch: blocks for dW (16 channels each, the first adds dB up), blocks for dX; each is a few round trips
+// to L2 long, and one behind the other they were three launches.  With the loss gradient,
+// three launches / one: 128 x 256->10 10.4 / 3.2 us, 512 x 512 15.8 / 5.9, 1024 x 1024 25.4 / 13.4.  Above HEAD_DW_ROWS rows dW and dB are sums of parts
+// (head_dw_partial_kernel below).
+//
+// dx[p][c] = sum_d dy[p][d] * w[c][d]: a block is row lanes x four-channel groups; the filter is read transposed from shared memory, the
+// row of dy is the same address for every thread of a row.  dw[c][d] = sum_p x[p][c] * dy[p][d]: a thread keeps four channels x Cout
+// sums over every 64th row (x read once, in 64-byte pieces; dy from shared memory), the sums meet in halving exchanges, then over the warps.
 // CCE: dy is not there yet -- it is the combined softmax / cross-entropy gradient (prob - y_smooth) / rows, which is computed
-// from the probabilities and the labels of the row (as softmax_cce_kernel does) and written to dz on the way.
+// from the probabilities and the labels of the row (as softmax_cce_kernel does) wherever it is read, and written to dz by the dX blocks.
 struct HeadCce {
     const float* prob;
     const int* labels;             // one of the three
@@ -214,50 +254,183 @@ struct HeadCce {
     float* dz;
     float smooth, inv_rows;
 };
+struct HeadBwd {
+    const float *x, *dy, *w;
+    float *dx, *dw, *db;           // each nullable
+    long long rows;
+    int Cin, Cout;
+    int dw_blocks;                 // the first blocks of the grid (the first of them: dB, too); the rest are dX's
+    int lanes, groups;             // dX: rows of a block, threads of a row
+    HeadCce cce;
+};
+static constexpr int HEAD_DW_CH = 16, HEAD_DW_CHUNK = 256, HEAD_DZ_LD = 20;      // (rows of 20 floats: eight rows' reads on 32 banks)
+static constexpr int HEAD_DW_SMEM = (HEAD_DW_CHUNK * HEAD_DZ_LD + 8 * 16 * HEAD_DW_CH) * (int)sizeof(float);
+
+__device__ __forceinline__ int head_label(const HeadCce& cce, long long row) {
+    return cce.labels ? cce.labels[row] : cce.labels64 ? (int)cce.labels64[row] : -1;
+}
+// dy at (row, d) from what `v` holds: dy itself or the probability.
+template <bool CCE>
+__device__ __forceinline__ float head_dy(const HeadCce& cce, float v, long long row, int d, int Cout, int label) {
+    if (!CCE) return v;
+    const float onehot = cce.targets ? cce.targets[(size_t)row * Cout + d] : (d == label ? 1.f : 0.f);
+    const float tb = onehot * (1.f - cce.smooth) + cce.smooth / Cout;
+    return (v - tb) * cce.inv_rows;
+}
+
 template <int MAXD, bool CCE>
-__global__ void __launch_bounds__(256) head_dx_kernel(const float* __restrict__ dy, const float* __restrict__ w,
-                                                      float* __restrict__ dx, long long rows, int Cin, int Cout, const HeadCce cce) {
-    pdl_wait();
-    extern __shared__ __align__(16) float head_wT[];
-    head_load_filter_T(w, head_wT, Cin, Cout);
-    const int C4 = Cin >> 2;
-    const float* src = CCE ? cce.prob : dy;
+__device__ __forceinline__ void head_dx_block(const HeadBwd& p, int block, int blocks, float* wT) {
+    head_load_filter_T(p.w, wT, p.Cin, p.Cout);
+    const int C4 = p.Cin >> 2;
+    const int rl = (int)threadIdx.x / p.groups, cl = (int)threadIdx.x - rl * p.groups;
+    if (rl >= p.lanes) return;
+    const float* src = CCE ? p.cce.prob : p.dy;
+    const long long row0 = (long long)block * p.lanes + rl, step = (long long)blocks * p.lanes;
     float gn[MAXD];                                     // the next row's dy values, requested one row ahead
 #pragma unroll
-    for (int d = 0; d < MAXD; ++d) gn[d] = (d < Cout && blockIdx.x < rows) ? __ldg(src + (size_t)blockIdx.x * Cout + d) : 0.f;
-    for (long long row = blockIdx.x; row < rows; row += gridDim.x) {
+    for (int d = 0; d < MAXD; ++d) gn[d] = (d < p.Cout && row0 < p.rows) ? __ldg(src + (size_t)row0 * p.Cout + d) : 0.f;
+    for (long long row = row0; row < p.rows; row += step) {
         float g[MAXD];
-        const long long nrow = row + gridDim.x;
+        const long long nrow = row + step;
+        const int label = CCE ? head_label(p.cce, row) : 0;
 #pragma unroll
         for (int d = 0; d < MAXD; ++d) {
-            g[d] = gn[d];
-            gn[d] = (d < Cout && nrow < rows) ? __ldg(src + (size_t)nrow * Cout + d) : 0.f;
+            if (d < p.Cout) g[d] = head_dy<CCE>(p.cce, gn[d], row, d, p.Cout, label);
+            gn[d] = (d < p.Cout && nrow < p.rows) ? __ldg(src + (size_t)nrow * p.Cout + d) : 0.f;
+            if (CCE && d < p.Cout && cl == d) p.cce.dz[(size_t)row * p.Cout + d] = g[d];
         }
-        if (CCE) {
-            const int label = cce.labels ? cce.labels[row] : cce.labels64 ? (int)cce.labels64[row] : -1;
-#pragma unroll
-            for (int d = 0; d < MAXD; ++d) {
-                if (d < Cout) {
-                    const float onehot = cce.targets ? cce.targets[(size_t)row * Cout + d] : (d == label ? 1.f : 0.f);
-                    const float tb = onehot * (1.f - cce.smooth) + cce.smooth / Cout;
-                    g[d] = (g[d] - tb) * cce.inv_rows;
-                    if ((int)threadIdx.x == d) cce.dz[(size_t)row * Cout + d] = g[d];
-                }
-            }
-        }
-        float4* out = reinterpret_cast<float4*>(dx + (size_t)row * Cin);
-        for (int c4 = threadIdx.x; c4 < C4; c4 += blockDim.x) {
+        float4* out = reinterpret_cast<float4*>(p.dx + (size_t)row * p.Cin);
+        for (int c4 = cl; c4 < C4; c4 += p.groups) {
             float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
             for (int d = 0; d < MAXD; ++d) {
-                if (d < Cout) {
-                    const float4 k = *reinterpret_cast<const float4*>(head_wT + d * (Cin + 4) + 4 * c4);
+                if (d < p.Cout) {
+                    const float4 k = *reinterpret_cast<const float4*>(wT + d * (p.Cin + 4) + 4 * c4);
                     a.x = fmaf(g[d], k.x, a.x); a.y = fmaf(g[d], k.y, a.y); a.z = fmaf(g[d], k.z, a.z); a.w = fmaf(g[d], k.w, a.w);
                 }
             }
             out[c4] = a;
         }
     }
+}
+
+template <int MAXD, bool CCE>
+__device__ __forceinline__ void head_dw_block(const HeadBwd& p, int block, float* smem) {
+    static_assert(MAXD == 16, "the halving exchange below");
+    float* dz_s = smem;
+    float* red = smem + HEAD_DW_CHUNK * HEAD_DZ_LD;     // [warp][output][channel]
+    const int lane = threadIdx.x & 31, cg = threadIdx.x & 3, rl = threadIdx.x >> 2;
+    const int C4 = p.Cin >> 2, c4 = block * (HEAD_DW_CH / 4) + cg, rows = (int)p.rows;
+    const float* src = CCE ? p.cce.prob : p.dy;
+    float4 acc[MAXD];
+#pragma unroll
+    for (int d = 0; d < MAXD; ++d) acc[d] = make_float4(0.f, 0.f, 0.f, 0.f);
+    float sdy = 0.f;                                    // block 0: column sums of dy, output threadIdx.x & 15, every 16th row
+    float4 v[HEAD_DW_CHUNK / 64];                       // this chunk's x, and dy of the thread's own row: requested a chunk ahead
+    float g[MAXD];
+    int label = 0;
+    auto request = [&](int r0) {
+#pragma unroll
+        for (int u = 0; u < HEAD_DW_CHUNK / 64; ++u) {
+            const int r = r0 + u * 64 + rl;
+            v[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (r < rows && c4 < C4) v[u] = __ldg(reinterpret_cast<const float4*>(p.x) + (size_t)r * C4 + c4);
+        }
+        const int r = r0 + (int)threadIdx.x;
+        if (r < rows) {
+#pragma unroll
+            for (int d = 0; d < MAXD; ++d)
+                if (d < p.Cout) g[d] = __ldg(src + (size_t)r * p.Cout + d);
+            if (CCE) label = head_label(p.cce, r);
+        }
+    };
+    request(0);
+    for (int r0 = 0; r0 < rows; r0 += HEAD_DW_CHUNK) {
+        if (r0 > 0) __syncthreads();
+        if (r0 + (int)threadIdx.x < rows) {
+#pragma unroll
+            for (int d = 0; d < MAXD; ++d)
+                if (d < p.Cout) dz_s[threadIdx.x * HEAD_DZ_LD + d] = head_dy<CCE>(p.cce, g[d], r0 + (int)threadIdx.x, d, p.Cout, label);
+        }
+        float4 xv[HEAD_DW_CHUNK / 64];
+#pragma unroll
+        for (int u = 0; u < HEAD_DW_CHUNK / 64; ++u) xv[u] = v[u];
+        if (r0 + HEAD_DW_CHUNK < rows) request(r0 + HEAD_DW_CHUNK);
+        __syncthreads();
+#pragma unroll
+        for (int u = 0; u < HEAD_DW_CHUNK / 64; ++u) {
+            if (r0 + u * 64 + rl >= rows) continue;
+            const float4* gr = reinterpret_cast<const float4*>(dz_s + (u * 64 + rl) * HEAD_DZ_LD);
+#pragma unroll
+            for (int q = 0; q < MAXD / 4; ++q) {
+                if (4 * q >= p.Cout) break;
+                const float4 g4 = gr[q];                // (entries from Cout on are read and not used)
+                const float gk[4] = {g4.x, g4.y, g4.z, g4.w};
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    if (4 * q + k < p.Cout) {
+                        float4& a = acc[4 * q + k];
+                        a.x = fmaf(xv[u].x, gk[k], a.x); a.y = fmaf(xv[u].y, gk[k], a.y);
+                        a.z = fmaf(xv[u].z, gk[k], a.z); a.w = fmaf(xv[u].w, gk[k], a.w);
+                    }
+                }
+            }
+        }
+        if (block == 0 && p.db != nullptr && (threadIdx.x & 15) < p.Cout) {
+            const int n = rows - r0 < HEAD_DW_CHUNK ? rows - r0 : HEAD_DW_CHUNK;
+            float t[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+            for (int l = 0; l < HEAD_DW_CHUNK / 16; ++l) {
+                const int r = ((int)threadIdx.x >> 4) + 16 * l;
+                if (r < n) t[l & 3] += dz_s[r * HEAD_DZ_LD + (threadIdx.x & 15)];
+            }
+            sdy += (t[0] + t[1]) + (t[2] + t[3]);
+        }
+    }
+    // A warp's eight rows: partner 2 n lanes on, each keeps n of the 2 n outputs.
+#pragma unroll
+    for (int n = MAXD / 2; n > 1; n >>= 1) {
+        const bool hi = lane & (2 * n);
+#pragma unroll
+        for (int d = 0; d < n; ++d) {
+            const float4 give = hi ? acc[d] : acc[d + n], keep = hi ? acc[d + n] : acc[d];
+            acc[d].x = keep.x + __shfl_xor_sync(0xffffffffu, give.x, 2 * n);
+            acc[d].y = keep.y + __shfl_xor_sync(0xffffffffu, give.y, 2 * n);
+            acc[d].z = keep.z + __shfl_xor_sync(0xffffffffu, give.z, 2 * n);
+            acc[d].w = keep.w + __shfl_xor_sync(0xffffffffu, give.w, 2 * n);
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < 2; ++k)
+        *reinterpret_cast<float4*>(red + ((threadIdx.x >> 5) * MAXD + (lane >> 2) * 2 + k) * HEAD_DW_CH + cg * 4) = acc[k];
+    __syncthreads();
+    const int c = (int)(threadIdx.x / (unsigned)p.Cout), d = (int)threadIdx.x - c * p.Cout;
+    if (p.dw != nullptr && c < HEAD_DW_CH && block * HEAD_DW_CH + c < p.Cin) {
+        float s = 0.f;
+#pragma unroll
+        for (int w = 0; w < 8; ++w) s += red[(w * MAXD + d) * HEAD_DW_CH + c];
+        p.dw[(size_t)(block * HEAD_DW_CH + c) * p.Cout + d] = s;
+    }
+    if (block == 0 && p.db != nullptr) {
+        __syncthreads();
+        red[threadIdx.x] = sdy;
+        __syncthreads();
+        if (threadIdx.x < p.Cout) {
+            float t[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+            for (int l = 0; l < 16; ++l) t[l & 3] += red[l * 16 + threadIdx.x];
+            p.db[threadIdx.x] = (t[0] + t[1]) + (t[2] + t[3]);
+        }
+    }
+}
+
+template <int MAXD, bool CCE>
+__global__ void __launch_bounds__(256, 2) head_bwd_kernel(const HeadBwd p) {
+    pdl_wait();
+    extern __shared__ __align__(16) float head_smem[];
+    const int b = blockIdx.x;
+    if (b < p.dw_blocks) head_dw_block<MAXD, CCE>(p, b, head_smem);
+    else head_dx_block<MAXD, CCE>(p, b - p.dw_blocks, gridDim.x - p.dw_blocks, head_smem);
 }
 
 // dw[c][d] = sum_p x[p][c] * dy[p][d], db[d] = sum_p dy[p][d] over a part of the rows: partials [part][Cout + 1][Cin]
@@ -363,23 +536,6 @@ int generic_head_softmax_fwd(const AetherConvDesc& d, const float* x, const floa
     return head_fwd(d, x, w, b, y, prob, st);
 }
 
-static int head_dx(const AetherConvDesc& d, const float* dy, const float* w, float* dx, const HeadCce* cce, cudaStream_t st) {
-    const long long rows = 1LL * d.S * d.H * d.W;
-    const int smem = (d.Cin + 4) * d.Cout * (int)sizeof(float);
-    static PerDeviceSmem configured[2];
-    const auto kernel = cce ? head_dx_kernel<16, true> : head_dx_kernel<16, false>;
-    if (int rc = ensure_dynamic_smem(kernel, 96 * 1024, configured[cce ? 1 : 0], "head dX")) return rc;
-    const long long nb = rows < 2LL * num_sms() ? rows : 2LL * num_sms();
-    launch(kernel, (int)nb, 256, smem, st, dy, w, dx, rows, d.Cin, d.Cout, cce ? *cce : HeadCce{});
-    count_launch();
-    return check_launch("head_dx_kernel");
-}
-int generic_head_cce_bwd(const AetherConvDesc& d, const float* prob, const int* labels, const long long* labels64, const float* targets,
-                         float smooth, const float* w, float* dz, float* dx, cudaStream_t st) {
-    const HeadCce cce = {prob, labels, labels64, targets, dz, smooth, 1.f / (float)(1LL * d.S * d.H * d.W)};
-    return head_dx(d, nullptr, w, dx, &cce, st);
-}
-
 template <int CIN, int FB>
 static void dx_fewc_launch(const AetherConvDesc& d, const float* dy, const float* w, float* dx, int Ho, int Wo, cudaStream_t st) {
     const bool vec = d.Cout % 4 == 0 && ((reinterpret_cast<uintptr_t>(dy) | reinterpret_cast<uintptr_t>(w)) & 15u) == 0;
@@ -412,7 +568,6 @@ int generic_conv_bwd_data(const AetherConvDesc& d, const float* dy, const float*
             default: return dx_fewc<4>(d, dy, w, dx, Ho, Wo, st);
         }
     }
-    if (head_shape(d) && (reinterpret_cast<uintptr_t>(dx) & 15u) == 0) return head_dx(d, dy, w, dx, nullptr, st);
     return simt_conv_bwd_data(d, dy, w, dx, ws, ws_bytes, st);
 }
 
@@ -431,21 +586,70 @@ size_t generic_conv_workspace_bytes(const AetherConvDesc& d) {
 
 int generic_conv_bwd_filter(const AetherConvDesc& d, const float* x, const float* dy, float* dw, float* db, void* ws,
                             size_t ws_bytes, cudaStream_t st) {
-    if (!head_shape(d) || x == nullptr || (reinterpret_cast<uintptr_t>(x) & 15u)) return simt_conv_bwd_filter(d, x, dy, dw, db, ws, ws_bytes, st);
-    if (!ws || ws_bytes < generic_conv_workspace_bytes(d))
+    return simt_conv_bwd_filter(d, x, dy, dw, db, ws, ws_bytes, st);
+}
+
+// Most rows whose dW comes out of one launch: a thread's sum is over every 64th row, 16 of them here, as long as the parts' below.  One
+// launch is faster for more rows, too (2048 x 256->10 18.8 us against 21.7, 4096 x 1024->10 41.7 against 58.8), but from there on its longer
+// sums are the less accurate ones (dW at 4096 rows 1.30e-7 off float64 against 1.14e-7; at 1024 1.00e-7 against 1.05e-7).
+static constexpr int HEAD_DW_ROWS = 1024;
+
+static int head_bwd(const AetherConvDesc& d, const float* x, const float* dy, const float* w, float* dx, float* dw, float* db, void* ws,
+                    size_t ws_bytes, const HeadCce* cce, cudaStream_t st) {
+    const bool sums = dw != nullptr || db != nullptr;
+    if (sums && (!ws || ws_bytes < generic_conv_workspace_bytes(d)))
         return set_error(AE_BAD_ARG, "conv workspace too small: %zu < %zu", ws_bytes, generic_conv_workspace_bytes(d));
-    const int parts = head_dw_parts(d), C4 = d.Cin / 4;
+    const int C4 = d.Cin / 4;
+    HeadBwd p = {};
+    p.x = x; p.dy = dy; p.w = w; p.dx = dx; p.dw = dw; p.db = db;
+    p.rows = 1LL * d.S * d.H * d.W;
+    p.Cin = d.Cin;
+    p.Cout = d.Cout;
+    if (cce) p.cce = *cce;
+    const bool parted = p.rows > HEAD_DW_ROWS;
+    p.dw_blocks = !sums || parted ? 0 : dw ? ceil_div(d.Cin, HEAD_DW_CH) : 1;
+    p.groups = C4 < 256 ? C4 : 256;
+    p.lanes = 256 / p.groups;
+    long long dx_blocks = 0;
+    if (dx) {
+        dx_blocks = (p.rows + p.lanes - 1) / p.lanes;
+        // What is resident at once, for every block copies the filter.
+        const long long most = p.dw_blocks < num_sms() ? 2LL * num_sms() - p.dw_blocks : num_sms();
+        if (dx_blocks > most) dx_blocks = most;
+    }
+    if (const int grid = p.dw_blocks + (int)dx_blocks) {
+        static PerDeviceSmem configured[2];
+        const auto kernel = cce ? head_bwd_kernel<16, true> : head_bwd_kernel<16, false>;
+        if (int rc = ensure_dynamic_smem(kernel, 96 * 1024, configured[cce ? 1 : 0], "head backward")) return rc;
+        const int filter = dx ? (d.Cin + 4) * d.Cout * (int)sizeof(float) : 0, tile = p.dw_blocks ? HEAD_DW_SMEM : 0;
+        launch(kernel, grid, 256, filter > tile ? filter : tile, st, p);
+        count_launch();
+        if (int rc = check_launch("head_bwd_kernel")) return rc;
+    }
+    if (!sums || !parted) return AE_OK;
+    const int parts = head_dw_parts(d);
     int lanes = 1;                                       // row lanes per block: as many as whole channel rows fit 256 threads
     while (lanes * 2 <= parts && C4 * lanes * 2 <= 256) lanes *= 2;
     const int groups = 256 / lanes;
     float* part = static_cast<float*>(ws);
-    launch(head_dw_partial_kernel<16>, dim3(ceil_div(parts, lanes), ceil_div(C4, groups)), 256, 0, st, x, dy, part, 1LL * d.S * d.H * d.W, d.Cin,
+    launch(head_dw_partial_kernel<16>, dim3(ceil_div(parts, lanes), ceil_div(C4, groups)), 256, 0, st, x, cce ? cce->dz : dy, part, p.rows, d.Cin,
            d.Cout, lanes, parts);
     count_launch();
     if (int rc = check_launch("head_dw_partial_kernel")) return rc;
     launch(head_dw_reduce_kernel, ceil_div((d.Cin + 1) * d.Cout, 32), 256, 0, st, part, parts, d.Cin, d.Cout, dw, db);
     count_launch();
     return check_launch("head_dw_reduce_kernel");
+}
+
+int generic_head_bwd(const AetherConvDesc& d, const float* x, const float* dy, const float* w, float* dx, float* dw, float* db, void* ws,
+                     size_t ws_bytes, cudaStream_t st) {
+    return head_bwd(d, x, dy, w, dx, dw, db, ws, ws_bytes, nullptr, st);
+}
+int generic_head_cce_bwd(const AetherConvDesc& d, const float* prob, const int* labels, const long long* labels64, const float* targets,
+                         float smooth, const float* x, const float* w, float* dz, float* dx, float* dw, float* db, void* ws, size_t ws_bytes,
+                         cudaStream_t st) {
+    const HeadCce cce = {prob, labels, labels64, targets, dz, smooth, 1.f / (float)(1LL * d.S * d.H * d.W)};
+    return head_bwd(d, x, nullptr, w, dx, dw, db, ws, ws_bytes, &cce, st);
 }
 
 }  // namespace aether

@@ -141,7 +141,7 @@ struct Entry<int (*)(A...)> {
     X(aether_bn_act_pool_fwd_copy) X(aether_chain_fwd) X(aether_pool_fwd) X(aether_pool_bwd) X(aether_leaky_relu_fwd)                      \
     X(aether_leaky_relu_bwd) X(aether_channel_scale) X(aether_dropout_fwd) X(aether_mul) X(aether_adam_step)           \
     X(aether_adam_step_dev) X(aether_dropout_fwd_dev) X(aether_channel_mask_dev) X(aether_regularizer_grad)            \
-    X(aether_regularizer_loss) X(aether_copy) X(aether_conv2d_act_fwd) X(aether_act_bwd_copy) X(aether_head_softmax_fwd) X(aether_head_cce_bwd) X(aether_softmax_cce) X(aether_softmax_cce_i64) X(aether_softmax_bwd) X(aether_softmax_cce_targets)
+    X(aether_regularizer_loss) X(aether_copy) X(aether_conv2d_act_fwd) X(aether_act_bwd_copy) X(aether_head_softmax_fwd) X(aether_head_cce_bwd_ex) X(aether_softmax_cce) X(aether_softmax_cce_i64) X(aether_softmax_bwd) X(aether_softmax_cce_targets)
 
 #define DECLARE(name)                                                                                                  \
     void* fn_##name = nullptr;                                                                                         \

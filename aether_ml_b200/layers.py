@@ -1036,8 +1036,13 @@ class Layer_Dense(_TakesCopies, _Saved):
         dz, dx = H.empty_like(prob), H.empty_like(self.inputs)
         kinds = [None, None, None]
         kinds[2 if labels.ndim == 2 else 1 if labels.dtype is torch.int64 else 0] = labels
-        H.aether_head_cce_bwd(p.raw, prob, *kinds, smooth, self.weights, dz, dx)
-        self._backward(dz, False, p, dx)
+        x, w = self.inputs, self.weights
+        ws = self._ws.get(p.ws_bytes)
+        if not (self._copies.flags(ws, x, w) & _lib.CONV_X_COPY_READY):
+            _require_written(x, "Layer_Dense.backward")
+        H.aether_head_cce_bwd_ex(p.raw, prob, *kinds, smooth, x, w, dz, dx, self.dweights, self.dbiases, ws, self._ws.size)
+        self._regularize()
+        self.dinputs = dx
         return dz
 
     def _gradients(self):
@@ -1062,29 +1067,31 @@ class Layer_Dense(_TakesCopies, _Saved):
                               lay.dy_copy_ld, self.dbiases)
         return dy, self._backward(dy, True, p)
 
-    def _backward(self, dy, dy_ready, p, dx=None):
-        """``dy_ready``: the operand copy of dy and dbiases are there already; ``dx``: dinputs, when they are."""
+    def _backward(self, dy, dy_ready, p):
+        """``dy_ready``: the operand copy of dy and dbiases are there already."""
         x = self.inputs
         w = self.weights
         H = host()
         ws = self._ws.get(p.ws_bytes)
-        want = None
-        if dx is None:
-            dx = want = H.empty_like(x)
+        dx = H.empty_like(x)
         flags = self._copies.flags(ws, x, w)
         if not (flags & _lib.CONV_X_COPY_READY):
             _require_written(x, "Layer_Dense.backward")
         if dy_ready:
-            H.aether_conv2d_bwd_ex(p.raw, x, dy, w, want, self.dweights, None, ws, self._ws.size, flags | _lib.CONV_DY_COPY_READY, 1)
+            H.aether_conv2d_bwd_ex(p.raw, x, dy, w, dx, self.dweights, None, ws, self._ws.size, flags | _lib.CONV_DY_COPY_READY, 1)
         else:
-            H.aether_conv2d_bwd_ex(p.raw, x, dy, w, want, self.dweights, self.dbiases, ws, self._ws.size, flags, 0)
-        if self.weight_regularizer_l1 > 0 or self.weight_regularizer_l2 > 0:
-            H.aether_regularizer_grad(w, self.dweights, w.numel(), self.weight_regularizer_l1, self.weight_regularizer_l2)
-        if self.bias_regularizer_l1 > 0 or self.bias_regularizer_l2 > 0:
-            H.aether_regularizer_grad(self.biases, self.dbiases, self.biases.numel(), self.bias_regularizer_l1,
-                                      self.bias_regularizer_l2)
+            H.aether_conv2d_bwd_ex(p.raw, x, dy, w, dx, self.dweights, self.dbiases, ws, self._ws.size, flags, 0)
+        self._regularize()
         self.dinputs = dx
         return self.dinputs
+
+    def _regularize(self):
+        w = self.weights
+        if self.weight_regularizer_l1 > 0 or self.weight_regularizer_l2 > 0:
+            host().aether_regularizer_grad(w, self.dweights, w.numel(), self.weight_regularizer_l1, self.weight_regularizer_l2)
+        if self.bias_regularizer_l1 > 0 or self.bias_regularizer_l2 > 0:
+            host().aether_regularizer_grad(self.biases, self.dbiases, self.biases.numel(), self.bias_regularizer_l1,
+                                           self.bias_regularizer_l2)
 
     def get_parameters(self):
         return self.weights, self.biases

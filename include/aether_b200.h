@@ -154,13 +154,17 @@ int aether_act_bwd_copy(const float* x, const float* dy, float* dx, int rows, in
                         float* db, void* stream);
 
 /* A classifier head (a Dense layer with at most 16 outputs) and the SoftMax behind it: logits y and probabilities prob in one
- * launch, and the combined softmax / cross-entropy gradient (aether_softmax_cce's dz) with the head's dX in one.  One of
- * labels, labels64 and targets is given.  aether_head_supported: whether the shape is such a head. */
+ * launch, and the combined softmax / cross-entropy gradient (aether_softmax_cce's dz) with the head's dX in one; _ex: its
+ * dW and dB, too (each nullable; ws as for aether_conv2d_bwd).  One of labels, labels64 and targets is given.
+ * aether_head_supported: whether the shape is such a head. */
 int aether_head_supported(const AetherConvDesc* desc);
 int aether_head_softmax_fwd(const AetherConvDesc* desc, const float* x, const float* w, const float* b, float* y, float* prob,
                             void* stream);
 int aether_head_cce_bwd(const AetherConvDesc* desc, const float* prob, const int32_t* labels, const int64_t* labels64,
                         const float* targets, float smooth, const float* w, float* dz, float* dx, void* stream);
+int aether_head_cce_bwd_ex(const AetherConvDesc* desc, const float* prob, const int32_t* labels, const int64_t* labels64,
+                           const float* targets, float smooth, const float* x, const float* w, float* dz, float* dx, float* dw,
+                           float* db, void* ws, size_t ws_bytes, void* stream);
 int aether_conv2d_bwd_ex(const AetherConvDesc* desc, const float* x, const float* dy, const float* w, float* dx, float* dw,
                          float* db, void* ws, size_t ws_bytes, int x_shadow_valid, int dy_colsum_rows, void* stream);
 
