@@ -238,7 +238,8 @@ __global__ void __launch_bounds__(256, 2) dx_fewc_kernel(const float* __restrict
 // ---------------------------------------------------------------------------------- classifier heads, backward
 // All of a head's backward pass in one launch: blocks for dW (16 channels each, the first adds dB up), blocks for dX; each is a few round trips
 // to L2 long, and one behind the other they were three launches.  With the loss gradient,
-// three launches / one: 128 x 256->10 10.4 / 3.2 us, 512 x 512 15.8 / 5.9, 1024 x 1024 25.4 / 13.4.  Above HEAD_DW_ROWS rows dW and dB are sums of parts
+// three launches / one: 128 x 256->10 10.4 / 3.2 us, 512 x 512 15.8 / 6.1, 1024 x 1024 25.4 / 12.7, 4096 x 1024 (three launches here, too: labels
+// are requested a row ahead) 55.9 / 52.6.  Above HEAD_DW_ROWS rows dW and dB are sums of parts
 // (head_dw_partial_kernel below).
 //
 // dx[p][c] = sum_d dy[p][d] * w[c][d]: a block is row lanes x four-channel groups; the filter is read transposed from shared memory, the
@@ -286,18 +287,28 @@ __device__ __forceinline__ void head_dx_block(const HeadBwd& p, int block, int b
     if (rl >= p.lanes) return;
     const float* src = CCE ? p.cce.prob : p.dy;
     const long long row0 = (long long)block * p.lanes + rl, step = (long long)blocks * p.lanes;
-    float gn[MAXD];                                     // the next row's dy values, requested one row ahead
+    float gn[MAXD];                                     // the next row's dy values and label, requested one row ahead
+    int next_label = CCE && row0 < p.rows ? head_label(p.cce, row0) : 0;
 #pragma unroll
     for (int d = 0; d < MAXD; ++d) gn[d] = (d < p.Cout && row0 < p.rows) ? __ldg(src + (size_t)row0 * p.Cout + d) : 0.f;
     for (long long row = row0; row < p.rows; row += step) {
         float g[MAXD];
         const long long nrow = row + step;
-        const int label = CCE ? head_label(p.cce, row) : 0;
+        const int label = next_label;
+        if (CCE && nrow < p.rows) next_label = head_label(p.cce, nrow);
 #pragma unroll
         for (int d = 0; d < MAXD; ++d) {
-            if (d < p.Cout) g[d] = head_dy<CCE>(p.cce, gn[d], row, d, p.Cout, label);
+            g[d] = gn[d];
             gn[d] = (d < p.Cout && nrow < p.rows) ? __ldg(src + (size_t)nrow * p.Cout + d) : 0.f;
-            if (CCE && d < p.Cout && cl == d) p.cce.dz[(size_t)row * p.Cout + d] = g[d];
+        }
+        if (CCE) {
+#pragma unroll
+            for (int d = 0; d < MAXD; ++d) {
+                if (d < p.Cout) {
+                    g[d] = head_dy<CCE>(p.cce, g[d], row, d, p.Cout, label);
+                    if (cl == d) p.cce.dz[(size_t)row * p.Cout + d] = g[d];
+                }
+            }
         }
         float4* out = reinterpret_cast<float4*>(p.dx + (size_t)row * p.Cin);
         for (int c4 = cl; c4 < C4; c4 += p.groups) {
@@ -590,7 +601,7 @@ int generic_conv_bwd_filter(const AetherConvDesc& d, const float* x, const float
 }
 
 // Most rows whose dW comes out of one launch: a thread's sum is over every 64th row, 16 of them here, as long as the parts' below.  One
-// launch is faster for more rows, too (2048 x 256->10 18.8 us against 21.7, 4096 x 1024->10 41.7 against 58.8), but from there on its longer
+// launch is faster for more rows, too (2048 x 256->10 18.8 us against 21.1, 4096 x 1024->10 41.7 against 52.6), but from there on its longer
 // sums are the less accurate ones (dW at 4096 rows 1.30e-7 off float64 against 1.14e-7; at 1024 1.00e-7 against 1.05e-7).
 static constexpr int HEAD_DW_ROWS = 1024;
 
