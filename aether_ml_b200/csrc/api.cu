@@ -276,8 +276,8 @@ extern "C" int aether_head_cce_bwd_ex(const AetherConvDesc* d, const float* prob
                                       const float* targets, float smooth, const float* x, const float* w, float* dz, float* dx, float* dw,
                                       float* db, void* ws, size_t ws_bytes, void* stream) {
     if (int rc = head_check(d, "aether_head_cce_bwd")) return rc;
-    if (!prob || !w || !dz || !dx || (dw && !x) || (labels != nullptr) + (labels64 != nullptr) + (targets != nullptr) != 1)
-        return set_error(AE_BAD_ARG, "aether_head_cce_bwd: null pointer, or not one kind of labels");
+    if (!prob || !w || !dz || !dx || ((dw || db) && !x) || (labels != nullptr) + (labels64 != nullptr) + (targets != nullptr) != 1)
+        return set_error(AE_BAD_ARG, "aether_head_cce_bwd: null pointer (dw and db need x), or not one kind of labels");
     if (!aligned16(x) || !aligned16(w) || !aligned16(dx) || !aligned16(ws)) return set_error(AE_BAD_ARG, "aether_head_cce_bwd: arrays must be 16-byte aligned");
     return generic_head_cce_bwd(*d, prob, labels, reinterpret_cast<const long long*>(labels64), targets, smooth, x, w, dz, dx, dw, db, ws, ws_bytes,
                                 static_cast<cudaStream_t>(stream));

@@ -155,7 +155,7 @@ int aether_act_bwd_copy(const float* x, const float* dy, float* dx, int rows, in
 
 /* A classifier head (a Dense layer with at most 16 outputs) and the SoftMax behind it: logits y and probabilities prob in one
  * launch, and the combined softmax / cross-entropy gradient (aether_softmax_cce's dz) with the head's dX in one; _ex: its
- * dW and dB, too (each nullable; ws as for aether_conv2d_bwd).  One of labels, labels64 and targets is given.
+ * dW and dB, too (each nullable; either needs x, and ws as for aether_conv2d_bwd).  One of labels, labels64 and targets is given.
  * aether_head_supported: whether the shape is such a head. */
 int aether_head_supported(const AetherConvDesc* desc);
 int aether_head_softmax_fwd(const AetherConvDesc* desc, const float* x, const float* w, const float* b, float* y, float* prob,

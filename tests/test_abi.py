@@ -57,6 +57,16 @@ def test_conv_argument_checks(lib):
     assert lib.aether_conv2d_workspace_bytes(C.byref(mode)) == 0
 
 
+def test_head_gradient_argument_checks(lib):
+    head = _lib.AetherConvDesc(64, 1, 1, 256, 10, 1, 1, 1, 1, 0, 0, 0)
+    assert lib.aether_head_supported(C.byref(head))
+    call = lambda x, dw, db: lib.aether_head_cce_bwd_ex(C.byref(head), 16, 16, None, None, 0.0, x, 16, 16, 16, dw, db, 16, 1 << 30, None)
+    for dw, db in ((16, None), (None, 16), (16, 16)):                        # both are sums over x's rows in one kernel
+        assert call(None, dw, db) == -1
+        assert b"need x" in lib.aether_last_error()
+    assert call(8, 16, 16) == -1 and b"aligned" in lib.aether_last_error()
+
+
 def test_workspace_query_is_pure(lib):
     for mode in (0, 1, 2):
         d = _lib.AetherConvDesc(256, 56, 56, 64, 128, 3, 3, 1, 1, 1, 1, mode)
