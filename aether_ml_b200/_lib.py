@@ -51,6 +51,8 @@ SIGNATURES = {
     "aether_profile_read": (_I, [_I, C.POINTER(C.c_double), C.POINTER(C.c_int)]),
     "aether_profile_reset": (None, []),
     "aether_conv2d_workspace_bytes": (_SZ, [_D]),
+    "aether_conv2d_fwd_workspace_bytes": (_SZ, [_D]),
+    "aether_conv2d_least_workspace_bytes": (_SZ, [_D]),
     "aether_conv2d_fwd": (_I, [_D, _P, _P, _P, _P, _P, _SZ, _P]),
     "aether_conv2d_bnstats_blocks": (_I64, [_D]),
     "aether_conv2d_fwd_bnstats": (_I, [_D, _P, _P, _P, _P, _P, _SZ, _P, _SZ, _P]),

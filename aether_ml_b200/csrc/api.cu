@@ -196,6 +196,16 @@ extern "C" size_t aether_conv2d_workspace_bytes(const AetherConvDesc* d) {
     return t > g ? t : g;
 }
 
+extern "C" size_t aether_conv2d_fwd_workspace_bytes(const AetherConvDesc* d) {
+    const size_t all = aether_conv2d_workspace_bytes(d);
+    return all && split_route(*d) ? split_conv_fwd_workspace_bytes(*d) : all;
+}
+
+extern "C" size_t aether_conv2d_least_workspace_bytes(const AetherConvDesc* d) {
+    const size_t all = aether_conv2d_workspace_bytes(d);
+    return all && split_route(*d) ? generic_conv_workspace_bytes(*d) : all;
+}
+
 extern "C" int aether_conv2d_operand_layout(const AetherConvDesc* d, AetherOperandLayout* out) {
     if (!out) return 0;
     memset(out, 0, sizeof(*out));
@@ -295,7 +305,7 @@ extern "C" int aether_conv2d_fwd(const AetherConvDesc* d, const float* x, const 
     if (tc_conv_eligible(*d)) return tc_conv_fwd(*d, x, w, b, y, nullptr, ws, ws_bytes, 0, st);
     if (first_tc_eligible(*d)) return first_tc_fwd(*d, x, w, b, y, nullptr, st);
     if (smallc_conv_eligible(*d) && (!b || aligned16(b))) return smallc_conv_fwd(*d, x, w, b, y, nullptr, st);
-    if (split_route(*d) && ws && ws_bytes >= split_conv_workspace_bytes(*d)) return split_conv_fwd(*d, x, w, b, y, ws, st);
+    if (split_route(*d) && ws && ws_bytes >= split_conv_fwd_workspace_bytes(*d)) return split_conv_fwd(*d, x, w, b, y, ws, st);
     return generic_conv_fwd(*d, x, w, b, y, ws, ws_bytes, st);
 }
 

@@ -75,6 +75,7 @@ size_t simt_conv_workspace_bytes(const AetherConvDesc& d);
 // channel counts from 16); which shapes gain from it: split_conv_eligible
 bool split_conv_eligible(const AetherConvDesc& d);
 size_t split_conv_workspace_bytes(const AetherConvDesc& d);
+size_t split_conv_fwd_workspace_bytes(const AetherConvDesc& d);      // of that, what a forward pass uses
 int split_conv_fwd(const AetherConvDesc& d, const float* x, const float* w, const float* b, float* y, void* ws, cudaStream_t st);
 int split_conv_bwd(const AetherConvDesc& d, const float* x, const float* dy, const float* w, float* dx, float* dw, float* db, void* ws,
                    int copies_valid, cudaStream_t st);

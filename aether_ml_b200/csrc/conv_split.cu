@@ -704,7 +704,7 @@ struct SplitPlan {
     int Ho, Wo, taps, Cin_p, Cout_p, PH, PW;      // PH, PW: a phase's extent
     PixelTiling til_fwd, til_dx, til_dw;
     int nt_fwd, nt_dx, kc_in, kc_out, splits, cblocks, U, ldn, db_blocks;
-    size_t off_wf, off_wd, off_x, off_dy, off_part, off_dbpart, total;
+    size_t off_wf, off_wd, off_x, off_dy, off_part, off_dbpart, fwd_total, total;      // (what a forward pass needs lies in front)
 };
 
 // The box of at most `most` pixels with the least to do: tiles times rows to the next `unit`, and half a unit for each tile (28x28 in boxes
@@ -788,6 +788,7 @@ static SplitPlan compute_split_plan(const AetherConvDesc& d) {
     pl.off_wf = take((size_t)3 * pl.taps * d.Cout * pl.Cin_p * 2);
     pl.off_wd = take((size_t)3 * pl.taps * d.Cin * pl.Cout_p * 2);
     pl.off_x = take(3 * in_rows * pl.Cin_p * 2);
+    pl.fwd_total = off;
     pl.off_dy = take(3 * out_rows * pl.Cout_p * 2);
     pl.off_part = take((size_t)pl.splits * pl.U * pl.kc_in * pl.ldn * 4);
     pl.off_dbpart = take((size_t)pl.db_blocks * d.Cout * 4);
@@ -798,6 +799,7 @@ static const SplitPlan& split_plan(const AetherConvDesc& d) { return cached_plan
 
 bool split_conv_eligible(const AetherConvDesc& d) { return split_plan(d).use; }
 size_t split_conv_workspace_bytes(const AetherConvDesc& d) { return split_plan(d).total; }
+size_t split_conv_fwd_workspace_bytes(const AetherConvDesc& d) { return split_plan(d).fwd_total; }
 
 // (C, W, H, N, part x phase) bf16, box kc channels x the pixels of `t`.
 static int split_pixel_map(CUtensorMap* m, const void* base, int Cp, int W, int H, int N, int phases, const PixelTiling& t, int kc) {

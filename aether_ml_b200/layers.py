@@ -10,6 +10,7 @@ Inputs may be torch CUDA tensors, objects exposing ``__cuda_array_interface__`` 
 NumPy arrays (copied to the device).  Outputs are torch CUDA tensors.
 """
 import ctypes as C
+import math
 import os
 import weakref
 
@@ -126,12 +127,25 @@ class _Workspace:
     def __init__(self):
         self.buf = None
         self.size = 0
+        self.refused = math.inf     # bytes that there was no memory for: from there on the least has to do
 
-    def get(self, nbytes):
+    def get(self, nbytes, plan=None):
+        """The buffer, of at least ``nbytes`` or, where there is no memory for that, of what the plan's calls can do with."""
         if self.size < nbytes or self.buf is None:
-            nbytes = max(int(nbytes), 256)
-            self.buf = host().empty_u8((nbytes,))
-            self.size = nbytes
+            if plan is None or nbytes < self.refused:
+                try:
+                    return self._grow(nbytes)
+                except torch.OutOfMemoryError:
+                    if plan is None or plan.least_ws_bytes() >= nbytes:
+                        raise
+                    self.refused = nbytes
+            return self.get(plan.least_ws_bytes())
+        return self.buf
+
+    def _grow(self, nbytes):
+        nbytes = max(int(nbytes), 256)
+        self.buf = host().empty_u8((nbytes,))
+        self.size = nbytes
         return self.buf
 
 
@@ -222,7 +236,7 @@ def _operand_layout(d):
 
 class _ConvPlan:
     """Sizes and queries of one convolution shape: the descriptor's bytes, the output shape (None when the filter does
-    not fit the padded input), the workspace, the operand layout and the blocks of epilogue statistics."""
+    not fit the padded input), the workspaces, the operand layout and the blocks of epilogue statistics."""
 
     def __init__(self, desc, Ho, Wo):
         d = C.byref(desc)
@@ -236,6 +250,14 @@ class _ConvPlan:
             self.stats_blocks = int(lib().aether_conv2d_bnstats_blocks(d))
             self.layout = _operand_layout(desc)
             self.head = bool(lib().aether_head_supported(d))
+        self.fwd_ws_bytes = self.ws_bytes              # of the workspace, what inference uses
+        # (less than all of it only where neither the kernels on operand copies nor those of first layers and heads serve the shape)
+        if self.layout is None and self.y_shape is not None and self.stats_blocks == 0 and not self.head:
+            self.fwd_ws_bytes = int(lib().aether_conv2d_fwd_workspace_bytes(d))
+
+    def least_ws_bytes(self):
+        """The workspace that every call can do with."""
+        return int(lib().aether_conv2d_least_workspace_bytes(AetherConvDesc.from_buffer_copy(self.raw)))
 
 
 # ------------------------------------------------------------------------------------- Conv_Layer
@@ -369,7 +391,7 @@ class Conv_Layer(_TakesCopies, _Saved):
         if p.y_shape is None:
             raise ValueError("filter larger than the padded input")
         H = host()
-        ws = self._ws.get(p.ws_bytes)
+        ws = self._ws.get(p.ws_bytes if training else p.fwd_ws_bytes, p)
         y = H.empty(p.y_shape)
         w = self.filter_weights
         flags = 0
@@ -405,7 +427,7 @@ class Conv_Layer(_TakesCopies, _Saved):
         if dy.shape != p.y_shape:
             raise ValueError(f"dvalues has shape {tuple(dy.shape)}, expected {p.y_shape}")
         H = host()
-        ws = self._ws.get(p.ws_bytes)
+        ws = self._ws.get(p.ws_bytes, p)
         w = self.filter_weights
         if getattr(self, "_grad_views", None) is not None:
             self.dweights, self.dbiases = self._grad_views
@@ -971,9 +993,9 @@ class Layer_Dense(_TakesCopies, _Saved):
             p = self._plan(self.inputs.shape[0])
         return p
 
-    def _operands(self, x, p):
+    def _operands(self, x, p, training=True):
         """(workspace, which operand copies in it are valid) for a forward pass over `x` by plan `p`."""
-        ws = self._ws.get(p.ws_bytes)
+        ws = self._ws.get(p.ws_bytes if training else p.fwd_ws_bytes, p)
         flags = 0
         if self._handed.x is not None:
             flags = _lib.CONV_X_COPY_READY if self._handed.x_ready(ws, x) else 0
@@ -990,7 +1012,7 @@ class Layer_Dense(_TakesCopies, _Saved):
         if x.ndim != 2 or x.shape[1] != w.shape[0]:
             raise ValueError(f"Layer_Dense expects (samples, {w.shape[0]}), got {tuple(x.shape)}")
         p = self._plan(x.shape[0])
-        ws, flags = self._operands(x, p)
+        ws, flags = self._operands(x, p, training)
         H = host()
         y = H.empty((x.shape[0], w.shape[1]))
         H.aether_conv2d_fwd_ex(p.raw, x, w, self.biases, y, None, 0, ws, self._ws.size, flags)
@@ -1072,7 +1094,7 @@ class Layer_Dense(_TakesCopies, _Saved):
         x = self.inputs
         w = self.weights
         H = host()
-        ws = self._ws.get(p.ws_bytes)
+        ws = self._ws.get(p.ws_bytes, p)
         dx = H.empty_like(x)
         flags = self._copies.flags(ws, x, w)
         if not (flags & _lib.CONV_X_COPY_READY):

@@ -969,7 +969,7 @@ class Model:
         limit = self.INFERENCE_PASS_BYTES
         n = min(most, max(1, limit // (per_sample * batch_size)) * batch_size)
         while n > batch_size:
-            need = n * per_sample + sum(l._plan((n, *shape) if shape else n).ws_bytes for l, shape in working)
+            need = n * per_sample + sum(l._plan((n, *shape) if shape else n).fwd_ws_bytes for l, shape in working)
             if need <= limit:
                 break
             n = max(1, min(n // batch_size - 1, n * limit // need // batch_size)) * batch_size

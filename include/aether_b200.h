@@ -86,6 +86,12 @@ void aether_profile_reset(void);
  * precision, split-K partial sums).  The same buffer should be passed to the forward and the
  * backward call of a layer. */
 size_t aether_conv2d_workspace_bytes(const AetherConvDesc* desc);
+/* The same for callers short of memory: what forward calls use of it, and the least that every call accepts.  They differ from the above
+ * for the layers that run in single precision on the tensor cores (AETHER_MATH_FP32): those keep 6 bytes per element of x and of dy,
+ * channels rounded up to 32 or 64, at most 2 GiB.  Forward calls use the part for x alone; with less than that forward calls, with less than the whole
+ * backward calls run on the CUDA cores. */
+size_t aether_conv2d_fwd_workspace_bytes(const AetherConvDesc* desc);
+size_t aether_conv2d_least_workspace_bytes(const AetherConvDesc* desc);
 
 /* Conv_Layer.forward, CNN_classes_cupy.py:70-120: y = conv(x, w) + b with zero padding.
  * x (S,H,W,Cin), w (fH,fW,Cin,Cout), b (Cout) or NULL, y (S,Ho,Wo,Cout). */

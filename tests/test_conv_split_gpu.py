@@ -16,6 +16,50 @@ SHAPES = [(9, 19, 17, 65, 130, 3, (1, 1), "same", "fp32"), (60, 15, 13, 37, 71, 
           (120, 12, 11, 100, 129, 1, (2, 2), "same", "fp32"), (60, 20, 21, 16, 50, 5, (1, 1), "same", "fp32"), (40, 33, 20, 90, 17, 3, (2, 1), "valid", "bf16"), (16, 7, 7, 256, 256, 3, (1, 1), "same", "fp32"), (90, 9, 10, 32, 144, 3, (1, 4), "same", "tf32")]
 
 
+def _split(shape):
+    """Whether the library takes these kernels for the shape (then forward calls use a part of the workspace only)."""
+    from aether_ml_b200 import _lib
+    S, H, W, Cin, Cout, f, st, pad, mode = shape
+    P = (f - 1) // 2 if pad == "same" else 0
+    d = _lib.AetherConvDesc(S, H, W, Cin, Cout, f, f, *st, P, P, _lib.MATH_MODES[mode])
+    return _lib.lib().aether_conv2d_fwd_workspace_bytes(d) < _lib.lib().aether_conv2d_workspace_bytes(d)
+
+
+def _reference(shape, x, w, b, dy):
+    """y, dX, dW and dB in float64 for arrays on the device."""
+    import torch
+    S, H, W, Cin, Cout, f, st, pad, mode = shape
+    xd, wd = x.double().requires_grad_(), w.double().requires_grad_()
+    y = torch.nn.functional.conv2d(xd.permute(0, 3, 1, 2), wd.permute(3, 2, 0, 1), stride=st, padding=(f - 1) // 2 if pad == "same" else 0).permute(0, 2, 3, 1)
+    y.backward(dy.double())
+    return y.detach() + b.double(), xd.grad, wd.grad, dy.double().sum((0, 1, 2))
+
+
+def _off(got, want):
+    return float((got.double() - want).norm() / want.norm())
+
+
+def _random(shape, seed, scale=(1.0, 1.0, 1.0), positive=False):
+    """A layer and x, dy for it, from N(0, 1) times `scale` of x, w and dy; all positive if asked for."""
+    import torch
+    from aether_ml_b200 import layers
+    S, H, W, Cin, Cout, f, st, pad, mode = shape
+    np.random.seed(seed)
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    layer = layers.Conv_Layer((H, W, Cin), Cout, (f, f), st, pad, math_mode=mode)
+    make = lambda t, k: (t.abs() if positive else t) * k
+    layer.filter_weights.copy_(make(layer.filter_weights, scale[1]))
+    x = make(torch.randn((S, H, W, Cin), generator=g, device="cuda"), scale[0])
+    _, Ho, Wo = layer._extent(H, W)
+    dy = make(torch.randn((S, Ho, Wo, Cout), generator=g, device="cuda"), scale[2])
+    return layer, x, dy
+
+
+def _pass(layer, x, dy):
+    y = layer.forward(x, True)
+    return y, layer.backward(dy), layer.dweights, layer.dbiases
+
+
 def _layer(shape, x, b):
     from aether_ml_b200 import layers
     S, H, W, Cin, Cout, f, st, pad, mode = shape
@@ -67,3 +111,30 @@ def test_values_without_remainders():
         big = np.isfinite(want) & ~small
         assert O.rel_l2(got[small], want[small]) <= 3e-6
         assert np.allclose(got[big].astype(np.float64), want[big].astype(np.float64), rtol=3e-6)
+
+
+def test_less_memory(monkeypatch):
+    """Inference asks for the part of the workspace that forward calls use; without the memory for a workspace the layer runs as it can."""
+    import torch
+    from aether_ml_b200 import layers
+    shape = SHAPES[2]
+    layer, x, dy = _random(shape, 8)
+    p = layer._plan(tuple(x.shape))
+    want = _reference(shape, x, layer.filter_weights, layer.biases, dy)
+    y = layer.forward(x, False)
+    assert layer._ws.size == p.fwd_ws_bytes < p.ws_bytes and _off(y, want[0]) <= 3e-6
+    grads = layer.backward(dy), layer.dweights, layer.dbiases
+    assert layer._ws.size == p.ws_bytes
+    again = _pass(layer, x, dy)
+    assert all(torch.equal(a, b) for a, b in zip((y, *grads), again))
+
+    def no_room(self, nbytes):
+        if nbytes > p.least_ws_bytes():
+            raise torch.OutOfMemoryError("no room")
+        return grow(self, nbytes)
+    grow = layers._Workspace._grow
+    monkeypatch.setattr(layers._Workspace, "_grow", no_room)
+    small, _, _ = _random(shape, 8)
+    for got, w in zip(_pass(small, x, dy), want):
+        assert _off(got, w) <= 3e-6
+    assert small._ws.size == p.least_ws_bytes() < p.fwd_ws_bytes
