@@ -27,10 +27,11 @@ namespace aether {
 
 // Producer warps, in groups of four that build tiles in turn: three groups where nothing but the gathers of few output channels holds the
 // kernel back (896 x 32x32 3->32 35 -> 29 us, 64 and 128 channels 1-4 %), two with statistics, whose epilogue is the longer
-// chain (128 x 32x32 3->32 10.9 us, 12.0 with three).
-__host__ __device__ static constexpr int ft_prod_warps(bool stats) { return stats ? 8 : 12; }
+// chain (128 x 32x32 3->32 10.9 us, 12.0 with three), and for windows of more than 48 values, which a thread keeps in registers: three groups
+// leave it 80 of those (84 bytes spilled; 512 x 32x32 1->64 7x7 33.7 us, 31.6 with two groups, 64 x 64x64 4->32 4x4 19.8 / 18.9).
+__host__ __device__ static constexpr int ft_prod_warps(bool stats, int KP) { return stats || KP > 48 ? 8 : 12; }
 static constexpr int FT_EPI_WARPS = 8;                                       // two teams of four
-__host__ __device__ static constexpr int ft_threads(bool stats) { return 32 * (ft_prod_warps(stats) + 1 + FT_EPI_WARPS); }      // producers, MMA issuer, epilogue
+__host__ __device__ static constexpr int ft_threads(bool stats, int KP) { return 32 * (ft_prod_warps(stats, KP) + 1 + FT_EPI_WARPS); }      // producers, MMA issuer, epilogue
 static constexpr int FT_STAGE_BYTES = 128 * 128;                             // 128 pixel rows of 128 bytes
 static constexpr int FT_TAIL = 2048;                                         // barriers, TMEM pointer, bias, tap table
 static constexpr int FT_OUT_BYTES = 2 * 2 * FT_STAGE_BYTES;                  // two staging tiles (128 rows x 32 floats) per team
@@ -139,8 +140,8 @@ static int ft_stats_bytes(int NT) {
 __device__ __forceinline__ float stats_tree(const float (&v)[8]) { return ((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7])); }
 
 template <bool STATS, int KP, int CIN>
-__global__ void __launch_bounds__(ft_threads(STATS), 1) first_conv_kernel(const __grid_constant__ FirstParams p) {
-    constexpr int FT_PROD_WARPS = ft_prod_warps(STATS);
+__global__ void __launch_bounds__(ft_threads(STATS, KP), 1) first_conv_kernel(const __grid_constant__ FirstParams p) {
+    constexpr int FT_PROD_WARPS = ft_prod_warps(STATS, KP);
     extern __shared__ uint8_t smem_raw[];
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t* gen_base = smem_raw + (smem_base - smem_u32(smem_raw));
@@ -695,7 +696,7 @@ int first_tc_fwd(const AetherConvDesc& d, const float* x, const float* w, const 
     static PerDeviceSmem configured[2][6];
     const int ki = first_variant(d, KP), si = stats ? 1 : 0;
     if (int rc = ensure_dynamic_smem(kernels[si][ki], 232448, configured[si][ki], "first_conv")) return rc;
-    launch(kernels[si][ki], first_tc_grid(p.ntiles), ft_threads(si != 0), smem, st, p);
+    launch(kernels[si][ki], first_tc_grid(p.ntiles), ft_threads(si != 0, KP), smem, st, p);
     count_launch();
     return check_launch("first_conv_kernel");
 }
