@@ -105,27 +105,6 @@ __device__ __forceinline__ void split_phase(int a, int s, int& phase, int& at) {
     phase = a - at * s;
 }
 
-// One output by FMAs in the order of the reduction.
-__device__ float split_direct(const SplitParams& p, int n, int h, int w, int col) {
-    float s = 0.f;
-    for (int i = 0; i < p.fH; ++i)
-        for (int j = 0; j < p.fW; ++j) {
-            int a = h * p.sH - p.pH + i, b = w * p.sW - p.pW + j;
-            if (p.dx) {
-                a = h + p.pH - i;
-                b = w + p.pW - j;
-                if (a < 0 || b < 0 || a % p.sH || b % p.sW) continue;
-                a /= p.sH;
-                b /= p.sW;
-            }
-            if ((unsigned)a >= (unsigned)p.IH || (unsigned)b >= (unsigned)p.IW) continue;
-            const float* x = p.in + (((size_t)n * p.IH + a) * p.IW + b) * p.IC;
-            const float* f = p.w + (size_t)(i * p.fW + j) * p.Cin * p.Cout;
-            for (int k = 0; k < p.IC; ++k) s = fmaf(x[k], p.dx ? f[(size_t)col * p.Cout + k] : f[(size_t)k * p.Cout + col], s);
-        }
-    return s;
-}
-
 // Pixel tile `t` of p's tiling: first column, row and image.
 __device__ __forceinline__ void split_tile_origin(const SplitParams& p, int t, int& w0, int& h0, int& n0) {
     const int a = split_quot(t, p.by_tw), n = split_quot(a, p.by_th);
@@ -134,20 +113,22 @@ __device__ __forceinline__ void split_tile_origin(const SplitParams& p, int t, i
     n0 = n * p.BN;
 }
 
-// The same for an entry (filter row i, column j, channel c; output channel d) of a split's partial filter gradient.
-__device__ float split_direct_dw(const SplitParams& p, int t0, int t1, int i, int j, int c, int d) {
-    float s = 0.f;
-    for (int t = t0; t < t1; ++t) {
-        int w0, h0, n0;
-        split_tile_origin(p, t, w0, h0, n0);
-        for (int r = 0; r < p.rows; ++r) {
-            const int w = w0 + r % p.BW, h = h0 + r / p.BW % p.BH, n = n0 + r / (p.BW * p.BH);
-            const int a = h * p.sH - p.pH + i, b = w * p.sW - p.pW + j;
-            if (w >= p.OW || h >= p.OH || n >= p.S || (unsigned)a >= (unsigned)p.IH || (unsigned)b >= (unsigned)p.IW) continue;
-            s = fmaf(p.in[(((size_t)n * p.IH + a) * p.IW + b) * p.Cin + c], p.w[(((size_t)n * p.OH + h) * p.OW + w) * p.Cout + d], s);
-        }
+// Unit -> column tile; igemm: pixel tile `mt` of class `cls`; dW: group of row units `mt`, range of pixel tiles [t0, t1) of split `cls`.
+template <bool DW>
+__device__ __forceinline__ void split_unit(const SplitParams& p, int u, int& nt, int& mt, int& cls, int& t0, int& t1) {
+    const int a = split_quot(u, p.by_ntn);
+    nt = u - a * p.n_tiles_n;
+    if (DW) {
+        const long long ptiles = p.by_tiles.d;
+        cls = split_quot(a, p.by_groups);
+        mt = a - cls * (int)p.by_groups.d;
+        t0 = (int)(ptiles * cls / p.splits);
+        t1 = (int)(ptiles * (cls + 1) / p.splits);
+    } else {
+        cls = split_quot(a, p.by_tiles);
+        mt = a - cls * (int)p.by_tiles.d;
+        t0 = t1 = 0;
     }
-    return s;
 }
 
 // Row `r` of a unit's 128, pixel (b, a, n) of its box: where it goes (null: nowhere) and what it is (igemm: output column, row, image;
@@ -169,23 +150,154 @@ __device__ __forceinline__ float* split_row(const SplitParams& p, int mt, int cl
     return (r < p.rows && h < c.MH && w < c.MW && x_n < p.S) ? p.out + (((size_t)x_n * p.OH + x_h) * p.OW + x_w) * p.N : nullptr;
 }
 
-// What this lane stored for a unit and is not finite, again by FMAs.
+// Outputs that are not finite, again by FMAs from the fp32 arrays, in the order of the reduction: a plain tiled product by the whole block, in
+// the shared memory of the pipeline, after that has ended -- however long it takes, nobody waits for it with a limit.  Blocks of 64 rows x
+// 64 columns that have such an output, steps of 32 channels (dW: a box of pixels), 16 x 16 threads with 4 x 4 sums each.  Sums that are NaN stay so:
+// when no other is left the block of outputs is done.  Padding is zeros that are multiplied like other pixels (0 * inf), but in dX, which
+// has none.  96 x 28x28 32->64, forward / backward, us: finite values 34 / 71, NaN throughout 229 / 417, infinite ones of one sign 610 / 1812, one
+// infinite value 172 / 876 (by the lanes that stored them, one output after the other, dW alone some 20 ms by estimate; by rows of a warp and columns of its
+// lanes 222 / 535, 1147 / 3105, 90 / 794).  What it costs other passes is in dW's kernel, 1.4 us of 103 for the layer's forward and backward: with an empty body for dW
+// that is gone, with one for the other passes not; registers, the form of the call and the size of the body make no difference.
+__device__ __forceinline__ bool split_finite(float v) { return fabsf(v) <= 3.402823466e38f; }
+
 template <bool DW, int KC>
-__device__ __noinline__ void split_repair(const SplitParams& p, int nt, int mt, int cls, int t0, int t1, int q, int part, int lane) {
-    int w0 = 0, h0 = 0, n0 = 0, x_w, x_h, x_n;
+__device__ __forceinline__ void split_repair(const SplitParams& p, int nt, int mt, int cls, int t0, int t1, int row0, int col0, float* smem) {
+    constexpr int WARPS = SPLIT_THREADS / 32, STEP = DW ? DW_PIXELS : 32, LD = 68;
+    float *A = smem, *B = A + STEP * LD;                     // [step][row], [step][column]
+    int* pix = reinterpret_cast<int*>(B + STEP * LD);        // column, row and image of pixel r of a box: pix[r], pix[128 + r], pix[256 + r]
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, ty = tid >> 4, tx = tid & 15;
+    const int last = min((nt + 1) * p.NT, p.N);              // columns [col0, last)
     const SplitClass& c = p.cls[DW ? 0 : cls];
+    int w0 = 0, h0 = 0, n0 = 0;
     if (!DW) split_tile_origin(p, mt, w0, h0, n0);
-    for (int j = 0; j < 4; ++j) {
-        const int r = q * 32 + (lane & ~3) + j;
-        float* row = split_row<DW, KC>(p, mt, cls, c, w0, h0, n0, r, r % p.BW, r / p.BW % p.BH, r / (p.BW * p.BH), x_w, x_h, x_n);
-        if (row == nullptr) continue;
-        for (int b = part; b * 16 < p.NT; b += 2)
-            for (int e = 0; e < 4; ++e) {
-                const int col = nt * p.NT + b * 16 + (lane & 3) * 4 + e;
-                if (col >= p.N || fabsf(row[col]) <= 3.402823466e38f) continue;
-                row[col] = DW ? split_direct_dw(p, t0, t1, x_h, x_w, x_n, col)
-                              : split_direct(p, x_n, x_h, x_w, col) + (p.bias != nullptr ? p.bias[col] : 0.f);
+    __syncthreads();                                         // (the outputs before these have been read)
+    if (tid < 128) {
+        pix[tid] = tid % p.BW;
+        pix[128 + tid] = tid / p.BW % p.BH;
+        pix[256 + tid] = tid / (p.BW * p.BH);
+    }
+    __syncthreads();
+    // this thread's outputs: rows row0 + 4 ty + m, columns col0 + 4 tx + e
+    auto out_row = [&](int m) {
+        const int r = row0 + ty * 4 + m;
+        int x_w, x_h, x_n;
+        return split_row<DW, KC>(p, mt, cls, c, w0, h0, n0, r, pix[r], pix[128 + r], pix[256 + r], x_w, x_h, x_n);
+    };
+    uint32_t bad = 0;
+    if (tid < 256) {
+#pragma unroll 1
+        for (int m = 0; m < 4; ++m) {
+            const float* row = out_row(m);
+#pragma unroll 1
+            for (int e = 0; e < 4 && row != nullptr; ++e)
+                if (col0 + tx * 4 + e < last && !split_finite(row[col0 + tx * 4 + e])) bad |= 1u << (4 * m + e);
+        }
+    }
+    float acc[4][4] = {};
+    bool open = bad != 0;
+    auto multiply = [&](uint32_t rows) {                     // `rows`: those that the products belong to
+        __syncthreads();
+        if (tid >= 256) return;
+#pragma unroll 1
+        for (int k = 0; k < STEP; ++k) {
+            const float4 a4 = *reinterpret_cast<const float4*>(A + k * LD + ty * 4), b4 = *reinterpret_cast<const float4*>(B + k * LD + tx * 4);
+            const float a[4] = {a4.x, a4.y, a4.z, a4.w}, b[4] = {b4.x, b4.y, b4.z, b4.w};
+#pragma unroll
+            for (int m = 0; m < 4; ++m)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const float s = fmaf(a[m], b[e], acc[m][e]);
+                    acc[m][e] = !DW && !(rows >> m & 1) ? acc[m][e] : s;
+                }
+        }
+        open = false;
+#pragma unroll
+        for (int m = 0; m < 4; ++m)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) open |= (bad >> (4 * m + e) & 1) && acc[m][e] == acc[m][e];
+    };
+    if constexpr (DW) {
+        for (int t = t0; t < t1; ++t) {
+            if (!__syncthreads_or(open)) break;
+            split_tile_origin(p, t, w0, h0, n0);
+#pragma unroll 1
+            for (int r = warp; r < DW_PIXELS; r += WARPS) {
+                const int w = w0 + pix[r], h = h0 + pix[128 + r], n = n0 + pix[256 + r];
+                const bool ok = r < p.rows && w < p.OW && h < p.OH && n < p.S;
+#pragma unroll
+                for (int g = 0; g < 64; g += 32) {
+                    const int unit = mt * (128 / KC) + (row0 + g) / KC, tap = unit / p.cblocks, i = tap / p.fW;
+                    const int ch = (unit - tap * p.cblocks) * KC + (row0 + g) % KC + lane;
+                    const int a = h * p.sH - p.pH + i, b = w * p.sW - p.pW + tap - i * p.fW, col = col0 + g + lane;
+                    const bool in = ok && (unsigned)a < (unsigned)p.IH && (unsigned)b < (unsigned)p.IW && ch < p.Cin && unit < p.U;
+                    const bool in_d = ok && col < last;
+                    const float x = __ldg(p.in + (in ? (((size_t)n * p.IH + a) * p.IW + b) * p.Cin + ch : 0));
+                    const float d = __ldg(p.w + (in_d ? (((size_t)n * p.OH + h) * p.OW + w) * p.Cout + col : 0));
+                    A[r * LD + g + lane] = in ? x : 0.f;
+                    B[r * LD + g + lane] = in_d ? d : 0.f;
+                }
             }
+            multiply(0xfu);
+        }
+    } else {
+        // input pixel (a, b) that row r of the tile sees at filter row i, column j; whether it is one
+        auto seen = [&](int r, int i, int j, int& a, int& b) {
+            const int h = h0 + pix[128 + r], w = w0 + pix[r];
+            a = p.dx ? h + c.hq - (i - c.ph) / p.sH : h * p.sH - p.pH + i;
+            b = p.dx ? w + c.wq - (j - c.pw) / p.sW : w * p.sW - p.pW + j;
+            return (unsigned)a < (unsigned)p.IH && (unsigned)b < (unsigned)p.IW && n0 + pix[256 + r] < p.S;
+        };
+        const int i_step = p.dx ? p.sH : 1, j_step = p.dx ? p.sW : 1;
+        bool more = true;
+        for (int i = p.dx ? c.ph : 0; i < p.fH && more; i += i_step)
+            for (int j = p.dx ? c.pw : 0; j < p.fW && more; j += j_step) {
+                const float* f = p.w + (size_t)(i * p.fW + j) * p.Cin * p.Cout;
+                uint32_t rows = 0;
+#pragma unroll 1
+                for (int m = 0; m < 4; ++m) {
+                    int a, b;
+                    rows |= (uint32_t)(!p.dx || seen((row0 + ty * 4 + m) & 127, i, j, a, b)) << m;
+                }
+                for (int k0 = 0; k0 < p.IC; k0 += STEP) {
+                    more = __syncthreads_or(open);
+                    if (!more) break;
+                    const int k = k0 + lane;
+#pragma unroll 2
+                    for (int r = warp; r < 64; r += WARPS) {
+                        int a, b;
+                        const bool in = seen(row0 + r, i, j, a, b) && k < p.IC;
+                        const float v = __ldg(p.in + (in ? (((size_t)(n0 + pix[256 + row0 + r]) * p.IH + a) * p.IW + b) * p.IC + k : 0));
+                        A[lane * LD + r] = in ? v : 0.f;
+                    }
+#pragma unroll 2
+                    for (int u = warp; u < 64; u += WARPS) {              // the filter's contiguous index on the lanes
+                        const int kk = p.dx ? lane : u >> 1, n = p.dx ? u : (u & 1) * 32 + lane;
+                        const bool in = k0 + kk < p.IC && col0 + n < last;
+                        const float v = __ldg(f + (in ? p.dx ? (size_t)(col0 + n) * p.Cout + k0 + kk : (size_t)(k0 + kk) * p.Cout + col0 + n : 0));
+                        B[kk * LD + n] = in ? v : 0.f;
+                    }
+                    multiply(rows);
+                }
+            }
+    }
+    if (bad == 0) return;
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {
+        float* row = out_row(m);
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+            if (bad >> (4 * m + e) & 1) row[col0 + tx * 4 + e] = acc[m][e] + (!DW && p.bias != nullptr ? p.bias[col0 + tx * 4 + e] : 0.f);
+    }
+}
+
+// ... of all units of this block.
+template <bool DW, int KC>
+__device__ __noinline__ void split_repair_units(const SplitParams& p, float* smem) {
+    for (int u = blockIdx.x; u < p.units; u += gridDim.x) {
+        int nt, mt, cls, t0, t1;
+        split_unit<DW>(p, u, nt, mt, cls, t0, t1);
+        for (int row0 = 0; row0 < 128; row0 += 64)
+            for (int col0 = nt * p.NT; col0 < min((nt + 1) * p.NT, p.N); col0 += 64) split_repair<DW, KC>(p, nt, mt, cls, t0, t1, row0, col0, smem);
     }
 }
 
@@ -208,6 +320,7 @@ __global__ void __launch_bounds__(SPLIT_THREADS, 1) split_conv_kernel(const __gr
     const uint32_t sTmemPtr = sBar + 8u * (2 * STAGES + 2 * NBG + 2 * NBC);
     uint8_t* gen_base = smem_raw + (smem_base - smem_u32(smem_raw));
     volatile uint32_t* tmem_ptr_generic = reinterpret_cast<volatile uint32_t*>(gen_base + (sTmemPtr - smem_base));
+    volatile uint32_t* repair_flag = tmem_ptr_generic + 1;         // whether this block stored something that is not finite
 
     const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);
     const int lane = threadIdx.x & 31;
@@ -232,6 +345,7 @@ __global__ void __launch_bounds__(SPLIT_THREADS, 1) split_conv_kernel(const __gr
         for (int b = 0; b < NBG; ++b) { mbar_init(gfull_bar(b), 1); mbar_init(gempty_bar(b), SPLIT_EPI_WARPS); }
         for (int b = 0; b < NBC; ++b) { mbar_init(cfull_bar(b), 1); mbar_init(cempty_bar(b), SPLIT_EPI_WARPS); }
         mbar_fence_init();
+        *repair_flag = 0;
         tma_prefetch_desc(&p.tm_a);
         tma_prefetch_desc(&p.tm_b);
     }
@@ -247,23 +361,8 @@ __global__ void __launch_bounds__(SPLIT_THREADS, 1) split_conv_kernel(const __gr
     const uint32_t tmem_c = tmem_base + NBG * NTMAX;           // accumulators of the small products
 
     const int NT = p.NT;
-    const int ptiles = p.tiles_w * p.tiles_h * p.tiles_n;
     const int b_part = DW ? DY_TILE : NT * Cfg::ROW;                       // bytes of one part of the columns' operand
-    // unit -> column tile; igemm: pixel tile `mt` of class `cls`; dW: group of row units `mt`, range of pixel tiles [t0, t1)
-    auto decode = [&](int u, int& nt, int& mt, int& cls, int& t0, int& t1) {
-        const int a = split_quot(u, p.by_ntn);
-        nt = u - a * p.n_tiles_n;
-        if (DW) {
-            cls = split_quot(a, p.by_groups);
-            mt = a - cls * (int)p.by_groups.d;
-            t0 = (int)((long long)ptiles * cls / p.splits);
-            t1 = (int)((long long)ptiles * (cls + 1) / p.splits);
-        } else {
-            cls = split_quot(a, p.by_tiles);
-            mt = a - cls * ptiles;
-            t0 = t1 = 0;
-        }
-    };
+    auto decode = [&](int u, int& nt, int& mt, int& cls, int& t0, int& t1) { split_unit<DW>(p, u, nt, mt, cls, t0, t1); };
     // stages of a unit, and steps of one of them
     auto unit_stages = [&](int cls, int t0, int t1) {
         if (DW) return t1 - t0;
@@ -536,7 +635,7 @@ __global__ void __launch_bounds__(SPLIT_THREADS, 1) split_conv_kernel(const __gr
                         if (rowp[j] == nullptr) continue;
 #pragma unroll
                         for (int e = 0; e < 4; ++e) {
-                            bad |= !(fabsf(m[j][e]) <= 3.402823466e38f);
+                            bad |= !split_finite(m[j][e]);
                             m[j][e] += bias[e];
                         }
                         if ((DW ? p.ldn : p.N) % 4 == 0) {
@@ -549,7 +648,7 @@ __global__ void __launch_bounds__(SPLIT_THREADS, 1) split_conv_kernel(const __gr
                     }
                 }
             }
-            if (bad) split_repair<DW, KC>(p, nt, mt, cls, t0, t1, q, part, lane);
+            if (bad) *repair_flag = 1;
         }
     }
 
@@ -559,6 +658,7 @@ __global__ void __launch_bounds__(SPLIT_THREADS, 1) split_conv_kernel(const __gr
         tc_fence_after();
         tmem_dealloc(tmem_base, 512);
     }
+    if (*repair_flag != 0) split_repair_units<DW, KC>(p, reinterpret_cast<float*>(gen_base));
 }
 
 // ====================================================================================== operands

@@ -113,6 +113,70 @@ def test_values_without_remainders():
         assert np.allclose(got[big].astype(np.float64), want[big].astype(np.float64), rtol=3e-6)
 
 
+# strided layers of odd channel counts, with rows of 32 channels, without padding; several column tiles; 5x5 taps
+@pytest.mark.parametrize("shape", [SHAPES[2], SHAPES[10], SHAPES[8], SHAPES[4], SHAPES[0], SHAPES[7]])
+@pytest.mark.parametrize("where", ["x and dy", "filter", "sums", "overflow"])
+def test_not_finite_anywhere(shape, where):
+    """Infinite, NaN, very large operands and sums that overflow in x, the filter and dy, which reach some outputs: those are what
+    fp32 sums are (padding is zeros: 0 * inf), the others are as exact as ever."""
+    from aether_ml_b200 import _lib
+    assert _split(shape)
+    S, H, W, Cin, Cout, f, st, pad, mode = shape
+    layer, x, dy = _random(shape, 5)
+    w = layer.filter_weights
+    if where == "x and dy":
+        x[0, 3, 4, 5], x[1, 2, 2, 0], x[2, 5, 5, 1], x[3, 0, 0, 2] = float("inf"), -float("inf"), float("nan"), 3.4e38
+        dy[1, 1, 1, 7], dy[5, 0, 1, 2] = float("inf"), float("nan")
+        w *= 1e-3                                            # (3.4e38 stays in range, with dy, too)
+        dy *= 1e-3
+    elif where == "filter":
+        w[0, 0, 3, 2], w[-1, -1, 6, 9], w[0, -1, 7, 4] = float("inf"), float("nan"), -float("inf")
+    elif where == "sums":
+        x *= 2.0**60                                         # sums of 2^95 and more, finite ones
+        w *= 2.0**40
+        dy *= 2.0**30
+    else:
+        w *= 2.0**10                                         # sums of 2^110, and some that overflow (of one sign: in any order)
+        w[..., 3] = w[..., 3].abs() * 2.0**20
+        x[0], dy[1] = x[0].abs() * 2.0**100, dy[1].abs() * 2.0**100
+    got = [t.cpu().numpy() for t in _pass(layer, x, dy)]
+    X, DY, Wt = (t.cpu().numpy().astype(np.float64) for t in (x, dy, w))
+    with np.errstate(all="ignore"):
+        want = [O.conv_forward(X, Wt, np.zeros(Cout), st, pad), *O.conv_backward(X, Wt, DY, st, pad)]
+        want = [np.where(np.abs(t) > 3.5e38, np.sign(t) * np.inf, t) for t in want]
+        X, DY, Wt = np.abs(X), np.abs(DY), np.abs(Wt)
+        sizes = [O.conv_forward(X, Wt, np.zeros(Cout), st, pad), *O.conv_backward(X, Wt, DY, st, pad)]
+        for a, b, size in zip(got, want, sizes):
+            sure = ~(np.abs(b) > 3e38) | np.isinf(b)         # (in between the order of the sum decides)
+            a, b, size = a[sure], b[sure], size[sure]
+            assert np.array_equal(np.isnan(a), np.isnan(b)) and np.array_equal(np.isposinf(a), np.isposinf(b)) and np.array_equal(np.isneginf(a), np.isneginf(b))
+            fine = np.isfinite(b)
+            assert (np.abs(a[fine] - b[fine]) <= 3e-6 * size[fine]).all()
+    assert _lib.device_status() == 0
+
+
+def test_time_of_values_that_are_not_finite():
+    """A diverged network's arrays are NaN or infinite throughout.  Such a pass may take longer than one of finite values, but not by orders of
+    magnitude: NaN ends a sum early, infinite ones of one sign go all the way."""
+    import torch
+    shape = (96, 28, 28, 32, 64, 3, (1, 1), "same", "fp32")
+    times = []
+    for value, positive in ((1.0, True), (float("nan"), False), (float("inf"), False), (float("inf"), True)):
+        layer, x, dy = _random(shape, 6, positive=positive)
+        x.mul_(value)
+        dy.mul_(value)
+        for _ in range(3):
+            _pass(layer, x, dy)
+        a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        a.record()
+        for _ in range(5):
+            _pass(layer, x, dy)
+        b.record()
+        b.synchronize()
+        times.append(a.elapsed_time(b) / 5)
+    assert max(times[1:3]) < 10 * times[0] and times[3] < 30 * times[0], times
+
+
 def test_less_memory(monkeypatch):
     """Inference asks for the part of the workspace that forward calls use; without the memory for a workspace the layer runs as it can."""
     import torch
