@@ -11,8 +11,7 @@
 // order are 2^-8 and 2^-16 of that and stay in two accumulators of their own for up to EPOCH_STAGES stages.  Relative error against
 // float64, FMA kernels / this one: 96 x 28x28 32->64 y 3.0e-7 / 8.2e-8, dX 4.2e-7 / 9.5e-8, dW 3.8e-7 / 1.4e-7, and smaller in
 // all of forty drawn layers.  An
-// output that is not finite (an infinite or NaN operand has no meaningful remainder, one above 3.39e38 rounds to infinity) is
-// summed again by FMAs from the fp32 arrays.  Operands below 2^-109 keep fewer than 24 bits (the last part is subnormal).
+// output that is not finite (an infinite or NaN operand has no meaningful remainder) is summed again by FMAs from the fp32 arrays.
 //
 // Time.  Six MMAs take the place of one, 1/6 of the bf16 rate is 3.7 times the FMA pipes'.  N columns of the filter (dy in dW) are
 // staged as [w0 | w1 | w2], so that x0 multiplies [w1 | w2] and x1 [w0 | w1] in one MMA of 2 N columns each: four MMAs
@@ -40,6 +39,11 @@ static constexpr int EPOCH_STAGES = 32;         // stages after which the small 
 static constexpr int SPLIT_EPI_WARPS = 8;       // 4 TMEM lane quarters x 2 (16-column blocks taken in turn)
 static constexpr int SPLIT_THREADS = 128 + 32 * SPLIT_EPI_WARPS;     // warps 0 and 1 copy, 2 and 3 multiply, the others add and store
 static constexpr int DW_PIXELS = 64;            // pixel rows per stage of dW
+// Operands are multiplied by 2^24 before they are split and sums by 2^-48 when they are stored: the lowest bit of the smallest subnormal
+// number is then 2^-125, so no part of a fp32 number is subnormal in bf16 (without it operands below 2^-109 lost bits: error 1.6e-7 at
+// 2^-112, 2.2e-6 at 2^-116, 3.5e-5 at 2^-120, everything at 2^-140).  Operands from 2^104 on, and sums from 2^80 on, come out infinite and are
+// summed again by FMAs.
+static constexpr float SPLIT_SCALE = 16777216.f, SPLIT_UNSCALE = 1.f / (SPLIT_SCALE * SPLIT_SCALE);
 
 // Quotients by a number known at launch (multiplication and shift; dividends below 2^31): the roles of the kernel decode their units by them
 // again and again, and an integer division is some 40 instructions.
@@ -636,7 +640,7 @@ __global__ void __launch_bounds__(SPLIT_THREADS, 1) split_conv_kernel(const __gr
 #pragma unroll
                         for (int e = 0; e < 4; ++e) {
                             bad |= !split_finite(m[j][e]);
-                            m[j][e] += bias[e];
+                            m[j][e] = fmaf(m[j][e], SPLIT_UNSCALE, bias[e]);
                         }
                         if ((DW ? p.ldn : p.N) % 4 == 0) {
                             if (col < p.N) *reinterpret_cast<float4*>(rowp[j] + col) = make_float4(m[j][0], m[j][1], m[j][2], m[j][3]);
@@ -663,6 +667,7 @@ __global__ void __launch_bounds__(SPLIT_THREADS, 1) split_conv_kernel(const __gr
 
 // ====================================================================================== operands
 __device__ __forceinline__ void split3(float v, __nv_bfloat16& a, __nv_bfloat16& b, __nv_bfloat16& c) {
+    v *= SPLIT_SCALE;                                    // exact, or infinite from 2^104 on
     a = __float2bfloat16_rn(v);
     const float r = v - __bfloat162float(a);             // exact
     b = __float2bfloat16_rn(r);

@@ -85,6 +85,17 @@ def test_against_float64(shape):
         assert O.rel_l2(got.cpu().numpy(), want) <= 3e-6
 
 
+@pytest.mark.parametrize("scale", [(2.0**-118, 1.0, 1.0), (1.0, 2.0**-116, 1.0), (1.0, 1.0, 2.0**-121), (2.0**-124, 2.0**20, 2.0**-80), (2.0**90, 2.0**-60, 2.0**-90)])
+@pytest.mark.parametrize("shape", [SHAPES[0], SHAPES[2]])
+def test_small_operands(shape, scale):
+    """Operands of which bf16 cannot hold the last bits, alone and beside others of ordinary size: 24 bits of each count.  (Outputs near the end of
+    the range are rounded to 2^-149.)"""
+    layer, x, dy = _random(shape, 4, scale)
+    x[1], dy[1] = x[1] * 2.0**8, dy[1] * 2.0**8
+    for got, want in zip(_pass(layer, x, dy), _reference(shape, x, layer.filter_weights, layer.biases, dy)):
+        assert float((got.double() - want).norm()) <= 3e-6 * float(want.norm()) + 2.0**-149 * want.numel()**0.5
+
+
 def test_values_without_remainders():
     """Infinite, NaN and very large operands: their parts are not numbers, the outputs are those of fp32 sums."""
     shape = SHAPES[1]
