@@ -377,6 +377,6 @@ extern "C" int aether_conv2d_bwd_ex(const AetherConvDesc* d, const float* x, con
         return first_tc_bwd_filter(*d, x, dy, dw, db, ws, ws_bytes, dy_ready ? dy_colsum_rows : 0, st);
     if ((dw || db) && smallc_conv_eligible(*d) && (!db || aligned16(db)))
         return smallc_conv_bwd_filter(*d, x, dy, dw, db, ws, ws_bytes, st);
-    if (dw || db) return generic_conv_bwd_filter(*d, x, dy, dw, db, ws, ws_bytes, st);
+    if (dw || db) return simt_conv_bwd_filter(*d, x, dy, dw, db, ws, ws_bytes, st);
     return AE_OK;
 }

@@ -92,8 +92,6 @@ int generic_head_cce_bwd(const AetherConvDesc& d, const float* prob, const int* 
 int generic_conv_fwd(const AetherConvDesc& d, const float* x, const float* w, const float* b, float* y, void* ws, size_t ws_bytes,
                      cudaStream_t st);
 int generic_conv_bwd_data(const AetherConvDesc& d, const float* dy, const float* w, float* dx, void* ws, size_t ws_bytes, cudaStream_t st);
-int generic_conv_bwd_filter(const AetherConvDesc& d, const float* x, const float* dy, float* dw, float* db, void* ws,
-                            size_t ws_bytes, cudaStream_t st);
 size_t generic_conv_workspace_bytes(const AetherConvDesc& d);
 
 // ---- conv_smallc.cu : fp32 first-layer convolution (1..4 input channels, fH*fW*Cin <= 64): forward, dW, dB

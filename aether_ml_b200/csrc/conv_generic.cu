@@ -595,11 +595,6 @@ size_t generic_conv_workspace_bytes(const AetherConvDesc& d) {
     return head > simt ? head : simt;
 }
 
-int generic_conv_bwd_filter(const AetherConvDesc& d, const float* x, const float* dy, float* dw, float* db, void* ws,
-                            size_t ws_bytes, cudaStream_t st) {
-    return simt_conv_bwd_filter(d, x, dy, dw, db, ws, ws_bytes, st);
-}
-
 // Most rows whose dW comes out of one launch: a thread's sum is over every 64th row, 16 of them here, as long as the parts' below.  One
 // launch is faster for more rows, too (2048 x 256->10 18.8 us against 21.1, 4096 x 1024->10 41.7 against 52.6), but from there on its longer
 // sums are the less accurate ones (dW at 4096 rows 1.30e-7 off float64 against 1.14e-7; at 1024 1.00e-7 against 1.05e-7).

@@ -34,7 +34,6 @@
 
 namespace aether {
 
-static constexpr int SPLIT_KC = 64;             // most channels per row of a tile (128 bytes)
 static constexpr int EPOCH_STAGES = 32;         // stages after which the small products' sums leave TMEM, too
 static constexpr int SPLIT_EPI_WARPS = 8;       // 4 TMEM lane quarters x 2 (16-column blocks taken in turn)
 static constexpr int SPLIT_THREADS = 128 + 32 * SPLIT_EPI_WARPS;     // warps 0 and 1 copy, 2 and 3 multiply, the others add and store
@@ -45,7 +44,8 @@ static constexpr int DW_PIXELS = 64;            // pixel rows per stage of dW
 // summed again by FMAs.
 static constexpr float SPLIT_SCALE = 16777216.f, SPLIT_UNSCALE = 1.f / (SPLIT_SCALE * SPLIT_SCALE);
 
-// Quotients by a number known at launch (multiplication and shift; dividends below 2^31): the roles of the kernel decode their units by them
+// Quotients by a number known at launch (Granlund and Montgomery, Division by Invariant Integers using Multiplication, 1994: a multiplication,
+// an addition and a shift; dividends below 2^31): the roles of the kernel decode their units by them
 // again and again, and an integer division is some 40 instructions.
 struct SplitDiv {
     uint32_t d, mul, shift;
