@@ -32,6 +32,7 @@ def test_against_oracle(shape):
     conv.emit_bn_stats = True
     y2 = conv.forward(x, True)
     mean, var = y.reshape(-1, Cout).mean(0), y.reshape(-1, Cout).var(0)
+    assert (conv.bn_partials is not None) == (conv._plan(tuple(x.shape)).stats_blocks > 0)
     if conv.bn_partials is not None:
         stats, blocks, _ = conv.bn_partials
         p = stats.view(dtype=__import__("torch").float32)[:blocks * 3 * Cout].cpu().numpy().reshape(blocks, 3, Cout).astype(np.float64)

@@ -15,6 +15,11 @@ SHAPES = [(9, 19, 17, 65, 130, 3, (1, 1), "same", "fp32"), (60, 15, 13, 37, 71, 
           (61, 8, 8, 128, 33, 3, (1, 1), "same", "fp32"), (30, 23, 20, 64, 64, 5, (3, 2), "valid", "tf32"), (70, 30, 31, 96, 32, 1, (1, 1), "same", "fp32"),
           (120, 12, 11, 100, 129, 1, (2, 2), "same", "fp32"), (60, 20, 21, 16, 50, 5, (1, 1), "same", "fp32"), (40, 33, 20, 90, 17, 3, (2, 1), "valid", "bf16"), (16, 7, 7, 256, 256, 3, (1, 1), "same", "fp32"), (90, 9, 10, 32, 144, 3, (1, 4), "same", "tf32")]
 
+# Pointwise layers that are large enough (rows of channels to the next 8 instead of whole tile rows), strided and not; a filter gradient of
+# 162 tiles and 39 stages each, so that 14 CTAs have a second one and all a second epoch; a column tile of 128 with 50 stages.
+MORE = [(6, 43, 43, 88, 188, 1, (1, 1), "same", "fp32"), (200, 23, 21, 300, 331, 1, (2, 1), "same", "bf16"), (50, 7, 7, 384, 384, 3, (1, 1), "same", "fp32"),
+        (24, 28, 28, 128, 128, 5, (1, 1), "same", "fp32")]
+
 
 def _split(shape):
     """Whether the library takes these kernels for the shape (then forward calls use a part of the workspace only)."""
@@ -83,6 +88,21 @@ def test_against_float64(shape):
     dxo, dwo, dbo = O.conv_backward(x.astype(np.float64), w.astype(np.float64), dy.astype(np.float64), st, pad)
     for got, want in ((y, yo), (dx, dxo), (layer.dweights, dwo), (layer.dbiases, dbo)):
         assert O.rel_l2(got.cpu().numpy(), want) <= 3e-6
+
+
+def test_routes():
+    """What the other tests here are about is what runs (two pointwise shapes of the list are too small for it)."""
+    assert [_split(s) for s in SHAPES] == [s[5] > 1 for s in SHAPES] and all(_split(s) for s in MORE)
+
+
+@pytest.mark.parametrize("positive", [False, True])
+@pytest.mark.parametrize("shape", MORE + [SHAPES[0], SHAPES[2], SHAPES[7]])
+def test_large_and_one_sided(shape, positive):
+    """Sums of one sign, too: those that the tensor cores truncate lose in one direction there.  A stage's sum is at most four truncations of 2^-24
+    off, the at most 50 stages are added with rounding: below 54 * 2^-24 = 3.2e-6 at worst; measured 2.5e-7."""
+    layer, x, dy = _random(shape, 3, positive=positive)
+    for got, want in zip(_pass(layer, x, dy), _reference(shape, x, layer.filter_weights, layer.biases, dy)):
+        assert _off(got, want) <= 3.2e-6
 
 
 @pytest.mark.parametrize("scale", [(2.0**-118, 1.0, 1.0), (1.0, 2.0**-116, 1.0), (1.0, 1.0, 2.0**-121), (2.0**-124, 2.0**20, 2.0**-80), (2.0**90, 2.0**-60, 2.0**-90)])
