@@ -9,8 +9,10 @@
 // four steps only: the x0 w0 products of each stage go to an accumulator of their own that the epilogue warps add to their running
 // sums in registers (rounding to nearest) while the next stages are multiplied.  The products of second and third
 // order are 2^-8 and 2^-16 of that and stay in two accumulators of their own for up to EPOCH_STAGES stages.  Relative error against
-// float64, FMA kernels / this one: 96 x 28x28 32->64 y 3.0e-7 / 8.2e-8, dX 4.2e-7 / 9.5e-8, dW 3.8e-7 / 1.4e-7, and smaller in
-// all of forty drawn layers.  An
+// float64, FMA kernels / this one: 96 x 28x28 32->64 y 3.0e-7 / 7.8e-8, dX 4.2e-7 / 9.5e-8, dW 3.8e-7 / 1.4e-7, and smaller in
+// all of forty drawn layers on N(0, 1) and in ten with x positive.  Where every product has one sign truncation always loses: there y 2.3e-7 / 6.8e-8,
+// dX 3.2e-7 / 9.1e-8, but dW 6.0e-8 / 8.9e-8, at worst 1.7 times the FMAs' error (dW of 6 x 43x43 88->188 1x1 5.2e-8 / 8.4e-8).  Sums taken out every
+// two steps lower that (dW 6.4e-8), but round more often (dW of N(0, 1) 1.6e-7, of 24 x 28x28 128->128 5x5 2.5e-7 -> 3.4e-7) and cost 2-3 %.  An
 // output that is not finite (an infinite or NaN operand has no meaningful remainder) is summed again by FMAs from the fp32 arrays.
 //
 // Time.  Six MMAs take the place of one, 1/6 of the bf16 rate is 3.7 times the FMA pipes'.  N columns of the filter (dy in dW) are
@@ -19,9 +21,10 @@
 // parts are made by a pass over x and dy (split3_kernel: 4 bytes read, 6 written, dB on the way) and copied by TMA, rows of 64
 // channels with zeros behind the last: channel counts need not be multiples of anything.  A strided layer's x is stored by
 // phases, so that a tap's pixels lie side by side (element strides in the tensor map halve the copies' rate).
-// Measured on B200, forward + backward, CUDA cores / this file: 40 x 33x32 64->128 444 / 132 us, 96 x 28x28 32->64 211 / 100, 100 x 57x45
-// 48->72 stride 2 432 / 196 (three sets of inputs in turn).  Bound by shared memory: the MMAs' operand reads (28 KB per step of 64
-// columns, 219 clocks) and the copies' writes (16-18 KB) share its 128 bytes a clock, the tensor pipe is 42-47 % busy, DRAM 5-14 %.
+// Measured on B200, forward + backward, CUDA cores / this file: 40 x 33x32 64->128 442 / 131 us, 96 x 28x28 32->64 207 / 100, 100 x 57x45
+// 48->72 stride 2 431 / 193 (one set of inputs; three in turn, as a program's arrays come: 211 / 104, 433 / 212).  No unit is saturated: the
+// tensor pipe is 24-48 % busy, L1 and shared memory 40-67 %, DRAM 6-31 % (a filter kept in shared memory changes 1 %).  What is left is the chain of a tile: the
+// first stages of a unit wait for their copies, and the warps that sum store (2-3 thousand clocks) before they take products again.
 #include <string.h>
 
 #include <cuda_bf16.h>

@@ -40,7 +40,9 @@ extern "C" {
 #define AETHER_MATH_FP32 2 /* single precision (also used for shapes the tensor path does not    */
                            /* take: stride > 1, Cin or Cout < 16 or not a multiple of 4): FMAs   */
                            /* on the CUDA cores or, for larger layers with a workspace, tensor   */
-                           /* cores on operands split into three bf16 numbers, which is closer   */
+                           /* cores on operands split into three bf16 numbers.  Error of those   */
+                           /* against exact sums, FMAs' = 1: 0.2 to 0.6 for operands of both     */
+                           /* signs, 0.2 to 1.7 where all products have one sign                 */
 
 #define AETHER_POOL_MAX 0
 #define AETHER_POOL_AVG 1
