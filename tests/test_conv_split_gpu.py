@@ -205,7 +205,7 @@ def test_time_of_values_that_are_not_finite():
         b.record()
         b.synchronize()
         times.append(a.elapsed_time(b) / 5)
-    assert max(times[1:3]) < 10 * times[0] and times[3] < 30 * times[0], times
+    assert max(times[1:3]) < 15 * times[0] and times[3] < 50 * times[0], times          # (measured 6 and 23 times)
 
 
 def test_less_memory(monkeypatch):
