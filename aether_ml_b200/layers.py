@@ -391,8 +391,8 @@ class Conv_Layer(_TakesCopies, _Saved):
         if p.y_shape is None:
             raise ValueError("filter larger than the padded input")
         H = host()
+        y = H.empty(p.y_shape)                  # (before the workspace, which can do with less)
         ws = self._ws.get(p.ws_bytes if training else p.fwd_ws_bytes, p)
-        y = H.empty(p.y_shape)
         w = self.filter_weights
         flags = 0
         if self._handed.x is not None:
@@ -427,7 +427,6 @@ class Conv_Layer(_TakesCopies, _Saved):
         if dy.shape != p.y_shape:
             raise ValueError(f"dvalues has shape {tuple(dy.shape)}, expected {p.y_shape}")
         H = host()
-        ws = self._ws.get(p.ws_bytes, p)
         w = self.filter_weights
         if getattr(self, "_grad_views", None) is not None:
             self.dweights, self.dbiases = self._grad_views
@@ -435,6 +434,7 @@ class Conv_Layer(_TakesCopies, _Saved):
             self.dweights = H.empty(w.shape)
             self.dbiases = H.empty(p.b_shape)
         dx = H.empty(p.x_shape) if need_dinputs else None
+        ws = self._ws.get(p.ws_bytes, p)
         shadow_ok = self._copies.flags(ws, x, w)
         rows = 0
         if self._handed.dy is not None:
@@ -1012,9 +1012,9 @@ class Layer_Dense(_TakesCopies, _Saved):
         if x.ndim != 2 or x.shape[1] != w.shape[0]:
             raise ValueError(f"Layer_Dense expects (samples, {w.shape[0]}), got {tuple(x.shape)}")
         p = self._plan(x.shape[0])
-        ws, flags = self._operands(x, p, training)
         H = host()
         y = H.empty((x.shape[0], w.shape[1]))
+        ws, flags = self._operands(x, p, training)
         H.aether_conv2d_fwd_ex(p.raw, x, w, self.biases, y, None, 0, ws, self._ws.size, flags)
         self.inputs = x
         self.output = y
@@ -1094,8 +1094,8 @@ class Layer_Dense(_TakesCopies, _Saved):
         x = self.inputs
         w = self.weights
         H = host()
-        ws = self._ws.get(p.ws_bytes, p)
         dx = H.empty_like(x)
+        ws = self._ws.get(p.ws_bytes, p)
         flags = self._copies.flags(ws, x, w)
         if not (flags & _lib.CONV_X_COPY_READY):
             _require_written(x, "Layer_Dense.backward")

@@ -233,3 +233,30 @@ def test_less_memory(monkeypatch):
     for got, w in zip(_pass(small, x, dy), want):
         assert _off(got, w) <= 3e-6
     assert small._ws.size == p.least_ws_bytes() < p.fwd_ws_bytes
+
+
+def test_outputs_come_before_scratch():
+    """A process that may take 700 MiB more: a layer's outputs (2 x 196) fit beside the least workspace, not beside the 592 it would rather have."""
+    import torch
+    from aether_ml_b200 import layers
+    np.random.seed(1)
+    layer = layers.Conv_Layer((112, 112, 64), 64, (3, 3), (1, 1), "same", math_mode="fp32")
+    x = torch.randn((64, 112, 112, 64), device="cuda")
+    dy = torch.randn(x.shape, device="cuda")
+    p = layer._plan(tuple(x.shape))
+    assert p.least_ws_bytes() < 200 << 20 < p.fwd_ws_bytes < 500 << 20 < p.ws_bytes
+    torch.cuda.empty_cache()
+    try:
+        torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + (700 << 20)) / torch.cuda.get_device_properties(0).total_memory)
+        y = layer.forward(x, True)
+        dx = layer.backward(dy)
+        assert layer._ws.size == p.least_ws_bytes()
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    rich, _, _ = _random((64, 112, 112, 64, 64, 3, (1, 1), "same", "fp32"), 1)
+    rich.filter_weights.copy_(layer.filter_weights)
+    for a, b in zip((y, dx, layer.dweights), _pass(rich, x, dy)):
+        assert _off(a, b.double()) <= 3e-6
+    assert rich._ws.size == p.ws_bytes
+    del rich, x, dy, y, dx
+    torch.cuda.empty_cache()
