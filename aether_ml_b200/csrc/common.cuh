@@ -80,7 +80,10 @@ int split_conv_fwd(const AetherConvDesc& d, const float* x, const float* w, cons
 int split_conv_bwd(const AetherConvDesc& d, const float* x, const float* dy, const float* w, float* dx, float* dw, float* db, void* ws,
                    int copies_valid, cudaStream_t st);
 
-// ---- conv_generic.cu : classifier heads and dX of first layers on the CUDA cores; everything else goes to conv_simt.cu
+// ---- conv_dx_few.cu : dX of first layers (1..4 input channels) on the CUDA cores
+int dx_few_conv_bwd_data(const AetherConvDesc& d, const float* dy, const float* w, float* dx, cudaStream_t st);
+
+// ---- conv_generic.cu : classifier heads on the CUDA cores; everything else goes to conv_dx_few.cu and conv_simt.cu
 // classifier heads (pointwise, few outputs) with the softmax / the combined softmax and cross-entropy gradient in the kernel
 bool generic_head_shape(const AetherConvDesc& d);
 int generic_head_softmax_fwd(const AetherConvDesc& d, const float* x, const float* w, const float* b, float* y, float* prob, cudaStream_t st);

@@ -1,6 +1,6 @@
 // Single-precision convolution (CNN/models/CNN_classes_cupy.py:70-154) for the shapes the tensor-core kernels do not take:
-// classifier heads (pointwise layers with few outputs per pixel) and the dX of first layers (1 to 4 input channels) have
-// kernels of their own here, everything else goes to the tiled implicit GEMMs of conv_simt.cu.
+// classifier heads (pointwise layers with few outputs per pixel) have kernels of their own here, the dX of first layers (1 to 4 input channels)
+// has conv_dx_few.cu, everything else goes to the tiled implicit GEMMs of conv_simt.cu.
 #include "common.cuh"
 #include "tc_host.cuh"
 
@@ -104,134 +104,6 @@ __global__ void __launch_bounds__(256) gen_fwd_pointwise_few_kernel(const float*
             for (int o = 16; o > 1; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
             if (out < Cout && !(lane & 1)) prob[(size_t)row * Cout + out] = e / sum;
         }
-    }
-}
-
-// ---------------------------------------------------------------------------------- dX of first layers
-// dx[s,h,w,c] = sum over taps (i,j) and d of dy[s,ho,wo,d] * w[i,j,c,d] with ho*sH + i - pH == h, for layers with 1..4
-// input channels (the first layer of a network), always in single precision.
-//
-// Bound by the FMA pipes and the L1: dy is small and every value of it meets CIN * taps filter values.  Eight lanes
-// share a column of four input pixels and take four output channels each, so a warp's load of dy is four whole
-// 128-byte lines, and a load of dy serves up to FB taps of the filter column (FB rows of the filter sit in registers at a
-// time: 3x3 filters read each dy value 1.5 times per column instead of three times).  Sums are pairs over even and odd
-// channels (fma.rn.f32x2), the lanes' sums meet in a fixed halving exchange.  A stride splits the input pixels into
-// sH*sW classes (blockIdx.z) that each see only the taps that reach them.
-// Measured: 128 x 32x32 3->32 3x3, 56 us with one thread per pixel (a warp's load touched 32 lines), 20 us now.
-static constexpr int DXF_PV = 4;                        // pixels (rows) per thread
-static constexpr int DXF_LANES = 8;                     // lanes that share them
-
-__device__ __forceinline__ void dxf_fma2(unsigned long long& d, unsigned long long a, unsigned long long b) {
-    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
-}
-
-// Four consecutive floats of an array as two pairs; of an unaligned row the n that are in it.
-template <bool VEC>
-__device__ __forceinline__ ulonglong2 dxf_load4(const float* p, int n) {
-    if (VEC) return __ldg(reinterpret_cast<const ulonglong2*>(p));
-    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (n > 0) v.x = __ldg(p);
-    if (n > 1) v.y = __ldg(p + 1);
-    if (n > 2) v.z = __ldg(p + 2);
-    if (n > 3) v.w = __ldg(p + 3);
-    ulonglong2 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r.x) : "f"(v.x), "f"(v.y));
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r.y) : "f"(v.z), "f"(v.w));
-    return r;
-}
-
-template <int CIN, int FB, bool VEC>
-__global__ void __launch_bounds__(256, 2) dx_fewc_kernel(const float* __restrict__ dy, const float* __restrict__ w, float* __restrict__ dx,
-                                                         int S, int H, int W, int Cout, int fH, int fW, int sH, int sW, int pH, int pW,
-                                                         int Ho, int Wo) {
-    pdl_wait();
-    constexpr int PV = DXF_PV;
-    // this class: rows h = hs + a * sH, taps i = ph + sH * ti, dy row a + hq - ti (columns alike)
-    const int ph = blockIdx.z / sW, pw = blockIdx.z - ph * sW;
-    const int nH = ph < fH ? (fH - ph - 1) / sH + 1 : 0, nW = pw < fW ? (fW - pw - 1) / sW + 1 : 0;
-    const int hs = ((ph - pH) % sH + sH) % sH, ws = ((pw - pW) % sW + sW) % sW;
-    const int hq = (hs + pH - ph) / sH, wq = (ws + pW - pw) / sW;
-    const int MH = hs < H ? (H - hs - 1) / sH + 1 : 0, MW = ws < W ? (W - ws - 1) / sW + 1 : 0;
-    if (MH == 0 || MW == 0) return;
-    const int strips = (MH + PV - 1) / PV;
-    const long long items = 1LL * S * strips * MW;
-    const long long item = blockIdx.x * (256LL / DXF_LANES) + threadIdx.x / DXF_LANES;
-    const bool live = item < items;                     // (every lane takes part in the exchange below)
-    const int sub = threadIdx.x % DXF_LANES;
-    int b, a0;
-    long long s;
-    if (items < 1LL << 31) {
-        const unsigned it = live ? (unsigned)item : 0u, q = it / (unsigned)MW;
-        b = (int)(it - q * MW);
-        const unsigned s32 = q / (unsigned)strips;
-        a0 = (int)(q - s32 * strips) * PV;
-        s = s32;
-    } else {
-        const long long it = live ? item : 0, q = it / MW;
-        b = (int)(it - q * MW);
-        s = q / strips;
-        a0 = (int)(q - s * strips) * PV;
-    }
-
-    unsigned long long acc[PV][CIN];
-#pragma unroll
-    for (int p = 0; p < PV; ++p)
-#pragma unroll
-        for (int c = 0; c < CIN; ++c) acc[p][c] = 0ull;
-    const float* dys = dy + s * Ho * Wo * Cout;
-#pragma unroll 1
-    for (int ti0 = 0; ti0 < nH; ti0 += FB) {            // (FB divides nH)
-        const int r0 = a0 + hq - ti0 - (FB - 1);        // dy row of the first load
-#pragma unroll 1
-        for (int tj = 0; tj < nW; ++tj) {
-            const int wo = b + wq - tj;
-            if (!live || (unsigned)wo >= (unsigned)Wo) continue;
-#pragma unroll 1
-            for (int d = sub * 4; d < Cout; d += DXF_LANES * 4) {
-                ulonglong2 k[FB][CIN], v[PV + FB - 1];
-#pragma unroll
-                for (int r = 0; r < PV + FB - 1; ++r) {
-                    const int ho = r0 + r;
-                    v[r] = (unsigned)ho < (unsigned)Ho ? dxf_load4<VEC>(dys + ((long long)ho * Wo + wo) * Cout + d, Cout - d) : make_ulonglong2(0ull, 0ull);
-                }
-                const float* wt = w + ((long long)(ph + ti0 * sH) * fW + pw + tj * sW) * CIN * Cout + d;
-#pragma unroll
-                for (int t = 0; t < FB; ++t)
-#pragma unroll
-                    for (int c = 0; c < CIN; ++c) k[t][c] = dxf_load4<VEC>(wt + ((long long)t * sH * fW * CIN + c) * Cout, Cout - d);
-#pragma unroll
-                for (int p = 0; p < PV; ++p)
-#pragma unroll
-                    for (int t = 0; t < FB; ++t)
-#pragma unroll
-                        for (int c = 0; c < CIN; ++c) {
-                            dxf_fma2(acc[p][c], v[p + FB - 1 - t].x, k[t][c].x);
-                            dxf_fma2(acc[p][c], v[p + FB - 1 - t].y, k[t][c].y);
-                        }
-            }
-        }
-    }
-
-    // Eight lanes' sums of four pixels: two exchanges that halve the pixels a lane keeps, one that adds.
-    float f[PV][CIN];
-#pragma unroll
-    for (int p = 0; p < PV; ++p)
-#pragma unroll
-        for (int c = 0; c < CIN; ++c) f[p][c] = __uint_as_float((unsigned)acc[p][c]) + __uint_as_float((unsigned)(acc[p][c] >> 32));
-    const bool hi4 = sub & 4, hi2 = sub & 2;
-#pragma unroll
-    for (int c = 0; c < CIN; ++c) {
-        const float s0 = __shfl_xor_sync(0xffffffffu, hi4 ? f[0][c] : f[2][c], 4), s1 = __shfl_xor_sync(0xffffffffu, hi4 ? f[1][c] : f[3][c], 4);
-        const float u0 = (hi4 ? f[2][c] : f[0][c]) + s0, u1 = (hi4 ? f[3][c] : f[1][c]) + s1;
-        const float s2 = __shfl_xor_sync(0xffffffffu, hi2 ? u0 : u1, 2);
-        const float u = (hi2 ? u1 : u0) + s2;
-        f[0][c] = u + __shfl_xor_sync(0xffffffffu, u, 1);
-    }
-    const int a = a0 + (sub >> 1);
-    if (live && !(sub & 1) && a < MH) {
-        float* o = dx + ((s * H + hs + (long long)a * sH) * W + ws + (long long)b * sW) * CIN;
-#pragma unroll
-        for (int c = 0; c < CIN; ++c) o[c] = f[0][c];
     }
 }
 
@@ -547,38 +419,9 @@ int generic_head_softmax_fwd(const AetherConvDesc& d, const float* x, const floa
     return head_fwd(d, x, w, b, y, prob, st);
 }
 
-template <int CIN, int FB>
-static void dx_fewc_launch(const AetherConvDesc& d, const float* dy, const float* w, float* dx, int Ho, int Wo, cudaStream_t st) {
-    const bool vec = d.Cout % 4 == 0 && ((reinterpret_cast<uintptr_t>(dy) | reinterpret_cast<uintptr_t>(w)) & 15u) == 0;
-    const int MH = ceil_div(d.H, d.sH), MW = ceil_div(d.W, d.sW);            // extent of the largest class
-    const long long items = 1LL * d.S * ceil_div(MH, DXF_PV) * MW;
-    const dim3 grid((unsigned)((items + 256 / DXF_LANES - 1) / (256 / DXF_LANES)), 1, d.sH * d.sW);
-    launch(vec ? dx_fewc_kernel<CIN, FB, true> : dx_fewc_kernel<CIN, FB, false>, grid, 256, 0, st, dy, w, dx, d.S, d.H, d.W, d.Cout, d.fH, d.fW,
-           d.sH, d.sW, d.padH, d.padW, Ho, Wo);
-}
-
-template <int CIN>
-static int dx_fewc(const AetherConvDesc& d, const float* dy, const float* w, float* dx, int Ho, int Wo, cudaStream_t st) {
-    // filter rows per pass: all of the usual filters' (their CIN * rows vectors fit the registers), else one
-    if (d.sH == 1 && d.fH == 3) dx_fewc_launch<CIN, 3>(d, dy, w, dx, Ho, Wo, st);
-    else if (d.sH == 1 && d.fH == 5) dx_fewc_launch<CIN, 5>(d, dy, w, dx, Ho, Wo, st);
-    else dx_fewc_launch<CIN, 1>(d, dy, w, dx, Ho, Wo, st);
-    count_launch();
-    return check_launch("dx_fewc_kernel");
-}
-
 int generic_conv_bwd_data(const AetherConvDesc& d, const float* dy, const float* w, float* dx, void* ws, size_t ws_bytes, cudaStream_t st) {
-    int Ho, Wo;
-    conv_out_hw(d, Ho, Wo);
     // (Few input channels leave a GEMM tile's columns empty.  More than 65535 pixel classes do not fit one grid.)
-    if (d.Cin <= 4 && 1LL * d.sH * d.sW <= 65535) {
-        switch (d.Cin) {
-            case 1: return dx_fewc<1>(d, dy, w, dx, Ho, Wo, st);
-            case 2: return dx_fewc<2>(d, dy, w, dx, Ho, Wo, st);
-            case 3: return dx_fewc<3>(d, dy, w, dx, Ho, Wo, st);
-            default: return dx_fewc<4>(d, dy, w, dx, Ho, Wo, st);
-        }
-    }
+    if (d.Cin <= 4 && 1LL * d.sH * d.sW <= 65535) return dx_few_conv_bwd_data(d, dy, w, dx, st);
     return simt_conv_bwd_data(d, dy, w, dx, ws, ws_bytes, st);
 }
 

@@ -1,0 +1,40 @@
+"""dX of first layers at stride 1 with 3x3 and 5x5 filters, tile by tile: strips of 4 and 8 rows, tiles of 8, 16 and 32 columns, strips of several images in
+a tile, one and several chunks of channels, more tiles than blocks (the two stages' barriers change phase), few output channels (two groups of columns),
+paddings other than "same".  fp32 sums of n products in any order: within n roundings of 2^-24 of the sum of absolute values."""
+import pytest
+
+from aether_ml_b200 import _lib
+
+pytestmark = pytest.mark.gpu
+
+# (S, H, W, Cin, Cout, f, padH, padW)
+SHAPES = [(128, 32, 32, 3, 32, 3, 1, 1), (600, 17, 33, 1, 64, 3, 1, 1), (330, 16, 40, 3, 36, 3, 1, 1), (700, 7, 7, 3, 100, 3, 1, 1), (701, 9, 14, 2, 12, 3, 1, 1),
+          (64, 28, 28, 4, 32, 3, 0, 0), (90, 33, 31, 3, 72, 5, 2, 2), (200, 20, 28, 1, 16, 5, 2, 2), (130, 30, 64, 3, 16, 5, 0, 0), (40, 8, 8, 4, 128, 5, 2, 2),
+          (3, 70, 41, 3, 33, 3, 1, 1), (150, 20, 21, 4, 61, 5, 2, 2), (20, 11, 13, 3, 24, 3, 2, 0), (9, 12, 10, 1, 32, 5, 4, 5), (1, 3, 3, 3, 4, 3, 0, 0)]
+
+
+@pytest.mark.parametrize("S,H,W,Cin,Cout,f,ph,pw", SHAPES)
+def test_dx_of_first_layers_by_tiles(S, H, W, Cin, Cout, f, ph, pw):
+    import torch
+    lib = _lib.lib()
+    g = torch.Generator(device="cuda").manual_seed(S + Cout)
+    Ho, Wo = H + 2 * ph - f + 1, W + 2 * pw - f + 1
+    dy, w = torch.randn((S, Ho, Wo, Cout), generator=g, device="cuda"), torch.randn((f, f, Cin, Cout), generator=g, device="cuda")
+    d = _lib.AetherConvDesc(S, H, W, Cin, Cout, f, f, 1, 1, ph, pw, 0)
+    ws = torch.empty(lib.aether_conv2d_workspace_bytes(d) + 16, dtype=torch.uint8, device="cuda")
+    dx = torch.full((S, H, W, Cin), float("nan"), device="cuda")
+    stream = torch.cuda.current_stream().cuda_stream
+    for _ in range(2):
+        assert lib.aether_conv2d_bwd(d, None, dy.data_ptr(), w.data_ptr(), dx.data_ptr(), None, None, ws.data_ptr(), ws.numel(), 0, stream) == 0
+
+    def gather(a, b):                                       # in float64: dy padded by what a tap can reach, a product per tap
+        pad = torch.nn.functional.pad(a, (0, 0, f, f + pw, f, f + ph))
+        out = torch.zeros((S, H, W, Cin), dtype=torch.float64, device="cuda")
+        for i in range(f):
+            for j in range(f):
+                r, c = ph - i + f, pw - j + f
+                out += pad[:, r:r + H, c:c + W] @ b[i, j].T
+        return out
+    want, size = gather(dy.double(), w.double()), gather(dy.double().abs(), w.double().abs())
+    assert bool(((dx.double() - want).abs() <= f * f * Cout * 2.0**-24 * size + 1e-30).all())
+    assert _lib.device_status() == 0
