@@ -22,9 +22,11 @@
 // channels with zeros behind the last: channel counts need not be multiples of anything.  A strided layer's x is stored by
 // phases, so that a tap's pixels lie side by side (element strides in the tensor map halve the copies' rate).
 // Measured on B200, forward + backward, CUDA cores / this file: 40 x 33x32 64->128 442 / 131 us, 96 x 28x28 32->64 207 / 100, 100 x 57x45
-// 48->72 stride 2 431 / 193 (one set of inputs; three in turn, as a program's arrays come: 211 / 104, 433 / 212).  No unit is saturated: the
-// tensor pipe is 24-48 % busy, L1 and shared memory 40-67 %, DRAM 6-31 % (a filter kept in shared memory changes 1 %).  What is left is the chain of a tile: the
-// first stages of a unit wait for their copies, and the warps that sum store (2-3 thousand clocks) before they take products again.
+// 48->72 stride 2 431 / 187 (one set of inputs; three in turn, as a program's arrays come: 211 / 104, 433 / 206).  No unit is saturated: the
+// tensor pipe is 24-48 % busy, L1 and shared memory 40-67 %, DRAM 6-31 %.  What bounds it is shared memory: the MMAs take 224 clocks for a step of 64 columns
+// by themselves (28 KB of operands), and with the copies' writes (18 KB a step) 340; about 150 bytes per clock in all, forward, dX and dW alike.  Neither the number of
+// threads that issue nor the stores matter then (both measured, two teams of summing warps and products spread over two threads: no change; all
+// sums of a stage side by side in 192 columns: 30 -> 35-39 us, TMEM gives some 110 bytes per clock beside the MMAs).
 #include <string.h>
 
 #include <cuda_bf16.h>
@@ -81,7 +83,7 @@ struct SplitParams {
     int fH, fW, sH, sW, pH, pW, Cin, Cout;
     int dx;               // gather over dy, a stride's input pixels in sH * sW classes
     int BW, BH, BN, rows, tiles_w, tiles_h, tiles_n;
-    int NT, n_tiles_n;    // column tile (a multiple of 16; dW: 64)
+    int NT, n_tiles_n;    // column tile (a multiple of 16; dW: 64 or 128)
     int kchunks, last_ksteps;
     int units;
     SplitDiv by_ntn, by_tiles, by_tw, by_th, by_groups;     // column tiles, pixel tiles, tile columns, tile rows, groups of row units
@@ -97,7 +99,7 @@ struct SplitCfg {
     static constexpr int UNITS = 128 / KC;                                  // dW: row units of the 128 accumulator rows
     static constexpr int A_PART = DW ? UNITS * DW_PIXELS * ROW : 128 * ROW; // one part of the 128 accumulator rows' operand
     static constexpr int STAGE_A = 3 * A_PART;
-    static constexpr int STAGE_B = 3 * NTMAX * (DW ? 2 * DW_PIXELS : ROW);  // (dW: 64 channels of dy per row)
+    static constexpr int STAGE_B = 3 * NTMAX * (DW ? 2 * DW_PIXELS : ROW);  // (dW: tiles of 64 channels of dy)
     static constexpr int FIT = (216 * 1024) / (STAGE_A + STAGE_B), STAGES = FIT < 6 ? FIT : 6;
     static constexpr int SMEM_BYTES = 1024 + STAGES * (STAGE_A + STAGE_B) + 256;
     static constexpr int NBG = NTMAX <= 64 ? 4 : 2;             // accumulators of a stage's x0 w0
@@ -314,7 +316,7 @@ __global__ void __launch_bounds__(SPLIT_THREADS, 1) split_conv_kernel(const __gr
     using Cfg = SplitCfg<NTMAX, DW, KC>;
     constexpr int STAGES = Cfg::STAGES, NBG = Cfg::NBG, NBC = Cfg::NBC, STAGE = Cfg::STAGE_A + Cfg::STAGE_B;
     constexpr int UNITS = Cfg::UNITS;
-    constexpr int TILE = DW_PIXELS * Cfg::ROW, DY_TILE = DW_PIXELS * 128;      // dW: KC channels of x, 64 channels of dy of a box of pixels
+    constexpr int TILE = DW_PIXELS * Cfg::ROW, DY_TILE = DW_PIXELS * 128, DY_TILES = NTMAX / 64;      // dW: KC channels of x, 64 channels of dy of a box of pixels
     extern __shared__ uint8_t smem_raw[];
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     const uint32_t sBar = smem_base + STAGES * STAGE;
@@ -368,7 +370,7 @@ __global__ void __launch_bounds__(SPLIT_THREADS, 1) split_conv_kernel(const __gr
     const uint32_t tmem_c = tmem_base + NBG * NTMAX;           // accumulators of the small products
 
     const int NT = p.NT;
-    const int b_part = DW ? DY_TILE : NT * Cfg::ROW;                       // bytes of one part of the columns' operand
+    const int b_part = DW ? DY_TILES * DY_TILE : NT * Cfg::ROW;                       // bytes of one part of the columns' operand
     auto decode = [&](int u, int& nt, int& mt, int& cls, int& t0, int& t1) { split_unit<DW>(p, u, nt, mt, cls, t0, t1); };
     // stages of a unit, and steps of one of them
     auto unit_stages = [&](int cls, int t0, int t1) {
@@ -384,7 +386,7 @@ __global__ void __launch_bounds__(SPLIT_THREADS, 1) split_conv_kernel(const __gr
         auto copies = [&](auto rows_tag) {
             constexpr bool ROWS = decltype(rows_tag)::value;
             uint32_t s = 0, ph = 0;
-            const uint32_t tx = 3u * (DW ? (uint32_t)p.rows * (ROWS ? 256u : 128u) : (uint32_t)(ROWS ? p.rows : NT) * Cfg::ROW);
+            const uint32_t tx = 3u * (DW ? (uint32_t)p.rows * (ROWS ? 256u : DY_TILES * 128u) : (uint32_t)(ROWS ? p.rows : NT) * Cfg::ROW);
             const int phases = p.dx ? 1 : p.sH * p.sW;
             auto free_stage = [&] { return __all_sync(0xffffffffu, mbar_wait_spin(empty_bar(s), ph ^ 1u, p.status, DS_TIMEOUT_EMPTY)) != 0; };
             for (int u = blockIdx.x; u < p.units; u += gridDim.x) {
@@ -415,7 +417,8 @@ __global__ void __launch_bounds__(SPLIT_THREADS, 1) split_conv_kernel(const __gr
                                     for (int k = 0; k < UNITS; ++k)
                                         tma_load_5d(at + q * Cfg::A_PART + k * TILE, &p.tm_a, bar, uc[k], w0 + uw[k], h0 + uh[k], n0, q * phases + uf[k]);
                                 } else {
-                                    tma_load_5d(at + q * DY_TILE, &p.tm_b, bar, nt * NT, w0, h0, n0, q);
+#pragma unroll
+                                    for (int k = 0; k < DY_TILES; ++k) tma_load_5d(at + (q * DY_TILES + k) * DY_TILE, &p.tm_b, bar, nt * NT + 64 * k, w0, h0, n0, q);
                                 }
                             }
                         }
@@ -811,7 +814,7 @@ struct SplitPlan {
     bool use;
     int Ho, Wo, taps, Cin_p, Cout_p, PH, PW;      // PH, PW: a phase's extent
     PixelTiling til_fwd, til_dx, til_dw;
-    int nt_fwd, nt_dx, kc_in, kc_out, splits, cblocks, U, ldn, db_blocks;
+    int nt_fwd, nt_dx, nt_dw, kc_in, kc_out, splits, cblocks, U, ldn, db_blocks;
     size_t off_wf, off_wd, off_x, off_dy, off_part, off_dbpart, fwd_total, total;      // (what a forward pass needs lies in front)
 };
 
@@ -886,10 +889,21 @@ static SplitPlan compute_split_plan(const AetherConvDesc& d) {
     pl.cblocks = ceil_div(d.Cin, pl.kc_in);
     pl.U = pl.taps * pl.cblocks;
     pl.ldn = (d.Cout + 3) / 4 * 4;
-    const long long cols = 1LL * ceil_div(pl.U, 128 / pl.kc_in) * ceil_div(d.Cout, 64), ptiles = pl.til_dw.total();
-    long long splits = num_sms() / cols;
-    if (splits > ptiles / 4) splits = ptiles / 4;
-    pl.splits = (int)(splits < 1 ? 1 : splits);
+    // dW: 64 or 128 channels of dy per unit.  Shared memory is what bounds the kernel (some 150 bytes per clock, copies and operand reads together): per
+    // step and 128 columns 40 KB of operands and 24 KB of copies, 56 and 36 in two units.  A stage takes 0.74 / 1.16 us, and the partial
+    // sums of a split are written and read again: 64 x 28x28 128->128 96 -> 78 us, 40 x 33x32 64->128 5x5 106 -> 82, 100 x 57x45 48->72 stride 2
+    // 74 -> 68; 200 x 14x14 72->144 90 -> 94, 16 x 7x7 256->256 16.2 -> 17.5 and 12 x 24x24 16->146 18.5 -> 20.3 stay with 64.
+    const long long ptiles = pl.til_dw.total();
+    double best = 1e300;
+    for (int nt = 64; nt <= (d.Cout > 64 ? 128 : 64); nt += 64) {
+        const long long cols = 1LL * ceil_div(pl.U, 128 / pl.kc_in) * ceil_div(d.Cout, nt);
+        long long splits = num_sms() / cols;
+        if (splits > ptiles / 4) splits = ptiles / 4;
+        if (splits < 1) splits = 1;
+        const double rounds = (double)((cols * splits + num_sms() - 1) / num_sms());
+        const double us = rounds * (double)((ptiles + splits - 1) / splits) * (nt == 64 ? 0.74 : 1.16) + 8.0 * splits * pl.U * pl.kc_in * pl.ldn / 5e6;
+        if (us < best) { best = us; pl.nt_dw = nt; pl.splits = (int)splits; }
+    }
     pl.db_blocks = (int)(out_rows < 4ull * num_sms() * 64 ? (out_rows + 63) / 64 : 4ull * num_sms());
     size_t off = 0;
     auto take = [&](size_t bytes) { size_t o = off; off = align_up(off + bytes, 1024); return o; };
@@ -1035,7 +1049,7 @@ int split_conv_bwd(const AetherConvDesc& d, const float* x, const float* dy, con
     SplitParams p;
     memset(&p, 0, sizeof(p));
     const PixelTiling& t = pl.til_dw;
-    p.NT = 64;
+    p.NT = pl.nt_dw;
     p.n_tiles_n = ceil_div(d.Cout, p.NT);
     split_geometry(p, d, t);
     p.in = x; p.w = dy; p.out = reinterpret_cast<float*>(wsb + pl.off_part);
@@ -1048,7 +1062,9 @@ int split_conv_bwd(const AetherConvDesc& d, const float* x, const float* dy, con
     p.units = groups * p.n_tiles_n * p.splits;
     if ((rc = split_pixel_map(&p.tm_a, wsb + pl.off_x, pl.Cin_p, pl.PW, pl.PH, d.S, d.sH * d.sW, t, pl.kc_in))) return rc;
     if ((rc = split_pixel_map(&p.tm_b, wsb + pl.off_dy, pl.Cout_p, pl.Wo, pl.Ho, d.S, 1, t, 64))) return rc;
-    if ((rc = pl.kc_in == 32 ? launch_split<64, true, 32>(p, PK_DW, st) : launch_split<64, true, 64>(p, PK_DW, st))) return rc;
+    if (p.NT == 64) rc = pl.kc_in == 32 ? launch_split<64, true, 32>(p, PK_DW, st) : launch_split<64, true, 64>(p, PK_DW, st);
+    else rc = pl.kc_in == 32 ? launch_split<128, true, 32>(p, PK_DW, st) : launch_split<128, true, 64>(p, PK_DW, st);
+    if (rc) return rc;
     return dw_reduce(p.out, dw, p.splits, p.U, pl.kc_in, p.ldn, p.cblocks, pl.taps, d.Cin, d.Cout, pl.taps, p.splits, dbpart, pl.db_blocks, db, st);
 }
 
