@@ -232,6 +232,15 @@ extern "C" int aether_conv2d_fwd_ex(const AetherConvDesc* d, const float* x, con
     return aether_conv2d_fwd(d, x, w, b, y, ws, ws_bytes, stream);
 }
 
+extern "C" int aether_conv2d_filter_copies(const AetherConvDesc* d, const float* w, void* ws, size_t ws_bytes, void* stream) {
+    int rc = validate_desc(d, "aether_conv2d_filter_copies");
+    if (rc) return rc;
+    if (!w || !ws || !aligned16(w) || !aligned16(ws)) return set_error(AE_BAD_ARG, "aether_conv2d_filter_copies: null pointer or not 16-byte aligned");
+    if (!tc_conv_eligible(*d) || d->math_mode != AETHER_MATH_BF16)
+        return set_error(AE_UNSUPPORTED, "aether_conv2d_filter_copies: this shape / math mode has no copies that a forward call reads");
+    return tc_conv_filter_copies(*d, w, ws, ws_bytes, static_cast<cudaStream_t>(stream));
+}
+
 extern "C" int aether_conv2d_act_fwd(const AetherConvDesc* d, const float* x, const float* w, const float* b, float* y, float* act_out,
                                      float alpha, void* act_copy, int copy_ld, void* ws, size_t ws_bytes, int flags, void* stream) {
     int rc = validate_desc(d, "aether_conv2d_act_fwd");

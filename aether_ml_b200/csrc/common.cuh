@@ -135,6 +135,7 @@ struct ActEpilogue {
 };
 int tc_conv_fwd(const AetherConvDesc& d, const float* x, const float* w, const float* b, float* y, float* stats, void* ws,
                 size_t ws_bytes, int flags, cudaStream_t st, const ActEpilogue* act = nullptr, bool* act_done = nullptr);
+int tc_conv_filter_copies(const AetherConvDesc& d, const float* w, void* ws, size_t ws_bytes, cudaStream_t st);
 bool tc_conv_operand_layout(const AetherConvDesc& d, AetherOperandLayout* out);
 long long tc_conv_stats_blocks(const AetherConvDesc& d);
 int tc_conv_bwd(const AetherConvDesc& d, const float* x, const float* dy, const float* w, float* dx, float* dw,

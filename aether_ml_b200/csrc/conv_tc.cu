@@ -1407,6 +1407,15 @@ long long tc_conv_stats_blocks(const AetherConvDesc& d) {
     return 2LL * (grid / n_tiles_n);
 }
 
+// Both filter operands (forward: transposed, dX: as stored) from one read of w.
+int tc_conv_filter_copies(const AetherConvDesc& d, const float* w, void* ws, size_t ws_bytes, cudaStream_t st) {
+    const TcPlan& pl = make_plan(d);
+    if (ws_bytes < pl.total) return set_error(AE_BAD_ARG, "conv workspace too small: %zu < %zu", ws_bytes, pl.total);
+    uint8_t* wsb = static_cast<uint8_t*>(ws);
+    return launch_filter_shadows<__nv_bfloat16>(w, reinterpret_cast<__nv_bfloat16*>(wsb + pl.off_wf), reinterpret_cast<__nv_bfloat16*>(wsb + pl.off_wd),
+                                                pl.taps, d.Cin, d.Cout, pl.Cin_p, pl.Cout_p, st);
+}
+
 int tc_conv_fwd(const AetherConvDesc& d, const float* x, const float* w, const float* b, float* y, float* stats, void* ws,
                 size_t ws_bytes, int flags, cudaStream_t st, const ActEpilogue* act, bool* act_done) {
     const TcPlan& pl = make_plan(d);
@@ -1427,12 +1436,8 @@ int tc_conv_fwd(const AetherConvDesc& d, const float* x, const float* w, const f
     if (!(flags & AETHER_CONV_X_COPY_READY) &&
         (rc = launch_cast(x, xsh, 1LL * d.S * d.H * d.W, d.Cin, pl.Cin_p, nullptr, 0, st)))
         return rc;
-    // both filter operands (forward: transposed, dX: as stored) from one read of w; a backward call that is told
-    // the weights have not changed since (x_shadow_valid bit 1) reuses the second one
-    __nv_bfloat16* wd = reinterpret_cast<__nv_bfloat16*>(wsb + pl.off_wd);
-    if (!(flags & AETHER_CONV_W_COPY_READY) &&
-        (rc = launch_filter_shadows<__nv_bfloat16>(w, wf, wd, pl.taps, d.Cin, d.Cout, pl.Cin_p, pl.Cout_p, st)))
-        return rc;
+    // (a backward call that is told the weights have not changed since -- x_shadow_valid bit 1 -- reuses the second of them)
+    if (!(flags & AETHER_CONV_W_COPY_READY) && (rc = tc_conv_filter_copies(d, w, ws, ws_bytes, st))) return rc;
     return run_igemm(false, xsh, pl.Cin_p, d.H, d.W, d.S, wf, pl.Cin_p, pl.Cout_p, pl.taps, y, d.Cout, pl.Ho, pl.Wo,
                      pl.til_out, pl.Cout_p, d.fH, d.fW, +1, -d.padH, -d.padW, d.Cin, b, stats, st, act, act_done);
 }

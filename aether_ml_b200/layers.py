@@ -202,8 +202,60 @@ def _array_tag(t):
     return host().tag(t)[:3]
 
 
+class _Branch:
+    """A second stream inside the capture of a train step: work that nothing on the main one waits for until its end.  Arrays that
+    the branch uses must outlive the capture or be held here: memory that the main stream's arrays give back is handed out
+    to its next ones whatever the branch still does."""
+
+    def __init__(self):
+        self.stream = torch.cuda.Stream()
+        self.open = False
+        self.held = []
+
+    def fork(self, *arrays):
+        """What is put on the branch from here on starts behind what the current stream has been given so far."""
+        self.stream.wait_stream(torch.cuda.current_stream())
+        self.open = True
+        self.held.extend(arrays)
+
+    def join(self):
+        if self.open:
+            torch.cuda.current_stream().wait_stream(self.stream)
+            self.open = False
+
+
 class _TakesCopies:
     """What the layers with bf16 operand copies in their workspace share."""
+    _weights_fixed = False      # Model: the weights do not change between the batches of a predict / evaluate call, or have been copied ahead of a captured step
+    _branch = None              # a _Branch while Model captures a step
+
+    def _copy_weights(self):
+        """The operand copies of the weights alone, on the branch, for a forward pass like the last one; False: it makes its own."""
+        p, w = self._last_plan()
+        ws = self._ws
+        if p is None or p.layout is None or p.layout.x_copy_ld == 0 or ws.buf is None or ws.size < p.ws_bytes:
+            return False
+        self._branch.fork(w, ws.buf)
+        with torch.cuda.stream(self._branch.stream):
+            host().aether_conv2d_filter_copies(p.raw, w, ws.buf, ws.size)
+        self._copies.record(ws.buf, w, w)       # (of an x there is none)
+        return True
+
+    def _products(self, p, x, dy, w, dx, db, ws, flags, rows, behind=None):
+        """The backward pass's library call, then `behind` (of the parameters' gradients).  While a step is captured dW goes to the branch, beside
+        the kernels of the layers in front, which wait for dX only."""
+        H, b = host(), self._branch
+        if b is None or dx is None or not flags & _lib.CONV_DY_COPY_READY:
+            H.aether_conv2d_bwd_ex(p.raw, x, dy, w, dx, self.dweights, db, ws, self._ws.size, flags, rows)
+            if behind is not None:
+                behind()
+            return
+        b.fork(x, dy, w, ws, self.dweights, self.dbiases)
+        H.aether_conv2d_bwd_ex(p.raw, x, dy, w, dx, None, None, ws, self._ws.size, flags, rows)
+        with torch.cuda.stream(b.stream):
+            H.aether_conv2d_bwd_ex(p.raw, x, dy, w, None, self.dweights, db, ws, self._ws.size, flags, rows)
+            if behind is not None:
+                behind()
 
     def _forget_copies(self):
         """The workspace's contents are no longer what the last passes left there."""
@@ -270,7 +322,6 @@ class Conv_Layer(_TakesCopies, _Saved):
     reference's CUDA scatter kernel produces (:4-35), returned contiguous instead of as a sliced view.
     One extra keyword, ``math_mode`` in {"bf16", "tf32", "fp32"}, selects the operand precision of
     the tensor-core kernels (default from $AETHER_MATH_MODE, else bf16)."""
-    _weights_fixed = False      # Model.predict / evaluate: the weights do not change between the batches of the call
 
     def __init__(self, input_shape, num_filters=1, filter_size=(3, 3), strides=(1, 1), padding="same",
                  math_mode=None):
@@ -323,6 +374,9 @@ class Conv_Layer(_TakesCopies, _Saved):
     @weights.setter
     def weights(self, value):
         self.filter_weights = value
+
+    def _last_plan(self):
+        return self._desc, self.filter_weights
 
     def _plan(self, shape):
         """What follows from an input shape and this layer's settings, worked out once per combination."""
@@ -402,6 +456,8 @@ class Conv_Layer(_TakesCopies, _Saved):
             _require_written(x, "Conv_Layer.forward")
         if self._weights_fixed and p.layout is not None and self._copies.weights_valid(ws, w):
             flags |= _lib.CONV_W_COPY_READY
+            if self._branch is not None:
+                self._branch.join()
         # With emit_bn_stats the kernel's epilogue also writes the per-channel partial statistics that the
         # Batch_Norm behind this layer would otherwise compute in a pass of its own over y (:467-470).
         nblk = p.stats_blocks if (training and self.emit_bn_stats) else 0
@@ -448,7 +504,7 @@ class Conv_Layer(_TakesCopies, _Saved):
             _require_written(dy, "Conv_Layer.backward")
         if not (shadow_ok & _lib.CONV_X_COPY_READY):
             _require_written(x, "Conv_Layer.backward")
-        H.aether_conv2d_bwd_ex(p.raw, x, dy, w, dx, self.dweights, self.dbiases, ws, self._ws.size, shadow_ok, rows)
+        self._products(p, x, dy, w, dx, self.dbiases, ws, shadow_ok, rows)
         self.dinputs = dx
         return dx
 
@@ -929,7 +985,6 @@ class Layer_Dense(_TakesCopies, _Saved):
     convolution kernels as a 1x1 convolution on a 1x1 image (x (S,n_in) is NHWC with H=W=1; weights
     (n_in,n_out) are a (1,1,Cin,Cout) filter), so they use the same tensor-core path.  Parameters are
     fp32 (the reference's are fp64 because ``randn`` is); biases keep the (1, n_out) shape."""
-    _weights_fixed = False
 
     def __init__(self, n_inputs, n_neurons, weight_regularizer_l1=0, bias_regularizer_l1=0,
                  weight_regularizer_l2=0, bias_regularizer_l2=0, math_mode=None):
@@ -953,6 +1008,9 @@ class Layer_Dense(_TakesCopies, _Saved):
         self._copies = _OperandCopies()
         self._handed = _HandedIn()
         self._used = (None, None)       # plan and weights of the last forward pass
+
+    def _last_plan(self):
+        return self._used[0], self.weights
 
     def x_copy_target(self, shape):
         """(address, row length) where the bf16 copy of an input of `shape` (any shape that flattens to
@@ -1004,6 +1062,8 @@ class Layer_Dense(_TakesCopies, _Saved):
             _require_written(x, "Layer_Dense.forward")
         if self._weights_fixed and p.layout is not None and self._copies.weights_valid(ws, self.weights):
             flags |= _lib.CONV_W_COPY_READY
+            if self._branch is not None:
+                self._branch.join()
         return ws, flags
 
     def forward(self, inputs, training):
@@ -1100,10 +1160,9 @@ class Layer_Dense(_TakesCopies, _Saved):
         if not (flags & _lib.CONV_X_COPY_READY):
             _require_written(x, "Layer_Dense.backward")
         if dy_ready:
-            H.aether_conv2d_bwd_ex(p.raw, x, dy, w, dx, self.dweights, None, ws, self._ws.size, flags | _lib.CONV_DY_COPY_READY, 1)
+            self._products(p, x, dy, w, dx, None, ws, flags | _lib.CONV_DY_COPY_READY, 1, self._regularize)
         else:
-            H.aether_conv2d_bwd_ex(p.raw, x, dy, w, dx, self.dweights, self.dbiases, ws, self._ws.size, flags, 0)
-        self._regularize()
+            self._products(p, x, dy, w, dx, self.dbiases, ws, flags, 0, self._regularize)
         self.dinputs = dx
         return self.dinputs
 

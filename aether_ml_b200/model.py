@@ -11,6 +11,7 @@ Additions that the reference does not have, all optional:
     parallelism -- one all-reduce cover the whole network;
   * ``train_step(X, y)`` runs one forward/backward/update without printing or host synchronisation.
 """
+import contextlib
 import math
 import pickle
 import weakref
@@ -20,7 +21,7 @@ import torch
 
 from ._lib import host
 from .layers import (Activation_Softmax_Loss_CategoricalCrossEntropy, Batch_Norm, Conv_Layer, Flatten, Layer_Dense, Layer_Dropout,
-                     Layer_Dropout_Spatial, Leaky_ReLU, Loss_CategoricalCrossEntropy, Optimizer_Adam, Pooling, ReLU, SoftMax, to_device, _labels,
+                     Layer_Dropout_Spatial, Leaky_ReLU, Loss_CategoricalCrossEntropy, Optimizer_Adam, Pooling, ReLU, SoftMax, to_device, _Branch, _labels,
                      _labels_i32, _link, _softmax_cce, _Saved, _TakesCopies, _Workspace)
 
 
@@ -799,9 +800,10 @@ class Model:
             self._graph = torch.cuda.CUDAGraph()
             held, self._bucket_of_layer = self._bucket_of_layer, {}
             try:
-                with torch.cuda.graph(self._graph, capture_error_mode="thread_local"):
+                with torch.cuda.graph(self._graph, capture_error_mode="thread_local"), self._branched() as branch:
                     self._g_out = self.forward(self._g_X, training=True)
                     self.backward(self._g_out, self._g_y)
+                    branch.join()
                     if not eager_between:
                         self._apply_optimizer()
                         if self._graph_metrics:
@@ -818,6 +820,22 @@ class Model:
                     self.capture_note = "two graphs, collectives eager"
         opt.iterations = saved_it           # capture records work, it does not run it
         return self._graph
+
+    @contextlib.contextmanager
+    def _branched(self):
+        """Inside it the layers put on a second stream what the layers behind them do not wait for: the operand copies of the weights, made beside
+        the first layers, and the parameters' gradients, made beside the layers in front."""
+        layers = [l for l in self.layers if isinstance(l, _TakesCopies)]
+        branch = _Branch()
+        try:
+            for l in layers:
+                l._branch = branch
+            for l in layers:
+                l._weights_fixed = l._copy_weights()
+            yield branch
+        finally:
+            for l in layers:
+                l._branch, l._weights_fixed = None, False
 
     def release_graphs(self):
         """Drops the captured graphs (and the batch buffers they read).  A graph that recorded collectives keeps the

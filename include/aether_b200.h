@@ -149,6 +149,9 @@ enum { AETHER_CONV_X_COPY_READY = 1, AETHER_CONV_W_COPY_READY = 2, AETHER_CONV_D
 int aether_conv2d_operand_layout(const AetherConvDesc* desc, AetherOperandLayout* out);
 int aether_conv2d_fwd_ex(const AetherConvDesc* desc, const float* x, const float* w, const float* b, float* y, float* stats,
                          size_t stats_bytes, void* ws, size_t ws_bytes, int flags, void* stream);
+/* The filter's copies alone, as a forward call of this layer would leave them in ws: calls with AETHER_CONV_W_COPY_READY find them there (a
+ * program that runs several layers can have them made beside the first ones).  bf16 mode, shapes with operand copies of x. */
+int aether_conv2d_filter_copies(const AetherConvDesc* desc, const float* w, void* ws, size_t ws_bytes, void* stream);
 
 /* The forward pass and the (leaky) ReLU behind it (a Dense layer of a small network is a launch of its own for each): y as
  * aether_conv2d_fwd_ex writes it, act_out = y > 0 ? y : alpha * y and, when given, the bf16 operand copy of act_out for the
