@@ -251,21 +251,16 @@ int run_rows_dw(const void* x_sh, int Cin_p, int H, int W, int S, const void* dy
     const int rows_a = 2;
     const int smem_max = 232448;
     const int avail = smem_max - 1024 - 256;
-    int BH = 0, stages = 0, ksteps = 0, dyr = 0, xr = 0;
-    for (int bh = (Ho < 16 ? Ho : 16); bh >= 1; --bh) {
-        if (bh + rows_a - 1 > 256) continue;
-        const int ks = ceil_div(bh * Wp, 16);
-        const int dyr_b = (int)align_up((size_t)ks * 16 * 128, 1024);
+    auto dy_bytes = [&](int bh) { return (int)align_up((size_t)ceil_div(bh * Wp, 16) * 16 * 128, 1024); };
+    auto x_bytes = [&](int bh) {
         // the MMAs of filter row r, tap j read x rows up to ks*16 + (rows_a-1)*Wp + fW-1
-        const int x_rows = ks * 16 + (rows_a - 1) * Wp + fW;
-        const int x_need = (bh + rows_a - 1) * Wp;
-        const int xr_b = (int)align_up((size_t)(x_rows > x_need ? x_rows : x_need) * 128, 1024);
-        const int stage = 2 * dyr_b + xr_b;
-        const int stg = avail / stage;
-        if (stg >= 3) { BH = bh; stages = stg > 4 ? 4 : stg; ksteps = ks; dyr = dyr_b; xr = xr_b; break; }
-        if (stg >= 2 && BH == 0) { BH = bh; stages = 2; ksteps = ks; dyr = dyr_b; xr = xr_b; }
-    }
+        const int x_rows = ceil_div(bh * Wp, 16) * 16 + (rows_a - 1) * Wp + fW, x_need = (bh + rows_a - 1) * Wp;
+        return (int)align_up((size_t)(x_rows > x_need ? x_rows : x_need) * 128, 1024);
+    };
+    int stages = 0;
+    const int BH = pick_strip_rows(Ho, Wp, avail, [&](int bh) { return 2 * dy_bytes(bh) + x_bytes(bh); }, &stages);
     if (BH == 0) return AE_OK;
+    const int ksteps = ceil_div(BH * Wp, 16), dyr = dy_bytes(BH), xr = x_bytes(BH);
     const int tiles_h = ceil_div(Ho, BH);
     const int units = (Cin_p / 64) * (Cout_p / 128);
     int sa = 0, sb = 0;

@@ -213,18 +213,11 @@ int run_halo_dw(const void* x_sh, int Cin_p, int H, int W, int S, const void* dy
     const int npairs = (taps + 1) / 2;
     const int smem_max = 232448;
     const int avail = smem_max - 1024 - 256;
-    int best_bh = 0, best_stages = 0;
-    for (int bh = (Ho < 16 ? Ho : 16); bh >= 1; --bh) {
-        if (bh + fH - 1 > 256) continue;
-        const int xr = (int)align_up((size_t)(bh + fH - 1) * Wp * 128, 1024);
-        const int ks = ceil_div(bh * Wp, 16);
-        const int stage = xr + (int)align_up((size_t)ks * 16 * 128, 1024);
-        const int stg = avail / stage;
-        if (stg >= 3) { best_bh = bh; best_stages = stg > 4 ? 4 : stg; break; }
-        if (stg >= 2 && best_bh == 0) { best_bh = bh; best_stages = 2; }
-    }
-    if (best_bh == 0) return AE_OK;
-    const int BH = best_bh;
+    int best_stages = 0;
+    const int BH = pick_strip_rows(Ho, Wp, avail, [&](int bh) {
+        return (int)(align_up((size_t)(bh + fH - 1) * Wp * 128, 1024) + align_up((size_t)ceil_div(bh * Wp, 16) * 16 * 128, 1024));
+    }, &best_stages);
+    if (BH == 0) return AE_OK;
     DwHaloParams p;
     memset(&p, 0, sizeof(p));
     int rc;

@@ -1126,9 +1126,9 @@ static TcPlan compute_plan(const AetherConvDesc& d) {
     pl.dw_cblocks = pl.Cin_p / UC;
     pl.dw_U = pl.taps * pl.dw_cblocks;
     const long long ptiles = pl.til_out.total();
-    auto decompose = [&](int pf) {       // pf CTAs per M group and column tile; returns the split count
+    auto decompose = [&](int pf, int max_gpc) {       // pf CTAs per M group and column tile, groups of a CTA (0: as many as TMEM holds); returns the split count
         pl.dw_MG = ceil_div(pl.dw_U, MB * pf);
-        const int max_gpc = 512 / (pl.dw_nt * pf);
+        if (max_gpc == 0) max_gpc = 512 / (pl.dw_nt * pf);
         pl.dw_ngc = ceil_div(pl.dw_MG, max_gpc);
         pl.dw_gpc = ceil_div(pl.dw_MG, pl.dw_ngc);
         pl.dw_ngc = ceil_div(pl.dw_MG, pl.dw_gpc);
@@ -1162,17 +1162,30 @@ static TcPlan compute_plan(const AetherConvDesc& d) {
         return best_splits;
     };
     // pairs: the channel counts must fill 256 rows and two column halves, and every pair needs a few pixel tiles
-    pl.dw_halo_splits = decompose(1);
+    pl.dw_halo_splits = decompose(1, 0);
     if (pl.dw_halo_splits < 1) pl.dw_halo_splits = 1;
     pl.dw_splits = pl.dw_halo_splits;
     pl.dw_pair = pl.dw_nb == 2 && pl.Cout_p % (2 * pl.dw_nt) == 0 && pl.dw_U >= 2 * MB && cta_pairs_available();
     if (pl.dw_pair) {
-        const int ps = decompose(2);
+        const int ps = decompose(2, 0);
         if (ps < 1 || ptiles < 4LL * ps) {
             pl.dw_pair = false;
-            decompose(1);
+            decompose(1, 0);
         } else {
-            pl.dw_splits = ps;
+            // M groups per CTA: a tile of pixels takes some 0.72 us for each, whether or not they share dy's half, so the count is chosen by how evenly the
+            // groups and pixels divide and by the partials (written, and read again).  One group instead of two, dW with its reduction, us: 256 x 8x8
+            // 256->256 28.8 -> 21.9, 512 x 16x16 128->256 68.7 -> 61.5, 4096 x 8x8 256->512 414 -> 376, 64 x 9x9 256->256 5x5 33 -> 28, TF32 256 x
+            // 16x16 128->128 48.2 -> 43.9.
+            const double dw_us = 2.0 * pl.dw_U * UC * pl.Cout_p * 4.0 / 4e6;        // as below
+            double best = 1e30;
+            int gpc = 0;
+            for (int g = 512 / (pl.dw_nt * 2); g >= 1; --g) {
+                const int splits = decompose(2, g);
+                if (splits < 1) continue;
+                const double cost = (double)((ptiles + splits - 1) / splits) * pl.dw_gpc * 0.72 + pl.dw_gpc + (splits > 1 ? splits * dw_us : 0.0);
+                if (cost < best - 1e-9) { best = cost; gpc = g; }
+            }
+            pl.dw_splits = decompose(2, gpc);
         }
     }
     pl.dw_small = false;
@@ -1182,7 +1195,7 @@ static TcPlan compute_plan(const AetherConvDesc& d) {
             pl.dw_splits = s;
             pl.dw_small = true;
         } else {
-            decompose(1);
+            decompose(1, 0);
         }
     }
     const long long out_rows = 1LL * d.S * pl.Ho * pl.Wo;
@@ -1521,12 +1534,12 @@ int tc_conv_bwd(const AetherConvDesc& d, const float* x, const float* dy, const 
         return dw_reduce(part, dw, splits, pl.dw_U, pl.KC, pl.Cout_p, pl.dw_cblocks, pl.taps, d.Cin, d.Cout, tap_split, splits2, dbpart,
                          db_rows, db, st);
     };
-    // Which dW kernel (bf16).  The kernels that reuse a shared-memory window across the taps win on wide images; on
-    // 16..20-pixel rows the per-tap kernel on CTA pairs is faster (a fifth of such a window is halo).  Measured on B200,
-    // 128 -> 256 channels, window kernel / pair kernel in ms: 32x32 (batch 1024) 0.518 / 0.545, 24x24 (2048) 0.556 /
-    // 0.654, 20x20 (2048) 0.474 / 0.452, 16x16 (4096) 0.597 / 0.531, 16x16 256 -> 256 (2048) 0.656 / 0.486,
-    // 12x12 (4096) 0.296 / 0.326.
-    const bool per_tap_pairs = pl.dw_pair && pl.Wo >= 16 && pl.Wo <= 20;
+    // Which dW kernel (bf16).  The kernels that reuse a shared-memory window across the taps win on wide images, but for channel counts that fill
+    // the per-tap kernel's pairs of CTAs (256 output channels; of 64 input channels every fourth group would be padding).  Measured on
+    // B200, window kernel / pair kernel in us, 80 GFLOP: 256 -> 256 channels 12x12 73 / 60, 16x16 71 / 60, 24x24 74 / 63, 32x32 70 / 60, 64x64
+    // 72 / 58; 128 -> 256 12x12 71 / 68, 16x16 70 / 69, 24x24 72 / 70, 32x32 69 / 70, 64x64 75 / 67; on single CTAs 128 -> 128 69-77 / 79-87, 192
+    // -> 192 107-121 / 113-129, 64 -> 64 106-114 / 123-144.
+    const bool per_tap_pairs = pl.dw_pair && (pl.Cin_p >= 128 || (pl.Wo >= 16 && pl.Wo <= 20));
     // Small layers take the per-tap kernel, too: the window kernels spread one strip per CTA over as many splits as there are
     // SMs, and the partials cost more than the products (128 images 16x16 32->64: 17 + 7 us against 9 + 4).
     if (dw && !pl.tf32 && !per_tap_pairs && !pl.dw_small) {   // wide images: halo-reuse kernel (every tap re-reads one shared-memory window)

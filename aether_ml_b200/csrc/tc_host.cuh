@@ -78,6 +78,26 @@ int run_rows_dw(const void* x_sh, int Cin_p, int H, int W, int S, const void* dy
 int dw_reduce(const float* part, float* dw, int splits, int U, int UC, int ldn, int cblocks, int taps, int Cin, int Cout, int tap_split,
               int splits2, const float* dbpart, int db_rows, float* db, cudaStream_t st);
 
+// Rows of a strip for the dW kernels that walk images in strips: among the heights that leave three stages in `avail` bytes (two, if there are
+// none) the one with the fewest steps of 16 pixels over an image, two more per strip for what a strip costs by itself.  stage(bh): bytes of a stage.  (The
+// highest strip instead: 16 rows in strips of 12 are a third padding; dW of 4238 x 16x16 64->64 190 us, in strips of 8 113.)
+template <typename Stage>
+static inline int pick_strip_rows(int Ho, int Wp, int avail, Stage stage, int* stages) {
+    int best = 0;
+    for (int most = 3; most >= 2 && best == 0; --most) {
+        long long best_cost = 0;
+        for (int bh = Ho < 16 ? Ho : 16; bh >= 1; --bh) {
+            const int stg = avail / stage(bh);
+            const long long cost = 1LL * ceil_div(Ho, bh) * (ceil_div(bh * Wp, 16) + 2);
+            if (stg < most || (best != 0 && cost >= best_cost)) continue;
+            best = bh;
+            best_cost = cost;
+            *stages = stg > 4 ? 4 : stg;
+        }
+    }
+    return best;
+}
+
 // MMAs (32 bytes of K each) that the last of `kchunks` 128-byte chunks needs when only k_real of the channels are not padding.
 static inline int last_ksteps(int k_real, int kchunks, int KC) {
     const int rest = k_real - (kchunks - 1) * KC, step = KC / 4;
