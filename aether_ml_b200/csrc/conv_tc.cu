@@ -156,7 +156,8 @@ struct IgemmCfg {
     // with one chunk per stage its per-stage work (barrier wait, four MMAs, two commits) is not hidden behind the MMAs; a pair's stage takes two
     static constexpr int KS = RB == 64 ? 4 : PAIR || NT <= 64 ? 2 : 1;
     static constexpr int STAGE_A_BYTES = KS * TILE_A_BYTES, STAGE_B_BYTES = KS * TILE_B_BYTES;
-    static constexpr int STAGES = RB == 64 ? (NT == 128 ? 3 : 4) : PAIR ? (NT == 256 ? 3 : 4) : ((NT == 256) ? 4 : (NT == 128 ? 6 : NT == 64 ? 4 : 5));
+    static constexpr int STAGES = RB == 64 ? (NT >= 96 ? 3 : 4) : PAIR ? (NT >= 192 ? 3 : 4) : NT == 256 ? 4 : NT == 192 ? 5 : NT == 128 ? 6 : NT == 96 ? 7 : NT == 64 ? 4 : 5;
+    static constexpr int TMEM_COLS = NT == 192 ? 512 : NT == 96 ? 256 : 2 * NT;
     static constexpr int SMEM_BYTES = 1024 + STAGES * (STAGE_A_BYTES + STAGE_B_BYTES) + IGEMM_TAIL + IGEMM_STATS_BYTES;
 };
 
@@ -213,10 +214,10 @@ __global__ void __launch_bounds__(IGEMM_THREADS, 1) igemm_conv_kernel(const __gr
     }
     if (warp == 1) {
         if (PAIR) {
-            tmem_alloc_pair(sTmemPtr, 2 * NT);
+            tmem_alloc_pair(sTmemPtr, Cfg::TMEM_COLS);
             tmem_relinquish_pair();
         } else {
-            tmem_alloc(sTmemPtr, 2 * NT);
+            tmem_alloc(sTmemPtr, Cfg::TMEM_COLS);
             tmem_relinquish();
         }
     }
@@ -521,8 +522,8 @@ __global__ void __launch_bounds__(IGEMM_THREADS, 1) igemm_conv_kernel(const __gr
     else __syncthreads();
     if (warp == 1) {
         tc_fence_after();
-        if (PAIR) tmem_dealloc_pair(tmem_base, 2 * NT);
-        else tmem_dealloc(tmem_base, 2 * NT);
+        if (PAIR) tmem_dealloc_pair(tmem_base, Cfg::TMEM_COLS);
+        else tmem_dealloc(tmem_base, Cfg::TMEM_COLS);
     }
 }
 
@@ -1253,16 +1254,6 @@ bool tc_conv_operand_layout(const AetherConvDesc& d, AetherOperandLayout* out) {
     return true;
 }
 
-// Column tile: the widest that divides the padded output channels (fewest reads of the pixel operand), halved while there
-// are tiles for less than half of the SMs: with few tiles a CTA waits for its own stream of operands out of L2 (some 145
-// GB/s per SM), and narrower tiles split the filter's part of that over idle SMs (128 rows of a
-// Dense layer 2048 -> 256: 15.7 -> 12.3 us; 64 images 7x7 128 -> 256: 12.0 -> 9.2 us).
-static int pick_nt(int n_padded, long long m_tiles) {
-    int nt = n_padded % 256 == 0 ? 256 : n_padded % 128 == 0 ? 128 : n_padded % 64 == 0 ? 64 : 32;
-    while (nt > 32 && m_tiles * (n_padded / nt) * 2 <= num_sms()) nt /= 2;
-    return nt;
-}
-
 // CTAs of the per-tap kernel.  With statistics the grid is a multiple of the number of column tiles, so that a
 // CTA (tiles blockIdx.x + k * grid, column tile = tile % n_tiles_n) keeps one column tile throughout.
 static int igemm_grid(long long m_tiles, int n_tiles_n, bool stats) {
@@ -1279,13 +1270,34 @@ static int igemm_grid(long long m_tiles, int n_tiles_n, bool stats) {
 // has 256 tensor clocks per stage for a barrier wait, four MMAs and two commits; two chunks per stage fixed that
 // and also gave the 256-column pair 3-4 %.
 static bool igemm_use_pairs(long long m_tiles, int nt, int n_tiles_n) {
-    return (nt == 256 || nt == 128) && (m_tiles + 1) / 2 * n_tiles_n >= 2LL * (num_sms() / 2) && cta_pairs_available();
+    return (nt == 256 || nt == 192 || nt == 128) && (m_tiles + 1) / 2 * n_tiles_n >= 2LL * (num_sms() / 2) && cta_pairs_available();
 }
 static int igemm_pair_grid(long long m_tiles, int n_tiles_n, bool stats) {
     const long long units = (m_tiles + 1) / 2 * n_tiles_n;
     int pairs = (int)(units < num_sms() / 2 ? units : num_sms() / 2);
     if (stats && pairs > n_tiles_n) pairs -= pairs % n_tiles_n;
     return 2 * pairs;
+}
+
+// Column tile: the one whose rounds of units are through first.  What a 128-byte chunk of K takes, in clocks, is its operands' way from L2 (128 rows of
+// pixels, some 63 bytes per clock and SM) and the filter rows'; a tile that overhangs the channels costs what it copies, several tiles copy the pixels again.
+// (Only widths that divide the channels made 192 channels three tiles of 64 and TF32's 160 five of 32.  Before / now, us: bf16 256 x 8x8 256->192 forward
+// 22.0 / 13.6, 192->160 17.6 / 11.2, 100 x 11x11 192->256 dX 21.4 / 13.2; TF32 150 x 16x16 160->96 forward and dX 54 / 29, 53 / 27, 100 x 12x12 224->180
+// dX 85 / 38.  Few tiles are narrow: 128 rows of a Dense layer 2048 -> 256 15.7 in one tile, 12.3 in eight; 64 images 7x7 128 -> 256 12.0 / 9.2.)
+static int pick_nt(int n_padded, long long m_tiles, int kiters) {
+    static const int widths[6] = {256, 192, 128, 96, 64, 32};
+    int best = 32;
+    double best_cost = 1e300;
+    for (int nt : widths) {
+        const int cols = ceil_div(n_padded, nt);
+        if (cols > 1 && nt > 128 && n_padded % nt) continue;          // (a filter tile reads on into the next tap's rows, a wide one by much)
+        const bool pair = igemm_use_pairs(m_tiles, nt, cols);
+        const long long units = pair ? (m_tiles + 1) / 2 * cols : m_tiles * cols, slots = pair ? num_sms() / 2 : num_sms();
+        const double chunk = 260.0 + (pair ? 1.0 : 2.0) * nt;
+        const double cost = (double)((units + slots - 1) / slots) * kiters * chunk + 8.0 * nt;
+        if (cost < best_cost - 1e-9) { best_cost = cost; best = nt; }
+    }
+    return best;
 }
 
 template <bool TF32, int NT, bool STATS, bool PAIR, bool ACT = false, int RB = 128>
@@ -1314,7 +1326,7 @@ static int launch_igemm(const IgemmParams& p, bool pair, bool narrow, cudaStream
     if constexpr (!TF32 && NT <= 128) {
         if (narrow) return p.stats ? launch_igemm_k<false, NT, true, false, false, 64>(p, st) : launch_igemm_k<false, NT, false, false, false, 64>(p, st);
     }
-    if constexpr (NT == 256 || NT == 128) {
+    if constexpr (NT == 256 || NT == 192 || NT == 128) {
         if (pair) return p.stats ? launch_igemm_k<TF32, NT, true, true>(p, st) : launch_igemm_k<TF32, NT, false, true>(p, st);
     }
     if constexpr (!TF32) {
@@ -1327,7 +1339,9 @@ template <bool TF32>
 static int dispatch_igemm(IgemmParams& p, int nt, bool pair, bool narrow, cudaStream_t st) {
     switch (nt) {
         case 256: return launch_igemm<TF32, 256>(p, pair, narrow, st);
+        case 192: return launch_igemm<TF32, 192>(p, pair, narrow, st);
         case 128: return launch_igemm<TF32, 128>(p, pair, narrow, st);
+        case 96: return launch_igemm<TF32, 96>(p, false, narrow, st);
         case 64: return launch_igemm<TF32, 64>(p, false, narrow, st);
         default: return launch_igemm<TF32, 32>(p, false, narrow, st);
     }
@@ -1351,7 +1365,7 @@ static int run_igemm(bool tf32, const void* in, int in_C, int in_H, int in_W, in
     memset(&p, 0, sizeof(p));
     const int elt = tf32 ? 4 : 2;
     const CUtensorMapDataType dt = tf32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
-    const int nt = pick_nt(n_padded, til.total());
+    const int nt = pick_nt(n_padded, til.total(), taps * ceil_div(in_C, 128 / elt));
     const bool pair = igemm_use_pairs(til.total(), nt, ceil_div(n_padded, nt));   // each CTA of a pair stages half the filter rows
     const bool narrow = !tf32 && !pair && k_real <= 32 && nt <= 128 && (act == nullptr || stats != nullptr);
     const int KC = narrow ? 32 : 128 / elt;
@@ -1408,7 +1422,7 @@ long long tc_conv_stats_blocks(const AetherConvDesc& d) {
                                                  halo_n(d.Cout, pl.Cout_p), d.fH, d.fW);
     if (hb > 0) return hb;
     // per-tap kernel: two rows per CTA group (the CTAs of one set of pixel tiles)
-    const int nt = pick_nt(pl.Cout_p, pl.til_out.total());
+    const int nt = pick_nt(pl.Cout_p, pl.til_out.total(), pl.taps * ceil_div(pl.tf32 ? d.Cin : pl.Cin_p, pl.KC));
     const int n_tiles_n = ceil_div(pl.Cout_p, nt);
     if (igemm_use_pairs(pl.til_out.total(), nt, n_tiles_n)) {       // one block group per CTA of a pair
         const int pairs = igemm_pair_grid(pl.til_out.total(), n_tiles_n, true) / 2;
