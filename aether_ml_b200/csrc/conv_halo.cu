@@ -425,9 +425,14 @@ static bool halo_geometry(bool tf32, int in_C, int S, int taps, int out_C, int o
     if (g.BH + fH - 1 > 256) return false;
     g.tiles_h = ceil_div(out_H, g.BH);
     if (1LL * g.tiles_h * S > 0x3fffffffLL) return false;
-    // useful fraction of the 128 accumulator rows, including the ragged last strip of each image
+    // Useful fraction of the 128 accumulator rows, including the ragged last strip of each image, that makes up for the per-tap kernel's copies: less of
+    // it where those weigh more (few columns; TF32 of one chunk of channels).  Per-tap / this kernel, us at 40 GFLOP: bf16 64->64 15x15 (0.59) 78 / 70,
+    // 13x13 (0.66) 77 / 62, 16x16 (0.67) 75 / 61, 31x31 (0.68) 75 / 65, 44x44 (0.69) 79 / 65, 64->128 16x16 55 / 51, 44x44 59 / 52, but 12x12 (0.56) 51 / 55;
+    // 64->192 13x13 11.5 / 15.8 (6 GFLOP), 19x19 (0.71) 11.5 / 15.8, 26x26 (0.75) 52 / 55, 28x28 (0.88) 55 / 47; TF32 32->64 13x13 147 / 116, 16x16 144 /
+    // 119, 64->64 44x44 129 / 113, 64->128 16x16 17.0 / 18.2 (6 GFLOP).
     const double eff = (double)out_H * out_W / ((double)g.tiles_h * 128.0);
-    if (eff < 0.70) return false;
+    const double least = tf32 ? (in_C <= 32 ? 0.58 : n_padded <= 64 ? 0.66 : 0.70) : n_padded <= 128 ? 0.58 : 0.72;
+    if (eff < least) return false;
     g.kchunks = ceil_div(in_C, KC);
     g.region_rows = (g.BH + fH - 1) * g.Wp;
     g.region_stride = (int)align_up((size_t)g.region_rows * 128, 1024);
