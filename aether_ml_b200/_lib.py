@@ -89,6 +89,8 @@ SIGNATURES = {
     "aether_pool_bwd": (_I, [_P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _I, _P]),
     "aether_leaky_relu_fwd": (_I, [_P, _P, _I64, _F, _P]),
     "aether_leaky_relu_bwd": (_I, [_P, _P, _P, _I64, _F, _P]),
+    "aether_leaky_relu_fwd_mask": (_I, [_P, _P, _P, _I64, _F, _P]),
+    "aether_leaky_relu_bwd_mask": (_I, [_P, _P, _P, _I64, _F, _P]),
     "aether_channel_scale": (_I, [_P, _P, _P, _I64, _I, _P]),
     "aether_dropout_fwd": (_I, [_P, _P, _P, _I64, _F, _U64, _U64, _P]),
     "aether_copy": (_I, [_P, _P, _I64, _P]),

@@ -139,7 +139,7 @@ struct Entry<int (*)(A...)> {
     X(aether_conv2d_fwd_ex) X(aether_conv2d_bwd_ex) X(aether_conv2d_filter_copies) X(aether_bn_fwd_train) X(aether_bn_fwd_train_partials)             \
     X(aether_bn_fwd_eval) X(aether_bn_bwd) X(aether_bn_act_fwd_train) X(aether_bn_act_fwd_eval) X(aether_bn_act_bwd)   \
     X(aether_bn_act_pool_fwd_copy) X(aether_chain_fwd) X(aether_pool_fwd) X(aether_pool_bwd) X(aether_leaky_relu_fwd)                      \
-    X(aether_leaky_relu_bwd) X(aether_channel_scale) X(aether_dropout_fwd) X(aether_mul) X(aether_adam_step)           \
+    X(aether_leaky_relu_bwd) X(aether_leaky_relu_fwd_mask) X(aether_leaky_relu_bwd_mask) X(aether_channel_scale) X(aether_dropout_fwd) X(aether_mul) X(aether_adam_step)           \
     X(aether_adam_step_dev) X(aether_dropout_fwd_dev) X(aether_channel_mask_dev) X(aether_regularizer_grad)            \
     X(aether_regularizer_loss) X(aether_copy) X(aether_conv2d_act_fwd) X(aether_act_bwd_copy) X(aether_head_softmax_fwd) X(aether_head_cce_bwd_ex) X(aether_softmax_cce) X(aether_softmax_cce_i64) X(aether_softmax_bwd) X(aether_softmax_cce_targets)
 

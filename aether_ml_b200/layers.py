@@ -598,6 +598,10 @@ class ReLU(_Saved):
     Batch_Norm's kernels and this layer only hands tensors through."""
     _alpha = 0.0
     fused_into_prev = False
+    # From this many values on a training pass keeps a bit of each for the way back, which then need not read the inputs again:
+    # arrays of 16 MB, several of which L2 does not hold (256 x 32x32x64, the layer alone, us: 42 -> 35).
+    MASK_FROM = 1 << 22
+    _mask = None                # (bits, the inputs they are of, their version)
 
     def forward(self, inputs, training):
         x = to_device(inputs)
@@ -606,7 +610,14 @@ class ReLU(_Saved):
             return self.output
         h = host()
         y = h.empty_like(x)
-        h.aether_leaky_relu_fwd(x, y, x.numel(), self._alpha)
+        n = x.numel()
+        if training and n >= self.MASK_FROM and n % 4 == 0:
+            bits = h.empty_u8(((n + 127) // 128 * 16,))
+            h.aether_leaky_relu_fwd_mask(x, y, bits, n, self._alpha)
+            self._mask = (bits, weakref.ref(x), x._version)
+        else:
+            self._mask = None
+            h.aether_leaky_relu_fwd(x, y, n, self._alpha)
         self.inputs = x
         self.output = y
         return self.output
@@ -618,7 +629,11 @@ class ReLU(_Saved):
             return self.dinputs
         h = host()
         dx = h.empty_like(dy)
-        h.aether_leaky_relu_bwd(self.inputs, dy, dx, dy.numel(), self._alpha)
+        x, mask = self.inputs, self._mask
+        if mask is not None and mask[1]() is x and mask[2] == x._version and dy.numel() == x.numel():
+            h.aether_leaky_relu_bwd_mask(mask[0], dy, dx, dy.numel(), self._alpha)
+        else:
+            h.aether_leaky_relu_bwd(x, dy, dx, dy.numel(), self._alpha)
         self.dinputs = dx
         return self.dinputs
 

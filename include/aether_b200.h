@@ -317,6 +317,10 @@ int aether_pool_bwd(const float* dy, const uint8_t* argmax, float* dx, int S, in
 int aether_leaky_relu_fwd(const float* x, float* y, int64_t n, float alpha, void* stream);
 /* dx = dy where x >= 0, alpha*dy where x < 0. */
 int aether_leaky_relu_bwd(const float* x, const float* dy, float* dx, int64_t n, float alpha, void* stream);
+/* The same by way of a bit per value, x < 0 (n a multiple of 4): mask holds 16 bytes for every 128 values begun, 16-byte aligned, in an
+ * order that only these two know.  Going back, dy and dx are read and written and n / 8 bytes of mask instead of x. */
+int aether_leaky_relu_fwd_mask(const float* x, float* y, void* mask, int64_t n, float alpha, void* stream);
+int aether_leaky_relu_bwd_mask(const void* mask, const float* dy, float* dx, int64_t n, float alpha, void* stream);
 
 /* ---- Layer_Dropout_Spatial :384-404: y = x * scale[c], scale = channel mask / keep_prob (C floats);
  *      the same call with dy gives the backward. */
