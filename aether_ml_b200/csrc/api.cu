@@ -241,6 +241,33 @@ extern "C" int aether_conv2d_filter_copies(const AetherConvDesc* d, const float*
     return tc_conv_filter_copies(*d, w, ws, ws_bytes, static_cast<cudaStream_t>(stream));
 }
 
+extern "C" int aether_conv2d_pool_supported(const AetherConvDesc* d) {
+    if (validate_desc(d, "aether_conv2d_pool_supported")) return 0;
+    int Ho, Wo;
+    conv_out_hw(*d, Ho, Wo);
+    return tc_conv_pool_eligible(*d) || (!tc_conv_eligible(*d) && first_tc_eligible(*d) && Ho % 2 == 0 && Wo % 2 == 0);
+}
+
+extern "C" int aether_conv2d_pool_fwd(const AetherConvDesc* d, const float* x, const float* w, const float* b, const float* gamma, const float* beta,
+                                      const float* running_mean, const float* running_var, float eps, float alpha, float* pooled, void* operand_copy,
+                                      int copy_ld, void* ws, size_t ws_bytes, int flags, void* stream) {
+    int rc = validate_desc(d, "aether_conv2d_pool_fwd");
+    if (rc) return rc;
+    if (!x || !w || !gamma || !beta || !running_mean || !running_var || !pooled) return set_error(AE_BAD_ARG, "aether_conv2d_pool_fwd: null pointer");
+    if (!aligned16(x) || !aligned16(w) || !aligned16(pooled) || (ws && !aligned16(ws))) return set_error(AE_BAD_ARG, "aether_conv2d_pool_fwd: arrays must be 16-byte aligned");
+    if (!(alpha >= 0.f && alpha < 1.f)) return set_error(AE_BAD_ARG, "aether_conv2d_pool_fwd: alpha must be in [0, 1)");
+    if (operand_copy && (copy_ld < d->Cout || copy_ld % 4 || (reinterpret_cast<uintptr_t>(operand_copy) & 7)))
+        return set_error(AE_BAD_ARG, "aether_conv2d_pool_fwd: operand copy needs ld >= Cout, ld %% 4 == 0, 8-byte alignment");
+    if (flags & ~(AETHER_CONV_X_COPY_READY | AETHER_CONV_W_COPY_READY)) return set_error(AE_BAD_ARG, "aether_conv2d_pool_fwd: unknown flag bits 0x%x", flags);
+    const bool tc = tc_conv_eligible(*d);
+    if (!aether_conv2d_pool_supported(d) || (operand_copy && copy_ld > (d->Cout + 63) / 64 * 64) || (!tc && (flags & AETHER_CONV_X_COPY_READY)))
+        return set_error(AE_UNSUPPORTED, "aether_conv2d_pool_fwd: not a shape for it (aether_conv2d_pool_supported), rows of the copy longer than the padded channels, or no copy of x");
+    if ((rc = pending_timeout("aether_conv2d_pool_fwd"))) return rc;
+    const PoolEpilogue e = {gamma, beta, running_mean, running_var, eps, alpha, pooled, operand_copy, operand_copy ? copy_ld : 0};
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    return tc ? tc_conv_fwd_pool(*d, x, w, b, e, ws, ws_bytes, flags, st) : first_tc_fwd(*d, x, w, b, nullptr, nullptr, st, &e);
+}
+
 extern "C" int aether_conv2d_act_fwd(const AetherConvDesc* d, const float* x, const float* w, const float* b, float* y, float* act_out,
                                      float alpha, void* act_copy, int copy_ld, void* ws, size_t ws_bytes, int flags, void* stream) {
     int rc = validate_desc(d, "aether_conv2d_act_fwd");

@@ -106,11 +106,20 @@ long long smallc_conv_stats_blocks(const AetherConvDesc& d);
 int smallc_conv_bwd_filter(const AetherConvDesc& d, const float* x, const float* dy, float* dw, float* db, void* ws,
                            size_t ws_bytes, cudaStream_t st);
 
+// The layers behind a convolution that its kernels may apply in inference (pool_epilogue.cuh): Batch_Norm, (leaky) ReLU, 2x2 max pooling.
+struct PoolEpilogue {
+    const float *gamma, *beta, *mean, *var;
+    float eps, alpha;
+    float* pooled;
+    void* copy;          // nullable: bf16, rows of ld
+    int ld;
+};
+
 // ---- conv_first_tc.cu : first-layer forward on tensor cores (bf16 mode, thread-built im2col operand)
 bool first_tc_eligible(const AetherConvDesc& d);
 long long first_tc_stats_blocks(const AetherConvDesc& d);
 int first_tc_fwd(const AetherConvDesc& d, const float* x, const float* w, const float* b, float* y, float* stats,
-                 cudaStream_t st);
+                 cudaStream_t st, const PoolEpilogue* pool = nullptr);
 bool first_tc_bwd_eligible(const AetherConvDesc& d);
 int first_tc_bwd_filter(const AetherConvDesc& d, const float* x, const float* dy, float* dw, float* db, void* ws,
                         size_t ws_bytes, int dy_colsum_rows, cudaStream_t st);
@@ -135,6 +144,9 @@ struct ActEpilogue {
 };
 int tc_conv_fwd(const AetherConvDesc& d, const float* x, const float* w, const float* b, float* y, float* stats, void* ws,
                 size_t ws_bytes, int flags, cudaStream_t st, const ActEpilogue* act = nullptr, bool* act_done = nullptr);
+bool tc_conv_pool_eligible(const AetherConvDesc& d);
+int tc_conv_fwd_pool(const AetherConvDesc& d, const float* x, const float* w, const float* b, const PoolEpilogue& pool, void* ws, size_t ws_bytes, int flags,
+                     cudaStream_t st);
 int tc_conv_filter_copies(const AetherConvDesc& d, const float* w, void* ws, size_t ws_bytes, cudaStream_t st);
 bool tc_conv_operand_layout(const AetherConvDesc& d, AetherOperandLayout* out);
 long long tc_conv_stats_blocks(const AetherConvDesc& d);

@@ -20,6 +20,7 @@
 #include "common.cuh"
 #include "finish_columns.cuh"
 #include "sm100_ptx.cuh"
+#include "pool_epilogue.cuh"
 #include "stats_epilogue.cuh"
 #include "store_block.cuh"
 #include "tc_host.cuh"
@@ -134,6 +135,7 @@ struct IgemmParams {
     int kchunks;
     int last_ksteps;     // MMAs that the last K chunk of a tap needs
     ActEpilogue act;     // ACT only
+    PoolEpilogue pool;   // POOLED only
 };
 
 static constexpr int TILE_A_BYTES = 128 * 128;  // 128 pixel rows x 128 B
@@ -142,6 +144,8 @@ static constexpr int IGEMM_EPI_UB = 4;          // 16-column TMEM loads in fligh
 static constexpr int IGEMM_THREADS = 64 + 32 * IGEMM_EPI_WARPS;   // warp 0 TMA producer, warp 1 MMA issuer, then epilogue
 static constexpr int IGEMM_TAIL = 1024;         // barriers, TMEM pointer
 static constexpr int IGEMM_STATS_BYTES = IGEMM_EPI_WARPS * STATS_WARP_FLOATS * 4;   // per-warp running column sums and pivots
+static constexpr int IGEMM_POOL_CHANNELS = 1024;                                    // most output channels of POOLED, whose coefficients lie there
+static_assert(2 * IGEMM_POOL_CHANNELS * 4 <= IGEMM_STATS_BYTES, "coefficients");
 
 // PAIR: two CTAs of a cluster share one 256-row MMA (cta_group::2).  Each holds its own 128 pixel rows and HALF of the
 // filter tile (NT/2 rows), so a stage is smaller and every SM pulls a third less from L2 per FLOP.
@@ -174,7 +178,11 @@ struct IgemmCfg {
 // ACT: the epilogue also writes the (leaky) ReLU of the output and, when asked, the bf16 operand copy of that for the layer
 // behind (zero in the padded columns): a Dense layer and its activation of a small network are two launches of two
 // microseconds otherwise, three with the cast.
-template <bool TF32, int NT, bool STATS, bool PAIR, bool ACT = false, int RB = 128>
+//
+// POOLED (inference): Batch_Norm by its running statistics, (leaky) ReLU and 2x2 max pooling in the epilogue, which writes the pooled values and
+// their bf16 operand copy only.  Boxes are 8 or 16 pixels wide and an even number of rows high, so that the two rows of a window are 8 or 16 accumulator
+// rows apart, in one thread, and its columns in neighbouring ones (lane ^ 4).  (896 x 16x16 32->64 30.8 us, 27.6 and 19.6 apart; 8x8 64->128 20.4, 17.9 and 12.)
+template <bool TF32, int NT, bool STATS, bool PAIR, bool ACT = false, int RB = 128, bool POOLED = false>
 __global__ void __launch_bounds__(IGEMM_THREADS, 1) igemm_conv_kernel(const __grid_constant__ IgemmParams p) {
     using Cfg = IgemmCfg<NT, PAIR, RB>;
     constexpr int STAGES = Cfg::STAGES, TILE_A_BYTES = Cfg::TILE_A_BYTES;
@@ -222,6 +230,9 @@ __global__ void __launch_bounds__(IGEMM_THREADS, 1) igemm_conv_kernel(const __gr
         }
     }
     pdl_wait();                       // set-up done; from here on global memory is touched
+    float* scale_s = reinterpret_cast<float*>(gen_base + (sBar - smem_base) + IGEMM_TAIL);      // POOLED: scale and shift of all channels
+    if (POOLED)
+        for (int i = threadIdx.x; i < p.n_out; i += IGEMM_THREADS) pool_coefficients(p.pool, i, p.n_out, scale_s[i], scale_s[IGEMM_POOL_CHANNELS + i]);
     tc_fence_before();
     if (PAIR) cluster_sync_all();     // the other CTA's barriers exist before anything is sent to them
     else __syncthreads();
@@ -388,6 +399,11 @@ __global__ void __launch_bounds__(IGEMM_THREADS, 1) igemm_conv_kernel(const __gr
                 rowp[j] = (w < p.out_W && h < p.out_H && n < p.out_N) ? p.out + at * p.n_out + col0 : nullptr;
                 if (ACT) pix[ACT ? j : 0] = at;
             }
+            long long window = -1;                 // POOLED: the window that this lane finishes
+            if (POOLED) {
+                const int j = (trow & 1) == 0 ? 0 : p.BW == 16 ? 1 : 2;
+                if (rowp[j] != nullptr) window = ((long long)(n0 + r_n[j]) * (p.out_H >> 1) + ((h0 + r_h[j]) >> 1)) * (p.out_W >> 1) + ((w0 + r_w[j]) >> 1);
+            }
             float tile_rows = 0.f;                 // valid rows of this tile in this warp's quarter
             if (STATS) {
 #pragma unroll
@@ -436,6 +452,11 @@ __global__ void __launch_bounds__(IGEMM_THREADS, 1) igemm_conv_kernel(const __gr
                         }
                         float4 pv = make_float4(0.f, 0.f, 0.f, 0.f);      // pivot of this lane's four columns
                         if (STATS) pv = *reinterpret_cast<const float4*>(stat_w + 256 + cc + tcol4);
+                        float4 act4[POOLED ? 4 : 1], s4 = pv, t4 = pv;
+                        if (POOLED && cols_ok) {
+                            s4 = *reinterpret_cast<const float4*>(scale_s + col0 + cc);
+                            t4 = *reinterpret_cast<const float4*>(scale_s + IGEMM_POOL_CHANNELS + col0 + cc);
+                        }
 #pragma unroll
                         for (int j = 0; j < 4; ++j) {
                             const uint32_t a0 = v[j >> 1][u][(j & 1) * 2 + 0], a1 = v[j >> 1][u][(j & 1) * 2 + 1];
@@ -453,6 +474,10 @@ __global__ void __launch_bounds__(IGEMM_THREADS, 1) igemm_conv_kernel(const __gr
                             a.y = __uint_as_float(odd ? g1 : e1);
                             a.z = __uint_as_float(odd ? f0 : g0);
                             a.w = __uint_as_float(odd ? f1 : g1);
+                            if (POOLED) {
+                                act4[POOLED ? j : 0] = pool_activation(make_float4(a.x + b4.x, a.y + b4.y, a.z + b4.z, a.w + b4.w), s4, t4, p.pool.alpha);
+                                continue;
+                            }
                             const bool wr = cols_ok && rowp[j] != nullptr;
                             if (ACT && rowp[j] != nullptr) {
                                 const int col = col0 + cc;
@@ -477,6 +502,19 @@ __global__ void __launch_bounds__(IGEMM_THREADS, 1) igemm_conv_kernel(const __gr
                                 st_q[u].x = fmaf(a.x, a.x, st_q[u].x); st_q[u].y = fmaf(a.y, a.y, st_q[u].y);
                                 st_q[u].z = fmaf(a.z, a.z, st_q[u].z); st_q[u].w = fmaf(a.w, a.w, st_q[u].w);
                             }
+                        }
+                        if constexpr (POOLED) {
+                            // two windows of two rows here, their other column in lane ^ 4: a lane of an even column finishes the first, of an odd one the second
+                            const bool wide = p.BW == 16, right = (trow & 1) != 0;
+                            const float4 a_top = act4[0], a_low = wide ? act4[2] : act4[1], b_top = wide ? act4[1] : act4[2], b_low = act4[3];
+                            const float4 top = right ? b_top : a_top, low = right ? b_low : a_low, s_top = right ? a_top : b_top, s_low = right ? a_low : b_low;
+                            auto other = [](float4 v) {
+                                return make_float4(__shfl_xor_sync(0xffffffffu, v.x, 4), __shfl_xor_sync(0xffffffffu, v.y, 4), __shfl_xor_sync(0xffffffffu, v.z, 4),
+                                                   __shfl_xor_sync(0xffffffffu, v.w, 4));
+                            };
+                            const float4 o_top = other(s_top), o_low = other(s_low);
+                            const float4 best = right ? pool_first_max(o_top, top, o_low, low) : pool_first_max(top, o_top, low, o_low);
+                            if (window >= 0) pool_store(p.pool, window, col0 + cc, p.n_out, best);
                         }
                     }
                 }
@@ -1284,14 +1322,14 @@ static int igemm_pair_grid(long long m_tiles, int n_tiles_n, bool stats) {
 // (Only widths that divide the channels made 192 channels three tiles of 64 and TF32's 160 five of 32.  Before / now, us: bf16 256 x 8x8 256->192 forward
 // 22.0 / 13.6, 192->160 17.6 / 11.2, 100 x 11x11 192->256 dX 21.4 / 13.2; TF32 150 x 16x16 160->96 forward and dX 54 / 29, 53 / 27, 100 x 12x12 224->180
 // dX 85 / 38.  Few tiles are narrow: 128 rows of a Dense layer 2048 -> 256 15.7 in one tile, 12.3 in eight; 64 images 7x7 128 -> 256 12.0 / 9.2.)
-static int pick_nt(int n_padded, long long m_tiles, int kiters) {
+static int pick_nt(int n_padded, long long m_tiles, int kiters, bool pairs = true) {
     static const int widths[6] = {256, 192, 128, 96, 64, 32};
     int best = 32;
     double best_cost = 1e300;
     for (int nt : widths) {
         const int cols = ceil_div(n_padded, nt);
         if (cols > 1 && nt > 128 && n_padded % nt) continue;          // (a filter tile reads on into the next tap's rows, a wide one by much)
-        const bool pair = igemm_use_pairs(m_tiles, nt, cols);
+        const bool pair = pairs && igemm_use_pairs(m_tiles, nt, cols);
         const long long units = pair ? (m_tiles + 1) / 2 * cols : m_tiles * cols, slots = pair ? num_sms() / 2 : num_sms();
         const double chunk = 260.0 + (pair ? 1.0 : 2.0) * nt;
         const double cost = (double)((units + slots - 1) / slots) * kiters * chunk + 8.0 * nt;
@@ -1300,11 +1338,12 @@ static int pick_nt(int n_padded, long long m_tiles, int kiters) {
     return best;
 }
 
-template <bool TF32, int NT, bool STATS, bool PAIR, bool ACT = false, int RB = 128>
+template <bool TF32, int NT, bool STATS, bool PAIR, bool ACT = false, int RB = 128, bool POOLED = false>
 static int launch_igemm_k(const IgemmParams& p, cudaStream_t st) {
     using Cfg = IgemmCfg<NT, PAIR, RB>;
     static PerDeviceSmem configured;
-    if (int rc = ensure_dynamic_smem(igemm_conv_kernel<TF32, NT, STATS, PAIR, ACT, RB>, Cfg::SMEM_BYTES, configured, "igemm_conv")) return rc;
+    const auto kernel = igemm_conv_kernel<TF32, NT, STATS, PAIR, ACT, RB, POOLED>;
+    if (int rc = ensure_dynamic_smem(kernel, Cfg::SMEM_BYTES, configured, "igemm_conv")) return rc;
     const long long m_tiles = 1LL * p.tiles_w * p.tiles_h * p.tiles_n;
     const int grid = PAIR ? igemm_pair_grid(m_tiles, p.n_tiles_n, STATS) : igemm_grid(m_tiles, p.n_tiles_n, STATS);
     if (STATS && (grid / (PAIR ? 2 : 1)) % p.n_tiles_n)
@@ -1312,9 +1351,9 @@ static int launch_igemm_k(const IgemmParams& p, cudaStream_t st) {
     const int pk = p.sgn > 0 ? PK_IGEMM_FWD : PK_IGEMM_DX;
     prof_begin(pk, st);
     if (PAIR) {
-        launch_cluster(igemm_conv_kernel<TF32, NT, STATS, PAIR, ACT, RB>, 2, grid, IGEMM_THREADS, Cfg::SMEM_BYTES, st, p);
+        launch_cluster(kernel, 2, grid, IGEMM_THREADS, Cfg::SMEM_BYTES, st, p);
     } else {
-        launch(igemm_conv_kernel<TF32, NT, STATS, PAIR, ACT, RB>, grid, IGEMM_THREADS, Cfg::SMEM_BYTES, st, p);
+        launch(kernel, grid, IGEMM_THREADS, Cfg::SMEM_BYTES, st, p);
     }
     prof_end(pk, st);
     count_launch();
@@ -1347,12 +1386,20 @@ static int dispatch_igemm(IgemmParams& p, int nt, bool pair, bool narrow, cudaSt
     }
 }
 
+template <int NT>
+static int launch_igemm_pooled(const IgemmParams& p, bool narrow, cudaStream_t st) {
+    if constexpr (NT <= 128) {
+        if (narrow) return launch_igemm_k<false, NT, false, false, false, 64, true>(p, st);
+    }
+    return launch_igemm_k<false, NT, false, false, false, 128, true>(p, st);
+}
+
 // Runs out[p, n] = sum_{tap,k} in[p (+/-) tap, k] * Wm[tap][n][k] (+ bias).
 static int run_igemm(bool tf32, const void* in, int in_C, int in_H, int in_W, int S, const void* wmat, int w_inner,
                      int rows_per_tap, int taps, float* out, int out_C, int out_H, int out_W, const PixelTiling& til,
                      int n_padded, int fH, int fW, int sgn, int off_h, int off_w, int k_real, const float* bias, float* stats,
-                     cudaStream_t st, const ActEpilogue* act = nullptr, bool* act_done = nullptr) {
-    {   // wide images with a filter that fits in shared memory: halo-reuse kernel
+                     cudaStream_t st, const ActEpilogue* act = nullptr, bool* act_done = nullptr, const PoolEpilogue* pool = nullptr) {
+    if (pool == nullptr) {   // wide images with a filter that fits in shared memory: halo-reuse kernel
         bool used = false;
         const int padT = sgn > 0 ? -off_h : fH - 1 - off_h;
         const int padL = sgn > 0 ? -off_w : fW - 1 - off_w;
@@ -1365,8 +1412,8 @@ static int run_igemm(bool tf32, const void* in, int in_C, int in_H, int in_W, in
     memset(&p, 0, sizeof(p));
     const int elt = tf32 ? 4 : 2;
     const CUtensorMapDataType dt = tf32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
-    const int nt = pick_nt(n_padded, til.total(), taps * ceil_div(in_C, 128 / elt));
-    const bool pair = igemm_use_pairs(til.total(), nt, ceil_div(n_padded, nt));   // each CTA of a pair stages half the filter rows
+    const int nt = pick_nt(n_padded, til.total(), taps * ceil_div(in_C, 128 / elt), pool == nullptr);
+    const bool pair = pool == nullptr && igemm_use_pairs(til.total(), nt, ceil_div(n_padded, nt));   // each CTA of a pair stages half the filter rows
     const bool narrow = !tf32 && !pair && k_real <= 32 && nt <= 128 && (act == nullptr || stats != nullptr);
     const int KC = narrow ? 32 : 128 / elt;
     const CUtensorMapSwizzle swz = narrow ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B;
@@ -1392,6 +1439,17 @@ static int run_igemm(bool tf32, const void* in, int in_C, int in_H, int in_W, in
     p.fH = fH; p.fW = fW; p.sgn = sgn; p.off_h = off_h; p.off_w = off_w;
     p.kchunks = narrow ? 1 : ceil_div(in_C, KC);
     p.last_ksteps = narrow ? ceil_div(k_real, 16) : last_ksteps(k_real, p.kchunks, KC);
+    if (pool != nullptr) {
+        p.pool = *pool;
+        switch (nt) {
+            case 256: return launch_igemm_pooled<256>(p, narrow, st);
+            case 192: return launch_igemm_pooled<192>(p, narrow, st);
+            case 128: return launch_igemm_pooled<128>(p, narrow, st);
+            case 96: return launch_igemm_pooled<96>(p, narrow, st);
+            case 64: return launch_igemm_pooled<64>(p, narrow, st);
+            default: return launch_igemm_pooled<32>(p, narrow, st);
+        }
+    }
     return tf32 ? dispatch_igemm<true>(p, nt, pair, false, st) : dispatch_igemm<false>(p, nt, pair, narrow, st);
 }
 
@@ -1483,6 +1541,41 @@ static int launch_dw(const DwParams& p, int splits, int grid_y, cudaStream_t st)
     prof_end(PK_DW, st);
     count_launch();
     return check_launch("dw_conv_kernel");
+}
+
+// Boxes of 2x2 windows: 8 or 16 pixels wide, an even number of rows high, several images once a box is as high as one.
+static PixelTiling choose_pool_tiling(int S, int H, int W) {
+    PixelTiling best{};
+    long long best_tiles = -1;
+    for (int bw = 16; bw >= 8; bw -= 8)
+        for (int bh = 2; bh <= H && bw * bh <= 128; bh += 2) {
+            int bn = bh < H ? 1 : 128 / (bw * bh);
+            if (bn > S) bn = S;
+            const long long t = 1LL * ceil_div(W, bw) * ceil_div(H, bh) * ceil_div(S, bn);
+            if (best_tiles < 0 || t < best_tiles) {
+                best_tiles = t;
+                best = PixelTiling{bw, bh, bn, bw * bh * bn, ceil_div(W, bw), ceil_div(H, bh), ceil_div(S, bn)};
+            }
+        }
+    return best;
+}
+bool tc_conv_pool_eligible(const AetherConvDesc& d) {
+    int Ho, Wo;
+    conv_out_hw(d, Ho, Wo);
+    return tc_conv_eligible(d) && d.math_mode == AETHER_MATH_BF16 && Ho % 2 == 0 && Wo % 2 == 0 && d.Cout <= IGEMM_POOL_CHANNELS;
+}
+int tc_conv_fwd_pool(const AetherConvDesc& d, const float* x, const float* w, const float* b, const PoolEpilogue& pool, void* ws, size_t ws_bytes, int flags,
+                     cudaStream_t st) {
+    const TcPlan& pl = make_plan(d);
+    if (ws_bytes < pl.total || !ws) return set_error(AE_BAD_ARG, "conv workspace too small: %zu < %zu", ws_bytes, pl.total);
+    uint8_t* wsb = static_cast<uint8_t*>(ws);
+    __nv_bfloat16* xsh = reinterpret_cast<__nv_bfloat16*>(wsb + pl.off_xsh);
+    int rc;
+    if (!(flags & AETHER_CONV_X_COPY_READY) && (rc = launch_cast(x, xsh, 1LL * d.S * d.H * d.W, d.Cin, pl.Cin_p, nullptr, 0, st))) return rc;
+    if (!(flags & AETHER_CONV_W_COPY_READY) && (rc = tc_conv_filter_copies(d, w, ws, ws_bytes, st))) return rc;
+    // (the output itself is not written: its rows are told from rows outside the image by their addresses)
+    return run_igemm(false, xsh, pl.Cin_p, d.H, d.W, d.S, wsb + pl.off_wf, pl.Cin_p, pl.Cout_p, pl.taps, pool.pooled, d.Cout, pl.Ho, pl.Wo,
+                     choose_pool_tiling(d.S, pl.Ho, pl.Wo), pl.Cout_p, d.fH, d.fW, +1, -d.padH, -d.padW, d.Cin, b, nullptr, st, nullptr, nullptr, &pool);
 }
 
 int tc_conv_bwd(const AetherConvDesc& d, const float* x, const float* dy, const float* w, float* dx, float* dw,

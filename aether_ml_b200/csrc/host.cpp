@@ -136,7 +136,7 @@ struct Entry<int (*)(A...)> {
 };
 
 #define ENTRY_POINTS(X)                                                                                                \
-    X(aether_conv2d_fwd_ex) X(aether_conv2d_bwd_ex) X(aether_conv2d_filter_copies) X(aether_bn_fwd_train) X(aether_bn_fwd_train_partials)             \
+    X(aether_conv2d_fwd_ex) X(aether_conv2d_bwd_ex) X(aether_conv2d_filter_copies) X(aether_conv2d_pool_fwd) X(aether_bn_fwd_train) X(aether_bn_fwd_train_partials)             \
     X(aether_bn_fwd_eval) X(aether_bn_bwd) X(aether_bn_act_fwd_train) X(aether_bn_act_fwd_eval) X(aether_bn_act_bwd)   \
     X(aether_bn_act_pool_fwd_copy) X(aether_chain_fwd) X(aether_pool_fwd) X(aether_pool_bwd) X(aether_leaky_relu_fwd)                      \
     X(aether_leaky_relu_bwd) X(aether_leaky_relu_fwd_mask) X(aether_leaky_relu_bwd_mask) X(aether_channel_scale) X(aether_dropout_fwd) X(aether_mul) X(aether_adam_step)           \

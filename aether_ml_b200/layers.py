@@ -10,6 +10,7 @@ Inputs may be torch CUDA tensors, objects exposing ``__cuda_array_interface__`` 
 NumPy arrays (copied to the device).  Outputs are torch CUDA tensors.
 """
 import ctypes as C
+import functools
 import math
 import os
 import weakref
@@ -307,6 +308,11 @@ class _ConvPlan:
         if self.layout is None and self.y_shape is not None and self.stats_blocks == 0 and not self.head:
             self.fwd_ws_bytes = int(lib().aether_conv2d_fwd_workspace_bytes(d))
 
+    @functools.cached_property
+    def pools(self):
+        """Whether the library has a forward call that goes on to the pooled output (aether_conv2d_pool_fwd)."""
+        return bool(lib().aether_conv2d_pool_supported(AetherConvDesc.from_buffer_copy(self.raw)))
+
     def least_ws_bytes(self):
         """The workspace that every call can do with."""
         return int(lib().aether_conv2d_least_workspace_bytes(AetherConvDesc.from_buffer_copy(self.raw)))
@@ -473,6 +479,24 @@ class Conv_Layer(_TakesCopies, _Saved):
         self._desc = p
         self._copies.record(ws, x, w)
         return y
+
+    def forward_pooled(self, x, p, bn, alpha, pooled, target):
+        """Inference over `x` by plan `p` up to the pooled output of the Batch_Norm, activation and 2x2 max Pooling behind this layer
+        (Model), with its operand copy at `target`; the layers' attributes stay as they are."""
+        H = host()
+        ws = self._ws.get(p.fwd_ws_bytes, p)
+        w = self.filter_weights
+        flags = 0
+        if self._handed.x is not None:
+            flags = _lib.CONV_X_COPY_READY if self._handed.x_ready(ws, x) else 0
+            self._handed.x = None
+        if not flags:
+            _require_written(x, "Conv_Layer.forward")
+        if self._weights_fixed and p.layout is not None and self._copies.weights_valid(ws, w):
+            flags |= _lib.CONV_W_COPY_READY
+        H.aether_conv2d_pool_fwd(p.raw, x, w, self.biases, bn.gamma, bn.beta, bn._rm, bn._rv, bn.epsilon, alpha, pooled, target[0] if target else None,
+                                 target[1] if target else 0, ws, self._ws.size, flags)
+        self._copies.record(ws, x, w)
 
     def backward(self, dvalues, need_dinputs=True):
         p = self._desc

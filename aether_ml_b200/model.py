@@ -257,6 +257,46 @@ class _Chain:
         return True
 
 
+class _ConvChain:
+    """A Conv_Layer and the chain behind it that ends in a 2x2 max Pooling, which an inference pass whose layers keep nothing runs in one launch: the
+    convolution's epilogue goes on to the pooled output, and the arrays in between are never written.  Conditions as for _Chain."""
+
+    def __init__(self, conv, chain):
+        self.conv, self.chain = conv, chain
+        self.links = _links([conv, chain.bn])
+        self.length = 1 + chain.length
+
+    @staticmethod
+    def find(layers, i, chain):
+        pool = chain.pool
+        if type(layers[i]) is Conv_Layer and pool is not None and tuple(pool.filter_size) == (2, 2):
+            return _ConvChain(layers[i], chain)
+        return None
+
+    def forward(self, layers, i, inputs, training, keep_all=True):
+        conv, chain = self.conv, self.chain
+        if training or keep_all or layers[i] is not conv or "forward" in conv.__dict__ or not chain._intact(layers, i + 1, False) or not _as_wired(self.links[0]):
+            return False
+        bn = chain.bn
+        x = to_device(inputs)
+        if (x.ndim != 4 or x.shape[3] != conv.filter_weights.shape[2] or bn.gamma is None or chain.pool.filter_size != (2, 2) or tuple(chain.pool.strides) != (2, 2)
+                or bn.gamma.numel() != conv.num_filters):
+            return False
+        alpha = chain.act._alpha
+        p = conv._plan(x.shape)
+        if p.y_shape is None or not p.pools or not 0.0 <= alpha < 1.0:
+            return False
+        S, H, W, Cc = p.y_shape
+        pooled = host().empty((S, H // 2, W // 2, Cc))
+        target = chain.consumer.x_copy_target(tuple(pooled.shape)) if chain.consumer is not None else None
+        conv.forward_pooled(x, p, bn, alpha, pooled, target)
+        if target:
+            chain.consumer.x_copy_written(pooled)
+        chain.live = None
+        chain.pool.output = pooled
+        return True
+
+
 class _DenseAct:
     """A Layer_Dense and the (Leaky_)ReLU behind it, run in one call each way; every attribute of both layers is as the layers
     leave it.  Same conditions as _Chain, and only where the library has one launch for it."""
@@ -506,6 +546,8 @@ class Model:
         self._chains = {i: c for i in range(len(self.layers))
                         if (c := (None if fuse else _Chain.find(self.layers, i)) or _DenseAct.find(self.layers, i) or _Head.find(self.layers, i)) is not None}
         self._chain_ends = {i + c.length - 1: i for i, c in self._chains.items() if type(c) is not _Head}
+        self._chains.update({i - 1: c for i, chain in list(self._chains.items()) if i > 0 and type(chain) is _Chain
+                             and (c := _ConvChain.find(self.layers, i - 1, chain)) is not None})
         self.trainable_layers = [l for l in self.layers if hasattr(l, "weights")]
         if self.loss is not None:
             self.loss.remember_trainable_layers(self.trainable_layers)

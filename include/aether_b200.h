@@ -153,6 +153,16 @@ int aether_conv2d_fwd_ex(const AetherConvDesc* desc, const float* x, const float
  * program that runs several layers can have them made beside the first ones).  bf16 mode, shapes with operand copies of x. */
 int aether_conv2d_filter_copies(const AetherConvDesc* desc, const float* w, void* ws, size_t ws_bytes, void* stream);
 
+/* Inference: the forward pass and, in its epilogue, the layers behind it -- Batch_Norm by its running statistics (y * gamma / sqrt(running_var + eps)
+ * + ..., CNN_classes_cupy.py:484-488), (leaky) ReLU and max pooling over 2x2 windows with stride 2 -- of which only the pooled values [S][Ho/2][Wo/2][Cout] are
+ * written and, when given, their bf16 operand copy (rows of copy_ld, a multiple of four, Cout <= copy_ld <= Cout rounded up to 64; 8-byte aligned; padded
+ * columns are zeroed).  The same numbers as aether_conv2d_fwd_ex followed by aether_chain_fwd give, up to the order of the convolution's sums.
+ * bf16 mode, output heights and widths that are even (aether_conv2d_pool_supported); ws as for a forward pass (first layers: not used). */
+int aether_conv2d_pool_supported(const AetherConvDesc* desc);
+int aether_conv2d_pool_fwd(const AetherConvDesc* desc, const float* x, const float* w, const float* b, const float* gamma, const float* beta,
+                           const float* running_mean, const float* running_var, float eps, float alpha, float* pooled, void* operand_copy,
+                           int copy_ld, void* ws, size_t ws_bytes, int flags, void* stream);
+
 /* The forward pass and the (leaky) ReLU behind it (a Dense layer of a small network is a launch of its own for each): y as
  * aether_conv2d_fwd_ex writes it, act_out = y > 0 ? y : alpha * y and, when given, the bf16 operand copy of act_out for the
  * layer behind, in rows of copy_ld (a multiple of four, Cout <= copy_ld <= Cout rounded up to 64; 8-byte aligned; padded columns are zeroed).  Shapes of the
