@@ -368,7 +368,7 @@ __global__ void __launch_bounds__(256) chain_fwd_kernel(const float* __restrict_
             if (arg != nullptr) reinterpret_cast<uchar4*>(arg)[opix * C4 + cv] = code;
             if (copy != nullptr) store_operand_copy(copy, copy_ld, opix, (int)cv, C4, best);
         } else if (pooled == nullptr && copy != nullptr) {
-            store_operand_copy(copy, copy_ld, first / C4, (int)cv, C4, best);
+            store_operand_copy(copy, copy_ld, ((size_t)smp * H + ho) * W + wo, (int)cv, C4, best);
         }
     }
 }

@@ -7,11 +7,15 @@
 // CTA, 296: 114 KB out of L2 per CTA, which is why there is one per SM and not two; double precision, fixed order -- the same
 // bits in every CTA), and the coefficients go straight from shared memory into its pass.  The first chunk's CTA writes the
 // statistics.  (Clusters of four CTAs that share the merge through distributed shared memory start later than they save.)
+// What a thread reads first of its windows is on its way while the merge runs (forward pass of 128 x 32x32x32, 16x16x64, 8x8x128: 10.7, 9.0, 7.8 -> 10.5, 8.8,
+// 7.5 us); going back the activation's derivative is taken at the selected cell only and its coefficients come out of shared memory, so that 64
+// registers hold a window (13.7, 10.9, 8.4 -> 12.6, 9.2, 7.5 us; of 376 bytes of spills 64 are left, around the merge).
 // Only below BN_SMALL (tail.cuh): a large tensor is a stream of HBM traffic, for which the CTAs' 128-byte pieces and the
 // repeated merge cost more than the 7 us they save.
 #include <cuda_bf16.h>
 
 #include "common.cuh"
+#include "sm100_ptx.cuh"
 #include "stats_epilogue.cuh"
 #include "tail.cuh"
 #include "tc_host.cuh"
@@ -65,9 +69,34 @@ __global__ void __launch_bounds__(BNS_THREADS, 1) bn_small_fwd_kernel(const BnSm
     __shared__ __align__(16) float sc_s[32], sh_s[32], mk_s[32];
     const int ncb = (p.C + 31) >> 5;
     const int cb = blockIdx.x % ncb, chunk = blockIdx.x / ncb, chunks = gridDim.x / ncb;
+    const int g8 = threadIdx.x & 7, C4 = p.C >> 2, cv = cb * 8 + g8;
+    const int fH = F ? F : p.fH, fW = F ? F : p.fW;
+    const int Ho = p.H / fH, Wo = p.W / fW;
+    // a thread's next window: its first value and, of windows of a known size, all of them
+    unsigned win = chunk * BNS_LANES + (threadIdx.x >> 3), smp = 0;
+    int ho = 0, wo = 0;
+    unsigned first = 0;                                  // (32 bits: BN_SMALL)
+    bool whole = false;
+    float4 pre[F ? F * F : 1];
+    auto load = [&]() {
+        if (win >= p.windows || cv >= C4) return;
+        wo = (int)(win % (unsigned)p.Wc);
+        const unsigned r = win / (unsigned)p.Wc;
+        ho = (int)(r % (unsigned)p.Hc);
+        smp = r / (unsigned)p.Hc;
+        first = ((smp * p.H + ho * fH) * p.W + wo * fW) * C4 + cv;
+        whole = ho < Ho && wo < Wo;
+        if (F) {
+#pragma unroll
+            for (int k = 0; k < F * F; ++k)
+                if (whole || (ho * F + k / (F ? F : 1) < p.H && wo * F + k % (F ? F : 1) < p.W))
+                    pre[k] = reinterpret_cast<const float4*>(p.x)[first + ((unsigned)(k / (F ? F : 1)) * p.W + k % (F ? F : 1)) * C4];
+        }
+    };
+    load();                                              // (does not wait for the merge)
     {
         const int c = cb * 32 + (threadIdx.x & 31);
-        float ga = 0.f, be = 0.f, mk = 1.f;              // (loads that need not wait for the merge)
+        float ga = 0.f, be = 0.f, mk = 1.f;
         if (threadIdx.x < 32 && c < p.C) {
             ga = p.gamma[c];
             be = p.beta[c];
@@ -105,27 +134,11 @@ __global__ void __launch_bounds__(BNS_THREADS, 1) bn_small_fwd_kernel(const BnSm
         }
         __syncthreads();
     }
-    const int g8 = threadIdx.x & 7, C4 = p.C >> 2, cv = cb * 8 + g8;
     if (cv >= C4) return;
     const float4 s = *reinterpret_cast<const float4*>(sc_s + 4 * g8), t = *reinterpret_cast<const float4*>(sh_s + 4 * g8);
     const float4 k4 = *reinterpret_cast<const float4*>(mk_s + 4 * g8);
-    const int fH = F ? F : p.fH, fW = F ? F : p.fW;
-    const int Ho = p.H / fH, Wo = p.W / fW;
     const bool act = p.alpha >= 0.f;
-    for (unsigned win = chunk * BNS_LANES + (threadIdx.x >> 3); win < p.windows; win += chunks * BNS_LANES) {
-        const int wo = (int)(win % (unsigned)p.Wc);
-        unsigned r = win / (unsigned)p.Wc;
-        const int ho = (int)(r % (unsigned)p.Hc);
-        const unsigned smp = r / (unsigned)p.Hc;
-        const size_t first = (((size_t)smp * p.H + (size_t)ho * fH) * p.W + (size_t)wo * fW) * C4 + cv;
-        const bool whole = ho < Ho && wo < Wo;
-        float4 pre[F ? F * F : 1];
-        if (F) {
-#pragma unroll
-            for (int k = 0; k < F * F; ++k)
-                if (whole || (ho * F + k / (F ? F : 1) < p.H && wo * F + k % (F ? F : 1) < p.W))
-                    pre[k] = reinterpret_cast<const float4*>(p.x)[first + ((size_t)(k / (F ? F : 1)) * p.W + k % (F ? F : 1)) * C4];
-        }
+    for (; win < p.windows; win += chunks * BNS_LANES, load()) {
         float4 best = make_float4(0.f, 0.f, 0.f, 0.f), sel = best;
         uchar4 code = make_uchar4(0, 0, 0, 0);
 #pragma unroll
@@ -133,7 +146,7 @@ __global__ void __launch_bounds__(BNS_THREADS, 1) bn_small_fwd_kernel(const BnSm
 #pragma unroll
             for (int j = 0; j < fW; ++j) {
                 if (!whole && (ho * fH + i >= p.H || wo * fW + j >= p.W)) continue;
-                const size_t cell = first + ((size_t)i * p.W + j) * C4;
+                const unsigned cell = first + ((unsigned)i * p.W + j) * C4;
                 const float4 v = F ? pre[F ? i * F + j : 0] : reinterpret_cast<const float4*>(p.x)[cell];
                 float4 o = make_float4(fmaf(v.x, s.x, t.x), fmaf(v.y, s.y, t.y), fmaf(v.z, s.z, t.z), fmaf(v.w, s.w, t.w));
                 if (p.bn_out != nullptr) reinterpret_cast<float4*>(p.bn_out)[cell] = o;
@@ -155,7 +168,7 @@ __global__ void __launch_bounds__(BNS_THREADS, 1) bn_small_fwd_kernel(const BnSm
                 }
             }
         if (!whole) continue;
-        const size_t opix = ((size_t)smp * Ho + ho) * Wo + wo;
+        const unsigned opix = (smp * Ho + ho) * Wo + wo;
         if (p.pooled != nullptr) reinterpret_cast<float4*>(p.pooled)[opix * C4 + cv] = best;
         if (p.arg != nullptr) reinterpret_cast<uchar4*>(p.arg)[opix * C4 + cv] = code;
         if (p.xsel != nullptr) reinterpret_cast<float4*>(p.xsel)[opix * C4 + cv] = sel;
@@ -169,16 +182,39 @@ template <int F>
 __global__ void __launch_bounds__(BNS_THREADS, 1) bn_small_bwd_kernel(const BnSmallBwd p) {
     pdl_wait();
     __shared__ double red[2][BNS_WARPS][32];
-    __shared__ __align__(16) float k_s[3][32];
+    __shared__ __align__(16) float k_s[3][32], act_s[4][32];
     const int ncb = (p.C + 31) >> 5;
     const int cb = blockIdx.x % ncb, chunk = blockIdx.x / ncb, chunks = gridDim.x / ncb;
+    const int g8 = threadIdx.x & 7, C4 = p.C >> 2, cv = cb * 8 + g8, c4 = cv * 4;
+    const bool c_ok = cv < C4;
+    const int fH = F ? F : p.fH, fW = F ? F : p.fW;
+    const int Wo = p.W / fW;                              // (pooling windows tile the input here)
+    unsigned win = chunk * BNS_LANES + (threadIdx.x >> 3);
+    unsigned first = 0;
+    float4 g = make_float4(0.f, 0.f, 0.f, 0.f), pre[F ? F * F : 1];
+    uchar4 cd = make_uchar4(0, 0, 0, 0);
+    auto load = [&]() {
+        if (win >= p.windows || !c_ok) return;
+        const int wo = (int)(win % (unsigned)Wo);
+        const unsigned hrow = win / (unsigned)Wo;         // s * Ho + ho
+        first = hrow * fH * p.W + wo * fW;
+        g = reinterpret_cast<const float4*>(p.dy)[win * C4 + cv];
+        if (p.arg != nullptr) cd = reinterpret_cast<const uchar4*>(p.arg)[win * C4 + cv];
+        if (F) {
+#pragma unroll
+            for (int k = 0; k < F * F; ++k)
+                pre[k] = reinterpret_cast<const float4*>(p.x)[(first + (unsigned)(k / (F ? F : 1)) * p.W + k % (F ? F : 1)) * C4 + cv];
+        }
+    };
+    load();                                               // (does not wait for the merge)
     {
         const int c = cb * 32 + (threadIdx.x & 31);
-        float ga = 0.f, va = 0.f, me = 0.f, ps = 1.f;
+        float ga = 0.f, be = 0.f, va = 0.f, me = 0.f, ps = 1.f;
         if (threadIdx.x < 32 && c < p.C) {
             ga = p.gamma[c];
             va = p.var[c];
             me = p.mean[c];
+            if (p.beta != nullptr) be = p.beta[c];
             if (p.pscale != nullptr) ps = p.pscale[c];
         }
         merge_partials<2>(red, p.part, p.nblocks, p.C, c, c < p.C, [](const float (&q)[2], double (&v)[2]) {
@@ -203,59 +239,59 @@ __global__ void __launch_bounds__(BNS_THREADS, 1) bn_small_bwd_kernel(const BnSm
             k_s[0][threadIdx.x] = k1;
             k_s[1][threadIdx.x] = k2;
             k_s[2][threadIdx.x] = k3;
+            act_s[0][threadIdx.x] = me;
+            act_s[1][threadIdx.x] = rsqrtf(va + p.eps);
+            act_s[2][threadIdx.x] = ga;
+            act_s[3][threadIdx.x] = be;
         }
         __syncthreads();
     }
-    const int g8 = threadIdx.x & 7, C4 = p.C >> 2, cv = cb * 8 + g8, c = cv * 4;
-    const bool c_ok = cv < C4;
     float4 csum = make_float4(0.f, 0.f, 0.f, 0.f);
     if (c_ok) {
         const float4 k1 = *reinterpret_cast<const float4*>(k_s[0] + 4 * g8), k2 = *reinterpret_cast<const float4*>(k_s[1] + 4 * g8);
         const float4 k3 = *reinterpret_cast<const float4*>(k_s[2] + 4 * g8);
         const bool act = p.alpha >= 0.f;
-        float4 mu = csum, inv = csum, ga = csum, be = csum;
-        if (act) {
-            const float4 vr = *reinterpret_cast<const float4*>(p.var + c);
-            mu = *reinterpret_cast<const float4*>(p.mean + c);
-            ga = *reinterpret_cast<const float4*>(p.gamma + c);
-            be = *reinterpret_cast<const float4*>(p.beta + c);
-            inv = make_float4(rsqrtf(vr.x + p.eps), rsqrtf(vr.y + p.eps), rsqrtf(vr.z + p.eps), rsqrtf(vr.w + p.eps));
-        }
-        const int fH = F ? F : p.fH, fW = F ? F : p.fW;
-        const int Wo = p.W / fW;                          // (pooling windows tile the input here)
-        for (unsigned win = chunk * BNS_LANES + (threadIdx.x >> 3); win < p.windows; win += chunks * BNS_LANES) {
-            const int wo = (int)(win % (unsigned)Wo);
-            const unsigned hrow = win / (unsigned)Wo;     // s * Ho + ho
-            const size_t first = ((size_t)hrow * fH * p.W + (size_t)wo * fW) * C4 + cv;
-            const float4 g = reinterpret_cast<const float4*>(p.dy)[(size_t)win * C4 + cv];
-            uchar4 cd = make_uchar4(0, 0, 0, 0);
-            if (p.arg != nullptr) cd = reinterpret_cast<const uchar4*>(p.arg)[(size_t)win * C4 + cv];
-            float4 pre[F ? F * F : 1];
+        auto coeffs = [&](int k) {                        // (out of shared memory for every window: sixteen registers fewer)
+            float4 v;
+            asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(smem_u32(act_s[k] + 4 * g8)));
+            return v;
+        };
+        // dy of a window's selected cell, whose value is v, through the activation
+        auto back = [&](float4 v) {
+            if (!act) return g;
+            const float4 mu = coeffs(0), inv = coeffs(1), ga = coeffs(2), be = coeffs(3);
+            return make_float4(g.x * lrelu_grad(fmaf(ga.x, (v.x - mu.x) * inv.x, be.x), p.alpha), g.y * lrelu_grad(fmaf(ga.y, (v.y - mu.y) * inv.y, be.y), p.alpha),
+                               g.z * lrelu_grad(fmaf(ga.z, (v.z - mu.z) * inv.z, be.z), p.alpha), g.w * lrelu_grad(fmaf(ga.w, (v.w - mu.w) * inv.w, be.w), p.alpha));
+        };
+        for (; win < p.windows; win += chunks * BNS_LANES, load()) {
+            float4 d = g;
             if (F) {
+                float4 v = pre[0];
 #pragma unroll
-                for (int k = 0; k < F * F; ++k)
-                    pre[k] = reinterpret_cast<const float4*>(p.x)[first + ((size_t)(k / (F ? F : 1)) * p.W + k % (F ? F : 1)) * C4];
+                for (int k = 1; k < F * F; ++k) {
+                    if (cd.x == k) v.x = pre[k].x;
+                    if (cd.y == k) v.y = pre[k].y;
+                    if (cd.z == k) v.z = pre[k].z;
+                    if (cd.w == k) v.w = pre[k].w;
+                }
+                d = back(v);
             }
 #pragma unroll
             for (int i = 0; i < fH; ++i)
 #pragma unroll
                 for (int j = 0; j < fW; ++j) {
-                    const size_t cell = first + ((size_t)i * p.W + j) * C4;
+                    const unsigned pixel = first + (unsigned)i * p.W + j, cell = pixel * C4 + cv;
                     const float4 v = F ? pre[F ? i * F + j : 0] : reinterpret_cast<const float4*>(p.x)[cell];
                     const unsigned char k = (unsigned char)(i * fW + j);
                     float4 o = make_float4(fmaf(k2.x, v.x, k3.x), fmaf(k2.y, v.y, k3.y), fmaf(k2.z, v.z, k3.z), fmaf(k2.w, v.w, k3.w));
-                    float4 d = g;
-                    if (act) {
-                        d.x *= lrelu_grad(fmaf(ga.x, (v.x - mu.x) * inv.x, be.x), p.alpha); d.y *= lrelu_grad(fmaf(ga.y, (v.y - mu.y) * inv.y, be.y), p.alpha);
-                        d.z *= lrelu_grad(fmaf(ga.z, (v.z - mu.z) * inv.z, be.z), p.alpha); d.w *= lrelu_grad(fmaf(ga.w, (v.w - mu.w) * inv.w, be.w), p.alpha);
-                    }
+                    if (!F) d = back(v);
                     if (cd.x == k) o.x = fmaf(k1.x, d.x, o.x);
                     if (cd.y == k) o.y = fmaf(k1.y, d.y, o.y);
                     if (cd.z == k) o.z = fmaf(k1.z, d.z, o.z);
                     if (cd.w == k) o.w = fmaf(k1.w, d.w, o.w);
                     if (p.dx != nullptr) reinterpret_cast<float4*>(p.dx)[cell] = o;
                     if (p.copy != nullptr) {
-                        store_operand_copy(p.copy, p.copy_ld, cell / C4, cv, C4, o);
+                        store_operand_copy(p.copy, p.copy_ld, pixel, cv, C4, o);
                         csum.x += o.x; csum.y += o.y; csum.z += o.z; csum.w += o.w;
                     }
                 }
@@ -275,7 +311,7 @@ __global__ void __launch_bounds__(BNS_THREADS, 1) bn_small_bwd_kernel(const BnSm
             float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
             for (int l = 0; l < BNS_WARPS; ++l) { const float4 v = sums[l * 8 + threadIdx.x]; t.x += v.x; t.y += v.y; t.z += v.z; t.w += v.w; }
-            *reinterpret_cast<float4*>(p.colsum_part + (size_t)chunk * p.C + c) = t;
+            *reinterpret_cast<float4*>(p.colsum_part + (size_t)chunk * p.C + c4) = t;
         }
     }
 }
