@@ -17,7 +17,7 @@ HOST_DIGEST_PATH = HOST_PATH + ".digest"
 HOST_SOURCE = os.path.join(CSRC, "host.cpp")
 HEADER = os.path.join(HERE, "..", "include", "aether_b200.h")
 HOST_FLAGS = ["-O2", "-std=c++17", "-shared", "-fPIC"]
-SOURCES = ["api.cu", "conv_tc.cu", "conv_halo.cu", "conv_halo_dw.cu", "conv_dw_rows.cu", "conv_generic.cu", "conv_dx_few.cu", "conv_simt.cu", "conv_split.cu", "conv_smallc.cu", "conv_first_tc.cu", "layers.cu",
+SOURCES = ["api.cu", "conv_tc.cu", "conv_halo.cu", "conv_halo_dw.cu", "conv_dw_rows.cu", "conv_generic.cu", "conv_dx_few.cu", "conv_simt.cu", "conv_split.cu", "conv_smallc.cu", "conv_first_tc.cu", "conv_first_fp32.cu", "layers.cu",
            "block_fused.cu", "bn_small.cu"]
 # tcgen05 / TMA PTX only assembles for the arch-specific target, hence compute_100a + sm_100a.
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",

@@ -107,6 +107,9 @@ static bool split_route(const AetherConvDesc& d) {
     return !tc_conv_eligible(d) && !first_tc_eligible(d) && !smallc_conv_eligible(d) && !generic_head_shape(d) && split_conv_eligible(d);
 }
 
+// First layers whose products are summed in single precision, from the arrays themselves.
+static bool first_fp32_dw_route(const AetherConvDesc& d) { return !tc_conv_eligible(d) && !split_route(d) && first_fp32_dw_eligible(d); }
+
 static int pending_timeout(const char* fn) {
     if (g_status_host && *reinterpret_cast<volatile int*>(g_status_host) != 0)
         return set_error(AE_DEVICE_TIMEOUT, "%s: an earlier kernel abandoned a bounded wait (status %d)", fn,
@@ -190,6 +193,10 @@ extern "C" size_t aether_conv2d_workspace_bytes(const AetherConvDesc* d) {
     }
     if (first_tc_bwd_eligible(*d)) {
         size_t s = first_tc_bwd_workspace_bytes(*d);
+        if (s > g) g = s;
+    }
+    if (first_fp32_dw_route(*d)) {
+        size_t s = first_fp32_dw_workspace_bytes(*d);
         if (s > g) g = s;
     }
     const size_t t = tc_conv_eligible(*d) ? tc_conv_workspace_bytes(*d) : split_route(*d) ? split_conv_workspace_bytes(*d) : 0;
@@ -340,6 +347,7 @@ extern "C" int aether_conv2d_fwd(const AetherConvDesc* d, const float* x, const 
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (tc_conv_eligible(*d)) return tc_conv_fwd(*d, x, w, b, y, nullptr, ws, ws_bytes, 0, st);
     if (first_tc_eligible(*d)) return first_tc_fwd(*d, x, w, b, y, nullptr, st);
+    if (!split_route(*d) && first_fp32_fwd_eligible(*d)) return first_fp32_fwd(*d, x, w, b, y, st);
     if (smallc_conv_eligible(*d) && (!b || aligned16(b))) return smallc_conv_fwd(*d, x, w, b, y, nullptr, st);
     if (split_route(*d) && ws && ws_bytes >= split_conv_fwd_workspace_bytes(*d)) return split_conv_fwd(*d, x, w, b, y, ws, st);
     return generic_conv_fwd(*d, x, w, b, y, ws, ws_bytes, st);
@@ -409,8 +417,9 @@ extern "C" int aether_conv2d_bwd_ex(const AetherConvDesc* d, const float* x, con
         dx = nullptr;
     }
     if (dx && (rc = generic_conv_bwd_data(*d, dy, w, dx, ws, ws_bytes, st))) return rc;
-    if (dw && first_tc_bwd_eligible(*d))
+    if (dw && first_tc_bwd_eligible(*d) && (dy_ready || !first_fp32_dw_route(*d) || !first_fp32_dw_faster(*d)))
         return first_tc_bwd_filter(*d, x, dy, dw, db, ws, ws_bytes, dy_ready ? dy_colsum_rows : 0, st);
+    if (dw && first_fp32_dw_route(*d)) return first_fp32_bwd_filter(*d, x, dy, dw, db, ws, ws_bytes, st);
     if ((dw || db) && smallc_conv_eligible(*d) && (!db || aligned16(db)))
         return smallc_conv_bwd_filter(*d, x, dy, dw, db, ws, ws_bytes, st);
     if (dw || db) return simt_conv_bwd_filter(*d, x, dy, dw, db, ws, ws_bytes, st);

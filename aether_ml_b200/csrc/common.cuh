@@ -106,6 +106,14 @@ long long smallc_conv_stats_blocks(const AetherConvDesc& d);
 int smallc_conv_bwd_filter(const AetherConvDesc& d, const float* x, const float* dy, float* dw, float* db, void* ws,
                            size_t ws_bytes, cudaStream_t st);
 
+// ---- conv_first_fp32.cu : the same layers with 3x3 and 5x5 filters, pieces of rows through registers
+bool first_fp32_fwd_eligible(const AetherConvDesc& d);
+bool first_fp32_dw_eligible(const AetherConvDesc& d);
+bool first_fp32_dw_faster(const AetherConvDesc& d);       // than first_tc_bwd_filter without a copy of dy
+size_t first_fp32_dw_workspace_bytes(const AetherConvDesc& d);
+int first_fp32_fwd(const AetherConvDesc& d, const float* x, const float* w, const float* b, float* y, cudaStream_t st);
+int first_fp32_bwd_filter(const AetherConvDesc& d, const float* x, const float* dy, float* dw, float* db, void* ws, size_t ws_bytes, cudaStream_t st);
+
 // The layers behind a convolution that its kernels may apply in inference (pool_epilogue.cuh): Batch_Norm, (leaky) ReLU, 2x2 max pooling.
 struct PoolEpilogue {
     const float *gamma, *beta, *mean, *var;

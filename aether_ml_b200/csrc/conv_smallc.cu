@@ -11,6 +11,7 @@
 // eight or more FMAs.  Pixel and filter-entry coordinates are decoded once into small shared tables, so the
 // gather itself has no divisions.  dW keeps its accumulators in registers across all tiles of the CTA and
 // writes one partial per CTA; a second kernel adds the partials in fixed order (bit-reproducible, no atomics).
+// (3x3 and 5x5 filters with columns at stride 1 are conv_first_fp32.cu's, except for what these are faster at and forward passes with statistics.)
 #include "common.cuh"
 #include "finish_columns.cuh"
 
