@@ -1011,27 +1011,37 @@ __global__ void __launch_bounds__(256) pool_fwd_kernel(const float* __restrict__
     }
 }
 
-// Backward for windows that tile the input exactly (stride == filter, H and W multiples of it; the 2x2/2 pooling of
-// every reference network): one thread per (window, 4 channels) reads dy and the argmax code once and writes the
-// fH*fW cells of its window -- no per-cell index decode, every byte moved exactly once.
-template <bool MAX>
+// Backward for windows that do not overlap (stride == filter): one thread per (window, 4 channels) reads dy and the argmax code once and writes the fH*fW
+// cells of its window -- no per-cell index decode, every byte moved exactly once.  Cells that no window covers (H, W no multiples of it) are windows without dy.
+// Bound by the write of dx.  (In gather form, us: 633 x 27x28x248 by 3x3 216 / 92, 837 x 19x19x32 by 3x3 20.2 / 9.8.)
+template <bool MAX, int F>
 __global__ void __launch_bounds__(256) pool_bwd_tiled_kernel(const float* __restrict__ dy, const uint8_t* __restrict__ arg,
-                                                             float* __restrict__ dx, unsigned total, int W, int C4,
-                                                             int fH, int fW, int Ho, int Wo) {
+                                                             float* __restrict__ dx, unsigned total, int H, int W, int C4,
+                                                             int fH_, int fW_, int Ho, int Wo, int Hc, int Wc) {
     pdl_wait();
+    const int fH = F ? F : fH_, fW = F ? F : fW_;
     const float inv = 1.f / (float)(fH * fW);
     for (unsigned idx = blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += gridDim.x * blockDim.x) {
         const unsigned cv = idx % (unsigned)C4;
         unsigned pix = idx / (unsigned)C4;
-        const unsigned wo = pix % (unsigned)Wo;
-        pix /= (unsigned)Wo;                                   // = s * Ho + ho
-        const float4 g = __ldcs(reinterpret_cast<const float4*>(dy) + idx);
+        const int wo = (int)(pix % (unsigned)Wc);
+        pix /= (unsigned)Wc;
+        const unsigned s = pix / (unsigned)Hc;
+        const int ho = (int)(pix - s * Hc);
+        const bool whole = ho < Ho && wo < Wo;
+        float4 g = make_float4(0.f, 0.f, 0.f, 0.f);
         uchar4 a = make_uchar4(0, 0, 0, 0);
-        if (MAX) a = reinterpret_cast<const uchar4*>(arg)[idx];
-        // first cell of the window: input row pix*fH (rows of all samples are stacked: H = Ho*fH), column wo*fW
-        float4* out = reinterpret_cast<float4*>(dx) + ((size_t)pix * fH * W + (size_t)wo * fW) * C4 + cv;
+        if (whole) {
+            const size_t at = (((size_t)s * Ho + ho) * Wo + wo) * C4 + cv;
+            g = __ldcs(reinterpret_cast<const float4*>(dy) + at);
+            if (MAX) a = reinterpret_cast<const uchar4*>(arg)[at];
+        }
+        float4* out = reinterpret_cast<float4*>(dx) + (((size_t)s * H + (size_t)ho * fH) * W + (size_t)wo * fW) * C4 + cv;
+#pragma unroll
         for (int i = 0; i < fH; ++i)
+#pragma unroll
             for (int j = 0; j < fW; ++j) {
+                if (!whole && (ho * fH + i >= H || wo * fW + j >= W)) continue;
                 float4 o;
                 if (MAX) {
                     const unsigned char code = (unsigned char)(i * fW + j);
@@ -1519,10 +1529,11 @@ extern "C" int aether_pool_fwd(const float* x, float* y, uint8_t* argmax, int S,
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const int nb = blocks_for(total, 256, 16);
     const bool small = total < (1LL << 31);
-    const bool two = vec == 4 && fH == 2 && fW == 2;
+    const int F = vec == 4 && fH == fW && (fH == 2 || fH == 3) ? fH : 0;
 #define AETHER_POOL_FWD(MAXK, I, ARG)                                                                                  \
     do {                                                                                                               \
-        if (two) launch(pool_fwd_kernel<MAXK, I, 2>, nb, 256, 0, st, x, y, ARG, S, H, W, C, fH, fW, sH, sW, Ho, Wo, vec);  \
+        if (F == 2) launch(pool_fwd_kernel<MAXK, I, 2>, nb, 256, 0, st, x, y, ARG, S, H, W, C, fH, fW, sH, sW, Ho, Wo, vec);  \
+        else if (F == 3) launch(pool_fwd_kernel<MAXK, I, 3>, nb, 256, 0, st, x, y, ARG, S, H, W, C, fH, fW, sH, sW, Ho, Wo, vec);  \
         else launch(pool_fwd_kernel<MAXK, I, 0>, nb, 256, 0, st, x, y, ARG, S, H, W, C, fH, fW, sH, sW, Ho, Wo, vec);      \
     } while (0)
     if (kind == AETHER_POOL_MAX) {
@@ -1548,13 +1559,15 @@ extern "C" int aether_pool_bwd(const float* dy, const uint8_t* argmax, float* dx
     const long long total = 1LL * S * H * W * (vec ? C / 4 : C);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const int nb = blocks_for(total, 256, 16);
-    const long long windows4 = 1LL * S * Ho * Wo * (C / 4);
-    if (vec && sH == fH && sW == fW && H == Ho * fH && W == Wo * fW && windows4 < (1LL << 32) - (1LL << 22)) {
-        const int nbt = blocks_for(windows4, 256, 16);
-        if (kind == AETHER_POOL_MAX)
-            launch(pool_bwd_tiled_kernel<true>, nbt, 256, 0, st, dy, argmax, dx, (unsigned)windows4, W, C / 4, fH, fW, Ho, Wo);
-        else
-            launch(pool_bwd_tiled_kernel<false>, nbt, 256, 0, st, dy, nullptr, dx, (unsigned)windows4, W, C / 4, fH, fW, Ho, Wo);
+    const int Hc = ceil_div(H, fH), Wc = ceil_div(W, fW);
+    const long long windows4 = 1LL * S * Hc * Wc * (C / 4);
+    if (vec && sH == fH && sW == fW && windows4 < (1LL << 32) - (1LL << 22)) {
+        const bool max = kind == AETHER_POOL_MAX;
+        const int F = fH == fW && (fH == 2 || fH == 3) ? fH : 0;
+        const auto kernel = F == 2 ? (max ? pool_bwd_tiled_kernel<true, 2> : pool_bwd_tiled_kernel<false, 2>)
+                          : F == 3 ? (max ? pool_bwd_tiled_kernel<true, 3> : pool_bwd_tiled_kernel<false, 3>)
+                                   : (max ? pool_bwd_tiled_kernel<true, 0> : pool_bwd_tiled_kernel<false, 0>);
+        launch(kernel, blocks_for(windows4, 256, 16), 256, 0, st, dy, argmax, dx, (unsigned)windows4, H, W, C / 4, fH, fW, Ho, Wo, Hc, Wc);
         count_launch();
         return check_launch("aether_pool_bwd");
     }
