@@ -7,6 +7,8 @@
 #include <math.h>
 #include <string.h>
 
+#include <type_traits>
+
 #include "common.cuh"
 #include "stats_epilogue.cuh"
 #include "tail.cuh"
@@ -431,10 +433,25 @@ __global__ void __launch_bounds__(256) affine_channels_kernel(const float* __res
             y4[i] = o;
         }
     } else {
-        for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += stride) {
-            const int c = (int)(i % C);
-            const float o = shift ? fmaf(x[i], scale[c], shift[c]) : x[i] * scale[c];
-            y[i] = (act && o <= 0.f) ? act_alpha * o : o;
+        // (rows that are no multiple of 16 bytes: pieces of 16 bytes all the same, their channels counted one by one, where the arrays are aligned: 200 x 28x28x61
+        // 22 -> 11 us)
+        const bool vec = ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) & 15u) == 0;
+        const long long n4 = vec ? n >> 2 : 0, i0 = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+        auto apply = [&](float v, int c) {
+            const float o = shift ? fmaf(v, scale[c], shift[c]) : v * scale[c];
+            return act && o <= 0.f ? act_alpha * o : o;
+        };
+        for (long long i = (n4 << 2) + i0; i < n; i += stride) y[i] = apply(x[i], (int)(i % C));
+        if (i0 >= n4) return;
+        const long long last = i0 + (n4 - 1 - i0) / stride * stride;
+        const int cstep = (int)(4 * stride % C);
+        int cq = (int)(4 * last % C);
+        for (long long i = last; i >= 0; i -= stride) {
+            const float4 v = __ldcs(reinterpret_cast<const float4*>(x) + i);
+            const int c1 = cq + 1 < C ? cq + 1 : 0, c2 = c1 + 1 < C ? c1 + 1 : 0, c3 = c2 + 1 < C ? c2 + 1 : 0;
+            reinterpret_cast<float4*>(y)[i] = make_float4(apply(v.x, cq), apply(v.y, c1), apply(v.z, c2), apply(v.w, c3));
+            cq -= cstep;
+            if (cq < 0) cq += C;
         }
     }
 }
@@ -529,12 +546,22 @@ __global__ void __launch_bounds__(256) bn_bwd_apply_kernel(const float* __restri
             o.w = fmaf(k1.w, g.w, fmaf(k2.w, xv.w, k3.w));
             reinterpret_cast<float4*>(dx)[i] = o;
         }
-    } else {
-        for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += stride) {
-            const int c = (int)(i % C);
-            const float g = act_gamma ? dy[i] * act_grad(fmaf(act_gamma[c], (x[i] - mean[c]) * rsqrtf(var[c] + eps), act_beta[c]), alpha)
-                                      : dy[i];
-            dx[i] = fmaf(coeff[c], g, fmaf(coeff[C + c], x[i], coeff[2 * C + c]));
+    } else {                                                                      // (as in affine_channels_kernel: 40 -> 17 us)
+        const bool vec = ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(dy) | reinterpret_cast<uintptr_t>(dx)) & 15u) == 0;
+        const long long n4 = vec ? n >> 2 : 0, i0 = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+        auto apply = [&](float xv, float g, int c) {
+            if (act_gamma) g *= act_grad(fmaf(act_gamma[c], (xv - mean[c]) * rsqrtf(var[c] + eps), act_beta[c]), alpha);
+            return fmaf(coeff[c], g, fmaf(coeff[C + c], xv, coeff[2 * C + c]));
+        };
+        for (long long i = (n4 << 2) + i0; i < n; i += stride) dx[i] = apply(x[i], dy[i], (int)(i % C));
+        const int cstep = (int)(4 * stride % C);
+        int cq = (int)(4 * i0 % C);
+        for (long long i = i0; i < n4; i += stride) {
+            const float4 v = __ldcs(reinterpret_cast<const float4*>(x) + i), g = __ldcs(reinterpret_cast<const float4*>(dy) + i);
+            const int c1 = cq + 1 < C ? cq + 1 : 0, c2 = c1 + 1 < C ? c1 + 1 : 0, c3 = c2 + 1 < C ? c2 + 1 : 0;
+            reinterpret_cast<float4*>(dx)[i] = make_float4(apply(v.x, g.x, cq), apply(v.y, g.y, c1), apply(v.z, g.z, c2), apply(v.w, g.w, c3));
+            cq += cstep;
+            if (cq >= C) cq -= C;
         }
     }
 }
@@ -940,7 +967,7 @@ namespace aether {
 // i*fW + j of the FIRST maximum in row-major window order (ties keep the earlier cell).
 // I is the flat-index type: unsigned int whenever the element count fits (32-bit divisions are several times
 // cheaper than 64-bit ones and the index decode is most of the kernel's instructions), else long long.
-// F > 0: F x F windows known at compile time (vec == 4 only): the window's loads are issued together -- one 16-byte
+// F > 0: F x F windows known at compile time: the window's loads are issued together -- one 16-byte
 // load in flight per thread does not cover the HBM latency.
 template <bool MAX, typename I, int F>
 __global__ void __launch_bounds__(256) pool_fwd_kernel(const float* __restrict__ x, float* __restrict__ y,
@@ -995,7 +1022,9 @@ __global__ void __launch_bounds__(256) pool_fwd_kernel(const float* __restrict__
         } else {
             float best = 0.f;
             unsigned char code = 0;
+#pragma unroll
             for (int i = 0; i < fH; ++i)
+#pragma unroll
                 for (int j = 0; j < fW; ++j) {
                     const float v = x[(((size_t)s * H + ho * sH + i) * W + wo * sW + j) * C + cv];
                     const unsigned char k = (unsigned char)(i * fW + j);
@@ -1011,32 +1040,37 @@ __global__ void __launch_bounds__(256) pool_fwd_kernel(const float* __restrict__
     }
 }
 
-// Backward for windows that do not overlap (stride == filter): one thread per (window, 4 channels) reads dy and the argmax code once and writes the fH*fW
+// Backward for windows that do not overlap (stride == filter): one thread per (window, VEC channels) reads dy and the argmax code once and writes the fH*fW
 // cells of its window -- no per-cell index decode, every byte moved exactly once.  Cells that no window covers (H, W no multiples of it) are windows without dy.
-// Bound by the write of dx.  (In gather form, us: 633 x 27x28x248 by 3x3 216 / 92, 837 x 19x19x32 by 3x3 20.2 / 9.8.)
-template <bool MAX, int F>
+// Bound by the write of dx.  (In gather form, us: 633 x 27x28x248 by 3x3 216 / 91, 837 x 19x19x32 by 3x3 20.2 / 8.6, 200 x 28x28x61 by 2x2 69 / 18.)
+template <bool MAX, int F, int VEC>
 __global__ void __launch_bounds__(256) pool_bwd_tiled_kernel(const float* __restrict__ dy, const uint8_t* __restrict__ arg,
-                                                             float* __restrict__ dx, unsigned total, int H, int W, int C4,
+                                                             float* __restrict__ dx, unsigned total, int H, int W, int Cv,
                                                              int fH_, int fW_, int Ho, int Wo, int Hc, int Wc) {
     pdl_wait();
     const int fH = F ? F : fH_, fW = F ? F : fW_;
     const float inv = 1.f / (float)(fH * fW);
     for (unsigned idx = blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += gridDim.x * blockDim.x) {
-        const unsigned cv = idx % (unsigned)C4;
-        unsigned pix = idx / (unsigned)C4;
+        const unsigned cv = idx % (unsigned)Cv;
+        unsigned pix = idx / (unsigned)Cv;
         const int wo = (int)(pix % (unsigned)Wc);
         pix /= (unsigned)Wc;
         const unsigned s = pix / (unsigned)Hc;
         const int ho = (int)(pix - s * Hc);
         const bool whole = ho < Ho && wo < Wo;
-        float4 g = make_float4(0.f, 0.f, 0.f, 0.f);
+        float4 g = make_float4(0.f, 0.f, 0.f, 0.f);           // (VEC 1: the first of them)
         uchar4 a = make_uchar4(0, 0, 0, 0);
         if (whole) {
-            const size_t at = (((size_t)s * Ho + ho) * Wo + wo) * C4 + cv;
-            g = __ldcs(reinterpret_cast<const float4*>(dy) + at);
-            if (MAX) a = reinterpret_cast<const uchar4*>(arg)[at];
+            const size_t at = (((size_t)s * Ho + ho) * Wo + wo) * Cv + cv;
+            if constexpr (VEC == 4) {
+                g = __ldcs(reinterpret_cast<const float4*>(dy) + at);
+                if (MAX) a = reinterpret_cast<const uchar4*>(arg)[at];
+            } else {
+                g.x = __ldcs(dy + at);
+                if (MAX) a.x = arg[at];
+            }
         }
-        float4* out = reinterpret_cast<float4*>(dx) + (((size_t)s * H + (size_t)ho * fH) * W + (size_t)wo * fW) * C4 + cv;
+        const size_t first = (((size_t)s * H + (size_t)ho * fH) * W + (size_t)wo * fW) * Cv + cv;
 #pragma unroll
         for (int i = 0; i < fH; ++i)
 #pragma unroll
@@ -1050,7 +1084,9 @@ __global__ void __launch_bounds__(256) pool_bwd_tiled_kernel(const float* __rest
                 } else {
                     o = make_float4(g.x * inv, g.y * inv, g.z * inv, g.w * inv);
                 }
-                out[((size_t)i * W + j) * C4] = o;
+                const size_t cell = first + ((size_t)i * W + j) * Cv;
+                if constexpr (VEC == 4) reinterpret_cast<float4*>(dx)[cell] = o;
+                else dx[cell] = o.x;
             }
     }
 }
@@ -1529,7 +1565,7 @@ extern "C" int aether_pool_fwd(const float* x, float* y, uint8_t* argmax, int S,
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const int nb = blocks_for(total, 256, 16);
     const bool small = total < (1LL << 31);
-    const int F = vec == 4 && fH == fW && (fH == 2 || fH == 3) ? fH : 0;
+    const int F = fH == fW && (fH == 2 || fH == 3) ? fH : 0;
 #define AETHER_POOL_FWD(MAXK, I, ARG)                                                                                  \
     do {                                                                                                               \
         if (F == 2) launch(pool_fwd_kernel<MAXK, I, 2>, nb, 256, 0, st, x, y, ARG, S, H, W, C, fH, fW, sH, sW, Ho, Wo, vec);  \
@@ -1560,14 +1596,19 @@ extern "C" int aether_pool_bwd(const float* dy, const uint8_t* argmax, float* dx
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const int nb = blocks_for(total, 256, 16);
     const int Hc = ceil_div(H, fH), Wc = ceil_div(W, fW);
-    const long long windows4 = 1LL * S * Hc * Wc * (C / 4);
-    if (vec && sH == fH && sW == fW && windows4 < (1LL << 32) - (1LL << 22)) {
+    const int Cv = vec ? C / 4 : C;
+    const long long windows = 1LL * S * Hc * Wc * Cv;
+    if (sH == fH && sW == fW && windows < (1LL << 32) - (1LL << 22)) {
         const bool max = kind == AETHER_POOL_MAX;
         const int F = fH == fW && (fH == 2 || fH == 3) ? fH : 0;
-        const auto kernel = F == 2 ? (max ? pool_bwd_tiled_kernel<true, 2> : pool_bwd_tiled_kernel<false, 2>)
-                          : F == 3 ? (max ? pool_bwd_tiled_kernel<true, 3> : pool_bwd_tiled_kernel<false, 3>)
-                                   : (max ? pool_bwd_tiled_kernel<true, 0> : pool_bwd_tiled_kernel<false, 0>);
-        launch(kernel, blocks_for(windows4, 256, 16), 256, 0, st, dy, argmax, dx, (unsigned)windows4, H, W, C / 4, fH, fW, Ho, Wo, Hc, Wc);
+        const auto pick = [&](auto v) {
+            constexpr int VEC = decltype(v)::value;
+            return F == 2 ? (max ? pool_bwd_tiled_kernel<true, 2, VEC> : pool_bwd_tiled_kernel<false, 2, VEC>)
+                 : F == 3 ? (max ? pool_bwd_tiled_kernel<true, 3, VEC> : pool_bwd_tiled_kernel<false, 3, VEC>)
+                          : (max ? pool_bwd_tiled_kernel<true, 0, VEC> : pool_bwd_tiled_kernel<false, 0, VEC>);
+        };
+        launch(vec ? pick(std::integral_constant<int, 4>()) : pick(std::integral_constant<int, 1>()), blocks_for(windows, 256, 16), 256, 0, st, dy, argmax, dx,
+               (unsigned)windows, H, W, Cv, fH, fW, Ho, Wo, Hc, Wc);
         count_launch();
         return check_launch("aether_pool_bwd");
     }
