@@ -136,6 +136,7 @@ struct IgemmParams {
     int last_ksteps;     // MMAs that the last K chunk of a tap needs
     ActEpilogue act;     // ACT only
     PoolEpilogue pool;   // POOLED only
+    int splits;          // SPLIT only: CTAs of a cluster
 };
 
 static constexpr int TILE_A_BYTES = 128 * 128;  // 128 pixel rows x 128 B
@@ -146,6 +147,8 @@ static constexpr int IGEMM_TAIL = 1024;         // barriers, TMEM pointer
 static constexpr int IGEMM_STATS_BYTES = IGEMM_EPI_WARPS * STATS_WARP_FLOATS * 4;   // per-warp running column sums and pivots
 static constexpr int IGEMM_POOL_CHANNELS = 1024;                                    // most output channels of POOLED, whose coefficients lie there
 static_assert(2 * IGEMM_POOL_CHANNELS * 4 <= IGEMM_STATS_BYTES, "coefficients");
+static constexpr int IGEMM_SPLIT_BYTES = 4096;                                      // beyond those, SPLIT
+static_assert(IGEMM_EPI_WARPS * 2048 <= IGEMM_STATS_BYTES + IGEMM_SPLIT_BYTES, "SPLIT: a warp's 32 x 16 sums of every CTA's epilogue warp");
 
 // PAIR: two CTAs of a cluster share one 256-row MMA (cta_group::2).  Each holds its own 128 pixel rows and HALF of the
 // filter tile (NT/2 rows), so a stage is smaller and every SM pulls a third less from L2 per FLOP.
@@ -182,9 +185,14 @@ struct IgemmCfg {
 // POOLED (inference): Batch_Norm by its running statistics, (leaky) ReLU and 2x2 max pooling in the epilogue, which writes the pooled values and
 // their bf16 operand copy only.  Boxes are 8 or 16 pixels wide and an even number of rows high, so that the two rows of a window are 8 or 16 accumulator
 // rows apart, in one thread, and its columns in neighbouring ones (lane ^ 4).  (896 x 16x16 32->64 30.8 us, 27.6 and 19.6 apart; 8x8 64->128 20.4, 17.9 and 12.)
-template <bool TF32, int NT, bool STATS, bool PAIR, bool ACT = false, int RB = 128, bool POOLED = false>
+//
+// SPLIT (one tap, 32 columns): the CTAs of a cluster share the K chunks of one tile, and each adds up, in order of rank, and finishes its part of the
+// epilogue warps' sums.  A Dense layer of a small batch is a handful of tiles, each of which pulled all of its rows' K through one SM at 65
+// bytes a clock.
+template <bool TF32, int NT, bool STATS, bool PAIR, bool ACT = false, int RB = 128, bool POOLED = false, bool SPLIT = false>
 __global__ void __launch_bounds__(IGEMM_THREADS, 1) igemm_conv_kernel(const __grid_constant__ IgemmParams p) {
     using Cfg = IgemmCfg<NT, PAIR, RB>;
+    static_assert(!SPLIT || (NT == 32 && !PAIR && !STATS && !POOLED), "one batch of columns a warp");
     constexpr int STAGES = Cfg::STAGES, TILE_A_BYTES = Cfg::TILE_A_BYTES;
     constexpr int KC = TF32 ? RB / 4 : RB / 2;    // K elements per row
     extern __shared__ uint8_t smem_raw[];
@@ -204,8 +212,9 @@ __global__ void __launch_bounds__(IGEMM_THREADS, 1) igemm_conv_kernel(const __gr
 
     const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);      // (warp-uniform for the compiler, too)
     const int lane = threadIdx.x & 31;
-    const int cta_rank = PAIR ? (int)cluster_cta_rank() : 0;
-    const bool issuer = cta_rank == 0;            // the CTA whose warp 1 issues the MMAs
+    const int cta_rank = PAIR || SPLIT ? (int)cluster_cta_rank() : 0;
+    const bool issuer = !PAIR || cta_rank == 0;   // the CTA whose warp 1 issues the MMAs
+    const uint32_t gather_bar = sBar + 512, sGather = sBar + IGEMM_TAIL;  // SPLIT: the other CTAs' sums are there (where statistics would be)
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; ++s) {
@@ -216,6 +225,7 @@ __global__ void __launch_bounds__(IGEMM_THREADS, 1) igemm_conv_kernel(const __gr
             mbar_init(tfull_bar(b), 1);
             mbar_init(tempty_bar(b), (PAIR ? 2 : 1) * IGEMM_EPI_WARPS);
         }
+        if (SPLIT) mbar_init(gather_bar, (p.splits - 1) * (IGEMM_EPI_WARPS / p.splits));
         mbar_fence_init();
         tma_prefetch_desc(&p.tm_in);
         tma_prefetch_desc(&p.tm_w);
@@ -229,6 +239,7 @@ __global__ void __launch_bounds__(IGEMM_THREADS, 1) igemm_conv_kernel(const __gr
             tmem_relinquish();
         }
     }
+    if (SPLIT) cluster_sync_all();    // the other CTAs' barriers exist before anything is sent to them
     pdl_wait();                       // set-up done; from here on global memory is touched
     float* scale_s = reinterpret_cast<float*>(gen_base + (sBar - smem_base) + IGEMM_TAIL);      // POOLED: scale and shift of all channels
     if (POOLED)
@@ -243,8 +254,8 @@ __global__ void __launch_bounds__(IGEMM_THREADS, 1) igemm_conv_kernel(const __gr
     // Work units: pixel tiles (PAIR: pairs of consecutive pixel tiles) x column tiles, unit u -> column tile u % n_tiles_n.
     const long long m_tiles = 1LL * p.tiles_w * p.tiles_h * p.tiles_n;
     const long long total_tiles = (PAIR ? (m_tiles + 1) / 2 : m_tiles) * p.n_tiles_n;
-    const long long t_first = PAIR ? (blockIdx.x >> 1) : blockIdx.x;
-    const long long t_step = PAIR ? (gridDim.x >> 1) : gridDim.x;
+    const long long t_first = PAIR ? (blockIdx.x >> 1) : SPLIT ? blockIdx.x / p.splits : blockIdx.x;
+    const long long t_step = PAIR ? (gridDim.x >> 1) : SPLIT ? gridDim.x / p.splits : gridDim.x;
     // pixel tile of this CTA in unit t; one past the last tile (odd tile count) decodes to an image index outside the
     // tensor: its loads are zero-filled and none of its rows is stored
     auto decode = [&](long long t, int& nt, int& w0, int& h0, int& n0) {
@@ -257,6 +268,7 @@ __global__ void __launch_bounds__(IGEMM_THREADS, 1) igemm_conv_kernel(const __gr
     };
     const int taps = p.fH * p.fW;
     const int kiters = taps * p.kchunks;
+    const int k_begin = SPLIT ? cta_rank * kiters / p.splits : 0, k_end = SPLIT ? (cta_rank + 1) * kiters / p.splits : kiters;
     // bytes per stage on the full barrier: this CTA's two boxes, in a pair those of both CTAs
     const uint32_t chunk_tx = ((uint32_t)p.rows + (uint32_t)Cfg::B_ROWS) * (uint32_t)RB * (PAIR ? 2u : 1u);
     constexpr int KS = Cfg::KS;
@@ -272,10 +284,10 @@ __global__ void __launch_bounds__(IGEMM_THREADS, 1) igemm_conv_kernel(const __gr
             for (long long t = t_first; t < total_tiles && ok; t += t_step) {
                 int nt, w0, h0, n0;
                 decode(t, nt, w0, h0, n0);
-                int kc = 0, j = 0;                         // the (K chunk, filter column) of the next chunk to load
+                int kc = k_begin, j = 0;                   // the (K chunk, filter column) of the next chunk to load
                 int cw = w0 + p.off_w, ch = h0 + p.off_h, wrow = nt * NT + (PAIR ? cta_rank * Cfg::B_ROWS : 0);
-                for (int k0 = 0; k0 < kiters; k0 += KS) {
-                    const int nsub = kiters - k0 < KS ? kiters - k0 : KS;
+                for (int k0 = k_begin; k0 < k_end; k0 += KS) {
+                    const int nsub = k_end - k0 < KS ? k_end - k0 : KS;
                     if (!mbar_wait(empty_bar(s), ph ^ 1u, p.status, DS_TIMEOUT_EMPTY)) { ok = false; break; }
                     if (issuer) mbar_arrive_expect_tx(full_bar(s), chunk_tx * (uint32_t)nsub);
                     const uint32_t bar = PAIR ? cluster_map_shared(full_bar(s), 0) : full_bar(s);   // PAIR: the even CTA's
@@ -316,9 +328,9 @@ __global__ void __launch_bounds__(IGEMM_THREADS, 1) igemm_conv_kernel(const __gr
                 if (!mbar_wait(tempty_bar(buf), aph ^ 1u, p.status, DS_TIMEOUT_TMEM_EMPTY)) { ok = false; break; }
                 tc_fence_after();
                 const uint32_t d_tmem = tmem_base + buf * NT;
-                int kc = 0;
-                for (int k0 = 0; k0 < kiters; k0 += KS) {
-                    const int nsub = kiters - k0 < KS ? kiters - k0 : KS;
+                int kc = k_begin;
+                for (int k0 = k_begin; k0 < k_end; k0 += KS) {
+                    const int nsub = k_end - k0 < KS ? k_end - k0 : KS;
                     if (!mbar_wait(full_bar(s), ph, p.status, DS_TIMEOUT_FULL)) { ok = false; break; }
                     tc_fence_after();
 #pragma unroll
@@ -330,7 +342,7 @@ __global__ void __launch_bounds__(IGEMM_THREADS, 1) igemm_conv_kernel(const __gr
                             if (kc == p.kchunks) kc = 0;
 #pragma unroll
                             for (int k = 0; k < RB / 32; ++k) {            // 32 bytes of K each: two 16-byte units further
-                                const uint32_t acc = (k0 + c > 0 || k > 0) ? 1u : 0u;
+                                const uint32_t acc = (k0 + c > k_begin || k > 0) ? 1u : 0u;
                                 if (k >= nk) break;
                                 if (PAIR) umma_pair<TF32>(d_tmem, da + 2u * k, db + 2u * k, idesc, acc);
                                 else umma<TF32>(d_tmem, da + 2u * k, db + 2u * k, idesc, acc);
@@ -432,6 +444,39 @@ __global__ void __launch_bounds__(IGEMM_THREADS, 1) igemm_conv_kernel(const __gr
                     }
                 }
                 tmem_ld_wait();
+                if constexpr (SPLIT) {
+                    // every CTA adds up and finishes the warps of its rank (mod splits): their registers go to it, [rank][warp][16 bytes of a thread][lane]
+                    const int own = ew % p.splits, per = IGEMM_EPI_WARPS / p.splits;
+                    const uint32_t slot = (uint32_t)((cta_rank * per + ew / p.splits) * 2048 + lane * 16);
+                    if (own != cta_rank) {
+                        const uint32_t dst = cluster_map_shared(sGather, own) + slot;
+#pragma unroll
+                        for (int h = 0; h < 4; ++h) {
+                            const uint32_t* q4 = &v[h >> 1][0][(h & 1) * 4];
+                            asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(dst + h * 512u), "r"(q4[0]), "r"(q4[1]), "r"(q4[2]), "r"(q4[3]) : "memory");
+                        }
+                        asm volatile("fence.acq_rel.cluster;" ::: "memory");
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive_cluster(cluster_map_shared(gather_bar, own));
+                        break;
+                    }
+                    if (!mbar_wait(gather_bar, 0, p.status, DS_TIMEOUT_FULL)) { ok = false; break; }
+                    asm volatile("fence.acq_rel.cluster;" ::: "memory");
+                    float sum[16];
+#pragma unroll
+                    for (int e = 0; e < 16; ++e) sum[e] = 0.f;
+                    for (int r = 0; r < p.splits; ++r)                // (in order of rank, whichever CTA adds)
+#pragma unroll
+                        for (int h = 0; h < 4; ++h) {
+                            const uint32_t* q4 = &v[h >> 1][0][(h & 1) * 4];
+                            float4 o = make_float4(__uint_as_float(q4[0]), __uint_as_float(q4[1]), __uint_as_float(q4[2]), __uint_as_float(q4[3]));
+                            if (r != cta_rank)
+                                o = *reinterpret_cast<const float4*>(gen_base + (sGather - smem_base) + (r * per + ew / p.splits) * 2048 + h * 512 + lane * 16);
+                            sum[4 * h] += o.x; sum[4 * h + 1] += o.y; sum[4 * h + 2] += o.z; sum[4 * h + 3] += o.w;
+                        }
+#pragma unroll
+                    for (int e = 0; e < 16; ++e) v[e >> 3][0][e & 7] = __float_as_uint(sum[e]);
+                }
                 if (cb + 16 * IGEMM_EPI_UB >= ncols) {           // accumulator fully read by this warp
                     tc_fence_before();
                     __syncwarp();
@@ -556,7 +601,7 @@ __global__ void __launch_bounds__(IGEMM_THREADS, 1) igemm_conv_kernel(const __gr
     }
 
     tc_fence_before();
-    if (PAIR) cluster_sync_all();     // neither CTA leaves while the other may still address its barriers or TMEM
+    if (PAIR || SPLIT) cluster_sync_all();     // no CTA leaves while another may still address its barriers, memory or TMEM
     else __syncthreads();
     if (warp == 1) {
         tc_fence_after();
@@ -1338,12 +1383,13 @@ static int pick_nt(int n_padded, long long m_tiles, int kiters, bool pairs = tru
     return best;
 }
 
-template <bool TF32, int NT, bool STATS, bool PAIR, bool ACT = false, int RB = 128, bool POOLED = false>
+template <bool TF32, int NT, bool STATS, bool PAIR, bool ACT = false, int RB = 128, bool POOLED = false, bool SPLIT = false>
 static int launch_igemm_k(const IgemmParams& p, cudaStream_t st) {
     using Cfg = IgemmCfg<NT, PAIR, RB>;
+    constexpr int SMEM = Cfg::SMEM_BYTES + (SPLIT ? IGEMM_SPLIT_BYTES : 0);
     static PerDeviceSmem configured;
-    const auto kernel = igemm_conv_kernel<TF32, NT, STATS, PAIR, ACT, RB, POOLED>;
-    if (int rc = ensure_dynamic_smem(kernel, Cfg::SMEM_BYTES, configured, "igemm_conv")) return rc;
+    const auto kernel = igemm_conv_kernel<TF32, NT, STATS, PAIR, ACT, RB, POOLED, SPLIT>;
+    if (int rc = ensure_dynamic_smem(kernel, SMEM, configured, "igemm_conv")) return rc;
     const long long m_tiles = 1LL * p.tiles_w * p.tiles_h * p.tiles_n;
     const int grid = PAIR ? igemm_pair_grid(m_tiles, p.n_tiles_n, STATS) : igemm_grid(m_tiles, p.n_tiles_n, STATS);
     if (STATS && (grid / (PAIR ? 2 : 1)) % p.n_tiles_n)
@@ -1351,9 +1397,11 @@ static int launch_igemm_k(const IgemmParams& p, cudaStream_t st) {
     const int pk = p.sgn > 0 ? PK_IGEMM_FWD : PK_IGEMM_DX;
     prof_begin(pk, st);
     if (PAIR) {
-        launch_cluster(kernel, 2, grid, IGEMM_THREADS, Cfg::SMEM_BYTES, st, p);
+        launch_cluster(kernel, 2, grid, IGEMM_THREADS, SMEM, st, p);
+    } else if (SPLIT) {
+        launch_cluster(kernel, p.splits, (unsigned)(m_tiles * p.n_tiles_n * p.splits), IGEMM_THREADS, SMEM, st, p);
     } else {
-        launch(kernel, grid, IGEMM_THREADS, Cfg::SMEM_BYTES, st, p);
+        launch(kernel, grid, IGEMM_THREADS, SMEM, st, p);
     }
     prof_end(pk, st);
     count_launch();
@@ -1367,6 +1415,10 @@ static int launch_igemm(const IgemmParams& p, bool pair, bool narrow, cudaStream
     }
     if constexpr (NT == 256 || NT == 192 || NT == 128) {
         if (pair) return p.stats ? launch_igemm_k<TF32, NT, true, true>(p, st) : launch_igemm_k<TF32, NT, false, true>(p, st);
+    }
+    if constexpr (!TF32 && NT == 32) {
+        if (p.splits > 1)
+            return p.act.out ? launch_igemm_k<false, 32, false, false, true, 128, false, true>(p, st) : launch_igemm_k<false, 32, false, false, false, 128, false, true>(p, st);
     }
     if constexpr (!TF32) {
         if (p.act.out) return launch_igemm_k<TF32, NT, false, false, true>(p, st);
@@ -1392,6 +1444,15 @@ static int launch_igemm_pooled(const IgemmParams& p, bool narrow, cudaStream_t s
         if (narrow) return launch_igemm_k<false, NT, false, false, false, 64, true>(p, st);
     }
     return launch_igemm_k<false, NT, false, false, false, 128, true>(p, st);
+}
+
+// CTAs that share a tile's K chunks (SPLIT): as many as there are SMs for, with four chunks each at least, where that takes out twenty chunks of a CTA
+// (a chunk is 0.16 us, the exchange 1.5; 896 x 2048->256 by two, 16 chunks less, 8.9 / 9.0 us).  A GPC takes whole clusters, so that of 148 SMs some 130 are there
+// for eight CTAs each.  (us: 256 x 3136->128 11.8 / 7.8, 128 x 2048->256 9.3 / 7.5, 256 x 8192->1024 24 / 16.7.)
+static int k_splits(long long tiles, int kchunks) {
+    for (int s = 8; s > 1; s >>= 1)
+        if (tiles * s <= num_sms() * 7 / 8 && kchunks >= 4 * s && kchunks - kchunks / s >= 20) return s;
+    return 1;
 }
 
 // Runs out[p, n] = sum_{tap,k} in[p (+/-) tap, k] * Wm[tap][n][k] (+ bias).
@@ -1439,6 +1500,7 @@ static int run_igemm(bool tf32, const void* in, int in_C, int in_H, int in_W, in
     p.fH = fH; p.fW = fW; p.sgn = sgn; p.off_h = off_h; p.off_w = off_w;
     p.kchunks = narrow ? 1 : ceil_div(in_C, KC);
     p.last_ksteps = narrow ? ceil_div(k_real, 16) : last_ksteps(k_real, p.kchunks, KC);
+    p.splits = nt == 32 && taps == 1 && !tf32 && !narrow && stats == nullptr ? k_splits(til.total() * p.n_tiles_n, p.kchunks) : 1;
     if (pool != nullptr) {
         p.pool = *pool;
         switch (nt) {
