@@ -29,13 +29,14 @@ namespace aether {
 // Producer warps, in groups of four that build tiles in turn: three groups where nothing but the gathers of few output channels holds the
 // kernel back (896 x 32x32 3->32 35 -> 29 us, 64 and 128 channels 1-4 %), two with statistics, whose epilogue is the longer
 // chain (128 x 32x32 3->32 10.9 us, 12.0 with three), and for windows of more than 48 values, which a thread keeps in registers: three groups
-// leave it 80 of those (84 bytes spilled; 512 x 32x32 1->64 7x7 33.7 us, 31.6 with two groups, 64 x 64x64 4->32 4x4 19.8 / 18.9).
-__host__ __device__ static constexpr int ft_prod_warps(bool stats, int KP) { return stats || KP > 48 ? 8 : 12; }
-static constexpr int FT_EPI_WARPS = 8;                                       // two teams of four
-__host__ __device__ static constexpr int ft_threads(bool stats, int KP) { return 32 * (ft_prod_warps(stats, KP) + 1 + FT_EPI_WARPS); }      // producers, MMA issuer, epilogue
+// leave it 80 of those (84 bytes spilled; 512 x 32x32 1->64 7x7 33.7 us, 31.6 with two groups, 64 x 64x64 4->32 4x4 19.8 / 18.9).  The pooling epilogue is the
+// longer chain, too: four teams beside two groups (three and three: 784 x 32x32 3->128 30 us, 27.7 so; 1800 x 28x28 1->32 51.6 / 49.5).
+__host__ __device__ static constexpr int ft_prod_warps(bool stats, int KP, bool pooled) { return stats || KP > 48 || pooled ? 8 : 12; }
+__host__ __device__ static constexpr int ft_teams(bool pooled) { return pooled ? 4 : 2; }       // of four epilogue warps
+__host__ __device__ static constexpr int ft_threads(bool stats, int KP, bool pooled) { return 32 * (ft_prod_warps(stats, KP, pooled) + 1 + 4 * ft_teams(pooled)); }      // producers, MMA issuer, epilogue
 static constexpr int FT_STAGE_BYTES = 128 * 128;                             // 128 pixel rows of 128 bytes
 static constexpr int FT_TAIL = 2048;                                         // barriers, TMEM pointer, bias, tap table
-static constexpr int FT_OUT_BYTES = 2 * 2 * FT_STAGE_BYTES;                  // two staging tiles (128 rows x 32 floats) per team
+__host__ __device__ static constexpr int ft_out_bytes(bool pooled) { return ft_teams(pooled) * 2 * FT_STAGE_BYTES; }      // two staging tiles (128 rows x 32 floats) per team
 
 __device__ __forceinline__ void ft_umma(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t hi, uint32_t idesc,
                                         uint32_t accumulate) {
@@ -146,10 +147,12 @@ __device__ __forceinline__ float stats_tree(const float (&v)[8]) { return ((v[0]
 
 // POOLED (inference): the epilogue applies the Batch_Norm behind the layer by its running statistics, the (leaky) ReLU behind that and a 2x2
 // max pooling, and writes the pooled values and their bf16 operand copy only, a quarter of the pixels.  A tile is 32 windows, whose four pixels are
-// four rows of the staged tile.  (896 x 32x32 3->32: 47 us, 30 and 36 for the convolution and the pass over its output.)
+// four rows of the staged tile, which takes the sums as they are: a thread reads four channels of a window again and keeps their coefficients, the eight lanes of
+// a window read whole lines of banks.  (896 x 32x32 3->32: 39.7 us, 30 and 36 for the convolution and the pass over its output; with the activation
+// before the staging, eight channels a thread and two teams 47, 784 x 32x32 3->128 39 against 27.7.)
 template <bool STATS, int KP, int CIN, bool POOLED = false>
-__global__ void __launch_bounds__(ft_threads(STATS, KP), 1) first_conv_kernel(const __grid_constant__ FirstParams p) {
-    constexpr int FT_PROD_WARPS = ft_prod_warps(STATS, KP);
+__global__ void __launch_bounds__(ft_threads(STATS, KP, POOLED), 1) first_conv_kernel(const __grid_constant__ FirstParams p) {
+    constexpr int FT_PROD_WARPS = ft_prod_warps(STATS, KP, POOLED), TEAMS = ft_teams(POOLED);
     extern __shared__ uint8_t smem_raw[];
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t* gen_base = smem_raw + (smem_base - smem_u32(smem_raw));
@@ -157,7 +160,7 @@ __global__ void __launch_bounds__(ft_threads(STATS, KP), 1) first_conv_kernel(co
     const uint32_t sW = smem_base;                                  // filter: NT rows of 128 bytes
     const uint32_t sA = sW + (uint32_t)NT * 128u;                   // NT is a multiple of 32: stays 1024-byte aligned
     const uint32_t sOut = sA + (uint32_t)S * FT_STAGE_BYTES;
-    const uint32_t sBar = sOut + FT_OUT_BYTES;
+    const uint32_t sBar = sOut + ft_out_bytes(POOLED);
     auto full_bar = [&](int s) { return sBar + 8u * s; };
     auto empty_bar = [&](int s) { return sBar + 8u * (S + s); };
     auto tfull_bar = [&](int b) { return sBar + 8u * (2 * S + b); };
@@ -278,7 +281,7 @@ __global__ void __launch_bounds__(ft_threads(STATS, KP), 1) first_conv_kernel(co
         const uint32_t out_u = sOut + (uint32_t)(team * 2 * FT_STAGE_BYTES);
         int cnt = 0, it = team;
         bool ok = true, in_turn = true;
-        for (int t = blockIdx.x + team * grid; t < p.ntiles && ok; t += 2 * grid, it += 2) {
+        for (int t = blockIdx.x + team * grid; t < p.ntiles && ok; t += TEAMS * grid, it += TEAMS) {
             const int buf = it % NB;
             bool mine = in_turn && mbar_wait(tfull_bar(buf), (uint32_t)(it / NB) & 1u, p.status, DS_TIMEOUT_TMEM_FULL);
             tc_fence_after();
@@ -298,12 +301,11 @@ __global__ void __launch_bounds__(ft_threads(STATS, KP), 1) first_conv_kernel(co
                     }
 #pragma unroll
                     for (int c4 = 0; c4 < 8; ++c4) {
-                        const float4 b = *reinterpret_cast<const float4*>(bias_s + ch * 32 + 4 * c4);
-                        float4 a = make_float4(__uint_as_float(v[4 * c4]) + b.x, __uint_as_float(v[4 * c4 + 1]) + b.y,
-                                               __uint_as_float(v[4 * c4 + 2]) + b.z, __uint_as_float(v[4 * c4 + 3]) + b.w);
-                        if (POOLED)
-                            a = pool_activation(a, *reinterpret_cast<const float4*>(scale_s + ch * 32 + 4 * c4),
-                                                *reinterpret_cast<const float4*>(shift_s + ch * 32 + 4 * c4), p.pool.alpha);
+                        float4 a = make_float4(__uint_as_float(v[4 * c4]), __uint_as_float(v[4 * c4 + 1]), __uint_as_float(v[4 * c4 + 2]), __uint_as_float(v[4 * c4 + 3]));
+                        if (!POOLED) {                                // (POOLED: where they are read again)
+                            const float4 b = *reinterpret_cast<const float4*>(bias_s + ch * 32 + 4 * c4);
+                            a = make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w);
+                        }
                         *reinterpret_cast<float4*>(o + row * 128 + ((c4 ^ (row & 7)) << 4)) = a;
                     }
                     if (!POOLED) fence_proxy_async_smem();
@@ -312,25 +314,26 @@ __global__ void __launch_bounds__(ft_threads(STATS, KP), 1) first_conv_kernel(co
                 ok = named_bar_and(1 + team, 128, mine);              // the tile is staged; a failed wait ends the whole team
                 if (!ok) break;
                 if (POOLED) {
-                    // eight channels of a window per thread (who writes this staging tile again has passed the other one's barrier, as everyone
-                    // who reads here has)
-                    const int window = tt >> 2, c8 = (tt & 3) * 8, col = ch * 32 + c8;
-                    const long long at = (long long)t * 32 + window;
-                    if (at * 4 < p.g.P) {
+                    // four channels of two windows per thread, eight neighbours a window's 32 (who writes this staging tile again has passed the other one's
+                    // barrier, as everyone who reads here has)
+                    const int c4 = tt & 7, col = ch * 32 + 4 * c4;
+                    const float4 bi = *reinterpret_cast<const float4*>(bias_s + col), sc = *reinterpret_cast<const float4*>(scale_s + col);
+                    const float4 sh = *reinterpret_cast<const float4*>(shift_s + col);
 #pragma unroll
-                        for (int h = 0; h < 2; ++h) {
-                            float4 m[4];
+                    for (int h = 0; h < 2; ++h) {
+                        const int window = (tt >> 3) + 16 * h;
+                        const long long at = (long long)t * 32 + window;
+                        if (at * 4 >= p.g.P) break;
+                        float4 m[4];
 #pragma unroll
-                            for (int k = 0; k < 4; ++k) {
-                                const int r = window * 4 + k;
-                                m[k] = *reinterpret_cast<const float4*>(o + r * 128 + (((c8 / 4 + h) ^ (r & 7)) << 4));
-                            }
-                            pool_store(p.pool, at, col + 4 * h, p.Cout, pool_first_max(m[0], m[1], m[2], m[3]));
+                        for (int k = 0; k < 4; ++k) {
+                            const int r = window * 4 + k;
+                            const float4 a = *reinterpret_cast<const float4*>(o + r * 128 + ((c4 ^ (r & 7)) << 4));
+                            m[k] = pool_activation(make_float4(a.x + bi.x, a.y + bi.y, a.z + bi.z, a.w + bi.w), sc, sh, p.pool.alpha);
                         }
-                        for (int pad = NT + c8; ch == NC - 1 && pad < p.pool.ld; pad += 32) {          // (columns of padding behind the last chunk)
+                        pool_store(p.pool, at, col, p.Cout, pool_first_max(m[0], m[1], m[2], m[3]));
+                        for (int pad = NT + 4 * c4; ch == NC - 1 && pad < p.pool.ld; pad += 32)       // (columns of padding behind the last chunk)
                             pool_store(p.pool, at, pad, p.Cout, make_float4(0.f, 0.f, 0.f, 0.f));
-                            pool_store(p.pool, at, pad + 4, p.Cout, make_float4(0.f, 0.f, 0.f, 0.f));
-                        }
                     }
                 } else if (tt == 0) {
                     tma_store_2d(&p.tm_y, out_u + (uint32_t)((cnt & 1) * FT_STAGE_BYTES), ch * 32, t * 128);
@@ -720,11 +723,11 @@ int first_tc_fwd(const AetherConvDesc& d, const float* x, const float* w, const 
     p.w = w; p.bias = b; p.stats = stats; p.status = device_status_word();
     p.Cout = d.Cout; p.NT = NT; p.K = K;
     p.ntiles = (p.g.P + 127) / 128;
-    p.stages = 4;
+    p.stages = pool ? 3 : 4;
     if (pool) p.pool = *pool;
     else if (int rc = make_map_2d(&p.tm_y, y, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, d.Cout, p.g.P, 32, 128)) return rc;
     const int stat_bytes = stats ? ft_stats_bytes(NT) : pool ? NT * 8 : 0;
-    const int smem = 1024 + NT * 128 + p.stages * FT_STAGE_BYTES + FT_OUT_BYTES + FT_TAIL + stat_bytes;
+    const int smem = 1024 + NT * 128 + p.stages * FT_STAGE_BYTES + ft_out_bytes(pool != nullptr) + FT_TAIL + stat_bytes;
     using KernelFn = void (*)(const FirstParams);
     static const KernelFn kernels[3][6] = {{first_conv_kernel<false, 16, 0>, first_conv_kernel<false, 32, 0>, first_conv_kernel<false, 48, 0>,
                                             first_conv_kernel<false, 64, 0>, first_conv_kernel<false, 16, 1>, first_conv_kernel<false, 32, 3>},
@@ -735,7 +738,7 @@ int first_tc_fwd(const AetherConvDesc& d, const float* x, const float* w, const 
     static PerDeviceSmem configured[3][6];
     const int ki = first_variant(d, KP), si = stats ? 1 : pool ? 2 : 0;
     if (int rc = ensure_dynamic_smem(kernels[si][ki], 232448, configured[si][ki], "first_conv")) return rc;
-    launch(kernels[si][ki], first_tc_grid(p.ntiles), ft_threads(stats != nullptr, KP), smem, st, p);
+    launch(kernels[si][ki], first_tc_grid(p.ntiles), ft_threads(stats != nullptr, KP, pool != nullptr), smem, st, p);
     count_launch();
     return check_launch("first_conv_kernel");
 }
