@@ -108,7 +108,7 @@ static bool split_route(const AetherConvDesc& d) {
 }
 
 // First layers whose products are summed in single precision, from the arrays themselves.
-static bool first_fp32_dw_route(const AetherConvDesc& d) { return !tc_conv_eligible(d) && !split_route(d) && first_fp32_dw_eligible(d); }
+static bool first_fp32_dw_route(const AetherConvDesc& d) { return first_fp32_dw_eligible(d) && !tc_conv_eligible(d) && !split_route(d); }
 
 static int pending_timeout(const char* fn) {
     if (g_status_host && *reinterpret_cast<volatile int*>(g_status_host) != 0)
@@ -347,7 +347,7 @@ extern "C" int aether_conv2d_fwd(const AetherConvDesc* d, const float* x, const 
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (tc_conv_eligible(*d)) return tc_conv_fwd(*d, x, w, b, y, nullptr, ws, ws_bytes, 0, st);
     if (first_tc_eligible(*d)) return first_tc_fwd(*d, x, w, b, y, nullptr, st);
-    if (!split_route(*d) && first_fp32_fwd_eligible(*d)) return first_fp32_fwd(*d, x, w, b, y, st);
+    if (first_fp32_fwd_eligible(*d) && !split_route(*d)) return first_fp32_fwd(*d, x, w, b, y, st);
     if (smallc_conv_eligible(*d) && (!b || aligned16(b))) return smallc_conv_fwd(*d, x, w, b, y, nullptr, st);
     if (split_route(*d) && ws && ws_bytes >= split_conv_fwd_workspace_bytes(*d)) return split_conv_fwd(*d, x, w, b, y, ws, st);
     return generic_conv_fwd(*d, x, w, b, y, ws, ws_bytes, st);

@@ -1369,13 +1369,15 @@ static int igemm_pair_grid(long long m_tiles, int n_tiles_n, bool stats) {
 // dX 85 / 38.  Few tiles are narrow: 128 rows of a Dense layer 2048 -> 256 15.7 in one tile, 12.3 in eight; 64 images 7x7 128 -> 256 12.0 / 9.2.)
 static int pick_nt(int n_padded, long long m_tiles, int kiters, bool pairs = true) {
     static const int widths[6] = {256, 192, 128, 96, 64, 32};
+    const int sms = num_sms();
+    if (m_tiles * ceil_div(n_padded, 32) <= sms) return 32;           // (one round of the shortest)
     int best = 32;
     double best_cost = 1e300;
     for (int nt : widths) {
         const int cols = ceil_div(n_padded, nt);
         if (cols > 1 && nt > 128 && n_padded % nt) continue;          // (a filter tile reads on into the next tap's rows, a wide one by much)
-        const bool pair = pairs && igemm_use_pairs(m_tiles, nt, cols);
-        const long long units = pair ? (m_tiles + 1) / 2 * cols : m_tiles * cols, slots = pair ? num_sms() / 2 : num_sms();
+        const bool pair = pairs && nt >= 128 && igemm_use_pairs(m_tiles, nt, cols);
+        const long long units = pair ? (m_tiles + 1) / 2 * cols : m_tiles * cols, slots = pair ? sms / 2 : sms;
         const double chunk = 260.0 + (pair ? 1.0 : 2.0) * nt;
         const double cost = (double)((units + slots - 1) / slots) * kiters * chunk + 8.0 * nt;
         if (cost < best_cost - 1e-9) { best_cost = cost; best = nt; }
@@ -1450,8 +1452,10 @@ static int launch_igemm_pooled(const IgemmParams& p, bool narrow, cudaStream_t s
 // (a chunk is 0.16 us, the exchange 1.5; 896 x 2048->256 by two, 16 chunks less, 8.9 / 9.0 us).  A GPC takes whole clusters, so that of 148 SMs some 130 are there
 // for eight CTAs each.  (us: 256 x 3136->128 11.8 / 7.8, 128 x 2048->256 9.3 / 7.5, 256 x 8192->1024 24 / 16.7.)
 static int k_splits(long long tiles, int kchunks) {
+    if (kchunks < 23) return 1;
+    const int room = num_sms() * 7 / 8;
     for (int s = 8; s > 1; s >>= 1)
-        if (tiles * s <= num_sms() * 7 / 8 && kchunks >= 4 * s && kchunks - kchunks / s >= 20) return s;
+        if (tiles * s <= room && kchunks >= 4 * s && kchunks - kchunks / s >= 20) return s;
     return 1;
 }
 

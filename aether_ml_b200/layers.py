@@ -243,10 +243,10 @@ class _TakesCopies:
         return True
 
     def _products(self, p, x, dy, w, dx, db, ws, flags, rows, behind=None):
-        """The backward pass's library call, then `behind` (of the parameters' gradients).  While a step is captured dW goes to the branch, beside
+        """The backward pass's library call while a step is captured, then `behind` (of the parameters' gradients): dW goes to the branch, beside
         the kernels of the layers in front, which wait for dX only."""
         H, b = host(), self._branch
-        if b is None or dx is None or not flags & _lib.CONV_DY_COPY_READY:
+        if dx is None or not flags & _lib.CONV_DY_COPY_READY:
             H.aether_conv2d_bwd_ex(p.raw, x, dy, w, dx, self.dweights, db, ws, self._ws.size, flags, rows)
             if behind is not None:
                 behind()
@@ -528,7 +528,10 @@ class Conv_Layer(_TakesCopies, _Saved):
             _require_written(dy, "Conv_Layer.backward")
         if not (shadow_ok & _lib.CONV_X_COPY_READY):
             _require_written(x, "Conv_Layer.backward")
-        self._products(p, x, dy, w, dx, self.dbiases, ws, shadow_ok, rows)
+        if self._branch is None:
+            H.aether_conv2d_bwd_ex(p.raw, x, dy, w, dx, self.dweights, self.dbiases, ws, self._ws.size, shadow_ok, rows)
+        else:
+            self._products(p, x, dy, w, dx, self.dbiases, ws, shadow_ok, rows)
         self.dinputs = dx
         return dx
 
@@ -1198,10 +1201,14 @@ class Layer_Dense(_TakesCopies, _Saved):
         flags = self._copies.flags(ws, x, w)
         if not (flags & _lib.CONV_X_COPY_READY):
             _require_written(x, "Layer_Dense.backward")
+        db, rows = self.dbiases, 0
         if dy_ready:
-            self._products(p, x, dy, w, dx, None, ws, flags | _lib.CONV_DY_COPY_READY, 1, self._regularize)
+            db, rows, flags = None, 1, flags | _lib.CONV_DY_COPY_READY
+        if self._branch is None:
+            H.aether_conv2d_bwd_ex(p.raw, x, dy, w, dx, self.dweights, db, ws, self._ws.size, flags, rows)
+            self._regularize()
         else:
-            self._products(p, x, dy, w, dx, self.dbiases, ws, flags, 0, self._regularize)
+            self._products(p, x, dy, w, dx, db, ws, flags, rows, self._regularize)
         self.dinputs = dx
         return self.dinputs
 

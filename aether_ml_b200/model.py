@@ -433,6 +433,7 @@ class Model:
         self._updated_early = set()
         self._chains = {}          # position of a Batch_Norm or Layer_Dense -> the _Chain or _DenseAct that starts there
         self._chain_ends = {}      # position of a chain's last layer -> where it starts
+        self._pass_chains = {}     # _chains and, for inference passes that keep nothing, position of a Conv_Layer -> the _ConvChain that starts there
 
     def add(self, layer):
         self.layers.append(layer)
@@ -546,8 +547,8 @@ class Model:
         self._chains = {i: c for i in range(len(self.layers))
                         if (c := (None if fuse else _Chain.find(self.layers, i)) or _DenseAct.find(self.layers, i) or _Head.find(self.layers, i)) is not None}
         self._chain_ends = {i + c.length - 1: i for i, c in self._chains.items() if type(c) is not _Head}
-        self._chains.update({i - 1: c for i, chain in list(self._chains.items()) if i > 0 and type(chain) is _Chain
-                             and (c := _ConvChain.find(self.layers, i - 1, chain)) is not None})
+        self._pass_chains = {**self._chains, **{i - 1: c for i, chain in self._chains.items() if i > 0 and type(chain) is _Chain
+                                                and (c := _ConvChain.find(self.layers, i - 1, chain)) is not None}}
         self.trainable_layers = [l for l in self.layers if hasattr(l, "weights")]
         if self.loss is not None:
             self.loss.remember_trainable_layers(self.trainable_layers)
@@ -609,7 +610,7 @@ class Model:
         """``keep=False`` (inference passes whose layers' attributes the next pass replaces): a chain of layers run in one
         pass writes its last output only."""
         self.input_layer.forward(X, training)
-        layers, chains, i = self.layers, self._chains, 0
+        layers, chains, i = self.layers, self._chains if training or keep or not self._chains else self._pass_chains, 0
         while i < len(layers):
             layer = layers[i]
             link = layer.__dict__.get("_link_prev")       # (layer.prev, the layer in front unless the caller has wired it otherwise)
