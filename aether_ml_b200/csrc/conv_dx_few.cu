@@ -402,9 +402,9 @@ static int dx_few(const AetherConvDesc& d, const float* dy, const float* w, floa
     int Ho, Wo;
     conv_out_hw(d, Ho, Wo);
     // (1x1 filters read each value of dy once, whichever way: 64 x 40x40 3->64 9.0 us through registers, 9.4 through shared memory.  3x3 layers of a few
-    // microseconds wait for the host, which takes 0.8 us longer with two tensor maps to encode: 6 x 21x21 1->32, both passes, 16.4 / 17.3.  Strips and tiles are
-    // counted in 32 bits.)
-    const bool short_call = d.fH == 3 && 1LL * d.S * Ho * Wo * d.Cout * CIN <= 1 << 17;
+    // microseconds wait for the host, which takes 0.8 us longer with two tensor maps to encode: 6 x 21x21 1->32, both passes, 16.4 / 17.3; not with more
+    // input channels or several chunks of output channels, tap by tap: 5 x 8x8 3->80 11 against 4.  Strips and tiles are counted in 32 bits.)
+    const bool short_call = CIN == 1 && d.fH == 3 && d.Cout <= 32 && 1LL * d.S * Ho * Wo * d.Cout <= 1 << 17;
     if (!short_call && d.sH == 1 && d.sW == 1 && d.fH == d.fW && (d.fH == 3 || d.fH == 5) && 1LL * d.S * d.H * d.W < 0x7fffffffLL)
         return d.fH == 3 ? dx_few_tile<CIN, 3>(d, dy, w, dx, Ho, Wo, st) : dx_few_tile<CIN, 5>(d, dy, w, dx, Ho, Wo, st);
     const bool vec = d.Cout % 4 == 0 && aligned16(dy) && aligned16(w);
