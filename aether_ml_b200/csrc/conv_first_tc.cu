@@ -7,7 +7,7 @@
 // 128 output pixels (one pixel per thread, all of a row's loads in flight together), convert them to bf16 and write them
 // as a K-major, 128-byte-swizzled operand tile (16-byte chunk c of row r is stored at chunk c ^ (r % 8)); the filter is
 // laid out the same way once per CTA.  One thread issues K/16 (two for a 3x3 RGB filter) 128 x Cout x 16 MMAs per tile into
-// one of up to four TMEM accumulators.  Two epilogue teams of four warps take alternate tiles: a thread reads 32 columns of
+// one of up to four TMEM accumulators.  Epilogue teams of four warps (two; up to four that pool) take tiles in turn: a thread reads 32 columns of
 // its accumulator row, adds the bias and writes them to a swizzled staging tile that TMA stores to global memory; the
 // statistics the following Batch_Norm needs are summed from the staged tile, a column per lane, so neither the exchange of
 // columns between lanes nor their reduction across lanes is left.  A tile costs about 1700 warp instructions at 32 filters
@@ -180,7 +180,11 @@ __global__ void __launch_bounds__(ft_threads(STATS, KP, POOLED), 1) first_conv_k
 
     const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);
     const int lane = threadIdx.x & 31;
+    // Accumulators, and the teams that take tiles: never more of these than of those.  A team waits for the parity of its tile's round, which an accumulator
+    // that is two rounds behind shows as well: a third team on two accumulators would read one that the first still waits for.
     const int NB = (4 * NT <= 512) ? 4 : (3 * NT <= 512) ? 3 : 2;
+    const int teams = POOLED ? min(TEAMS, NB) : TEAMS;
+    static_assert(POOLED || TEAMS <= 2, "no more teams than accumulators");
     const uint32_t need_cols = (uint32_t)(NB * NT);
     const uint32_t tmem_cols = (need_cols <= 128) ? 128u : (need_cols <= 256) ? 256u : 512u;
 
@@ -269,7 +273,7 @@ __global__ void __launch_bounds__(ft_threads(STATS, KP, POOLED), 1) first_conv_k
         }
     } else {
         // ------------------------------------------------------------------ epilogue
-        const int et = threadIdx.x - 32 * (FT_PROD_WARPS + 1);       // 0 .. 255
+        const int et = threadIdx.x - 32 * (FT_PROD_WARPS + 1);       // 0 .. 128 * TEAMS - 1
         const int team = et >> 7, tt = et & 127;
         const int q = warp & 3;                                      // TMEM lane quarter this warp may access
         const int row = q * 32 + lane;                               // accumulator row of this thread
@@ -281,7 +285,7 @@ __global__ void __launch_bounds__(ft_threads(STATS, KP, POOLED), 1) first_conv_k
         const uint32_t out_u = sOut + (uint32_t)(team * 2 * FT_STAGE_BYTES);
         int cnt = 0, it = team;
         bool ok = true, in_turn = true;
-        for (int t = blockIdx.x + team * grid; t < p.ntiles && ok; t += TEAMS * grid, it += TEAMS) {
+        for (int t = team < teams ? blockIdx.x + team * grid : p.ntiles; t < p.ntiles && ok; t += teams * grid, it += teams) {
             const int buf = it % NB;
             bool mine = in_turn && mbar_wait(tfull_bar(buf), (uint32_t)(it / NB) & 1u, p.status, DS_TIMEOUT_TMEM_FULL);
             tc_fence_after();

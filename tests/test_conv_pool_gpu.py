@@ -9,10 +9,12 @@ from aether_ml_b200 import _lib
 pytestmark = pytest.mark.gpu
 
 # (S, H, W, Cin, Cout, f, pad): first layers (tap tables and not, channels to the next 32, several chunks) and per-tap shapes (boxes of 8 and 16 columns, cut
-# off at the image, several images, narrow rows, wide and overhanging column tiles)
+# off at the image, several images, narrow rows, wide and overhanging column tiles); first layers of so many channels that only two or three accumulators are there
+# for a CTA's tiles, of which it takes five and more, and ones with as many tiles of four accumulators
 SHAPES = [(5, 32, 32, 3, 32, 3, 1), (3, 28, 28, 1, 64, 3, 1), (2, 10, 12, 3, 20, 3, 1), (2, 9, 11, 4, 128, 2, 0), (1, 6, 6, 1, 256, 7, 1), (300, 32, 32, 3, 96, 3, 1),
           (7, 16, 16, 32, 64, 3, 1), (9, 8, 8, 64, 128, 3, 1), (3, 14, 14, 32, 64, 3, 1), (2, 20, 24, 64, 40, 3, 1), (5, 4, 6, 16, 192, 3, 1), (200, 8, 8, 128, 256, 3, 1),
-          (11, 2, 2, 68, 100, 1, 0), (3, 18, 34, 96, 160, 5, 2), (90, 16, 16, 64, 128, 3, 1)]
+          (11, 2, 2, 68, 100, 1, 0), (3, 18, 34, 96, 160, 5, 2), (90, 16, 16, 64, 128, 3, 1),
+          (100, 32, 32, 3, 160, 3, 1), (100, 32, 32, 3, 192, 3, 1), (200, 28, 28, 1, 256, 3, 1), (130, 30, 30, 4, 132, 3, 1), (120, 32, 32, 2, 200, 5, 2), (110, 32, 32, 3, 128, 3, 1)]
 
 
 @pytest.mark.parametrize("S,H,W,Cin,Cout,f,pad", SHAPES)
@@ -62,7 +64,7 @@ def test_refused_where_the_epilogue_does_not_fit():
         assert not lib.aether_conv2d_pool_supported(d)
 
 
-@pytest.mark.parametrize("hw,channels,batch,images", [(32, (32, 64, 128), 128, 1000), (28, (32, 64), 50, 230), (12, (20, 48), 16, 90)])
+@pytest.mark.parametrize("hw,channels,batch,images", [(32, (32, 64, 128), 128, 1000), (28, (32, 64), 50, 230), (12, (20, 48), 16, 90), (32, (192, 32), 64, 400)])
 def test_predictions_are_those_of_single_batches(hw, channels, batch, images):
     """Several batches in one pass (convolutions go on to their pooled outputs) and batch by batch with every layer's arrays."""
     import torch
