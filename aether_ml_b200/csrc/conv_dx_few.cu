@@ -66,6 +66,25 @@ __device__ __forceinline__ uint32_t dxt_at(uint32_t px, uint32_t q) {
 }
 __host__ __device__ constexpr int dxt_filter_bytes(int rows, int QW) { return (rows * QW * 16 + 1023) / 1024 * 1024; }
 
+// A value of dx next to the left or right end of its row, again, from the arrays: the tile's zeros beside the image times a filter value that is not finite
+// are NaN.  (Skipping them in the loop over the filter's columns takes every call longer, 256 x 64x64 3->32 59.3 -> 63.4 us; looking at the results 59.5.)
+template <int CIN, int F>
+__device__ __noinline__ float dxt_again(const DxtParams& p, int n, int h, int w, int c) {
+    float sum = 0.f;
+    for (int i = 0; i < F; ++i) {
+        const int ho = h + p.pH - i;
+        for (int j = 0; j < F; ++j) {
+            const int wo = w + p.pW - j;
+            if ((unsigned)wo >= (unsigned)p.Wo) continue;
+            const bool in = (unsigned)ho < (unsigned)p.Ho;
+            const float* g = p.dy + (((size_t)n * p.Ho + (in ? ho : 0)) * p.Wo + wo) * p.Cout;
+            const float* k = p.w + (size_t)((i * F + j) * CIN + c) * p.Cout;
+            for (int d = 0; d < p.Cout; ++d) sum = fmaf(in ? g[d] : 0.f, k[d], sum);
+        }
+    }
+    return sum;
+}
+
 template <int CIN, int F, int QW, int R, bool TMA>
 __global__ void __launch_bounds__(DXT_THREADS, 2) dx_few_tile_kernel(const __grid_constant__ DxtParams p) {
     constexpr int ROWS = R + F - 1, PG = 8 / QW, PART = R * 32 * CIN, FILTER = dxt_filter_bytes(F * F * CIN, QW);
@@ -220,6 +239,7 @@ __global__ void __launch_bounds__(DXT_THREADS, 2) dx_few_tile_kernel(const __gri
             for (int c = 0; c < CIN; ++c) red[warp * PART + (a * 32 + lane) * CIN + c] = dxf_pair_sum(acc[a][c]);
         __syncthreads();
         const int w0 = first_column(tile);
+        bool bad = false;
         for (int e = tid; e < PG * PART; e += DXT_THREADS) {
             const int g = PG > 1 ? e / PART : 0, f = e - g * PART, col = f / CIN, c = f - col * CIN, l = col & 31, a = col >> 5;
             float t[QW];
@@ -230,7 +250,20 @@ __global__ void __launch_bounds__(DXT_THREADS, 2) dx_few_tile_kernel(const __gri
 #pragma unroll
                 for (int k = 0; k < n; ++k) t[k] += t[k + n];
             const int strip = g * G + (l >> p.tc_log2), b = l & (TC - 1);
-            if (a < rows_s[strip] && w0 + b < p.W) out_s[strip][((size_t)a * p.W + b) * CIN + c] = t[0];
+            if (a < rows_s[strip] && w0 + b < p.W) {
+                out_s[strip][((size_t)a * p.W + b) * CIN + c] = t[0];
+                bad = bad || !isfinite(t[0]);
+            }
+        }
+        for (int e = tid; bad && e < PG * PART; e += DXT_THREADS) {              // (its own values of the loop above)
+            const int g = PG > 1 ? e / PART : 0, f = e - g * PART, col = f / CIN, c = f - col * CIN, a = col >> 5;
+            const int strip = g * G + ((col & 31) >> p.tc_log2), b = col & (TC - 1), w = w0 + b;
+            if (a >= rows_s[strip] || w >= p.W || (w + p.pW >= F - 1 && w + p.pW < p.Wo)) continue;
+            float* o = out_s[strip] + ((size_t)a * p.W + b) * CIN + c;
+            if (isfinite(*o)) continue;
+            int n, a0;
+            strip_of(tile, strip, n, a0);
+            *o = dxt_again<CIN, F>(p, n, a0 + a, w, c);
         }
         if (TMA) {
             fence_proxy_async_smem();                        // (TMA writes next where the sums were)
