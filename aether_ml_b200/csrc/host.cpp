@@ -12,6 +12,7 @@
 
 #include <ATen/ATen.h>
 #include <ATen/cuda/EmptyTensor.h>
+#include <c10/cuda/CUDACachingAllocator.h>
 #include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAStream.h>
 #include <dlfcn.h>
@@ -381,6 +382,20 @@ PyObject* py_same(PyObject*, PyObject* const* args, Py_ssize_t n) try {
     return translated();
 }
 
+// In-place changes so far of a tensor whose every writer counts them, else -1: inference mode counts none, and memory that another library owns (an array
+// handed in by its address) is changed by that library's kernels.
+PyObject* py_counted(PyObject*, PyObject* o) try {
+    if (!THPVariable_Check(o)) {
+        PyErr_SetString(PyExc_TypeError, "expected a tensor");
+        return nullptr;
+    }
+    const at::Tensor& t = THPVariable_Unpack(o);
+    const bool own = !t.is_inference() && t.has_storage() && t.storage().data_ptr().get_deleter() == c10::cuda::CUDACachingAllocator::get()->raw_deleter();
+    return PyLong_FromLongLong(own ? (long long)t._version() : -1);
+} catch (...) {
+    return translated();
+}
+
 #define METHOD(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_##name)), METH_FASTCALL, nullptr},
 PyMethodDef methods[] = {
     ENTRY_POINTS(METHOD)
@@ -395,6 +410,7 @@ PyMethodDef methods[] = {
     {"empty_i32", py_empty<at::kInt>, METH_O, "uninitialised int32 array on the current device"},
     {"empty_like", py_empty_like, METH_O, "uninitialised contiguous array of the argument's shape and type on the current device"},
     {"tag", py_tag, METH_O, "(address, elements, version, row length) of a tensor"},
+    {"counted", py_counted, METH_O, "in-place changes of a tensor so far, -1 where not every writer counts them"},
     {"same", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_same)), METH_FASTCALL, "whether a tensor still has the values of a tag"},
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_host", "native host path of aether_ml_b200", -1, methods};

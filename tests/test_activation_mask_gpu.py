@@ -1,5 +1,5 @@
 """The (leaky) ReLU's way back by the bits its forward pass kept: the same numbers as from the inputs, at sizes around the groups of 128 values, with
-zeros, signed zeros, infinities and NaN; inputs replaced or changed in between are read again."""
+zeros, signed zeros, infinities and NaN; inputs replaced or changed in between are read again, and none are kept of arrays whose changes nobody counts."""
 import pytest
 
 pytestmark = pytest.mark.gpu
@@ -45,3 +45,38 @@ def test_changed_inputs_are_read_again():
     layer.forward(x, True)
     layer.forward(other, False)                             # an inference pass keeps none
     assert layer._mask is None and torch.equal(layer.backward(dy), torch.where(other < 0, torch.zeros_like(dy), dy))
+
+
+class Foreign:
+    """An array of another library: torch learns its address, and of changes nothing."""
+
+    def __init__(self, t):
+        self.t = t
+        self.__cuda_array_interface__ = dict(t.__cuda_array_interface__)
+
+
+@pytest.mark.parametrize("wrapped", [False, True])
+def test_changes_of_an_array_that_another_library_owns(wrapped):
+    import torch
+    from aether_ml_b200 import layers as L
+    layer = L.Leaky_ReLU(0.25)
+    layer.MASK_FROM = 1
+    memory, dy = torch.randn(4096, device="cuda"), torch.randn(4096, device="cuda")
+    x = Foreign(memory)
+    layer.forward(torch.as_tensor(x, device="cuda") if wrapped else x, True)
+    memory.neg_()                                           # the owner's kernel, behind torch's back
+    assert torch.equal(layer.backward(dy), torch.where(memory < 0, 0.25 * dy, dy))
+
+
+def test_inputs_of_inference_mode():
+    import torch
+    from aether_ml_b200 import layers as L
+    layer = L.ReLU()
+    layer.MASK_FROM = 1
+    dy = torch.randn(4096, device="cuda")
+    with torch.inference_mode():
+        x = torch.randn(4096, device="cuda")
+        y = layer.forward(x, True)
+        assert torch.equal(y, x.clamp(min=0))
+        x.neg_()
+        assert torch.equal(layer.backward(dy), torch.where(x < 0, torch.zeros_like(dy), dy))
