@@ -257,6 +257,9 @@ class _Chain:
         return True
 
 
+_OWN = Conv_Layer.__module__     # where this package's layers are
+
+
 class _ConvChain:
     """A Conv_Layer and the chain behind it that ends in a 2x2 max Pooling, which an inference pass whose layers keep nothing runs in one launch: the
     convolution's epilogue goes on to the pooled output, and the arrays in between are never written.  Conditions as for _Chain."""
@@ -433,6 +436,7 @@ class Model:
         self._updated_early = set()
         self._chains = {}          # position of a Batch_Norm or Layer_Dense -> the _Chain or _DenseAct that starts there
         self._chain_ends = {}      # position of a chain's last layer -> where it starts
+        self._built, self._wiring = [], []      # the layers as they were wired; of each the attributes and, among them, the layer in front
         self._pass_chains = {}     # _chains and, for inference passes that keep nothing, position of a Conv_Layer -> the _ConvChain that starts there
 
     def add(self, layer):
@@ -547,8 +551,11 @@ class Model:
         self._chains = {i: c for i in range(len(self.layers))
                         if (c := (None if fuse else _Chain.find(self.layers, i)) or _DenseAct.find(self.layers, i) or _Head.find(self.layers, i)) is not None}
         self._chain_ends = {i + c.length - 1: i for i, c in self._chains.items() if type(c) is not _Head}
-        self._pass_chains = {**self._chains, **{i - 1: c for i, chain in self._chains.items() if i > 0 and type(chain) is _Chain
-                                                and (c := _ConvChain.find(self.layers, i - 1, chain)) is not None}}
+        self._built, self._wiring = list(self.layers), [(vars(l), vars(l).get("_link_prev")) for l in self.layers]
+        self._pass_chains = self._chains
+        if all(type(l).__module__ == _OWN for l in self.layers):
+            self._pass_chains = {**self._chains, **{i - 1: c for i, chain in self._chains.items() if i > 0 and type(chain) is _Chain
+                                                    and (c := _ConvChain.find(self.layers, i - 1, chain)) is not None}}
         self.trainable_layers = [l for l in self.layers if hasattr(l, "weights")]
         if self.loss is not None:
             self.loss.remember_trainable_layers(self.trainable_layers)
@@ -610,7 +617,9 @@ class Model:
         """``keep=False`` (inference passes whose layers' attributes the next pass replaces): a chain of layers run in one
         pass writes its last output only."""
         self.input_layer.forward(X, training)
-        layers, chains, i = self.layers, self._chains if training or keep or not self._chains else self._pass_chains, 0
+        layers, chains, i = self.layers, self._chains, 0
+        if not training and not keep and chains:
+            chains, keep = self._inference_chains()
         while i < len(layers):
             layer = layers[i]
             link = layer.__dict__.get("_link_prev")       # (layer.prev, the layer in front unless the caller has wired it otherwise)
@@ -622,6 +631,19 @@ class Model:
             layer.forward(inputs, training)
             i += 1
         return layers[-1].output
+
+    def _inference_chains(self):
+        """The chains of an inference pass that need not keep what lies between its layers, and whether it has to after all: where a layer reads another
+        one than the model was built with, every output stands.  A layer of the caller's may hold on to any convolution's."""
+        if self.layers != self._built:
+            return self._chains, True
+        chains = self._pass_chains
+        for attributes, front in self._wiring:
+            if attributes.get("_link_prev") is not front:
+                return self._chains, True
+            if "forward" in attributes:
+                chains = self._chains
+        return chains, False
 
     def backward(self, output, y):
         layers = self.layers
@@ -868,7 +890,7 @@ class Model:
         """Whether the passes run this package's code alone.  Methods of the caller's (a subclass, a patched instance) may use any array that the
         layers in front of them have been asked for, a gradient that they clip, say."""
         own = (type(self).forward is Model.forward and type(self).backward is Model.backward and "forward" not in vars(self) and "backward" not in vars(self))
-        return own and all(type(l).__module__ == Conv_Layer.__module__ and "forward" not in vars(l) and "backward" not in vars(l) for l in self.layers)
+        return own and all(type(l).__module__ == _OWN and "forward" not in vars(l) and "backward" not in vars(l) for l in self.layers)
 
     @contextlib.contextmanager
     def _branched(self):

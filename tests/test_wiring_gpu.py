@@ -50,3 +50,49 @@ def test_a_skipped_layer(kinds, skip):
         assert torch.equal(o, l.output), type(l).__name__
         for a, b in zip(grads, (getattr(l, "dweights", None), getattr(l, "dbiases", None))):
             assert float((a - b).norm()) <= 1e-6 * float(b.norm()) + 1e-7, type(l).__name__       # (dB's order differs, fp32)
+
+
+def _inference_network(kinds):
+    """`network` with a head that fits what the Flatten in front of it reads."""
+    from aether_ml_b200 import layers as L
+    m = network(kinds)
+    m.layers[kinds.split().index("head")].__dict__.update(L.Layer_Dense(8 * 8 * 16, 10).__dict__)
+    m.finalize()
+    return m
+
+
+def _batch_by_batch(m, X, batch):
+    import torch
+    return torch.vstack([m.forward(X[k:k + batch], training=False).clone() for k in range(0, len(X), batch)])
+
+
+@pytest.mark.parametrize("source", [0, 1, 2])
+def test_inference_of_several_batches_with_a_layer_that_reads_an_earlier_one(source):
+    """The Flatten reads the output of the convolution, the Batch_Norm or the activation, past the layers that would have run in one pass."""
+    import torch
+    m = _inference_network("conv bn relu pool flat head softmax")
+    m.layers[4].prev = m.layers[source]
+    X = torch.randn((90, 8, 8, 16), generator=torch.Generator(device="cuda").manual_seed(2), device="cuda")
+    assert torch.equal(m.predict(X, batch_size=16), _batch_by_batch(m, X, 16))
+
+
+def test_inference_of_several_batches_with_a_layer_of_the_callers():
+    """It keeps a convolution's output as its own input, whatever it is handed."""
+    import torch
+    from aether_ml_b200 import layers as L
+    m = _inference_network("conv bn relu pool flat head softmax")
+
+    class Skip(L.Flatten):
+        def forward(self, inputs, training):
+            return super().forward(self.source.output, training)
+    m.layers[4].__class__ = Skip
+    m.layers[4].source = m.layers[0]
+    m.finalize()
+    X = torch.randn((90, 8, 8, 16), generator=torch.Generator(device="cuda").manual_seed(3), device="cuda")
+    assert torch.equal(m.predict(X, batch_size=16), _batch_by_batch(m, X, 16))
+    del m.layers[4].source
+    m.layers[4].__class__ = L.Flatten                       # the same with a patched instance
+    inner, conv = m.layers[4].forward, m.layers[0]
+    m.layers[4].forward = lambda inputs, training: inner(conv.output, training)
+    m.finalize()
+    assert torch.equal(m.predict(X, batch_size=16), _batch_by_batch(m, X, 16))
