@@ -6,6 +6,8 @@
 #include <math.h>
 #include <string.h>
 
+#include <type_traits>
+
 #include "common.cuh"
 #include "sm100_ptx.cuh"
 #include "tc_host.cuh"
@@ -333,13 +335,15 @@ static int dx_few_tile(const AetherConvDesc& d, const float* dy, const float* w,
 }
 
 // ---------------------------------------------------------------------------------- any filter and stride
-// Eight lanes share a column of four input pixels and take four output channels each, so a warp's load of dy is four whole 128-byte lines.
+// Eight lanes share a column of four input pixels and take four output channels each, so a warp's load of dy is four whole 128-byte lines, and one load
+// serves FB rows of the filter, which sit in registers: all of a filter of three or five rows at row stride 1, else one at a time.  (us, one at a time / all:
+// 128 x 32x32 3->32 3x5 34.4 / 27.4, 5x3 35.0 / 25.5, 3x3 at column stride 2 16.5 / 13.8, 64 x 64x64 3->64 5x1 48.1 / 34.7, 6 x 21x21 1->32 3x5 7.3 / 4.9.)
 // Sums are pairs over even and odd channels, the lanes' sums meet in a fixed halving exchange.  A stride splits the input pixels into
 // sH * sW classes (blockIdx.z) that each see only the taps that reach them.
 static constexpr int DXF_PV = 4;                        // pixels (rows) per thread
 static constexpr int DXF_LANES = 8;                     // lanes that share them
 
-template <int CIN, bool VEC>
+template <int CIN, int FB, bool VEC>
 __global__ void __launch_bounds__(256, 2) dx_few_kernel(const float* __restrict__ dy, const float* __restrict__ w, float* __restrict__ dx,
                                                          int S, int H, int W, int Cout, int fH, int fW, int sH, int sW, int pH, int pW,
                                                          int Ho, int Wo) {
@@ -379,30 +383,34 @@ __global__ void __launch_bounds__(256, 2) dx_few_kernel(const float* __restrict_
         for (int c = 0; c < CIN; ++c) acc[p][c] = 0ull;
     const float* dys = dy + s * Ho * Wo * Cout;
 #pragma unroll 1
-    for (int ti = 0; ti < nH; ++ti) {
-        const int r0 = a0 + hq - ti;                    // dy row of the first load
+    for (int ti0 = 0; ti0 < nH; ti0 += FB) {            // (FB divides nH)
+        const int r0 = a0 + hq - ti0 - (FB - 1);        // dy row of the first load
 #pragma unroll 1
         for (int tj = 0; tj < nW; ++tj) {
             const int wo = b + wq - tj;
             if (!live || (unsigned)wo >= (unsigned)Wo) continue;
 #pragma unroll 1
             for (int d = sub * 4; d < Cout; d += DXF_LANES * 4) {
-                ulonglong2 k[CIN], v[PV];
+                ulonglong2 k[FB][CIN], v[PV + FB - 1];
 #pragma unroll
-                for (int r = 0; r < PV; ++r) {
+                for (int r = 0; r < PV + FB - 1; ++r) {
                     const int ho = r0 + r;
                     v[r] = (unsigned)ho < (unsigned)Ho ? dxf_load4<VEC>(dys + ((long long)ho * Wo + wo) * Cout + d, Cout - d) : make_ulonglong2(0ull, 0ull);
                 }
-                const float* wt = w + ((long long)(ph + ti * sH) * fW + pw + tj * sW) * CIN * Cout + d;
+                const float* wt = w + ((long long)(ph + ti0 * sH) * fW + pw + tj * sW) * CIN * Cout + d;
 #pragma unroll
-                for (int c = 0; c < CIN; ++c) k[c] = dxf_load4<VEC>(wt + (long long)c * Cout, Cout - d);
+                for (int t = 0; t < FB; ++t)
+#pragma unroll
+                    for (int c = 0; c < CIN; ++c) k[t][c] = dxf_load4<VEC>(wt + ((long long)t * sH * fW * CIN + c) * Cout, Cout - d);
 #pragma unroll
                 for (int p = 0; p < PV; ++p)
 #pragma unroll
-                    for (int c = 0; c < CIN; ++c) {
-                        dxf_fma2(acc[p][c], v[p].x, k[c].x);
-                        dxf_fma2(acc[p][c], v[p].y, k[c].y);
-                    }
+                    for (int t = 0; t < FB; ++t)
+#pragma unroll
+                        for (int c = 0; c < CIN; ++c) {
+                            dxf_fma2(acc[p][c], v[p + FB - 1 - t].x, k[t][c].x);
+                            dxf_fma2(acc[p][c], v[p + FB - 1 - t].y, k[t][c].y);
+                        }
             }
         }
     }
@@ -436,15 +444,18 @@ static int dx_few(const AetherConvDesc& d, const float* dy, const float* w, floa
     conv_out_hw(d, Ho, Wo);
     // (1x1 filters read each value of dy once, whichever way: 64 x 40x40 3->64 9.0 us through registers, 9.4 through shared memory.  3x3 layers of a few
     // microseconds wait for the host, which takes 0.8 us longer with two tensor maps to encode: 6 x 21x21 1->32, both passes, 16.4 / 17.3; not with more
-    // input channels or several chunks of output channels, tap by tap: 5 x 8x8 3->80 11 against 4.  Strips and tiles are counted in 32 bits.)
-    const bool short_call = CIN == 1 && d.fH == 3 && d.Cout <= 32 && 1LL * d.S * Ho * Wo * d.Cout <= 1 << 17;
+    // input channels or several chunks of output channels: 5 x 8x8 3->80 11 against 4, one filter row at a time.  Channel counts without tensor maps wait for
+    // nothing: 100 x 28x28 1->1 12.9 us through registers, 8.5 so.  Strips and tiles are counted in 32 bits.)
+    const bool short_call = CIN == 1 && d.fH == 3 && d.Cout % 4 == 0 && d.Cout <= 32 && 1LL * d.S * Ho * Wo * d.Cout <= 1 << 17;
     if (!short_call && d.sH == 1 && d.sW == 1 && d.fH == d.fW && (d.fH == 3 || d.fH == 5) && 1LL * d.S * d.H * d.W < 0x7fffffffLL)
         return d.fH == 3 ? dx_few_tile<CIN, 3>(d, dy, w, dx, Ho, Wo, st) : dx_few_tile<CIN, 5>(d, dy, w, dx, Ho, Wo, st);
     const bool vec = d.Cout % 4 == 0 && aligned16(dy) && aligned16(w);
     const int MH = ceil_div(d.H, d.sH), MW = ceil_div(d.W, d.sW);            // extent of the largest class
     const long long items = 1LL * d.S * ceil_div(MH, DXF_PV) * MW;
     const dim3 grid((unsigned)((items + 256 / DXF_LANES - 1) / (256 / DXF_LANES)), 1, d.sH * d.sW);
-    launch(vec ? dx_few_kernel<CIN, true> : dx_few_kernel<CIN, false>, grid, 256, 0, st, dy, w, dx, d.S, d.H, d.W, d.Cout, d.fH, d.fW, d.sH, d.sW,
+    const auto pick = [&](auto fb) { return vec ? dx_few_kernel<CIN, decltype(fb)::value, true> : dx_few_kernel<CIN, decltype(fb)::value, false>; };
+    const int rows = d.sH == 1 && (d.fH == 3 || d.fH == 5) ? d.fH : 1;
+    launch(rows == 3 ? pick(std::integral_constant<int, 3>()) : rows == 5 ? pick(std::integral_constant<int, 5>()) : pick(std::integral_constant<int, 1>()), grid, 256, 0, st, dy, w, dx, d.S, d.H, d.W, d.Cout, d.fH, d.fW, d.sH, d.sW,
            d.padH, d.padW, Ho, Wo);
     count_launch();
     return check_launch("dx_few_kernel");

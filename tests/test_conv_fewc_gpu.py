@@ -30,3 +30,20 @@ def test_dx_of_first_layers(shape):
     torch.cuda.synchronize()
     want, _, _ = O.conv_backward(x.astype(np.float64), w.astype(np.float64), dy.astype(np.float64), st, pad)
     assert O.rel_l2(dx.cpu().numpy(), want) <= 1e-5
+
+
+@pytest.mark.parametrize("S,H,W,Cin,Cout,f,st", [(3, 9, 11, 3, 32, (3, 1), (1, 1)), (2, 13, 12, 1, 36, (3, 5), (1, 1)), (2, 11, 10, 4, 33, (5, 3), (1, 1)), (4, 10, 21, 2, 16, (3, 3), (1, 2)),
+                                                 (1, 17, 9, 3, 260, (5, 5), (1, 3)), (2, 8, 15, 1, 7, (5, 2), (1, 1)), (2, 9, 9, 3, 24, (3, 3), (2, 1)), (3, 28, 28, 1, 1, (3, 3), (1, 1))])
+def test_dx_of_filters_that_are_not_square(S, H, W, Cin, Cout, f, st):
+    """Filters of three and five rows at row stride 1, whatever their width and the columns' stride: their rows in one pass."""
+    import torch
+    from aether_ml_b200 import layers
+    rng = np.random.default_rng(S + 7 * Cout)
+    x = rng.standard_normal((S, H, W, Cin)).astype(np.float32)
+    layer = layers.Conv_Layer((H, W, Cin), Cout, f, st, "valid", math_mode="fp32")
+    y = layer.forward(x, True)
+    dy = rng.standard_normal(tuple(y.shape)).astype(np.float32)
+    dx = layer.backward(dy)
+    torch.cuda.synchronize()
+    want, _, _ = O.conv_backward(x.astype(np.float64), layer.filter_weights.cpu().numpy().astype(np.float64), dy.astype(np.float64), st, "valid")
+    assert O.rel_l2(dx.cpu().numpy(), want) <= 1e-5
