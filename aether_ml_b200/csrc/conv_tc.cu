@@ -1363,10 +1363,12 @@ static int igemm_pair_grid(long long m_tiles, int n_tiles_n, bool stats) {
 }
 
 // Column tile: the one whose rounds of units are through first.  What a 128-byte chunk of K takes, in clocks, is its operands' way from L2 (128 rows of
-// pixels, some 63 bytes per clock and SM) and the filter rows'; a tile that overhangs the channels costs what it copies, several tiles copy the pixels again.
-// (Only widths that divide the channels made 192 channels three tiles of 64 and TF32's 160 five of 32.  Before / now, us: bf16 256 x 8x8 256->192 forward
-// 22.0 / 13.6, 192->160 17.6 / 11.2, 100 x 11x11 192->256 dX 21.4 / 13.2; TF32 150 x 16x16 160->96 forward and dX 54 / 29, 53 / 27, 100 x 12x12 224->180
-// dX 85 / 38.  Few tiles are narrow: 128 rows of a Dense layer 2048 -> 256 15.7 in one tile, 12.3 in eight; 64 images 7x7 128 -> 256 12.0 / 9.2.)
+// pixels and the filter rows'); a unit's columns are stored while the next one's products run, so the longer of both counts, and a little of the other.  A tile
+// that overhangs the channels costs what it copies, several tiles copy the pixels again.  The figures are fitted to every width's times over 1265 shapes of one
+// and nine taps in both modes (K 16 to 2304, 64 to 3256 columns, 100 to 128000 rows): the choice is within 7 % of the fastest width everywhere, 0.2 % in the mean.
+// (Without the stores, 3.3 %, up to 53 %: 1364 x 112->3256 15.3 us where 7.9 are there; widths that divide the channels only, 3.9 % in bf16, 9.7 % in TF32.  Before /
+// now, us: bf16 256 x 8x8 256->192 forward 22.0 / 13.6, 192->160 17.6 / 11.2; TF32 150 x 16x16 160->96 54 / 29.  Few tiles are narrow: 128 rows of a Dense layer
+// 2048 -> 256 15.7 in one tile, 12.3 in eight.)
 static int pick_nt(int n_padded, long long m_tiles, int kiters, bool pairs = true) {
     static const int widths[6] = {256, 192, 128, 96, 64, 32};
     const int sms = num_sms();
@@ -1378,8 +1380,8 @@ static int pick_nt(int n_padded, long long m_tiles, int kiters, bool pairs = tru
         if (cols > 1 && nt > 128 && n_padded % nt) continue;          // (a filter tile reads on into the next tap's rows, a wide one by much)
         const bool pair = pairs && nt >= 128 && igemm_use_pairs(m_tiles, nt, cols);
         const long long units = pair ? (m_tiles + 1) / 2 * cols : m_tiles * cols, slots = pair ? sms / 2 : sms;
-        const double chunk = 260.0 + (pair ? 1.0 : 2.0) * nt;
-        const double cost = (double)((units + slots - 1) / slots) * kiters * chunk + 8.0 * nt;
+        const double mma = kiters * (170.0 + (pair ? 0.95 : 1.4) * nt), store = pair ? 1900.0 + 16.0 * nt : 400.0 + 11.0 * nt;
+        const double cost = (double)((units + slots - 1) / slots) * (mma > store ? mma : store) + 0.4 * (mma > store ? store : mma);
         if (cost < best_cost - 1e-9) { best_cost = cost; best = nt; }
     }
     return best;
