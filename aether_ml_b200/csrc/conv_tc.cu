@@ -1256,17 +1256,21 @@ static TcPlan compute_plan(const AetherConvDesc& d) {
             pl.dw_pair = false;
             decompose(1, 0);
         } else {
-            // M groups per CTA: a tile of pixels takes some 0.72 us for each, whether or not they share dy's half, so the count is chosen by how evenly the
-            // groups and pixels divide and by the partials (written, and read again).  One group instead of two, dW with its reduction, us: 256 x 8x8
-            // 256->256 28.8 -> 21.9, 512 x 16x16 128->256 68.7 -> 61.5, 4096 x 8x8 256->512 414 -> 376, 64 x 9x9 256->256 5x5 33 -> 28, TF32 256 x
-            // 16x16 128->128 48.2 -> 43.9.
+            // M groups per CTA: the count is chosen by how evenly the groups and pixels divide and by the partials (written, and read again).  In bf16 a tile of
+            // pixels takes some 0.72 us for each, whether or not they share dy's half; in TF32, bound by the operands' way, sharing counts, more so where rows
+            // of channels are no multiple of 128 bytes.  One group instead of two, dW with its reduction, us: 256 x 8x8 256->256 28.8 -> 21.9, 512 x 16x16
+            // 128->256 68.7 -> 61.5, 4096 x 8x8 256->512 414 -> 376, 64 x 9x9 256->256 5x5 33 -> 28, TF32 256 x 16x16 128->128 48.2 -> 43.9; but TF32 81 x 104x12
+            // 148->236 271 with one, 209 with three, 31 x 81x28 292->236 5x5 713 / 566.  Over 1659 shapes in bf16 and 2437 in TF32 the choice is at most 5 and 18 % behind
+            // the best count, 0.1 and 0.8 % in the mean; with bf16's figure TF32 is up to 52 and 5.1 %, with as many groups as TMEM holds bf16 up to 84 %, TF32 63 %.
             const double dw_us = 2.0 * pl.dw_U * UC * pl.Cout_p * 4.0 / 4e6;        // as below
+            const double tile = !pl.tf32 ? 0.0 : d.Cout % UC ? 0.13 : 0.07, group = !pl.tf32 ? 0.72 : d.Cin % UC ? 0.52 : 0.45;
             double best = 1e30;
             int gpc = 0;
             for (int g = 512 / (pl.dw_nt * 2); g >= 1; --g) {
                 const int splits = decompose(2, g);
                 if (splits < 1) continue;
-                const double cost = (double)((ptiles + splits - 1) / splits) * pl.dw_gpc * 0.72 + pl.dw_gpc + (splits > 1 ? splits * dw_us : 0.0);
+                const double cost = (double)((ptiles + splits - 1) / splits) * (tile + pl.dw_gpc * group) + (pl.tf32 ? 0.2 : 1.0) * pl.dw_gpc +
+                                    (splits == 1 ? 0.0 : pl.tf32 ? 1.9 + 0.42 * splits * dw_us : splits * dw_us);
                 if (cost < best - 1e-9) { best = cost; gpc = g; }
             }
             pl.dw_splits = decompose(2, gpc);

@@ -1,5 +1,5 @@
 """Filter gradients at the image heights where strips are divided differently (13 to 24 rows, and heights that no strip divides) and with one group of
-rows per pair of CTAs (256 output channels), against float64 on operands rounded as the kernels round them.  Sums of n fp32 products in
+rows per pair of CTAs (256 output channels; TF32: one, two and four, channels that fill no row of 128 bytes), against float64 on operands rounded as the kernels round them.  Sums of n fp32 products in
 any order are within n roundings of the sum of absolute values, of which tcgen05 truncates each: n * 2^-23."""
 import ctypes
 
@@ -12,7 +12,8 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("S,H,W,Cin,Cout,f,mode", [(300, 16, 16, 64, 64, 3, "bf16"), (200, 13, 13, 64, 128, 3, "bf16"), (150, 15, 14, 128, 128, 3, "bf16"), (120, 18, 18, 96, 160, 3, "bf16"),
                                                    (90, 24, 24, 32, 64, 5, "bf16"), (60, 23, 21, 128, 64, 3, "bf16"), (100, 17, 30, 64, 64, 3, "bf16"), (200, 13, 13, 128, 256, 3, "bf16"),
-                                                   (100, 25, 24, 128, 256, 3, "bf16"), (256, 8, 8, 256, 256, 3, "bf16"), (64, 9, 9, 256, 256, 5, "bf16"), (128, 16, 16, 128, 128, 3, "tf32")])
+                                                   (100, 25, 24, 128, 256, 3, "bf16"), (256, 8, 8, 256, 256, 3, "bf16"), (64, 9, 9, 256, 256, 5, "bf16"), (128, 16, 16, 128, 128, 3, "tf32"),
+                                                   (200, 13, 13, 96, 116, 3, "tf32"), (100, 16, 16, 148, 236, 3, "tf32"), (40, 20, 20, 64, 500, 5, "tf32"), (60, 13, 13, 292, 236, 5, "tf32")])
 def test_filter_gradient(S, H, W, Cin, Cout, f, mode):
     import torch
     lib, pad = _lib.lib(), (f - 1) // 2
