@@ -414,8 +414,8 @@ struct HaloGeom {
 static constexpr int HALO_SMEM_MAX = 232448;
 
 // Decides whether the halo kernel takes the problem and, if so, its tiling.
-static bool halo_geometry(bool tf32, int in_C, int S, int taps, int out_C, int out_H, int out_W, int n_padded, int fH,
-                          int fW, HaloGeom& g) {
+static bool halo_geometry(bool tf32, int in_C, int S, int taps, int out_C, int out_H, int out_W, int n_padded, int tap_n, long long tap_tiles,
+                          int fH, int fW, HaloGeom& g) {
     const int KC = tf32 ? 32 : 64;
     g.Wp = out_W + fW - 1;
     if (n_padded > 256 || n_padded % (16 * HALO_EPI_PARTS) || out_C % 4) return false;
@@ -425,15 +425,19 @@ static bool halo_geometry(bool tf32, int in_C, int S, int taps, int out_C, int o
     if (g.BH + fH - 1 > 256) return false;
     g.tiles_h = ceil_div(out_H, g.BH);
     if (1LL * g.tiles_h * S > 0x3fffffffLL) return false;
-    // Useful fraction of the 128 accumulator rows, including the ragged last strip of each image, that makes up for the per-tap kernel's copies: less of
-    // it where those weigh more (few columns; TF32 of one chunk of channels).  Per-tap / this kernel, us at 40 GFLOP: bf16 64->64 15x15 (0.59) 78 / 70,
-    // 13x13 (0.66) 77 / 62, 16x16 (0.67) 75 / 61, 31x31 (0.68) 75 / 65, 44x44 (0.69) 79 / 65, 64->128 16x16 55 / 51, 44x44 59 / 52, but 12x12 (0.56) 51 / 55;
-    // 64->192 13x13 11.5 / 15.8 (6 GFLOP), 19x19 (0.71) 11.5 / 15.8, 26x26 (0.75) 52 / 55, 28x28 (0.88) 55 / 47; TF32 32->64 13x13 147 / 116, 16x16 144 /
-    // 119, 64->64 44x44 129 / 113, 64->128 16x16 17.0 / 18.2 (6 GFLOP).
-    const double eff = (double)out_H * out_W / ((double)g.tiles_h * 128.0);
-    const double least = tf32 ? (in_C <= 32 ? 0.58 : n_padded <= 64 ? 0.66 : 0.70) : n_padded <= 128 ? 0.58 : 0.72;
-    if (eff < least) return false;
     g.kchunks = ceil_div(in_C, KC);
+    // Useful fraction of the 128 accumulator rows, including the ragged last strip of each image.  Down to 0.58 of it the kernel can be ahead of the per-tap
+    // one, whose copies it saves, where both take many rounds: bf16 64->64, 40 GFLOP, 13x13 (0.66) 77 us per tap, 62 here, 16x16 (0.67) 75 / 61, 31x31 (0.68) 75 / 65.
+    // Small layers and many columns are not: 3 x 31x42 28->28 5x5 9.7 / 10.7, TF32 64 x 15x17 64->64 7.3 / 9.7, 12x12 64->128 51 / 55, 64->192 13x13
+    // 11.5 / 15.8.  So the rounds' clocks decide, of either kernel the longer of products and stores and a part of the other (fitted to 305 shapes below 0.72: at
+    // most 20 % behind the faster kernel, 0.7 % in the mean; by the fraction alone 32 and 5 %).
+    const double eff = (double)out_H * out_W / ((double)g.tiles_h * 128.0);
+    if (eff < 0.58) return false;
+    if (eff < (!tf32 && n_padded > 128 ? 0.72 : 0.70)) {
+        const double mma = taps * g.kchunks * (93.0 + n_padded), store = 270.0 + 7.0 * n_padded;
+        const double rounds = (double)((1LL * g.tiles_h * S + num_sms() - 1) / num_sms());
+        if (1100.0 + rounds * (mma > store ? mma : store) + 0.6 * (mma > store ? store : mma) >= per_tap_clocks(tap_n, tap_tiles, taps * g.kchunks)) return false;
+    }
     g.region_rows = (g.BH + fH - 1) * g.Wp;
     g.region_stride = (int)align_up((size_t)g.region_rows * 128, 1024);
     const long long total = 1LL * g.tiles_h * S;
@@ -469,21 +473,21 @@ static bool halo_geometry(bool tf32, int in_C, int S, int taps, int out_C, int o
 // Number of (count, mean, M2) partial blocks the kernel writes per output channel when asked for statistics
 // (two per CTA), or 0 when the halo kernel does not take this problem.
 long long halo_igemm_stats_blocks(bool tf32, int in_C, int S, int taps, int out_C, int out_H, int out_W, int n_padded,
-                                  int fH, int fW) {
+                                  int tap_n, long long tap_tiles, int fH, int fW) {
     HaloGeom g;
-    if (!halo_geometry(tf32, in_C, S, taps, out_C, out_H, out_W, n_padded, fH, fW, g)) return 0;
+    if (!halo_geometry(tf32, in_C, S, taps, out_C, out_H, out_W, n_padded, tap_n, tap_tiles, fH, fW, g)) return 0;
     return 2LL * g.grid;       // two rows per CTA (stats_epilogue.cuh)
 }
 
 int run_halo_igemm(bool tf32, const void* in, int in_C, int in_H, int in_W, int S, const void* wmat, int w_inner,
-                   int rows_per_tap, int taps, float* out, int out_C, int out_H, int out_W, int n_padded, int fH, int fW,
+                   int rows_per_tap, int taps, float* out, int out_C, int out_H, int out_W, int n_padded, int tap_n, long long tap_tiles, int fH, int fW,
                    int padT, int padL, int flip, int k_real, const float* bias, float* stats, int prof_kind, cudaStream_t st,
                    bool* used) {
     *used = false;
     const int elt = tf32 ? 4 : 2;
     const int KC = 128 / elt;
     HaloGeom g;
-    if (!halo_geometry(tf32, in_C, S, taps, out_C, out_H, out_W, n_padded, fH, fW, g)) return AE_OK;
+    if (!halo_geometry(tf32, in_C, S, taps, out_C, out_H, out_W, n_padded, tap_n, tap_tiles, fH, fW, g)) return AE_OK;
     const int Wp = g.Wp, BH = g.BH, tiles_h = g.tiles_h, kchunks = g.kchunks, w_bytes = g.w_bytes;
     const int region_rows = g.region_rows, region_stride = g.region_stride, stages = g.stages, fixed = g.fixed;
     const int smem_max = HALO_SMEM_MAX;

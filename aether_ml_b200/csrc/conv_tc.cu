@@ -1373,13 +1373,15 @@ static int igemm_pair_grid(long long m_tiles, int n_tiles_n, bool stats) {
 // (Without the stores, 3.3 %, up to 53 %: 1364 x 112->3256 15.3 us where 7.9 are there; widths that divide the channels only, 3.9 % in bf16, 9.7 % in TF32.  Before /
 // now, us: bf16 256 x 8x8 256->192 forward 22.0 / 13.6, 192->160 17.6 / 11.2; TF32 150 x 16x16 160->96 54 / 29.  Few tiles are narrow: 128 rows of a Dense layer
 // 2048 -> 256 15.7 in one tile, 12.3 in eight.)
-static int pick_nt(int n_padded, long long m_tiles, int kiters, bool pairs = true) {
+static int pick_nt(int n_padded, long long m_tiles, int kiters, bool pairs = true, double* clocks = nullptr) {
     static const int widths[6] = {256, 192, 128, 96, 64, 32};
     const int sms = num_sms();
-    if (m_tiles * ceil_div(n_padded, 32) <= sms) return 32;           // (one round of the shortest)
+    const bool short_one = m_tiles * ceil_div(n_padded, 32) <= sms;   // (one round of the shortest)
+    if (short_one && !clocks) return 32;
     int best = 32;
     double best_cost = 1e300;
     for (int nt : widths) {
+        if (short_one && nt > 32) continue;
         const int cols = ceil_div(n_padded, nt);
         if (cols > 1 && nt > 128 && n_padded % nt) continue;          // (a filter tile reads on into the next tap's rows, a wide one by much)
         const bool pair = pairs && nt >= 128 && igemm_use_pairs(m_tiles, nt, cols);
@@ -1388,7 +1390,13 @@ static int pick_nt(int n_padded, long long m_tiles, int kiters, bool pairs = tru
         const double cost = (double)((units + slots - 1) / slots) * (mma > store ? mma : store) + 0.4 * (mma > store ? store : mma);
         if (cost < best_cost - 1e-9) { best_cost = cost; best = nt; }
     }
+    if (clocks) *clocks = best_cost;
     return best;
+}
+double per_tap_clocks(int n_padded, long long m_tiles, int kiters) {
+    double c;
+    pick_nt(n_padded, m_tiles, kiters, true, &c);
+    return c;
 }
 
 template <bool TF32, int NT, bool STATS, bool PAIR, bool ACT = false, int RB = 128, bool POOLED = false, bool SPLIT = false>
@@ -1475,7 +1483,7 @@ static int run_igemm(bool tf32, const void* in, int in_C, int in_H, int in_W, in
         const int padT = sgn > 0 ? -off_h : fH - 1 - off_h;
         const int padL = sgn > 0 ? -off_w : fW - 1 - off_w;
         int rc0 = run_halo_igemm(tf32, in, in_C, in_H, in_W, S, wmat, w_inner, rows_per_tap, taps, out, out_C, out_H, out_W,
-                                 halo_n(out_C, n_padded), fH, fW, padT, padL, sgn > 0 ? 0 : 1, k_real, bias, stats,
+                                 halo_n(out_C, n_padded), n_padded, til.total(), fH, fW, padT, padL, sgn > 0 ? 0 : 1, k_real, bias, stats,
                                  sgn > 0 ? PK_IGEMM_FWD : PK_IGEMM_DX, st, &used);
         if (rc0 || used) return rc0;
     }
@@ -1549,7 +1557,7 @@ long long tc_conv_stats_blocks(const AetherConvDesc& d) {
     if (!tc_conv_eligible(d)) return 0;
     const TcPlan& pl = make_plan(d);
     const long long hb = halo_igemm_stats_blocks(pl.tf32, pl.tf32 ? d.Cin : pl.Cin_p, d.S, pl.taps, d.Cout, pl.Ho, pl.Wo,
-                                                 halo_n(d.Cout, pl.Cout_p), d.fH, d.fW);
+                                                 halo_n(d.Cout, pl.Cout_p), pl.Cout_p, pl.til_out.total(), d.fH, d.fW);
     if (hb > 0) return hb;
     // per-tap kernel: two rows per CTA group (the CTAs of one set of pixel tiles)
     const int nt = pick_nt(pl.Cout_p, pl.til_out.total(), pl.taps * ceil_div(pl.tf32 ? d.Cin : pl.Cin_p, pl.KC));

@@ -52,15 +52,18 @@ int make_map(CUtensorMap* m, const void* base, CUtensorMapDataType dt, int rank,
 // Row-major matrix (inner = K elements contiguous, `rows` rows), box (box_k, box_rows); 128-byte swizzle unless told otherwise.
 int make_map_2d(CUtensorMap* m, const void* base, CUtensorMapDataType dt, int elt, int inner, long long rows, int box_k,
                 int box_rows, CUtensorMapSwizzle swz = CU_TENSOR_MAP_SWIZZLE_128B);
-// Halo-reuse kernel (conv_halo.cu): launches and sets *used when the problem fits it, else leaves *used false.
+// What the per-tap kernel (conv_tc.cu) takes for a product, in clocks: padded columns, tiles of 128 pixels, 128-byte chunks of K over all taps.
+double per_tap_clocks(int n_padded, long long m_tiles, int kiters);
+// Halo-reuse kernel (conv_halo.cu): launches and sets *used when the problem fits it, else leaves *used false.  tap_n, tap_tiles: the per-tap kernel's
+// padded columns and tiles of pixels.
 int run_halo_igemm(bool tf32, const void* in, int in_C, int in_H, int in_W, int S, const void* wmat, int w_inner,
-                   int rows_per_tap, int taps, float* out, int out_C, int out_H, int out_W, int n_padded, int fH, int fW,
+                   int rows_per_tap, int taps, float* out, int out_C, int out_H, int out_W, int n_padded, int tap_n, long long tap_tiles, int fH, int fW,
                    int padT, int padL, int flip, int k_real, const float* bias, float* stats, int prof_kind, cudaStream_t st,
                    bool* used);
 // Partial-statistics blocks ([block][3][out_C]: count, mean, M2) the halo kernel writes when `stats` is given; 0 when
 // the halo kernel does not take the problem.
 long long halo_igemm_stats_blocks(bool tf32, int in_C, int S, int taps, int out_C, int out_H, int out_W, int n_padded,
-                                  int fH, int fW);
+                                  int tap_n, long long tap_tiles, int fH, int fW);
 
 // Halo-reuse dW kernel (conv_halo_dw.cu), bf16 shadows with 64-channel blocks.  `part` must have room for
 // max_splits split slices; the split count actually used is returned in *splits_out.
