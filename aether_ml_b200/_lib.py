@@ -61,6 +61,7 @@ SIGNATURES = {
     "aether_conv2d_fwd_ex": (_I, [_D, _P, _P, _P, _P, _P, _SZ, _P, _SZ, _I, _P]),
     "aether_conv2d_filter_copies": (_I, [_D, _P, _P, _SZ, _P]),
     "aether_conv2d_pool_supported": (_I, [_D]),
+    "aether_conv2d_pool_faster": (_I, [_D]),
     "aether_conv2d_pool_fwd": (_I, [_D] + [_P] * 7 + [_F, _F, _P, _P, _I, _P, _SZ, _I, _P]),
     "aether_conv2d_act_fwd": (_I, [_D, _P, _P, _P, _P, _P, _F, _P, _I, _P, _SZ, _I, _P]),
     "aether_head_supported": (_I, [_D]),

@@ -255,6 +255,10 @@ extern "C" int aether_conv2d_pool_supported(const AetherConvDesc* d) {
     return tc_conv_pool_eligible(*d) || (!tc_conv_eligible(*d) && first_tc_eligible(*d) && Ho % 2 == 0 && Wo % 2 == 0);
 }
 
+extern "C" int aether_conv2d_pool_faster(const AetherConvDesc* d) {
+    return aether_conv2d_pool_supported(d) && (!tc_conv_eligible(*d) || tc_conv_pool_faster(*d));       // (first layers: 1.5 to 2.3 times as fast)
+}
+
 extern "C" int aether_conv2d_pool_fwd(const AetherConvDesc* d, const float* x, const float* w, const float* b, const float* gamma, const float* beta,
                                       const float* running_mean, const float* running_var, float eps, float alpha, float* pooled, void* operand_copy,
                                       int copy_ld, void* ws, size_t ws_bytes, int flags, void* stream) {

@@ -153,6 +153,7 @@ struct ActEpilogue {
 int tc_conv_fwd(const AetherConvDesc& d, const float* x, const float* w, const float* b, float* y, float* stats, void* ws,
                 size_t ws_bytes, int flags, cudaStream_t st, const ActEpilogue* act = nullptr, bool* act_done = nullptr);
 bool tc_conv_pool_eligible(const AetherConvDesc& d);
+bool tc_conv_pool_faster(const AetherConvDesc& d);
 int tc_conv_fwd_pool(const AetherConvDesc& d, const float* x, const float* w, const float* b, const PoolEpilogue& pool, void* ws, size_t ws_bytes, int flags,
                      cudaStream_t st);
 int tc_conv_filter_copies(const AetherConvDesc& d, const float* w, void* ws, size_t ws_bytes, cudaStream_t st);

@@ -408,6 +408,7 @@ __global__ void __launch_bounds__(HALO_THREADS, 1) halo_conv_kernel(const __grid
 // Decides whether the halo kernel takes this problem; if so launches it and sets *used.
 struct HaloGeom {
     int Wp, BH, tiles_h, kchunks, w_bytes, region_rows, region_stride, stages, fixed;
+    double clocks;  // what it takes, in the measure of per_tap_clocks
     bool pair;      // CTA pairs: w_bytes is then the half filter each CTA keeps
     int grid;       // CTAs (2 x pairs)
 };
@@ -433,11 +434,10 @@ static bool halo_geometry(bool tf32, int in_C, int S, int taps, int out_C, int o
     // most 20 % behind the faster kernel, 0.7 % in the mean; by the fraction alone 32 and 5 %).
     const double eff = (double)out_H * out_W / ((double)g.tiles_h * 128.0);
     if (eff < 0.58) return false;
-    if (eff < (!tf32 && n_padded > 128 ? 0.72 : 0.70)) {
-        const double mma = taps * g.kchunks * (93.0 + n_padded), store = 270.0 + 7.0 * n_padded;
-        const double rounds = (double)((1LL * g.tiles_h * S + num_sms() - 1) / num_sms());
-        if (1100.0 + rounds * (mma > store ? mma : store) + 0.6 * (mma > store ? store : mma) >= per_tap_clocks(tap_n, tap_tiles, taps * g.kchunks)) return false;
-    }
+    const double mma = taps * g.kchunks * (93.0 + n_padded), store = 270.0 + 7.0 * n_padded;
+    const double rounds = (double)((1LL * g.tiles_h * S + num_sms() - 1) / num_sms());
+    g.clocks = 1100.0 + rounds * (mma > store ? mma : store) + 0.6 * (mma > store ? store : mma);
+    if (eff < (!tf32 && n_padded > 128 ? 0.72 : 0.70) && g.clocks >= per_tap_clocks(tap_n, tap_tiles, taps * g.kchunks)) return false;
     g.region_rows = (g.BH + fH - 1) * g.Wp;
     g.region_stride = (int)align_up((size_t)g.region_rows * 128, 1024);
     const long long total = 1LL * g.tiles_h * S;
@@ -477,6 +477,11 @@ long long halo_igemm_stats_blocks(bool tf32, int in_C, int S, int taps, int out_
     HaloGeom g;
     if (!halo_geometry(tf32, in_C, S, taps, out_C, out_H, out_W, n_padded, tap_n, tap_tiles, fH, fW, g)) return 0;
     return 2LL * g.grid;       // two rows per CTA (stats_epilogue.cuh)
+}
+
+double halo_igemm_clocks(bool tf32, int in_C, int S, int taps, int out_C, int out_H, int out_W, int n_padded, int tap_n, long long tap_tiles, int fH, int fW) {
+    HaloGeom g;
+    return halo_geometry(tf32, in_C, S, taps, out_C, out_H, out_W, n_padded, tap_n, tap_tiles, fH, fW, g) ? g.clocks : 0.0;
 }
 
 int run_halo_igemm(bool tf32, const void* in, int in_C, int in_H, int in_W, int S, const void* wmat, int w_inner,

@@ -1644,6 +1644,22 @@ bool tc_conv_pool_eligible(const AetherConvDesc& d) {
     conv_out_hw(d, Ho, Wo);
     return tc_conv_eligible(d) && d.math_mode == AETHER_MATH_BF16 && Ho % 2 == 0 && Wo % 2 == 0 && d.Cout <= IGEMM_POOL_CHANNELS;
 }
+// Whether that is ahead of the convolution by itself, which may keep windows or run on pairs and whose boxes fit any image, and the pass over its output.  Clocks of the
+// rounds on either side (pick_nt; a pooled unit stores more slowly), the pass 2700 and 0.55 a KB.  us, pooled / apart: 896 x 16x16 32->64 30.8 / 47, 900 x 16x16
+// 128->256 77 / 117, 128 x 8x8 256->512 31 / 36; but 900 x 18x18 16->16 82 / 33, 900 x 10x10 512->1024 1430 / 767, 128 x 10x10 256->256 34 / 24, 900 x 4x4
+// 256->256 42 / 32.  Over 726 shapes at most 39 % behind the faster way, 0.6 % in the mean; pooled everywhere 145 % and 9 %.
+bool tc_conv_pool_faster(const AetherConvDesc& d) {
+    if (!tc_conv_pool_eligible(d)) return false;
+    const TcPlan& pl = make_plan(d);
+    const int kiters = pl.taps * ceil_div(pl.Cin_p, pl.KC), sms = num_sms();
+    const long long tiles = choose_pool_tiling(d.S, pl.Ho, pl.Wo).total();
+    const int nt = pick_nt(pl.Cout_p, tiles, kiters, false);
+    const double mma = kiters * (210.0 + 1.1 * nt), store = 550.0 + 34.0 * nt;
+    const double one = (double)((tiles * ceil_div(pl.Cout_p, nt) + sms - 1) / sms) * (mma > store ? mma : store) + 0.4 * (mma > store ? store : mma);
+    double two = halo_igemm_clocks(false, pl.Cin_p, d.S, pl.taps, d.Cout, pl.Ho, pl.Wo, halo_n(d.Cout, pl.Cout_p), pl.Cout_p, pl.til_out.total(), d.fH, d.fW);
+    if (two == 0.0) two = per_tap_clocks(pl.Cout_p, pl.til_out.total(), kiters);
+    return one < two + 2700.0 + 0.55e-3 * 4.0 * d.S * pl.Ho * pl.Wo * d.Cout;
+}
 int tc_conv_fwd_pool(const AetherConvDesc& d, const float* x, const float* w, const float* b, const PoolEpilogue& pool, void* ws, size_t ws_bytes, int flags,
                      cudaStream_t st) {
     const TcPlan& pl = make_plan(d);

@@ -64,6 +64,8 @@ int run_halo_igemm(bool tf32, const void* in, int in_C, int in_H, int in_W, int 
 // the halo kernel does not take the problem.
 long long halo_igemm_stats_blocks(bool tf32, int in_C, int S, int taps, int out_C, int out_H, int out_W, int n_padded,
                                   int tap_n, long long tap_tiles, int fH, int fW);
+// What the halo kernel takes for such a problem, in clocks; 0 when it does not take it.
+double halo_igemm_clocks(bool tf32, int in_C, int S, int taps, int out_C, int out_H, int out_W, int n_padded, int tap_n, long long tap_tiles, int fH, int fW);
 
 // Halo-reuse dW kernel (conv_halo_dw.cu), bf16 shadows with 64-channel blocks.  `part` must have room for
 // max_splits split slices; the split count actually used is returned in *splits_out.

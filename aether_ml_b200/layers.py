@@ -310,8 +310,8 @@ class _ConvPlan:
 
     @functools.cached_property
     def pools(self):
-        """Whether the library has a forward call that goes on to the pooled output (aether_conv2d_pool_fwd)."""
-        return bool(lib().aether_conv2d_pool_supported(AetherConvDesc.from_buffer_copy(self.raw)))
+        """Whether a forward call that goes on to the pooled output (aether_conv2d_pool_fwd) is the faster way there."""
+        return bool(lib().aether_conv2d_pool_faster(AetherConvDesc.from_buffer_copy(self.raw)))
 
     def least_ws_bytes(self):
         """The workspace that every call can do with."""

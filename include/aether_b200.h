@@ -159,6 +159,8 @@ int aether_conv2d_filter_copies(const AetherConvDesc* desc, const float* w, void
  * columns are zeroed).  The same numbers as aether_conv2d_fwd_ex followed by aether_chain_fwd give, up to the order of the convolution's sums.
  * bf16 mode, output heights and widths that are even (aether_conv2d_pool_supported); ws as for a forward pass (first layers: not used). */
 int aether_conv2d_pool_supported(const AetherConvDesc* desc);
+/* Whether it is (estimated to be) faster than those two calls: 1 or 0, also where it is not supported. */
+int aether_conv2d_pool_faster(const AetherConvDesc* desc);
 int aether_conv2d_pool_fwd(const AetherConvDesc* desc, const float* x, const float* w, const float* b, const float* gamma, const float* beta,
                            const float* running_mean, const float* running_var, float eps, float alpha, float* pooled, void* operand_copy,
                            int copy_ld, void* ws, size_t ws_bytes, int flags, void* stream);

@@ -64,7 +64,16 @@ def test_refused_where_the_epilogue_does_not_fit():
         assert not lib.aether_conv2d_pool_supported(d)
 
 
-@pytest.mark.parametrize("hw,channels,batch,images", [(32, (32, 64, 128), 128, 1000), (28, (32, 64), 50, 230), (12, (20, 48), 16, 90), (32, (192, 32), 64, 400)])
+def test_taken_where_it_is_faster():
+    """Boxes of windows fill little of 10- and 18-pixel rows; what a whole prediction runs follows from it."""
+    lib = _lib.lib()
+    for S, H, W, Cin, Cout, f, mode, want in [(896, 16, 16, 32, 64, 3, "bf16", 1), (512, 8, 8, 256, 512, 3, "bf16", 1), (300, 14, 14, 32, 64, 3, "bf16", 1), (900, 32, 32, 3, 192, 3, "bf16", 1), (900, 18, 18, 16, 16, 3, "bf16", 0),
+                                              (900, 10, 10, 512, 1024, 3, "bf16", 0), (128, 10, 10, 256, 256, 3, "bf16", 0), (900, 4, 4, 256, 256, 3, "bf16", 0), (896, 16, 16, 32, 64, 3, "tf32", 0), (9, 7, 8, 64, 64, 3, "bf16", 0)]:
+        d = _lib.AetherConvDesc(S, H, W, Cin, Cout, f, f, 1, 1, f // 2, f // 2, _lib.MATH_MODES[mode])
+        assert lib.aether_conv2d_pool_faster(d) == want, (S, H, W, Cin, Cout)
+
+
+@pytest.mark.parametrize("hw,channels,batch,images", [(32, (32, 64, 128), 128, 1000), (28, (32, 64), 50, 230), (12, (20, 48), 16, 90), (32, (192, 32), 64, 400), (20, (32, 64, 32), 60, 900)])
 def test_predictions_are_those_of_single_batches(hw, channels, batch, images):
     """Several batches in one pass (convolutions go on to their pooled outputs) and batch by batch with every layer's arrays."""
     import torch
