@@ -12,6 +12,7 @@
 #include "common.cuh"
 #include "stats_epilogue.cuh"
 #include "tail.cuh"
+#include "tc_host.cuh"
 
 namespace aether {
 
@@ -1071,11 +1072,12 @@ __global__ void __launch_bounds__(256) pool_bwd_tiled_kernel(const float* __rest
             }
         }
         const size_t first = (((size_t)s * H + (size_t)ho * fH) * W + (size_t)wo * fW) * Cv + cv;
+        const int rows = F ? F : min(fH, H - ho * fH), columns = F ? F : min(fW, W - wo * fW);
 #pragma unroll
-        for (int i = 0; i < fH; ++i)
+        for (int i = 0; i < rows; ++i)
 #pragma unroll
-            for (int j = 0; j < fW; ++j) {
-                if (!whole && (ho * fH + i >= H || wo * fW + j >= W)) continue;
+            for (int j = 0; j < columns; ++j) {
+                if (F && !whole && (ho * fH + i >= H || wo * fW + j >= W)) continue;
                 float4 o;
                 if (MAX) {
                     const unsigned char code = (unsigned char)(i * fW + j);
@@ -1584,6 +1586,17 @@ extern "C" int aether_pool_fwd(const float* x, float* y, uint8_t* argmax, int S,
     return check_launch("aether_pool_fwd");
 }
 
+// Whether the way back goes window by window or gathers cell by cell.  A thread writes its window's cells one after the other, 0.12 us each, which takes longer than
+// a thread per cell where the windows are large and few; that one takes 0.87 us and 5.9 ps per element of `total`, the stores 2.4 ps.  (us, windows / cells: 4 x
+// 57x57x64 by 15x17 24 / 3.2, 1 x 100x100x3 by 8x8 6.1 / 2.2, 128 x 32x32x64 by 14x14 14 / 16, 128 x 28x28x61 by 7x7 10 / 42.  Over 324 shapes at most 19 % behind the
+// faster one, 0.4 % in the mean.)  Rows of one piece of 16 bytes are half sectors, which L2 holds until the next cell comes while the array fits: 364 x 201x206x4
+// by 5x5 178 / 112.
+static bool pool_by_windows(int cells, long long windows, long long total, int vec_channels) {
+    if (vec_channels == 4 && total > (128LL << 20) / 16) return false;
+    const double serial = 0.12 * cells * (double)((windows + num_sms() * 2048 - 1) / (num_sms() * 2048)), stores = 2.4e-6 * total;
+    return (serial > stores ? serial : stores) < 0.87 + 5.9e-6 * total;
+}
+
 extern "C" int aether_pool_bwd(const float* dy, const uint8_t* argmax, float* dx, int S, int H, int W, int C, int fH,
                                int fW, int sH, int sW, int kind, void* stream) {
     if (!dy || !dx || (kind == AETHER_POOL_MAX && !argmax)) return set_error(AE_BAD_ARG, "aether_pool_bwd: null pointer");
@@ -1598,7 +1611,7 @@ extern "C" int aether_pool_bwd(const float* dy, const uint8_t* argmax, float* dx
     const int Hc = ceil_div(H, fH), Wc = ceil_div(W, fW);
     const int Cv = vec ? C / 4 : C;
     const long long windows = 1LL * S * Hc * Wc * Cv;
-    if (sH == fH && sW == fW && windows < (1LL << 32) - (1LL << 22)) {
+    if (sH == fH && sW == fW && windows < (1LL << 32) - (1LL << 22) && pool_by_windows(fH * fW, windows, total, vec ? C : 0)) {
         const bool max = kind == AETHER_POOL_MAX;
         const int F = fH == fW && (fH == 2 || fH == 3) ? fH : 0;
         const auto pick = [&](auto v) {

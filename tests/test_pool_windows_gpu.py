@@ -9,7 +9,9 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("C", [4, 5, 61, 128, 1])
-@pytest.mark.parametrize("S,H,W,fH,fW", [(3, 9, 10, 2, 2), (2, 11, 10, 3, 3), (2, 12, 14, 3, 3), (5, 8, 8, 2, 2), (2, 10, 13, 4, 3), (1, 3, 3, 3, 3), (2, 7, 15, 1, 2)])
+@pytest.mark.parametrize("S,H,W,fH,fW", [(3, 9, 10, 2, 2), (2, 11, 10, 3, 3), (2, 12, 14, 3, 3), (5, 8, 8, 2, 2), (2, 10, 13, 4, 3), (1, 3, 3, 3, 3), (2, 7, 15, 1, 2),
+                                           # large windows: few of them cell by cell, many window by window
+                                           (3, 29, 30, 14, 9), (1, 60, 51, 15, 17), (40, 41, 50, 4, 3), (64, 43, 50, 14, 9), (96, 33, 31, 8, 8)])
 @pytest.mark.parametrize("kind", ["max", "average"])
 def test_windows_that_leave_cells_over(C, S, H, W, fH, fW, kind):
     import torch
