@@ -421,7 +421,7 @@ extern "C" int aether_conv2d_bwd_ex(const AetherConvDesc* d, const float* x, con
         dx = nullptr;
     }
     if (dx && (rc = generic_conv_bwd_data(*d, dy, w, dx, ws, ws_bytes, st))) return rc;
-    if (dw && first_tc_bwd_eligible(*d) && (dy_ready || !first_fp32_dw_route(*d) || !first_fp32_dw_faster(*d)))
+    if (dw && first_tc_bwd_eligible(*d) && (dy_ready || !first_fp32_dw_faster(*d) || !first_fp32_dw_route(*d)))
         return first_tc_bwd_filter(*d, x, dy, dw, db, ws, ws_bytes, dy_ready ? dy_colsum_rows : 0, st);
     if (dw && first_fp32_dw_route(*d)) return first_fp32_bwd_filter(*d, x, dy, dw, db, ws, ws_bytes, st);
     if ((dw || db) && smallc_conv_eligible(*d) && (!db || aligned16(db)))

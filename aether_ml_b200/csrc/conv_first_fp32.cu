@@ -300,17 +300,25 @@ static int first_dw_most(const AetherConvDesc& d) {
     const int rows = fd_rows(d.Cin, d.fH);
     return num_sms() * fp_ctas(d.Cin * d.fW * rows) / (d.fH / rows);
 }
-// Against the GEMM of simt_dw_kernel, which fills its tiles of 64 columns where there are that many, and rounds less: 12 products a nanosecond there, a
-// step of all pieces in 12 ns per value here.  (us: 60 x 50x50 3->192 79 / 97, 60 x 64x64 3->208 167 / 155, 103 x 15x15 1->208 5x5 21 / 24, 128 x 56x56 1->224 5x5
-// 226 / 193; with fewer channels, one input channel or in place of smallc_dw_kernel this one is 1.05 to 3 times as fast.)
+// Against the kernels that took these layers before (us): smallc_dw_kernel 10 and a product in 1/15 or, of up to 64 values, 1/6.8 ps, the GEMM of simt_dw_kernel 10 and
+// a product of its tiles in 1/14 ps, 1/23 of four input channels.  Here a step of all pieces takes 10.7 ns per value, half of that where two CTAs share an SM, unless
+// dy, read again by every row of a filter of more than 27 values, takes longer (3.1 TB/s), and the sums of a CTA meet in 1.65 ns per value and thread.  (us, there /
+// here: 300 x 16x18 4->256 5x5 123 / 213, 100 x 28x28 4->128 5x5 62 / 104, 84 x 116x88 2->54 5x5 227 / 422, 60 x 64x64 3->208 167 / 155, 128 x 56x56 1->224
+// 5x5 226 / 193.  Over 972 layers at most 38 % behind the faster one, 1.0 % in the mean, here everywhere 86 and 2.7 %.  Few values or channels: always here.)
 bool first_fp32_dw_eligible(const AetherConvDesc& d) {
     if (!first_fp32_eligible(d)) return false;
-    const int K = d.Cin * d.fH * d.fW;
-    if (K < 25 || d.Cout <= 160 || smallc_conv_eligible(d)) return true;
+    const int K = d.Cin * d.fH * d.fW, rows = fd_rows(d.Cin, d.fH), values = d.Cin * d.fW * rows;
+    if (K < 25 || d.Cout <= 32) return true;
     FirstWalk g;
     unsigned steps;
     first_walk(d, nullptr, first_dw_most(d), g, &steps);
-    return 1.0 * steps * d.Cin * d.fW * fd_rows(d.Cin, d.fH) * 12e3 < 1.0 * d.S * g.Ho * g.Wo * (ceil_div(K, 32) * 32) * (ceil_div(d.Cout, 64) * 64) / 12.0;
+    const double pixels = 1.0 * d.S * g.Ho * g.Wo, ragged = d.Cout % 4 ? 1.0 : 0.0;
+    const double walk = steps * values * (fp_ctas(values) == 2 ? 5.6e-3 : 10.7e-3) * (1.0 + 0.14 * ragged);
+    const double reads = d.fH / rows * pixels * d.Cout * 4.0 * 0.32e-6 * (1.0 + 0.26 * ragged);
+    const double here = 5.4 + (walk > reads ? walk : reads) + g.lanes * K * 1.65e-3;
+    const double there = smallc_conv_eligible(d) ? 10.0 + pixels * K * d.Cout * (K > 64 ? 1e-6 / 15.0 : 1e-6 / 6.8)
+                                                 : 10.0 + pixels * (ceil_div(K, 32) * 32) * (ceil_div(d.Cout, 64) * 64) * (d.Cin == 4 && !ragged ? 1e-6 / 23.0 : 1e-6 / 14.0);
+    return here < there;
 }
 // Against first_tc_bwd_filter without a copy of dy: 10.5 products a nanosecond here, 36 ns per 1000 pixels and a fixed part that is 3.5 us longer there.
 // (us: 14 x 8x9 3->16 10.8 there, 6.5 here; 211 x 28x28 3->16 16.9 / 13.2, 300 x 40x40 1->16 26.0 / 14.5, 512 x 28x28 1->32 23.4 / 21; 128 x 32x32 3->32 14.3 / 14.8,

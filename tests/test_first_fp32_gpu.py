@@ -11,7 +11,9 @@ pytestmark = pytest.mark.gpu
 # (S, H, W, Cin, Cout, f, sH, padH, padW)
 SHAPES = [(128, 32, 32, 3, 32, 3, 1, 1, 1), (7, 13, 11, 3, 20, 3, 1, 0, 0), (40, 9, 70, 1, 16, 3, 1, 1, 1), (3, 30, 31, 1, 208, 3, 1, 1, 1), (90, 28, 28, 2, 50, 3, 1, 1, 1),
           (5, 17, 19, 4, 33, 3, 2, 1, 1), (20, 24, 29, 1, 80, 5, 1, 2, 2), (6, 21, 23, 3, 28, 5, 1, 0, 0), (4, 15, 18, 2, 37, 5, 1, 4, 3), (3, 12, 40, 4, 17, 5, 3, 2, 2),
-          (200, 7, 7, 3, 64, 5, 1, 0, 0), (1, 3, 3, 3, 4, 3, 1, 0, 0), (2, 5, 6, 1, 1, 5, 1, 2, 2), (300, 20, 20, 3, 3, 3, 1, 2, 0), (2, 64, 64, 3, 256, 3, 1, 1, 1)]
+          (200, 7, 7, 3, 64, 5, 1, 0, 0), (1, 3, 3, 3, 4, 3, 1, 0, 0), (2, 5, 6, 1, 1, 5, 1, 2, 2), (300, 20, 20, 3, 3, 3, 1, 2, 0), (2, 64, 64, 3, 256, 3, 1, 1, 1),
+          # (the filter gradient goes the other way)
+          (30, 16, 18, 4, 256, 5, 1, 2, 2), (40, 20, 21, 2, 54, 5, 1, 2, 2), (30, 28, 28, 4, 128, 5, 1, 2, 2)]
 
 
 @pytest.mark.parametrize("S,H,W,Cin,Cout,f,sH,ph,pw", SHAPES)
