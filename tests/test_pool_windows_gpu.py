@@ -37,7 +37,7 @@ def test_windows_that_leave_cells_over(C, S, H, W, fH, fW, kind):
     assert bool(((dx.double() - want).abs() <= tol * want.abs()).all())
 
 
-@pytest.mark.parametrize("rows,C,shift", [(1000, 61, 0), (1001, 3, 0), (77, 1, 0), (512, 30, 0), (333, 7, 1)])
+@pytest.mark.parametrize("rows,C,shift", [(1000, 61, 0), (1001, 3, 0), (77, 1, 0), (512, 30, 0), (333, 7, 1), (255, 3, 0), (256, 3, 0), (769, 1, 0), (20, 5, 0)])
 def test_channel_passes_of_ragged_rows(rows, C, shift):
     """shift: arrays that begin between two 16-byte boundaries."""
     import torch
