@@ -57,6 +57,33 @@ def test_one_launch_against_two(S, H, W, Cin, Cout, f, pad, alpha):
     assert _lib.device_status() == 0
 
 
+@pytest.mark.parametrize("S,H,W,Cin,Cout", [(9, 12, 14, 3, 32), (40, 16, 16, 1, 192), (20, 16, 16, 32, 64), (9, 10, 10, 64, 132)])
+def test_values_that_are_not_finite(S, H, W, Cin, Cout):
+    """Infinities and NaN in the images and in the filter: in the same places as from the convolution and the pass behind it, with the signs."""
+    import torch
+    lib = _lib.lib()
+    d = _lib.AetherConvDesc(S, H, W, Cin, Cout, 3, 3, 1, 1, 1, 1, _lib.MATH_MODES["bf16"])
+    g = torch.Generator(device="cuda").manual_seed(Cout)
+    R = lambda *shape: torch.randn(shape, generator=g, device="cuda")
+    x, w, b, gamma, beta, mean, var = R(S, H, W, Cin), R(3, 3, Cin, Cout), R(Cout), R(Cout), R(Cout), R(Cout), R(Cout).abs() + 0.1
+    x[0, 2, 3, 0], x[1, H - 1, W - 1, Cin - 1], x[2, 0, 0, 0], x[S - 1, 5, 6, 0] = float("inf"), -float("inf"), float("nan"), float("inf")
+    w[1, 1, 0, Cout - 1], w[0, 2, Cin - 1, 1] = float("inf"), float("nan")
+    n = max(lib.aether_conv2d_workspace_bytes(d), 16)
+    ws, ws2 = (torch.zeros(n, dtype=torch.uint8, device="cuda") for _ in range(2))
+    bws = torch.empty(lib.aether_bn_workspace_bytes(S * H * W, Cout), dtype=torch.uint8, device="cuda")
+    y, two, one = torch.empty((S, H, W, Cout), device="cuda"), torch.empty((S, H // 2, W // 2, Cout), device="cuda"), torch.empty((S, H // 2, W // 2, Cout), device="cuda")
+    P, st = (lambda t: t.data_ptr()), torch.cuda.current_stream().cuda_stream
+    assert lib.aether_conv2d_fwd(d, P(x), P(w), P(b), P(y), P(ws), n, st) == 0
+    assert lib.aether_chain_fwd(P(y), None, 0, P(gamma), P(beta), P(mean), P(var), None, None, None, None, None, P(two), None, S, H, W, Cout, 2, 2, 1e-5, 0.9, 0.1, None, 0, None, 0, P(bws),
+                                bws.numel(), st) == 0
+    assert lib.aether_conv2d_pool_fwd(d, P(x), P(w), P(b), P(gamma), P(beta), P(mean), P(var), 1e-5, 0.1, P(one), None, 0, P(ws2), n, 0, st) == 0
+    assert bool(two.isnan().any()) and bool(two.isinf().any()) and bool(two[3, :, :, 2:Cout - 1].isfinite().all())
+    finite = two.isfinite()
+    assert torch.equal(one.isnan(), two.isnan()) and torch.equal(one.nan_to_num(0.0)[~finite], two.nan_to_num(0.0)[~finite])
+    assert float((one - two)[finite].norm() / two[finite].norm()) <= 9 * Cin * 2.0**-23
+    assert _lib.device_status() == 0
+
+
 def test_refused_where_the_epilogue_does_not_fit():
     lib = _lib.lib()
     for S, H, W, Cin, Cout, f, s, pad, mode in [(2, 7, 8, 64, 64, 3, 1, 1, "bf16"), (2, 8, 7, 3, 32, 3, 1, 1, "bf16"), (2, 8, 8, 64, 64, 3, 1, 1, "tf32"), (2, 8, 8, 64, 64, 3, 2, 1, "bf16"), (2, 8, 8, 64, 1028, 1, 1, 0, "bf16")]:

@@ -30,3 +30,23 @@ def test_dense_forward(rows, K, N):
         assert bool(((y.double() - want).abs() <= (K + 8) * 2.0**-23 * size).all())
         outs.append(y)
     assert torch.equal(*outs) and _lib.device_status() == 0
+
+
+def test_values_that_are_not_finite():
+    """An infinity and a NaN in two CTAs' parts of K: in the rows that hold them, as in float64."""
+    import torch
+    lib = _lib.lib()
+    rows, K, N = 130, 2048, 64
+    d = _lib.AetherConvDesc(rows, 1, 1, K, N, 1, 1, 1, 1, 0, 0, _lib.MATH_MODES["bf16"])
+    g = torch.Generator(device="cuda").manual_seed(4)
+    x, w, b = torch.randn((rows, K), generator=g, device="cuda").bfloat16().float(), torch.randn((K, N), generator=g, device="cuda").bfloat16().float(), torch.randn((N,), generator=g, device="cuda")
+    x[3, 7], x[4, K - 1], x[5, 1000], x[6, 0], x[6, K - 2], x[129, 512] = float("inf"), -float("inf"), float("nan"), float("inf"), -float("inf"), float("inf")
+    n = lib.aether_conv2d_workspace_bytes(ctypes.byref(d))
+    ws, y = torch.empty(n, dtype=torch.uint8, device="cuda"), torch.empty((rows, N), device="cuda")
+    P = lambda t: t.data_ptr()
+    assert lib.aether_conv2d_fwd(ctypes.byref(d), P(x), P(w), P(b), P(y), P(ws), n, torch.cuda.current_stream().cuda_stream) == 0
+    want = x.double() @ w.double() + b.double()
+    finite = want.isfinite()
+    assert int((~finite).any(1).sum()) == 5 and torch.equal(y.isnan(), want.isnan()) and torch.equal(y.isposinf(), want.isposinf()) and torch.equal(y.isneginf(), want.isneginf())
+    size = (x.double().abs() @ w.double().abs() + b.double().abs())[finite]
+    assert bool(((y.double() - want)[finite].abs() <= (K + 8) * 2.0**-23 * size).all()) and _lib.device_status() == 0

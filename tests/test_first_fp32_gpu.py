@@ -43,3 +43,31 @@ def test_first_layers_in_single_precision(S, H, W, Cin, Cout, f, sH, ph, pw):
         for got, want, most, r in zip((y, dw, db), both(x, w, b, dy), both(x.abs(), w.abs(), b.abs(), dy.abs()), rounds):
             assert bool(((got.double() - want).abs() <= r * 2.0 ** -24 * most + 1e-30).all())
     assert lib.aether_device_status() == 0
+
+
+@pytest.mark.parametrize("S,H,W,Cin,Cout,f", [(6, 13, 17, 3, 20, 3), (3, 20, 33, 1, 16, 5), (4, 11, 12, 4, 33, 3), (5, 9, 30, 2, 7, 3)])
+def test_values_that_are_not_finite(S, H, W, Cin, Cout, f):
+    """Infinities and NaN in the images reach the pixels whose windows hold them and the filter values that they meet, at the images' edges, too."""
+    import torch
+    lib, p = _lib.lib(), f // 2
+    g = torch.Generator(device="cuda").manual_seed(S + Cout)
+    new = lambda *shape: torch.randn(shape, generator=g, device="cuda")
+    x, w, b, dy = new(S, H, W, Cin), new(f, f, Cin, Cout), new(Cout), new(S, H, W, Cout)
+    x[0, 0, 0, 0], x[1, H - 1, W - 1, Cin - 1], x[2, 4, 5, 0] = float("inf"), float("nan"), -float("inf")
+    d = _lib.AetherConvDesc(S, H, W, Cin, Cout, f, f, 1, 1, p, p, _lib.MATH_MODES["fp32"])
+    n = lib.aether_conv2d_workspace_bytes(d)
+    ws = torch.empty(n + 16, dtype=torch.uint8, device="cuda")
+    y, dw, db = torch.empty_like(dy), torch.empty_like(w), torch.empty_like(b)
+    stream = torch.cuda.current_stream().cuda_stream
+    assert lib.aether_conv2d_fwd(d, x.data_ptr(), w.data_ptr(), b.data_ptr(), y.data_ptr(), ws.data_ptr(), n, stream) == 0
+    assert lib.aether_conv2d_bwd(d, x.data_ptr(), dy.data_ptr(), w.data_ptr(), None, dw.data_ptr(), db.data_ptr(), ws.data_ptr(), n, 0, stream) == 0
+    pads = torch.nn.functional.pad(x.double(), (0, 0, p, p, p, p))
+    taps = [[pads[:, i:i + H, j:j + W] for j in range(f)] for i in range(f)]
+    want = b.double() + sum(taps[i][j] @ w[i, j].double() for i in range(f) for j in range(f))
+    grad = torch.stack([torch.stack([taps[i][j].reshape(-1, Cin).T @ dy.double().reshape(-1, Cout) for j in range(f)]) for i in range(f)])
+    for got, exact in ((y, want), (dw, grad)):
+        finite = exact.isfinite()
+        assert torch.equal(got.isnan(), exact.isnan()) and torch.equal(got.isposinf(), exact.isposinf()) and torch.equal(got.isneginf(), exact.isneginf()) and not bool(finite.all())
+        if bool(finite.any()):
+            assert float((got.double() - exact)[finite].norm() / exact[finite].norm()) <= 1e-5
+    assert bool(want[:, :, :, 0].isfinite().any()) and _lib.device_status() == 0
