@@ -30,9 +30,9 @@ namespace aether {
 // kernel back (896 x 32x32 3->32 35 -> 29 us, 64 and 128 channels 1-4 %), two with statistics, whose epilogue is the longer
 // chain (128 x 32x32 3->32 10.9 us, 12.0 with three), and for windows of more than 48 values, which a thread keeps in registers: three groups
 // leave it 80 of those (84 bytes spilled; 512 x 32x32 1->64 7x7 33.7 us, 31.6 with two groups, 64 x 64x64 4->32 4x4 19.8 / 18.9).  The pooling epilogue is the
-// longer chain, too: four teams beside two groups (three and three: 784 x 32x32 3->128 30 us, 27.7 so; 1800 x 28x28 1->32 51.6 / 49.5).
+// longer chain, too: four teams beside two groups (three and three: 1800 x 28x28 1->32 51.6 us, 49.5 so), as far as there are accumulators for them.
 __host__ __device__ static constexpr int ft_prod_warps(bool stats, int KP, bool pooled) { return stats || KP > 48 || pooled ? 8 : 12; }
-__host__ __device__ static constexpr int ft_teams(bool pooled) { return pooled ? 4 : 2; }       // of four epilogue warps
+__host__ __device__ static constexpr int ft_teams(bool pooled) { return pooled ? 4 : 2; }       // of four epilogue warps, at most
 __host__ __device__ static constexpr int ft_threads(bool stats, int KP, bool pooled) { return 32 * (ft_prod_warps(stats, KP, pooled) + 1 + 4 * ft_teams(pooled)); }      // producers, MMA issuer, epilogue
 static constexpr int FT_STAGE_BYTES = 128 * 128;                             // 128 pixel rows of 128 bytes
 static constexpr int FT_TAIL = 2048;                                         // barriers, TMEM pointer, bias, tap table
@@ -148,8 +148,8 @@ __device__ __forceinline__ float stats_tree(const float (&v)[8]) { return ((v[0]
 // POOLED (inference): the epilogue applies the Batch_Norm behind the layer by its running statistics, the (leaky) ReLU behind that and a 2x2
 // max pooling, and writes the pooled values and their bf16 operand copy only, a quarter of the pixels.  A tile is 32 windows, whose four pixels are
 // four rows of the staged tile, which takes the sums as they are: a thread reads four channels of a window again and keeps their coefficients, the eight lanes of
-// a window read whole lines of banks.  (896 x 32x32 3->32: 39.7 us, 30 and 36 for the convolution and the pass over its output; with the activation
-// before the staging, eight channels a thread and two teams 47, 784 x 32x32 3->128 39 against 27.7.)
+// a window read whole lines of banks.  (us, with the operand copy, against the convolution and the pass over its output: 900 x 32x32 3->32 35.6 / 66.6, 784 x 32x32
+// 3->128 72.6, 900 x 32x32 3->192 153 / 433 on two teams; with the activation before the staging, eight channels a thread and two teams the first 47.)
 template <bool STATS, int KP, int CIN, bool POOLED = false>
 __global__ void __launch_bounds__(ft_threads(STATS, KP, POOLED), 1) first_conv_kernel(const __grid_constant__ FirstParams p) {
     constexpr int FT_PROD_WARPS = ft_prod_warps(STATS, KP, POOLED), TEAMS = ft_teams(POOLED);

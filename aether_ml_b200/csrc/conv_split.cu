@@ -22,11 +22,11 @@
 // channels with zeros behind the last: channel counts need not be multiples of anything.  A strided layer's x is stored by
 // phases, so that a tap's pixels lie side by side (element strides in the tensor map halve the copies' rate).
 // Measured on B200, forward + backward, CUDA cores / this file: 40 x 33x32 64->128 442 / 131 us, 96 x 28x28 32->64 207 / 100, 100 x 57x45
-// 48->72 stride 2 431 / 187 (one set of inputs; three in turn, as a program's arrays come: 211 / 104, 433 / 206).  No unit is saturated: the
-// tensor pipe is 24-48 % busy, L1 and shared memory 40-67 %, DRAM 6-31 %.  What bounds it is shared memory: the MMAs take 224 clocks for a step of 64 columns
-// by themselves (28 KB of operands), and with the copies' writes (18 KB a step) 340; about 150 bytes per clock in all, forward, dX and dW alike.  Neither the number of
-// threads that issue nor the stores matter then (both measured, two teams of summing warps and products spread over two threads: no change; all
-// sums of a stage side by side in 192 columns: 30 -> 35-39 us, TMEM gives some 110 bytes per clock beside the MMAs).
+// 48->72 stride 2 431 / 187 (one set of inputs; three in turn, as a program's arrays come: 211 / 104, 433 / 206).  No counter is saturated: the
+// tensor pipe is 24-48 % busy, L1 and shared memory 40-67 %, DRAM 6-31 %.  By the clock, the MMAs take 224 for a step of 64 columns by themselves (28 KB of
+// operands) and 340 with the copies' writes beside them (18 KB a step): some 150 bytes per clock through shared memory, forward, dX and dW alike, although its
+// counters show room.  What holds a step up there is not settled.  Not the number of threads that issue and not the stores (two teams of summing warps and products
+// spread over two threads: no change); all sums of a stage side by side in 192 columns: 30 -> 35-39 us, TMEM gives some 110 bytes per clock beside the MMAs.
 #include <string.h>
 
 #include <cuda_bf16.h>
@@ -889,7 +889,7 @@ static SplitPlan compute_split_plan(const AetherConvDesc& d) {
     pl.cblocks = ceil_div(d.Cin, pl.kc_in);
     pl.U = pl.taps * pl.cblocks;
     pl.ldn = (d.Cout + 3) / 4 * 4;
-    // dW: 64 or 128 channels of dy per unit.  Shared memory is what bounds the kernel (some 150 bytes per clock, copies and operand reads together): per
+    // dW: 64 or 128 channels of dy per unit.  Copies and operand reads together go at some 150 bytes per clock whichever it is: per
     // step and 128 columns 40 KB of operands and 24 KB of copies, 56 and 36 in two units.  A stage takes 0.74 / 1.16 us, and the partial
     // sums of a split are written and read again: 64 x 28x28 128->128 96 -> 78 us, 40 x 33x32 64->128 5x5 106 -> 82, 100 x 57x45 48->72 stride 2
     // 74 -> 68; 200 x 14x14 72->144 90 -> 94, 16 x 7x7 256->256 16.2 -> 17.5 and 12 x 24x24 16->146 18.5 -> 20.3 stay with 64.
