@@ -1462,14 +1462,44 @@ static int launch_igemm_pooled(const IgemmParams& p, bool narrow, cudaStream_t s
     return launch_igemm_k<false, NT, false, false, false, 128, true>(p, st);
 }
 
-// CTAs that share a tile's K chunks (SPLIT): as many as there are SMs for, with four chunks each at least, where that takes out twenty chunks of a CTA
-// (a chunk is 0.16 us, the exchange 1.5; 896 x 2048->256 by two, 16 chunks less, 8.9 / 9.0 us).  A GPC takes whole clusters, so that of 148 SMs some 130 are there
-// for eight CTAs each.  (us: 256 x 3136->128 11.8 / 7.8, 128 x 2048->256 9.3 / 7.5, 256 x 8192->1024 24 / 16.7.)
+// Clusters of `size` CTAs of the SPLIT kernel that this device runs at once (looked up once per device and size): a GPC takes whole clusters, and how many SMs it has
+// differs from one GPC and one GPU to the next.  74, 33 and 15 clusters of two, four and eight where this was measured.
+static int split_clusters(int size) {
+    static std::atomic<int> cache[AE_MAX_DEVICES][4];        // by log2 of the size, plus one
+    const int dev = current_device(), k = size == 2 ? 1 : size == 4 ? 2 : 3;
+    const int held = cache[dev][k].load(std::memory_order_relaxed);
+    if (held > 0) return held - 1;
+    const auto kernel = igemm_conv_kernel<false, 32, false, false, false, 128, false, true>;
+    constexpr int SMEM = IgemmCfg<32, false>::SMEM_BYTES + IGEMM_SPLIT_BYTES;
+    int clusters = 0;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM) == cudaSuccess) {
+        cudaLaunchConfig_t cfg;
+        memset(&cfg, 0, sizeof(cfg));
+        cfg.gridDim = dim3(size * num_sms(), 1, 1);
+        cfg.blockDim = dim3(IGEMM_THREADS, 1, 1);
+        cfg.dynamicSmemBytes = SMEM;
+        cudaLaunchAttribute attr;
+        attr.id = cudaLaunchAttributeClusterDimension;
+        attr.val.clusterDim.x = size;
+        attr.val.clusterDim.y = 1;
+        attr.val.clusterDim.z = 1;
+        cfg.attrs = &attr;
+        cfg.numAttrs = 1;
+        if (cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) != cudaSuccess) clusters = 0;
+    }
+    (void)cudaGetLastError();
+    cache[dev][k].store(clusters + 1, std::memory_order_relaxed);
+    return clusters;
+}
+
+// CTAs that share a tile's K chunks (SPLIT): as many as there are SMs for in one round of clusters, with four chunks each at least, where that takes out twenty chunks of a
+// CTA (a chunk is 0.16 us, the exchange 1.5; 896 x 2048->256 by two, 16 chunks less, 8.9 / 9.0 us).  (us: 256 x 3136->128 11.8 / 7.8, 128 x 2048->256 9.3 / 7.5, 256 x
+// 8192->1024 24 / 16.7; 512 x 3136->128, 16 tiles, 16.1 / 13.3 by four, 18.4 by eight in two rounds.)
 static int k_splits(long long tiles, int kchunks) {
     if (kchunks < 23) return 1;
     const int room = num_sms() * 7 / 8;
     for (int s = 8; s > 1; s >>= 1)
-        if (tiles * s <= room && kchunks >= 4 * s && kchunks - kchunks / s >= 20) return s;
+        if (tiles * s <= room && kchunks >= 4 * s && kchunks - kchunks / s >= 20 && tiles <= split_clusters(s)) return s;
     return 1;
 }
 

@@ -10,7 +10,7 @@ from aether_ml_b200 import _lib
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("rows,K,N", [(100, 3136, 128), (256, 2048, 256), (300, 1800, 320), (500, 2600, 416), (1, 5000, 32), (129, 1028, 36), (40, 1024, 64), (128, 960, 512)])
+@pytest.mark.parametrize("rows,K,N", [(100, 3136, 128), (256, 2048, 256), (300, 1800, 320), (500, 2600, 416), (1, 5000, 32), (129, 1028, 36), (40, 1024, 64), (128, 960, 512), (512, 3136, 128), (480, 4096, 128), (512, 2112, 256), (500, 3000, 512)])
 def test_dense_forward(rows, K, N):
     import torch
     lib = _lib.lib()
